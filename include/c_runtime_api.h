@@ -271,6 +271,7 @@ int DLGpuAdam_o(void ****n4list, const void ***indexlist, const int count,
  * `nccl_id_path` names a file rank 0 creates; the other ranks wait for it, at most
  * TINYFLOW_DP_INIT_TIMEOUT_S seconds (default 120).  Returns 0 on success. */
 int TfDpInit(int rank, int world_size, const char *nccl_id_path);
+int TfDpActive(void);   /* 1 between TfDpInit and TfDpShutdown */
 /* Flush every pending bucket and make the stream wait for the updates (end of a
  * step).  A blocking host<->device DLArrayCopyFromTo does the same, so a training
  * loop that knows nothing of this layer stays correct.  Returns -1 if NCCL reported
@@ -297,6 +298,31 @@ int TfDpPlanBucketsTail(const long long *counts, int n, long long capacity_float
  * elements (-1 beyond that).  All calls share the array, so calls that overlap on the GPU race.  The first
  * call on a device resolves the array's address and should precede any stream capture. */
 int DLGpuReduceSumAllStatic(const DLArrayHandle input, DLArrayHandle output, void **cudaStream);
+
+/* x + c and x * c with c the one element of a device array (what a graph's shape-(1,) operand is). */
+int TfMatrixElementwiseAddByArray(const DLArrayHandle input, const DLArrayHandle scalar, DLArrayHandle output, void **cudaStream);
+int TfMatrixMultiplyByArray(const DLArrayHandle input, const DLArrayHandle scalar, DLArrayHandle output, void **cudaStream);
+
+/* One launch for the optimiser updates of many tensors; per tensor the same arithmetic as DLGpuSgdUpdate, and as
+ * DLGpuAdam_mv followed by DLGpuAdam.  Refused while the data-parallel exchange is active. */
+int TfSgdUpdateMany(const DLArrayHandle *w, const DLArrayHandle *g, int count, float lr, void **cudaStream);
+int TfAdamUpdateMany(const DLArrayHandle *w, const DLArrayHandle *m, const DLArrayHandle *v, const DLArrayHandle *g,
+                     int count, float b1, float b2, float b1t, float b2t, float e, float lr, void **cudaStream);
+
+/* Device-to-device copy enqueued on the stream; no host wait. */
+int TfArrayCopyOnStream(DLArrayHandle from, DLArrayHandle to, void **cudaStream);
+
+/* Recording a step and replaying it with one call.  Between Begin and End the calling thread issues the step's calls on
+ * the stream Begin returns; they are recorded, not executed.  The arrays the calls name have to outlive the recording.
+ * Calls that need the host in the middle (blocking copies, the legacy default stream) cannot be recorded: End returns 1
+ * then, as it does with keep = 0.  TfStepReplay: `seeds` for the dropout calls in order, Adam's beta powers of this step;
+ * 0 = enqueued, 1 = out of date, record again (buffers moved or the arithmetic changed), 2 = not now (per-kernel timing
+ * or the data-parallel exchange is on): use ordinary calls. */
+int TfStepRecordBegin(void **graph, void **stream_cell);
+int TfStepRecordEnd(void **graph, int keep);
+int TfStepReplay(void *graph, const unsigned *seeds, int nseeds, float b1t, float b2t,
+                 const DLArrayHandle *params, int nparams, void **cudaStream);
+int TfStepGraphFree(void *graph);
 
 /* Test / profiling hooks. */
 int TfPoolingArgmax(const DLArrayHandle input, int32_t *indices_dev, void ***cudnnlist,

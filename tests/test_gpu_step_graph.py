@@ -1,0 +1,125 @@
+"""Recorded steps: a replay has to give the bits the ordinary calls give, whatever the caller does between steps."""
+import random
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 9
+
+
+def _train(monkeypatch, recorded, build, optimizer, between=None, fresh_batch=False):
+    from tinyflow_b200 import autodiff as ad, gpu_op, models, ndarray, step_graph
+    monkeypatch.setattr(step_graph, "ENABLED", recorded)
+    random.seed(3)
+    model = build(models)
+    ex = ad.Executor(model.loss, model.y, 0.001, None, None, None, optimizer=optimizer)
+    ctx = ndarray.gpu(0)
+    feed = {n: ndarray.array(v, ctx) for n, v in model.init_params(seed=5).items()}
+    for var in list(feed):
+        for moment in ex.Variable_node_to_mv.get(var, ()):
+            feed[moment] = ndarray.array(np.zeros(model.param_shapes[var], np.float32), ctx)
+    all_feeds = dict(feed)
+    X, Y = models.synthetic_batch(model, seed=8)
+    x, y = ndarray.array(X, ctx), ndarray.array(Y, ctx)
+    losses = []
+    for step in range(STEPS):
+        if fresh_batch:
+            x = ndarray.array(np.roll(X, step, axis=0), ctx)
+        all_feeds[model.X], all_feeds[model.y_] = x, y
+        if between:
+            between(step, model, ex, all_feeds, x)
+        loss, _ = ex.run(all_feeds)
+        losses.append(loss)
+    gpu_op.device_synchronize()
+    replayed = any(f.recording or any(b.recording for b in f.batches.values()) for f in ex._recordings.sets.values())
+    return [v.asnumpy() for v in losses], {n.name: v.asnumpy() for n, v in all_feeds.items() if n.isw == 1}, replayed
+
+
+def _same(a, b):
+    for la, lb in zip(a[0], b[0]):
+        np.testing.assert_array_equal(la, lb)
+    for name in a[1]:
+        np.testing.assert_array_equal(a[1][name], b[1][name], err_msg=name)
+
+
+BUILDS = {
+    "mlp": lambda m: m.mlp(batch=33),
+    "lenet5": lambda m: m.lenet5(batch=9),
+    "vgg16": lambda m: m.vgg16(batch=8, classes=20, image=32),                  # dropout: new seeds every step
+    "resnet50": lambda m: m.resnet50(batch=16, classes=10, image=64),           # the fused and the held-back calls
+    "inceptionv3": lambda m: m.inceptionv3(batch=2, classes=10, image=107),
+}
+
+
+@pytest.mark.parametrize("optimizer", ["sgd", "adam"])
+@pytest.mark.parametrize("name", sorted(BUILDS))
+def test_a_replayed_step_has_the_bits_of_the_ordinary_one(lib_path, monkeypatch, name, optimizer):
+    want = _train(monkeypatch, False, BUILDS[name], optimizer)
+    got = _train(monkeypatch, True, BUILDS[name], optimizer)
+    assert got[2] and not want[2]
+    _same(got, want)
+
+
+def _overwrite_inputs(step, model, ex, feed, x):
+    x[:] = np.random.RandomState(step).rand(*x.shape).astype(np.float32)
+
+
+def _overwrite_a_parameter(step, model, ex, feed, x):
+    if step in (5, 7):
+        node = next(iter(model.param_shapes))
+        feed[node][:] = (0.5 if step == 5 else 40.0) * feed[node].asnumpy()
+
+
+def _change_the_rate(step, model, ex, feed, x):
+    if step == 6:
+        for node in ex.optimizer_nodes:
+            node.learning_rate = 0.01
+
+
+_held = []
+
+
+def _hold_values(step, model, ex, feed, x):
+    if step == 5:
+        _held.append((ex.value_of(model.y), ex.value_of(model.y).asnumpy()))
+    if step == 8:
+        view, copy = _held.pop()
+        np.testing.assert_array_equal(view.asnumpy(), copy)          # later steps left it alone
+
+
+@pytest.mark.parametrize("between", [_overwrite_inputs, _overwrite_a_parameter, _change_the_rate, _hold_values])
+@pytest.mark.parametrize("name", ["mlp", "resnet50"])
+def test_what_a_caller_does_between_steps_reaches_the_replay(lib_path, monkeypatch, name, between):
+    _same(_train(monkeypatch, True, BUILDS[name], "sgd", between), _train(monkeypatch, False, BUILDS[name], "sgd", between))
+
+
+@pytest.mark.parametrize("name", ["mlp", "vgg16"])
+def test_new_mini_batch_arrays_every_step(lib_path, monkeypatch, name):
+    want = _train(monkeypatch, False, BUILDS[name], "sgd", fresh_batch=True)
+    got = _train(monkeypatch, True, BUILDS[name], "sgd", fresh_batch=True)
+    assert got[2]
+    _same(got, want)
+
+
+@pytest.mark.parametrize("count", [1, 5, 400])
+def test_many_updates_in_one_launch(lib_path, count):
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, stream, rng = nd.gpu(0), gpu_op.create_cudaStream(), np.random.RandomState(count)
+    sizes = [int(s) for s in rng.choice([1, 3, 4, 127, 4095, 4096, 4097, 20000], size=count)]
+    host = [[rng.randn(n).astype(np.float32) for n in sizes] for _ in range(2)] + [[np.abs(rng.randn(n)).astype(np.float32) for n in sizes] for _ in range(2)]
+    w, g, m, v = ([nd.array(a, ctx) for a in col] for col in host)
+    w2, m2, v2 = ([nd.array(a, ctx) for a in host[k]] for k in (0, 2, 3))
+    gpu_op.sgd_update_many(gpu_op.handle_array(w), gpu_op.handle_array(g), 0.1, stream)
+    for a, b in zip(w2, g):
+        gpu_op.sgd_update(a, b, 0.1, stream)
+    for a, b in zip(w, w2):
+        np.testing.assert_array_equal(a.asnumpy(), b.asnumpy())
+    gpu_op.adam_update_many(*(gpu_op.handle_array(c) for c in (w, m, v, g)), 0.9, 0.999, 0.9, 0.999, 1e-8, 0.01, stream)
+    for a, b, c, d in zip(w2, m2, v2, g):
+        gpu_op.adam_mv(b, c, d, 0.9, 0.999, stream)
+        gpu_op.adam_compute(a, b, c, 0.9, 0.999, 1e-8, 0.01, stream)
+    for one, many in ((w, w2), (m, m2), (v, v2)):
+        for a, b in zip(one, many):
+            np.testing.assert_allclose(a.asnumpy(), b.asnumpy(), rtol=2e-6, atol=1e-7)

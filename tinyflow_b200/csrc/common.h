@@ -10,6 +10,8 @@
 
 namespace tf {
 
+struct StepGraph;          // a recorded training step (step_graph.cu)
+
 // ---- error reporting (never abort; entry points return -1) -----------------
 void set_error(const char* fmt, ...);
 #define TF_FAIL(...) do { ::tf::set_error(__VA_ARGS__); return -1; } while (0)
@@ -58,7 +60,8 @@ enum { kDeferReluBwd = 1, kDeferAdd = 2 };
 struct DeferredOp { int kind; const float* a; const float* b; float* out; int64_t n; cudaStream_t stream; };   // relu-bwd: a = the ReLU's input (mask), b = dy
 extern std::atomic<int> g_deferred_pending;
 void flush_deferred_slow();
-inline void flush_deferred() { if (g_deferred_pending.load(std::memory_order_relaxed)) flush_deferred_slow(); }
+extern thread_local StepGraph* t_recording;              // a thread that records a step has a slot of its own
+inline void flush_deferred() { if (g_deferred_pending.load(std::memory_order_relaxed) || t_recording) flush_deferred_slow(); }
 void flush_deferred_if_uses(const void* data);                  // the array free: only if `data` is an operand of the held-back call
 void defer_op(const DeferredOp& op);                            // the slot must be empty (flush first)
 bool take_deferred(int kind, const float* out, int64_t n, DeferredOp* op);   // the held-back op if it is of this kind and writes `out`; on true the slot stays locked ...
@@ -79,6 +82,7 @@ cudaStream_t last_compute_stream();         // launches a held-back kernel first
 void note_write(const void* p);
 uint64_t version_of(const void* p);
 inline float* out_f32(DLArray* a) { note_write(a->data); return (float*)a->data; }
+void invalidate_all_versions();             // every tensor counts as rewritten (a recording was abandoned)
 
 // ---- largest magnitude of a tensor, tracked by its producer ---------------------------
 // The tensor path scales each operand by a power of two chosen from max|x|.  Kernels that write a whole tensor
@@ -89,6 +93,13 @@ inline float* out_f32(DLArray* a) { note_write(a->data); return (float*)a->data;
 struct AmaxOut { uint32_t* word = nullptr; uint32_t* clear = nullptr; };
 AmaxOut amax_track_begin(const void* data);
 const uint32_t* amax_tracked(const void* data);
+// The maximum of a tensor that a recorded step reads before it writes it (see step_graph.cu): `carry` keeps the value
+// between replays, valid while the tensor's version is `*version`.
+struct AmaxCarry { const void* data; uint32_t* carry; const uint32_t* from; };       // from: the word the step itself writes, or null
+bool amax_take_carries(StepGraph* g, AmaxCarry* out, int max, int* count);           // the carries the recording g asked for
+bool amax_carry_valid(const void* data);
+void amax_set_carry_valid(const void* data);
+void bump_versions(const void* const* ptrs, size_t n);
 #ifdef __CUDACC__
 __device__ __forceinline__ uint32_t amax_bits(float v) { return __float_as_uint(fabsf(v)); }
 // Every thread of the block calls this once, after its last store, with the largest bit pattern it produced.
@@ -114,6 +125,26 @@ __device__ __forceinline__ void amax_commit(const AmaxOut& am, uint32_t m) {
 int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cudaStream_t s);
 void tc_note_relu_output(const void* node, const void* y);     // the plain ReLU of graph node `node` wrote y (after the version bump)
 bool contraction_path_is_cuda_cores();
+
+// ---- recording a training step for replay (step_graph.cu) -----------------------------------------
+// While a step is recorded, its calls (of ONE thread) run on a private stream in capture mode and nothing executes; the
+// launch sequence becomes a CUDA graph that later replays the step with one host call.  What a call would keep on the
+// host from one step to the next has to be fixed for the graph instead:
+//  * scratch blocks freed during the recording stay with the graph (its kernels use their addresses at every replay);
+//  * a tracked maximum gets a device word of the graph's own, cleared at the start of every replay, in place of the pair
+//    of words that alternates between calls; the maxima of tensors that a step reads before it writes them (parameters)
+//    are carried to the next replay in a word per tensor;
+//  * values that change from step to step (dropout seeds, Adam's bias corrections) are read from device words.
+uint32_t* recording_word();                        // a zeroed-per-replay device word of the graph being recorded
+void* recording_take_block(size_t bytes);          // a block of exactly this (rounded) size freed earlier in the recording, or nullptr
+void recording_keep_block(void* p, size_t bytes);  // instead of handing the block back to the pool
+const uint32_t* recording_seed(unsigned seed);     // device word that will hold the seed of this dropout call at every replay
+const float* recording_adam_corrections(float c1, float c2);   // two device words with this step's bias corrections
+void recording_note_launches(int n);
+void recording_note_write(const void* p);
+cudaStream_t recording_stream();
+// Buffers that outlive a call (packs, scratch) were reallocated or the arithmetic changed: recorded steps are out of date.
+void bump_layout_epoch();
 
 // ---- shapes -------------------------------------------------------------------
 inline int64_t numel(const DLArray* a) {
@@ -226,6 +257,7 @@ struct DropoutState {
   int kind;
   float p;
   unsigned long long seed;
+  const uint32_t* seed_word;   // a recorded step's seed of this replay, in device memory
   int64_t count;
 };
 

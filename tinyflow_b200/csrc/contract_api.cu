@@ -52,6 +52,7 @@ int TfTensorPathTimeoutProbe(long long limit_cycles, void** cudaStream) { return
 
 int TfSetContractionPath(int path) {
   TF_REQUIRE(path >= 0 && path <= 2, "TfSetContractionPath: path must be 0, 1 or 2");
+  if (g_path != path) bump_layout_epoch();
   g_path = path;
   return 0;
 }

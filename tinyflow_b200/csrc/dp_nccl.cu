@@ -399,6 +399,7 @@ int dp_flush(cudaStream_t s) {
   }
   return 0;
 }
+bool dp_active() { return g_dp.on; }
 // Called by host<->device copies: a step boundary for drivers that do not call TfDpFlush.
 int dp_flush_if_pending() {
   if (!g_dp.on) return 0;
@@ -501,6 +502,7 @@ int TfDpInit(int rank, int world_size, const char* nccl_id_path) {
   return 0;
 }
 
+int TfDpActive(void) { return dp_active() ? 1 : 0; }
 int TfDpFlush(void** cudaStream) {
   if (!g_dp.on) return 0;
   if (dp_flush(stream_of(cudaStream))) return -1;

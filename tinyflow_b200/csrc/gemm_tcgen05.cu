@@ -50,6 +50,7 @@ static uint64_t version_locked(const void* p) {
   return it->second;
 }
 void note_write(const void* p) {
+  if (t_recording) recording_note_write(p);
   std::lock_guard<std::mutex> lk(g_ver_mu);
   g_versions[p] = ++g_ver_counter;
 }
@@ -57,29 +58,54 @@ uint64_t version_of(const void* p) {
   std::lock_guard<std::mutex> lk(g_ver_mu);
   return version_locked(p);
 }
+void bump_versions(const void* const* ptrs, size_t n) {
+  std::lock_guard<std::mutex> lk(g_ver_mu);
+  for (size_t i = 0; i < n; ++i) g_versions[ptrs[i]] = ++g_ver_counter;
+}
+void invalidate_all_versions() {
+  std::lock_guard<std::mutex> lk(g_ver_mu);
+  for (auto& kv : g_versions) kv.second = ++g_ver_counter;
+}
 
-// producer-tracked maxima: two device words per tensor, handed out from zero-filled chunks
-struct AmaxSlot { uint32_t* words = nullptr; unsigned uses = 0; uint64_t version = 0; int cur = 0; };
+// producer-tracked maxima: two device words per tensor, handed out from zero-filled chunks.  A third word per tensor
+// carries the maximum from one replay of a recorded step to the next, and `rec_*` is the word of the recording that is
+// being made (valid inside it only).
+struct AmaxSlot {
+  uint32_t* words = nullptr; unsigned uses = 0; uint64_t version = 0; int cur = 0;
+  uint32_t* carry = nullptr; uint64_t carry_version = 0;
+  const StepGraph* rec = nullptr; uint32_t* rec_word = nullptr; uint64_t rec_version = 0; bool rec_wants_carry = false;
+};
 static std::unordered_map<const void*, AmaxSlot> g_amax;
 static uint32_t* g_amax_chunk = nullptr;
 static int g_amax_left = 0;
+static uint32_t* amax_chunk_words(int n) {
+  if (g_amax_left < n) {
+    const int kWords = 16384;
+    uint32_t* chunk = nullptr;
+    if (cudaMalloc((void**)&chunk, kWords * sizeof(uint32_t)) != cudaSuccess || cudaMemset(chunk, 0, kWords * sizeof(uint32_t)) != cudaSuccess ||
+        cudaDeviceSynchronize() != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    g_amax_chunk = chunk; g_amax_left = kWords;
+  }
+  uint32_t* w = g_amax_chunk;
+  g_amax_chunk += n; g_amax_left -= n;
+  return w;
+}
+static void amax_enter_recording(AmaxSlot& sl) {
+  if (sl.rec != t_recording) { sl.rec = t_recording; sl.rec_word = nullptr; sl.rec_version = 0; sl.rec_wants_carry = false; }
+}
 AmaxOut amax_track_begin(const void* data) {
   std::lock_guard<std::mutex> lk(g_ver_mu);
   AmaxSlot& sl = g_amax[data];
-  if (!sl.words) {
-    if (g_amax_left < 2) {
-      const int kWords = 16384;
-      uint32_t* chunk = nullptr;
-      if (cudaMalloc((void**)&chunk, kWords * sizeof(uint32_t)) != cudaSuccess || cudaMemset(chunk, 0, kWords * sizeof(uint32_t)) != cudaSuccess ||
-          cudaDeviceSynchronize() != cudaSuccess) {
-        cudaGetLastError();
-        g_amax.erase(data);
-        return AmaxOut{};
-      }
-      g_amax_chunk = chunk; g_amax_left = kWords;
-    }
-    sl.words = g_amax_chunk; g_amax_chunk += 2; g_amax_left -= 2;
+  if (t_recording) {
+    amax_enter_recording(sl);
+    sl.rec_word = recording_word();
+    sl.rec_version = version_locked(data);
+    return AmaxOut{sl.rec_word, nullptr};
   }
+  if (!sl.words && !(sl.words = amax_chunk_words(2))) return AmaxOut{};
   const int k = (int)(sl.uses++ & 1u);
   sl.cur = k;
   sl.version = version_locked(data);
@@ -88,8 +114,41 @@ AmaxOut amax_track_begin(const void* data) {
 const uint32_t* amax_tracked(const void* data) {
   std::lock_guard<std::mutex> lk(g_ver_mu);
   auto it = g_amax.find(data);
-  if (it == g_amax.end() || !it->second.words) return nullptr;
-  return it->second.version == version_locked(data) ? it->second.words + it->second.cur : nullptr;
+  if (it == g_amax.end()) return nullptr;
+  AmaxSlot& sl = it->second;
+  const uint64_t v = version_locked(data);
+  if (t_recording && sl.rec == t_recording && sl.rec_word && sl.rec_version == v) return sl.rec_word;
+  const uint32_t* found = sl.words && sl.version == v ? sl.words + sl.cur : (sl.carry && sl.carry_version == v ? sl.carry : nullptr);
+  if (!t_recording || !found) return found;
+  // read before the recorded step has written it: at a replay the value has to come from the step before
+  if (!sl.carry && !(sl.carry = amax_chunk_words(1))) return nullptr;
+  amax_enter_recording(sl);
+  sl.rec_wants_carry = true;
+  return sl.carry;
+}
+bool amax_take_carries(StepGraph* g, AmaxCarry* out, int max, int* count) {
+  std::lock_guard<std::mutex> lk(g_ver_mu);
+  *count = 0;
+  for (auto& kv : g_amax) {
+    AmaxSlot& sl = kv.second;
+    if (sl.rec != g) continue;
+    if (sl.rec_wants_carry) {
+      if (*count >= max) return false;
+      const bool rewritten = sl.rec_word && sl.rec_version == version_locked(kv.first);     // by a kernel that tracks its maximum, last
+      out[(*count)++] = AmaxCarry{kv.first, sl.carry, rewritten ? sl.rec_word : nullptr};
+    }
+    sl.rec = nullptr;
+  }
+  return true;
+}
+bool amax_carry_valid(const void* data) {
+  std::lock_guard<std::mutex> lk(g_ver_mu);
+  auto it = g_amax.find(data);
+  return it != g_amax.end() && it->second.carry && it->second.carry_version == version_locked(data);
+}
+void amax_set_carry_valid(const void* data) {
+  std::lock_guard<std::mutex> lk(g_ver_mu);
+  g_amax[data].carry_version = version_locked(data);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -1430,7 +1489,7 @@ int tensor_path_timeout_probe(long long limit_cycles, cudaStream_t s) {
 // Arithmetic of the tensor path: 0 = 3xFP16 (scaled fp16 hi/lo pairs, kind::f16), 1 = 3xTF32 (tf32 hi/lo pairs, kind::tf32).
 static std::atomic<int> g_arith{[] { const char* e = getenv("TINYFLOW_ARITH"); return (e && (!strcmp(e, "3xtf32") || !strcmp(e, "1"))) ? 1 : 0; }()};
 int tensor_arithmetic() { return g_arith.load(std::memory_order_relaxed); }
-void set_tensor_arithmetic(int a) { g_arith.store(a, std::memory_order_relaxed); }
+void set_tensor_arithmetic(int a) { if (g_arith.exchange(a, std::memory_order_relaxed) != a) bump_layout_epoch(); }
 
 // ---- schedule: whole waves of tiles, then the partial wave cut into equal per-CTA ranges of stages -------------------
 // Costs are in units of one stage of one tile.  Splitting the tail pays a fixed price per CTA (the partial sums make a
@@ -1565,6 +1624,7 @@ struct Pack {           // a packed operand living in pooled device memory
   uint32_t* words = nullptr;       // device: amax[0], amax[1] (alternating between uses), scale (float), spare
   unsigned uses = 0;
   int arith = kArithF16;           // element type of hi / lo
+  bool transient = false;          // belongs to one call (matrix products)
   long long rows = 0, cols = 0, pitch = 0;
   const void* src = nullptr; uint64_t version = 0; int tag = 0;   // cache key
   size_t bytes() const { return (size_t)rows * pitch * elem_of(arith); }
@@ -1572,13 +1632,17 @@ struct Pack {           // a packed operand living in pooled device memory
 };
 static int pack_alloc(Pack& pk, int ar, long long rows, long long cols, cudaStream_t s, int* oom) {
   long long pitch = round_up(cols, 64);
+  if (!pk.words && t_recording && pk.transient) {
+    for (int i = 0; i < 4; ++i) { uint32_t* w = recording_word(); if (!i) pk.words = w; }       // consecutive, cleared at every replay
+  }
   if (!pk.words) {
+    if (t_recording) TF_FAIL("a packed operand of a recorded step has never been packed before");    // its words could not be cleared now
     pk.words = (uint32_t*)pool_alloc(16);
     if (!pk.words || cudaMemsetAsync(pk.words, 0, 16, s) != cudaSuccess) { if (oom) *oom = 16; return 1; }
     pk.uses = 0;
   }
   if (pk.hi && pk.rows == rows && pk.pitch == pitch && pk.arith == ar) { pk.cols = cols; return 0; }
-  if (pk.hi) { pool_free(pk.hi); pool_free(pk.lo); pk.hi = pk.lo = nullptr; }
+  if (pk.hi) { pool_free(pk.hi); pool_free(pk.lo); pk.hi = pk.lo = nullptr; bump_layout_epoch(); }
   pk.rows = rows; pk.cols = cols; pk.pitch = pitch; pk.src = nullptr; pk.arith = ar;
   pk.hi = pool_alloc(pk.bytes());
   pk.lo = pk.hi ? pool_alloc(pk.bytes()) : nullptr;
@@ -1592,23 +1656,36 @@ static int pack_alloc(Pack& pk, int ar, long long rows, long long cols, cudaStre
 }
 static void pack_release(Pack& pk) {
   if (pk.hi) { pool_free(pk.hi); pool_free(pk.lo); pk.hi = pk.lo = nullptr; }
-  if (pk.words) { pool_free(pk.words); pk.words = nullptr; }
+  if (pk.words && !(t_recording && pk.transient)) pool_free(pk.words);
+  pk.words = nullptr;
 }
 // Starts one use of the pack: reduces max|src| over n contiguous floats into this use's amax word and returns the
 // references the pack kernel needs.  Several pack launches of the same use (stride phases) share one ScaleRef.
 // A tf32 pack needs no maximum: its scale is 1.
 static ScaleRef begin_pack(Pack& pk, const float* src, long long n, cudaStream_t s) {
   if (pk.arith == kArithTF32) return ScaleRef{nullptr, nullptr, reinterpret_cast<float*>(pk.words + 2)};
-  const unsigned k = pk.uses++ & 1;
-  ScaleRef r{pk.words + k, pk.words + (k ^ 1), reinterpret_cast<float*>(pk.words + 2)};
+  ScaleRef r{nullptr, nullptr, reinterpret_cast<float*>(pk.words + 2)};
+  uint32_t* fresh;                      // zero when the amax kernel below adds to it
+  if (t_recording) {
+    fresh = recording_word();
+  } else {
+    const unsigned k = pk.uses++ & 1;
+    fresh = pk.words + k;
+    r.amax_next = pk.words + (k ^ 1);
+  }
+  r.amax_cur = fresh;
   static const bool no_track = getenv("TINYFLOW_NO_AMAX_TRACKING") != nullptr;
   if (const uint32_t* tracked = no_track ? nullptr : amax_tracked(src)) {
     r.amax_cur = tracked;               // the producer of src already reduced max|src| in its own pass
     return r;
   }
   KernelTimer kt("amax", s, 0, 4.0 * n);
-  launch_dep(amax_kernel, dim3(grid_for(n, 256, 32)), dim3(256), 0, s, src, n, pk.words + k);
+  launch_dep(amax_kernel, dim3(grid_for(n, 256, 32)), dim3(256), 0, s, src, n, fresh);
   return r;
+}
+// *word (zero, or a maximum to add to) becomes the largest magnitude of n contiguous floats
+void amax_of_array(const float* src, int64_t n, uint32_t* word, cudaStream_t s) {
+  launch_dep(amax_kernel, dim3(grid_for(n, 256, 32)), dim3(256), 0, s, src, (long long)n, word);
 }
 // Calls `fn(hi, lo)` with the pack's buffers typed by its element type.
 template <class F> static void with_elems(const Pack& pk, F&& fn) {
@@ -1637,6 +1714,7 @@ int tc_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_
   const int ar = tensor_arithmetic(), bk = bk_of(ar);
   // A is stored [M][K] (K-major) or, transposed, [K][M] (M-major); B is stored [K][N] (N-major) or [N][K] (K-major)
   Pack pa, pb;
+  pa.transient = pb.transient = true;
   long long a_rows = tA ? K : M, a_cols = tA ? M : K, b_rows = tB ? N : K, b_cols = tB ? K : N;
   if (pack_alloc(pa, ar, a_rows, a_cols, s, oom)) { pack_release(pa); return 0; }
   if (pack_alloc(pb, ar, b_rows, b_cols, s, oom)) { pack_release(pa); pack_release(pb); return 0; }

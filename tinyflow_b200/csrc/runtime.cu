@@ -38,14 +38,15 @@ int device_sm_count() {
 }
 
 int after_launch(cudaStream_t s, const char* what, int nkernels) {
-  g_launches.fetch_add(nkernels, std::memory_order_relaxed);
+  if (t_recording) recording_note_launches(nkernels);      // counted when the recorded step is replayed
+  else g_launches.fetch_add(nkernels, std::memory_order_relaxed);
   cudaError_t e = cudaPeekAtLastError();
   if (e != cudaSuccess) {
     cudaGetLastError();
     set_error("%s: launch failed: %s", what, cudaGetErrorString(e));
     return -1;
   }
-  if (g_sync_every_op) {
+  if (g_sync_every_op && !t_recording) {
     e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) { set_error("%s: %s", what, cudaGetErrorString(e)); return -1; }
   }
@@ -95,8 +96,8 @@ void KernelTimer::end() {
 }
 
 static std::atomic<cudaStream_t> g_compute_stream{(cudaStream_t)0};
-void note_compute_stream(cudaStream_t s) { g_compute_stream.store(s, std::memory_order_relaxed); }
-cudaStream_t last_compute_stream() { flush_deferred(); return g_compute_stream.load(std::memory_order_relaxed); }
+void note_compute_stream(cudaStream_t s) { if (!t_recording) g_compute_stream.store(s, std::memory_order_relaxed); }     // a recording's stream concerns nobody else
+cudaStream_t last_compute_stream() { flush_deferred(); return t_recording ? recording_stream() : g_compute_stream.load(std::memory_order_relaxed); }
 
 // ---- the held-back elementwise call (see common.h) ----------------------------------------------
 std::atomic<int> g_deferred_pending{0};
@@ -109,7 +110,12 @@ bool deferral_enabled() {
   }();
   return on;
 }
+// A thread that records a step keeps its held-back call to itself: nothing of the recording executes, so no other thread
+// can be waiting for it.
+static thread_local DeferredOp t_rec_deferred;
+static thread_local bool t_rec_pending = false;
 void defer_op(const DeferredOp& op) {
+  if (t_recording) { t_rec_deferred = op; t_rec_pending = true; return; }
   std::lock_guard<std::mutex> lk(g_deferred_mu);
   g_deferred = op;
   g_deferred_pending.store(1, std::memory_order_release);
@@ -118,6 +124,11 @@ void defer_op(const DeferredOp& op) {
 // stays up until then: another thread (a swap worker about to copy the held-back call's output) that finds the flag up
 // waits on the mutex and so cannot order its own work in front of that kernel.
 bool take_deferred(int kind, const float* out, int64_t n, DeferredOp* op) {
+  if (t_recording) {
+    if (!t_rec_pending || t_rec_deferred.kind != kind || t_rec_deferred.out != out || t_rec_deferred.n != n) return false;
+    *op = t_rec_deferred;
+    return true;
+  }
   if (!g_deferred_pending.load(std::memory_order_acquire)) return false;
   g_deferred_mu.lock();
   if (!g_deferred_pending.load(std::memory_order_relaxed) || g_deferred.kind != kind || g_deferred.out != out || g_deferred.n != n) { g_deferred_mu.unlock(); return false; }
@@ -125,11 +136,18 @@ bool take_deferred(int kind, const float* out, int64_t n, DeferredOp* op) {
   return true;        // still locked: the caller launches, then calls release_deferred()
 }
 void release_deferred() {
+  if (t_recording) { t_rec_pending = false; return; }
   g_deferred_pending.store(0, std::memory_order_release);
   g_deferred_mu.unlock();
 }
+static void flush_recorded() {
+  if (!t_rec_pending) return;
+  t_rec_pending = false;
+  launch_deferred_now(t_rec_deferred);
+}
 // Freeing an array only concerns the held-back call if the array is one of its operands.
 void flush_deferred_if_uses(const void* data) {
+  if (t_recording) { if (data == t_rec_deferred.a || data == t_rec_deferred.b || data == t_rec_deferred.out) flush_recorded(); return; }
   if (!g_deferred_pending.load(std::memory_order_acquire)) return;
   std::lock_guard<std::mutex> lk(g_deferred_mu);
   if (!g_deferred_pending.load(std::memory_order_relaxed)) return;
@@ -138,6 +156,7 @@ void flush_deferred_if_uses(const void* data) {
   g_deferred_pending.store(0, std::memory_order_release);
 }
 void flush_deferred_slow() {
+  if (t_recording) { flush_recorded(); return; }
   std::lock_guard<std::mutex> lk(g_deferred_mu);
   if (!g_deferred_pending.load(std::memory_order_relaxed)) return;
   launch_deferred_now(g_deferred);      // a launch failure is recorded as the thread's last error and surfaces at the next synchronising call
@@ -195,6 +214,7 @@ struct Pool {
   void* alloc(size_t bytes, bool* hard = nullptr) {
     if (hard) *hard = false;
     size_t b = round(bytes);
+    if (t_recording && !host) if (void* p = recording_take_block(b)) return p;      // still counted as in use
     std::lock_guard<std::mutex> lk(mu);
     auto it = free_by_size.find(b);
     if (it != free_by_size.end() && !it->second.empty()) {
@@ -228,6 +248,7 @@ struct Pool {
     std::lock_guard<std::mutex> lk(mu);
     auto it = size_of.find(p);
     if (it == size_of.end()) return false;
+    if (t_recording && !host) { recording_keep_block(p, it->second); return true; }
     if (!host) {
       Freed& f = freed[p];
       f.state = 1;
@@ -290,7 +311,7 @@ void* persistent_scratch(int slot, size_t bytes) {
   if (cap[slot] >= bytes) return ptr[slot];
   // Growing while earlier kernels may still read the old block: hand the old block back
   // to the pool (stream order on the single compute stream keeps that safe).
-  if (ptr[slot]) pool_free(ptr[slot]);
+  if (ptr[slot]) { pool_free(ptr[slot]); bump_layout_epoch(); }
   size_t want = bytes + bytes / 4;
   ptr[slot] = pool_alloc(want);
   cap[slot] = ptr[slot] ? Pool::round(want) : 0;
@@ -402,6 +423,16 @@ int DLArrayCopyFromTo(DLArrayHandle from, DLArrayHandle to, DLStreamHandle strea
   TF_CUDA(cudaMemcpyAsync(to->data, from->data, bytes, kind, s));
   if (kind == cudaMemcpyDeviceToDevice && s == cs) return 0;   // same-stream reshape copy: no host wait needed
   TF_CUDA(cudaStreamSynchronize(s));
+  return 0;
+}
+
+// Device-to-device copy in stream order: never waits on the host, whatever stream computed last.
+int TfArrayCopyOnStream(DLArrayHandle from, DLArrayHandle to, void** cudaStream) {
+  TF_REQUIRE(from && to && from->data && to->data && from->ctx.device_type == kGPU && to->ctx.device_type == kGPU && numel(from) == numel(to), "TfArrayCopyOnStream: needs two device arrays of one size");
+  cudaStream_t s = stream_of(cudaStream);
+  note_compute_stream(s);
+  note_write(to->data);
+  if (numel(from) > 0) TF_CUDA(cudaMemcpyAsync(to->data, from->data, data_bytes(from), cudaMemcpyDeviceToDevice, s));
   return 0;
 }
 

@@ -19,11 +19,13 @@ stream through ``DLArrayCopyFromTo`` into pinned host arrays.
 from __future__ import annotations
 
 import queue
+import random
 import threading
 import time
+import weakref
 
-from . import gpu_op, ndarray
-from .graph import (Variable, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
+from . import gpu_op, ndarray, step_graph
+from .graph import (AdamOp, SgdOp, Variable, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
 
 
 def getcomputelist(Variable_node_list, Variable_node_grad_list, b1, b2, b1t, b2t, e, learning_rate):
@@ -172,6 +174,10 @@ class Executor(object):
             + [self.Variable_node_to_mv[v][1] for v in variables if v in self.Variable_node_to_mv] + [y]
         for i, node in enumerate(self.topo_order):
             node.index = i
+        # a recorded step repeats the launches of the moment it was recorded: assignments to nodes outdate it
+        self._changes = [0]
+        for node in self.topo_order:
+            node._changes = (node._changes or ()) + (self._changes,)
         self.total_node = len(self.topo_order)
 
         self.top_control_queue, self.top_message_queue = top_control_queue, top_message_queue
@@ -180,12 +186,33 @@ class Executor(object):
         self.ctx_cpu, self.ctx_gpu = ndarray.cpu(0), ndarray.gpu(0)
         self.node_to_shape_map = None
         self.feed_shapes = None
-        self.values = {}           # node index -> NDArray on the GPU (None while swapped out)
+        self._values = {}          # node index -> NDArray on the GPU (None while swapped out)
+        self._feed = {}            # what the most recent run was fed: node -> NDArray on the GPU
+        self._leases = {}          # node index -> weak references to the views of its array that were handed out
+        self._recordings = step_graph.Recordings()
+        self._record_failures = 0
         self.host_values = {}      # node index -> pinned host NDArray holding a swapped-out tensor
         self.have_plan = False
         self._swap_worker = None
         self._values_lock = threading.Lock()
         self.passive_swap_in = 0
+
+    @property
+    def values(self):
+        """Node index -> NDArray on the GPU.  Whoever holds this dict may hold any array of it, so none is written again."""
+        self._forget_recordings()
+        self._values, self._values_exposed = dict(self._values), True
+        return self._values
+
+    @values.setter
+    def values(self, values):
+        self._forget_recordings()
+        self._values = values
+
+    _values_exposed = False
+
+    def _forget_recordings(self):
+        self._recordings.clear()
 
     def _ensure_handles(self):
         if self.cudaStream is None:
@@ -195,6 +222,7 @@ class Executor(object):
 
     # ---- shape inference (autodiff.py:2318-2336): builds every descriptor exactly once ----------
     def infer_shape(self, feed_shapes):
+        self._forget_recordings()
         self.node_to_shape_map = dict(feed_shapes)
         for node in self.topo_order:
             if node in self.node_to_shape_map:
@@ -204,6 +232,7 @@ class Executor(object):
 
     # ---- memory-plan messages ---------------------------------------------------------------------
     def _apply_plan(self, swap_list, release_list, recompute_list):
+        self._forget_recordings()
         for node in self.topo_order:
             node.control_message_out, node.control_message_out_time = [], 0
             node.release_list, node.recompute_list = [], []
@@ -224,16 +253,16 @@ class Executor(object):
         shape = self.node_to_shape_map[self.topo_order[index]]
         if to_gpu:
             with self._values_lock:
-                if self.values.get(index) is not None or index not in self.host_values:
+                if self._values.get(index) is not None or index not in self.host_values:
                     return
             dev = ndarray.empty(shape, self.ctx_gpu)
             self.host_values[index].copyto(dev, stream)
             with self._values_lock:
-                if self.values.get(index) is None:
-                    self.values[index] = dev
+                if self._values.get(index) is None:
+                    self._values[index] = dev
         else:
             with self._values_lock:
-                dev = self.values.get(index)
+                dev = self._values.get(index)
             if dev is None:
                 return
             host = self.host_values.get(index)
@@ -242,7 +271,7 @@ class Executor(object):
             dev.copyto(host, stream)             # returns once the copy has completed
             with self._values_lock:
                 self.host_values[index] = host
-                self.values[index] = None
+                self._values[index] = None
             dev.free_gpu()
 
     def _after_node(self, node):
@@ -250,8 +279,8 @@ class Executor(object):
             self._swap_worker.submit(wait, tensor_index, to_gpu)
         for tensor_index in node.release_list:
             with self._values_lock:
-                arr = self.values.get(tensor_index)
-                self.values[tensor_index] = None
+                arr = self._values.get(tensor_index)
+                self._values[tensor_index] = None
             if arr is not None and self.topo_order[tensor_index].isw == 0:
                 arr.free_gpu()
 
@@ -259,87 +288,218 @@ class Executor(object):
         """The GPU array of node ``n``, swapping it in on demand (the reference's passive swap-in)."""
         if self._swap_worker is not None:
             self._swap_worker.wait_for(n.index)      # a queued swap-out would free the array under the reader
-        arr = self.values.get(n.index)
+        arr = self._values.get(n.index)
         if arr is not None:
             return arr
+        if not self.have_plan and n in self._feed:
+            return self._feed[n]
         host = self.host_values.get(n.index)
         if host is None:
             raise RuntimeError("tensor of node %d (%s) is neither on the GPU nor swapped out" % (n.index, n.name))
         self.passive_swap_in += 1
         arr = ndarray.empty(self.node_to_shape_map[n], self.ctx_gpu)
         host.copyto(arr, self.cudaStream)
-        self.values[n.index] = arr
+        self._values[n.index] = arr
         return arr
 
-    def _compute(self, node):
+    def _lease(self, n):
+        """A view of node ``n``'s array for the caller; the next step leaves the array alone while a view is alive."""
+        view = self._resident(n).borrow()
+        self._leases.setdefault(n.index, []).append(weakref.ref(view))
+        return view
+
+    def _live_leases(self):
+        if self._leases:
+            self._leases = {i: live for i, live in ((i, [r for r in refs if r() is not None]) for i, refs in self._leases.items()) if live}
+        return self._leases
+
+    def _compute(self, node, out, stream):
         inputs = [self._resident(n) for n in node.inputs]
         if node.issgd:
-            node.op.compute(node, inputs, None, self.cudnnHandle, self.cublasHandle, self.cudaStream, False)
+            node.op.compute(node, inputs, None, self.cudnnHandle, self.cublasHandle, stream, False)
             return
-        out = ndarray.empty(self.node_to_shape_map[node], self.ctx_gpu)
+        if out is None:
+            out = ndarray.empty(self.node_to_shape_map[node], self.ctx_gpu)
         if isinstance(out, int):
             raise MemoryError("device out of memory allocating %d bytes for node %d (%s)" % (out, node.index, node.name))
-        short = node.op.compute(node, inputs, out, self.cudnnHandle, self.cublasHandle, self.cudaStream, False)
+        short = node.op.compute(node, inputs, out, self.cudnnHandle, self.cublasHandle, stream, False)
         if short:
             raise MemoryError("device out of memory inside node %d (%s): %d bytes short" % (node.index, node.name, short))
-        self.values[node.index] = out
+        self._values[node.index] = out
+
+    def _update_parameters(self, nodes, stream):
+        """The optimiser nodes of a step, one launch for all that share a rule (their place in the order is behind every
+        reader of their parameter, so the end of the step will do)."""
+        groups = {}
+        for node in nodes:
+            if type(node.op) is SgdOp:
+                rule = (node.learning_rate,)
+            else:
+                rule = (node.b1, node.b2, node.b1t[0], node.b2t[0], node.e, node.learning_rate)
+            groups.setdefault(rule, []).append([self._resident(n) for n in node.inputs])
+        for rule, rows in groups.items():
+            arrays = [gpu_op.handle_array(column) for column in zip(*rows)]
+            if len(rule) == 1:
+                gpu_op.sgd_update_many(arrays[0], arrays[1], rule[0], stream)
+            else:
+                gpu_op.adam_update_many(arrays[0], arrays[1], arrays[2], arrays[3], *rule, stream)
+
+    def _issue(self, feed_dict, stream, recording=False):
+        """Issues every node's calls on ``stream``.  Returns (arrays by node index, loss array)."""
+        # Without a plan a node writes the array it wrote in the previous step, unless a caller still looks at that.  Under
+        # a plan the arrays come and go: the previous step's go back to the pool one at a time, each just before its node
+        # runs again (dropping all of them here would leave a synchronised GPU idle for a millisecond or two).
+        previous = {} if self._values_exposed else dict(self._values)
+        self._values, self._values_exposed = {}, False
+        if self.have_plan:
+            self._values = {n.index: v for n, v in self._feed.items()}        # a plan may move these too
+        else:
+            for index in self._live_leases():
+                previous.pop(index, None)
+        previous.pop(self.targetloss.index, None)        # the loss belongs to the caller
+        shapes, timed = self.node_to_shape_map, self.top_message_queue is not None
+        together = not (self.have_plan or timed or gpu_op.data_parallel_active())
+        updates = []
+        for node in self.topo_order:
+            if not node.inputs and node in self._feed:
+                if self.have_plan:
+                    self._after_node(node)
+                continue
+            if together and node.issgd and type(node.op) in (SgdOp, AdamOp):
+                updates.append(node)
+                continue
+            out = previous.pop(node.index, None)
+            if out is not None and (self.have_plan or out.is_freed or out.shape != shapes[node]):
+                out = None
+            if self.have_plan:
+                for idx in node.recompute_list:
+                    self._compute(self.topo_order[idx], None, stream)
+            if timed:
+                t0 = time.perf_counter()
+                self._compute(node, out, stream)
+                node.runtime = (time.perf_counter() - t0) * 1000.0
+            else:
+                self._compute(node, out, stream)
+            if self.have_plan:
+                self._after_node(node)
+        if updates:
+            self._update_parameters(updates, stream)
+        previous.clear()
+        return self._values, self._values.get(self.targetloss.index)
 
     # ---- one training step ----------------------------------------------------------------------------
     def run(self, feed_dict, convert_to_numpy_ret_vals=False):
         self._ensure_handles()
-        # The previous step's intermediates go back to the pool one at a time, each just before the node that produced it
-        # runs again (its new output then takes the very block that was freed): dropping all ~600-1800 arrays here would
-        # be a millisecond or two of DLArrayFree calls during which a GPU that has just been synchronised sits idle.
-        stale, self.values = self.values, {}
+        loss = self._run_recorded(feed_dict)
+        if loss is None:
+            loss = self._run_nodes(feed_dict)
+        self.b1t[0] *= self.b1
+        self.b2t[0] *= self.b2
+        if self.have_plan:
+            next_feed = {n: self._values[n.index] for n in feed_dict if n.isw == 1}
+        else:
+            next_feed = {n: self._feed[n] for n in feed_dict if n.isw == 1}
+        if convert_to_numpy_ret_vals:
+            return [loss.asnumpy(), {n: v.asnumpy() for n, v in next_feed.items()}]
+        return [loss, next_feed]
+
+    def _run_nodes(self, feed_dict):
+        self._feed = {}
         feed_shapes = {}
         for node, value in feed_dict.items():
             if not ndarray.is_gpu_ctx(value.ctx):
                 value = value.copyto(self.ctx_gpu, None)
-            self.values[node.index] = value
+            self._feed[node] = value
             feed_shapes[node] = value.shape
         if self.feed_shapes != feed_shapes:
             self.infer_shape(feed_shapes)
             self.feed_shapes = feed_shapes
         if self.top_control_queue is not None and not self.top_control_queue.empty():
             self._apply_plan(*self.top_control_queue.get())
-
-        timed = self.top_message_queue is not None
-        for node in self.topo_order:
-            if node.index in self.values and not node.inputs:
-                if self.have_plan:
-                    self._after_node(node)
-                continue
-            stale.pop(node.index, None)
-            if self.have_plan:
-                for idx in node.recompute_list:
-                    self._compute(self.topo_order[idx])
-            if timed:
-                t0 = time.perf_counter()
-                self._compute(node)
-                node.runtime = (time.perf_counter() - t0) * 1000.0
-            else:
-                self._compute(node)
-            if self.have_plan:
-                self._after_node(node)
-
-        stale.clear()
-        self.b1t[0] *= self.b1
-        self.b2t[0] *= self.b2
+        self._issue(feed_dict, self.cudaStream)
         if self._swap_worker is not None:
             self._swap_worker.drain()
-        loss = self._resident(self.targetloss)
-        next_feed = {n: self.values[n.index] for n in feed_dict if n.isw == 1}
-        if convert_to_numpy_ret_vals:
-            return [loss.asnumpy(), {n: v.asnumpy() for n, v in next_feed.items()}]
-        return [loss, next_feed]
+        return self._resident(self.targetloss)
+
+    # ---- the same step, recorded (step_graph.py) --------------------------------------------------------
+    def _run_recorded(self, feed_dict):
+        """The loss of this step if it could be replayed from a recording (made here once the feed has come often
+        enough), else None."""
+        if not step_graph.ENABLED or self.have_plan or self.top_message_queue is not None or self._record_failures > 1:
+            return None
+        if self.top_control_queue is not None and not self.top_control_queue.empty():
+            return None
+        top, below = self._recordings.find(feed_dict)
+        recording, staged = below.recording, False
+        if recording is None and below.runs < step_graph.RUNS_BEFORE_RECORDING and top.runs >= step_graph.RUNS_BEFORE_STAGING:
+            recording, staged = top.recording, True
+        if recording is not None and recording.changes != self._changes[0]:
+            recording = None
+        wanted = top.runs >= step_graph.RUNS_BEFORE_STAGING if staged else below.runs >= step_graph.RUNS_BEFORE_RECORDING
+        top.runs += 1
+        below.runs += 1
+        if self._live_leases() or gpu_op.data_parallel_active():
+            return None
+        if recording is None:
+            if not wanted or any(v.shape != self.feed_shapes.get(n) for n, v in feed_dict.items()):
+                return None
+            recording = self._record(feed_dict, staged)
+            if recording is None:
+                return None
+            if staged:
+                top.recording = recording
+            else:
+                below.recording = recording
+        self._feed = dict(feed_dict)
+        if staged:
+            for node, array in recording.staged:
+                value = feed_dict[node]
+                if value.shape != array.shape:
+                    return None
+                if ndarray.is_gpu_ctx(value.ctx):
+                    gpu_op.copy_on_stream(value, array, self.cudaStream)
+                else:
+                    value.copyto(array, None)
+                self._feed[node] = array
+        rc = recording.replay(self, random.randint)
+        if rc != 0:
+            if rc == 1:
+                top.recording = below.recording = None
+            return None
+        self._values = recording.values
+        loss = ndarray.empty(recording.loss.shape, self.ctx_gpu)
+        gpu_op.copy_on_stream(recording.loss, loss, self.cudaStream)
+        recording.values[self.targetloss.index] = loss
+        return loss
+
+    def _record(self, feed_dict, staged):
+        if any(not ndarray.is_gpu_ctx(v.ctx) for n, v in feed_dict.items() if not (staged and n.isw == 2)):
+            return None
+        feed, copies = dict(feed_dict), []
+        if staged:
+            for node in feed_dict:
+                if node.isw == 2:
+                    feed[node] = ndarray.empty(feed_dict[node].shape, self.ctx_gpu)
+                    copies.append((node, feed[node]))
+        draws = random.getstate()                # the recorded step is not run: its seeds have not been drawn
+        before = self._feed, self._values
+        self._feed = feed
+        try:
+            return step_graph.record(self, feed, copies)
+        except RuntimeError:
+            self._record_failures += 1
+            self._feed, self._values = before
+            return None
+        finally:
+            random.setstate(draws)
 
     # ---- inspection helpers (no counterpart in the reference) ---------------------------------------------
     def value_of(self, node):
         """GPU array computed for ``node`` in the most recent ``run``."""
-        return self._resident(node)
+        return self._lease(node)
 
     def gradient_of(self, variable):
-        return self._resident(self.Variable_node_to_grad[variable])
+        return self._lease(self.Variable_node_to_grad[variable])
 
     def synchronize(self):
         gpu_op.device_synchronize()

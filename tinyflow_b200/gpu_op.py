@@ -161,6 +161,16 @@ def matrix_elementwise_multiply_by_const(in_mat, val, out_mat, cudaStream):
     check_call(_LIB.DLGpuMatrixMultiplyByConst(_h(in_mat), _F(val), _h(out_mat), cudaStream))
 
 
+def matrix_elementwise_add_by_array(in_mat, scalar, out_mat, cudaStream):
+    """in_mat + the one element of the device array ``scalar``."""
+    check_call(_LIB.TfMatrixElementwiseAddByArray(_h(in_mat), _h(scalar), _h(out_mat), cudaStream))
+
+
+def matrix_elementwise_multiply_by_array(in_mat, scalar, out_mat, cudaStream):
+    """in_mat * the one element of the device array ``scalar``."""
+    check_call(_LIB.TfMatrixMultiplyByArray(_h(in_mat), _h(scalar), _h(out_mat), cudaStream))
+
+
 def matrix_multiply(matA, transA, matB, transB, matC, cublasHandle, cudaStream):
     check_call(_LIB.DLGpuMatrixMultiply(_h(matA), bool(transA), _h(matB), bool(transB), _h(matC), cublasHandle, cudaStream))
 
@@ -397,6 +407,30 @@ def sgd_compute_o(n2list, indexinfolist, count, learning_rate):
 
 def adam_compute_o(n4list, indexinfolist, count, b1, b2, b1t, b2t, e, learning_rate):
     check_call(_LIB.DLGpuAdam_o(n4list, indexinfolist, ctypes.c_int(count), _F(b1), _F(b2), _F(b1t), _F(b2t), _F(e), _F(learning_rate)))
+
+
+def copy_on_stream(source, target, cudaStream):
+    """Device-to-device copy in stream order (``NDArray.copyto`` waits on the host unless the stream computed last)."""
+    check_call(_LIB.TfArrayCopyOnStream(_h(source), _h(target), cudaStream))
+
+
+def data_parallel_active() -> bool:
+    return _LIB.TfDpActive() != 0
+
+
+def handle_array(arrs):
+    """The C array of handles the many-tensor calls take."""
+    return (_nd.DLArrayHandle * len(arrs))(*[_h(a) for a in arrs])
+
+
+def sgd_update_many(params, grads, learning_rate, cudaStream):
+    """``sgd_update`` of every pair in one launch; ``params`` and ``grads`` come from :func:`handle_array`."""
+    check_call(_LIB.TfSgdUpdateMany(params, grads, len(params), _F(learning_rate), cudaStream))
+
+
+def adam_update_many(params, m, v, grads, b1, b2, b1t, b2t, e, learning_rate, cudaStream):
+    """``adam_mv`` and ``adam_compute`` of every tensor in one launch."""
+    check_call(_LIB.TfAdamUpdateMany(params, m, v, grads, len(params), _F(b1), _F(b2), _F(b1t), _F(b2t), _F(e), _F(learning_rate), cudaStream))
 
 
 def getInt(intp):

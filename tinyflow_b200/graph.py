@@ -24,6 +24,16 @@ from . import gpu_op, ndarray
 class Node(object):
     """A graph node (autodiff.py:153-215)."""
 
+    _changes = None         # set by an executor: counts assignments to the node's attributes
+    _FREE = frozenset(("runtime", "n"))     # bookkeeping that no operator's launch depends on
+
+    def __setattr__(self, name, value):
+        object.__setattr__(self, name, value)
+        changes = self._changes
+        if changes is not None and name not in Node._FREE:
+            for counter in changes:
+                counter[0] += 1
+
     def __init__(self):
         self.inputs = []
         self.op = None
@@ -103,10 +113,6 @@ class Op(object):
         raise NotImplementedError
 
 
-def _scalar_of(arr):
-    return float(arr.asnumpy().reshape(-1)[0])
-
-
 # ---- arithmetic (AddOp, AddByConstOp, MulOp, MulByConstOp: autodiff.py:302-438) ----------
 class AddOp(Op):
     name = "+"
@@ -120,9 +126,9 @@ class AddOp(Op):
         if a.shape == b.shape:
             gpu_op.matrix_elementwise_add(a, b, output_val, cudaStream)
         elif b.shape == (1,):
-            gpu_op.matrix_elementwise_add_by_const(a, _scalar_of(b), output_val, cudaStream)
+            gpu_op.matrix_elementwise_add_by_array(a, b, output_val, cudaStream)
         elif a.shape == (1,):
-            gpu_op.matrix_elementwise_add_by_const(b, _scalar_of(a), output_val, cudaStream)
+            gpu_op.matrix_elementwise_add_by_array(b, a, output_val, cudaStream)
         else:
             raise ValueError("add: shapes %s and %s do not match" % (a.shape, b.shape))
         return 0
@@ -167,9 +173,9 @@ class MulOp(Op):
         if a.shape == b.shape:
             gpu_op.matrix_elementwise_multiply(a, b, output_val, cudaStream)
         elif b.shape == (1,):
-            gpu_op.matrix_elementwise_multiply_by_const(a, _scalar_of(b), output_val, cudaStream)
+            gpu_op.matrix_elementwise_multiply_by_array(a, b, output_val, cudaStream)
         elif a.shape == (1,):
-            gpu_op.matrix_elementwise_multiply_by_const(b, _scalar_of(a), output_val, cudaStream)
+            gpu_op.matrix_elementwise_multiply_by_array(b, a, output_val, cudaStream)
         else:
             raise ValueError("mul: shapes %s and %s do not match" % (a.shape, b.shape))
         return 0

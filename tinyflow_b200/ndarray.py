@@ -65,11 +65,12 @@ def _borrow_numpy(np_data):
 
 class NDArray(object):
     """A buffer with a shape on the CPU (pinned) or GPU; no arithmetic."""
-    __slots__ = ["handle", "is_freed", "_shape"]
+    __slots__ = ["handle", "is_freed", "_shape", "_owner", "__weakref__"]
 
     def __init__(self, handle):
         self.handle = handle
         self.is_freed = False
+        self._owner = None
         c = handle.contents
         self._shape = tuple(c.shape[i] for i in range(c.ndim))
 
@@ -96,6 +97,12 @@ class NDArray(object):
     @property
     def data_ptr(self):
         return self.handle.contents.data
+
+    def borrow(self):
+        """Another NDArray over the same memory, which stays this one's to free; keeps this one alive."""
+        other = NDArray.__new__(NDArray)
+        other.handle, other.is_freed, other._shape, other._owner = self.handle, True, self._shape, self
+        return other
 
     def __setitem__(self, in_slice, value):
         if not isinstance(in_slice, slice) or in_slice.start is not None or in_slice.stop is not None:

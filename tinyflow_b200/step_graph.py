@@ -1,0 +1,115 @@
+"""Recorded training steps.
+
+A step of a graph is the same sequence of launches every time, on the same arrays, as long as the caller feeds the same
+ones.  The executor therefore records the step once it has seen the same feed repeatedly and replays it with one call
+(``TfStepReplay``) from then on: the host work per step no longer grows with the number of nodes.
+
+What is replayed is keyed by identity.  Parameters and moments (updated in place) are one key; the mini-batch arrays are a
+second one below it.  A caller that brings new mini-batch arrays every step gets a *staged* recording, whose inputs are
+copied into arrays of the executor's own first.  Entries disappear with the arrays they name.
+"""
+from __future__ import annotations
+
+import ctypes
+import os
+import weakref
+
+from . import gpu_op, ndarray
+from ._base import _LIB, check_call, new_cell
+
+ENABLED = os.environ.get("TINYFLOW_STEP_GRAPH", "1") != "0"
+RUNS_BEFORE_RECORDING = 2        # of the same arrays: the first calls of a plan still learn what follows what
+RUNS_BEFORE_STAGING = 4          # of the same parameters with ever new mini-batches
+MAX_FEEDS = 4                    # parameter sets, and mini-batches per set, that keep a recording
+
+
+class Recording(object):
+    """A replayable step: the library's graph and the arrays it writes."""
+
+    def __init__(self, graph, values, loss, kept, seed_nodes, arrays, staged, changes):
+        self.graph, self.values, self.loss, self.kept, self.staged, self.changes = graph, values, loss, kept, staged, changes
+        self.seed_nodes = seed_nodes
+        self.seeds = (ctypes.c_uint * max(1, len(seed_nodes)))()
+        self.arrays = gpu_op.handle_array(arrays)
+
+    def __del__(self):
+        if self.graph is not None and _LIB is not None:
+            _LIB.TfStepGraphFree(self.graph)
+            self.graph = None
+
+    def replay(self, executor, draw):
+        """0 when the step is on its way, else the library's reason (see ``TfStepReplay``)."""
+        for i, node in enumerate(self.seed_nodes):
+            node.seed[0] = self.seeds[i] = draw(0, 100)
+        rc = _LIB.TfStepReplay(self.graph, self.seeds, len(self.seed_nodes), ctypes.c_float(executor.b1t[0]), ctypes.c_float(executor.b2t[0]),
+                               self.arrays, len(self.arrays), executor.cudaStream)
+        if rc < 0:
+            check_call(rc)
+        return rc
+
+
+class _Feed(object):
+    """How often a set of arrays was run, and what was recorded for it."""
+    __slots__ = ("runs", "refs", "recording", "batches", "__weakref__")
+
+    def __init__(self):
+        self.runs, self.refs, self.recording, self.batches = 0, None, None, {}
+
+
+class Recordings(object):
+    def __init__(self):
+        self.sets = {}
+
+    def clear(self):
+        self.sets.clear()
+
+    @staticmethod
+    def _entry(table, key, arrays):
+        entry = table.pop(key, None)
+        if entry is None:
+            entry = _Feed()
+            gone = lambda _ref, t=weakref.ref(entry), k=key: _forget(table, k, t)     # noqa: E731
+            entry.refs = [weakref.ref(a, gone) for a in arrays]
+            while len(table) >= MAX_FEEDS:
+                del table[next(iter(table))]
+        table[key] = entry                      # most recently used last
+        return entry
+
+    def find(self, feed_dict):
+        """(entry of the parameters, entry of the mini-batch below it) for this feed."""
+        params, batch = [], []
+        for node, value in feed_dict.items():
+            (batch if node.isw == 2 else params).append((node, value))
+        key = tuple((id(n), id(v)) for n, v in params)
+        top = self._entry(self.sets, key, [v for _, v in params])
+        below = self._entry(top.batches, tuple((id(n), id(v)) for n, v in batch), [v for _, v in batch])
+        return top, below
+
+
+def _forget(table, key, entry_ref):
+    entry = entry_ref()
+    if entry is not None and table.get(key) is entry:
+        del table[key]
+
+
+def record(executor, feed_dict, staged):
+    """Records one step of ``executor`` on ``feed_dict`` (nothing is executed).  None if the step cannot be recorded."""
+    graph, stream = ctypes.c_void_p(), new_cell(2)
+    rc = _LIB.TfStepRecordBegin(ctypes.byref(graph), stream)
+    if rc != 0:
+        if rc < 0:
+            raise RuntimeError("recording is not available")
+        return None
+    values, loss, keep = {}, None, 0
+    try:
+        values, loss = executor._issue(feed_dict, stream, recording=True)
+        keep = 1
+    except Exception:                           # whatever stopped it: the ordinary step that follows reports it
+        pass
+    finally:
+        rc = _LIB.TfStepRecordEnd(ctypes.byref(graph), keep)
+    if rc != 0:
+        raise RuntimeError("the step cannot be recorded")
+    kept = [n for n in feed_dict if n.isw == 1]
+    seed_nodes = [n for n in executor.topo_order if hasattr(n, "seed")]
+    return Recording(graph, values, loss, kept, seed_nodes, list(feed_dict.values()), staged, executor._changes[0])
