@@ -1,0 +1,56 @@
+"""CUDA-core kernels for small sizes: products, convolutions of few channels, split reductions."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_ops import env  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("M,K,N", [(1, 1, 1), (8, 33, 64), (7, 4100, 130), (9, 64, 31), (33, 127, 65), (32, 256, 32), (64, 3, 1029), (640, 65, 1030), (2, 2048, 1000)])
+@pytest.mark.parametrize("tA,tB", [(False, False), (True, False), (False, True), (True, True)])
+def test_simt_product_at_tile_edges(env, M, K, N, tA, tB):
+    rng = np.random.RandomState(M + K + N)
+    a, b = rng.randn(M, K).astype(np.float32), rng.randn(K, N).astype(np.float32)
+    A, B = env.nd.array(np.ascontiguousarray(a.T) if tA else a, env.ctx), env.nd.array(np.ascontiguousarray(b.T) if tB else b, env.ctx)
+    C = env.nd.empty((M, N), env.ctx)
+    env.gpu_op.set_contraction_path(1)
+    try:
+        env.gpu_op.matrix_multiply(A, tA, B, tB, C, env.cublas, env.stream)
+    finally:
+        env.gpu_op.set_contraction_path(0)
+    want, mag = a.astype(np.float64) @ b.astype(np.float64), np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+    assert np.all(np.abs(C.asnumpy() - want) <= 1e-5 * np.abs(want) + 8 * 2.0 ** -24 * mag)
+
+
+@pytest.mark.parametrize("case", [(3, 1, 28, 28, 6, 5, 5, "SAME"), (5, 6, 14, 14, 16, 5, 5, "VALID"), (2, 3, 9, 7, 5, 3, 3, "SAME"), (300, 2, 8, 8, 3, 7, 7, "SAME"),
+                                  (2, 8, 11, 13, 32, 1, 3, "SAME"), (1, 5, 40, 33, 7, 3, 3, "VALID")])
+def test_direct_convolution_of_few_channels(env, case):
+    N, C, H, W, K, R, S, padding = case
+    rng = np.random.RandomState(N + C)
+    x, w = rng.randn(N, C, H, W).astype(np.float32), rng.randn(K, C, R, S).astype(np.float32)
+    out, cell = env.gpu_op.convolution_2d_forward_get_out_shape(x.shape, w.shape, "NCHW", padding, 1, 1)
+    dy = rng.randn(*out).astype(np.float32)
+    X, Wd, DY = (env.nd.array(v, env.ctx) for v in (x, w, dy))
+    got = {}
+    for path in (0, 1):                      # the direct kernels, and the implicit product as the cross-check
+        env.gpu_op.set_contraction_path(path)
+        try:
+            y, dx, dw = env.nd.empty(out, env.ctx), env.nd.empty(x.shape, env.ctx), env.nd.empty(w.shape, env.ctx)
+            env.gpu_op.convolution_2d_forward(X, Wd, y, cell, env.cudnn, env.stream)
+            env.gpu_op.convolution_backward_data(X, DY, Wd, dx, cell, env.cudnn, env.stream)
+            env.gpu_op.convolution_backward_filter(X, DY, Wd, dw, cell, env.cudnn, env.stream)
+            got[path] = [v.asnumpy() for v in (y, dx, dw)]
+        finally:
+            env.gpu_op.set_contraction_path(0)
+    for a, b in zip(got[0], got[1]):
+        np.testing.assert_allclose(a, b, rtol=1e-4, atol=3e-5 * np.abs(b).max())
+
+
+@pytest.mark.parametrize("shape", [(1, 1, 1, 1), (256, 6, 28, 28), (3, 300, 5, 7), (64, 16, 10, 10), (1, 2, 129, 3)])
+def test_channel_sums(env, shape):
+    x = np.random.RandomState(1).randn(*shape).astype(np.float32)
+    X, out = env.nd.array(x, env.ctx), env.nd.empty((shape[1],), env.ctx)
+    env.gpu_op.broadcast_to_backward(X, out, "NCHW")
+    want, mag = x.astype(np.float64).sum((0, 2, 3)), np.abs(x).astype(np.float64).sum((0, 2, 3))
+    assert np.all(np.abs(out.asnumpy() - want) <= 1e-6 * mag)

@@ -89,7 +89,23 @@ def _hold_values(step, model, ex, feed, x):
         np.testing.assert_array_equal(view.asnumpy(), copy)          # later steps left it alone
 
 
-@pytest.mark.parametrize("between", [_overwrite_inputs, _overwrite_a_parameter, _change_the_rate, _hold_values])
+def _hold_and_write_gradients(step, model, ex, feed, x):
+    if step in (4, 6):
+        views = [ex.value_of(n) for n in ex.topo_order if n.name in ("+", "Zeroslike", "Oneslike")]
+        copies = [v.asnumpy() for v in views]
+        if step == 4:
+            _held.extend(zip(views, copies))
+        for n in ex.topo_order:
+            if n.name == "Zeroslike":
+                ex.value_of(n)[:] = np.full(ex.value_of(n).shape, 3.0, np.float32)
+    if step == 8:
+        for view, copy in _held:
+            if copy.any():                                           # (the zeros were overwritten above)
+                np.testing.assert_array_equal(view.asnumpy(), copy)
+        del _held[:]
+
+
+@pytest.mark.parametrize("between", [_overwrite_inputs, _hold_and_write_gradients, _overwrite_a_parameter, _change_the_rate, _hold_values])
 @pytest.mark.parametrize("name", ["mlp", "resnet50"])
 def test_what_a_caller_does_between_steps_reaches_the_replay(lib_path, monkeypatch, name, between):
     _same(_train(monkeypatch, True, BUILDS[name], "sgd", between), _train(monkeypatch, False, BUILDS[name], "sgd", between))

@@ -56,8 +56,11 @@ struct KernelTimer {
 // last_compute_stream(), which the stream-less operators and the copies call, the array free, the synchronising calls -
 // launches the held-back kernel first (flush_deferred), so no caller can observe the difference.  One slot, guarded by
 // a mutex; the fast path is one relaxed load.
-enum { kDeferReluBwd = 1, kDeferAdd = 2 };
-struct DeferredOp { int kind; const float* a; const float* b; float* out; int64_t n; cudaStream_t stream; };   // relu-bwd: a = the ReLU's input (mask), b = dy
+//  * DLGpuBroadcastTo0/1 (while a step is recorded): the sum that reads the broadcast joins it in the slot, and the ReLU of
+//    that sum, if it is next, completes the layer's bias in one kernel that writes all three tensors.
+enum { kDeferReluBwd = 1, kDeferAdd = 2, kDeferBcast = 3, kDeferBiasAdd = 4 };
+struct BiasBcast { const float* bias; int64_t C, low; float* out; };     // out[i] = bias[(i / low) % C]
+struct DeferredOp { int kind; const float* a; const float* b; float* out; int64_t n; cudaStream_t stream; BiasBcast bc; };   // relu-bwd: a = the ReLU's input (mask), b = dy
 extern std::atomic<int> g_deferred_pending;
 void flush_deferred_slow();
 extern thread_local StepGraph* t_recording;              // a thread that records a step has a slot of its own
@@ -125,6 +128,7 @@ __device__ __forceinline__ void amax_commit(const AmaxOut& am, uint32_t m) {
 int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cudaStream_t s);
 void tc_note_relu_output(const void* node, const void* y);     // the plain ReLU of graph node `node` wrote y (after the version bump)
 bool contraction_path_is_cuda_cores();
+int contraction_path();
 
 // ---- recording a training step for replay (step_graph.cu) -----------------------------------------
 // While a step is recorded, its calls (of ONE thread) run on a private stream in capture mode and nothing executes; the

@@ -4,10 +4,15 @@
 
 namespace tf {
 
-int cudacore_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, cudaStream_t s);
+int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, cudaStream_t s, const char* what);
 int cudacore_conv_fwd(const ConvPlan* p, const float* x, const float* w, float* y, cudaStream_t s);
 int cudacore_conv_dgrad(const ConvPlan* p, const float* dy, const float* w, float* dx, cudaStream_t s);
 int cudacore_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float* dw, cudaStream_t s);
+
+// Small images with few channels (conv_direct.cu); same return convention as the tensor-core path.
+int direct_conv_fwd(const ConvPlan* p, const float* x, const float* w, float* y, cudaStream_t s);
+int direct_conv_dgrad(const ConvPlan* p, const float* dy, const float* w, float* dx, cudaStream_t s);
+int direct_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float* dw, cudaStream_t s);
 
 // Tensor-core path (gemm_tcgen05.cu).  Each returns 1 when it handled the call, 0 when the
 // shape is outside what it takes (caller falls through to the CUDA-core path), -1 on error.
@@ -78,7 +83,7 @@ int DLGpuMatrixMultiply(const DLArrayHandle matA, bool transposeA, const DLArray
     TF_REQUIRE(g_path != 2, "DLGpuMatrixMultiply: shape not taken by the tensor-core path (forced)");
   }
   t_last_path = 1;
-  return cudacore_matmul(A, transposeA, B, transposeB, C, M, N, K, matA->shape[1], matB->shape[1], s);
+  return simt_matmul(A, transposeA, B, transposeB, C, M, N, K, matA->shape[1], matB->shape[1], N, s, "DLGpuMatrixMultiply");
 }
 
 // Output extent = 1 + (in + 2*pad - window) / stride with pad = window/2 for SAME, 0 for VALID
@@ -126,6 +131,11 @@ int DLGpuConvolution2DForward(const DLArrayHandle input, const DLArrayHandle fil
   ConvPlan* p = plan_of<ConvPlan>(cudnnlist, kPlanConv);
   if (check_conv(p, input, filter, output, "DLGpuConvolution2DForward")) return -1;
   cudaStream_t s = stream_of(cudaStream);
+  if (g_path == 0) {
+    int r = direct_conv_fwd(p, (const float*)input->data, (const float*)filter->data, out_f32(output), s);
+    if (r < 0) return -1;
+    if (r == 1) { t_last_path = 1; return 0; }
+  }
   if (g_path != 1) {
     int oom = 0;
     int r = tc_conv_fwd(p, (const float*)input->data, (const float*)filter->data, out_f32(output), s, &oom);
@@ -145,6 +155,11 @@ int DLGpuConvolutionBackwardData(const DLArrayHandle input, const DLArrayHandle 
   if (check_conv(p, input, filter, doutput, "DLGpuConvolutionBackwardData")) return -1;
   TF_REQUIRE(dinput && numel(dinput) == numel(input), "DLGpuConvolutionBackwardData: dinput does not match input");
   cudaStream_t s = stream_of(cudaStream);
+  if (g_path == 0) {
+    int r = direct_conv_dgrad(p, (const float*)doutput->data, (const float*)filter->data, out_f32(dinput), s);
+    if (r < 0) return -1;
+    if (r == 1) { t_last_path = 1; return 0; }
+  }
   if (g_path != 1) {
     int oom = 0;
     int r = tc_conv_dgrad(p, (const float*)doutput->data, (const float*)filter->data, out_f32(dinput), s, &oom);
@@ -164,6 +179,11 @@ int DLGpuConvolutionBackwardFilter(const DLArrayHandle input, const DLArrayHandl
   if (check_conv(p, input, filter, doutput, "DLGpuConvolutionBackwardFilter")) return -1;
   TF_REQUIRE(dfilter && numel(dfilter) == numel(filter), "DLGpuConvolutionBackwardFilter: dfilter does not match filter");
   cudaStream_t s = stream_of(cudaStream);
+  if (g_path == 0) {
+    int r = direct_conv_wgrad(p, (const float*)input->data, (const float*)doutput->data, out_f32(dfilter), s);
+    if (r < 0) return -1;
+    if (r == 1) { t_last_path = 1; return 0; }
+  }
   if (g_path != 1) {
     int oom = 0;
     int r = tc_conv_wgrad(p, (const float*)input->data, (const float*)doutput->data, out_f32(dfilter), s, &oom);

@@ -1,8 +1,8 @@
-// CUDA-core (fp32 FMA) implicit-GEMM contraction kernels: matmul with either operand
-// transposed, convolution forward, backward-data and backward-filter for any window, stride
-// and padding.  This is the exact-fp32 general path; it serves the shapes the tensor-core
-// path does not take (tiny channel counts, strided backward-data, very small problems) and is
-// the cross-check for the tcgen05 kernels.
+// CUDA-core (fp32 FMA) implicit-GEMM contraction kernels: convolution forward, backward-data and
+// backward-filter for any window, stride and padding (matrix products: gemm_simt.cu; small images
+// with few channels: conv_direct.cu).  This is the exact-fp32 general path; it serves the shapes
+// the tensor-core path does not take (strided backward-data, very small problems) and is the
+// cross-check for the tcgen05 kernels.
 //
 // One kernel template: C[M x N] += A[M x K] * B[K x N] on 64x64x16 tiles, 256 threads, a 4x4
 // register micro-tile per thread.  Operand elements are fetched through small "view" structs
@@ -15,10 +15,6 @@ namespace tf {
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
 // ---- operand views -----------------------------------------------------------------------
-struct MatView {            // plain row-major matrix, optionally read transposed
-  const float* p; int64_t ld; int trans;
-  __device__ __forceinline__ float at(int64_t r, int64_t c) const { return trans ? p[c * ld + r] : p[r * ld + c]; }
-};
 struct ConvGeom {
   int N, C, H, W, K, R, S, P, Q, ph, pw, sh, sw;
 };
@@ -216,26 +212,23 @@ static ConvGeom geom_of(const ConvPlan* p) {
   return g;
 }
 
-// Entry points used by the dispatchers in contract_api.cu
-int cudacore_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, cudaStream_t s) {
-  MatView a{A, lda, tA ? 1 : 0};
-  MatView bt{B, ldb, tB ? 1 : 0};
-  MatOut o{C, N};
-  // B is [K x N] logically; when stored transposed ([N x K]) it is contiguous along K.
-  if (tB) return launch_contract<MatView, MatView, MatOut, true>(a, bt, o, M, N, K, C, sizeof(float) * M * N, true, s, "DLGpuMatrixMultiply");
-  return launch_contract<MatView, MatView, MatOut, false>(a, bt, o, M, N, K, C, sizeof(float) * M * N, true, s, "DLGpuMatrixMultiply");
-}
+// Entry points used by the dispatchers in contract_api.cu.  A 1x1 window on 1x1 images is a matrix product.
+int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, cudaStream_t s, const char* what);
+static bool is_matrix(const ConvPlan* p) { return p->H == 1 && p->W == 1 && p->R == 1 && p->S == 1 && p->P == 1 && p->Q == 1 && p->pad_h == 0 && p->pad_w == 0; }
 int cudacore_conv_fwd(const ConvPlan* p, const float* x, const float* w, float* y, cudaStream_t s) {
+  if (is_matrix(p)) return simt_matmul(x, false, w, true, y, p->N, p->K, p->C, p->C, p->C, p->K, s, "DLGpuConvolution2DForward");
   ConvGeom g = geom_of(p);
   int64_t CRS = (int64_t)g.C * g.R * g.S, NPQ = (int64_t)g.N * g.P * g.Q;
   return launch_contract<FwdA, FwdB, NchwOut, false>(FwdA{w, CRS}, FwdB{x, g}, NchwOut{y, g.K, (int64_t)g.P * g.Q}, g.K, NPQ, CRS, y, sizeof(float) * g.K * NPQ, false, s, "DLGpuConvolution2DForward");
 }
 int cudacore_conv_dgrad(const ConvPlan* p, const float* dy, const float* w, float* dx, cudaStream_t s) {
+  if (is_matrix(p)) return simt_matmul(dy, false, w, false, dx, p->N, p->C, p->K, p->K, p->C, p->C, s, "DLGpuConvolutionBackwardData");
   ConvGeom g = geom_of(p);
   int64_t KRS = (int64_t)g.K * g.R * g.S, NHW = (int64_t)g.N * g.H * g.W;
   return launch_contract<DgradA, DgradB, NchwOut, false>(DgradA{w, g}, DgradB{dy, g}, NchwOut{dx, g.C, (int64_t)g.H * g.W}, g.C, NHW, KRS, dx, sizeof(float) * g.C * NHW, false, s, "DLGpuConvolutionBackwardData");
 }
 int cudacore_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float* dw, cudaStream_t s) {
+  if (is_matrix(p)) return simt_matmul(dy, true, x, false, dw, p->K, p->C, p->N, p->K, p->C, p->C, s, "DLGpuConvolutionBackwardFilter");
   ConvGeom g = geom_of(p);
   int64_t CRS = (int64_t)g.C * g.R * g.S, NPQ = (int64_t)g.N * g.P * g.Q;
   return launch_contract<WgradA, WgradB, MatOut, true>(WgradA{dy, g}, WgradB{x, g}, MatOut{dw, CRS}, g.K, CRS, NPQ, dw, sizeof(float) * g.K * CRS, true, s, "DLGpuConvolutionBackwardFilter");

@@ -1709,7 +1709,9 @@ static int run_pack_matrix(const float* src, long long ld, Pack& pk, cudaStream_
 
 // ---- matmul ---------------------------------------------------------------------------------------
 int tc_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_t M, int64_t N, int64_t K, cudaStream_t s, int* oom) {
-  if (M < 16 || N < 16 || K < 64 || (double)M * N * K < 4e6) return 0;      // launch-bound sizes stay on the CUDA cores
+  // Two packs, their maxima, the product and the sum of its split tiles cost about 20 us before the first multiply-add counts:
+  // below 0.3 GFLOP the CUDA-core kernel is through sooner (figures at its pick of tiles).  Forced (path 2): whatever fits.
+  if (M < 16 || N < 16 || K < 64 || (double)M * N * K < (contraction_path() == 2 ? 4e6 : 1.5e8)) return 0;
   if (!encode_fn()) return 0;
   const int ar = tensor_arithmetic(), bk = bk_of(ar);
   // A is stored [M][K] (K-major) or, transposed, [K][M] (M-major); B is stored [K][N] (N-major) or [N][K] (K-major)

@@ -4,6 +4,8 @@
 // and reduces with warp shuffles.
 #include "common.h"
 #include <math.h>
+#include <algorithm>
+#include <mutex>
 
 namespace tf {
 
@@ -33,6 +35,42 @@ __device__ __forceinline__ float block_sum(float v, float* red /* >= 33 floats *
   }
   __syncthreads();
   return red[32];
+}
+
+// Split reductions are finished inside their own kernel: every block leaves its partial result in a scratch array, and the
+// block that arrives last adds them in block order - the same order every run, and one launch instead of two.
+// atomicInc wraps the counter back to zero with the last arrival.
+__device__ __forceinline__ bool arrives_last(uint32_t* counter, uint32_t blocks) {
+  __shared__ uint32_t order;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) order = atomicInc(counter, blocks - 1);
+  __syncthreads();
+  const bool last = order == blocks - 1;
+  if (last) __threadfence();
+  return last;
+}
+// `n` consecutive zeroed counters; a ring far longer than the launches that can be in flight at once.
+static uint32_t* arrival_counters(int n) {
+  constexpr int kCounters = 65536;
+  static std::mutex mu;
+  static uint32_t* ring[64] = {nullptr};
+  static int at[64] = {0};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || n > kCounters) { cudaGetLastError(); return nullptr; }
+  std::lock_guard<std::mutex> lk(mu);
+  if (!ring[dev]) {
+    uint32_t* p = nullptr;
+    if (cudaMalloc((void**)&p, sizeof(uint32_t) * kCounters) != cudaSuccess || cudaMemset(p, 0, sizeof(uint32_t) * kCounters) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    ring[dev] = p;
+  }
+  if (at[dev] + n > kCounters) at[dev] = 0;
+  uint32_t* p = ring[dev] + at[dev];
+  at[dev] += n;
+  return p;
 }
 
 // ---- generic vectorised map kernels ---------------------------------------------
@@ -171,33 +209,83 @@ __global__ void __launch_bounds__(kBlock) bcast_channel_kernel(const float* __re
 
 // ---- reductions --------------------------------------------------------------------
 // Column sums of a row-major [rows x cols] matrix, out[c] = sum_r in[r, c].
-// Block = 32 columns x 8 row lanes; grid.x tiles the columns, grid.y splits the rows; with several row
-// splits each writes its partial sums to out[split * cols + c] (a scratch array) and colsum_final_kernel
-// adds the splits in order, so the result does not depend on scheduling.
-__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ in, float* __restrict__ out, int64_t rows, int64_t cols, int64_t rows_per_split) {
+// Block = 32 columns x 8 row lanes; grid.x tiles the columns, grid.y splits the rows.
+__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ in, float* __restrict__ out, float* __restrict__ part, int64_t rows, int64_t cols, int64_t rows_per_split, uint32_t* counters) {
   __shared__ float sm[8][33];
-  int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  int64_t c = (int64_t)blockIdx.x * 32 + tx;
-  int64_t r0 = (int64_t)blockIdx.y * rows_per_split, r1 = min(rows, r0 + rows_per_split);
-  float acc = 0.f;
-  if (c < cols) for (int64_t r = r0 + ty; r < r1; r += 8) acc += in[r * cols + c];
-  sm[ty][tx] = acc;
-  __syncthreads();
-  if (ty == 0 && c < cols) {
-    float t = 0.f;
+  grid_dep_sync();
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int64_t c = (int64_t)blockIdx.x * 32 + tx;
+  const int64_t r0 = (int64_t)blockIdx.y * rows_per_split, r1 = min(rows, r0 + rows_per_split);
+  auto across = [&](float acc, float* dst) {
+    sm[ty][tx] = acc;
+    __syncthreads();
+    if (ty == 0 && c < cols) {
+      float t = 0.f;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) t += sm[j][tx];
-    out[(int64_t)blockIdx.y * cols + c] = t;
+      for (int j = 0; j < 8; ++j) t += sm[j][tx];
+      *dst = t;
+    }
+  };
+  float acc = 0.f;
+  if (c < cols) {
+#pragma unroll 4
+    for (int64_t r = r0 + ty; r < r1; r += 8) acc += in[r * cols + c];
   }
+  if (gridDim.y == 1) { across(acc, out + c); return; }
+  across(acc, part + (int64_t)blockIdx.y * cols + c);
+  if (!arrives_last(counters + blockIdx.x, gridDim.y)) return;
+  acc = 0.f;
+  if (c < cols) {
+#pragma unroll 4
+    for (int z = ty; z < (int)gridDim.y; z += 8) acc += __ldcg(part + (int64_t)z * cols + c);
+  }
+  across(acc, out + c);
 }
-__global__ void __launch_bounds__(256) colsum_final_kernel(const float* __restrict__ part, float* __restrict__ out, int64_t cols, int splits) {
-  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols) return;
-  float t = 0.f;
-  for (int z = 0; z < splits; ++z) t += part[(int64_t)z * cols + c];
-  out[c] = t;
+// Sum over images and positions of every channel, in = [N][C][L] (the bias gradient of a convolution).  One block per
+// channel left all but 6 SMs idle on LeNet's first layer (467 us for 4.8 MB): the images are split over grid.y as well.
+__global__ void __launch_bounds__(kBlock) channel_sum_kernel(const float* __restrict__ in, float* __restrict__ out, float* __restrict__ part, int64_t N, int64_t C, int64_t L, int64_t n_per_split, int vec,
+                                                             uint32_t* counters) {
+  __shared__ float red[33];
+  grid_dep_sync();
+  const int64_t c = blockIdx.x, n0 = (int64_t)blockIdx.y * n_per_split, n1 = min(N, n0 + n_per_split);
+  float acc = 0.f;
+  if (vec) {
+    const uint32_t q = (uint32_t)(L >> 2), count = (uint32_t)(n1 - n0) * q;
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < count; i += kBlock) {
+      const uint32_t n = i / q, l = i - n * q;
+      const float4 v = __ldg(reinterpret_cast<const float4*>(in + ((n0 + n) * C + c) * L) + l);
+      acc += (v.x + v.y) + (v.z + v.w);
+    }
+  } else {
+    for (int64_t n = n0; n < n1; ++n)
+      for (int64_t l = threadIdx.x; l < L; l += kBlock) acc += in[(n * C + c) * L + l];
+  }
+  acc = block_sum(acc, red);
+  if (gridDim.y == 1) { if (threadIdx.x == 0) out[c] = acc; return; }
+  if (threadIdx.x == 0) part[(int64_t)blockIdx.y * C + c] = acc;
+  if (!arrives_last(counters + blockIdx.x, gridDim.y)) return;
+  acc = 0.f;
+  for (int z = threadIdx.x; z < (int)gridDim.y; z += kBlock) acc += __ldcg(part + (int64_t)z * C + c);
+  acc = block_sum(acc, red);
+  if (threadIdx.x == 0) out[c] = acc;
 }
-// Sum of n contiguous floats into out[0]; two launches: per-block partials then one block.
+// Sum of n contiguous floats into out[0], finished by the last block.
+__global__ void __launch_bounds__(kBlock) sum_kernel(const float* __restrict__ in, float* __restrict__ out, float* __restrict__ part, int64_t n, float scale, uint32_t* counter) {
+  __shared__ float red[33];
+  grid_dep_sync();
+  float acc = 0.f;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) acc += in[i];
+  acc = block_sum(acc, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc;
+  if (!arrives_last(counter, gridDim.x)) return;
+  acc = 0.f;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) acc += __ldcg(part + i);
+  acc = block_sum(acc, red);
+  if (threadIdx.x == 0) out[0] = acc * scale;
+}
+// The same in two launches: per-block partials, then one block (for the fixed scratch array of the allocation-free sum).
 __global__ void __launch_bounds__(kBlock) partial_sum_kernel(const float* __restrict__ in, float* __restrict__ part, int64_t n) {
   __shared__ float red[33];
   float acc = 0.f;
@@ -283,11 +371,14 @@ __global__ void __launch_bounds__(kBlock) row_softmax_bwd_kernel(const float* __
     for (int64_t c = lane; c < cols; c += 32) dx[r * cols + c] = yr[c] * (dr[c] - s);
   }
 }
-// mean over rows of -sum_c label*log(softmax(logits)); one block, one warp per row
-// (src/gpu_op.cu:261-301, without its 4096-row limit).
-__global__ void __launch_bounds__(1024) softmax_xent_kernel(const float* __restrict__ logits, const float* __restrict__ labels, float* __restrict__ out, int64_t rows, int64_t cols) {
+// mean over rows of -sum_c label*log(softmax(logits)); one warp per row, rows dealt to the blocks, the last block adds the
+// blocks' sums (src/gpu_op.cu:261-301, without its 4096-row limit).  A single block took 57 us for 1000 rows of 10.
+__global__ void __launch_bounds__(kBlock) softmax_xent_kernel(const float* __restrict__ logits, const float* __restrict__ labels, float* __restrict__ out, float* __restrict__ part, int64_t rows, int64_t cols,
+                                                              uint32_t* counter) {
   __shared__ float red[33];
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  grid_dep_sync();
+  const int lane = threadIdx.x & 31;
+  const int64_t w = (int64_t)blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5), nw = (int64_t)gridDim.x * (kBlock / 32);
   float acc = 0.f;
   for (int64_t r = w; r < rows; r += nw) {
     const float* x = logits + r * cols;
@@ -302,6 +393,11 @@ __global__ void __launch_bounds__(1024) softmax_xent_kernel(const float* __restr
     for (int64_t c = lane; c < cols; c += 32) l -= t[c] * (x[c] - m - ls);
     acc += l;   // every lane holds a partial of this row
   }
+  acc = block_sum(acc, red);
+  if (threadIdx.x == 0) part[blockIdx.x] = acc;
+  if (!arrives_last(counter, gridDim.x)) return;
+  acc = 0.f;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += kBlock) acc += __ldcg(part + i);
   acc = block_sum(acc, red);
   if (threadIdx.x == 0) out[0] = acc / (float)rows;
 }
@@ -539,7 +635,68 @@ static inline float* FM(DLArrayHandle a) { return out_f32(a); }
 
 namespace tf {
 // The plain kernel of a held-back call (the output's write version was bumped when the call was recorded).
+// The bias of a layer in one pass: the broadcast tensor, the sum and (relu_out) its ReLU.  Launch-bound: these are the
+// 64 x 256 tensors of small steps, 2 us a launch.
+template <bool VEC>
+__global__ void __launch_bounds__(kBlock) bias_kernel(const float* __restrict__ x, BiasBcast bc, float* __restrict__ sum, float* __restrict__ relu_out, int64_t n, AmaxOut am) {
+  grid_dep_sync();
+  const FRelu relu;
+  uint32_t m = 0;
+  if (VEC) {                 // runs of 4 share one channel (low % 4 == 0) or read 4 neighbouring ones (low == 1, C % 4 == 0)
+    const uint32_t nv = (uint32_t)(n >> 2), low = (uint32_t)bc.low, C = (uint32_t)bc.C, stride = gridDim.x * blockDim.x;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += stride) {
+      float4 b;
+      if (low == 1) b = __ldg(reinterpret_cast<const float4*>(bc.bias) + i % (C >> 2));
+      else b.x = b.y = b.z = b.w = __ldg(bc.bias + (i / (low >> 2)) % C);
+      reinterpret_cast<float4*>(bc.out)[i] = b;
+      if (!sum) continue;
+      const float4 v = reinterpret_cast<const float4*>(x)[i];
+      const float4 t = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+      reinterpret_cast<float4*>(sum)[i] = t;
+      if (!relu_out) continue;
+      const float4 u = make_float4(relu(t.x), relu(t.y), relu(t.z), relu(t.w));
+      reinterpret_cast<float4*>(relu_out)[i] = u;
+      m = amax4(m, u);
+    }
+  } else {
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+      const float b = __ldg(bc.bias + (bc.low == 1 ? i : i / bc.low) % bc.C);
+      bc.out[i] = b;
+      if (!sum) continue;
+      const float t = x[i] + b;
+      sum[i] = t;
+      if (relu_out) { const float u = relu(t); relu_out[i] = u; m = max(m, amax_bits(u)); }
+    }
+  }
+  amax_commit(am, m);
+}
+static int launch_bias(const DeferredOp& op, float* relu_out, cudaStream_t s) {
+  note_compute_stream(s);
+  const bool sum = op.kind == kDeferBiasAdd;
+  KernelTimer kt("bias", s, 0, (sum ? relu_out ? 16.0 : 12.0 : 4.0) * op.n);
+  const bool vec = op.n % 4 == 0 && op.n < (1ll << 31) && (op.bc.low % 4 == 0 || (op.bc.low == 1 && op.bc.C % 4 == 0 && aligned16(op.bc.bias))) && aligned16(op.bc.out) &&
+                   (!sum || (aligned16(op.a) && aligned16(op.out))) && (!relu_out || aligned16(relu_out));
+  float* const sum_out = sum ? op.out : nullptr;
+  const AmaxOut am = relu_out ? amax_track_begin(relu_out) : AmaxOut{};
+  if (vec) launch_dep(bias_kernel<true>, dim3(grid_for(op.n, kBlock, 4)), dim3(kBlock), 0, s, op.a, op.bc, sum_out, relu_out, op.n, am);
+  else launch_dep(bias_kernel<false>, dim3(grid_for(op.n, kBlock)), dim3(kBlock), 0, s, op.a, op.bc, sum_out, relu_out, op.n, am);
+  TF_AFTER(s, "bias");
+  return 0;
+}
+// ReLU forward of a held-back bias sum.  True when it was done here.
+static bool relu_of_bias_sum(const DLArrayHandle input, DLArrayHandle output, cudaStream_t s, int* rc) {
+  DeferredOp op;
+  if (!take_deferred(kDeferBiasAdd, (const float*)input->data, numel(input), &op)) return false;
+  float* r = (float*)output->data;
+  const bool fused = op.stream == s && r != op.out && r != op.a && r != op.bc.out && r != op.bc.bias;
+  if (fused) { note_write(r); *rc = launch_bias(op, r, s); }
+  else launch_deferred_now(op);
+  release_deferred();
+  return fused;
+}
 int launch_deferred_now(const DeferredOp& op) {
+  if (op.kind == kDeferBcast || op.kind == kDeferBiasAdd) return launch_bias(op, nullptr, op.stream);
   if (op.kind == kDeferAdd) return run_map2(op.a, op.b, op.out, op.n, op.stream, "DLGpuMatrixElementwiseAdd", FAdd{});
   return run_map2(op.a, op.b, op.out, op.n, op.stream, "DLGpuActivationBackward(relu)", FReluGrad{});
 }
@@ -594,6 +751,10 @@ int DLGpuBroadcastTo0(const DLArrayHandle input, DLArrayHandle output, void** cu
   int64_t inner = numel(input), total = numel(output);
   TF_REQUIRE(inner > 0 && total % inner == 0, "DLGpuBroadcastTo0: output size %lld is not a multiple of input size %lld", (long long)total, (long long)inner);
   cudaStream_t s = stream_of(cudaStream);
+  if (t_recording && deferral_enabled() && input->data != output->data) {
+    defer_op(DeferredOp{kDeferBcast, nullptr, nullptr, nullptr, total, s, BiasBcast{F(input), inner, 1, FM(output)}});
+    return 0;
+  }
   note_compute_stream(s);
   bcast_tail_kernel<<<grid_for(total, kBlock), kBlock, 0, s>>>(F(input), FM(output), inner, total);
   TF_AFTER(s, "DLGpuBroadcastTo0");
@@ -607,6 +768,10 @@ int DLGpuBroadcastTo1(const DLArrayHandle input, DLArrayHandle output, void** cu
   for (int i = 2; i < output->ndim; ++i) low *= output->shape[i];
   int64_t total = numel(output);
   cudaStream_t s = stream_of(cudaStream);
+  if (t_recording && deferral_enabled() && input->data != output->data) {
+    defer_op(DeferredOp{kDeferBcast, nullptr, nullptr, nullptr, total, s, BiasBcast{F(input), output->shape[1], low, FM(output)}});
+    return 0;
+  }
   note_compute_stream(s);
   bcast_channel_kernel<<<grid_for(total, kBlock), kBlock, 0, s>>>(F(input), FM(output), output->shape[1], low, total);
   TF_AFTER(s, "DLGpuBroadcastTo1");
@@ -618,10 +783,34 @@ static int reduce_to_scalar(const float* in, float* out, int64_t n, float scale,
   float* part = (float*)persistent_scratch(0, sizeof(float) * 4096);
   TF_REQUIRE(part, "%s: scratch allocation failed", what);
   if (blocks > 4096) blocks = 4096;
+  uint32_t* counter = arrival_counters(1);
+  TF_REQUIRE(counter, "%s: scratch allocation failed", what);
   note_compute_stream(s);
-  partial_sum_kernel<<<blocks, kBlock, 0, s>>>(in, part, n);
-  final_sum_kernel<<<1, kBlock, 0, s>>>(part, out, blocks, scale);
-  if (after_launch(s, what, 2) != 0) return -1;
+  launch_dep(sum_kernel, dim3(blocks), dim3(kBlock), 0, s, in, out, part, n, scale, counter);
+  TF_AFTER(s, what);
+  return 0;
+}
+
+// Channel sums of [N][C][L]: the images split so that about four blocks per SM run, each with a few thousand elements.
+static int channel_sums(const float* in, float* out, int64_t N, int64_t C, int64_t L, cudaStream_t s, const char* what) {
+  TF_REQUIRE(C < (1ll << 31), "%s: too many channels", what);
+  int64_t splits = std::max<int64_t>(1, 4 * device_sm_count() / C);
+  splits = std::min(splits, std::max<int64_t>(1, N * L / 4096));
+  splits = std::min<int64_t>(std::min(splits, N), 65535);
+  splits = std::max<int64_t>(splits, 1);
+  const int64_t nps = std::max<int64_t>(1, (N + splits - 1) / splits);
+  splits = std::max<int64_t>(1, (N + nps - 1) / nps);
+  float* part = nullptr;
+  uint32_t* counters = nullptr;
+  if (splits > 1) {
+    part = (float*)persistent_scratch(2, sizeof(float) * (size_t)splits * (size_t)C);
+    counters = arrival_counters((int)C);
+    TF_REQUIRE(part && counters, "%s: scratch allocation failed", what);
+  }
+  const int vec = L % 4 == 0 && aligned16(in) && nps * (L / 4) < (1ll << 31);
+  note_compute_stream(s);
+  launch_dep(channel_sum_kernel, dim3((unsigned)C, (unsigned)splits), dim3(kBlock), 0, s, in, out, part, N, C, L, nps, vec, counters);
+  TF_AFTER(s, what);
   return 0;
 }
 
@@ -636,18 +825,16 @@ static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, 
   }
   int64_t rps = (rows + splits - 1) / splits;
   splits = (int)((rows + rps - 1) / rps);
-  note_compute_stream(s);
+  float* part = nullptr;
+  uint32_t* counters = nullptr;
   if (splits > 1) {
-    float* part = (float*)persistent_scratch(2, sizeof(float) * (size_t)splits * (size_t)cols);
-    if (part) {
-      colsum_kernel<<<dim3(gx, splits), 256, 0, s>>>(in, part, rows, cols, rps);
-      colsum_final_kernel<<<(unsigned)((cols + 255) / 256), 256, 0, s>>>(part, out, cols, splits);
-      return after_launch(s, what, 2) != 0 ? -1 : 0;
-    }
-    rps = rows;                                  // no scratch: one split
+    part = (float*)persistent_scratch(2, sizeof(float) * (size_t)splits * (size_t)cols);
+    counters = arrival_counters(gx);
+    if (!part || !counters) { splits = 1; rps = rows; }                                  // no scratch: one split
   }
-  colsum_kernel<<<dim3(gx, 1), 256, 0, s>>>(in, out, rows, cols, rps);
-  if (after_launch(s, what, 1) != 0) return -1;
+  note_compute_stream(s);
+  launch_dep(colsum_kernel, dim3(gx, splits), dim3(256), 0, s, in, out, part, rows, cols, rps, counters);
+  TF_AFTER(s, what);
   return 0;
 }
 
@@ -683,6 +870,16 @@ int DLGpuReduceSum(const DLArrayHandle input, DLArrayHandle output, void*** cudn
   bool tail_kept = true;
   for (int i = first_kept; i < p->ndim; ++i) if (p->out_dims[i] != p->in_dims[i]) tail_kept = false;
   if (tail_kept) return column_sums(F(input), FM(output), nin / nout, nout, s, "DLGpuReduceSum");
+  int last_kept = p->ndim - 1;
+  while (last_kept > first_kept && p->out_dims[last_kept] == 1) --last_kept;
+  bool one_run = true;                 // [reduced...][kept...][reduced...]
+  for (int i = first_kept; i <= last_kept; ++i) if (p->out_dims[i] != p->in_dims[i]) one_run = false;
+  if (one_run) {
+    int64_t lead = 1, tail = 1;
+    for (int i = 0; i < first_kept; ++i) lead *= p->in_dims[i];
+    for (int i = last_kept + 1; i < p->ndim; ++i) tail *= p->in_dims[i];
+    return channel_sums(F(input), FM(output), lead, nout, tail, s, "DLGpuReduceSum");
+  }
   ReduceGeom g;
   g.ndim = p->ndim; g.nred = 1;
   int64_t st = 1;
@@ -715,19 +912,8 @@ int DLGpuBroadcastToBackward0(const DLArrayHandle input, DLArrayHandle output) {
 }
 int DLGpuBroadcastToBackward1(const DLArrayHandle input, DLArrayHandle output) {
   TF_REQUIRE(input && output && input->ndim >= 2 && output->ndim == 1 && output->shape[0] == input->shape[1], "DLGpuBroadcastToBackward1: output must be (C,)");
-  ReduceGeom g;
-  g.ndim = input->ndim; g.nred = 1;
-  TF_REQUIRE(g.ndim <= 5, "DLGpuBroadcastToBackward1: rank > 5");
-  int64_t st = 1;
-  for (int d = g.ndim - 1; d >= 0; --d) {
-    g.in_dims[d] = input->shape[d]; g.in_strides[d] = st; st *= input->shape[d];
-    g.reduced[d] = d != 1;
-    if (g.reduced[d]) g.nred *= input->shape[d];
-  }
-  note_compute_stream(0);
-  reduce_general_kernel<<<(unsigned)output->shape[0], kBlock, 0, 0>>>(F(input), FM(output), g);
-  TF_AFTER(0, "DLGpuBroadcastToBackward1");
-  return 0;
+  const int64_t C = input->shape[1], N = input->shape[0];
+  return channel_sums(F(input), FM(output), N, C, N && C ? numel(input) / (N * C) : 0, 0, "DLGpuBroadcastToBackward1");
 }
 int DLGpuReduceSumAxisN(const DLArrayHandle input, DLArrayHandle output, const int axis) {
   TF_REQUIRE(input && output && axis >= 0 && axis < input->ndim, "DLGpuReduceSumAxisN: bad axis");
@@ -827,10 +1013,25 @@ int DLGpuReduceSumAllBackward(const DLArrayHandle input, DLArrayHandle output) {
 
 int DLGpuMatrixElementwiseAdd(const DLArrayHandle matA, const DLArrayHandle matB, DLArrayHandle output, void** cudaStream) {
   TF_SAME(matA, matB, "DLGpuMatrixElementwiseAdd"); TF_SAME(matA, output, "DLGpuMatrixElementwiseAdd");
+  if (t_recording) {           // the sum of a layer and its broadcast bias joins the held-back broadcast
+    DeferredOp op;
+    const cudaStream_t s_here = stream_of_keep_deferred(cudaStream);
+    if (take_deferred(kDeferBcast, nullptr, numel(output), &op)) {
+      const float* x = op.bc.out == F(matB) ? F(matA) : op.bc.out == F(matA) ? F(matB) : nullptr;
+      const bool joins = x && x != op.bc.out && op.stream == s_here && output->data != (void*)op.bc.out && output->data != (const void*)op.bc.bias;
+      release_deferred();
+      if (joins) {
+        op.kind = kDeferBiasAdd; op.a = x; op.out = FM(output);
+        defer_op(op);
+        return 0;
+      }
+      launch_deferred_now(op);
+    }
+  }
   cudaStream_t s = stream_of(cudaStream);
   // Held back for one call: if the ReLU forward of this sum comes next, one kernel writes both.
   if (deferral_enabled() && numel(output) >= (1 << 16)) {
-    defer_op(DeferredOp{kDeferAdd, F(matA), F(matB), FM(output), numel(output), s});
+    defer_op(DeferredOp{kDeferAdd, F(matA), F(matB), FM(output), numel(output), s, BiasBcast{}});
     return 0;
   }
   return run_map2(F(matA), F(matB), FM(output), numel(output), s, "DLGpuMatrixElementwiseAdd", FAdd{});
@@ -860,6 +1061,8 @@ int TfMatrixMultiplyByArray(const DLArrayHandle input, const DLArrayHandle scala
 }
 int DLGpuRelu(const DLArrayHandle input, DLArrayHandle output) {
   TF_SAME(input, output, "DLGpuRelu");
+  int rc = 0;
+  if (t_recording && relu_of_bias_sum(input, output, recording_stream(), &rc)) return rc;
   return run_map1(F(input), FM(output), numel(output), last_compute_stream(), "DLGpuRelu", FRelu{});
 }
 int DLGpuReluGradient(const DLArrayHandle input, const DLArrayHandle in_grad, DLArrayHandle output) {
@@ -896,7 +1099,12 @@ int DLGpuSoftmaxCrossEntropy(const DLArrayHandle input_a, const DLArrayHandle in
   TF_REQUIRE(input_a && input_b && output && input_a->ndim == 2 && same_shape(input_a, input_b) && numel(output) == 1, "DLGpuSoftmaxCrossEntropy: expects two matching 2-D arrays and a 1-element output");
   cudaStream_t s = stream_of(cudaStream);
   note_compute_stream(s);
-  softmax_xent_kernel<<<1, 1024, 0, s>>>(F(input_a), F(input_b), FM(output), input_a->shape[0], input_a->shape[1]);
+  const int64_t rows = input_a->shape[0];
+  const int blocks = (int)std::min<int64_t>(std::max<int64_t>(1, (rows + kBlock / 32 - 1) / (kBlock / 32)), 2 * device_sm_count());
+  float* part = (float*)persistent_scratch(0, sizeof(float) * 4096);
+  uint32_t* counter = arrival_counters(1);
+  TF_REQUIRE(part && counter, "DLGpuSoftmaxCrossEntropy: scratch allocation failed");
+  launch_dep(softmax_xent_kernel, dim3(blocks), dim3(kBlock), 0, s, F(input_a), F(input_b), FM(output), part, rows, input_a->shape[1], counter);
   TF_AFTER(s, "DLGpuSoftmaxCrossEntropy");
   return 0;
 }
@@ -1010,6 +1218,11 @@ int DLGpuActivationForward(const DLArrayHandle input, DLArrayHandle output, int 
     // the sum this ReLU reads was held back: one kernel writes the sum and its ReLU
     DeferredOp add;
     const cudaStream_t s_here = stream_of_keep_deferred(cudaStream);
+    int rc = 0;
+    if (t_recording && relu_of_bias_sum(input, output, s_here, &rc)) {
+      tc_note_relu_output(plan_of<TensorPlan>(cudnnlist, kPlanTensor), output->data);
+      return rc;
+    }
     if (take_deferred(kDeferAdd, F(input), n, &add)) {
       // the slot is locked until release_deferred(): nothing below may call stream_of() / last_compute_stream()
       float* r = (float*)output->data;
@@ -1065,7 +1278,7 @@ int DLGpuActivationBackward(const DLArrayHandle input, DLArrayHandle dinput, con
     case 1:
       // Held back for one call: if the batch-norm backward that consumes this gradient comes next, one kernel does both.
       if (deferral_enabled() && n >= (1 << 16)) {
-        defer_op(DeferredOp{kDeferReluBwd, F(input), F(doutput), FM(dinput), n, s});
+        defer_op(DeferredOp{kDeferReluBwd, F(input), F(doutput), FM(dinput), n, s, BiasBcast{}});
         return 0;
       }
       return run_map2(F(input), F(doutput), FM(dinput), n, s, "DLGpuActivationBackward(relu)", FReluGrad{});

@@ -147,7 +147,10 @@ static void flush_recorded() {
 }
 // Freeing an array only concerns the held-back call if the array is one of its operands.
 void flush_deferred_if_uses(const void* data) {
-  if (t_recording) { if (data == t_rec_deferred.a || data == t_rec_deferred.b || data == t_rec_deferred.out) flush_recorded(); return; }
+  if (t_recording) {
+    if (data == t_rec_deferred.a || data == t_rec_deferred.b || data == t_rec_deferred.out || data == t_rec_deferred.bc.bias || data == t_rec_deferred.bc.out) flush_recorded();
+    return;
+  }
   if (!g_deferred_pending.load(std::memory_order_acquire)) return;
   std::lock_guard<std::mutex> lk(g_deferred_mu);
   if (!g_deferred_pending.load(std::memory_order_relaxed)) return;

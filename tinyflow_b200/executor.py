@@ -25,7 +25,7 @@ import time
 import weakref
 
 from . import gpu_op, ndarray, step_graph
-from .graph import (AdamOp, SgdOp, Variable, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
+from .graph import (AddOp, AdamOp, OnesLikeOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
 
 
 def getcomputelist(Variable_node_list, Variable_node_grad_list, b1, b2, b1t, b2t, e, learning_rate):
@@ -191,6 +191,7 @@ class Executor(object):
         self._leases = {}          # node index -> weak references to the views of its array that were handed out
         self._recordings = step_graph.Recordings()
         self._record_failures = 0
+        self._constants = set()    # indices of the fill nodes whose array holds their constant already
         self.host_values = {}      # node index -> pinned host NDArray holding a swapped-out tensor
         self.have_plan = False
         self._swap_worker = None
@@ -213,6 +214,7 @@ class Executor(object):
 
     def _forget_recordings(self):
         self._recordings.clear()
+        self._constants.clear()
 
     def _ensure_handles(self):
         if self.cudaStream is None:
@@ -305,7 +307,12 @@ class Executor(object):
     def _lease(self, n):
         """A view of node ``n``'s array for the caller; the next step leaves the array alone while a view is alive."""
         view = self._resident(n).borrow()
-        self._leases.setdefault(n.index, []).append(weakref.ref(view))
+        if n.index in self._constants:           # whoever looks may write: the constant is filled in anew
+            self._forget_recordings()
+        ref = weakref.ref(view)
+        while n is not None:                     # a sum that is a view of its operand keeps that one's array, too
+            self._leases.setdefault(n.index, []).append(ref)
+            n = self._unchanged_operand(n) if type(n.op) is AddOp else None
         return view
 
     def _live_leases(self):
@@ -326,6 +333,17 @@ class Executor(object):
         if short:
             raise MemoryError("device out of memory inside node %d (%s): %d bytes short" % (node.index, node.name, short))
         self._values[node.index] = out
+
+    def _unchanged_operand(self, node):
+        """The operand a sum is equal to because the other one is a zeros node (the gradient of a broadcast's shape
+        operand, which every bias adds to its layer's gradient), or None."""
+        a, b = node.inputs
+        shapes = self.node_to_shape_map
+        if shapes[a] != shapes[b] or a in self._feed or b in self._feed:
+            return None
+        if type(b.op) is ZerosLikeOp:
+            return a
+        return b if type(a.op) is ZerosLikeOp else None
 
     def _update_parameters(self, nodes, stream):
         """The optimiser nodes of a step, one launch for all that share a rule (their place in the order is behind every
@@ -371,6 +389,19 @@ class Executor(object):
             out = previous.pop(node.index, None)
             if out is not None and (self.have_plan or out.is_freed or out.shape != shapes[node]):
                 out = None
+            if together and type(node.op) in (ZerosLikeOp, OnesLikeOp):
+                # nobody else writes its array, so the constant of the first step is still there
+                if out is None or node.index not in self._constants:
+                    self._compute(node, out, stream)
+                    self._constants.add(node.index)
+                else:
+                    self._values[node.index] = out
+                continue
+            if together and type(node.op) is AddOp:
+                same = self._unchanged_operand(node)
+                if same is not None:               # x + 0 is x: a view of it
+                    self._values[node.index] = self._resident(same).borrow()
+                    continue
             if self.have_plan:
                 for idx in node.recompute_list:
                     self._compute(self.topo_order[idx], None, stream)
