@@ -1,0 +1,45 @@
+"""Schedules of the one-CTA tensor-core kernel: shared activation blocks, resident filters, clusters, accumulator layouts."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_ops import env  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+# N, C, H, W, K, R, S, padding
+@pytest.mark.parametrize("case", [
+    (16, 64, 5, 5, 64, 3, 3, "SAME"),         # all nine taps in one block
+    (2, 64, 9, 29, 96, 3, 3, "SAME"),         # two rows of taps in a block
+    (1, 72, 6, 61, 132, 3, 3, "SAME"),        # one row of taps in a block, ragged channels
+    (3, 128, 30, 7, 64, 7, 1, "SAME"), (3, 64, 7, 30, 200, 1, 7, "SAME"),
+    (12, 64, 42, 42, 64, 3, 3, "SAME"),       # more tiles than SMs: filters stay in shared memory
+    (13, 64, 40, 40, 256, 1, 1, "VALID"), (13, 248, 40, 41, 60, 1, 1, "VALID"),
+    (2, 384, 8, 8, 384, 1, 3, "SAME"), (9, 1024, 4, 4, 96, 1, 1, "SAME"), (2, 512, 6, 6, 136, 3, 3, "SAME"), (5, 256, 17, 17, 160, 3, 3, "SAME"),    # few tiles: clusters of several sizes
+    (20, 512, 30, 30, 128, 3, 3, "SAME"),     # cross terms promoted twice in a tile
+])
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+def test_convolution_schedules(env, case, arith):
+    N, C, H, W, K, R, S, padding = case
+    rng = np.random.RandomState(C + K + W)
+    x, w = rng.randn(N, C, H, W).astype(np.float32), rng.randn(K, C, R, S).astype(np.float32)
+    out, cell = env.gpu_op.convolution_2d_forward_get_out_shape(x.shape, w.shape, "NCHW", padding, 1, 1)
+    dy = rng.randn(*out).astype(np.float32)
+
+    def run(path, x, w, dy):
+        X, Wd, DY = (env.nd.array(v, env.ctx) for v in (x, w, dy))
+        y, dx, dw = env.nd.empty(out, env.ctx), env.nd.empty(x.shape, env.ctx), env.nd.empty(w.shape, env.ctx)
+        env.gpu_op.set_contraction_path(path)
+        env.gpu_op.set_tensor_arithmetic(arith)
+        try:
+            env.gpu_op.convolution_2d_forward(X, Wd, y, cell, env.cudnn, env.stream)
+            env.gpu_op.convolution_backward_data(X, DY, Wd, dx, cell, env.cudnn, env.stream)
+            env.gpu_op.convolution_backward_filter(X, DY, Wd, dw, cell, env.cudnn, env.stream)
+        finally:
+            env.gpu_op.set_contraction_path(0)
+            env.gpu_op.set_tensor_arithmetic("3xfp16")
+        return [v.asnumpy().astype(np.float64) for v in (y, dx, dw)]
+
+    got, want, mag = run(2, x, w, dy), run(1, x, w, dy), run(1, np.abs(x), np.abs(w), np.abs(dy))
+    for name, g, e, m in zip(("forward", "backward-data", "backward-filter"), got, want, mag):
+        assert np.all(np.abs(g - e) <= 2e-6 * m + 1e-30), (name, float(np.max(np.abs(g - e) / (m + 1e-30))))

@@ -23,11 +23,11 @@
 //                     are M/N-major, the reduction runs over pixel rows, split over CTAs and combined
 //                     with fp32 atomics.
 //
-// Kernel roles (320 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2-9 =
-// epilogue (two per TMEM lane quarter, half the columns each).  Shared memory holds a ring of stages {A_hi, A_lo, B_hi, B_lo}
-// (128-byte swizzle, 64 halves of K per stage); TMEM holds two accumulators so that promoting one group of
-// stages to registers overlaps the MMAs of the next.  Every mbarrier wait is bounded: on time-out the CTA raises an
-// error flag the host reads, drains its outstanding copies, frees its TMEM and returns.
+// Kernel roles (384 threads): warps 0 and 11 = TMA producers of A and B, warp 1 = TMEM owner and issuer of the wide MMAs, warp
+// 10 = issuer of the narrow ones, warps 2-9 = epilogue (two per TMEM lane quarter, half the columns each).  Shared memory holds
+// a ring of A blocks and a ring of B tiles (hi and lo, 128-byte swizzle, 64 halves of K per stage); TMEM holds two accumulator
+// sets so that promoting one group of stages to registers overlaps the MMAs of the next.  Every mbarrier wait is bounded: on
+// time-out the CTA raises an error flag the host reads, drains its outstanding copies, frees its TMEM and returns.
 #include "common.h"
 #include <cuda.h>
 #include <cuda_fp16.h>
@@ -156,6 +156,7 @@ void amax_set_carry_valid(const void* data) {
 // ------------------------------------------------------------------------------------------------
 constexpr int BM = 128;            // UMMA M (TMEM lanes)
 constexpr int kThreads = 320;
+constexpr int kNarrowWarp = 10, kBWarp = 11, kGemmThreads = 384;     // one-CTA kernel: two more warps issue
 // The two arithmetic modes differ only in the element type of the packed operands.  A stage always holds one
 // 128-byte swizzle row of K per tile row (K-major) or 128 bytes of M/N per K row (M/N-major), and is consumed by four
 // MMAs; the tile byte sizes are therefore the same in both modes and only the element counts change.
@@ -225,6 +226,34 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     if (clock64() - t0 > limit_cycles) { *abort_flag = 1; return false; }
   }
 }
+// One lane of a converged warp.  tcgen05.mma and the bulk copies take their operands from uniform registers: under a branch the
+// compiler knows to be taken by one elected lane of a converged warp it moves them there directly, under `lane == 0` it
+// serialises over the (possibly) active lanes first.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t yes;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(yes));
+  return yes != 0;
+}
+// The same for the warps that issue copies and MMAs.  Nothing their loops do may branch on the outcome: as long as all control
+// flow is uniform the compiler keeps stage counters, descriptors and coordinates in uniform registers, where these
+// instructions take them from.  So a wait that gives up only marks the role as `bad`, which then issues nothing more and runs
+// through the rest of its loop.
+__device__ __forceinline__ void mbar_wait_mark(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int& bad) {
+  if (!bad && !mbar_wait(bar, parity, abort_flag)) bad = 1;
+}
+// Non-blocking look at a phase; true: complete (and the data it guards visible to this lane)
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ void tensormap_prefetch(const CUtensorMap* map) {
+  asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar)) : "memory");
@@ -232,14 +261,6 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z) : "memory");
-}
-// im2col-mode load over a [N][H][W][C] tensor: `pixels` consecutive base pixels starting at (w, h, n) - walking w, then h,
-// then n inside the map's bounding box - each displaced by the window offset (off_w, off_h); positions outside the
-// tensor read as zero.  Lands [pixels][channels of one 128-byte row], swizzled like a tiled load.
-__device__ __forceinline__ void tma_load_im2col(void* dst, const CUtensorMap* map, int c, int w, int h, int n, int off_w, int off_h, uint64_t* bar) {
-  asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.im2col.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2], {%7, %8};"
-               ::"r"(smem_u32(dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(c), "r"(w), "r"(h), "r"(n),
-                 "h"((unsigned short)off_w), "h"((unsigned short)off_h) : "memory");
 }
 __device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
@@ -252,15 +273,20 @@ __device__ __forceinline__ void umma(uint32_t tmem_d, uint64_t adesc, uint64_t b
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0) : "memory");
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
   } else {
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(0), "r"(0), "r"(0), "r"(0) : "memory");
+        "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
   }
+}
+// The same with descriptors in two words each: only the low word (the address) differs from one MMA to the next
+template <int AR>
+__device__ __forceinline__ void umma_at(uint32_t tmem_d, uint32_t a_low, uint32_t a_high, uint32_t b_low, uint32_t b_high, uint32_t idesc, uint32_t accumulate) {
+  umma<AR>(tmem_d, (uint64_t)a_low | (uint64_t)a_high << 32, (uint64_t)b_low | (uint64_t)b_high << 32, idesc, accumulate);
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float* v) {
   uint32_t* r = reinterpret_cast<uint32_t*>(v);
@@ -346,6 +372,7 @@ __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr, uint32_t lbo_bytes
 // ------------------------------------------------------------------------------------------------
 enum { kModeGemm = 0, kModeConv = 1, kModeWgrad = 2 };
 enum { kEpiRowMajor = 0, kEpiNchw = 1, kEpiWgrad = 2 };
+enum { kAccPair = 0, kAccThree = 1 };
 constexpr int kMaxTaps = 49;
 
 struct alignas(64) GemmParams {
@@ -373,31 +400,29 @@ struct alignas(64) GemmParams {
   // rows with i >= valid_h, j >= valid_w or (oi, oj) outside the plane are dropped
   int frame_h, frame_w, valid_h, valid_w, out_c, out_h, out_w, out_sh, out_sw, out_off_h, out_off_w;
   int* err;                       // device-visible error word (mapped host memory)
-  // im2col != 0: the activation operand A is a halo-free [N][im_h'][im_w'][C] pack read through an im2col tensor map;
-  // rows of the GEMM are the im_h x im_w base pixels per image (the output positions), the map's lower corner is
-  // (im_lo_w, im_lo_h) and tap t adds the window offset (tap_off[t] & 0xffff, tap_off[t] >> 16)
-  int im2col, im_w, im_h, im_lo_w, im_lo_h;
   int slot, taps_per_tile;        // kModeWgrad: M-tile rows are taps_per_tile slots of `slot` input channels, one filter tap per slot
   int group_iters;                // stages accumulated in TMEM before the epilogue promotes them to registers
   int data_by_data;               // both operands are activations / gradients (filter gradients, X^T dY): host-side hint for group_iters
-  // Where the two small cross terms accumulate.  0: A_lo*B_hi joins A_hi*B_hi (block 0), A_hi*B_lo alone in block 1.
-  // 1: both cross terms in block 1.  2: the B stage is laid out [B_lo ; B_hi], so the wide MMA leaves A_hi*B_lo in block 0
-  // and A_hi*B_hi in block 1, and A_lo*B_hi joins block 0.  In 1 and 2 the large accumulator sees one truncating
-  // accumulation per K step instead of two; in 2 the narrow MMA depends on the first half of the wide one, not the last.
-  int acc_layout;
-  int tap_off[kMaxTaps];          // row shift per tap (applied to the activation operand A)
+  // Shared memory: a ring of A blocks and a ring of B tiles.  A filter's taps read the same rows of the activation matrix
+  // at different shifts, so in kModeConv an A block holds a_rows >= 128 rows, fetched once, and serves every tap of a run (taps
+  // whose shifts lie within a_rows - 128 of one another); a tap's operand is the block's start address plus shift * 128 bytes.
+  // Everywhere else a block serves one stage.  b_resident: one B tile per CTA for the whole launch, all its stages kept.
+  int a_rows, a_slots, b_slots, b_resident;
+  int one_ring;                   // A and B of a stage share slot number and barriers (every block serves one stage)
+  int acc_mode;                   // where the accumulators sit in TMEM: kAccPair or kAccThree (see the MMA issuer)
+  int cross_groups;               // kAccThree: groups whose cross terms accumulate before they are promoted
+  int cluster;                    // > 1: the reduction of every tile is cut over the CTAs of a cluster and added up in shared memory
+  // kModeConv, taps in the order they are walked for every chunk of channels (runs one after the other):
+  uint32_t tap_word[kMaxTaps];    // row shift inside the run's block | first tap of its run << 8 | last << 9
+  int tap_off[kMaxTaps];          // row shift of the run's first tap, applied to A (filter gradients, pair kernel: of the tap itself)
   short tap_col[kMaxTaps];        // first column of the tap's channels in A (space-to-depth packs keep one phase per column block)
-  short tap_b[kMaxTaps];          // kModeConv: which tap block of the packed filter the tap multiplies
+  short tap_b[kMaxTaps];          // which tap block of the packed filter the tap multiplies
+  short pair_shift[kMaxTaps];     // pair kernel: the tap's own row shift is tap_off + pair_shift
 };
-
-template <int BN> struct SmemLayout {
-  static constexpr int kStages = BN <= 96 ? 4 : 3;
-  static constexpr int kABytes = BM * 128;              // 16 KiB: 128 tile rows x one 128-byte swizzle row
-  static constexpr int kBBytes = BN * 128;
-  static constexpr int kStageBytes = 2 * kABytes + 2 * kBBytes;
-  static constexpr int kBarrierBytes = 256;
-  static constexpr int kTotal = kStages * kStageBytes + kBarrierBytes + 1024;   // + slack to align to 1024
-};
+constexpr int kMaxASlots = 4, kMaxBSlots = 16, kMaxCluster = 8;
+constexpr int kSmemBarriers = 512;
+constexpr int kSmemLimit = 232448 - 1024;            // 227 KiB less the slack to align to 1024
+static inline int gemm_smem_bytes(const GemmParams& p, int bn) { return p.a_slots * p.a_rows * 256 + p.b_slots * bn * 256 + kSmemBarriers + 1024; }
 
 // One unit of a CTA's work: `kcount` stages of tile `tile` starting at stage k0.  slot < 0: the item is the tile's
 // whole reduction and its epilogue stores to the output; otherwise its partial sums go to that workspace slot.
@@ -408,6 +433,7 @@ struct WorkIter {
   __device__ __forceinline__ explicit WorkIter(const GemmParams& p) {
     tile = blockIdx.x;
     u = u1 = first_tail_tile = 0;
+    if (p.cluster > 1) return;
     if (p.tail_share > 0) {
       u = blockIdx.x * p.tail_share;
       u1 = min(u + p.tail_share, p.tail_tiles * p.k_total);
@@ -415,6 +441,15 @@ struct WorkIter {
     }
   }
   __device__ __forceinline__ bool next(const GemmParams& p, WorkItem& w) {
+    if (p.cluster > 1) {                  // one item per CTA: its share of the cluster's tile
+      if (tile < 0) return false;
+      const int rank = tile % p.cluster;
+      w.tile = tile / p.cluster; w.slot = -1;
+      w.k0 = (int)((long long)p.k_total * rank / p.cluster);
+      w.kcount = (int)((long long)p.k_total * (rank + 1) / p.cluster) - w.k0;
+      tile = -1;
+      return true;
+    }
     const int whole = p.tail_share > 0 ? p.full_tiles : p.full_tiles + p.tail_tiles;
     if (tile < whole) {
       w.tile = tile; w.k0 = 0; w.kcount = p.k_total; w.slot = -1;
@@ -463,153 +498,231 @@ __device__ __forceinline__ RowAddr row_address(const GemmParams& p, int mt, int 
   return r;
 }
 
+// Per-tap values of a convolution, spread over the lanes of a warp: a look-up by a counter that every lane knows is one
+// reduction, where an indexed read of the parameter space is a chain of constant-cache loads in front of every stage.  (A
+// reduction and not a shuffle: its result is known to be the same in all lanes, so what is computed from it can stay in
+// uniform registers.)
+struct TapTable {
+  uint32_t v0, v1;
+  int lane;
+  template <class F> __device__ __forceinline__ TapTable(int n, int lane_, F&& f) : lane(lane_) {
+    v0 = lane < n ? f(lane) : 0u;
+    v1 = lane + 32 < n ? f(lane + 32) : 0u;
+  }
+  __device__ __forceinline__ uint32_t at(int i) const { return __reduce_or_sync(0xffffffffu, lane == (i & 31) ? (i < 32 ? v0 : v1) : 0u); }
+};
+__device__ __forceinline__ float ld_cluster(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+// 32 (16) columns of BLOCKS accumulator blocks, block_cols columns apart, of this thread's row, added
+template <int NC, int BLOCKS> __device__ __forceinline__ void load_sum(uint32_t taddr, uint32_t block_cols, float2* v) {
+  float2 b[BLOCKS > 1 ? BLOCKS - 1 : 1][NC / 2];
+  if (NC == 32) {
+    tmem_ld32(taddr, reinterpret_cast<float*>(v));
+#pragma unroll
+    for (int i = 1; i < BLOCKS; ++i) tmem_ld32(taddr + i * block_cols, reinterpret_cast<float*>(b[i - 1]));
+  } else {
+    tmem_ld16(taddr, reinterpret_cast<float*>(v));
+#pragma unroll
+    for (int i = 1; i < BLOCKS; ++i) tmem_ld16(taddr + i * block_cols, reinterpret_cast<float*>(b[i - 1]));
+  }
+  tmem_ld_wait();
+#pragma unroll
+  for (int i = 1; i < BLOCKS; ++i)
+#pragma unroll
+    for (int q = 0; q < NC / 2; ++q) v[q] = __fadd2_rn(v[q], b[i - 1][q]);
+}
+
+// What bounds it.  A K step of 16 is 192 tensor cycles at BN = 128 (N = 2*BN and N = BN).  Its operands are read from shared
+// memory at 128 bytes per cycle: 12 KB for the wide and 8 KB for the narrow instruction, 160 cycles; TMA writes another 64 KB per
+// stage of four K steps, 512 cycles, so with one block per stage shared memory alone takes 1152 cycles against 768 of the
+// tensor pipe, and that is what long reductions ran at (1160 measured).  Runs of taps fetch the activation rows once for up to 9
+// stages (36 KB a stage for a 3x3 window of a 28-wide image) and filters of one tile that fit stay in shared memory: with
+// 512 channels, 28 x 28, 3x3, batch 64 the product went from 625 to 548 us, with 64 channels, 224 x 224, from 1128 to 886.
+// Short reductions are bound by start and epilogue: 4000 cycles to the first MMA, 2500-4000 from the last to the end.
 template <int BN, int AR>
-__global__ void __launch_bounds__(kThreads, 1) gemm3x_kernel(const __grid_constant__ GemmParams p) {
+__global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_constant__ GemmParams p) {
   using T = Arith<AR>;
   constexpr int BK = T::kBK;
   constexpr uint32_t kGroupStride = BK * 128;               // M/N-major operands: bytes between 128-byte-wide column groups
-  constexpr int kTmemCols = 4 * BN <= 256 ? 256 : 512;      // two accumulators of 2*BN columns; the allocation is a power of two
-  using L = SmemLayout<BN>;
+  constexpr int kTmemCols = 512;                            // all of it: one CTA per SM
+  constexpr bool kSets3 = BN == 64;                         // room for two complete sets of three accumulator blocks
+  constexpr int kSetCols = kSets3 ? 3 * BN : 2 * BN;
+  constexpr int kBTile = BN * 128, kBSlot = 2 * kBTile;     // the hi and the lo tile, in the order the accumulators ask for
+  const bool three = !kSets3 && p.acc_mode == kAccThree;
+  // Main plus first cross term and the second cross term accumulate into different blocks (unless kAccPair puts them into
+  // one), so two warps issue them, each at its own pace.
+  const int issuers = kSets3 || three ? 2 : 1;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::kStages * L::kStageBytes);
-  uint64_t* empty = full + L::kStages;
-  uint64_t* acc_full = empty + L::kStages;
+  const int a_half = p.a_rows * 128, a_slot_bytes = 2 * a_half;       // hi rows, then lo rows
+  uint8_t* const b_smem = smem + p.a_slots * a_slot_bytes;
+  uint64_t* a_full = reinterpret_cast<uint64_t*>(b_smem + p.b_slots * kBSlot);
+  uint64_t* a_empty = a_full + kMaxASlots;
+  uint64_t* b_full = a_empty + kMaxASlots;
+  uint64_t* b_empty = b_full + kMaxBSlots;
+  uint64_t* acc_full = b_empty + kMaxBSlots;
   uint64_t* acc_empty = acc_full + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* cross_empty = acc_empty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(cross_empty + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < L::kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&acc_full[b], 1); mbar_init(&acc_empty[b], 8); }
-    *abort_flag = 0;
+  if (warp == 0) {         // the whole warp: one thread took 500 cycles over it
+    constexpr int kBars = 2 * kMaxASlots + 2 * kMaxBSlots + 5;
+    for (int i = lane; i < kBars; i += 32) {
+      const int k = i - 2 * kMaxASlots, j = k - 2 * kMaxBSlots;
+      const int count = k < 0 ? (i < kMaxASlots ? 1 : issuers) : j < 0 ? (k < kMaxBSlots ? (p.one_ring ? 2 : 1) : issuers) : j < 2 ? issuers : 8;
+      mbar_init(&a_full[i], count);
+    }
+    if (lane == 0) *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    __syncwarp();
   }
-  if (warp == 1) {   // TMEM: two accumulators of 2*BN fp32 columns each
+  if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
-  grid_dep_sync();          // everything above (barriers, TMEM) overlapped the tail of the kernel in front; operands are read below
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  // Everything up to grid_dep_sync() in the roles below (barriers, TMEM, tap tables) overlaps the tail of the kernel in front.
 
-  if (warp == 0) {
+  if (warp == 0 || warp == kBWarp) {
     // ===================== TMA producer =====================
-    if (lane == 0) {
-      int stage = 0; uint32_t phase = 0;
-      bool armed[L::kStages]; uint32_t armed_phase[L::kStages];
-      for (int s = 0; s < L::kStages; ++s) { armed[s] = false; armed_phase[s] = 0; }
-      bool ok = true;
+    // the whole warp walks the work and waits; one elected lane issues the copies
+    {
+      int as = 0, bs = 0;
+      uint32_t aph = 0, bph = 0;
+      uint32_t armed_a = 0, armed_b = 0, phase_a = 0, phase_b = 0;         // per slot: filled at least once, phase of the last fill
+      int bad = 0;
+      const bool do_a = warp == 0, do_b = !do_a;
+      bool b_loaded = false;
+      int group = 0;                      // as the MMA issuer counts them: the parity decides the order of the B tiles
+      const bool conv = p.mode == kModeConv;
+      const int period = conv ? p.ntaps : 1;
+      const TapTable words(conv ? p.ntaps : 0, lane, [&](int t) { return p.tap_word[t]; });
+      const TapTable offs(conv ? p.ntaps : 0, lane, [&](int t) { return (uint32_t)p.tap_off[t]; });
+      const TapTable cols(conv ? p.ntaps : 0, lane, [&](int t) { return (uint32_t)(uint16_t)p.tap_col[t] | (uint32_t)p.tap_b[t] << 16; });
+      if (elect_one()) {
+        tensormap_prefetch(do_a ? &p.a_hi : &p.b_hi);
+        tensormap_prefetch(do_a ? &p.a_lo : &p.b_lo);
+      }
+      grid_dep_sync();
       WorkIter iter(p);
       WorkItem w;
-      while (ok && iter.next(p, w)) {
+      while (iter.next(p, w)) {
         int mt, nt, tap;
         decode_tile(p, w.tile, mt, nt, tap);
         const int m0 = mt * BM, n0 = nt * BN;
-        // im2col convolution: base pixel (image, row, column) of the tile's first GEMM row
-        int im_n = 0, im_y = 0, im_x = 0;
-        if (p.im2col && p.mode == kModeConv) {
-          const int per_img = p.im_w * p.im_h;
-          im_n = m0 / per_img;
-          const int rem = m0 - im_n * per_img;
-          im_y = rem / p.im_w; im_x = rem - im_y * p.im_w;
-        }
+        int ch = w.k0 / period, ti = w.k0 - ch * period;
+        int left = p.group_iters;         // stages to the next accumulator group
         for (int it = 0; it < w.kcount; ++it) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag)) { ok = false; break; }
-          uint8_t* st = smem + stage * L::kStageBytes;
-          uint8_t *a_hi = st, *a_lo = st + L::kABytes;
-          uint8_t *b_hi = st + 2 * L::kABytes + (p.acc_layout == 2 ? L::kBBytes : 0), *b_lo = st + 2 * L::kABytes + (p.acc_layout == 2 ? 0 : L::kBBytes);
-          mbar_expect_tx(&full[stage], L::kStageBytes);
-          armed[stage] = true; armed_phase[stage] = phase;
           const int git = w.k0 + it;                  // stage index within the tile's reduction
-          int a_col, a_row, b_col, b_row;
-          if (p.mode == kModeConv) {
-            int t = git / p.chunks_per_tap, ch = git - t * p.chunks_per_tap;
-            a_col = p.tap_col[t] + ch * BK; a_row = m0 + p.tap_off[t];
-            b_col = p.tap_b[t] * p.b_tap_pitch + ch * BK; b_row = n0;
-          } else if (p.mode == kModeWgrad) {
-            int krow = git * BK;
-            a_col = mt * p.slot; a_row = krow;      // per-box tap shift applied below
-            b_col = n0; b_row = krow;
-          } else {
-            int kk = git * BK;
-            if (p.a_mn) { a_col = m0; a_row = kk; } else { a_col = kk; a_row = m0; }
-            if (p.b_mn) { b_col = n0; b_row = kk; } else { b_col = kk; b_row = n0; }
+          const uint32_t word = conv ? words.at(ti) : 0x300u, tc = conv ? cols.at(ti) : 0u;
+          const int off = conv ? (int)offs.at(ti) : 0;
+          const bool fetch_a = it == 0 || (word & 0x100u);
+          if (p.one_ring) {
+            mbar_wait_mark(&b_empty[bs], bph ^ 1, abort_flag, bad);
+            armed_b |= 1u << bs; phase_b = (phase_b & ~(1u << bs)) | (bph << bs);
           }
-          // M/N-major operands come through a 3-D view {group width, rows, column groups}: one copy lands
-          // [groups][BK rows][128 B], the layout the M/N-major descriptor expects.
-          if (p.mode == kModeConv && p.im2col) {
-            const int t = git / p.chunks_per_tap;
-            const int ow = p.tap_off[t] & 0xffff, oh = p.tap_off[t] >> 16;
-            tma_load_im2col(a_hi, &p.a_hi, a_col, im_x + p.im_lo_w, im_y + p.im_lo_h, im_n, ow, oh, &full[stage]);
-            tma_load_im2col(a_lo, &p.a_lo, a_col, im_x + p.im_lo_w, im_y + p.im_lo_h, im_n, ow, oh, &full[stage]);
-          } else if (p.mode == kModeWgrad && p.im2col) {
-            // the K rows of this stage are BK consecutive output pixels; every tap slot reads the input pixels they
-            // touch through the im2col map, one 128-byte channel group per copy.  A slot past the last tap asks for
-            // an image index beyond the batch and receives zeros.
-            const int per_img = p.im_w * p.im_h;
-            const int pn = a_row / per_img, prem = a_row - pn * per_img, py = prem / p.im_w, px = prem - py * p.im_w;
-            const int gps = p.slot / T::kGW;
-            for (int sl = 0; sl < p.taps_per_tile; ++sl) {
-              const int t = tap * p.taps_per_tile + sl;
-              const bool live = t < p.ntaps;
-              const int ow = live ? (p.tap_off[t] & 0xffff) : 0, oh = live ? (p.tap_off[t] >> 16) : 0;
-              const int bn_img = live ? pn : 0x00400000;
-              for (int gq = 0; gq < gps; ++gq) {
-                const int c = a_col + gq * T::kGW;
-                tma_load_im2col(a_hi + (sl * gps + gq) * kGroupStride, &p.a_hi, c, px + p.im_lo_w, py + p.im_lo_h, bn_img, ow, oh, &full[stage]);
-                tma_load_im2col(a_lo + (sl * gps + gq) * kGroupStride, &p.a_lo, c, px + p.im_lo_w, py + p.im_lo_h, bn_img, ow, oh, &full[stage]);
+          if (do_a && fetch_a) {
+            if (!p.one_ring) {
+              mbar_wait_mark(&a_empty[as], aph ^ 1, abort_flag, bad);
+              armed_a |= 1u << as; phase_a = (phase_a & ~(1u << as)) | (aph << as);
+            }
+            uint8_t *a_hi = smem + as * a_slot_bytes, *a_lo = a_hi + a_half;
+            uint64_t* bar = p.one_ring ? &b_full[bs] : &a_full[as];
+            if (elect_one() && !bad) {
+              mbar_expect_tx(bar, a_slot_bytes);
+              if (conv) {
+                const int col = (int)(short)(tc & 0xffffu) + ch * BK, row = m0 + off;
+                tma_load_2d(a_hi, &p.a_hi, col, row, bar);
+                tma_load_2d(a_lo, &p.a_lo, col, row, bar);
+              } else if (p.mode == kModeWgrad) {
+                // M/N-major operands come through a 3-D view {group width, rows, column groups}: one copy lands
+                // [groups][BK rows][128 B], the layout the M/N-major descriptor expects.  One copy per tap slot; a slot past
+                // the last tap reads rows beyond the pack (the copy still completes with its full byte count and fills zeros).
+                const int gps = p.slot / T::kGW;
+                for (int sl = 0; sl < p.taps_per_tile; ++sl) {
+                  const int t = tap * p.taps_per_tile + sl;
+                  const int row = t < p.ntaps ? git * BK + p.tap_off[t] : 0x40000000;
+                  const int grp = (mt * p.slot + (t < p.ntaps ? p.tap_col[t] : 0)) / T::kGW;
+                  tma_load_3d(a_hi + sl * gps * kGroupStride, &p.a_hi, 0, row, grp, bar);
+                  tma_load_3d(a_lo + sl * gps * kGroupStride, &p.a_lo, 0, row, grp, bar);
+                }
+              } else if (p.a_mn) {
+                tma_load_3d(a_hi, &p.a_hi, 0, git * BK, m0 / T::kGW, bar);
+                tma_load_3d(a_lo, &p.a_lo, 0, git * BK, m0 / T::kGW, bar);
+              } else {
+                tma_load_2d(a_hi, &p.a_hi, git * BK, m0, bar);
+                tma_load_2d(a_lo, &p.a_lo, git * BK, m0, bar);
               }
             }
-          } else if (p.mode == kModeWgrad) {
-            // One copy per tap slot; a slot past the last tap reads rows beyond the pack (the copy still completes
-            // with its full byte count and fills zeros).
-            const int gps = p.slot / T::kGW;
-            for (int sl = 0; sl < p.taps_per_tile; ++sl) {
-              int t = tap * p.taps_per_tile + sl;
-              int row = t < p.ntaps ? a_row + p.tap_off[t] : 0x40000000;
-              int grp = (a_col + (t < p.ntaps ? p.tap_col[t] : 0)) / T::kGW;
-              tma_load_3d(a_hi + sl * gps * kGroupStride, &p.a_hi, 0, row, grp, &full[stage]);
-              tma_load_3d(a_lo + sl * gps * kGroupStride, &p.a_lo, 0, row, grp, &full[stage]);
+            if (++as == p.a_slots) { as = 0; aph ^= 1; }
+          }
+          if (p.one_ring && !do_b && ++bs == p.b_slots) { bs = 0; bph ^= 1; }
+          if (do_b && !b_loaded) {
+            if (!p.one_ring) {
+              if (!p.b_resident) mbar_wait_mark(&b_empty[bs], bph ^ 1, abort_flag, bad);
+              armed_b |= 1u << bs; phase_b = (phase_b & ~(1u << bs)) | (bph << bs);
             }
-          } else if (p.a_mn) {
-            tma_load_3d(a_hi, &p.a_hi, 0, a_row, a_col / T::kGW, &full[stage]);
-            tma_load_3d(a_lo, &p.a_lo, 0, a_row, a_col / T::kGW, &full[stage]);
-          } else {
-            tma_load_2d(a_hi, &p.a_hi, a_col, a_row, &full[stage]);
-            tma_load_2d(a_lo, &p.a_lo, a_col, a_row, &full[stage]);
+            const bool hi_first = three && (group & 1) == 0;
+            uint8_t *b_lo = b_smem + bs * kBSlot + (hi_first ? kBTile : 0), *b_hi = b_smem + bs * kBSlot + (hi_first ? 0 : kBTile);
+            if (elect_one() && !bad) {
+              mbar_expect_tx(&b_full[bs], kBSlot);
+              if (conv) {
+                const int col = (int)(tc >> 16) * p.b_tap_pitch + ch * BK;
+                tma_load_2d(b_lo, &p.b_lo, col, n0, &b_full[bs]);
+                tma_load_2d(b_hi, &p.b_hi, col, n0, &b_full[bs]);
+              } else if (p.b_mn) {
+                tma_load_3d(b_lo, &p.b_lo, 0, git * BK, n0 / T::kGW, &b_full[bs]);
+                tma_load_3d(b_hi, &p.b_hi, 0, git * BK, n0 / T::kGW, &b_full[bs]);
+              } else {
+                tma_load_2d(b_lo, &p.b_lo, git * BK, n0, &b_full[bs]);
+                tma_load_2d(b_hi, &p.b_hi, git * BK, n0, &b_full[bs]);
+              }
+            }
+            if (++bs == p.b_slots) { bs = 0; bph ^= 1; }
           }
-          if (p.b_mn) {
-            tma_load_3d(b_hi, &p.b_hi, 0, b_row, b_col / T::kGW, &full[stage]);
-            tma_load_3d(b_lo, &p.b_lo, 0, b_row, b_col / T::kGW, &full[stage]);
-          } else {
-            tma_load_2d(b_hi, &p.b_hi, b_col, b_row, &full[stage]);
-            tma_load_2d(b_lo, &p.b_lo, b_col, b_row, &full[stage]);
-          }
-          if (++stage == L::kStages) { stage = 0; phase ^= 1; }
+          if (++ti == period) { ti = 0; ++ch; }
+          if (--left == 0) { left = p.group_iters; ++group; }
         }
+        if (left != p.group_iters) ++group;
+        if (p.b_resident) b_loaded = true;
       }
       if (*abort_flag) {
         // let copies that are still in flight land before the CTA gives its shared memory back
-        for (int s = 0; s < L::kStages; ++s) {
-          if (!armed[s]) continue;
+        for (int s = 0; s < kMaxASlots + kMaxBSlots; ++s) {
+          const bool is_a = s < kMaxASlots;
+          const int i = is_a ? s : s - kMaxASlots;
+          if (!(((is_a ? armed_a : armed_b) >> i) & 1)) continue;
           long long t0 = clock64();
-          while (!mbar_try_wait(&full[s], armed_phase[s]) && clock64() - t0 < 100000000ll) {}
+          while (!mbar_try_wait(is_a ? &a_full[i] : &b_full[i], ((is_a ? phase_a : phase_b) >> i) & 1) && clock64() - t0 < 100000000ll) {}
         }
       }
     }
-  } else if (warp == 1) {
+  } else if (warp == 1 || warp == kNarrowWarp) {
     // ===================== MMA issuer =====================
-    if (lane == 0) {
-      // The B stage holds the two B tiles back to back ([B_lo ; B_hi] in the default accumulator layout 2), so ONE
-      // instruction with N = 2*BN computes A_hi*B_lo (TMEM columns 0..BN-1) and A_hi*B_hi (columns BN..2BN-1); a second
-      // one with N = BN adds A_lo*B_hi to the first block.  The two small cross terms share a block on purpose: every
-      // accumulation into TMEM truncates the sum, an error proportional to the accumulator's magnitude, and the cross
-      // terms are 2^-11 of the main one, so the large accumulator sees one truncation per K step instead of two.
+    {
+      // Three products per K step: A_hi*B_hi (main) and the cross terms A_hi*B_lo, A_lo*B_hi.  The two B tiles lie back to back
+      // in their slot, so ONE instruction with N = 2*BN computes main and the first cross term into neighbouring TMEM blocks.
+      // Every accumulation into TMEM truncates the sum, an error proportional to the accumulator's magnitude; the cross
+      // terms are 2^-11 of the main one and have blocks of their own, so the large accumulator sees one truncation per K step.
+      // Where the blocks lie, and who issues.  One warp issues 8 MMAs, 1-3 commits and the bookkeeping of a stage in some 1250
+      // cycles, where the tensor pipe needs 768 (BN = 128) or 448 (BN = 64).  MMAs into different blocks need no order among
+      // them, so where the two cross terms have blocks of their own two warps issue, one the wide instructions and one the
+      // narrow ones, each at its own pace (512 channels, 28 x 28, 3x3, batch 64: 603 -> 548 us; 64 channels, 224 x 224: 985 -> 886):
+      //   BN = 64           two sets of {cross, main, cross'}: 384 columns;
+      //   kAccThree         main0, cross, main1, cross' (4*BN columns): main alternates between its two blocks from group to group,
+      //                     the cross terms accumulate for cross_groups groups before the epilogue takes them.  The wide
+      //                     instruction goes to (main0, cross) or (cross, main1), hence the order of the B tiles;
+      //   kAccPair          two sets of {cross, main} and one issuer: short reductions, where the next tile must not wait for the
+      //                     epilogue to read the cross terms, and groups of one stage, where the epilogue is the bound anyway.
       // instruction descriptor: D = f32 (bits 4-5 = 1), A format at bit 7, B format at bit 10, majors at bits 15 / 16,
       // N >> 3 at bit 17, M >> 4 at bit 24
       const uint32_t idesc_base = (1u << 4) | (T::kFormat << 7) | (T::kFormat << 10) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16) |
@@ -621,50 +734,99 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_kernel(const __grid_consta
       const uint32_t a_kstep = p.a_mn ? kGroupStride / 4 : 32u, b_kstep = p.b_mn ? kGroupStride / 4 : 32u;
       const uint32_t a_sbo = p.a_mn ? T::kMnSbo : 1024u, b_sbo = p.b_mn ? T::kMnSbo : 1024u;
       const uint32_t a_lt = p.a_mn ? T::kMnLayout : 2u, b_lt = p.b_mn ? T::kMnLayout : 2u;
-      int stage = 0; uint32_t phase = 0;
-      int group = 0;            // accumulator groups issued so far (alternating TMEM buffers)
-      bool ok = true;
-      WorkIter iter(p);
-      WorkItem w;
-      while (ok && iter.next(p, w)) {
-        for (int it0 = 0; it0 < w.kcount && ok; it0 += p.group_iters, ++group) {
-          const int acc = group & 1;
-          if (!mbar_wait(&acc_empty[acc], ((group >> 1) & 1) ^ 1, abort_flag)) { ok = false; break; }
-          tcgen05_fence_after();
-          const uint32_t d_tmem = tmem_base + acc * 2 * BN;
-          const int it1 = min(it0 + p.group_iters, w.kcount);
-          for (int it = it0; it < it1; ++it) {
-            if (!mbar_wait(&full[stage], phase, abort_flag)) { ok = false; break; }
-            tcgen05_fence_after();
-            const uint32_t st = smem_u32(smem + stage * L::kStageBytes);
-            const uint32_t a_hi = st, a_lo = st + L::kABytes, b_pair = st + 2 * L::kABytes;     // [B_hi ; B_lo], or [B_lo ; B_hi] in layout 2
-            const uint32_t b_hi = b_pair + (p.acc_layout == 2 ? L::kBBytes : 0);
-            const uint32_t d_narrow = d_tmem + (p.acc_layout == 1 ? BN : 0);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const uint64_t ah = umma_desc(a_hi + k * a_kstep, a_lbo, a_sbo, a_lt), al = umma_desc(a_lo + k * a_kstep, a_lbo, a_sbo, a_lt);
-              const uint64_t bw = umma_desc(b_pair + k * b_kstep, b_lbo, b_sbo, b_lt);    // N = 2*BN runs on into the second B tile
-              const uint64_t bh = umma_desc(b_hi + k * b_kstep, b_lbo, b_sbo, b_lt);
-              umma<AR>(d_tmem, ah, bw, idesc_wide, (it > it0 || k > 0) ? 1u : 0u);
-              umma<AR>(d_narrow, al, bh, idesc_narrow, 1u);
+      // Only the low word of a descriptor changes: its address field (16-byte units, no carry out of it below 256 KB)
+      const uint64_t a_desc = umma_desc(smem_u32(smem), a_lbo, a_sbo, a_lt), b_desc = umma_desc(smem_u32(b_smem), b_lbo, b_sbo, b_lt);
+      const uint32_t a_word = (uint32_t)a_desc, a_high = (uint32_t)(a_desc >> 32), b_word = (uint32_t)b_desc, b_high = (uint32_t)(b_desc >> 32);
+      const uint32_t a_step = a_kstep >> 4, b_step = b_kstep >> 4, a_slot16 = (uint32_t)a_slot_bytes >> 4, a_half16 = (uint32_t)a_half >> 4;
+      constexpr uint32_t kBSlot16 = kBSlot >> 4, kBTile16 = kBTile >> 4;
+      const bool conv = p.mode == kModeConv, one_ring = p.one_ring, resident = p.b_resident;
+      const int period = conv ? p.ntaps : 1, group_iters = p.group_iters, a_slots = p.a_slots, b_slots = p.b_slots, cross_groups = p.cross_groups;
+      const TapTable words(conv ? p.ntaps : 0, lane, [&](int t) { return p.tap_word[t]; });
+      auto issue = [&](auto role_of) {
+        constexpr int kRole = decltype(role_of)::value;     // 1: the wide instructions, 2: the narrow ones, 3: both
+        int as = 0, bs = 0;
+        uint32_t aph = 0, bph = 0;
+        int group = 0;            // accumulator groups issued so far (alternating TMEM buffers)
+        int epoch = 0;            // kAccThree: times the cross terms started afresh
+        int bad = 0;
+        bool ready = false;       // the next stage's operands were seen to have arrived
+        uint32_t word = 0x300u;
+        WorkIter iter(p);
+        WorkItem w;
+        while (iter.next(p, w)) {
+          int ti = 0;
+          if (conv) { ti = w.k0 % period; word = words.at(ti); }
+          if (resident) { bs = 0; bph = 0; }           // the slots were filled once: their first phase stays complete
+          bool first = true;
+          int in_epoch = 0;                            // groups since the cross terms started afresh
+          for (int it0 = 0; it0 < w.kcount; it0 += group_iters, ++group) {
+            const int acc = group & 1;
+            mbar_wait_mark(&acc_empty[acc], ((group >> 1) & 1) ^ 1, abort_flag, bad);
+            if (three && in_epoch == 0) {
+              mbar_wait_mark(cross_empty, (epoch & 1) ^ 1, abort_flag, bad);
+              ++epoch;
             }
-            tcgen05_commit(&empty[stage]);       // frees the stage once the MMAs above have read it
-            if (++stage == L::kStages) { stage = 0; phase ^= 1; }
+            const uint32_t d_wide = tmem_base + acc * (three ? BN : kSetCols);
+            const uint32_t d_narrow = three ? tmem_base + 3 * BN : d_wide + (kSets3 ? 2 * BN : 0);
+            const bool hi_first = three && acc == 0;
+            const uint32_t hi_at = hi_first ? 0u : kBTile16, lo_at = kBTile16 - hi_at;
+            const int it1 = min(it0 + group_iters, w.kcount);
+            for (int it = it0; it < it1; ++it) {
+              if (first && !one_ring) mbar_wait_mark(&a_full[as], aph, abort_flag, bad);
+              if (!ready) mbar_wait_mark(&b_full[bs], bph, abort_flag, bad);
+              tcgen05_fence_after();
+              const bool last = (word & 0x200u) != 0 || it == w.kcount - 1;
+              const uint32_t ah = a_word + as * a_slot16 + (word & 0xffu) * 8u, al = ah + a_half16;
+              const uint32_t bw = b_word + bs * kBSlot16, bh = bw + hi_at;                  // bw: N = 2*BN runs on into the second B tile
+              const uint32_t keep_main = it > it0 ? 1u : 0u, keep_cross = three ? (it > it0 || in_epoch > 0 ? 1u : 0u) : keep_main;
+              uint64_t* const b_done = &b_empty[bs];
+              uint64_t* const a_done = &a_empty[as];
+              if (++bs == b_slots) { bs = 0; if (!resident) bph ^= 1; }
+              if (last && ++as == a_slots) { as = 0; aph ^= 1; }
+              ready = mbar_test(&b_full[bs], bph);
+              if (conv) { if (++ti == period) ti = 0; word = words.at(ti); }
+              first = (word & 0x100u) != 0;
+              if (elect_one() && !bad) {
+                if (kRole & 1) {
+                  if (three && !keep_main && keep_cross) {      // main starts afresh, the cross terms go on
+                    umma_at<AR>(hi_first ? d_wide : d_wide + BN, ah, a_high, bh, b_high, idesc_narrow, 0u);
+                    umma_at<AR>(hi_first ? d_wide + BN : d_wide, ah, a_high, bw + lo_at, b_high, idesc_narrow, 1u);
+                  } else {
+                    umma_at<AR>(d_wide, ah, a_high, bw, b_high, idesc_wide, keep_main);
+                  }
+                }
+                if (kRole & 2) umma_at<AR>(d_narrow, al, a_high, bh, b_high, idesc_narrow, three || kSets3 ? keep_cross : 1u);
+#pragma unroll
+                for (int q = 1; q < 4; ++q) {
+                  if (kRole & 1) umma_at<AR>(d_wide, ah + q * a_step, a_high, bw + q * b_step, b_high, idesc_wide, 1u);
+                  if (kRole & 2) umma_at<AR>(d_narrow, al + q * a_step, a_high, bh + q * b_step, b_high, idesc_narrow, 1u);
+                }
+                // the commits free the slots once the MMAs above have read them
+                if (!resident) tcgen05_commit(b_done);
+                if (last && !one_ring) tcgen05_commit(a_done);
+                if (it == it1 - 1) tcgen05_commit(&acc_full[acc]);
+              }
+            }
+            if (++in_epoch == cross_groups) in_epoch = 0;
           }
-          if (ok) tcgen05_commit(&acc_full[acc]);
         }
-      }
+      };
+      if (issuers == 1) { if (warp == 1) issue(std::integral_constant<int, 3>()); }
+      else if (warp == 1) issue(std::integral_constant<int, 1>());
+      else issue(std::integral_constant<int, 2>());
     }
   } else {
     // ===================== epilogue: warps 2..9 =====================
     // A warp may only read the TMEM lane quarter (warp % 4); two warps share each quarter and take one half of
-    // the tile's columns each, so that every scheduler has two epilogue warps to alternate between (the
-    // epilogue is a chain of dependent address/convert/store instructions and is issue-latency bound).
+    // the tile's columns each, so that every scheduler has two epilogue warps to alternate between.
+    grid_dep_sync();
     const int quarter = warp & 3;
     const int half = (warp - 2) >> 2;
     constexpr int HC = BN / 2;                  // columns per epilogue warp
+    constexpr int NC = HC % 32 == 0 ? 32 : 16;  // columns per TMEM load
     const int row_in_tile = quarter * 32 + lane;
     const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));     // powers of two: exact
+    const float2 scale2 = make_float2(inv_scale, inv_scale);
     int group = 0;
     bool ok = true;
     WorkIter iter(p);
@@ -676,8 +838,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_kernel(const __grid_consta
       const int n0 = nt * BN + half * HC;
       const RowAddr ra = row_address(p, mt, tap, row_in_tile);
       const bool row_ok = ra.ok;
-      const uint32_t col_stride = ra.col_stride;
-      float* const row_out = p.out + ra.base + (long long)n0 * col_stride;
+      const uint32_t col_bytes = ra.col_stride * 4u;
+      char* const row_out = reinterpret_cast<char*>(p.out + ra.base + (long long)n0 * ra.col_stride);
       const int ncols = max(0, min(HC, p.N - n0));
       const bool vec_ok = p.epi == kEpiRowMajor && ((ra.base + n0) & 3) == 0;
 
@@ -685,48 +847,43 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_kernel(const __grid_consta
         int got = lane == 0 ? (int)mbar_wait(&acc_full[acc_buf], (grp >> 1) & 1, abort_flag) : 1;
         return __shfl_sync(0xffffffffu, got, 0) != 0;
       };
-      // NC values of this thread's row, columns c0.. of the warp's half; the offsets are independent of one
-      // another (no serial pointer chain) and fit 32 bits (BN * plane size is far below 2^32 elements).
-      auto store_cols = [&](const float* v, int c0, auto nc_tag) {
-        constexpr int NC = decltype(nc_tag)::value;
+      // NC values of this thread's row at columns c0.. of the warp's half: base + constant * stride, one wide multiply-add each
+      auto store_cols = [&](const float2* v2, int c0) {
+        const float* v = reinterpret_cast<const float*>(v2);
         if (!row_ok || c0 >= ncols) return;
+        char* dst = row_out + (uint64_t)col_bytes * (uint32_t)c0;
         if (vec_ok && c0 + NC <= ncols) {
-          float4* dst = reinterpret_cast<float4*>(row_out + c0);
 #pragma unroll
-          for (int q = 0; q < NC / 4; ++q) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+          for (int q = 0; q < NC / 4; ++q) reinterpret_cast<float4*>(dst)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
         } else if (c0 + NC <= ncols) {
-          float* dst = row_out + (size_t)((uint32_t)c0 * col_stride);
 #pragma unroll
-          for (int q = 0; q < NC; ++q) dst[(size_t)((uint32_t)q * col_stride)] = v[q];
+          for (int q = 0; q < NC; ++q) *reinterpret_cast<float*>(dst + (uint64_t)col_bytes * (uint32_t)q) = v[q];
         } else {
-          float* dst = row_out + (size_t)((uint32_t)c0 * col_stride);
 #pragma unroll
           for (int q = 0; q < NC; ++q)
-            if (c0 + q < ncols) dst[(size_t)((uint32_t)q * col_stride)] = v[q];
+            if (c0 + q < ncols) *reinterpret_cast<float*>(dst + (uint64_t)col_bytes * (uint32_t)q) = v[q];
         }
       };
+      const uint32_t t_lane = tmem_base + half * HC + ((uint32_t)(quarter * 32) << 16);
 
-      if (w.slot < 0 && kcount <= p.group_iters) {
-        // One accumulator group: stream TMEM straight to memory, 32 columns at a time.
+      if (w.slot < 0 && kcount <= p.group_iters && p.cluster <= 1 && !three) {
+        // One accumulator group: stream TMEM straight to memory.
         const int acc = group & 1;
         if (!wait_group(acc, group)) { ok = false; break; }
         ++group;
         tcgen05_fence_after();
-        const uint32_t t_base = tmem_base + acc * 2 * BN + half * HC + ((uint32_t)(quarter * 32) << 16);
 #pragma unroll 1
-        for (int c0 = 0; c0 < HC; c0 += 32) {
-          float v1[32], v2[32];
-          tmem_ld32(t_base + c0, v1);
-          tmem_ld32(t_base + BN + c0, v2);
-          tmem_ld_wait();
-          if (c0 + 32 >= HC) {     // last chunk read: the accumulator can be reused while we store
+        for (int c0 = 0; c0 < HC; c0 += NC) {
+          float2 v[NC / 2];
+          load_sum<NC, kSets3 ? 3 : 2>(t_lane + acc * kSetCols + c0, BN, v);
+          if (c0 + NC >= HC) {     // last chunk read: the accumulator can be reused while we store
             tcgen05_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&acc_empty[acc]);
           }
 #pragma unroll
-          for (int q = 0; q < 32; ++q) v1[q] = (v1[q] + v2[q]) * inv_scale;
-          store_cols(v1, c0, std::integral_constant<int, 32>{});
+          for (int q = 0; q < NC / 2; ++q) v[q] = __fmul2_rn(v[q], scale2);
+          store_cols(v, c0);
         }
         continue;
       }
@@ -734,39 +891,108 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_kernel(const __grid_consta
       // The tensor core accumulates with truncation, so a long chain of MMAs into one TMEM accumulator
       // drifts; each group of group_iters stages is therefore accumulated in TMEM on its own and promoted
       // here into fp32 registers with round-to-nearest adds.
-      float accv[HC];
+      float2 accv[HC / 2];
 #pragma unroll
-      for (int q = 0; q < HC; ++q) accv[q] = 0.f;
+      for (int q = 0; q < HC / 2; ++q) accv[q] = make_float2(0.f, 0.f);
+      int in_epoch = 0;
       for (int it0 = 0; it0 < kcount && ok; it0 += p.group_iters, ++group) {
         const int acc = group & 1;
         if (!wait_group(acc, group)) { ok = false; break; }
         tcgen05_fence_after();
-        const uint32_t t_base = tmem_base + acc * 2 * BN + half * HC + ((uint32_t)(quarter * 32) << 16);
+        if (three) {
 #pragma unroll
-        for (int c0 = 0; c0 < HC; c0 += 16) {
-          float v1[16], v2[16];
-          tmem_ld16(t_base + c0, v1);              // the two accumulator blocks (which terms sit where: acc_layout)
-          tmem_ld16(t_base + BN + c0, v2);
-          tmem_ld_wait();
+          for (int c0 = 0; c0 < HC; c0 += NC) {
+            float2 v[NC / 2];
+            load_sum<NC, 1>(t_lane + acc * 2 * BN + c0, 0, v);
 #pragma unroll
-          for (int q = 0; q < 16; ++q) accv[c0 + q] += v1[q] + v2[q];
+            for (int q = 0; q < NC / 2; ++q) accv[c0 / 2 + q] = __fadd2_rn(accv[c0 / 2 + q], v[q]);
+          }
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[acc]);
+          if (++in_epoch < p.cross_groups && it0 + p.group_iters < kcount) continue;
+          in_epoch = 0;
+#pragma unroll
+          for (int c0 = 0; c0 < HC; c0 += NC) {
+            float2 v[NC / 2];
+            load_sum<NC, 2>(t_lane + BN + c0, 2 * BN, v);
+#pragma unroll
+            for (int q = 0; q < NC / 2; ++q) accv[c0 / 2 + q] = __fadd2_rn(accv[c0 / 2 + q], v[q]);
+          }
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(cross_empty);
+        } else {
+#pragma unroll
+          for (int c0 = 0; c0 < HC; c0 += NC) {
+            float2 v[NC / 2];
+            load_sum<NC, kSets3 ? 3 : 2>(t_lane + acc * kSetCols + c0, BN, v);
+#pragma unroll
+            for (int q = 0; q < NC / 2; ++q) accv[c0 / 2 + q] = __fadd2_rn(accv[c0 / 2 + q], v[q]);
+          }
+          tcgen05_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&acc_empty[acc]);
         }
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&acc_empty[acc]);
       }
       if (!ok) break;
-      if (w.slot >= 0) {
-        // a piece of a split tile: raw partial sums to the workspace, [column][row] so that a warp's 32 rows coalesce
-        float* ws = p.workspace + ((size_t)w.slot * BN + half * HC) * BM + row_in_tile;
+      if (w.slot >= 0 || p.cluster > 1) {
+        // a piece of a tile: raw partial sums, [column][row] so that a warp's 32 rows coalesce - to the workspace (split tail), or
+        // to this CTA's own shared memory, whose operands have all been read by now (cluster)
+        float* ws = (p.cluster > 1 ? reinterpret_cast<float*>(smem) : p.workspace + (size_t)w.slot * BN * BM) + half * HC * BM + row_in_tile;
 #pragma unroll
-        for (int q = 0; q < HC; ++q) ws[(size_t)q * BM] = accv[q];
+        for (int q = 0; q < HC / 2; ++q) { ws[(size_t)(2 * q) * BM] = accv[q].x; ws[(size_t)(2 * q + 1) * BM] = accv[q].y; }
         continue;
       }
 #pragma unroll
-      for (int q = 0; q < HC; ++q) accv[q] *= inv_scale;
-      store_cols(accv, 0, std::integral_constant<int, HC>{});
+      for (int c0 = 0; c0 < HC; c0 += NC) {
+#pragma unroll
+        for (int q = 0; q < NC / 2; ++q) accv[c0 / 2 + q] = __fmul2_rn(accv[c0 / 2 + q], scale2);
+        store_cols(accv + c0 / 2, c0);
+      }
     }
+  }
+
+  if (p.cluster > 1) {
+    // Every CTA of the cluster adds up its share of the tile's columns, in rank order (bit-reproducible).  kUnroll columns of all
+    // pieces are in flight at once.  The traffic between the SMs bounds it (some 15 cycles per 128-byte load: 8000 cycles for 6
+    // pieces of 128 x 96); bulk copies between the CTAs took as long.
+    constexpr int kUnroll = 4, kLanes = kGemmThreads / BM;
+    const int rank = blockIdx.x % p.cluster, tile = blockIdx.x / p.cluster;
+    int mt, nt, tap;
+    decode_tile(p, tile, mt, nt, tap);
+    const int row = threadIdx.x & (BM - 1);
+    const RowAddr ra = row_address(p, mt, tap, row);
+    const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));
+    const int c1 = min(BN * (rank + 1) / p.cluster, p.N - nt * BN);
+    __syncwarp();
+    cluster_sync_all();
+    if (!*abort_flag) {
+      for (int c0 = BN * rank / p.cluster + (int)threadIdx.x / BM; c0 < c1; c0 += kUnroll * kLanes) {
+        float sum[kUnroll] = {0.f, 0.f, 0.f, 0.f};
+        float v[kMaxCluster][kUnroll];
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r)
+          if (r < p.cluster) {
+            const uint32_t piece = smem_of_cta(smem_u32(smem), r) + row * 4u;
+#pragma unroll
+            for (int j = 0; j < kUnroll; ++j) v[r][j] = ld_cluster(piece + (uint32_t)min(c0 + j * kLanes, c1 - 1) * (BM * 4u));
+          }
+#pragma unroll
+        for (int r = 0; r < kMaxCluster; ++r)
+          if (r < p.cluster) {
+#pragma unroll
+            for (int j = 0; j < kUnroll; ++j) sum[j] += v[r][j];
+          }
+#pragma unroll
+        for (int j = 0; j < kUnroll; ++j) {
+          const int c = c0 + j * kLanes;
+          if (ra.ok && c < c1) p.out[ra.base + (long long)(nt * BN + c) * ra.col_stride] = sum[j] * inv_scale;
+        }
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();        // nobody leaves while its shared memory is still read
   }
 
   // ===================== teardown =====================
@@ -862,7 +1088,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_pair_kernel(const __grid_c
           int a_col, a_row, b_col;
           if (p.mode == kModeConv) {
             const int t = it / p.chunks_per_tap, ch = it - t * p.chunks_per_tap;
-            a_col = p.tap_col[t] + ch * BK; a_row = m0 + p.tap_off[t];
+            a_col = p.tap_col[t] + ch * BK; a_row = m0 + p.tap_off[t] + p.pair_shift[t];
             b_col = p.tap_b[t] * p.b_tap_pitch + ch * BK;
           } else {
             a_col = it * BK; a_row = m0; b_col = it * BK;
@@ -1419,39 +1645,6 @@ static int make_map_mn(CUtensorMap* m, int ar, const void* base, long long rows,
   return 0;
 }
 
-// im2col-mode map over a halo-free pixel-major pack [N][H][W][pitch]: base pixels range over the box
-// [-lo_w, W - lo_w' ) x [-lo_h, ...) that holds one base pixel per output position of a stride-1 window of
-// win_w x win_h with lo_w / lo_h zero columns / rows in front (and as many behind as the output extent needs);
-// a copy brings `pixels` base pixels x `chans` channels (128 bytes).
-typedef CUresult (*EncodeIm2colFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*, const int*, const int*,
-                                   cuuint32_t, cuuint32_t, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                   CUtensorMapFloatOOBfill);
-static EncodeIm2colFn encode_im2col_fn() {
-  static EncodeIm2colFn fn = [] {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeIm2col", &p, cudaEnableDefault, &q) != cudaSuccess || q != cudaDriverEntryPointSuccess) p = nullptr;
-    return (EncodeIm2colFn)p;
-  }();
-  return fn;
-}
-static int make_map_im2col(CUtensorMap* m, int ar, const void* base, int N, int H, int W, long long pitch, int lo_w, int lo_h, int win_w, int win_h,
-                           int pixels, int chans) {
-  EncodeIm2colFn fn = encode_im2col_fn();
-  TF_REQUIRE(fn, "cuTensorMapEncodeIm2col is not available from this driver");
-  const int es = elem_of(ar);
-  cuuint64_t dims[4] = {(cuuint64_t)pitch, (cuuint64_t)W, (cuuint64_t)H, (cuuint64_t)N};
-  cuuint64_t strides[3] = {(cuuint64_t)pitch * es, (cuuint64_t)W * pitch * es, (cuuint64_t)H * W * pitch * es};
-  int lower[2] = {-lo_w, -lo_h};
-  int upper[2] = {lo_w - (win_w - 1), lo_h - (win_h - 1)};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  CUresult r = fn(m, map_type(ar), 4, (void*)base, dims, strides, lower, upper, (cuuint32_t)chans, (cuuint32_t)pixels, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  TF_REQUIRE(r == CUDA_SUCCESS, "cuTensorMapEncodeIm2col failed with %d (N %d H %d W %d pitch %lld lower %d,%d upper %d,%d)", (int)r, N, H, W, pitch, lower[0],
-             lower[1], upper[0], upper[1]);
-  return 0;
-}
-
 static std::mutex g_tc_mu;      // guards the lazily created process-wide state below
 static int* error_word() {      // mapped pinned word: the kernels raise it, the host polls it for free
   static int* host = nullptr;
@@ -1497,44 +1690,93 @@ void set_tensor_arithmetic(int a) { if (g_arith.exchange(a, std::memory_order_re
 // unbalanced and its reductions are long enough to share.
 static float g_tail_gain = [] { const char* e = getenv("TINYFLOW_TAIL_GAIN"); return e ? (float)atof(e) : 0.9f; }();
 static float g_tail_cost = [] { const char* e = getenv("TINYFLOW_TAIL_COST"); return e ? (float)atof(e) : 12.f; }();     // workspace round trip + second kernel, in stages
-static int plan_schedule(GemmParams& g, int bn, cudaStream_t s, int* oom) {
+// A reduction over few tiles is cut over clusters of 2-8 CTAs instead (sum in shared memory, no workspace and no second
+// kernel); `max_clusters(c)` says how many clusters of c the device runs at once.  The sum costs about 6 stages whatever
+// the cluster (768 -> 192 channels, 17 x 17, 1x1, batch 2: 17.0 -> 15.3 us in clusters of 6).  Against it the workspace costs
+// 4 stages and 0.15 per tile (its traffic): 70 tiles of 36 stages 34.0 us split and 29.7 in clusters of 2, 40 of 72
+// stages 33.8 and 32.5 in clusters of 3, but 12 of 72 stages 19.2 and 23 in clusters of 8.
+template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, int* oom, MaxClusters max_clusters) {
   const int sms = device_sm_count();
   const int tiles = g.m_tiles * g.n_tiles * g.tap_tiles;
-  g.full_tiles = tiles; g.tail_tiles = 0; g.tail_share = 0; g.slots_per_cta = 0; g.workspace = nullptr;
+  g.full_tiles = tiles; g.tail_tiles = 0; g.tail_share = 0; g.slots_per_cta = 0; g.workspace = nullptr; g.cluster = 1;
   const int rem = tiles % sms;
   static const bool no_split = getenv("TINYFLOW_NO_TAIL_SPLIT") != nullptr;
-  if (rem == 0 || g.k_total < 8 || no_split) return 0;
+  if (rem == 0 || no_split) return 0;
+  const double whole = g.k_total + 8.0;
+  const double limit = g_tail_gain * whole;
+  double best = limit;
+  if (tiles < sms) {
+    for (int c = 2; c <= kMaxCluster && c <= g.k_total && tiles * c <= sms; ++c) {
+      const double cost = (g.k_total + c - 1) / c + 8.0 + 6.0;
+      if (cost < best && tiles <= max_clusters(c)) { best = cost; g.cluster = c; }
+    }
+  }
+  if (g.k_total < 8) return 0;
   const long long units = (long long)rem * g.k_total;
   int share = (int)((units + sms - 1) / sms);
   if (share < 4) share = 4;                                   // shorter pieces are all overhead
-  const double whole = g.k_total + 8.0, split = share + 8.0 + g_tail_cost;
-  if (split >= g_tail_gain * whole) return 0;
+  if (share + 8.0 + g_tail_cost >= limit || (g.cluster > 1 && share + 8.0 + 4.0 + 0.15 * rem >= best)) return 0;
+  g.cluster = 1;
   g.full_tiles = tiles - rem; g.tail_tiles = rem; g.tail_share = share;
   g.slots_per_cta = (share - 1 + g.k_total - 1) / g.k_total + 1;       // tiles a range of `share` stages can touch
   const int ctas = (int)((units + share - 1) / share);
   const size_t bytes = (size_t)ctas * g.slots_per_cta * bn * BM * sizeof(float);
   g.workspace = (float*)persistent_scratch(1, bytes);
   if (!g.workspace) { if (oom) *oom = bytes > 0x7fffffffu ? 0x7fffffff : (int)bytes; return 1; }
-  (void)s;
   return 0;
 }
-
-static bool g_attr_done[2][3] = {{false, false, false}, {false, false, false}};
-template <int BN, int AR> static int launch_gemm(const GemmParams& p, cudaStream_t s, double flops, const char* what) {
-  using L = SmemLayout<BN>;
-  constexpr int slot = BN == 64 ? 0 : (BN == 128 ? 1 : 2);
-  {
-    std::lock_guard<std::mutex> lk(g_tc_mu);
-    if (!g_attr_done[AR][slot]) {
-      TF_CUDA(cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotal));
-      g_attr_done[AR][slot] = true;
-    }
+// How shared memory is dealt to the two rings, and whether the B tile of a CTA stays there: with all of a CTA's tiles in one
+// column of the grid (its size a multiple of n_tiles) and room for every stage of B beside two A blocks.
+static int plan_smem(GemmParams& g, int bn, int grid) {
+  const int limit = kSmemLimit - kSmemBarriers, a = g.a_rows * 256, b = bn * 256;
+  const int tiles = g.full_tiles + g.tail_tiles;
+  g.b_resident = g.one_ring = 0;
+  if (g.acc_mode == kAccPair && g.mode != kModeWgrad && g.tail_share == 0 && g.cluster == 1 && tiles > grid && g.n_tiles <= 4 && g.k_total <= kMaxBSlots && g.k_total * b + 2 * a <= limit) {
+    g.b_resident = 1;
+    g.b_slots = g.k_total;
+    g.a_slots = std::min(kMaxASlots, (limit - g.k_total * b) / a);
+    return grid / g.n_tiles * g.n_tiles;
   }
+  if (g.a_rows > BM) {
+    g.a_slots = 2;
+    g.b_slots = std::min(kMaxBSlots, (limit - 2 * a) / b);
+  } else {
+    g.a_slots = g.b_slots = std::min(kMaxASlots, limit / (a + b));
+    g.one_ring = 1;
+  }
+  return grid;
+}
+
+template <int BN, int AR> static int max_clusters_of(int c) {
+  static std::atomic<int> known[9];
+  int n = known[c].load(std::memory_order_relaxed);
+  if (n == 0) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(c); cfg.blockDim = dim3(kGemmThreads); cfg.dynamicSmemBytes = kSmemLimit + 1024;
+    cudaLaunchAttribute attr;
+    memset(&attr, 0, sizeof(attr));
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = c; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, gemm3x_kernel<BN, AR>, &cfg) != cudaSuccess || n <= 0) { cudaGetLastError(); n = -1; }
+    known[c].store(n, std::memory_order_relaxed);
+  }
+  return n;
+}
+template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, double flops, const char* what, int* oom) {
+  static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  TF_CUDA(attr);
   TF_REQUIRE(tensor_path_error() == 0, "%s: an earlier tensor-core kernel timed out on a barrier; refusing to launch", what);
+  if (int rc = plan_schedule(p, BN, oom, max_clusters_of<BN, AR>)) return rc;
   static const int group_iters = getenv("TINYFLOW_GROUP_ITERS") ? atoi(getenv("TINYFLOW_GROUP_ITERS")) : 0;
-  const_cast<GemmParams&>(p).group_iters = group_iters > 0 ? group_iters : (p.data_by_data ? kGroupItersDataByData : (AR == kArithTF32 ? kGroupItersTF32 : kGroupIters));
-  static const int acc_layout = getenv("TINYFLOW_ACC_LAYOUT") ? atoi(getenv("TINYFLOW_ACC_LAYOUT")) : 2;
-  const_cast<GemmParams&>(p).acc_layout = acc_layout;
+  p.group_iters = group_iters > 0 ? group_iters : (p.data_by_data ? kGroupItersDataByData : (AR == kArithTF32 ? kGroupItersTF32 : kGroupIters));
+  // cross terms promoted every 64 stages: 256 accumulations into a sum 2^-12 of the whole truncate less than 2^-28 of it
+  p.cross_groups = 64 / p.group_iters;
+    // Two issuers gain from 8 stages per CTA on (equal at 18 of 128 columns, 1 us of 65 at 36); at 96 columns the narrow MMAs
+  // are short enough for one warp (12 stages: 19.2 against 21.2 us).
+  const int longest = p.tail_share > 0 && p.full_tiles == 0 ? p.tail_share : p.k_total / p.cluster;
+  p.acc_mode = BN != 64 && p.k_total > p.group_iters && longest >= (BN == 128 ? 8 : 24) && p.group_iters > 1 ? kAccThree : kAccPair;
   const int sms = device_sm_count();
   const int tiles = p.full_tiles + p.tail_tiles;
   int grid = tiles < sms ? tiles : sms;
@@ -1542,13 +1784,31 @@ template <int BN, int AR> static int launch_gemm(const GemmParams& p, cudaStream
     const int ctas = (int)(((long long)p.tail_tiles * p.k_total + p.tail_share - 1) / p.tail_share);
     grid = p.full_tiles > 0 ? sms : ctas;
   }
+  if (p.cluster > 1) grid = tiles * p.cluster;
+  grid = plan_smem(p, BN, grid);
+  TF_REQUIRE(p.cluster == 1 || BM * BN * 4 <= p.a_slots * p.a_rows * 256 + p.b_slots * BN * 256, "%s: a piece of a tile does not fit where its operands were", what);
   note_compute_stream(s);
   static const bool detail = getenv("TINYFLOW_TIMING_DETAIL") != nullptr;    // one timing row per distinct problem shape
   char name[192];
-  if (detail) snprintf(name, sizeof(name), "gemm3x%s mode%d M%d N%d ktotal%d taps%d bn%d tiles%d tail%d share%d %s", AR == kArithTF32 ? "tf32" : "f16", p.mode, p.M,
-                       p.N, p.k_total, p.tap_tiles, BN, tiles, p.tail_tiles, p.tail_share, what + 5);
+  if (detail) snprintf(name, sizeof(name), "gemm3x%s mode%d M%d N%d ktotal%d taps%d bn%d tiles%d tail%d share%d cl%d a%dx%d b%d%s %s", AR == kArithTF32 ? "tf32" : "f16", p.mode, p.M,
+                       p.N, p.k_total, p.tap_tiles, BN, tiles, p.tail_tiles, p.tail_share, p.cluster, p.a_slots, p.a_rows, p.b_slots, p.b_resident ? "r" : "", what + 5);
   KernelTimer kt(detail ? name : (AR == kArithTF32 ? "gemm3xtf32_tcgen05" : "gemm3xf16_tcgen05"), s, flops, 0, 1);
-  launch_dep(gemm3x_kernel<BN, AR>, dim3(grid), dim3(kThreads), (size_t)L::kTotal, s, p);
+  if (p.cluster > 1) {
+    static const bool no_dep = getenv("TINYFLOW_NO_DEPENDENT_LAUNCH") != nullptr;
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kGemmThreads); cfg.dynamicSmemBytes = (size_t)gemm_smem_bytes(p, BN); cfg.stream = s;
+    cudaLaunchAttribute attrs[2];
+    memset(attrs, 0, sizeof(attrs));
+    attrs[0].id = cudaLaunchAttributeClusterDimension;
+    attrs[0].val.clusterDim.x = p.cluster; attrs[0].val.clusterDim.y = 1; attrs[0].val.clusterDim.z = 1;
+    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attrs; cfg.numAttrs = (no_dep || s == (cudaStream_t)0) ? 1 : 2;
+    TF_CUDA(cudaLaunchKernelEx(&cfg, gemm3x_kernel<BN, AR>, p));
+  } else {
+    TF_CUDA(launch_dep(gemm3x_kernel<BN, AR>, dim3(grid), dim3(kGemmThreads), (size_t)gemm_smem_bytes(p, BN), s, p));
+  }
   TF_AFTER(s, what);
   if (p.tail_share > 0) {
     launch_dep(reduce_partials_kernel<BN>, dim3(p.tail_tiles, BN / kReduceCols), dim3(BM, kReduceWays), 0, s, p);
@@ -1600,14 +1860,14 @@ static bool pairs_wanted(int bn, int m_tiles, int n_tiles, int k_total) {
   if (g_pairs_mode >= 2) return true;                   // 2: wherever the kernel can run (tests)
   return k_total >= 8 && ((m_tiles + 1) / 2) * n_tiles >= 60;
 }
-template <int AR> static int launch_gemm_ar(int bn, const GemmParams& p, cudaStream_t s, double flops, const char* what) {
-  return bn == 64 ? launch_gemm<64, AR>(p, s, flops, what) : bn == 96 ? launch_gemm<96, AR>(p, s, flops, what) : launch_gemm<128, AR>(p, s, flops, what);
+template <int AR> static int launch_gemm_ar(int bn, GemmParams& p, cudaStream_t s, double flops, const char* what, int* oom) {
+  return bn == 64 ? launch_gemm<64, AR>(p, s, flops, what, oom) : bn == 96 ? launch_gemm<96, AR>(p, s, flops, what, oom) : launch_gemm<128, AR>(p, s, flops, what, oom);
 }
 // Plans the schedule (which may need workspace) and launches.  Returns 0 on success, -1 on error, 1 when the workspace
 // could not be allocated (*oom holds the byte count).
 static int launch_gemm_bn(int bn, int ar, GemmParams& p, cudaStream_t s, double flops, const char* what, int* oom) {
-  if (int rc = plan_schedule(p, bn, s, oom)) return rc;
-  return ar == kArithTF32 ? launch_gemm_ar<kArithTF32>(bn, p, s, flops, what) : launch_gemm_ar<kArithF16>(bn, p, s, flops, what);
+  if (p.a_rows == 0) p.a_rows = BM;
+  return ar == kArithTF32 ? launch_gemm_ar<kArithTF32>(bn, p, s, flops, what, oom) : launch_gemm_ar<kArithF16>(bn, p, s, flops, what, oom);
 }
 // N-tile width.  M/N-major B operands come in 64-column groups, so they take 64 or 128; K-major ones may also take
 // 96, which wastes less on widths such as 96, 160, 192 or 288.
@@ -1910,17 +2170,6 @@ static int pack_dy(ConvTc* st, int ar, const ConvPlan* p, const float* dy, cudaS
   pk.src = dy; pk.version = ver; pk.tag = 2;
   return 0;
 }
-// Halo-free pixel-major packs [N][H][W][C] of x and [N][P][Q][K] of dy for the im2col route (tags 20 / 21)
-static int pack_plain(Pack& pk, int ar, int tag, const float* src, int N, int chans, int H, int W, cudaStream_t s, int* oom) {
-  const uint64_t ver = version_of(src);
-  const long long rows = (long long)N * H * W;
-  if (pack_valid(pk, ar, src, ver, tag, rows, chans)) return 0;
-  if (pack_alloc(pk, ar, rows, chans, s, oom)) return 1;
-  ScaleRef sr = begin_pack(pk, src, rows * chans, s);
-  if (launch_pack_nchw(pk, sr, src, N, chans, H, W, H, W, 0, 0, 1, 1, 0, (int)pk.pitch, s)) return -1;
-  pk.src = src; pk.version = ver; pk.tag = tag;
-  return 0;
-}
 // Filter packs are keyed like the activation packs (pointer, write version): an optimiser step bumps the version.
 // `with_other` makes the forward call produce the backward-data pack in the same launch.
 static int pack_filter(ConvTc* st, int ar, const float* w, const ConvPlan* p, int flip, bool with_other, cudaStream_t s, int* oom) {
@@ -1965,37 +2214,62 @@ static int pack_filter(ConvTc* st, int ar, const float* w, const ConvPlan* p, in
 struct TapList { int n = 0; int off[kMaxTaps]; int col[kMaxTaps]; int b[kMaxTaps]; void add(int o, int c, int bb) { off[n] = o; col[n] = c; b[n] = bb; ++n; } };
 struct OutGeom { int valid_h, valid_w, out_h, out_w, out_sh, out_sw, out_off_h, out_off_w; };
 // returns 0 on success, -1 on error, 1 when scratch memory was short (*oom set)
-// Geometry of an im2col read of the activation pack: the pack is [N][H][W][pitch]; a stride-1 window of win_w x win_h
-// with lo_w / lo_h zero columns / rows in front gives box_w x box_h base pixels (= output positions) per image.
-struct Im2colGeom { int N, H, W, lo_w, lo_h, win_w, win_h, box_w, box_h; };
+// Orders the taps into runs that share one block of activation rows: same columns, shifts at most `span` apart.  The
+// span (up to 64 rows, a block of 192) is the one that fetches the fewest bytes per stage: runs of whole windows on narrow
+// images, of window rows on wide ones.
+static void plan_runs(GemmParams& g, const TapList& taps, int bn) {
+  int order[kMaxTaps];
+  for (int t = 0; t < taps.n; ++t) order[t] = t;
+  std::sort(order, order + taps.n, [&](int a, int b) { return taps.col[a] != taps.col[b] ? taps.col[a] < taps.col[b] : taps.off[a] < taps.off[b]; });
+  auto group = [&](int span, GemmParams* out) -> double {            // bytes of A and B per stage
+    int runs = 0, widest = 0, t0 = 0;
+    for (int i = 0; i < taps.n; ++i) {
+      const int t = order[i], f = order[t0];
+      const bool fresh = i == 0 || taps.col[t] != taps.col[f] || taps.off[t] - taps.off[f] > span;
+      if (fresh) { t0 = i; ++runs; }
+      const int shift = taps.off[t] - taps.off[order[t0]];
+      widest = std::max(widest, shift);
+      if (out) {
+        if (fresh && i) out->tap_word[i - 1] |= 0x200u;
+        out->tap_word[i] = (uint32_t)shift | (fresh ? 0x100u : 0u) | (i == taps.n - 1 ? 0x200u : 0u);
+        out->tap_off[i] = taps.off[order[t0]]; out->pair_shift[i] = (short)shift;
+        out->tap_col[i] = (short)taps.col[t];
+        out->tap_b[i] = (short)taps.b[t];
+      }
+    }
+    const int rows = BM + (widest + 7) / 8 * 8;
+    if (out) out->a_rows = rows;
+    return (double)runs * rows * 256 / taps.n + bn * 256;
+  };
+  int best = 0;
+  double least = group(0, nullptr);
+  for (int span = 1; span <= 64; ++span) {
+    const double bytes = group(span, nullptr);
+    if (bytes < least) { least = bytes; best = span; }
+  }
+  group(best, &g);
+}
 static int conv_like(const Pack& act, const Pack& filt, int ch_in, int ch_out, int frame_h, int frame_w, float* out, const TapList& taps,
-                     const OutGeom& og, double flops, cudaStream_t s, const char* what, int* oom, const Im2colGeom* im = nullptr) {
+                     const OutGeom& og, double flops, cudaStream_t s, const char* what, int* oom) {
   GemmParams g;
   memset(&g, 0, sizeof(g));
   const int ar = act.arith, bk = bk_of(ar);
   const int bn = pick_bn(ch_out, true);
   g.mode = kModeConv; g.epi = kEpiNchw;
-  int rc;
-  if (im) {
-    rc = make_map_im2col(&g.a_hi, ar, act.hi, im->N, im->H, im->W, act.pitch, im->lo_w, im->lo_h, im->win_w, im->win_h, BM, bk);
-    if (!rc) rc = make_map_im2col(&g.a_lo, ar, act.lo, im->N, im->H, im->W, act.pitch, im->lo_w, im->lo_h, im->win_w, im->win_h, BM, bk);
-    g.im2col = 1; g.im_w = im->box_w; g.im_h = im->box_h; g.im_lo_w = -im->lo_w; g.im_lo_h = -im->lo_h;
-  } else {
-    rc = make_map(&g.a_hi, ar, act.hi, act.rows, act.cols, act.pitch, BM);
-    if (!rc) rc = make_map(&g.a_lo, ar, act.lo, act.rows, act.cols, act.pitch, BM);
-  }
-  const long long m_rows = im ? (long long)im->N * im->box_w * im->box_h : act.rows;      // one GEMM row per output position
-  const bool pairs = !im && pairs_wanted(bn, (int)((m_rows + BM - 1) / BM), (ch_out + bn - 1) / bn, taps.n * ((ch_in + bk - 1) / bk));
-  if (!rc) rc = make_map(&g.b_hi, ar, filt.hi, filt.rows, filt.cols, filt.pitch, pairs ? bn / 2 : bn);      // a pair's CTAs load half a B tile each
-  if (!rc) rc = make_map(&g.b_lo, ar, filt.lo, filt.rows, filt.cols, filt.pitch, pairs ? bn / 2 : bn);
-  if (rc) return -1;
-  g.M = (int)m_rows; g.N = ch_out;
-  g.m_tiles = (int)((m_rows + BM - 1) / BM); g.n_tiles = (ch_out + bn - 1) / bn; g.tap_tiles = 1;
+  g.M = (int)act.rows; g.N = ch_out;
+  g.m_tiles = (int)((act.rows + BM - 1) / BM); g.n_tiles = (ch_out + bn - 1) / bn; g.tap_tiles = 1;
   g.ntaps = taps.n;
   g.chunks_per_tap = (ch_in + bk - 1) / bk;
   g.b_tap_pitch = (int)round_up(ch_in, 64);
   g.k_total = g.ntaps * g.chunks_per_tap;
-  for (int t = 0; t < taps.n; ++t) { g.tap_off[t] = taps.off[t]; g.tap_col[t] = (short)taps.col[t]; g.tap_b[t] = (short)taps.b[t]; }
+  plan_runs(g, taps, bn);
+  const bool pairs = pairs_wanted(bn, g.m_tiles, g.n_tiles, g.k_total);
+  if (pairs) g.a_rows = BM;
+  int rc = make_map(&g.a_hi, ar, act.hi, act.rows, act.cols, act.pitch, g.a_rows);
+  if (!rc) rc = make_map(&g.a_lo, ar, act.lo, act.rows, act.cols, act.pitch, g.a_rows);
+  if (!rc) rc = make_map(&g.b_hi, ar, filt.hi, filt.rows, filt.cols, filt.pitch, pairs ? bn / 2 : bn);      // a pair's CTAs load half a B tile each
+  if (!rc) rc = make_map(&g.b_lo, ar, filt.lo, filt.rows, filt.cols, filt.pitch, pairs ? bn / 2 : bn);
+  if (rc) return -1;
   g.out = out; g.err = error_word();
   g.a_scale = act.scale(); g.b_scale = filt.scale();
   g.frame_h = frame_h; g.frame_w = frame_w; g.valid_h = og.valid_h; g.valid_w = og.valid_w;
@@ -2004,17 +2278,6 @@ static int conv_like(const Pack& act, const Pack& filt, int ch_in, int ch_out, i
   return launch_gemm_bn(bn, ar, g, s, flops, what, oom);
 }
 static double conv_flops(const ConvPlan* p) { return 2.0 * p->N * p->K * p->P * p->Q * p->C * p->R * p->S; }
-// Stride-1 windows (class B) in the fp16 arithmetic read halo-free packs through im2col tensor maps: the GEMM's rows are
-// the real output positions only (a halo frame spends (H+R-1)(W+S-1)/(HW) times the multiplies, 1.65x at 7x7), and the
-// packs are smaller.  TINYFLOW_IM2COL=0 keeps the halo frames.
-static bool use_im2col(const ConvTc* st, int ar) {
-  static const bool on = [] { const char* e = getenv("TINYFLOW_IM2COL"); return e ? atoi(e) != 0 : false; }();
-  return on && st->cls == 2 && ar == kArithF16 && encode_im2col_fn() != nullptr;
-}
-// window offsets of every tap, packed as (r << 16) | s
-static void im2col_taps(TapList& taps, int R, int S) {
-  for (int r = 0; r < R; ++r) for (int q = 0; q < S; ++q) taps.add((r << 16) | q, 0, r * S + q);
-}
 // result of a tensor-path entry point from the launcher's code
 static inline int tc_result(int rc) { return rc < 0 ? -1 : (rc > 0 ? 1 : 1); }
 
@@ -2034,7 +2297,6 @@ int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cu
   if ((int64_t)t.N * t.C * t.H * t.W != n || x == y) return 0;
   const int ar = tensor_arithmetic();
   ConvTc* st = t.st;
-  if (use_im2col(st, ar)) return 0;
   const uint32_t* bound = ar == kArithF16 ? amax_tracked(x) : nullptr;
   if (ar == kArithF16 && !bound) return 0;
   std::lock_guard<std::mutex> lk(st->mu);
@@ -2059,15 +2321,6 @@ int tc_conv_fwd(ConvPlan* p, const float* x, const float* w, float* y, cudaStrea
   if (!st->cls || !encode_fn()) return 0;
   const int ar = tensor_arithmetic();
   std::lock_guard<std::mutex> lk(st->mu);
-  if (use_im2col(st, ar)) {
-    if (pack_plain(st->x, ar, 20, x, p->N, p->C, p->H, p->W, s, oom)) return *oom ? 1 : -1;
-    if (pack_filter(st, ar, w, p, 0, st->dgrad_seen, s, oom)) return *oom ? 1 : -1;
-    TapList taps;
-    im2col_taps(taps, p->R, p->S);
-    Im2colGeom im{p->N, p->H, p->W, p->pad_w, p->pad_h, p->S, p->R, p->Q, p->P};
-    OutGeom og{p->P, p->Q, p->P, p->Q, 1, 1, 0, 0};
-    return tc_result(conv_like(st->x, st->wf, st->eC, p->K, p->P, p->Q, y, taps, og, conv_flops(p), s, "DLGpuConvolution2DForward", oom, &im));
-  }
   if (pack_x(st, ar, p, x, s, oom)) return *oom ? 1 : -1;
   if (pack_filter(st, ar, w, p, 0, st->dgrad_seen, s, oom)) return *oom ? 1 : -1;
   TapList taps;
@@ -2086,17 +2339,6 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
   if (!st->cls || st->cls == 3 || !encode_fn()) return 0;
   const int ar = tensor_arithmetic();
   std::lock_guard<std::mutex> lk(st->mu);
-  if (use_im2col(st, ar)) {
-    // dx = correlation of dy with the flipped filter, R-1-pad zero rows / columns in front
-    if (pack_plain(st->dy, ar, 21, dy, p->N, p->K, p->P, p->Q, s, oom)) return *oom ? 1 : -1;
-    st->dgrad_seen = true;
-    if (pack_filter(st, ar, w, p, 1, false, s, oom)) return *oom ? 1 : -1;
-    TapList taps;
-    im2col_taps(taps, p->R, p->S);
-    Im2colGeom im{p->N, p->P, p->Q, p->S - 1 - p->pad_w, p->R - 1 - p->pad_h, p->S, p->R, p->W, p->H};
-    OutGeom og{p->H, p->W, p->H, p->W, 1, 1, 0, 0};
-    return tc_result(conv_like(st->dy, st->wd, p->K, p->C, p->H, p->W, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom, &im));
-  }
   if (pack_dy(st, ar, p, dy, s, oom)) return *oom ? 1 : -1;
   st->dgrad_seen = true;                                           // from now on forward packs both layouts in one launch
   if (pack_filter(st, ar, w, p, 1, false, s, oom)) return *oom ? 1 : -1;     // [C][flipped tap][K]; a no-op when forward made it
@@ -2141,33 +2383,6 @@ int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaS
   if (!st->cls || !encode_fn()) return 0;
   const int ar = tensor_arithmetic(), bk = bk_of(ar);
   std::lock_guard<std::mutex> lk(st->mu);
-  if (use_im2col(st, ar)) {
-    // dW[k][c][r][s] = sum over output pixels of dy[pixel][k] * x[pixel + (r, s) - pad][c]: the reduction runs over the
-    // real output pixels; x comes through an im2col map (BK pixels x one 128-byte channel group per copy), dy as it lies
-    if (pack_plain(st->x, ar, 20, x, p->N, p->C, p->H, p->W, s, oom)) return *oom ? 1 : -1;
-    if (pack_plain(st->dy, ar, 21, dy, p->N, p->K, p->P, p->Q, s, oom)) return *oom ? 1 : -1;
-    GemmParams g;
-    memset(&g, 0, sizeof(g));
-    g.err = error_word(); g.out = dw; g.data_by_data = 1;
-    const int bn = pick_bn(p->K);
-    g.mode = kModeWgrad; g.a_mn = 1; g.b_mn = 1; g.epi = kEpiWgrad;
-    g.M = p->C; g.N = p->K; g.ntaps = p->R * p->S;
-    g.slot = p->C > 64 ? BM : 64;
-    g.taps_per_tile = BM / g.slot;
-    int rc = make_map_im2col(&g.a_hi, ar, st->x.hi, p->N, p->H, p->W, st->x.pitch, p->pad_w, p->pad_h, p->S, p->R, bk, gw_of(ar));
-    if (!rc) rc = make_map_im2col(&g.a_lo, ar, st->x.lo, p->N, p->H, p->W, st->x.pitch, p->pad_w, p->pad_h, p->S, p->R, bk, gw_of(ar));
-    if (!rc) rc = make_map_mn(&g.b_hi, ar, st->dy.hi, st->dy.rows, st->dy.pitch, bn);
-    if (!rc) rc = make_map_mn(&g.b_lo, ar, st->dy.lo, st->dy.rows, st->dy.pitch, bn);
-    if (rc) return -1;
-    g.a_scale = st->x.scale(); g.b_scale = st->dy.scale();
-    g.m_tiles = (p->C + g.slot - 1) / g.slot;
-    g.tap_tiles = (g.ntaps + g.taps_per_tile - 1) / g.taps_per_tile;
-    g.n_tiles = (p->K + bn - 1) / bn;
-    g.im2col = 1; g.im_w = p->Q; g.im_h = p->P; g.im_lo_w = -p->pad_w; g.im_lo_h = -p->pad_h;
-    for (int r = 0; r < p->R; ++r) for (int q = 0; q < p->S; ++q) g.tap_off[r * p->S + q] = (r << 16) | q;
-    g.k_total = (int)((st->dy.rows + bk - 1) / bk);
-    return tc_result(launch_gemm_bn(bn, ar, g, s, conv_flops(p), "DLGpuConvolutionBackwardFilter", oom));
-  }
   if (pack_x(st, ar, p, x, s, oom)) return *oom ? 1 : -1;
   if (pack_dy(st, ar, p, dy, s, oom)) return *oom ? 1 : -1;
   GemmParams g;
