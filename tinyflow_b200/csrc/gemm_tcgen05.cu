@@ -847,7 +847,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
         int got = lane == 0 ? (int)mbar_wait(&acc_full[acc_buf], (grp >> 1) & 1, abort_flag) : 1;
         return __shfl_sync(0xffffffffu, got, 0) != 0;
       };
-      // NC values of this thread's row at columns c0.. of the warp's half: base + constant * stride, one wide multiply-add each
+      // NC values of this thread's row at columns c0.. of the warp's half; offsets of 32 bits (BN planes are far below 2^32 elements):
+      // 64-bit ones cost 1-2 us of 70 in stores alone
       auto store_cols = [&](const float2* v2, int c0) {
         const float* v = reinterpret_cast<const float*>(v2);
         if (!row_ok || c0 >= ncols) return;
@@ -857,11 +858,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
           for (int q = 0; q < NC / 4; ++q) reinterpret_cast<float4*>(dst)[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
         } else if (c0 + NC <= ncols) {
 #pragma unroll
-          for (int q = 0; q < NC; ++q) *reinterpret_cast<float*>(dst + (uint64_t)col_bytes * (uint32_t)q) = v[q];
+          for (int q = 0; q < NC; ++q) reinterpret_cast<float*>(dst)[(size_t)((uint32_t)q * ra.col_stride)] = v[q];
         } else {
 #pragma unroll
           for (int q = 0; q < NC; ++q)
-            if (c0 + q < ncols) *reinterpret_cast<float*>(dst + (uint64_t)col_bytes * (uint32_t)q) = v[q];
+            if (c0 + q < ncols) reinterpret_cast<float*>(dst)[(size_t)((uint32_t)q * ra.col_stride)] = v[q];
         }
       };
       const uint32_t t_lane = tmem_base + half * HC + ((uint32_t)(quarter * 32) << 16);
