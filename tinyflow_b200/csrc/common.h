@@ -50,6 +50,7 @@ struct KernelTimer {
 // Two operators do not launch at once; their arguments wait in a one-entry slot:
 //  * DLGpuActivationBackward(relu): if the very next call into the library is the per-activation batch-norm backward that
 //    consumes the ReLU's gradient, ONE kernel computes both (reads x and dy once, writes both gradients);
+//    if it is the backward call of the convolution in front of the ReLU, the kernel that packs that convolution's dy computes it;
 //  * DLGpuMatrixElementwiseAdd: if the very next call is the ReLU forward of the sum (the end of a residual block), ONE
 //    kernel writes the sum and its ReLU.
 // Every other way into the library - stream_of(), which every operator with a stream argument calls first,

@@ -1,6 +1,7 @@
 // C-ABI entry points of the dense contractions (matmul, convolution forward / backward-data /
 // backward-filter) and the dispatch between the tcgen05 tensor-core path and the CUDA-core path.
 #include "common.h"
+#include <vector>
 
 namespace tf {
 
@@ -30,6 +31,8 @@ int tensor_path_error();
 void tensor_path_error_clear();
 int tensor_path_timeout_probe(long long limit_cycles, cudaStream_t s);
 long long fused_relu_pack_count();
+int tc_pack_filters(const void* const* arrays, int n, cudaStream_t s);
+int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, float* out, cudaStream_t s);
 // which engine served this thread's most recent contraction: 1 = CUDA cores, 2 = tensor cores (0 = none yet)
 static thread_local int t_last_path = 0;
 
@@ -50,6 +53,13 @@ int TfGetArithmetic(void) { return tensor_arithmetic(); }
 
 int TfTensorPathError(void) { return tensor_path_error(); }
 int TfClearTensorPathError(void) { tensor_path_error_clear(); return 0; }
+int TfPackFilters(const DLArrayHandle* arrays, int n, void** cudaStream) {
+  TF_REQUIRE(arrays && n >= 0, "TfPackFilters: null argument");
+  if (!t_recording) return 0;
+  std::vector<const void*> data;
+  for (int i = 0; i < n; ++i) if (arrays[i] && arrays[i]->ctx.device_type == kGPU) data.push_back(arrays[i]->data);
+  return tc_pack_filters(data.data(), (int)data.size(), stream_of(cudaStream));
+}
 int TfFusedReluPackCount(long long* count) { if (count) *count = fused_relu_pack_count(); return 0; }
 int TfFusedReluBnBackwardCount(long long* count) { if (count) *count = fused_relu_bn_bwd_count(); return 0; }
 int TfFusedAddReluCount(long long* count) { if (count) *count = fused_add_relu_count(); return 0; }
@@ -148,12 +158,25 @@ int DLGpuConvolution2DForward(const DLArrayHandle input, const DLArrayHandle fil
   return cudacore_conv_fwd(p, (const float*)input->data, (const float*)filter->data, out_f32(output), s);
 }
 
+// A ReLU backward that was held back and whose output is this call's incoming gradient is computed by the kernel that packs it.
+static int relu_backward_of(ConvPlan* p, const DLArrayHandle doutput, void** cudaStream) {
+  DeferredOp relu;
+  const cudaStream_t s = stream_of_keep_deferred(cudaStream);
+  if (g_path == 1 || !take_deferred(kDeferReluBwd, (const float*)doutput->data, numel(doutput), &relu)) return 0;
+  // the slot is locked until release_deferred(): nothing below may call stream_of() / last_compute_stream()
+  const int fused = relu.stream == s ? tc_fused_relu_bwd_pack(p, relu.a, relu.b, relu.out, s) : 0;
+  if (!fused) launch_deferred_now(relu);
+  release_deferred();
+  return fused < 0 ? -1 : 0;
+}
+
 int DLGpuConvolutionBackwardData(const DLArrayHandle input, const DLArrayHandle doutput, const DLArrayHandle filter, DLArrayHandle dinput,
                                  void*** cudnnlist, void** cudnnHandle, int* memorytoSaving, void** cudaStream) {
   (void)cudnnHandle;
   ConvPlan* p = plan_of<ConvPlan>(cudnnlist, kPlanConv);
   if (check_conv(p, input, filter, doutput, "DLGpuConvolutionBackwardData")) return -1;
   TF_REQUIRE(dinput && numel(dinput) == numel(input), "DLGpuConvolutionBackwardData: dinput does not match input");
+  if (relu_backward_of(p, doutput, cudaStream)) return -1;
   cudaStream_t s = stream_of(cudaStream);
   if (g_path == 0) {
     int r = direct_conv_dgrad(p, (const float*)doutput->data, (const float*)filter->data, out_f32(dinput), s);
@@ -178,6 +201,7 @@ int DLGpuConvolutionBackwardFilter(const DLArrayHandle input, const DLArrayHandl
   ConvPlan* p = plan_of<ConvPlan>(cudnnlist, kPlanConv);
   if (check_conv(p, input, filter, doutput, "DLGpuConvolutionBackwardFilter")) return -1;
   TF_REQUIRE(dfilter && numel(dfilter) == numel(filter), "DLGpuConvolutionBackwardFilter: dfilter does not match filter");
+  if (relu_backward_of(p, doutput, cudaStream)) return -1;
   cudaStream_t s = stream_of(cudaStream);
   if (g_path == 0) {
     int r = direct_conv_wgrad(p, (const float*)input->data, (const float*)doutput->data, out_f32(dfilter), s);

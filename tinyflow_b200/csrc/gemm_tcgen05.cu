@@ -35,6 +35,8 @@
 #include <mutex>
 #include <type_traits>
 #include <unordered_map>
+#include <unordered_set>
+#include <vector>
 
 namespace tf {
 
@@ -393,6 +395,7 @@ struct alignas(64) GemmParams {
   int b_tap_pitch;                // kModeConv: columns per tap in the packed filter
   int ntaps;
   float* out;
+  uint32_t *amax, *amax_clear;    // where the epilogue leaves max|out| (null: nobody asked), and the word the next write of `out` will use
   const float* a_scale; const float* b_scale;   // device words: the power-of-two scales the packs were made with
   long long ldc;                  // kEpiRowMajor
   // kEpiNchw: row m -> (image, i, j) in a frame of frame_h x frame_w, stored at output pixel
@@ -828,6 +831,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
     const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));     // powers of two: exact
     const float2 scale2 = make_float2(inv_scale, inv_scale);
     int group = 0;
+    uint32_t top = 0;         // largest |value| this thread stored; one atomic per warp and launch
     bool ok = true;
     WorkIter iter(p);
     WorkItem w;
@@ -852,6 +856,10 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
       auto store_cols = [&](const float2* v2, int c0) {
         const float* v = reinterpret_cast<const float*>(v2);
         if (!row_ok || c0 >= ncols) return;
+        if (p.amax) {
+#pragma unroll
+          for (int q = 0; q < NC; ++q) top = max(top, amax_bits(v[q]));
+        }
         char* dst = row_out + (uint64_t)col_bytes * (uint32_t)c0;
         if (vec_ok && c0 + NC <= ncols) {
 #pragma unroll
@@ -952,6 +960,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
         store_cols(accv + c0 / 2, c0);
       }
     }
+    if (p.amax) {
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (lane == 0 && top) atomicMax(p.amax, top);
+      if (blockIdx.x == 0 && threadIdx.x == 64 && p.amax_clear) *p.amax_clear = 0u;
+    }
   }
 
   if (p.cluster > 1) {
@@ -966,6 +979,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
     const RowAddr ra = row_address(p, mt, tap, row);
     const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));
     const int c1 = min(BN * (rank + 1) / p.cluster, p.N - nt * BN);
+    uint32_t top = 0;
     __syncwarp();
     cluster_sync_all();
     if (!*abort_flag) {
@@ -988,9 +1002,16 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
 #pragma unroll
         for (int j = 0; j < kUnroll; ++j) {
           const int c = c0 + j * kLanes;
-          if (ra.ok && c < c1) p.out[ra.base + (long long)(nt * BN + c) * ra.col_stride] = sum[j] * inv_scale;
+          if (ra.ok && c < c1) {
+            p.out[ra.base + (long long)(nt * BN + c) * ra.col_stride] = sum[j] * inv_scale;
+            top = max(top, amax_bits(sum[j] * inv_scale));
+          }
         }
       }
+    }
+    if (p.amax) {
+      top = __reduce_max_sync(0xffffffffu, top);
+      if (lane == 0 && top) atomicMax(p.amax, top);
     }
     __syncwarp();
     cluster_sync_all();        // nobody leaves while its shared memory is still read
@@ -1220,6 +1241,8 @@ constexpr int kReduceCols = 8, kReduceWays = 4;
 template <int BN>
 __global__ void __launch_bounds__(BM * kReduceWays) reduce_partials_kernel(const __grid_constant__ GemmParams p) {
   __shared__ float part[kReduceWays][kReduceCols][BM];
+  __shared__ uint32_t block_top;
+  if (threadIdx.x == 0 && threadIdx.y == 0) block_top = 0u;
   grid_dep_sync();
   const int t = blockIdx.x;                            // tail tile
   int mt, nt, tap;
@@ -1258,8 +1281,8 @@ __global__ void __launch_bounds__(BM * kReduceWays) reduce_partials_kernel(const
   __syncthreads();
   // every row group finishes a quarter of the block's columns: subtotals added in row-group order
   const RowAddr ra = row_address(p, mt, tap, row);
-  if (!ra.ok) return;
   const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));
+  uint32_t top = 0;
   constexpr int kPer = kReduceCols / kReduceWays;
 #pragma unroll
   for (int j = 0; j < kPer; ++j) {
@@ -1268,8 +1291,16 @@ __global__ void __launch_bounds__(BM * kReduceWays) reduce_partials_kernel(const
 #pragma unroll
     for (int w2 = 1; w2 < kReduceWays; ++w2) v += part[w2][q][row];
     const int n = nt * BN + c_begin + q;
-    if (n < p.N) p.out[ra.base + (long long)n * ra.col_stride] = v * inv_scale;
+    if (ra.ok && n < p.N) {
+      p.out[ra.base + (long long)n * ra.col_stride] = v * inv_scale;
+      top = max(top, amax_bits(v * inv_scale));
+    }
   }
+  if (!p.amax) return;
+  top = __reduce_max_sync(0xffffffffu, top);
+  if ((threadIdx.x & 31) == 0 && top) atomicMax(&block_top, top);
+  __syncthreads();
+  if (threadIdx.x == 0 && threadIdx.y == 0 && block_top) atomicMax(p.amax, block_top);
 }
 
 // Exercises the bounded wait on its own: one thread waits, with a short limit, on a barrier that nothing arms; the wait
@@ -1406,12 +1437,14 @@ __global__ void __launch_bounds__(256) pack_matrix_kernel(const float* __restric
 // row through shared memory: reads run along w (TC/8 independent loads per thread in flight), writes along c as
 // 16-byte vectors (8 halves) of hi and of lo.
 struct PackGeom { int N, C, H, W, frame_h, frame_w, off_h, off_w, sh, sw, pitch, dst_c0, c_limit; };
-// RELU: the source is the input of a ReLU; the kernel applies it, writes the fp32 result to y_out (same layout as the
+// kPackRelu: the source is the input of a ReLU; the kernel applies it, writes the fp32 result to y_out (same layout as the
 // source), records max|y| like the stand-alone ReLU kernel does, and packs y.  The pack's scale then comes from max|x|, an
-// upper bound of max|y| that is known before the pass starts.
-template <int TC, class E, bool RELU>
+// upper bound of max|y| that is known before the pass starts.  kPackReluBwd: the same for the ReLU's backward, y = mask > 0 ? x : 0.
+// HBM-bound: 16 and 20 bytes an element where the two kernels one after the other move 20 and 24.
+enum { kPackPlain = 0, kPackRelu = 1, kPackReluBwd = 2 };
+template <int TC, class E, int MODE>
 __global__ void __launch_bounds__(256) pack_nchw_kernel(const float* __restrict__ src, E* __restrict__ hi, E* __restrict__ lo, PackGeom g, ScaleRef sr,
-                                                        float* __restrict__ y_out, AmaxOut am) {
+                                                        const float* __restrict__ mask, float* __restrict__ y_out, AmaxOut am) {
   grid_dep_sync();
   // tile[c][f ^ (c / 8)]: the XOR keeps both phases free of bank conflicts (stores: 32 lanes = 32 frame positions
   // of one channel; loads: lanes = 8-channel groups of a few positions that are TC/8 apart)
@@ -1443,14 +1476,23 @@ __global__ void __launch_bounds__(256) pack_nchw_kernel(const float* __restrict_
 #pragma unroll
       for (int k = 0; k < TC / 8; ++k) v[k] = 0.f;
     }
-    if (RELU) {
+    if (MODE != kPackPlain) {
       uint32_t m = 0;
       if (ok) {
-        float* yp = y_out + (sp - src) - (long long)(TC / 8) * step;        // the element the first load read
+        const long long at = (sp - src) - (long long)(TC / 8) * step;       // the element the first load read
+        float* yp = y_out + at;
+        if (MODE == kPackReluBwd) {
+          const float* mp = mask + at;
+          float u[TC / 8];
+#pragma unroll
+          for (int k = 0; k < TC / 8; ++k) { u[k] = 8 * k < avail ? __ldg(mp) : 0.f; mp += step; }
+#pragma unroll
+          for (int k = 0; k < TC / 8; ++k) v[k] = u[k] > 0.f ? v[k] : 0.f;
+        }
 #pragma unroll
         for (int k = 0; k < TC / 8; ++k) {
           const float x = v[k];
-          v[k] = x > 0.f ? x : (x != x ? x : 0.f);                           // NaN propagates
+          if (MODE == kPackRelu) v[k] = x > 0.f ? x : (x != x ? x : 0.f);    // NaN propagates
           if (8 * k < avail) { *yp = v[k]; m = max(m, amax_bits(v[k])); }
           yp += step;
         }
@@ -1536,65 +1578,65 @@ __global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restri
   }
 }
 
-// filters [K][C][R][S] -> forward pack [K][tap][cpad] (flip = 0) or backward-data pack [C][tap'][kpad] (flip = 1,
-// tap' = (R-1-r)*S + (S-1-s)), zero in the channel padding.
+// Filters [K][C][taps] -> the forward layout [K][tap][C up to pad_f] and / or the backward-data layout [C][flipped tap][K up to
+// pad_d].  One launch packs any number of filters: a step's 50-150 filters, packed when their convolution came up, were as
+// many launches of 5 us for 1-2 us of traffic.  A block moves 32 x 32 filters through shared memory, so that the fp32 words are
+// read in order and both layouts are written in rows of 64 bytes; read straight from the filter, the backward-data layout took a
+// sector per element.  Bound by HBM (12 bytes an element); few blocks per filter, so by latency where filters are few.
+struct FilterJob {
+  const float* w;
+  void *hi_f, *lo_f, *hi_d, *lo_d;       // a layout that is not wanted: null
+  const uint32_t* amax; uint32_t* amax_next;
+  float *scale_f, *scale_d;
+  int K, C, taps, pad_f, pad_d, k_blocks, first_block;
+};
+constexpr int kFilterJobs = 128, kFilterTaps = 9, kFilterTile = 32;
+struct FilterJobs { int n; FilterJob job[kFilterJobs]; };
 template <class E>
-__global__ void __launch_bounds__(256) pack_filter_kernel(const float* __restrict__ w, E* __restrict__ hi, E* __restrict__ lo,
-                                                          int K, int C, int R, int S, int flip, int inner_pad, ScaleRef sr) {
+__global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant__ FilterJobs jobs) {
   grid_dep_sync();
-  const float sc = pack_scale(sr, blockIdx.x == 0 && threadIdx.x == 0);
-  int taps = R * S;
-  long long rows = flip ? C : K, total = rows * taps * inner_pad, stride = (long long)gridDim.x * blockDim.x;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-    int in = (int)(idx % inner_pad);
-    long long t2 = idx / inner_pad;
-    int tap = (int)(t2 % taps), row = (int)(t2 / taps);
-    int inner_n = flip ? K : C;
-    float a = 0.f;
-    if (in < inner_n) {
-      int k = flip ? in : row, c = flip ? row : in;
-      int src_tap = flip ? (taps - 1 - tap) : tap;
-      a = w[((long long)k * C + c) * taps + src_tap] * sc;
-    }
-    E h, l;
-    split_pair(a, h, l);
-    hi[idx] = h; lo[idx] = l;
+  __shared__ float tile[kFilterTile][kFilterTile * kFilterTaps + 1];
+  int lo = 0, hi = jobs.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (jobs.job[mid].first_block <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
   }
-}
-
-// Both filter packs of one convolution in a single launch (the weights do not change between the forward and the
-// backward-data call of a step, so the second pack rides along with the first): element idx of the forward pack and
-// element idx of the backward-data pack per thread.
-template <class E>
-__global__ void __launch_bounds__(256) pack_filter_pair_kernel(const float* __restrict__ w, E* __restrict__ hi_f, E* __restrict__ lo_f,
-                                                               E* __restrict__ hi_d, E* __restrict__ lo_d, int K, int C, int R, int S,
-                                                               int pad_f, int pad_d, ScaleRef sr, float* __restrict__ scale_d) {
-  grid_dep_sync();
-  const bool first = blockIdx.x == 0 && threadIdx.x == 0;
-  const float sc = pack_scale(sr, first);
-  if (first) *scale_d = sc;
-  const int taps = R * S;
-  const long long total_f = (long long)K * taps * pad_f, total_d = (long long)C * taps * pad_d;
-  const long long total = total_f > total_d ? total_f : total_d, stride = (long long)gridDim.x * blockDim.x;
-  for (long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += stride) {
-    if (idx < total_f) {
-      int in = (int)(idx % pad_f);
-      long long t2 = idx / pad_f;
-      int tap = (int)(t2 % taps), k = (int)(t2 / taps);
-      float a = in < C ? w[((long long)k * C + in) * taps + tap] * sc : 0.f;
-      E h, l;
-      split_pair(a, h, l);
-      hi_f[idx] = h; lo_f[idx] = l;
+  const FilterJob& j = jobs.job[lo];
+  const int block = blockIdx.x - j.first_block, k0 = block % j.k_blocks * kFilterTile, c0 = block / j.k_blocks * kFilterTile;
+  const float sc = j.amax ? scale_from_amax(__ldg(j.amax)) : 1.f;
+  if (block == 0 && threadIdx.x == 0) {
+    if (j.scale_f) *j.scale_f = sc;
+    if (j.scale_d) *j.scale_d = sc;
+    if (j.amax_next) *j.amax_next = 0u;
+  }
+  const int taps = j.taps, K = j.K, C = j.C, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  E *const hi_f = (E*)j.hi_f, *const lo_f = (E*)j.lo_f, *const hi_d = (E*)j.hi_d, *const lo_d = (E*)j.lo_d;
+  for (int t0 = 0; t0 < taps; t0 += kFilterTaps) {
+    const int nt = min(kFilterTaps, taps - t0), row = kFilterTile * nt;
+    for (int r = warp; r < kFilterTile; r += 8) {
+      const float* src = j.w + ((long long)(k0 + r) * C + c0) * taps + t0;
+      for (int e = lane; e < row; e += 32) {
+        const int c = e / nt, t = e - c * nt;
+        tile[r][e] = k0 + r < K && c0 + c < C ? __ldg(src + (long long)c * taps + t) * sc : 0.f;
+      }
     }
-    if (idx < total_d) {
-      int in = (int)(idx % pad_d);
-      long long t2 = idx / pad_d;
-      int tap = (int)(t2 % taps), c = (int)(t2 / taps);
-      float a = in < K ? w[((long long)in * C + c) * taps + (taps - 1 - tap)] * sc : 0.f;
-      E h, l;
-      split_pair(a, h, l);
-      hi_d[idx] = h; lo_d[idx] = l;
+    __syncthreads();
+    const int pair = (threadIdx.x & 15) * 2, line0 = threadIdx.x >> 4;
+    for (int line = line0; line < row; line += 16) {
+      const int r = line / nt, t = line - r * nt;
+      E h0, l0, h1, l1;
+      if (hi_f && k0 + r < K && c0 + pair < j.pad_f) {
+        split_pair(tile[r][pair * nt + t], h0, l0); split_pair(tile[r][(pair + 1) * nt + t], h1, l1);
+        const long long at = ((long long)(k0 + r) * taps + t0 + t) * j.pad_f + c0 + pair;
+        store_two(hi_f + at, h0, h1); store_two(lo_f + at, l0, l1);
+      }
+      if (hi_d && c0 + r < C && k0 + pair < j.pad_d) {
+        split_pair(tile[pair][r * nt + t], h0, l0); split_pair(tile[pair + 1][r * nt + t], h1, l1);
+        const long long at = ((long long)(c0 + r) * taps + taps - 1 - t0 - t) * j.pad_d + k0 + pair;
+        store_two(hi_d + at, h0, h1); store_two(lo_d + at, l0, l1);
+      }
     }
+    __syncthreads();
   }
 }
 
@@ -2020,6 +2062,9 @@ struct ConvTc {
   int eC = 0, eR = 1, eS = 1;                            // reduction channels and window of the problem as the GEMM sees it
   int cp = 0;                                            // class D: columns per stride phase (C rounded up to 64)
   bool dgrad_seen = false;                               // backward-data has run on this plan: forward also packs its filter layout
+  bool track_y = false, track_dx = false;                // a ReLU asked for max|y| / max|dx|: the epilogue leaves it
+  const float* filter = nullptr;                         // the array the filter packs were last made from, and its plan
+  const ConvPlan* plan = nullptr;
   Pack x, dy, wf, wd;
   std::mutex mu;
 };
@@ -2069,25 +2114,26 @@ static ConvTc* conv_state(ConvPlan* p) {
 // One launch of the frame pack: `chans` channels of an NCHW tensor (spatial dims H x W) into columns dst_c0 .. dst_c0 + cover
 // of pk (zeros past `chans`)
 static int launch_pack_nchw(Pack& pk, const ScaleRef& sr, const float* src, int N, int chans, int H, int W, int frame_h, int frame_w, int off_h, int off_w,
-                            int sh, int sw, int dst_c0, int cover, cudaStream_t s, float* relu_out = nullptr, AmaxOut relu_am = AmaxOut{}) {
+                            int sh, int sw, int dst_c0, int cover, cudaStream_t s, float* relu_out = nullptr, AmaxOut relu_am = AmaxOut{}, const float* mask = nullptr) {
   PackGeom g{N, chans, H, W, frame_h, frame_w, off_h, off_w, sh, sw, (int)pk.pitch, dst_c0, cover};
   const int tc = cover > 64 ? 128 : cover > 32 ? 64 : 32;
   dim3 grid(N * ((cover + tc - 1) / tc), (frame_h * frame_w + 31) / 32);
   TF_REQUIRE(grid.y <= 65535, "pack: frame of %d x %d positions is too large", frame_h, frame_w);
-  KernelTimer kt(relu_out ? "relu_pack" : "pack_nchw", s, 0, (relu_out ? 8.0 : 4.0) * N * chans * H * W / (sh * sw) + 2.0 * elem_of(pk.arith) * pk.rows * cover);
+  const char* what = mask ? "relu_bwd_pack" : relu_out ? "relu_pack" : "pack_nchw";
+  KernelTimer kt(what, s, 0, (mask ? 12.0 : relu_out ? 8.0 : 4.0) * N * chans * H * W / (sh * sw) + 2.0 * elem_of(pk.arith) * pk.rows * cover);
   with_elems(pk, [&](auto* hi, auto* lo) {
     using E = std::remove_pointer_t<decltype(hi)>;
-    if (relu_out) {
-      if (tc == 128) launch_dep(pack_nchw_kernel<128, E, true>, grid, dim3(256), 0, s, src, hi, lo, g, sr, relu_out, relu_am);
-      else if (tc == 64) launch_dep(pack_nchw_kernel<64, E, true>, grid, dim3(256), 0, s, src, hi, lo, g, sr, relu_out, relu_am);
-      else launch_dep(pack_nchw_kernel<32, E, true>, grid, dim3(256), 0, s, src, hi, lo, g, sr, relu_out, relu_am);
-    } else {
-      if (tc == 128) launch_dep(pack_nchw_kernel<128, E, false>, grid, dim3(256), 0, s, src, hi, lo, g, sr, (float*)nullptr, AmaxOut{});
-      else if (tc == 64) launch_dep(pack_nchw_kernel<64, E, false>, grid, dim3(256), 0, s, src, hi, lo, g, sr, (float*)nullptr, AmaxOut{});
-      else launch_dep(pack_nchw_kernel<32, E, false>, grid, dim3(256), 0, s, src, hi, lo, g, sr, (float*)nullptr, AmaxOut{});
-    }
+    auto launch = [&](auto mode) {
+      constexpr int MODE = decltype(mode)::value;
+      if (tc == 128) launch_dep(pack_nchw_kernel<128, E, MODE>, grid, dim3(256), 0, s, src, hi, lo, g, sr, mask, relu_out, relu_am);
+      else if (tc == 64) launch_dep(pack_nchw_kernel<64, E, MODE>, grid, dim3(256), 0, s, src, hi, lo, g, sr, mask, relu_out, relu_am);
+      else launch_dep(pack_nchw_kernel<32, E, MODE>, grid, dim3(256), 0, s, src, hi, lo, g, sr, mask, relu_out, relu_am);
+    };
+    if (mask) launch(std::integral_constant<int, kPackReluBwd>());
+    else if (relu_out) launch(std::integral_constant<int, kPackRelu>());
+    else launch(std::integral_constant<int, kPackPlain>());
   });
-  TF_AFTER(s, relu_out ? "relu_pack" : "pack_nchw");
+  TF_AFTER(s, what);
   return 0;
 }
 static bool pack_valid(const Pack& pk, int ar, const void* src, uint64_t ver, int tag, long long rows, long long cols) {
@@ -2111,6 +2157,24 @@ void tc_note_relu_output(const void* node, const void* y) {     // call after th
   const uint64_t ver = version_of(y);
   std::lock_guard<std::mutex> lk(g_targets_mu);
   g_relu_writer[y] = ReluNote{node, ver};
+}
+// A convolution's output is what a ReLU reads, forward and backward; its maximum, folded into the epilogue, is the bound that
+// lets the ReLU write the next pack too.  Only outputs that a ReLU has asked about are tracked (behind a batch
+// norm nobody needs it, and ResNet-50 lost 0.5 % with all of them tracked).
+struct ConvNote { bool* wanted; uint64_t version; };
+static std::unordered_map<const void*, ConvNote> g_conv_writer;
+static void note_conv_output(const float* out, bool* wanted) {      // call after the output's write version was bumped
+  const uint64_t ver = version_of(out);
+  std::lock_guard<std::mutex> lk(g_targets_mu);
+  g_conv_writer[out] = ConvNote{wanted, ver};
+}
+static const uint32_t* bound_of(const float* x) {
+  if (const uint32_t* word = amax_tracked(x)) return word;
+  const uint64_t ver = version_of(x);
+  std::lock_guard<std::mutex> lk(g_targets_mu);
+  auto it = g_conv_writer.find(x);
+  if (it != g_conv_writer.end() && it->second.version == ver) *it->second.wanted = true;
+  return nullptr;
 }
 static void remember_pack_target(const void* x, uint64_t ver, ConvTc* st, const ConvPlan* p) {
   std::lock_guard<std::mutex> lk(g_targets_mu);
@@ -2172,43 +2236,83 @@ static int pack_dy(ConvTc* st, int ar, const ConvPlan* p, const float* dy, cudaS
   return 0;
 }
 // Filter packs are keyed like the activation packs (pointer, write version): an optimiser step bumps the version.
+// filter_job() prepares the pack of one filter (layouts: 1 forward, 2 backward-data) and stamps it as made; 0 on success.
+static std::mutex g_filter_plans_mu;
+static std::vector<ConvTc*> g_filter_plans;            // every plan that has packed a filter
+static int filter_job(ConvTc* st, int ar, const float* w, const ConvPlan* p, int layouts, cudaStream_t s, int* oom, FilterJob* job) {
+  const int taps = st->eR * st->eS;
+  memset(job, 0, sizeof(*job));
+  job->w = w; job->K = p->K; job->C = st->eC; job->taps = taps;
+  const uint64_t ver = version_of(w);
+  Pack* first = nullptr;
+  for (int d = 0; d < 2; ++d) {
+    if (!(layouts >> d & 1)) continue;
+    Pack& pk = d ? st->wd : st->wf;
+    const int rows = d ? st->eC : p->K, pad = (int)round_up(d ? p->K : st->eC, 64);
+    if (pack_alloc(pk, ar, rows, (long long)taps * pad, s, oom)) return 1;
+    (d ? job->hi_d : job->hi_f) = pk.hi; (d ? job->lo_d : job->lo_f) = pk.lo; (d ? job->pad_d : job->pad_f) = pad;
+    (d ? job->scale_d : job->scale_f) = reinterpret_cast<float*>(pk.words + 2);
+    if (!first) first = &pk;
+    pk.src = w; pk.version = ver; pk.tag = 10 + d;
+  }
+  const ScaleRef sr = begin_pack(*first, w, (long long)p->K * p->C * p->R * p->S, s);
+  job->amax = sr.amax_cur; job->amax_next = sr.amax_next;
+  if (!st->plan) {
+    std::lock_guard<std::mutex> lk(g_filter_plans_mu);
+    g_filter_plans.push_back(st);
+  }
+  st->plan = p; st->filter = w;
+  return 0;
+}
+static int launch_filter_jobs(FilterJobs& jobs, int ar, cudaStream_t s) {
+  int blocks = 0;
+  double elems = 0;
+  for (int i = 0; i < jobs.n; ++i) {
+    FilterJob& j = jobs.job[i];
+    j.first_block = blocks;
+    j.k_blocks = (std::max(j.K, j.pad_d) + kFilterTile - 1) / kFilterTile;
+    blocks += j.k_blocks * ((std::max(j.C, j.pad_f) + kFilterTile - 1) / kFilterTile);
+    elems += (double)j.K * j.C * j.taps;
+  }
+  KernelTimer kt("pack_filters", s, 0, elems * (4.0 + 4.0 * elem_of(ar)));
+  TF_CUDA(ar == kArithTF32 ? launch_dep(pack_filters_kernel<float>, dim3(blocks), dim3(256), 0, s, jobs) : launch_dep(pack_filters_kernel<__half>, dim3(blocks), dim3(256), 0, s, jobs));
+  TF_AFTER(s, "pack_filters");
+  return 0;
+}
 // `with_other` makes the forward call produce the backward-data pack in the same launch.
 static int pack_filter(ConvTc* st, int ar, const float* w, const ConvPlan* p, int flip, bool with_other, cudaStream_t s, int* oom) {
-  Pack& pk = flip ? st->wd : st->wf;
-  const uint64_t ver = version_of(w);
-  const int taps = st->eR * st->eS;
-  auto dims = [&](int f, int& rows, int& pad) { rows = f ? st->eC : p->K; pad = (int)round_up(f ? p->K : st->eC, 64); };
-  int rows, pad;
-  dims(flip, rows, pad);
-  if (pack_valid(pk, ar, w, ver, 10 + flip, rows, (long long)taps * pad)) return 0;
-  if (pack_alloc(pk, ar, rows, (long long)taps * pad, s, oom)) return 1;
-  const long long nw = (long long)p->K * p->C * p->R * p->S;
-  if (with_other && !flip) {
-    Pack& pd = st->wd;
-    int rows_d, pad_d;
-    dims(1, rows_d, pad_d);
-    if (pack_alloc(pd, ar, rows_d, (long long)taps * pad_d, s, oom)) return 1;
-    ScaleRef sr = begin_pack(pk, w, nw, s);
-    long long total = std::max((long long)rows * taps * pad, (long long)rows_d * taps * pad_d);
-    with_elems(pk, [&](auto* hi, auto* lo) {
-      using E = std::remove_pointer_t<decltype(hi)>;
-      launch_dep(pack_filter_pair_kernel<E>, dim3(grid_for(total, 256)), dim3(256), 0, s, w, hi, lo, (E*)pd.hi, (E*)pd.lo, p->K, st->eC, st->eR, st->eS, pad, pad_d, sr,
-                 reinterpret_cast<float*>(pd.words + 2));
-    });
-    TF_AFTER(s, "pack_filter");
-    pk.src = w; pk.version = ver; pk.tag = 10;
-    pd.src = w; pd.version = ver; pd.tag = 11;
-    return 0;
+  const Pack& pk = flip ? st->wd : st->wf;
+  const int rows = flip ? st->eC : p->K, pad = (int)round_up(flip ? p->K : st->eC, 64);
+  if (pack_valid(pk, ar, w, version_of(w), 10 + flip, rows, (long long)st->eR * st->eS * pad)) return 0;
+  FilterJobs one;
+  one.n = 1;
+  if (int rc = filter_job(st, ar, w, p, flip ? 2 : with_other ? 3 : 1, s, oom, &one.job[0])) return rc;
+  return launch_filter_jobs(one, ar, s);
+}
+// While a step is recorded: the filters among `arrays` whose plans were last fed from them, all in one launch, ahead of the
+// convolutions that find them packed.  What it leaves out, or guesses wrong, the convolution packs when it comes up.
+int tc_pack_filters(const void* const* arrays, int n, cudaStream_t s) {
+  if (contraction_path_is_cuda_cores() || !encode_fn()) return 0;
+  const int ar = tensor_arithmetic();
+  std::unordered_set<const void*> wanted(arrays, arrays + n);
+  std::vector<ConvTc*> plans;
+  {
+    std::lock_guard<std::mutex> lk(g_filter_plans_mu);
+    for (ConvTc* st : g_filter_plans) if (wanted.count(st->filter)) plans.push_back(st);
   }
-  ScaleRef sr = begin_pack(pk, w, nw, s);
-  long long total = (long long)rows * taps * pad;
-  with_elems(pk, [&](auto* hi, auto* lo) {
-    using E = std::remove_pointer_t<decltype(hi)>;
-    launch_dep(pack_filter_kernel<E>, dim3(grid_for(total, 256)), dim3(256), 0, s, w, hi, lo, p->K, st->eC, st->eR, st->eS, flip, pad, sr);
-  });
-  TF_AFTER(s, "pack_filter");
-  pk.src = w; pk.version = ver; pk.tag = 10 + flip;
-  return 0;
+  FilterJobs jobs;
+  jobs.n = 0;
+  for (ConvTc* st : plans) {
+    std::lock_guard<std::mutex> lk(st->mu);
+    const float* w = st->filter;
+    if (!wanted.count(w) || !st->wf.hi || st->wf.arith != ar || (ar == kArithF16 && !amax_tracked(w))) continue;
+    int oom = 0;
+    if (filter_job(st, ar, w, st->plan, st->dgrad_seen ? 3 : 1, s, &oom, &jobs.job[jobs.n])) continue;
+    if (++jobs.n < kFilterJobs) continue;
+    if (launch_filter_jobs(jobs, ar, s)) return -1;
+    jobs.n = 0;
+  }
+  return jobs.n ? launch_filter_jobs(jobs, ar, s) : 0;
 }
 
 // forward and backward-data share one launcher: out[pixel][ch_out] = sum_{tap, ch_in} act[pixel + off(tap)][col(tap) + ch_in] * filt[ch_out][b(tap)][ch_in]
@@ -2251,7 +2355,7 @@ static void plan_runs(GemmParams& g, const TapList& taps, int bn) {
   group(best, &g);
 }
 static int conv_like(const Pack& act, const Pack& filt, int ch_in, int ch_out, int frame_h, int frame_w, float* out, const TapList& taps,
-                     const OutGeom& og, double flops, cudaStream_t s, const char* what, int* oom) {
+                     const OutGeom& og, double flops, cudaStream_t s, const char* what, int* oom, AmaxOut* track) {
   GemmParams g;
   memset(&g, 0, sizeof(g));
   const int ar = act.arith, bk = bk_of(ar);
@@ -2275,6 +2379,10 @@ static int conv_like(const Pack& act, const Pack& filt, int ch_in, int ch_out, i
   g.a_scale = act.scale(); g.b_scale = filt.scale();
   g.frame_h = frame_h; g.frame_w = frame_w; g.valid_h = og.valid_h; g.valid_w = og.valid_w;
   g.out_c = ch_out; g.out_h = og.out_h; g.out_w = og.out_w; g.out_sh = og.out_sh; g.out_sw = og.out_sw; g.out_off_h = og.out_off_h; g.out_off_w = og.out_off_w;
+  if (track && ar == kArithF16 && g_pairs_mode == 0) {        // launches that write one output share the word
+    if (!track->word) *track = amax_track_begin(out);
+    g.amax = track->word; g.amax_clear = track->clear;
+  }
   if (pairs) return ar == kArithTF32 ? launch_gemm_pair<kArithTF32>(g, s, flops, what) : launch_gemm_pair<kArithF16>(g, s, flops, what);
   return launch_gemm_bn(bn, ar, g, s, flops, what, oom);
 }
@@ -2298,7 +2406,7 @@ int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cu
   if ((int64_t)t.N * t.C * t.H * t.W != n || x == y) return 0;
   const int ar = tensor_arithmetic();
   ConvTc* st = t.st;
-  const uint32_t* bound = ar == kArithF16 ? amax_tracked(x) : nullptr;
+  const uint32_t* bound = ar == kArithF16 ? bound_of(x) : nullptr;
   if (ar == kArithF16 && !bound) return 0;
   std::lock_guard<std::mutex> lk(st->mu);
   Pack& pk = st->x;
@@ -2313,6 +2421,27 @@ int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cu
   pk.src = y; pk.version = version_of(y); pk.tag = st->cls;
   tc_note_relu_output(node, y);
   g_fused_relu_packs.fetch_add(1, std::memory_order_relaxed);
+  return 1;
+}
+// ReLU backward (held back by its entry point) whose output is the dy of a convolution's backward call: out = mask > 0 ? dy : 0
+// and the plan's pack of it in one pass.  1 when it did that, 0 when the caller should run the ReLU on its own.
+int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, float* out, cudaStream_t s) {
+  static const bool on = [] { const char* e = getenv("TINYFLOW_FUSE_RELU_PACK"); return e ? atoi(e) != 0 : true; }();
+  ConvTc* st = conv_state(p);
+  if (!on || !st->cls || p->K < 16 || p->C < 16 || !encode_fn() || out == mask || out == dy) return 0;
+  const int ar = tensor_arithmetic();
+  const uint32_t* bound = ar == kArithF16 ? bound_of(dy) : nullptr;       // max|dy| >= max|out|
+  if (ar == kArithF16 && !bound) return 0;
+  std::lock_guard<std::mutex> lk(st->mu);
+  Pack& pk = st->dy;
+  int oom = 0;
+  if (pack_alloc(pk, ar, (long long)p->N * st->frame_h * st->frame_w, p->K, s, &oom)) return 0;
+  note_write(out);
+  const AmaxOut am = amax_track_begin(out);
+  note_compute_stream(s);
+  ScaleRef sr{bound, nullptr, reinterpret_cast<float*>(pk.words + 2)};
+  if (launch_pack_nchw(pk, sr, dy, p->N, p->K, p->P, p->Q, st->frame_h, st->frame_w, st->dy_off_h, st->dy_off_w, 1, 1, 0, (int)pk.pitch, s, out, am, mask)) return -1;
+  pk.src = out; pk.version = version_of(out); pk.tag = 2;
   return 1;
 }
 long long fused_relu_pack_count() { return g_fused_relu_packs.load(std::memory_order_relaxed); }
@@ -2332,7 +2461,9 @@ int tc_conv_fwd(ConvPlan* p, const float* x, const float* w, float* y, cudaStrea
       else taps.add(r * st->frame_w + q, 0, r * st->eS + q);
     }
   OutGeom og{p->P, p->Q, p->P, p->Q, 1, 1, 0, 0};
-  return tc_result(conv_like(st->x, st->wf, st->eC, p->K, st->frame_h, st->frame_w, y, taps, og, conv_flops(p), s, "DLGpuConvolution2DForward", oom));
+  AmaxOut track;
+  note_conv_output(y, &st->track_y);
+  return tc_result(conv_like(st->x, st->wf, st->eC, p->K, st->frame_h, st->frame_w, y, taps, og, conv_flops(p), s, "DLGpuConvolution2DForward", oom, st->track_y ? &track : nullptr));
 }
 
 int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaStream_t s, int* oom) {
@@ -2345,13 +2476,15 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
   if (pack_filter(st, ar, w, p, 1, false, s, oom)) return *oom ? 1 : -1;     // [C][flipped tap][K]; a no-op when forward made it
   const int ntap = p->R * p->S;
   int rc = 0;
+  AmaxOut track;
+  note_conv_output(dx, &st->track_dx);
   if (st->cls == 1) {
     // a strided 1x1 window reaches only every stride-th input position: the rest of dx is zero
     bool strided = p->stride_h > 1 || p->stride_w > 1;
     if (strided && cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)p->N * p->C * p->H * p->W, s) != cudaSuccess) return -1;
     TapList taps; taps.add(0, 0, 0);
     OutGeom og{p->P, p->Q, p->H, p->W, p->stride_h, p->stride_w, 0, 0};
-    rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom);
+    rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom, st->track_dx ? &track : nullptr);
   } else if (st->cls == 2) {
     TapList taps;
     // dx(h, w), anchored at frame position (h, w), reads dy(h - lo_h + r, w - lo_w + s) with lo = window - 1 - pad
@@ -2359,7 +2492,7 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
       for (int q = 0; q < p->S; ++q)
         taps.add((r - (p->R - 1 - p->pad_h) + st->dy_off_h) * st->frame_w + (q - (p->S - 1 - p->pad_w) + st->dy_off_w), 0, r * p->S + q);
     OutGeom og{p->H, p->W, p->H, p->W, 1, 1, 0, 0};
-    rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom);
+    rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom, st->track_dx ? &track : nullptr);
   } else {
     // One launch per stride phase (a, b): dx_padded(sh*u + a, sw*v + b) = sum over the taps r = sh*r' + a, s = sw*s' + b of
     // dy(u - r', v - s') * w(r, s); dy sits at frame offset (hh, hw), so the shift is (hh - r') rows and (hw - s') columns.
@@ -2373,7 +2506,7 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
             taps.add((st->dy_off_h - r / p->stride_h) * st->frame_w + (st->dy_off_w - q / p->stride_w), 0, ntap - 1 - (r * p->S + q));
         if (!taps.n) continue;      // no tap lands on this phase: it stays zero
         OutGeom og{st->frame_h, st->frame_w, p->H, p->W, p->stride_h, p->stride_w, a - p->pad_h, b - p->pad_w};
-        rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p) * taps.n / ntap, s, "DLGpuConvolutionBackwardData", oom);
+        rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p) * taps.n / ntap, s, "DLGpuConvolutionBackwardData", oom, st->track_dx ? &track : nullptr);
       }
   }
   return tc_result(rc);

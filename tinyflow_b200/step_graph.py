@@ -102,6 +102,8 @@ def record(executor, feed_dict, staged):
         return None
     values, loss, keep = {}, None, 0
     try:
+        params = gpu_op.handle_array([v for n, v in feed_dict.items() if n.isw == 1])
+        check_call(_LIB.TfPackFilters(params, len(params), stream))
         values, loss = executor._issue(feed_dict, stream, recording=True)
         keep = 1
     except Exception:                           # whatever stopped it: the ordinary step that follows reports it
