@@ -16,7 +16,7 @@ pytestmark = pytest.mark.gpu
     (12, 64, 42, 42, 64, 3, 3, "SAME"),       # more tiles than SMs: filters stay in shared memory
     (13, 64, 40, 40, 256, 1, 1, "VALID"), (13, 248, 40, 41, 60, 1, 1, "VALID"),
     (2, 384, 8, 8, 384, 1, 3, "SAME"), (9, 1024, 4, 4, 96, 1, 1, "SAME"), (2, 512, 6, 6, 136, 3, 3, "SAME"), (5, 256, 17, 17, 160, 3, 3, "SAME"),    # few tiles: clusters of several sizes
-    (9, 36, 9, 9, 44, 5, 5, "SAME"), (9, 33 * 4, 9, 9, 68, 1, 7, "SAME"),        # filters: more taps than a block holds, ragged blocks
+    (9, 36, 9, 9, 44, 5, 5, "SAME"), (9, 33 * 4, 9, 9, 68, 1, 7, "SAME"), (4, 160, 12, 12, 64, 7, 1, "SAME"), (4, 320, 9, 9, 136, 1, 3, "SAME"),        # filters: more taps than a block holds, ragged blocks; gradients: taps of 3 and 5 half tiles
     (20, 512, 30, 30, 128, 3, 3, "SAME"),     # cross terms promoted twice in a tile
 ])
 @pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])

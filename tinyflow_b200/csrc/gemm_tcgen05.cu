@@ -403,7 +403,9 @@ struct alignas(64) GemmParams {
   // rows with i >= valid_h, j >= valid_w or (oi, oj) outside the plane are dropped
   int frame_h, frame_w, valid_h, valid_w, out_c, out_h, out_w, out_sh, out_sw, out_off_h, out_off_w;
   int* err;                       // device-visible error word (mapped host memory)
-  int slot, taps_per_tile;        // kModeWgrad: M-tile rows are taps_per_tile slots of `slot` input channels, one filter tap per slot
+  // kModeWgrad: M-tile rows are taps_per_tile slots of `slot` input channels of one filter tap each.  slots_per_tap > 1: a tap takes that
+  // many slots in a row, and m_tiles is 1
+  int slot, taps_per_tile, slots_per_tap;
   int group_iters;                // stages accumulated in TMEM before the epilogue promotes them to registers
   int data_by_data;               // both operands are activations / gradients (filter gradients, X^T dY): host-side hint for group_iters
   // Shared memory: a ring of A blocks and a ring of B tiles.  A filter's taps read the same rows of the activation matrix
@@ -493,7 +495,8 @@ __device__ __forceinline__ RowAddr row_address(const GemmParams& p, int mt, int 
     r.col_stride = (uint32_t)(p.out_h * p.out_w);
     r.base = ((long long)img * p.out_c) * r.col_stride + (long long)oi * p.out_w + oj;
   } else {   // kEpiWgrad: tile row -> (tap slot, input channel c), column n = output channel: out[(n * C + c) * ntaps + tap]
-    const int sl = row_in_tile / p.slot, c = mt * p.slot + row_in_tile - sl * p.slot, t = tap * p.taps_per_tile + sl;
+    const int sl = row_in_tile / p.slot, u = tap * p.taps_per_tile + sl, t = u / p.slots_per_tap;
+    const int c = (mt + u - t * p.slots_per_tap) * p.slot + row_in_tile - sl * p.slot;
     r.ok = t < p.ntaps && c < p.M;
     r.base = (long long)c * p.ntaps + t;
     r.col_stride = (uint32_t)(p.M * p.ntaps);
@@ -624,6 +627,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
         const int m0 = mt * BM, n0 = nt * BN;
         int ch = w.k0 / period, ti = w.k0 - ch * period;
         int left = p.group_iters;         // stages to the next accumulator group
+        int slot_off[2] = {0, 0}, slot_grp[2] = {0, 0};       // kModeWgrad: row shift and column group of the tile's slots
+        if (p.mode == kModeWgrad && do_a) {
+#pragma unroll
+          for (int sl = 0; sl < 2; ++sl) {
+            const int u = tap * p.taps_per_tile + sl, t = u / p.slots_per_tap, cb = mt + u - t * p.slots_per_tap;
+            slot_off[sl] = t < p.ntaps ? p.tap_off[t] : 0x40000000;
+            slot_grp[sl] = (cb * p.slot + (t < p.ntaps ? p.tap_col[t] : 0)) / T::kGW;
+          }
+        }
         for (int it = 0; it < w.kcount; ++it) {
           const int git = w.k0 + it;                  // stage index within the tile's reduction
           const uint32_t word = conv ? words.at(ti) : 0x300u, tc = conv ? cols.at(ti) : 0u;
@@ -651,12 +663,12 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
                 // [groups][BK rows][128 B], the layout the M/N-major descriptor expects.  One copy per tap slot; a slot past
                 // the last tap reads rows beyond the pack (the copy still completes with its full byte count and fills zeros).
                 const int gps = p.slot / T::kGW;
-                for (int sl = 0; sl < p.taps_per_tile; ++sl) {
-                  const int t = tap * p.taps_per_tile + sl;
-                  const int row = t < p.ntaps ? git * BK + p.tap_off[t] : 0x40000000;
-                  const int grp = (mt * p.slot + (t < p.ntaps ? p.tap_col[t] : 0)) / T::kGW;
-                  tma_load_3d(a_hi + sl * gps * kGroupStride, &p.a_hi, 0, row, grp, bar);
-                  tma_load_3d(a_lo + sl * gps * kGroupStride, &p.a_lo, 0, row, grp, bar);
+#pragma unroll
+                for (int sl = 0; sl < 2; ++sl) {
+                  if (sl == p.taps_per_tile) break;
+                  const int row = slot_off[sl] < 0x40000000 ? git * BK + slot_off[sl] : 0x40000000;
+                  tma_load_3d(a_hi + sl * gps * kGroupStride, &p.a_hi, 0, row, slot_grp[sl], bar);
+                  tma_load_3d(a_lo + sl * gps * kGroupStride, &p.a_lo, 0, row, slot_grp[sl], bar);
                 }
               } else if (p.a_mn) {
                 tma_load_3d(a_hi, &p.a_hi, 0, git * BK, m0 / T::kGW, bar);
@@ -2551,16 +2563,20 @@ int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaS
   g.M = st->eC; g.N = p->K; g.ntaps = st->eR * st->eS;
   // Few input channels: two filter taps share one 128-row tile (slots of 64 channels), so that the tensor core's
   // M dimension is full and dy is read once for both.
-  g.slot = st->eC > 64 ? BM : 64;
+  // So do an odd number of 64-channel blocks of a filter with several taps: 160 channels in 7 taps are 21 blocks in 11 tiles, where
+  // whole tiles per tap are 14.
+  const int blocks64 = (st->eC + 63) / 64;
+  g.slot = blocks64 % 2 == 0 || (blocks64 > 1 && g.ntaps == 1) ? BM : 64;
   g.taps_per_tile = BM / g.slot;
+  g.slots_per_tap = g.slot == BM ? 1 : blocks64;
   int rc = make_map_mn(&g.a_hi, ar, st->x.hi, st->x.rows, st->x.pitch, g.slot);
   if (!rc) rc = make_map_mn(&g.a_lo, ar, st->x.lo, st->x.rows, st->x.pitch, g.slot);
   if (!rc) rc = make_map_mn(&g.b_hi, ar, st->dy.hi, st->dy.rows, st->dy.pitch, bn);
   if (!rc) rc = make_map_mn(&g.b_lo, ar, st->dy.lo, st->dy.rows, st->dy.pitch, bn);
   if (rc) return -1;
   g.a_scale = st->x.scale(); g.b_scale = st->dy.scale();
-  g.m_tiles = (st->eC + g.slot - 1) / g.slot;
-  g.tap_tiles = (g.ntaps + g.taps_per_tile - 1) / g.taps_per_tile;
+  g.m_tiles = g.slots_per_tap > 1 ? 1 : (st->eC + g.slot - 1) / g.slot;
+  g.tap_tiles = (g.ntaps * g.slots_per_tap + g.taps_per_tile - 1) / g.taps_per_tile;
   g.n_tiles = (p->K + bn - 1) / bn;
   // dy row m' holds output pixel (p, q) at frame position (p + dy_off_h, q + dy_off_w); tap (r, s) needs the padded
   // input at (p + r, q + s), which sits at frame row m' + (r - dy_off_h) * frame_w + (s - dy_off_w)
