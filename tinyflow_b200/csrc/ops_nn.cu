@@ -177,12 +177,12 @@ __global__ void __launch_bounds__(256) pool_bwd_gather_kernel(const int32_t* __r
     dx[i] = acc * scale;
   }
 }
-// Max-pool gradient for 3x3 windows, stride 2, no padding (the ResNet / Inception stem pools): one thread per 2x2
-// block of dx.  The four elements share their candidate windows (p in {a-1, a}, q in {b-1, b}), so the four index / dy
+// Max-pool gradient for 3x3 windows, stride 2, padding 0 or 1 (the stem pools of ResNet, Inception and DenseNet): one thread per 2x2
+// block of dx.  The four elements share their candidate windows (p in {a-1, a} + padding, q alike), so the four index / dy
 // pairs are loaded once instead of 2.25 times per element; contributions are added in the same (p, q) order as the
 // general gather, so the result is bit-identical to it.
 __global__ void __launch_bounds__(256) maxpool_bwd_3x3s2_kernel(const int32_t* __restrict__ idx, const float* __restrict__ dy, float* __restrict__ dx,
-                                                                int64_t blocks_total, int H, int W, int P, int Q, FastDiv dAB, FastDiv dB) {
+                                                                int64_t blocks_total, int H, int W, int P, int Q, int ph, int pw, FastDiv dAB, FastDiv dB) {
   grid_dep_sync();
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int PQ = P * Q, HW = H * W;
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_3x3s2_kernel(const int32_t* _
     int id[4]; float v[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-      const int p = a - 1 + (k >> 1), q = b - 1 + (k & 1);
+      const int p = a - 1 + ph + (k >> 1), q = b - 1 + pw + (k & 1);
       const bool ok = (unsigned)p < (unsigned)P && (unsigned)q < (unsigned)Q;
       id[k] = ok ? __ldg(ip + p * Q + q) : -1;
       v[k] = ok ? __ldg(dp + p * Q + q) : 0.f;
@@ -293,6 +293,60 @@ __global__ void __launch_bounds__(256) avgpool_fwd_kernel(const float* __restric
   amax_commit(am, amax);
 }
 
+// Mean over 3x3 windows, stride 1, padding 1 (the pooling branch of the Inception modules): forward, and backward, which is the same
+// sum over dy.  A block holds a few whole planes in shared memory (they are small and lie one after the other, so they come in as
+// float4) and a thread slides down four rows of a column: 18 shared loads for four results, where nine loads and an index division
+// per result kept the L1 busy at a quarter of the memory rate.  HBM-bound.  Planes up to 2048 elements: four of them
+// have to fit beside other blocks (and four keep the chunks of 16 bytes aligned).
+constexpr int kMean3Rows = 4, kMean3Floats = 6144, kMean3MaxPlane = 2048;
+__global__ void __launch_bounds__(256) mean3_kernel(const float* __restrict__ x, float* __restrict__ y, int64_t planes, int group, int H, int W, FastDiv dItems, FastDiv dW, float scale, AmaxOut am) {
+  extern __shared__ float4 mean3_smem[];
+  grid_dep_sync();
+  float* s = reinterpret_cast<float*>(mean3_smem);
+  const int64_t first = (int64_t)blockIdx.x * group;
+  const int n = (int)min((int64_t)group, planes - first), HW = H * W, count = n * HW;
+  const float* src = x + first * HW;
+  float* dst = y + first * HW;
+  for (int i = threadIdx.x; i < count >> 2; i += 256) mean3_smem[i] = __ldg(reinterpret_cast<const float4*>(src) + i);
+  for (int i = (count & ~3) + threadIdx.x; i < count; i += 256) s[i] = __ldg(src + i);
+  __syncthreads();
+  uint32_t top = 0;
+  for (int it = threadIdx.x; it < n * (int)dItems.d; it += 256) {
+    const int plane = dItems.div(it), rem = it - plane * dItems.d, seg = dW.div(rem), w = rem - seg * W, h0 = seg * kMean3Rows;
+    const float* sp = s + plane * HW + w;
+    const bool left = w > 0, right = w + 1 < W;
+    auto row = [&](int h) {
+      if (h < 0 || h >= H) return 0.f;
+      const float* r = sp + h * W;
+      return ((left ? r[-1] : 0.f) + r[0]) + (right ? r[1] : 0.f);
+    };
+    float above = row(h0 - 1), here = row(h0);
+    float* out = dst + plane * HW + h0 * W + w;
+#pragma unroll
+    for (int k = 0; k < kMean3Rows; ++k) {
+      if (h0 + k >= H) break;
+      const float below = row(h0 + k + 1), v = (above + here + below) * scale;
+      out[k * W] = v;
+      top = max(top, amax_bits(v));
+      above = here; here = below;
+    }
+  }
+  amax_commit(am, top);
+}
+static bool mean3_fits(const PoolPlan* p, const float* in) {
+  return p->win_h == 3 && p->win_w == 3 && p->stride_h == 1 && p->stride_w == 1 && p->pad_h == 1 && p->pad_w == 1 && p->P == p->H && p->Q == p->W &&
+         p->H * p->W <= kMean3MaxPlane && (reinterpret_cast<uintptr_t>(in) & 15) == 0;
+}
+static void launch_mean3(const PoolPlan* p, const float* in, float* out, cudaStream_t s, AmaxOut am) {
+  const int HW = p->H * p->W;
+  const int64_t planes = (int64_t)p->N * p->C;
+  int group = std::max(4, kMean3Floats / HW / 4 * 4);
+  while (group > 4 && planes / group < 2 * device_sm_count()) group -= 4;          // small batches: more blocks
+  FastDiv dItems, dW;
+  dItems.init((uint32_t)((p->H + kMean3Rows - 1) / kMean3Rows * p->W)); dW.init((uint32_t)p->W);
+  launch_dep(mean3_kernel, dim3((unsigned)((planes + group - 1) / group)), dim3(256), (size_t)group * HW * 4, s, in, out, planes, group, p->H, p->W, dItems, dW, 1.f / 9.f, am);
+}
+
 static PoolGeom geom_of(const PoolPlan* p) {
   PoolGeom g;
   g.C = p->C; g.H = p->H; g.W = p->W; g.P = p->P; g.Q = p->Q;
@@ -313,13 +367,13 @@ static void launch_maxpool_fwd(const PoolPlan* p, const float* x, float* y, int3
 }
 template <bool MAXPOOL> static void launch_pool_gather(const PoolPlan* p, const int32_t* idx, const float* dy, float* dx, int64_t total, float scale, cudaStream_t s) {
   PoolGeom g = geom_of(p);
-  if (MAXPOOL && p->win_h == 3 && p->win_w == 3 && p->stride_h == 2 && p->stride_w == 2 && p->pad_h == 0 && p->pad_w == 0 &&
+  if (MAXPOOL && p->win_h == 3 && p->win_w == 3 && p->stride_h == 2 && p->stride_w == 2 && p->pad_h <= 1 && p->pad_w <= 1 &&
       (reinterpret_cast<uintptr_t>(dx) & 7) == 0) {
     const int A = (p->H + 1) / 2, B = (p->W + 1) / 2;
     const int64_t blocks = (int64_t)p->N * p->C * A * B;
     FastDiv dAB, dB;
     dAB.init((uint32_t)(A * B)); dB.init((uint32_t)B);
-    launch_dep(maxpool_bwd_3x3s2_kernel, dim3(grid_for(blocks, 256)), dim3(256), 0, s, idx, dy, dx, blocks, p->H, p->W, p->P, p->Q, dAB, dB);
+    launch_dep(maxpool_bwd_3x3s2_kernel, dim3(grid_for(blocks, 256)), dim3(256), 0, s, idx, dy, dx, blocks, p->H, p->W, p->P, p->Q, p->pad_h, p->pad_w, dAB, dB);
     return;
   }
   if (MAXPOOL && p->win_h == 2 && p->win_w == 2 && p->stride_h == 2 && p->stride_w == 2 && p->pad_h == 0 && p->pad_w == 0 &&
@@ -703,7 +757,8 @@ int DLGpuPooling2DForward(const DLArrayHandle input, DLArrayHandle output, void*
   else {
     float* y = out_f32(output);
     AmaxOut am = amax_track_begin(y);
-    if (p->win_h == 3 && p->win_w == 3) launch_dep(avgpool_fwd_kernel<3, 3>, dim3(grid_for(total, 256)), dim3(256), 0, s, (const float*)input->data, y, total, geom_of(p), am);
+    if (mean3_fits(p, (const float*)input->data)) launch_mean3(p, (const float*)input->data, y, s, am);
+    else if (p->win_h == 3 && p->win_w == 3) launch_dep(avgpool_fwd_kernel<3, 3>, dim3(grid_for(total, 256)), dim3(256), 0, s, (const float*)input->data, y, total, geom_of(p), am);
     else launch_dep(avgpool_fwd_kernel<0, 0>, dim3(grid_for(total, 256)), dim3(256), 0, s, (const float*)input->data, y, total, geom_of(p), am);
   }
   TF_AFTER(s, "DLGpuPooling2DForward");
@@ -726,6 +781,7 @@ int DLGpuPooling2DBackward(const DLArrayHandle input, const DLArrayHandle output
     else
       maxpool_bwd_kernel<<<grid_for(total, 256), 256, 0, s>>>((const float*)input->data, (const float*)doutput->data, out_f32(dinput), total, geom_of(p));
   }
+  else if (mean3_fits(p, (const float*)doutput->data)) launch_mean3(p, (const float*)doutput->data, out_f32(dinput), s, AmaxOut{});
   else launch_pool_gather<false>(p, nullptr, (const float*)doutput->data, out_f32(dinput), total, 1.f / (float)(p->win_h * p->win_w), s);
   TF_AFTER(s, "DLGpuPooling2DBackward");
   return 0;
