@@ -2078,7 +2078,9 @@ struct ConvTc {
   const float* filter = nullptr;                         // the array the filter packs were last made from, and its plan
   const ConvPlan* plan = nullptr;
   Pack x, dy, wf, wd;
+  ConvTc* x_owner = this;                                // whose x pack the plan reads: another plan's of the same recorded step, or its own
   std::mutex mu;
+  const Pack& x_pack() const { return x_owner->x; }
 };
 static ConvTc* conv_state(ConvPlan* p) {
   if (!p->tc_state) {
@@ -2194,9 +2196,34 @@ static void remember_pack_target(const void* x, uint64_t ver, ConvTc* st, const 
   if (it != g_relu_writer.end() && it->second.version == ver) g_pack_targets[it->second.node] = PackTarget{st, p->N, p->C, p->H, p->W};
 }
 
+// Inside a recorded step the branches of a module read one pack of their common input: convolutions whose frames agree (1x1 windows
+// of any filter count, equal windows) find the pack an earlier one has made.  Only inside one recording: its launches
+// run in one order on one stream, so a pack that was valid when it was recorded is valid at every replay, and plans of a step are
+// not used by two threads at once.  (A pack written by a ReLU is not offered: its scale comes from a bound, and a replayed step
+// keeps the bits of the ordinary one.)
+struct SharedPack { const float* x; ConvTc* st; int N, C, H, W, sh, sw; };
+static thread_local std::vector<SharedPack> t_shared_packs;
+void tc_recording_begins() { t_shared_packs.clear(); }
+static void offer_pack(const float* x, ConvTc* st, int N, int C, int H, int W, int sh, int sw) {
+  if (t_recording) t_shared_packs.push_back(SharedPack{x, st, N, C, H, W, sh, sw});
+}
+static ConvTc* find_shared_pack(const ConvTc* st, int ar, const ConvPlan* p, const float* x, uint64_t ver, long long rows, long long cols) {
+  if (!t_recording) return nullptr;
+  for (const SharedPack& e : t_shared_packs) {
+    ConvTc* o = e.st;
+    if (e.x != x || o == st || e.N != p->N || e.C != p->C || e.H != p->H || e.W != p->W || e.sh != p->stride_h || e.sw != p->stride_w) continue;
+    if (o->cls != st->cls || o->frame_h != st->frame_h || o->frame_w != st->frame_w || o->x_off_h != st->x_off_h || o->x_off_w != st->x_off_w || !o->mu.try_lock()) continue;
+    const bool ok = pack_valid(o->x, ar, x, ver, o->cls, rows, cols);
+    o->mu.unlock();
+    if (ok) return o;
+  }
+  return nullptr;
+}
+
 // the x operand of a plan: frame pack (classes A, B), patch matrix (class C) or one frame per stride phase (class D)
 static int pack_x(ConvTc* st, int ar, const ConvPlan* p, const float* x, cudaStream_t s, int* oom) {
   Pack& pk = st->x;
+  st->x_owner = st;
   const uint64_t ver = version_of(x);
   const long long n_src = (long long)p->N * p->C * p->H * p->W;
   if (st->cls == 3) {
@@ -2218,6 +2245,8 @@ static int pack_x(ConvTc* st, int ar, const ConvPlan* p, const float* x, cudaStr
   const int phases = st->cls == 4 ? p->stride_h * p->stride_w : 1;
   const long long cols = st->cls == 4 ? (long long)phases * st->cp : p->C;
   if (pack_valid(pk, ar, x, ver, st->cls, rows, cols)) return 0;
+  if (st->cls == 1 || st->cls == 2)
+    if (ConvTc* o = find_shared_pack(st, ar, p, x, ver, rows, cols)) { st->x_owner = o; return 0; }
   if (pack_alloc(pk, ar, rows, cols, s, oom)) return 1;
   ScaleRef sr = begin_pack(pk, x, n_src, s);
   int rc = 0;
@@ -2233,6 +2262,7 @@ static int pack_x(ConvTc* st, int ar, const ConvPlan* p, const float* x, cudaStr
   }
   if (rc) return -1;
   pk.src = x; pk.version = ver; pk.tag = st->cls;
+  if (st->cls == 1 || st->cls == 2) offer_pack(x, st, p->N, p->C, p->H, p->W, p->stride_h, p->stride_w);
   if ((st->cls == 1 || st->cls == 2) && p->stride_h == 1 && p->stride_w == 1) remember_pack_target(x, ver, st, p);
   return 0;
 }
@@ -2475,7 +2505,7 @@ int tc_conv_fwd(ConvPlan* p, const float* x, const float* w, float* y, cudaStrea
   OutGeom og{p->P, p->Q, p->P, p->Q, 1, 1, 0, 0};
   AmaxOut track;
   note_conv_output(y, &st->track_y);
-  return tc_result(conv_like(st->x, st->wf, st->eC, p->K, st->frame_h, st->frame_w, y, taps, og, conv_flops(p), s, "DLGpuConvolution2DForward", oom, st->track_y ? &track : nullptr));
+  return tc_result(conv_like(st->x_pack(), st->wf, st->eC, p->K, st->frame_h, st->frame_w, y, taps, og, conv_flops(p), s, "DLGpuConvolution2DForward", oom, st->track_y ? &track : nullptr));
 }
 
 int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaStream_t s, int* oom) {
@@ -2547,10 +2577,10 @@ int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaS
       g.mode = kModeGemm; g.a_mn = 1; g.b_mn = 1; g.epi = kEpiRowMajor;
       int rc = make_map_mn(&g.a_hi, ar, st->dy.hi, st->dy.rows, st->dy.pitch, BM);
       if (!rc) rc = make_map_mn(&g.a_lo, ar, st->dy.lo, st->dy.rows, st->dy.pitch, BM);
-      if (!rc) rc = make_map_mn(&g.b_hi, ar, st->x.hi, st->x.rows, st->x.pitch, bn);
-      if (!rc) rc = make_map_mn(&g.b_lo, ar, st->x.lo, st->x.rows, st->x.pitch, bn);
+      if (!rc) rc = make_map_mn(&g.b_hi, ar, st->x_pack().hi, st->x_pack().rows, st->x_pack().pitch, bn);
+      if (!rc) rc = make_map_mn(&g.b_lo, ar, st->x_pack().lo, st->x_pack().rows, st->x_pack().pitch, bn);
       if (rc) return -1;
-      g.a_scale = st->dy.scale(); g.b_scale = st->x.scale();
+      g.a_scale = st->dy.scale(); g.b_scale = st->x_pack().scale();
       g.M = p->K; g.N = st->eC; g.ldc = st->eC;
       g.m_tiles = (p->K + BM - 1) / BM; g.n_tiles = (st->eC + bn - 1) / bn; g.tap_tiles = 1; g.ntaps = 1;
       g.k_total = kit;
@@ -2569,12 +2599,12 @@ int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaS
   g.slot = blocks64 % 2 == 0 || (blocks64 > 1 && g.ntaps == 1) ? BM : 64;
   g.taps_per_tile = BM / g.slot;
   g.slots_per_tap = g.slot == BM ? 1 : blocks64;
-  int rc = make_map_mn(&g.a_hi, ar, st->x.hi, st->x.rows, st->x.pitch, g.slot);
-  if (!rc) rc = make_map_mn(&g.a_lo, ar, st->x.lo, st->x.rows, st->x.pitch, g.slot);
+  int rc = make_map_mn(&g.a_hi, ar, st->x_pack().hi, st->x_pack().rows, st->x_pack().pitch, g.slot);
+  if (!rc) rc = make_map_mn(&g.a_lo, ar, st->x_pack().lo, st->x_pack().rows, st->x_pack().pitch, g.slot);
   if (!rc) rc = make_map_mn(&g.b_hi, ar, st->dy.hi, st->dy.rows, st->dy.pitch, bn);
   if (!rc) rc = make_map_mn(&g.b_lo, ar, st->dy.lo, st->dy.rows, st->dy.pitch, bn);
   if (rc) return -1;
-  g.a_scale = st->x.scale(); g.b_scale = st->dy.scale();
+  g.a_scale = st->x_pack().scale(); g.b_scale = st->dy.scale();
   g.m_tiles = g.slots_per_tap > 1 ? 1 : (st->eC + g.slot - 1) / g.slot;
   g.tap_tiles = (g.ntaps * g.slots_per_tap + g.taps_per_tile - 1) / g.taps_per_tile;
   g.n_tiles = (p->K + bn - 1) / bn;

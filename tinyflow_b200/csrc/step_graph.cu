@@ -19,6 +19,7 @@ thread_local StepGraph* t_recording = nullptr;
 static std::atomic<uint64_t> g_layout_epoch{1};
 void bump_layout_epoch() { g_layout_epoch.fetch_add(1, std::memory_order_relaxed); }
 int tensor_path_error();
+void tc_recording_begins();
 bool dp_active();
 
 constexpr int kZeroedWords = 12288;       // maxima of a step's tensors: one word per tracked write (Inception-v4: about 900)
@@ -112,6 +113,7 @@ int TfStepRecordBegin(void** graph, void** stream_cell) {
   }
   g->epoch = g_layout_epoch.load();
   t_recording = g;
+  tc_recording_begins();
   *graph = g;
   *stream_cell = (void*)g->stream;
   if (cudaMemsetAsync(g->words, 0, sizeof(uint32_t) * kZeroedWords, g->stream) != cudaSuccess) g->overflow = true;
