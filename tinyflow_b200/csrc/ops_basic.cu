@@ -423,38 +423,74 @@ template <int MODE> __global__ void __launch_bounds__(kBlock) loss_grad_kernel(c
 }
 
 // ---- concat along axis 1 ---------------------------------------------------------------
-// dst[n, off + j] = src[n, j] for j < src_inner; MODE 0 copies src -> dst slice, MODE 1 the
-// slice of dst -> src (the backward split).  Rows are n, `inner` counts floats per sample.
-// One grid row (blockIdx.y) per sample, so no per-element divide; V = float4 when both inner sizes and the offset
-// are multiples of 4 floats, else float.
+// whole[n, j] = a[n, j] for j < ia, b[n, j - ia] beyond (forward, one launch), and part[n, j] = whole[n, off + j] (the backward
+// split).  Rows are n, the sizes count floats per sample.  One grid row (blockIdx.y) per sample, so no per-element divide;
+// V = float4 when all sizes and offsets are multiples of 4 floats, else float.  HBM-bound; kCopyUnroll independent loads a
+// thread, because one at a time left the small tensors of a late module waiting for memory.
 __device__ __forceinline__ uint32_t amax_of(const float4& v) { return amax4(0u, v); }
 __device__ __forceinline__ uint32_t amax_of(float v) { return amax_bits(v); }
-template <int MODE, typename V> __global__ void __launch_bounds__(kBlock) slice_copy_kernel(V* __restrict__ part, V* __restrict__ whole, int64_t nrows, int64_t part_inner, int64_t whole_inner, int64_t off, AmaxOut am) {
+constexpr int kCopyUnroll = 4;
+template <typename V> __global__ void __launch_bounds__(kBlock) concat_kernel(const V* __restrict__ a, const V* __restrict__ b, V* __restrict__ whole, int64_t nrows, int64_t ia, int64_t ib, AmaxOut am) {
   grid_dep_sync();
   uint32_t m = 0;
+  const int64_t inner = ia + ib;
   for (int64_t r = blockIdx.y; r < nrows; r += gridDim.y) {
-    V* p = part + r * part_inner;
-    V* w = whole + r * whole_inner + off;
-    for (int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; j < part_inner; j += (int64_t)gridDim.x * blockDim.x) {
-      V v = MODE == 0 ? p[j] : w[j];
-      if (MODE == 0) w[j] = v; else p[j] = v;
-      m = max(m, amax_of(v));
+    const V *pa = a + r * ia, *pb = b + r * ib - ia;
+    V* w = whole + r * inner;
+    for (int64_t j0 = (int64_t)blockIdx.x * (kBlock * kCopyUnroll) + threadIdx.x; j0 < inner; j0 += (int64_t)gridDim.x * (kBlock * kCopyUnroll)) {
+      V v[kCopyUnroll];
+#pragma unroll
+      for (int k = 0; k < kCopyUnroll; ++k) {
+        const int64_t j = j0 + k * kBlock;
+        if (j < inner) v[k] = j < ia ? pa[j] : pb[j];
+      }
+#pragma unroll
+      for (int k = 0; k < kCopyUnroll; ++k) {
+        const int64_t j = j0 + k * kBlock;
+        if (j < inner) { w[j] = v[k]; m = max(m, amax_of(v[k])); }
+      }
     }
   }
   amax_commit(am, m);
 }
-// `am` accumulates max|copied values| for the written tensor; a tensor written by two launches (concat forward)
-// passes the clear word to the first launch only.
-template <int MODE> static void launch_slice_copy(float* part, float* whole, int64_t rows, int64_t part_inner, int64_t whole_inner, int64_t off, cudaStream_t s, AmaxOut am) {
+template <typename V> __global__ void __launch_bounds__(kBlock) slice_kernel(V* __restrict__ part, const V* __restrict__ whole, int64_t nrows, int64_t part_inner, int64_t whole_inner, int64_t off, AmaxOut am) {
+  grid_dep_sync();
+  uint32_t m = 0;
+  for (int64_t r = blockIdx.y; r < nrows; r += gridDim.y) {
+    V* p = part + r * part_inner;
+    const V* w = whole + r * whole_inner + off;
+    for (int64_t j0 = (int64_t)blockIdx.x * (kBlock * kCopyUnroll) + threadIdx.x; j0 < part_inner; j0 += (int64_t)gridDim.x * (kBlock * kCopyUnroll)) {
+      V v[kCopyUnroll];
+#pragma unroll
+      for (int k = 0; k < kCopyUnroll; ++k) if (j0 + k * kBlock < part_inner) v[k] = w[j0 + k * kBlock];
+#pragma unroll
+      for (int k = 0; k < kCopyUnroll; ++k)
+        if (j0 + k * kBlock < part_inner) { p[j0 + k * kBlock] = v[k]; m = max(m, amax_of(v[k])); }
+    }
+  }
+  amax_commit(am, m);
+}
+// blocks along a row: enough to cover it, no more than eight waves over all rows
+static dim3 copy_grid(int64_t rows, int64_t per_row) {
+  const int gy = (int)(rows < 65535 ? rows : 65535);
+  const int64_t want = (per_row + kBlock * kCopyUnroll - 1) / (kBlock * kCopyUnroll), cap = (int64_t)8 * device_sm_count() / gy + 1;
+  return dim3((unsigned)std::max<int64_t>(1, std::min(want, cap)), gy);
+}
+static void launch_concat(const float* a, const float* b, float* whole, int64_t rows, int64_t ia, int64_t ib, cudaStream_t s) {
+  if (rows <= 0 || ia + ib <= 0) return;
+  const AmaxOut am = amax_track_begin(whole);
+  if (ia % 4 == 0 && ib % 4 == 0 && aligned16(a) && aligned16(b) && aligned16(whole))
+    launch_dep(concat_kernel<float4>, copy_grid(rows, (ia + ib) / 4), dim3(kBlock), 0, s, (const float4*)a, (const float4*)b, (float4*)whole, rows, ia / 4, ib / 4, am);
+  else
+    launch_dep(concat_kernel<float>, copy_grid(rows, ia + ib), dim3(kBlock), 0, s, a, b, whole, rows, ia, ib, am);
+}
+static void launch_slice(float* part, const float* whole, int64_t rows, int64_t part_inner, int64_t whole_inner, int64_t off, cudaStream_t s) {
   if (rows <= 0 || part_inner <= 0) return;
-  bool vec = part_inner % 4 == 0 && whole_inner % 4 == 0 && off % 4 == 0 && ((uintptr_t)part % 16 == 0) && ((uintptr_t)whole % 16 == 0);
-  int64_t per_row = vec ? part_inner / 4 : part_inner;
-  int gy = (int)(rows < 65535 ? rows : 65535);
-  int64_t want = (per_row + kBlock - 1) / kBlock, cap = (int64_t)8 * 148 / gy + 1;
-  int gx = (int)(want < cap ? want : cap);
-  dim3 grid(gx < 1 ? 1 : gx, gy);
-  if (vec) launch_dep(slice_copy_kernel<MODE, float4>, grid, dim3(kBlock), 0, s, (float4*)part, (float4*)whole, rows, part_inner / 4, whole_inner / 4, off / 4, am);
-  else launch_dep(slice_copy_kernel<MODE, float>, grid, dim3(kBlock), 0, s, part, whole, rows, part_inner, whole_inner, off, am);
+  const AmaxOut am = amax_track_begin(part);
+  if (part_inner % 4 == 0 && whole_inner % 4 == 0 && off % 4 == 0 && aligned16(part) && aligned16(whole))
+    launch_dep(slice_kernel<float4>, copy_grid(rows, part_inner / 4), dim3(kBlock), 0, s, (float4*)part, (const float4*)whole, rows, part_inner / 4, whole_inner / 4, off / 4, am);
+  else
+    launch_dep(slice_kernel<float>, copy_grid(rows, part_inner), dim3(kBlock), 0, s, part, whole, rows, part_inner, whole_inner, off, am);
 }
 
 // ---- dropout: counter-based keep mask ---------------------------------------------------
@@ -1164,13 +1200,9 @@ int DLGpuConcatForward(const DLArrayHandle input1, const DLArrayHandle input2, D
   TF_REQUIRE(output && numel(output) == rows * (ia + ib), "DLGpuConcatForward: output size mismatch");
   cudaStream_t s = stream_of(cudaStream);
   note_compute_stream(s);
-  KernelTimer kt("DLGpuConcatForward", s, 0, 8.0 * rows * (ia + ib), 2);
-  float* whole = FM(output);
-  AmaxOut am = (rows > 0 && ia > 0 && ib > 0) ? amax_track_begin(whole) : AmaxOut{};
-  launch_slice_copy<0>((float*)input1->data, whole, rows, ia, ia + ib, 0, s, am);
-  am.clear = nullptr;
-  launch_slice_copy<0>((float*)input2->data, whole, rows, ib, ia + ib, ia, s, am);
-  if (after_launch(s, "DLGpuConcatForward", 2) != 0) return -1;
+  KernelTimer kt("DLGpuConcatForward", s, 0, 8.0 * rows * (ia + ib));
+  launch_concat(F(input1), F(input2), FM(output), rows, ia, ib, s);
+  TF_AFTER(s, "DLGpuConcatForward");
   return 0;
 }
 int DLGpuConcataBackward(const DLArrayHandle input1, const DLArrayHandle input2, const DLArrayHandle doutput, DLArrayHandle dinput1, void** cudaStream) {
@@ -1180,8 +1212,7 @@ int DLGpuConcataBackward(const DLArrayHandle input1, const DLArrayHandle input2,
   cudaStream_t s = stream_of(cudaStream);
   note_compute_stream(s);
   KernelTimer kt("DLGpuConcatBackward", s, 0, 8.0 * rows * ia);
-  float* part = FM(dinput1);
-  launch_slice_copy<1>(part, (float*)doutput->data, rows, ia, ia + ib, 0, s, (rows > 0 && ia > 0) ? amax_track_begin(part) : AmaxOut{});
+  launch_slice(FM(dinput1), F(doutput), rows, ia, ia + ib, 0, s);
   TF_AFTER(s, "DLGpuConcataBackward");
   return 0;
 }
@@ -1192,8 +1223,7 @@ int DLGpuConcatbBackward(const DLArrayHandle input1, const DLArrayHandle input2,
   cudaStream_t s = stream_of(cudaStream);
   note_compute_stream(s);
   KernelTimer kt("DLGpuConcatBackward", s, 0, 8.0 * rows * ib);
-  float* part = FM(dinput2);
-  launch_slice_copy<1>(part, (float*)doutput->data, rows, ib, ia + ib, ia, s, (rows > 0 && ib > 0) ? amax_track_begin(part) : AmaxOut{});
+  launch_slice(FM(dinput2), F(doutput), rows, ib, ia + ib, ia, s);
   TF_AFTER(s, "DLGpuConcatbBackward");
   return 0;
 }
