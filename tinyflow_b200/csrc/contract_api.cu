@@ -31,7 +31,7 @@ int tensor_path_error();
 void tensor_path_error_clear();
 int tensor_path_timeout_probe(long long limit_cycles, cudaStream_t s);
 long long fused_relu_pack_count();
-int tc_pack_filters(const void* const* arrays, int n, cudaStream_t s);
+int tc_pack_filters(const void* const* arrays, const int64_t* sizes, int n, cudaStream_t s);
 int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, float* out, cudaStream_t s);
 // which engine served this thread's most recent contraction: 1 = CUDA cores, 2 = tensor cores (0 = none yet)
 static thread_local int t_last_path = 0;
@@ -57,8 +57,10 @@ int TfPackFilters(const DLArrayHandle* arrays, int n, void** cudaStream) {
   TF_REQUIRE(arrays && n >= 0, "TfPackFilters: null argument");
   if (!t_recording) return 0;
   std::vector<const void*> data;
-  for (int i = 0; i < n; ++i) if (arrays[i] && arrays[i]->ctx.device_type == kGPU) data.push_back(arrays[i]->data);
-  return tc_pack_filters(data.data(), (int)data.size(), stream_of(cudaStream));
+  std::vector<int64_t> sizes;
+  for (int i = 0; i < n; ++i)
+    if (arrays[i] && arrays[i]->ctx.device_type == kGPU) { data.push_back(arrays[i]->data); sizes.push_back(numel(arrays[i])); }
+  return tc_pack_filters(data.data(), sizes.data(), (int)data.size(), stream_of(cudaStream));
 }
 int TfFusedReluPackCount(long long* count) { if (count) *count = fused_relu_pack_count(); return 0; }
 int TfFusedReluBnBackwardCount(long long* count) { if (count) *count = fused_relu_bn_bwd_count(); return 0; }

@@ -35,7 +35,6 @@
 #include <mutex>
 #include <type_traits>
 #include <unordered_map>
-#include <unordered_set>
 #include <vector>
 
 namespace tf {
@@ -1602,10 +1601,11 @@ struct FilterJob {
   float *scale_f, *scale_d;
   int K, C, taps, pad_f, pad_d, k_blocks, first_block;
 };
+// MAX is 1 or kFilterJobs: the table travels as a kernel parameter, and 13 KB of it cost a launch of one filter 10 us.
 constexpr int kFilterJobs = 128, kFilterTaps = 9, kFilterTile = 32;
-struct FilterJobs { int n; FilterJob job[kFilterJobs]; };
-template <class E>
-__global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant__ FilterJobs jobs) {
+template <int MAX> struct FilterJobs { int n; FilterJob job[MAX]; };
+template <class E, int MAX>
+__global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant__ FilterJobs<MAX> jobs) {
   grid_dep_sync();
   __shared__ float tile[kFilterTile][kFilterTile * kFilterTaps + 1];
   int lo = 0, hi = jobs.n - 1;
@@ -2067,6 +2067,7 @@ int tc_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_
 //   class D: strided windows: space-to-depth phases (see conv_state);
 //   class C: too few input channels for a per-tap reduction chunk: x is expanded into patches (C*R*S columns) and
 //            the problem runs as class A over C*R*S channels; forward and filter gradient only.
+constexpr size_t kFilterSets = 8;       // parameter sets a plan remembers: an executor keeps recordings of four
 struct ConvTc {
   int cls = 0;                 // 0 unsupported, 1 class A, 2 class B, 3 class C, 4 class D
   int frame_h = 0, frame_w = 0;                          // frame geometry shared by the x and dy packs
@@ -2075,7 +2076,7 @@ struct ConvTc {
   int cp = 0;                                            // class D: columns per stride phase (C rounded up to 64)
   bool dgrad_seen = false;                               // backward-data has run on this plan: forward also packs its filter layout
   bool track_y = false, track_dx = false;                // a ReLU asked for max|y| / max|dx|: the epilogue leaves it
-  const float* filter = nullptr;                         // the array the filter packs were last made from, and its plan
+  std::vector<const float*> filters;                     // arrays the filter packs were made from (the last kFilterSets), and the plan
   const ConvPlan* plan = nullptr;
   Pack x, dy, wf, wd;
   ConvTc* x_owner = this;                                // whose x pack the plan reads: another plan's of the same recorded step, or its own
@@ -2303,10 +2304,15 @@ static int filter_job(ConvTc* st, int ar, const float* w, const ConvPlan* p, int
     std::lock_guard<std::mutex> lk(g_filter_plans_mu);
     g_filter_plans.push_back(st);
   }
-  st->plan = p; st->filter = w;
+  st->plan = p;
+  auto& known = st->filters;
+  if (std::find(known.begin(), known.end(), w) == known.end()) {
+    if (known.size() == kFilterSets) known.erase(known.begin());
+    known.push_back(w);
+  }
   return 0;
 }
-static int launch_filter_jobs(FilterJobs& jobs, int ar, cudaStream_t s) {
+template <int MAX> static int launch_filter_jobs(FilterJobs<MAX>& jobs, int ar, cudaStream_t s) {
   int blocks = 0;
   double elems = 0;
   for (int i = 0; i < jobs.n; ++i) {
@@ -2317,7 +2323,7 @@ static int launch_filter_jobs(FilterJobs& jobs, int ar, cudaStream_t s) {
     elems += (double)j.K * j.C * j.taps;
   }
   KernelTimer kt("pack_filters", s, 0, elems * (4.0 + 4.0 * elem_of(ar)));
-  TF_CUDA(ar == kArithTF32 ? launch_dep(pack_filters_kernel<float>, dim3(blocks), dim3(256), 0, s, jobs) : launch_dep(pack_filters_kernel<__half>, dim3(blocks), dim3(256), 0, s, jobs));
+  TF_CUDA(ar == kArithTF32 ? launch_dep(pack_filters_kernel<float, MAX>, dim3(blocks), dim3(256), 0, s, jobs) : launch_dep(pack_filters_kernel<__half, MAX>, dim3(blocks), dim3(256), 0, s, jobs));
   TF_AFTER(s, "pack_filters");
   return 0;
 }
@@ -2326,30 +2332,36 @@ static int pack_filter(ConvTc* st, int ar, const float* w, const ConvPlan* p, in
   const Pack& pk = flip ? st->wd : st->wf;
   const int rows = flip ? st->eC : p->K, pad = (int)round_up(flip ? p->K : st->eC, 64);
   if (pack_valid(pk, ar, w, version_of(w), 10 + flip, rows, (long long)st->eR * st->eS * pad)) return 0;
-  FilterJobs one;
+  FilterJobs<1> one;
   one.n = 1;
   if (int rc = filter_job(st, ar, w, p, flip ? 2 : with_other ? 3 : 1, s, oom, &one.job[0])) return rc;
   return launch_filter_jobs(one, ar, s);
 }
-// While a step is recorded: the filters among `arrays` whose plans were last fed from them, all in one launch, ahead of the
-// convolutions that find them packed.  What it leaves out, or guesses wrong, the convolution packs when it comes up.
-int tc_pack_filters(const void* const* arrays, int n, cudaStream_t s) {
+// While a step is recorded: the filters among `arrays` (with their sizes) that a plan has been fed from, all in one launch, ahead of
+// the convolutions that find them packed.  What it leaves out, or guesses wrong, the convolution packs when it comes up.
+int tc_pack_filters(const void* const* arrays, const int64_t* sizes, int n, cudaStream_t s) {
   if (contraction_path_is_cuda_cores() || !encode_fn()) return 0;
   const int ar = tensor_arithmetic();
-  std::unordered_set<const void*> wanted(arrays, arrays + n);
+  std::unordered_map<const void*, int64_t> wanted;
+  for (int i = 0; i < n; ++i) wanted[arrays[i]] = sizes[i];
   std::vector<ConvTc*> plans;
   {
     std::lock_guard<std::mutex> lk(g_filter_plans_mu);
-    for (ConvTc* st : g_filter_plans) if (wanted.count(st->filter)) plans.push_back(st);
+    plans = g_filter_plans;
   }
-  FilterJobs jobs;
+  FilterJobs<kFilterJobs> jobs;
   jobs.n = 0;
   for (ConvTc* st : plans) {
     std::lock_guard<std::mutex> lk(st->mu);
-    const float* w = st->filter;
-    if (!wanted.count(w) || !st->wf.hi || st->wf.arith != ar || (ar == kArithF16 && !amax_tracked(w))) continue;
+    const ConvPlan* p = st->plan;
+    const float* w = nullptr;
+    for (const float* f : st->filters) {
+      auto it = wanted.find(f);
+      if (it != wanted.end() && it->second == (int64_t)p->K * p->C * p->R * p->S) w = f;
+    }
+    if (!w || !st->wf.hi || st->wf.arith != ar || (ar == kArithF16 && !amax_tracked(w))) continue;
     int oom = 0;
-    if (filter_job(st, ar, w, st->plan, st->dgrad_seen ? 3 : 1, s, &oom, &jobs.job[jobs.n])) continue;
+    if (filter_job(st, ar, w, p, st->dgrad_seen ? 3 : 1, s, &oom, &jobs.job[jobs.n])) continue;
     if (++jobs.n < kFilterJobs) continue;
     if (launch_filter_jobs(jobs, ar, s)) return -1;
     jobs.n = 0;
