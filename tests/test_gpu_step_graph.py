@@ -78,6 +78,11 @@ def _change_the_rate(step, model, ex, feed, x):
             node.learning_rate = 0.01
 
 
+def _overwrite_inputs_late(step, model, ex, feed, x):
+    if step >= 5:                                                    # the recording is made on a batch that nothing has rewritten
+        _overwrite_inputs(step, model, ex, feed, x)
+
+
 _held = []
 
 
@@ -109,6 +114,43 @@ def _hold_and_write_gradients(step, model, ex, feed, x):
 @pytest.mark.parametrize("name", ["mlp", "resnet50"])
 def test_what_a_caller_does_between_steps_reaches_the_replay(lib_path, monkeypatch, name, between):
     _same(_train(monkeypatch, True, BUILDS[name], "sgd", between), _train(monkeypatch, False, BUILDS[name], "sgd", between))
+
+
+# Graphs whose first node is a tensor-path convolution: it packs its input, and the pack is only as good as the batch in it.
+CONV_FIRST = {"vgg16": BUILDS["vgg16"], "inceptionv3": lambda m: m.inceptionv3(batch=8, classes=10, image=107)}
+
+
+@pytest.mark.parametrize("name", sorted(CONV_FIRST))
+def test_a_batch_rewritten_after_the_recording_reaches_the_replay(lib_path, monkeypatch, name):
+    got = _train(monkeypatch, True, CONV_FIRST[name], "sgd", _overwrite_inputs_late)
+    assert got[2]
+    _same(got, _train(monkeypatch, False, CONV_FIRST[name], "sgd", _overwrite_inputs_late))
+
+
+def _in_turn(order, held_from=None):
+    """Feeds resident batch arrays in the order given by letters; from step `held_from` on the caller holds a view."""
+    arrays = {}
+
+    def between(step, model, ex, feed, x):
+        from tinyflow_b200 import ndarray
+        if step == 0:
+            arrays.clear()
+            for k, letter in enumerate(sorted(set(order))):
+                arrays[letter] = ndarray.array(np.roll(x.asnumpy() * (1.0 + k), k, axis=0), ndarray.gpu(0))
+        if step == held_from:
+            _held.append(ex.value_of(model.y))
+        if step == STEPS - 1:
+            del _held[:]
+        feed[model.X] = arrays[order[step]]
+    return between
+
+
+@pytest.mark.parametrize("order, held_from", [("AAAABAABA", None), ("AAABBBABA", 7), ("ABABABABA", 7)])
+@pytest.mark.parametrize("name", sorted(CONV_FIRST))
+def test_resident_batches_in_turn(lib_path, monkeypatch, name, order, held_from):
+    got = _train(monkeypatch, True, CONV_FIRST[name], "sgd", _in_turn(order, held_from))
+    assert got[2]
+    _same(got, _train(monkeypatch, False, CONV_FIRST[name], "sgd", _in_turn(order, held_from)))
 
 
 @pytest.mark.parametrize("name", ["mlp", "vgg16"])

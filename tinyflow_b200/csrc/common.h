@@ -140,6 +140,9 @@ int contraction_path();
 //    of words that alternates between calls; the maxima of tensors that a step reads before it writes them (parameters)
 //    are carried to the next replay in a word per tensor;
 //  * values that change from step to step (dropout seeds, Adam's bias corrections) are read from device words.
+//  * data derived from a tensor (packed operands, the indices of a maximum) that an earlier call left behind does not count
+//    inside the recording: the caller may rewrite the tensor between replays.
+uint64_t recording_id();                           // of the recording this thread makes, never used again; 0 when it makes none
 uint32_t* recording_word();                        // a zeroed-per-replay device word of the graph being recorded
 void* recording_take_block(size_t bytes);          // a block of exactly this (rounded) size freed earlier in the recording, or nullptr
 void recording_keep_block(void* p, size_t bytes);  // instead of handing the block back to the pool
@@ -233,6 +236,7 @@ struct PoolPlan {
   int32_t* argmax;
   const void* argmax_src;
   uint64_t argmax_version;
+  uint64_t argmax_recording;   // the recording whose graph writes the indices, 0: an ordinary call did
 };
 struct TensorPlan {      // activation / dropout input descriptor
   int kind;

@@ -1942,6 +1942,8 @@ struct Pack {           // a packed operand living in pooled device memory
   bool transient = false;          // belongs to one call (matrix products)
   long long rows = 0, cols = 0, pitch = 0;
   const void* src = nullptr; uint64_t version = 0; int tag = 0;   // cache key
+  uint64_t recording = 0;          // the recording whose graph fills the pack, 0: an ordinary call did
+  void made_from(const void* s, uint64_t ver, int t) { src = s; version = ver; tag = t; recording = recording_id(); }
   size_t bytes() const { return (size_t)rows * pitch * elem_of(arith); }
   const float* scale() const { return reinterpret_cast<const float*>(words + 2); }
 };
@@ -2151,8 +2153,11 @@ static int launch_pack_nchw(Pack& pk, const ScaleRef& sr, const float* src, int 
   TF_AFTER(s, what);
   return 0;
 }
+// A pack counts only where it was made: a recorded step reads none that was there before (the caller may rewrite its source
+// between replays, and nothing of the step would pack it again), an ordinary call none that a recording has only announced.
 static bool pack_valid(const Pack& pk, int ar, const void* src, uint64_t ver, int tag, long long rows, long long cols) {
-  return pk.hi && pk.arith == ar && pk.src == src && pk.version == ver && pk.tag == tag && pk.rows == rows && pk.cols == cols;
+  return pk.hi && pk.arith == ar && pk.src == src && pk.version == ver && pk.tag == tag && pk.rows == rows && pk.cols == cols &&
+         pk.recording == recording_id();
 }
 // ---- producers that write a consumer's pack ---------------------------------------------------------------------------
 // The graph calls BN -> ReLU -> convolution as separate entry points, and the convolution then re-reads the ReLU's output
@@ -2239,7 +2244,7 @@ static int pack_x(ConvTc* st, int ar, const ConvPlan* p, const float* x, cudaStr
       launch_dep(pack_patches_kernel<E>, dim3(grid_for(rows * 32, 256, 4)), dim3(256), 0, s, x, hi, lo, g, sr);
     });
     TF_AFTER(s, "pack_patches");
-    pk.src = x; pk.version = ver; pk.tag = 3;
+    pk.made_from(x, ver, 3);
     return 0;
   }
   const long long rows = (long long)p->N * st->frame_h * st->frame_w;
@@ -2262,7 +2267,7 @@ static int pack_x(ConvTc* st, int ar, const ConvPlan* p, const float* x, cudaStr
     rc = launch_pack_nchw(pk, sr, x, p->N, p->C, p->H, p->W, st->frame_h, st->frame_w, st->x_off_h, st->x_off_w, p->stride_h, p->stride_w, 0, (int)pk.pitch, s);
   }
   if (rc) return -1;
-  pk.src = x; pk.version = ver; pk.tag = st->cls;
+  pk.made_from(x, ver, st->cls);
   if (st->cls == 1 || st->cls == 2) offer_pack(x, st, p->N, p->C, p->H, p->W, p->stride_h, p->stride_w);
   if ((st->cls == 1 || st->cls == 2) && p->stride_h == 1 && p->stride_w == 1) remember_pack_target(x, ver, st, p);
   return 0;
@@ -2275,7 +2280,7 @@ static int pack_dy(ConvTc* st, int ar, const ConvPlan* p, const float* dy, cudaS
   if (pack_alloc(pk, ar, rows, p->K, s, oom)) return 1;
   ScaleRef sr = begin_pack(pk, dy, (long long)p->N * p->K * p->P * p->Q, s);
   if (launch_pack_nchw(pk, sr, dy, p->N, p->K, p->P, p->Q, st->frame_h, st->frame_w, st->dy_off_h, st->dy_off_w, 1, 1, 0, (int)pk.pitch, s)) return -1;
-  pk.src = dy; pk.version = ver; pk.tag = 2;
+  pk.made_from(dy, ver, 2);
   return 0;
 }
 // Filter packs are keyed like the activation packs (pointer, write version): an optimiser step bumps the version.
@@ -2296,7 +2301,7 @@ static int filter_job(ConvTc* st, int ar, const float* w, const ConvPlan* p, int
     (d ? job->hi_d : job->hi_f) = pk.hi; (d ? job->lo_d : job->lo_f) = pk.lo; (d ? job->pad_d : job->pad_f) = pad;
     (d ? job->scale_d : job->scale_f) = reinterpret_cast<float*>(pk.words + 2);
     if (!first) first = &pk;
-    pk.src = w; pk.version = ver; pk.tag = 10 + d;
+    pk.made_from(w, ver, 10 + d);
   }
   const ScaleRef sr = begin_pack(*first, w, (long long)p->K * p->C * p->R * p->S, s);
   job->amax = sr.amax_cur; job->amax_next = sr.amax_next;
@@ -2472,7 +2477,7 @@ int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cu
   ScaleRef sr{bound, nullptr, reinterpret_cast<float*>(pk.words + 2)};       // scale from max|x| >= max|relu(x)|; tf32: no scale
   note_compute_stream(s);
   if (launch_pack_nchw(pk, sr, x, t.N, t.C, t.H, t.W, st->frame_h, st->frame_w, st->x_off_h, st->x_off_w, 1, 1, 0, (int)pk.pitch, s, y, am)) return -1;
-  pk.src = y; pk.version = version_of(y); pk.tag = st->cls;
+  pk.made_from(y, version_of(y), st->cls);
   tc_note_relu_output(node, y);
   g_fused_relu_packs.fetch_add(1, std::memory_order_relaxed);
   return 1;
@@ -2495,7 +2500,7 @@ int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, floa
   note_compute_stream(s);
   ScaleRef sr{bound, nullptr, reinterpret_cast<float*>(pk.words + 2)};
   if (launch_pack_nchw(pk, sr, dy, p->N, p->K, p->P, p->Q, st->frame_h, st->frame_w, st->dy_off_h, st->dy_off_w, 1, 1, 0, (int)pk.pitch, s, out, am, mask)) return -1;
-  pk.src = out; pk.version = version_of(out); pk.tag = 2;
+  pk.made_from(out, version_of(out), 2);
   return 1;
 }
 long long fused_relu_pack_count() { return g_fused_relu_packs.load(std::memory_order_relaxed); }

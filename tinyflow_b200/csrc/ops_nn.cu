@@ -753,6 +753,7 @@ int DLGpuPooling2DForward(const DLArrayHandle input, DLArrayHandle output, void*
     launch_maxpool_fwd(p, (const float*)input->data, out_f32(output), p->argmax, total, s);
     p->argmax_src = input->data;
     p->argmax_version = version_of(input->data);
+    p->argmax_recording = recording_id();
   }
   else {
     float* y = out_f32(output);
@@ -776,7 +777,7 @@ int DLGpuPooling2DBackward(const DLArrayHandle input, const DLArrayHandle output
   note_compute_stream(s);
   KernelTimer kt("DLGpuPooling2DBackward", s, 0, 4.0 * ((p->mode == 0 ? 2 : 1) * numel(input) + numel(output)));
   if (p->mode == 0) {
-    if (p->argmax && p->argmax_src == input->data && p->argmax_version == version_of(input->data))
+    if (p->argmax && p->argmax_src == input->data && p->argmax_version == version_of(input->data) && p->argmax_recording == recording_id())
       launch_pool_gather<true>(p, p->argmax, (const float*)doutput->data, out_f32(dinput), total, 1.f, s);
     else
       maxpool_bwd_kernel<<<grid_for(total, 256), 256, 0, s>>>((const float*)input->data, (const float*)doutput->data, out_f32(dinput), total, geom_of(p));

@@ -40,7 +40,10 @@ struct StepGraph {
   std::vector<AmaxCarry> carries;
   long long launches = 0;
   uint64_t epoch = 0;
+  uint64_t id = 0;
 };
+static std::atomic<uint64_t> g_recordings{0};
+uint64_t recording_id() { return t_recording ? t_recording->id : 0; }
 
 uint32_t* recording_word() {
   StepGraph* g = t_recording;
@@ -112,6 +115,7 @@ int TfStepRecordBegin(void** graph, void** stream_cell) {
     TF_FAIL("TfStepRecordBegin: stream capture is not available");
   }
   g->epoch = g_layout_epoch.load();
+  g->id = g_recordings.fetch_add(1) + 1;
   t_recording = g;
   tc_recording_begins();
   *graph = g;
