@@ -145,7 +145,7 @@ def _in_turn(order, held_from=None):
     return between
 
 
-@pytest.mark.parametrize("order, held_from", [("AAAABAABA", None), ("AAABBBABA", 7), ("ABABABABA", 7)])
+@pytest.mark.parametrize("order, held_from", [("AAAABAABA", None), ("AAABBBABA", 7), ("ABABABABA", 7), ("AAAABABAB", 6)])
 @pytest.mark.parametrize("name", sorted(CONV_FIRST))
 def test_resident_batches_in_turn(lib_path, monkeypatch, name, order, held_from):
     got = _train(monkeypatch, True, CONV_FIRST[name], "sgd", _in_turn(order, held_from))

@@ -143,6 +143,8 @@ int contraction_path();
 //  * data derived from a tensor (packed operands, the indices of a maximum) that an earlier call left behind does not count
 //    inside the recording: the caller may rewrite the tensor between replays.
 uint64_t recording_id();                           // of the recording this thread makes, never used again; 0 when it makes none
+void recording_note_made(const void** source);     // the graph writes data derived from *source, kept by a plan: every replay sets *source to null,
+                                                   // so that no ordinary call takes that data for what it left there itself
 uint32_t* recording_word();                        // a zeroed-per-replay device word of the graph being recorded
 void* recording_take_block(size_t bytes);          // a block of exactly this (rounded) size freed earlier in the recording, or nullptr
 void recording_keep_block(void* p, size_t bytes);  // instead of handing the block back to the pool

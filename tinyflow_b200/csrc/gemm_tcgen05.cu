@@ -1943,7 +1943,7 @@ struct Pack {           // a packed operand living in pooled device memory
   long long rows = 0, cols = 0, pitch = 0;
   const void* src = nullptr; uint64_t version = 0; int tag = 0;   // cache key
   uint64_t recording = 0;          // the recording whose graph fills the pack, 0: an ordinary call did
-  void made_from(const void* s, uint64_t ver, int t) { src = s; version = ver; tag = t; recording = recording_id(); }
+  void made_from(const void* s, uint64_t ver, int t) { src = s; version = ver; tag = t; recording = recording_id(); if (t_recording) recording_note_made(&src); }
   size_t bytes() const { return (size_t)rows * pitch * elem_of(arith); }
   const float* scale() const { return reinterpret_cast<const float*>(words + 2); }
 };

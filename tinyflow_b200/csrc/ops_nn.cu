@@ -754,6 +754,7 @@ int DLGpuPooling2DForward(const DLArrayHandle input, DLArrayHandle output, void*
     p->argmax_src = input->data;
     p->argmax_version = version_of(input->data);
     p->argmax_recording = recording_id();
+    if (t_recording) recording_note_made(&p->argmax_src);
   }
   else {
     float* y = out_f32(output);

@@ -6,7 +6,8 @@
 // The recording runs on a private non-blocking stream in relaxed mode: other threads' copies and the legacy default stream
 // are not drawn into it, and nothing of the step executes while it is recorded.  What has to differ from an ordinary call is
 // listed at the declarations in common.h.  A replay leaves the library's books as the step itself would: every tensor the
-// step writes gets a new write version, the launches are counted, and the maxima of the parameters stay known.
+// step writes gets a new write version, the packs it overwrites in the plans no longer count as what an ordinary call left
+// there, the launches are counted, and the maxima of the parameters stay known.
 #include "common.h"
 #include <algorithm>
 #include <mutex>
@@ -37,6 +38,7 @@ struct StepGraph {
   float c1 = 0.f, c2 = 0.f;
   std::unordered_map<size_t, std::vector<void*>> free_blocks;
   std::vector<const void*> written;
+  std::vector<const void**> made;         // sources of the packs and indices in plans that the graph writes
   std::vector<AmaxCarry> carries;
   long long launches = 0;
   uint64_t epoch = 0;
@@ -72,6 +74,7 @@ const float* recording_adam_corrections(float c1, float c2) {
 }
 void recording_note_launches(int n) { t_recording->launches += n; }
 void recording_note_write(const void* p) { t_recording->written.push_back(p); }
+void recording_note_made(const void** source) { t_recording->made.push_back(source); }
 cudaStream_t recording_stream() { return t_recording->stream; }
 
 // Values of this replay (bias corrections, seeds) into the words the recorded kernels read; up to 960 per launch by value.
@@ -161,6 +164,8 @@ int TfStepRecordEnd(void** graph, int keep) {
   }
   std::sort(g->written.begin(), g->written.end());
   g->written.erase(std::unique(g->written.begin(), g->written.end()), g->written.end());
+  std::sort(g->made.begin(), g->made.end());
+  g->made.erase(std::unique(g->made.begin(), g->made.end()), g->made.end());
   return 0;
 }
 
@@ -209,6 +214,7 @@ int TfStepReplay(void* graph, const unsigned* seeds, int nseeds, float b1t, floa
   TF_CUDA(cudaGraphLaunch(g->exec, s));
   g_launches.fetch_add(g->launches, std::memory_order_relaxed);
   bump_versions(g->written.data(), g->written.size());
+  for (const void** source : g->made) *source = nullptr;
   for (const AmaxCarry& c : g->carries) if (c.from) amax_set_carry_valid(c.data);
   return 0;
 }
