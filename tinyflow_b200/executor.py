@@ -460,15 +460,10 @@ class Executor(object):
             return None
         if self.top_control_queue is not None and not self.top_control_queue.empty():
             return None
-        top, below = self._recordings.find(feed_dict)
-        recording, staged = below.recording, False
-        if recording is None and below.runs < step_graph.RUNS_BEFORE_RECORDING and top.runs >= step_graph.RUNS_BEFORE_STAGING:
-            recording, staged = top.recording, True
+        entry, staged, wanted = self._recordings.choose(feed_dict)
+        recording = entry.recording
         if recording is not None and recording.changes != self._changes[0]:
-            recording = None
-        wanted = top.runs >= step_graph.RUNS_BEFORE_STAGING if staged else below.runs >= step_graph.RUNS_BEFORE_RECORDING
-        top.runs += 1
-        below.runs += 1
+            recording = entry.recording = None
         if self._live_leases() or gpu_op.data_parallel_active():
             return None
         if recording is None:
@@ -477,10 +472,7 @@ class Executor(object):
             recording = self._record(feed_dict, staged)
             if recording is None:
                 return None
-            if staged:
-                top.recording = recording
-            else:
-                below.recording = recording
+            entry.recording = recording
         self._feed = dict(feed_dict)
         if staged:
             for node, array in recording.staged:
@@ -495,7 +487,7 @@ class Executor(object):
         rc = recording.replay(self, random.randint)
         if rc != 0:
             if rc == 1:
-                top.recording = below.recording = None
+                entry.recording = None
             return None
         self._values = recording.values
         loss = ndarray.empty(recording.loss.shape, self.ctx_gpu)

@@ -5,8 +5,12 @@ ones.  The executor therefore records the step once it has seen the same feed re
 (``TfStepReplay``) from then on: the host work per step no longer grows with the number of nodes.
 
 What is replayed is keyed by identity.  Parameters and moments (updated in place) are one key; the mini-batch arrays are a
-second one below it.  A caller that brings new mini-batch arrays every step gets a *staged* recording, whose inputs are
-copied into arrays of the executor's own first.  Entries disappear with the arrays they name.
+second one below it.  A caller that brings new mini-batch arrays every step, or feeds several in turn, gets a *staged*
+recording, whose inputs are copied into arrays of the executor's own first.  Entries disappear with the arrays they name.
+
+A recording is paid for once, a staged input at every step.  ResNet-50 at batch 64: 5-16 ms of host time for the recording
+(calls 2-6, end of capture and instantiation 1.4-14), 15 us a step for the copies.  So arrays that come in turn get
+recordings of their own only after RUNS_WITHOUT_STAGING steps, when the copies have cost about as much.
 """
 from __future__ import annotations
 
@@ -19,7 +23,8 @@ from ._base import _LIB, check_call, new_cell
 
 ENABLED = os.environ.get("TINYFLOW_STEP_GRAPH", "1") != "0"
 RUNS_BEFORE_RECORDING = 2        # of the same arrays: the first calls of a plan still learn what follows what
-RUNS_BEFORE_STAGING = 4          # of the same parameters with ever new mini-batches
+RUNS_BEFORE_STAGING = 4          # of the same parameters with ever changing mini-batches
+RUNS_WITHOUT_STAGING = 512       # of the same arrays, others in between
 MAX_FEEDS = 4                    # parameter sets, and mini-batches per set, that keep a recording
 
 
@@ -49,11 +54,15 @@ class Recording(object):
 
 
 class _Feed(object):
-    """How often a set of arrays was run, and what was recorded for it."""
-    __slots__ = ("runs", "refs", "recording", "batches", "__weakref__")
+    """How often a set of arrays was run, how often since another one, and what was recorded for it."""
+    __slots__ = ("runs", "in_a_row", "refs", "recording", "batches", "latest", "__weakref__")
 
     def __init__(self):
-        self.runs, self.refs, self.recording, self.batches = 0, None, None, {}
+        self.runs, self.in_a_row, self.refs, self.recording, self.batches, self.latest = 0, 0, None, None, {}, None
+
+    def settled(self):
+        """Worth a recording on the arrays themselves."""
+        return self.in_a_row >= RUNS_BEFORE_RECORDING or self.runs >= RUNS_WITHOUT_STAGING
 
 
 class Recordings(object):
@@ -75,15 +84,23 @@ class Recordings(object):
         table[key] = entry                      # most recently used last
         return entry
 
-    def find(self, feed_dict):
-        """(entry of the parameters, entry of the mini-batch below it) for this feed."""
+    def choose(self, feed_dict):
+        """(entry, staged, wanted): the entry whose recording serves this run, whether its inputs are staged, and whether
+        the entry is due one if it has none.  Counts the run."""
         params, batch = [], []
         for node, value in feed_dict.items():
             (batch if node.isw == 2 else params).append((node, value))
-        key = tuple((id(n), id(v)) for n, v in params)
-        top = self._entry(self.sets, key, [v for _, v in params])
-        below = self._entry(top.batches, tuple((id(n), id(v)) for n, v in batch), [v for _, v in batch])
-        return top, below
+        top = self._entry(self.sets, tuple((id(n), id(v)) for n, v in params), [v for _, v in params])
+        key = tuple((id(n), id(v)) for n, v in batch)
+        below = self._entry(top.batches, key, [v for _, v in batch])
+        if top.latest != key:
+            top.latest, below.in_a_row = key, 0
+        staged = below.recording is None and not below.settled() and top.runs >= RUNS_BEFORE_STAGING
+        wanted = staged or below.settled()
+        top.runs += 1
+        below.runs += 1
+        below.in_a_row += 1
+        return top if staged else below, staged, wanted
 
 
 def _forget(table, key, entry_ref):
