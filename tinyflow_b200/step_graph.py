@@ -77,7 +77,8 @@ class Recordings(object):
         entry = table.pop(key, None)
         if entry is None:
             entry = _Feed()
-            gone = lambda _ref, t=weakref.ref(entry), k=key: _forget(table, k, t)     # noqa: E731
+            # (bound here: at interpreter exit the module's names go before the arrays do)
+            gone = lambda _ref, t=weakref.ref(entry), k=key, forget=_forget: forget(table, k, t)     # noqa: E731
             entry.refs = [weakref.ref(a, gone) for a in arrays]
             while len(table) >= MAX_FEEDS:
                 del table[next(iter(table))]
