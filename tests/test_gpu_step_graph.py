@@ -161,6 +161,27 @@ def test_new_mini_batch_arrays_every_step(lib_path, monkeypatch, name):
     _same(got, want)
 
 
+def test_a_recording_packs_filters_for_its_own_plans_only(lib_path, monkeypatch):
+    """Batches of other sizes build other plans; a step recorded after them has the launches it had before them."""
+    from tinyflow_b200 import autodiff as ad, gpu_op, models, ndarray, step_graph
+    monkeypatch.setattr(step_graph, "ENABLED", True)
+    model = models.resnet50(batch=16, classes=10, image=64)          # 53 filters; one launch packs up to 128
+    ex = ad.Executor(model.loss, model.y, 0.001, None, None, None, optimizer="sgd")
+    ctx = ndarray.gpu(0)
+    feed = {n: ndarray.array(v, ctx) for n, v in model.init_params(seed=5).items()}
+    X, Y = models.synthetic_batch(model, seed=8)
+    launches = []
+    for batch in (16, 15, 14, 16):
+        feed[model.X], feed[model.y_] = ndarray.array(X[:batch], ctx), ndarray.array(Y[:batch], ctx)
+        for _ in range(5):
+            before = gpu_op.launch_count()
+            ex.run(feed)
+        assert any(b.recording for f in ex._recordings.sets.values() for b in f.batches.values())
+        launches.append(gpu_op.launch_count() - before)
+    gpu_op.device_synchronize()
+    assert launches[0] == launches[-1]
+
+
 @pytest.mark.parametrize("count", [1, 5, 400])
 def test_many_updates_in_one_launch(lib_path, count):
     from tinyflow_b200 import gpu_op, ndarray as nd

@@ -31,7 +31,7 @@ int tensor_path_error();
 void tensor_path_error_clear();
 int tensor_path_timeout_probe(long long limit_cycles, cudaStream_t s);
 long long fused_relu_pack_count();
-int tc_pack_filters(const void* const* arrays, const int64_t* sizes, int n, cudaStream_t s);
+int tc_pack_filters(ConvPlan* const* plans, const float* const* filters, const int64_t* sizes, int n, cudaStream_t s);
 int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, float* out, cudaStream_t s);
 // which engine served this thread's most recent contraction: 1 = CUDA cores, 2 = tensor cores (0 = none yet)
 static thread_local int t_last_path = 0;
@@ -53,14 +53,18 @@ int TfGetArithmetic(void) { return tensor_arithmetic(); }
 
 int TfTensorPathError(void) { return tensor_path_error(); }
 int TfClearTensorPathError(void) { tensor_path_error_clear(); return 0; }
-int TfPackFilters(const DLArrayHandle* arrays, int n, void** cudaStream) {
-  TF_REQUIRE(arrays && n >= 0, "TfPackFilters: null argument");
+int TfPackFilters(const DLArrayHandle* filters, void*** const* plans, int n, void** cudaStream) {
+  TF_REQUIRE((filters && plans) || n == 0, "TfPackFilters: null argument");
   if (!t_recording) return 0;
-  std::vector<const void*> data;
+  std::vector<ConvPlan*> plan;
+  std::vector<const float*> data;
   std::vector<int64_t> sizes;
-  for (int i = 0; i < n; ++i)
-    if (arrays[i] && arrays[i]->ctx.device_type == kGPU) { data.push_back(arrays[i]->data); sizes.push_back(numel(arrays[i])); }
-  return tc_pack_filters(data.data(), sizes.data(), (int)data.size(), stream_of(cudaStream));
+  for (int i = 0; i < n; ++i) {
+    ConvPlan* p = plan_of<ConvPlan>(plans[i], kPlanConv);
+    if (!p || !filters[i] || filters[i]->ctx.device_type != kGPU) continue;
+    plan.push_back(p); data.push_back((const float*)filters[i]->data); sizes.push_back(numel(filters[i]));
+  }
+  return tc_pack_filters(plan.data(), data.data(), sizes.data(), (int)plan.size(), stream_of(cudaStream));
 }
 int TfFusedReluPackCount(long long* count) { if (count) *count = fused_relu_pack_count(); return 0; }
 int TfFusedReluBnBackwardCount(long long* count) { if (count) *count = fused_relu_bn_bwd_count(); return 0; }

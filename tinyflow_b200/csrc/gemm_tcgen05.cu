@@ -2069,7 +2069,6 @@ int tc_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_
 //   class D: strided windows: space-to-depth phases (see conv_state);
 //   class C: too few input channels for a per-tap reduction chunk: x is expanded into patches (C*R*S columns) and
 //            the problem runs as class A over C*R*S channels; forward and filter gradient only.
-constexpr size_t kFilterSets = 8;       // parameter sets a plan remembers: an executor keeps recordings of four
 struct ConvTc {
   int cls = 0;                 // 0 unsupported, 1 class A, 2 class B, 3 class C, 4 class D
   int frame_h = 0, frame_w = 0;                          // frame geometry shared by the x and dy packs
@@ -2078,8 +2077,6 @@ struct ConvTc {
   int cp = 0;                                            // class D: columns per stride phase (C rounded up to 64)
   bool dgrad_seen = false;                               // backward-data has run on this plan: forward also packs its filter layout
   bool track_y = false, track_dx = false;                // a ReLU asked for max|y| / max|dx|: the epilogue leaves it
-  std::vector<const float*> filters;                     // arrays the filter packs were made from (the last kFilterSets), and the plan
-  const ConvPlan* plan = nullptr;
   Pack x, dy, wf, wd;
   ConvTc* x_owner = this;                                // whose x pack the plan reads: another plan's of the same recorded step, or its own
   std::mutex mu;
@@ -2285,8 +2282,6 @@ static int pack_dy(ConvTc* st, int ar, const ConvPlan* p, const float* dy, cudaS
 }
 // Filter packs are keyed like the activation packs (pointer, write version): an optimiser step bumps the version.
 // filter_job() prepares the pack of one filter (layouts: 1 forward, 2 backward-data) and stamps it as made; 0 on success.
-static std::mutex g_filter_plans_mu;
-static std::vector<ConvTc*> g_filter_plans;            // every plan that has packed a filter
 static int filter_job(ConvTc* st, int ar, const float* w, const ConvPlan* p, int layouts, cudaStream_t s, int* oom, FilterJob* job) {
   const int taps = st->eR * st->eS;
   memset(job, 0, sizeof(*job));
@@ -2305,16 +2300,6 @@ static int filter_job(ConvTc* st, int ar, const float* w, const ConvPlan* p, int
   }
   const ScaleRef sr = begin_pack(*first, w, (long long)p->K * p->C * p->R * p->S, s);
   job->amax = sr.amax_cur; job->amax_next = sr.amax_next;
-  if (!st->plan) {
-    std::lock_guard<std::mutex> lk(g_filter_plans_mu);
-    g_filter_plans.push_back(st);
-  }
-  st->plan = p;
-  auto& known = st->filters;
-  if (std::find(known.begin(), known.end(), w) == known.end()) {
-    if (known.size() == kFilterSets) known.erase(known.begin());
-    known.push_back(w);
-  }
   return 0;
 }
 template <int MAX> static int launch_filter_jobs(FilterJobs<MAX>& jobs, int ar, cudaStream_t s) {
@@ -2342,31 +2327,21 @@ static int pack_filter(ConvTc* st, int ar, const float* w, const ConvPlan* p, in
   if (int rc = filter_job(st, ar, w, p, flip ? 2 : with_other ? 3 : 1, s, oom, &one.job[0])) return rc;
   return launch_filter_jobs(one, ar, s);
 }
-// While a step is recorded: the filters among `arrays` (with their sizes) that a plan has been fed from, all in one launch, ahead of
-// the convolutions that find them packed.  What it leaves out, or guesses wrong, the convolution packs when it comes up.
-int tc_pack_filters(const void* const* arrays, const int64_t* sizes, int n, cudaStream_t s) {
+// While a step is recorded: the filters that its convolutions read, each for its plan, all in one launch ahead of the
+// convolutions that find them packed.  What it leaves out the convolution packs when it comes up.
+int tc_pack_filters(ConvPlan* const* plans, const float* const* filters, const int64_t* sizes, int n, cudaStream_t s) {
   if (contraction_path_is_cuda_cores() || !encode_fn()) return 0;
   const int ar = tensor_arithmetic();
-  std::unordered_map<const void*, int64_t> wanted;
-  for (int i = 0; i < n; ++i) wanted[arrays[i]] = sizes[i];
-  std::vector<ConvTc*> plans;
-  {
-    std::lock_guard<std::mutex> lk(g_filter_plans_mu);
-    plans = g_filter_plans;
-  }
   FilterJobs<kFilterJobs> jobs;
   jobs.n = 0;
-  for (ConvTc* st : plans) {
+  for (int i = 0; i < n; ++i) {
+    const ConvPlan* p = plans[i];
+    ConvTc* st = (ConvTc*)p->tc_state;
+    if (!st || !st->cls || sizes[i] != (int64_t)p->K * p->C * p->R * p->S) continue;
     std::lock_guard<std::mutex> lk(st->mu);
-    const ConvPlan* p = st->plan;
-    const float* w = nullptr;
-    for (const float* f : st->filters) {
-      auto it = wanted.find(f);
-      if (it != wanted.end() && it->second == (int64_t)p->K * p->C * p->R * p->S) w = f;
-    }
-    if (!w || !st->wf.hi || st->wf.arith != ar || (ar == kArithF16 && !amax_tracked(w))) continue;
+    if (!st->wf.hi || st->wf.arith != ar || (ar == kArithF16 && !amax_tracked(filters[i]))) continue;
     int oom = 0;
-    if (filter_job(st, ar, w, p, st->dgrad_seen ? 3 : 1, s, &oom, &jobs.job[jobs.n])) continue;
+    if (filter_job(st, ar, filters[i], p, st->dgrad_seen ? 3 : 1, s, &oom, &jobs.job[jobs.n])) continue;
     if (++jobs.n < kFilterJobs) continue;
     if (launch_filter_jobs(jobs, ar, s)) return -1;
     jobs.n = 0;

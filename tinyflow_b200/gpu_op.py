@@ -423,6 +423,12 @@ def handle_array(arrs):
     return (_nd.DLArrayHandle * len(arrs))(*[_h(a) for a in arrs])
 
 
+def pack_filters(filters, cudnnlists, cudaStream):
+    """While a step is recorded: packs the filter of every (filter, convolution descriptor) pair in one launch."""
+    cells = (ctypes.c_void_p * len(cudnnlists))(*[ctypes.cast(c, ctypes.c_void_p) for c in cudnnlists])
+    check_call(_LIB.TfPackFilters(handle_array(filters), cells, len(filters), cudaStream))
+
+
 def sgd_update_many(params, grads, learning_rate, cudaStream):
     """``sgd_update`` of every pair in one launch; ``params`` and ``grads`` come from :func:`handle_array`."""
     check_call(_LIB.TfSgdUpdateMany(params, grads, len(params), _F(learning_rate), cudaStream))

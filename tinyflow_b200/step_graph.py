@@ -20,6 +20,7 @@ import weakref
 
 from . import gpu_op, ndarray
 from ._base import _LIB, check_call, new_cell
+from .graph import Convolution2DForwardOp
 
 ENABLED = os.environ.get("TINYFLOW_STEP_GRAPH", "1") != "0"
 RUNS_BEFORE_RECORDING = 2        # of the same arrays: the first calls of a plan still learn what follows what
@@ -120,8 +121,8 @@ def record(executor, feed_dict, staged):
         return None
     values, loss, keep = {}, None, 0
     try:
-        params = gpu_op.handle_array([v for n, v in feed_dict.items() if n.isw == 1])
-        check_call(_LIB.TfPackFilters(params, len(params), stream))
+        convs = [n for n in executor.topo_order if type(n.op) is Convolution2DForwardOp and feed_dict.get(n.inputs[1]) is not None]
+        gpu_op.pack_filters([feed_dict[n.inputs[1]] for n in convs], [n.cudnnlist[0] for n in convs], stream)
         values, loss = executor._issue(feed_dict, stream, recording=True)
         keep = 1
     except Exception:                           # whatever stopped it: the ordinary step that follows reports it
