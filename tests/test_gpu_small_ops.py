@@ -54,3 +54,42 @@ def test_channel_sums(env, shape):
     env.gpu_op.broadcast_to_backward(X, out, "NCHW")
     want, mag = x.astype(np.float64).sum((0, 2, 3)), np.abs(x).astype(np.float64).sum((0, 2, 3))
     assert np.all(np.abs(out.asnumpy() - want) <= 1e-6 * mag)
+
+
+def test_split_reductions_on_two_streams_at_once(env):
+    """Every stream has partial sums and arrival counters of its own: two threads get the bits that one gets."""
+    import threading
+    nd, op, runs = env.nd, env.gpu_op, 150
+    rng = np.random.RandomState(2)
+    state = []
+    for k in range(2):
+        stream = op.create_cudaStream()
+        logits = nd.array(rng.randn(2000 + k, 37).astype(np.float32), env.ctx)
+        labels = nd.array(np.eye(37, dtype=np.float32)[rng.randint(0, 37, 2000 + k)], env.ctx)
+        x = nd.array(rng.randn(64, 16, 33, 32 + k).astype(np.float32), env.ctx)
+        plan = op.reduce_sum_get_cudnnlist(x.shape, (1, 16, 1, 1), "NCHW", env.cudnn)
+        outs = [(nd.empty((1,), env.ctx), nd.empty((1, 16, 1, 1), env.ctx)) for _ in range(runs + 1)]
+        state.append((stream, logits, labels, x, plan, outs))
+
+    def work(k, which):
+        stream, logits, labels, x, plan, outs = state[k]
+        for loss, sums in which(outs):
+            op.softmax_cross_entropy(logits, labels, loss, stream)
+            op.reduce_sum_new(x, sums, plan, env.cudnn, stream)
+
+    for k in range(2):
+        work(k, lambda outs: outs[:1])
+    op.device_synchronize()
+    threads = [threading.Thread(target=work, args=(k, lambda outs: outs[1:])) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    op.device_synchronize()
+    for k in range(2):
+        want = [v.asnumpy() for v in state[k][-1][0]]
+        for pair in state[k][-1][1:]:
+            for got, one in zip(pair, want):
+                np.testing.assert_array_equal(got.asnumpy(), one)
+        mag = np.abs(state[k][3].asnumpy().astype(np.float64)).sum((0, 2, 3))
+        assert np.all(np.abs(want[1].ravel() - state[k][3].asnumpy().astype(np.float64).sum((0, 2, 3))) <= 1e-6 * mag)

@@ -146,6 +146,8 @@ uint64_t recording_id();                           // of the recording this thre
 void recording_note_made(const void** source);     // the graph writes data derived from *source, kept by a plan: every replay sets *source to null,
                                                    // so that no ordinary call takes that data for what it left there itself
 uint32_t* recording_word();                        // a zeroed-per-replay device word of the graph being recorded
+void* recording_scratch(int slot, size_t bytes);   // stream_scratch() and arrival_counters() inside a recording: the graph's own
+uint32_t* recording_counters(int n);
 void* recording_take_block(size_t bytes);          // a block of exactly this (rounded) size freed earlier in the recording, or nullptr
 void recording_keep_block(void* p, size_t bytes);  // instead of handing the block back to the pool
 const uint32_t* recording_seed(unsigned seed);     // device word that will hold the seed of this dropout call at every replay
@@ -153,7 +155,7 @@ const float* recording_adam_corrections(float c1, float c2);   // two device wor
 void recording_note_launches(int n);
 void recording_note_write(const void* p);
 cudaStream_t recording_stream();
-// Buffers that outlive a call (packs, scratch) were reallocated or the arithmetic changed: recorded steps are out of date.
+// Buffers that outlive a call (packs) were reallocated or the arithmetic changed: recorded steps are out of date.
 void bump_layout_epoch();
 
 // ---- shapes -------------------------------------------------------------------
@@ -173,9 +175,12 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // Returns nullptr when the device is out of memory even after the cache was released.
 void* pool_alloc(size_t bytes);
 void pool_free(void* p);
-// Scratch buffers that live as long as the library (grown on demand, never shrunk);
-// slot ids are per purpose so concurrent purposes do not collide.
-void* persistent_scratch(int slot, size_t bytes);
+// Scratch of at least `bytes` for kernels on stream s, the same block at every call until a larger one is asked for; slot
+// ids are per purpose.  Kernels of one stream may share it, for they run in order; every stream, and every recorded step, has its own.
+constexpr int kScratchSlots = 4;
+void* stream_scratch(int slot, size_t bytes, cudaStream_t s);
+// n arrival counters of stream s: zero when a kernel on it starts, and the kernel leaves them zero (atomicInc wraps).
+uint32_t* arrival_counters(int n, cudaStream_t s);
 
 // ---- grid sizing: whole multiples of the SM count -----------------------------
 inline int grid_for(int64_t work_items, int block, int per_thread = 1, int waves = 8) {

@@ -1750,7 +1750,7 @@ static float g_tail_cost = [] { const char* e = getenv("TINYFLOW_TAIL_COST"); re
 // the cluster (768 -> 192 channels, 17 x 17, 1x1, batch 2: 17.0 -> 15.3 us in clusters of 6).  Against it the workspace costs
 // 4 stages and 0.15 per tile (its traffic): 70 tiles of 36 stages 34.0 us split and 29.7 in clusters of 2, 40 of 72
 // stages 33.8 and 32.5 in clusters of 3, but 12 of 72 stages 19.2 and 23 in clusters of 8.
-template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, int* oom, MaxClusters max_clusters) {
+template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, cudaStream_t s, int* oom, MaxClusters max_clusters) {
   const int sms = device_sm_count();
   const int tiles = g.m_tiles * g.n_tiles * g.tap_tiles;
   g.full_tiles = tiles; g.tail_tiles = 0; g.tail_share = 0; g.slots_per_cta = 0; g.workspace = nullptr; g.cluster = 1;
@@ -1776,7 +1776,7 @@ template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, int
   g.slots_per_cta = (share - 1 + g.k_total - 1) / g.k_total + 1;       // tiles a range of `share` stages can touch
   const int ctas = (int)((units + share - 1) / share);
   const size_t bytes = (size_t)ctas * g.slots_per_cta * bn * BM * sizeof(float);
-  g.workspace = (float*)persistent_scratch(1, bytes);
+  g.workspace = (float*)stream_scratch(1, bytes, s);
   if (!g.workspace) { if (oom) *oom = bytes > 0x7fffffffu ? 0x7fffffff : (int)bytes; return 1; }
   return 0;
 }
@@ -1823,7 +1823,7 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
   static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
   TF_CUDA(attr);
   TF_REQUIRE(tensor_path_error() == 0, "%s: an earlier tensor-core kernel timed out on a barrier; refusing to launch", what);
-  if (int rc = plan_schedule(p, BN, oom, max_clusters_of<BN, AR>)) return rc;
+  if (int rc = plan_schedule(p, BN, s, oom, max_clusters_of<BN, AR>)) return rc;
   static const int group_iters = getenv("TINYFLOW_GROUP_ITERS") ? atoi(getenv("TINYFLOW_GROUP_ITERS")) : 0;
   p.group_iters = group_iters > 0 ? group_iters : (p.data_by_data ? kGroupItersDataByData : (AR == kArithTF32 ? kGroupItersTF32 : kGroupIters));
   // cross terms promoted every 64 stages: 256 accumulations into a sum 2^-12 of the whole truncate less than 2^-28 of it

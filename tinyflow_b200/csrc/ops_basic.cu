@@ -50,29 +50,6 @@ __device__ __forceinline__ bool arrives_last(uint32_t* counter, uint32_t blocks)
   if (last) __threadfence();
   return last;
 }
-// `n` consecutive zeroed counters; a ring far longer than the launches that can be in flight at once.
-static uint32_t* arrival_counters(int n) {
-  constexpr int kCounters = 65536;
-  static std::mutex mu;
-  static uint32_t* ring[64] = {nullptr};
-  static int at[64] = {0};
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64 || n > kCounters) { cudaGetLastError(); return nullptr; }
-  std::lock_guard<std::mutex> lk(mu);
-  if (!ring[dev]) {
-    uint32_t* p = nullptr;
-    if (cudaMalloc((void**)&p, sizeof(uint32_t) * kCounters) != cudaSuccess || cudaMemset(p, 0, sizeof(uint32_t) * kCounters) != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess) {
-      cudaGetLastError();
-      return nullptr;
-    }
-    ring[dev] = p;
-  }
-  if (at[dev] + n > kCounters) at[dev] = 0;
-  uint32_t* p = ring[dev] + at[dev];
-  at[dev] += n;
-  return p;
-}
-
 // ---- generic vectorised map kernels ---------------------------------------------
 // Functors whose outputs become operands of the tensor path (activations, their gradients, weights) carry a
 // `kTrackAmax` member: only their launches reduce max|y| on the side.
@@ -816,10 +793,10 @@ int DLGpuBroadcastTo1(const DLArrayHandle input, DLArrayHandle output, void** cu
 
 static int reduce_to_scalar(const float* in, float* out, int64_t n, float scale, cudaStream_t s, const char* what) {
   int blocks = grid_for(n, kBlock, 8, 4);
-  float* part = (float*)persistent_scratch(0, sizeof(float) * 4096);
+  float* part = (float*)stream_scratch(0, sizeof(float) * 4096, s);
   TF_REQUIRE(part, "%s: scratch allocation failed", what);
   if (blocks > 4096) blocks = 4096;
-  uint32_t* counter = arrival_counters(1);
+  uint32_t* counter = arrival_counters(1, s);
   TF_REQUIRE(counter, "%s: scratch allocation failed", what);
   note_compute_stream(s);
   launch_dep(sum_kernel, dim3(blocks), dim3(kBlock), 0, s, in, out, part, n, scale, counter);
@@ -839,8 +816,8 @@ static int channel_sums(const float* in, float* out, int64_t N, int64_t C, int64
   float* part = nullptr;
   uint32_t* counters = nullptr;
   if (splits > 1) {
-    part = (float*)persistent_scratch(2, sizeof(float) * (size_t)splits * (size_t)C);
-    counters = arrival_counters((int)C);
+    part = (float*)stream_scratch(2, sizeof(float) * (size_t)splits * (size_t)C, s);
+    counters = arrival_counters((int)C, s);
     TF_REQUIRE(part && counters, "%s: scratch allocation failed", what);
   }
   const int vec = L % 4 == 0 && aligned16(in) && nps * (L / 4) < (1ll << 31);
@@ -864,8 +841,8 @@ static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, 
   float* part = nullptr;
   uint32_t* counters = nullptr;
   if (splits > 1) {
-    part = (float*)persistent_scratch(2, sizeof(float) * (size_t)splits * (size_t)cols);
-    counters = arrival_counters(gx);
+    part = (float*)stream_scratch(2, sizeof(float) * (size_t)splits * (size_t)cols, s);
+    counters = arrival_counters(gx, s);
     if (!part || !counters) { splits = 1; rps = rows; }                                  // no scratch: one split
   }
   note_compute_stream(s);
@@ -1137,8 +1114,8 @@ int DLGpuSoftmaxCrossEntropy(const DLArrayHandle input_a, const DLArrayHandle in
   note_compute_stream(s);
   const int64_t rows = input_a->shape[0];
   const int blocks = (int)std::min<int64_t>(std::max<int64_t>(1, (rows + kBlock / 32 - 1) / (kBlock / 32)), 2 * device_sm_count());
-  float* part = (float*)persistent_scratch(0, sizeof(float) * 4096);
-  uint32_t* counter = arrival_counters(1);
+  float* part = (float*)stream_scratch(0, sizeof(float) * 4096, s);
+  uint32_t* counter = arrival_counters(1, s);
   TF_REQUIRE(part && counter, "DLGpuSoftmaxCrossEntropy: scratch allocation failed");
   launch_dep(softmax_xent_kernel, dim3(blocks), dim3(kBlock), 0, s, F(input_a), F(input_b), FM(output), part, rows, input_a->shape[1], counter);
   TF_AFTER(s, "DLGpuSoftmaxCrossEntropy");

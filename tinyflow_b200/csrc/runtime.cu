@@ -3,7 +3,10 @@
 // src/cuda_device_api.cc and src/cpu_device_api.cc of the reference.
 #include "common.h"
 #include <stdarg.h>
+#include <algorithm>
+#include <map>
 #include <mutex>
+#include <thread>
 #include <unordered_map>
 #include <vector>
 #include <chrono>
@@ -214,13 +217,14 @@ struct Pool {
   // *hard (optional) is set when the allocation failed for a reason other than running out of memory (the context is
   // unusable, e.g. after a kernel fault): the caller reports an error instead of the out-of-memory protocol.  The
   // flag describes this call only.
-  void* alloc(size_t bytes, bool* hard = nullptr) {
+  // `unused`: not a recycled block (whatever stream last worked on one may not be through with it).
+  void* alloc(size_t bytes, bool* hard = nullptr, bool unused = false) {
     if (hard) *hard = false;
     size_t b = round(bytes);
     if (t_recording && !host) if (void* p = recording_take_block(b)) return p;      // still counted as in use
     std::lock_guard<std::mutex> lk(mu);
     auto it = free_by_size.find(b);
-    if (it != free_by_size.end() && !it->second.empty()) {
+    if (!unused && it != free_by_size.end() && !it->second.empty()) {
       void* p = it->second.back();
       it->second.pop_back();
       cached -= (long long)b;
@@ -305,20 +309,63 @@ void pool_free(void* p) {
   }
 }
 
-void* persistent_scratch(int slot, size_t bytes) {
-  static std::mutex mu;
-  static void* ptr[16] = {nullptr};
-  static size_t cap[16] = {0};
-  std::lock_guard<std::mutex> lk(mu);
-  if (slot < 0 || slot >= 16) return nullptr;
-  if (cap[slot] >= bytes) return ptr[slot];
-  // Growing while earlier kernels may still read the old block: hand the old block back
-  // to the pool (stream order on the single compute stream keeps that safe).
-  if (ptr[slot]) { pool_free(ptr[slot]); bump_layout_epoch(); }
-  size_t want = bytes + bytes / 4;
-  ptr[slot] = pool_alloc(want);
-  cap[slot] = ptr[slot] ? Pool::round(want) : 0;
-  return ptr[slot];
+// Scratch per (device, stream): the kernels of one stream run one after the other, so they can share a block; those of two
+// streams (two executors, two threads) cannot.  An outgrown block stays until its stream is destroyed, because another thread may
+// be about to launch a kernel on it; with a growth of at least 1.5x all of a stream's blocks of a slot are below three times the last.
+constexpr int kCounterSlot = kScratchSlots;           // arrival counters, kept zero between kernels
+struct StreamScratch { void* ptr[kScratchSlots + 1] = {nullptr}; size_t cap[kScratchSlots + 1] = {0}; std::vector<void*> outgrown; };
+static std::mutex g_scratch_mu;
+static std::map<std::pair<int, std::pair<cudaStream_t, size_t>>, StreamScratch> g_scratch;
+static std::pair<int, std::pair<cudaStream_t, size_t>> scratch_key(cudaStream_t s) {        // a per-thread stream is another one in every thread
+  return {current_device(), {s, s == cudaStreamPerThread ? std::hash<std::thread::id>()(std::this_thread::get_id()) : 0}};
+}
+static void* scratch_block(int slot, size_t bytes, cudaStream_t s, bool* fresh) {           // g_scratch_mu held
+  StreamScratch& sc = g_scratch[scratch_key(s)];
+  if (sc.cap[slot] >= bytes) return sc.ptr[slot];
+  const size_t want = std::max(bytes + bytes / 4, sc.cap[slot] + sc.cap[slot] / 2);
+  void* p = device_pool().alloc(want, nullptr, true);
+  if (!p) return nullptr;
+  if (sc.ptr[slot]) sc.outgrown.push_back(sc.ptr[slot]);
+  sc.ptr[slot] = p;
+  sc.cap[slot] = Pool::round(want);
+  *fresh = true;
+  return p;
+}
+void* stream_scratch(int slot, size_t bytes, cudaStream_t s) {
+  if (slot < 0 || slot >= kScratchSlots) return nullptr;
+  if (t_recording) return recording_scratch(slot, bytes);
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  bool fresh = false;
+  return scratch_block(slot, bytes, s, &fresh);
+}
+uint32_t* arrival_counters(int n, cudaStream_t s) {
+  if (t_recording) return recording_counters(n);
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  bool fresh = false;
+  uint32_t* p = (uint32_t*)scratch_block(kCounterSlot, sizeof(uint32_t) * (size_t)n, s, &fresh);
+  if (p && fresh) {
+    StreamScratch& sc = g_scratch[scratch_key(s)];
+    if (cudaMemsetAsync(p, 0, sc.cap[kCounterSlot], s) != cudaSuccess) {
+      cudaGetLastError();
+      sc.outgrown.push_back(p);
+      sc.ptr[kCounterSlot] = nullptr; sc.cap[kCounterSlot] = 0;
+      return nullptr;
+    }
+  }
+  return p;
+}
+// The stream is idle and about to be destroyed.
+static void release_stream_scratch(cudaStream_t s) {
+  std::vector<void*> blocks;
+  {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    auto it = g_scratch.find(scratch_key(s));
+    if (it == g_scratch.end()) return;
+    blocks = std::move(it->second.outgrown);
+    for (void* p : it->second.ptr) if (p) blocks.push_back(p);
+    g_scratch.erase(it);
+  }
+  for (void* p : blocks) pool_free(p);
 }
 
 static inline size_t data_bytes(const DLArray* a) { return (size_t)numel(a) * 4; }
@@ -451,6 +498,7 @@ int DLGpuDestroycudaStream(void** cudaStream) {
   cudaStream_t s = (cudaStream_t)*cudaStream;
   if (last_compute_stream() == s) note_compute_stream(0);
   TF_CUDA(cudaStreamSynchronize(s));
+  release_stream_scratch(s);
   TF_CUDA(cudaStreamDestroy(s));
   *cudaStream = nullptr;
   return 0;

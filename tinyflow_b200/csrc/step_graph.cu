@@ -23,7 +23,7 @@ int tensor_path_error();
 void tc_recording_begins();
 bool dp_active();
 
-constexpr int kZeroedWords = 12288;       // maxima of a step's tensors: one word per tracked write (Inception-v4: about 900)
+constexpr int kZeroedWords = 16384;       // maxima of a step's tensors, one word per tracked write (Inception-v4: about 900), and arrival counters
 constexpr int kSeedWords = 1022;          // dropout calls of a step
 constexpr int kCarries = 1024;            // parameters whose maximum crosses steps
 
@@ -43,6 +43,9 @@ struct StepGraph {
   long long launches = 0;
   uint64_t epoch = 0;
   uint64_t id = 0;
+  struct { void* ptr = nullptr; size_t cap = 0; } scratch[kScratchSlots];
+  uint32_t* counters = nullptr;
+  int n_counters = 0;
 };
 static std::atomic<uint64_t> g_recordings{0};
 uint64_t recording_id() { return t_recording ? t_recording->id : 0; }
@@ -60,6 +63,25 @@ void* recording_take_block(size_t bytes) {
   return p;
 }
 void recording_keep_block(void* p, size_t bytes) { t_recording->free_blocks[bytes].push_back(p); }
+// An outgrown block goes to the recording's own free blocks: its kernels run in front of those of whoever takes it next.
+void* recording_scratch(int slot, size_t bytes) {
+  auto& sc = t_recording->scratch[slot];
+  if (sc.cap >= bytes) return sc.ptr;
+  if (sc.ptr) pool_free(sc.ptr);
+  sc.ptr = pool_alloc(bytes);
+  sc.cap = sc.ptr ? bytes : 0;
+  return sc.ptr;
+}
+uint32_t* recording_counters(int n) {
+  StepGraph* g = t_recording;
+  if (n > g->n_counters) {
+    int m = 64;
+    while (m < n) m *= 2;
+    if (g->used + m > kZeroedWords) return nullptr;
+    g->counters = g->words + g->used; g->n_counters = m; g->used += m;
+  }
+  return g->counters;
+}
 const uint32_t* recording_seed(unsigned seed) {
   StepGraph* g = t_recording;
   if ((int)g->seeds.size() >= kSeedWords) { g->overflow = true; return g->words; }
@@ -133,6 +155,7 @@ int TfStepRecordEnd(void** graph, int keep) {
   TF_REQUIRE(graph && *graph && t_recording == (StepGraph*)*graph, "TfStepRecordEnd: this thread is not recording that step");
   StepGraph* g = t_recording;
   flush_deferred();
+  for (auto& sc : g->scratch) if (sc.ptr) pool_free(sc.ptr);       // to the graph's own blocks, as all frees of a recording
   bool ok = keep != 0 && !g->overflow;
   if (ok) {
     g->carries.resize(kCarries);
