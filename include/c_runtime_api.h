@@ -356,6 +356,7 @@ int TfTensorPathTimeoutProbe(long long limit_cycles, void **cudaStream);
 int TfLastError(char *buf, int buflen);   /* message of the last -1 return on this thread */
 int TfAllocatorStats(long long *bytes_in_use, long long *bytes_cached);
 int TfReleaseCachedMemory(void);
+int TfSetMemoryLimit(long long bytes);    /* device memory the pool of each GPU may own, cached blocks included; 0 = no limit */
 
 #ifdef __cplusplus
 }

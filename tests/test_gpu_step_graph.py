@@ -182,6 +182,32 @@ def test_a_recording_packs_filters_for_its_own_plans_only(lib_path, monkeypatch)
     assert launches[0] == launches[-1]
 
 
+def test_an_allocation_gets_the_memory_of_recordings(lib_path, monkeypatch):
+    """What a recording keeps for its replays is given up before an allocation fails; the steps go on as ever."""
+    from tinyflow_b200 import gpu_op, ndarray
+    ctx, kept, seen = ndarray.gpu(0), [], {}
+
+    def between(step, model, ex, feed, x):
+        if step == 2:
+            seen["before"] = gpu_op.allocator_stats()[0]             # recorded in the fourth step
+        if step == 6 and ex._recordings.sets and not kept:
+            gpu_op.device_synchronize()
+            gpu_op.release_cached_memory()
+            seen["held"] = gpu_op.allocator_stats()[0] - seen["before"]
+            gpu_op.set_memory_limit(sum(gpu_op.allocator_stats()))
+            try:
+                kept.append(ndarray.empty((seen["held"] // 8,), ctx))
+            finally:
+                gpu_op.set_memory_limit(0)
+
+    def build(m):
+        return m.mlp(batch=512, sizes=(784, 1500, 1000, 10))         # products on the tensor path: packs of both operands
+    got = _train(monkeypatch, True, build, "sgd", between)
+    assert seen["held"] > (1 << 20) and got[2]
+    assert isinstance(kept[0], ndarray.NDArray)                      # an int: the bytes that were short
+    _same(got, _train(monkeypatch, False, build, "sgd"))
+
+
 @pytest.mark.parametrize("count", [1, 5, 400])
 def test_many_updates_in_one_launch(lib_path, count):
     from tinyflow_b200 import gpu_op, ndarray as nd

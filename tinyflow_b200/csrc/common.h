@@ -152,6 +152,7 @@ void* recording_take_block(size_t bytes);          // a block of exactly this (r
 void recording_keep_block(void* p, size_t bytes);  // instead of handing the block back to the pool
 const uint32_t* recording_seed(unsigned seed);     // device word that will hold the seed of this dropout call at every replay
 const float* recording_adam_corrections(float c1, float c2);   // two device words with this step's bias corrections
+bool recordings_give_up_memory();                  // every recording that is not being made returns its blocks to the pool and is out of date; false: there was none
 void recording_note_launches(int n);
 void recording_note_write(const void* p);
 cudaStream_t recording_stream();

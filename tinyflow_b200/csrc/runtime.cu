@@ -183,6 +183,7 @@ void flush_deferred_slow() {
 // can run ahead of, and overlap with, the compute queued in front of its consumer.
 // ---------------------------------------------------------------------------------
 static std::atomic<bool> g_side_copies_seen{false};
+static std::atomic<long long> g_memory_limit{0};          // device bytes a pool may own, 0: what the device has
 struct Pool {
   std::mutex mu;
   std::unordered_map<size_t, std::vector<void*>> free_by_size;
@@ -199,6 +200,8 @@ struct Pool {
     return (b + (size_t(1) << 16) - 1) & ~((size_t(1) << 16) - 1);   // 64 KiB granules above 1 MiB
   }
   cudaError_t raw_alloc(void** p, size_t b) {
+    const long long limit = host ? 0 : g_memory_limit.load(std::memory_order_relaxed);
+    if (limit > 0 && in_use + cached + (long long)b > limit) return cudaErrorMemoryAllocation;
     return host ? cudaHostAlloc(p, b, cudaHostAllocDefault) : cudaMalloc(p, b);
   }
   void raw_free(void* p) { host ? cudaFreeHost(p) : cudaFree(p); }
@@ -222,7 +225,7 @@ struct Pool {
     if (hard) *hard = false;
     size_t b = round(bytes);
     if (t_recording && !host) if (void* p = recording_take_block(b)) return p;      // still counted as in use
-    std::lock_guard<std::mutex> lk(mu);
+    std::unique_lock<std::mutex> lk(mu);
     auto it = free_by_size.find(b);
     if (!unused && it != free_by_size.end() && !it->second.empty()) {
       void* p = it->second.back();
@@ -245,6 +248,14 @@ struct Pool {
       if (!host) cudaDeviceSynchronize();
       release_cached_locked();
       e = raw_alloc(&p, b);
+      if (e != cudaSuccess && !host) {
+        // Then what recorded steps keep for their replays: they can be recorded again, or run as ordinary calls.
+        cudaGetLastError();
+        lk.unlock();
+        const bool some = recordings_give_up_memory();
+        lk.lock();
+        if (some) { release_cached_locked(); e = raw_alloc(&p, b); }
+      }
       if (e != cudaSuccess) { cudaGetLastError(); return nullptr; }
     }
     size_of[p] = b;
@@ -596,6 +607,11 @@ int TfAllocatorStats(long long* bytes_in_use, long long* bytes_cached) {
   std::lock_guard<std::mutex> lk(p.mu);
   if (bytes_in_use) *bytes_in_use = p.in_use;
   if (bytes_cached) *bytes_cached = p.cached;
+  return 0;
+}
+int TfSetMemoryLimit(long long bytes) {
+  TF_REQUIRE(bytes >= 0, "TfSetMemoryLimit: negative limit");
+  g_memory_limit.store(bytes);
   return 0;
 }
 int TfReleaseCachedMemory(void) {

@@ -112,13 +112,34 @@ __global__ void __launch_bounds__(256) step_carry_kernel(const __grid_constant__
 }
 void amax_of_array(const float* src, int64_t n, uint32_t* word, cudaStream_t s);
 
-static void step_graph_free(StepGraph* g) {
+// Finished recordings.  The lock is held while one is replayed, freed or made to give up its memory.
+static std::mutex g_graphs_mu;
+static std::vector<StepGraph*> g_graphs;
+static void step_graph_release(StepGraph* g) {
   if (g->exec) cudaGraphExecDestroy(g->exec);
   if (g->stream) cudaStreamDestroy(g->stream);
   if (g->words) pool_free(g->words);
   for (auto& kv : g->free_blocks) for (void* p : kv.second) pool_free(p);
-  delete g;
+  g->exec = nullptr; g->stream = nullptr; g->words = nullptr;
+  g->free_blocks.clear();
   cudaGetLastError();
+}
+static void step_graph_free(StepGraph* g) {
+  {
+    std::lock_guard<std::mutex> lk(g_graphs_mu);
+    g_graphs.erase(std::remove(g_graphs.begin(), g_graphs.end(), g), g_graphs.end());
+  }
+  step_graph_release(g);
+  delete g;
+}
+bool recordings_give_up_memory() {
+  if (t_recording) return false;         // the blocks would go to the recording, and a capture forbids waiting for the device
+  std::lock_guard<std::mutex> lk(g_graphs_mu);
+  if (g_graphs.empty()) return false;
+  if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return false; }      // no replay is in flight
+  for (StepGraph* g : g_graphs) step_graph_release(g);
+  g_graphs.clear();
+  return true;
 }
 
 }  // namespace tf
@@ -189,6 +210,8 @@ int TfStepRecordEnd(void** graph, int keep) {
   g->written.erase(std::unique(g->written.begin(), g->written.end()), g->written.end());
   std::sort(g->made.begin(), g->made.end());
   g->made.erase(std::unique(g->made.begin(), g->made.end()), g->made.end());
+  std::lock_guard<std::mutex> lk(g_graphs_mu);
+  g_graphs.push_back(g);
   return 0;
 }
 
@@ -197,8 +220,10 @@ int TfStepRecordEnd(void** graph, int keep) {
 // `params` are the arrays the step updates in place: a carried maximum that is out of date is taken from them.
 int TfStepReplay(void* graph, const unsigned* seeds, int nseeds, float b1t, float b2t, const DLArrayHandle* params, int nparams, void** cudaStream) {
   StepGraph* g = (StepGraph*)graph;
-  TF_REQUIRE(g && g->exec && !t_recording, "TfStepReplay: nothing to replay");
+  TF_REQUIRE(g && !t_recording, "TfStepReplay: nothing to replay");
   flush_deferred();
+  std::lock_guard<std::mutex> lk(g_graphs_mu);
+  if (!g->exec) return 1;                // gave up its memory
   if (g->epoch != g_layout_epoch.load()) return 1;
   if (g_timing_level > 0 || g_sync_every_op || dp_active()) return 2;
   TF_REQUIRE(tensor_path_error() == 0, "TfStepReplay: an earlier tensor-core kernel timed out on a barrier; refusing to launch");

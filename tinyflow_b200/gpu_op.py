@@ -491,6 +491,11 @@ def allocator_stats():
     return used.value, cached.value
 
 
+def set_memory_limit(nbytes):
+    """Device memory the pool of each GPU may own, cached blocks included; 0 = no limit."""
+    check_call(_LIB.TfSetMemoryLimit(ctypes.c_longlong(nbytes)))
+
+
 def release_cached_memory():
     """Returns every cached (free) block of the device and pinned-host pools to the driver."""
     check_call(_LIB.TfReleaseCachedMemory())
