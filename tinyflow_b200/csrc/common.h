@@ -54,7 +54,7 @@ struct KernelTimer {
 //  * DLGpuMatrixElementwiseAdd: if the very next call is the ReLU forward of the sum (the end of a residual block), ONE
 //    kernel writes the sum and its ReLU.
 // Every other way into the library - stream_of(), which every operator with a stream argument calls first,
-// last_compute_stream(), which the stream-less operators and the copies call, the array free, the synchronising calls -
+// last_compute_stream() and legacy_stream(), which the stream-less operators and the copies call, the array free, the synchronising calls -
 // launches the held-back kernel first (flush_deferred), so no caller can observe the difference.  One slot, guarded by
 // a mutex; the fast path is one relaxed load.
 //  * DLGpuBroadcastTo0/1 (while a step is recorded): the sum that reads the broadcast joins it in the slot, and the ReLU of
@@ -76,6 +76,7 @@ long long fused_relu_bn_bwd_count();
 long long fused_add_relu_count();
 
 inline cudaStream_t stream_of(void** cell) { flush_deferred(); return cell ? (cudaStream_t)(*cell) : (cudaStream_t)0; }
+inline cudaStream_t legacy_stream() { flush_deferred(); return (cudaStream_t)0; }       // of the operators that the reference runs without a stream
 inline cudaStream_t stream_of_keep_deferred(void** cell) { return cell ? (cudaStream_t)(*cell) : (cudaStream_t)0; }
 void note_compute_stream(cudaStream_t s);   // remembered so side-stream copies can order after compute
 cudaStream_t last_compute_stream();         // launches a held-back kernel first

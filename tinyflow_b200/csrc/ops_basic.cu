@@ -911,8 +911,9 @@ int DLGpuReduceSumAxisZero(const DLArrayHandle input, DLArrayHandle output) {
   TF_REQUIRE(input && output && input->ndim >= 1, "null array");
   int64_t rows = input->shape[0], cols = rows ? numel(input) / rows : 0;
   TF_REQUIRE(numel(output) == (cols ? cols : 1), "DLGpuReduceSumAxisZero: output size mismatch");
-  if (input->ndim == 1) return reduce_to_scalar(F(input), FM(output), rows, 1.f, 0, "DLGpuReduceSumAxisZero");
-  return column_sums(F(input), FM(output), rows, cols, 0, "DLGpuReduceSumAxisZero");
+  const cudaStream_t s = legacy_stream();
+  if (input->ndim == 1) return reduce_to_scalar(F(input), FM(output), rows, 1.f, s, "DLGpuReduceSumAxisZero");
+  return column_sums(F(input), FM(output), rows, cols, s, "DLGpuReduceSumAxisZero");
 }
 // The two legacy "broadcast backward" reductions: sum the leading axes down to the output's
 // shape (trailing broadcast) or sum everything but the channel axis.
@@ -920,13 +921,15 @@ int DLGpuBroadcastToBackward0(const DLArrayHandle input, DLArrayHandle output) {
   TF_REQUIRE(input && output, "null array");
   int64_t nout = numel(output), nin = numel(input);
   TF_REQUIRE(nout > 0 && nin % nout == 0, "DLGpuBroadcastToBackward0: size mismatch");
-  if (nout == 1) return reduce_to_scalar(F(input), FM(output), nin, 1.f, 0, "DLGpuBroadcastToBackward0");
-  return column_sums(F(input), FM(output), nin / nout, nout, 0, "DLGpuBroadcastToBackward0");
+  const cudaStream_t s = legacy_stream();
+  if (nout == 1) return reduce_to_scalar(F(input), FM(output), nin, 1.f, s, "DLGpuBroadcastToBackward0");
+  return column_sums(F(input), FM(output), nin / nout, nout, s, "DLGpuBroadcastToBackward0");
 }
 int DLGpuBroadcastToBackward1(const DLArrayHandle input, DLArrayHandle output) {
   TF_REQUIRE(input && output && input->ndim >= 2 && output->ndim == 1 && output->shape[0] == input->shape[1], "DLGpuBroadcastToBackward1: output must be (C,)");
   const int64_t C = input->shape[1], N = input->shape[0];
-  return channel_sums(F(input), FM(output), N, C, N && C ? numel(input) / (N * C) : 0, 0, "DLGpuBroadcastToBackward1");
+  const cudaStream_t s = legacy_stream();
+  return channel_sums(F(input), FM(output), N, C, N && C ? numel(input) / (N * C) : 0, s, "DLGpuBroadcastToBackward1");
 }
 int DLGpuReduceSumAxisN(const DLArrayHandle input, DLArrayHandle output, const int axis) {
   TF_REQUIRE(input && output && axis >= 0 && axis < input->ndim, "DLGpuReduceSumAxisN: bad axis");
@@ -934,9 +937,10 @@ int DLGpuReduceSumAxisN(const DLArrayHandle input, DLArrayHandle output, const i
   for (int i = 0; i < axis; ++i) outer *= input->shape[i];
   for (int i = axis + 1; i < input->ndim; ++i) inner *= input->shape[i];
   TF_REQUIRE(numel(output) == outer * inner, "DLGpuReduceSumAxisN: output size mismatch");
-  note_compute_stream(0);
-  axis_sum_kernel<<<grid_for(outer * inner, kBlock), kBlock>>>(F(input), FM(output), outer, red, inner);
-  TF_AFTER(0, "DLGpuReduceSumAxisN");
+  cudaStream_t s = legacy_stream();
+  note_compute_stream(s);
+  axis_sum_kernel<<<grid_for(outer * inner, kBlock), kBlock, 0, s>>>(F(input), FM(output), outer, red, inner);
+  TF_AFTER(s, "DLGpuReduceSumAxisN");
   return 0;
 }
 int DLGpuReduceSumAxisNBackward(const DLArrayHandle input, DLArrayHandle output, const int axis) {
@@ -945,14 +949,16 @@ int DLGpuReduceSumAxisNBackward(const DLArrayHandle input, DLArrayHandle output,
   for (int i = 0; i < axis; ++i) outer *= output->shape[i];
   for (int i = axis + 1; i < output->ndim; ++i) inner *= output->shape[i];
   TF_REQUIRE(numel(input) == outer * inner, "DLGpuReduceSumAxisNBackward: input size mismatch");
-  note_compute_stream(0);
-  axis_bcast_kernel<<<grid_for(numel(output), kBlock), kBlock>>>(F(input), FM(output), outer, red, inner);
-  TF_AFTER(0, "DLGpuReduceSumAxisNBackward");
+  cudaStream_t s = legacy_stream();
+  note_compute_stream(s);
+  axis_bcast_kernel<<<grid_for(numel(output), kBlock), kBlock, 0, s>>>(F(input), FM(output), outer, red, inner);
+  TF_AFTER(s, "DLGpuReduceSumAxisNBackward");
   return 0;
 }
 int DLGpuReduceSumAll(const DLArrayHandle input, DLArrayHandle output) {
   TF_REQUIRE(input && output && numel(output) == 1, "DLGpuReduceSumAll: output must hold one element");
-  return reduce_to_scalar(F(input), FM(output), numel(input), 1.f, 0, "DLGpuReduceSumAll");
+  const cudaStream_t s = legacy_stream();
+  return reduce_to_scalar(F(input), FM(output), numel(input), 1.f, s, "DLGpuReduceSumAll");
 }
 }  // extern "C" (reopened below)
 
@@ -1016,9 +1022,10 @@ int DLGpuReduceSumAllStatic(const DLArrayHandle input, DLArrayHandle output, voi
 int DLGpuReduceSumAllBackward(const DLArrayHandle input, DLArrayHandle output) {
   TF_REQUIRE(input && output && numel(input) >= 1, "null array");
   int64_t total = numel(output);
-  note_compute_stream(0);
-  bcast_tail_kernel<<<grid_for(total, kBlock), kBlock>>>(F(input), FM(output), 1, total);
-  TF_AFTER(0, "DLGpuReduceSumAllBackward");
+  cudaStream_t s = legacy_stream();
+  note_compute_stream(s);
+  bcast_tail_kernel<<<grid_for(total, kBlock), kBlock, 0, s>>>(F(input), FM(output), 1, total);
+  TF_AFTER(s, "DLGpuReduceSumAllBackward");
   return 0;
 }
 
