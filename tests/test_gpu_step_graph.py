@@ -153,6 +153,23 @@ def test_resident_batches_in_turn(lib_path, monkeypatch, name, order, held_from)
     _same(got, _train(monkeypatch, False, CONV_FIRST[name], "sgd", _in_turn(order, held_from)))
 
 
+def _column_sums_model(m):
+    """A loss over ReduceSumAxisZero, which the reference runs without a stream."""
+    from tinyflow_b200 import autodiff as ad
+    X, y_, W = ad.Placeholder("X"), ad.Placeholder("y_"), ad.Variable("W")
+    y = ad.matmul_op(X, W)
+    sums = ad.reducesumaxiszero_op(ad.mul_op(y, y_))
+    loss = ad.reduce_sum_op(ad.mul_op(sums, sums))
+    return m.Model("column sums", X, y_, loss, y, {W: (20, 7)}, (33, 20), (33, 7))
+
+
+@pytest.mark.parametrize("optimizer", ["sgd", "adam"])
+def test_operators_without_a_stream_are_part_of_the_recording(lib_path, monkeypatch, optimizer):
+    got = _train(monkeypatch, True, _column_sums_model, optimizer, _overwrite_inputs)
+    assert got[2]
+    _same(got, _train(monkeypatch, False, _column_sums_model, optimizer, _overwrite_inputs))
+
+
 @pytest.mark.parametrize("name", ["mlp", "vgg16"])
 def test_new_mini_batch_arrays_every_step(lib_path, monkeypatch, name):
     want = _train(monkeypatch, False, BUILDS[name], "sgd", fresh_batch=True)

@@ -76,7 +76,7 @@ long long fused_relu_bn_bwd_count();
 long long fused_add_relu_count();
 
 inline cudaStream_t stream_of(void** cell) { flush_deferred(); return cell ? (cudaStream_t)(*cell) : (cudaStream_t)0; }
-inline cudaStream_t legacy_stream() { flush_deferred(); return (cudaStream_t)0; }       // of the operators that the reference runs without a stream
+cudaStream_t legacy_stream();               // of the operators that the reference runs without a stream: the legacy default stream, in a recording the recording's
 inline cudaStream_t stream_of_keep_deferred(void** cell) { return cell ? (cudaStream_t)(*cell) : (cudaStream_t)0; }
 void note_compute_stream(cudaStream_t s);   // remembered so side-stream copies can order after compute
 cudaStream_t last_compute_stream();         // launches a held-back kernel first
@@ -157,6 +157,7 @@ bool recordings_give_up_memory();                  // every recording that is no
 void recording_note_launches(int n);
 void recording_note_write(const void* p);
 cudaStream_t recording_stream();
+void recording_refuse(const char* why);            // the step cannot be recorded: End gives this reason
 // Buffers that outlive a call (packs) were reallocated or the arithmetic changed: recorded steps are out of date.
 void bump_layout_epoch();
 

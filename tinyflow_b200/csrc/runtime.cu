@@ -99,7 +99,11 @@ void KernelTimer::end() {
 }
 
 static std::atomic<cudaStream_t> g_compute_stream{(cudaStream_t)0};
-void note_compute_stream(cudaStream_t s) { if (!t_recording) g_compute_stream.store(s, std::memory_order_relaxed); }     // a recording's stream concerns nobody else
+void note_compute_stream(cudaStream_t s) {
+  if (!t_recording) g_compute_stream.store(s, std::memory_order_relaxed);                 // a recording's stream concerns nobody else
+  else if (s != recording_stream()) recording_refuse("an operator was called on another stream than the recording's");      // it has run, and no replay would run it
+}
+cudaStream_t legacy_stream() { flush_deferred(); return t_recording ? recording_stream() : (cudaStream_t)0; }
 cudaStream_t last_compute_stream() { flush_deferred(); return t_recording ? recording_stream() : g_compute_stream.load(std::memory_order_relaxed); }
 
 // ---- the held-back elementwise call (see common.h) ----------------------------------------------
@@ -447,6 +451,10 @@ int DLArrayFree(DLArrayHandle handle) {
 int DLArrayCopyFromTo(DLArrayHandle from, DLArrayHandle to, DLStreamHandle stream) {
   flush_deferred();
   TF_REQUIRE(from && to && from->data && to->data, "DLArrayCopyFromTo: null array");
+  if (t_recording && (stream == nullptr || *(cudaStream_t*)stream != recording_stream() || from->ctx.device_type != kGPU || to->ctx.device_type != kGPU)) {
+    recording_refuse("a copy that the host waits for");
+    TF_FAIL("DLArrayCopyFromTo: a copy that the host waits for cannot be recorded");
+  }
   size_t bytes = data_bytes(from);
   TF_REQUIRE(bytes == data_bytes(to), "DLArrayCopyFromTo: size mismatch (%zu vs %zu bytes)", bytes, data_bytes(to));
   const bool fg = from->ctx.device_type == kGPU, tg = to->ctx.device_type == kGPU;

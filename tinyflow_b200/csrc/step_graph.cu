@@ -32,7 +32,7 @@ struct StepGraph {
   cudaGraphExec_t exec = nullptr;
   uint32_t* words = nullptr;              // [zeroed words][c1, c2][seeds]
   int used = 0;
-  bool overflow = false;
+  const char* refused = nullptr;          // why the step cannot be recorded
   std::vector<unsigned> seeds;            // of the recorded step, in call order
   bool has_adam = false;
   float c1 = 0.f, c2 = 0.f;
@@ -50,9 +50,10 @@ struct StepGraph {
 static std::atomic<uint64_t> g_recordings{0};
 uint64_t recording_id() { return t_recording ? t_recording->id : 0; }
 
+void recording_refuse(const char* why) { if (!t_recording->refused) t_recording->refused = why; }
 uint32_t* recording_word() {
   StepGraph* g = t_recording;
-  if (g->used >= kZeroedWords) { g->overflow = true; return g->words; }
+  if (g->used >= kZeroedWords) { recording_refuse("more tracked tensors than a recording has words for"); return g->words; }
   return g->words + g->used++;
 }
 void* recording_take_block(size_t bytes) {
@@ -84,13 +85,13 @@ uint32_t* recording_counters(int n) {
 }
 const uint32_t* recording_seed(unsigned seed) {
   StepGraph* g = t_recording;
-  if ((int)g->seeds.size() >= kSeedWords) { g->overflow = true; return g->words; }
+  if ((int)g->seeds.size() >= kSeedWords) { recording_refuse("more dropout calls than a recording has seeds for"); return g->words; }
   g->seeds.push_back(seed);
   return g->words + kZeroedWords + 2 + g->seeds.size() - 1;
 }
 const float* recording_adam_corrections(float c1, float c2) {
   StepGraph* g = t_recording;
-  if (g->has_adam && (g->c1 != c1 || g->c2 != c2)) g->overflow = true;      // one pair per step
+  if (g->has_adam && (g->c1 != c1 || g->c2 != c2)) recording_refuse("two pairs of Adam's bias corrections in one step");
   g->has_adam = true; g->c1 = c1; g->c2 = c2;
   return reinterpret_cast<const float*>(g->words + kZeroedWords);
 }
@@ -166,7 +167,7 @@ int TfStepRecordBegin(void** graph, void** stream_cell) {
   tc_recording_begins();
   *graph = g;
   *stream_cell = (void*)g->stream;
-  if (cudaMemsetAsync(g->words, 0, sizeof(uint32_t) * kZeroedWords, g->stream) != cudaSuccess) g->overflow = true;
+  if (cudaMemsetAsync(g->words, 0, sizeof(uint32_t) * kZeroedWords, g->stream) != cudaSuccess) recording_refuse("the capture failed");
   return 0;
 }
 
@@ -177,11 +178,12 @@ int TfStepRecordEnd(void** graph, int keep) {
   StepGraph* g = t_recording;
   flush_deferred();
   for (auto& sc : g->scratch) if (sc.ptr) pool_free(sc.ptr);       // to the graph's own blocks, as all frees of a recording
-  bool ok = keep != 0 && !g->overflow;
+  bool ok = keep != 0 && !g->refused;
   if (ok) {
     g->carries.resize(kCarries);
     int n = 0;
     ok = amax_take_carries(g, g->carries.data(), kCarries, &n);
+    if (!ok) recording_refuse("more parameters with a tracked maximum than a recording carries");
     g->carries.resize(n);
     CarryList list;
     int m = 0;
@@ -194,13 +196,17 @@ int TfStepRecordEnd(void** graph, int keep) {
   }
   cudaGraph_t raw = nullptr;
   cudaError_t e = cudaStreamEndCapture(g->stream, &raw);
-  t_recording = nullptr;
-  if (e != cudaSuccess || !raw) ok = false;
-  if (ok && cudaGraphInstantiate(&g->exec, raw, 0) != cudaSuccess) ok = false;
+  if (e != cudaSuccess || !raw) { ok = false; recording_refuse(cudaGetErrorString(e)); }
+  if (ok) {
+    e = cudaGraphInstantiate(&g->exec, raw, 0);
+    if (e != cudaSuccess) { ok = false; recording_refuse(cudaGetErrorString(e)); }
+  }
   if (raw) cudaGraphDestroy(raw);
-  ok = ok && g->epoch == g_layout_epoch.load();
+  if (ok && g->epoch != g_layout_epoch.load()) { ok = false; recording_refuse("packed operands moved while the step was recorded"); }
+  t_recording = nullptr;
   if (!ok) {
     cudaGetLastError();
+    if (keep) set_error("the step cannot be recorded: %s", g->refused);       // an abandoned recording keeps the error that stopped it
     invalidate_all_versions();       // calls of the recording marked operands as packed; nothing ran
     step_graph_free(g);
     *graph = nullptr;
