@@ -178,6 +178,33 @@ def test_new_mini_batch_arrays_every_step(lib_path, monkeypatch, name):
     _same(got, want)
 
 
+def test_another_thread_waits_for_the_device_while_a_step_is_recorded(lib_path, monkeypatch):
+    """Neither the recordings nor the waits fail; the waiting thread shares no array with the step."""
+    import threading
+    from tinyflow_b200 import gpu_op
+    want = _train(monkeypatch, False, BUILDS["lenet5"], "sgd", fresh_batch=True)
+    stop, errors, waits = threading.Event(), [], [0]
+
+    def wait():
+        while not stop.is_set():
+            try:
+                gpu_op.device_synchronize()
+                waits[0] += 1
+            except Exception as e:                                   # noqa: BLE001
+                errors.append(e)
+    thread = threading.Thread(target=wait)
+    thread.start()
+    try:
+        got = [_train(monkeypatch, True, BUILDS["lenet5"], "sgd", fresh_batch=True) for _ in range(8)]
+    finally:
+        stop.set()
+        thread.join()
+    assert not errors and waits[0] > 0
+    for run in got:
+        assert run[2]
+        _same(run, want)
+
+
 def test_a_recording_packs_filters_for_its_own_plans_only(lib_path, monkeypatch):
     """Batches of other sizes build other plans; a step recorded after them has the launches it had before them."""
     from tinyflow_b200 import autodiff as ad, gpu_op, models, ndarray, step_graph

@@ -81,6 +81,12 @@ inline cudaStream_t stream_of_keep_deferred(void** cell) { return cell ? (cudaSt
 void note_compute_stream(cudaStream_t s);   // remembered so side-stream copies can order after compute
 cudaStream_t last_compute_stream();         // launches a held-back kernel first
 
+// ---- waiting for the device ----------------------------------------------------------
+cudaError_t device_wait();                  // cudaDeviceSynchronize, between the recordings of other threads; an error inside a recording
+void capture_begins();
+void capture_ends();
+struct CaptureExclusion { CaptureExclusion(); ~CaptureExclusion(); };       // no other thread captures while one lives
+
 // ---- write versions -------------------------------------------------------------
 // Every entry point that writes a device array bumps the version of its data pointer; cached
 // derived data (packed tensor-core operands) is valid only while the version is unchanged.

@@ -83,8 +83,10 @@ static uint32_t* amax_chunk_words(int n) {
   if (g_amax_left < n) {
     const int kWords = 16384;
     uint32_t* chunk = nullptr;
-    if (cudaMalloc((void**)&chunk, kWords * sizeof(uint32_t)) != cudaSuccess || cudaMemset(chunk, 0, kWords * sizeof(uint32_t)) != cudaSuccess ||
-        cudaDeviceSynchronize() != cudaSuccess) {
+    // cleared on a stream of its own: the words are needed on any stream, and a recording forbids waiting for the device
+    static cudaStream_t clearing = nullptr;
+    if ((!clearing && cudaStreamCreateWithFlags(&clearing, cudaStreamNonBlocking) != cudaSuccess) || cudaMalloc((void**)&chunk, kWords * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMemsetAsync(chunk, 0, kWords * sizeof(uint32_t), clearing) != cudaSuccess || cudaStreamSynchronize(clearing) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }

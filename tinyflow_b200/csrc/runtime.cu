@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <shared_mutex>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -96,6 +97,19 @@ void KernelTimer::begin(const char* family, double flops, double bytes) {
 void KernelTimer::end() {
   std::lock_guard<std::mutex> lk(g_kt_mu);
   if (slot >= 0 && slot < (int)g_pending.size()) cudaEventRecord(g_pending[slot].b, stream);
+}
+
+// A wait for the whole device is an error while any stream of it is captured, and ends the capture: such waits take turns with
+// the recordings of other threads (which issue calls and wait for nothing).  No lock of the library may be held around one.
+static std::shared_mutex g_capture_mu;
+void capture_begins() { g_capture_mu.lock_shared(); }
+void capture_ends() { g_capture_mu.unlock_shared(); }
+CaptureExclusion::CaptureExclusion() { g_capture_mu.lock(); }
+CaptureExclusion::~CaptureExclusion() { g_capture_mu.unlock(); }
+cudaError_t device_wait() {
+  if (t_recording) return cudaErrorStreamCaptureUnsupported;
+  CaptureExclusion turn;
+  return cudaDeviceSynchronize();
 }
 
 static std::atomic<cudaStream_t> g_compute_stream{(cudaStream_t)0};
@@ -248,8 +262,9 @@ struct Pool {
     }
     if (e != cudaSuccess) {
       cudaGetLastError();
+      if (t_recording && !host) return nullptr;            // what follows waits for the device: the step is not recorded
       // Give cached blocks back to the driver and try once more before reporting OOM.
-      if (!host) cudaDeviceSynchronize();
+      if (!host) { lk.unlock(); device_wait(); lk.lock(); }
       release_cached_locked();
       e = raw_alloc(&p, b);
       if (e != cudaSuccess && !host) {
@@ -334,40 +349,33 @@ static std::map<std::pair<int, std::pair<cudaStream_t, size_t>>, StreamScratch> 
 static std::pair<int, std::pair<cudaStream_t, size_t>> scratch_key(cudaStream_t s) {        // a per-thread stream is another one in every thread
   return {current_device(), {s, s == cudaStreamPerThread ? std::hash<std::thread::id>()(std::this_thread::get_id()) : 0}};
 }
-static void* scratch_block(int slot, size_t bytes, cudaStream_t s, bool* fresh) {           // g_scratch_mu held
-  StreamScratch& sc = g_scratch[scratch_key(s)];
-  if (sc.cap[slot] >= bytes) return sc.ptr[slot];
-  const size_t want = std::max(bytes + bytes / 4, sc.cap[slot] + sc.cap[slot] / 2);
+static void* scratch_block(int slot, size_t bytes, cudaStream_t s) {
+  const auto key = scratch_key(s);
+  std::unique_lock<std::mutex> lk(g_scratch_mu);
+  StreamScratch* sc = &g_scratch[key];
+  if (sc->cap[slot] >= bytes) return sc->ptr[slot];
+  const size_t want = std::max(bytes + bytes / 4, sc->cap[slot] + sc->cap[slot] / 2), got = Pool::round(want);
+  lk.unlock();
   void* p = device_pool().alloc(want, nullptr, true);
+  if (p && slot == kCounterSlot && cudaMemsetAsync(p, 0, got, s) != cudaSuccess) { cudaGetLastError(); pool_free(p); p = nullptr; }
   if (!p) return nullptr;
-  if (sc.ptr[slot]) sc.outgrown.push_back(sc.ptr[slot]);
-  sc.ptr[slot] = p;
-  sc.cap[slot] = Pool::round(want);
-  *fresh = true;
+  lk.lock();
+  sc = &g_scratch[key];
+  if (sc->cap[slot] >= got) {              // another thread of this stream was faster
+    sc->outgrown.push_back(p);
+    return sc->ptr[slot];
+  }
+  if (sc->ptr[slot]) sc->outgrown.push_back(sc->ptr[slot]);
+  sc->ptr[slot] = p;
+  sc->cap[slot] = got;
   return p;
 }
 void* stream_scratch(int slot, size_t bytes, cudaStream_t s) {
   if (slot < 0 || slot >= kScratchSlots) return nullptr;
-  if (t_recording) return recording_scratch(slot, bytes);
-  std::lock_guard<std::mutex> lk(g_scratch_mu);
-  bool fresh = false;
-  return scratch_block(slot, bytes, s, &fresh);
+  return t_recording ? recording_scratch(slot, bytes) : scratch_block(slot, bytes, s);
 }
 uint32_t* arrival_counters(int n, cudaStream_t s) {
-  if (t_recording) return recording_counters(n);
-  std::lock_guard<std::mutex> lk(g_scratch_mu);
-  bool fresh = false;
-  uint32_t* p = (uint32_t*)scratch_block(kCounterSlot, sizeof(uint32_t) * (size_t)n, s, &fresh);
-  if (p && fresh) {
-    StreamScratch& sc = g_scratch[scratch_key(s)];
-    if (cudaMemsetAsync(p, 0, sc.cap[kCounterSlot], s) != cudaSuccess) {
-      cudaGetLastError();
-      sc.outgrown.push_back(p);
-      sc.ptr[kCounterSlot] = nullptr; sc.cap[kCounterSlot] = 0;
-      return nullptr;
-    }
-  }
-  return p;
+  return t_recording ? recording_counters(n) : (uint32_t*)scratch_block(kCounterSlot, sizeof(uint32_t) * (size_t)n, s);
 }
 // The stream is idle and about to be destroyed.
 static void release_stream_scratch(cudaStream_t s) {
@@ -562,7 +570,7 @@ int testPcie(void) {
     cudaMemcpy(dst, src, bytes, k);   // warm-up
     auto t0 = std::chrono::steady_clock::now();
     for (int i = 0; i < 4; ++i) cudaMemcpy(dst, src, bytes, k);
-    cudaDeviceSynchronize();
+    device_wait();
     double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return 4.0 * bytes / s / 1e9;
   };
@@ -601,7 +609,8 @@ int TfKernelTimingReport(char* buf, int buflen) {
 
 int TfDeviceSynchronize(void) {
   flush_deferred();
-  TF_CUDA(cudaDeviceSynchronize());
+  if (t_recording) recording_refuse("a wait for the device");
+  TF_CUDA(device_wait());
   TF_REQUIRE(tensor_path_error() == 0, "a tensor-core kernel timed out waiting on a barrier (results of that launch are invalid)");
   return 0;
 }
@@ -623,7 +632,8 @@ int TfSetMemoryLimit(long long bytes) {
   return 0;
 }
 int TfReleaseCachedMemory(void) {
-  cudaDeviceSynchronize();
+  if (t_recording) return 0;               // its steps may use any of the blocks
+  device_wait();
   { Pool& p = device_pool(); std::lock_guard<std::mutex> lk(p.mu); p.release_cached_locked(); }
   { Pool& p = host_pool(); std::lock_guard<std::mutex> lk(p.mu); p.release_cached_locked(); }
   return 0;

@@ -135,6 +135,7 @@ static void step_graph_free(StepGraph* g) {
 }
 bool recordings_give_up_memory() {
   if (t_recording) return false;         // the blocks would go to the recording, and a capture forbids waiting for the device
+  CaptureExclusion turn;                 // in front of the lock, which a thread that records takes when it drops an older recording
   std::lock_guard<std::mutex> lk(g_graphs_mu);
   if (g_graphs.empty()) return false;
   if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return false; }      // no replay is in flight
@@ -157,7 +158,9 @@ int TfStepRecordBegin(void** graph, void** stream_cell) {
   StepGraph* g = new StepGraph;
   g->words = (uint32_t*)pool_alloc(sizeof(uint32_t) * (kZeroedWords + 2 + kSeedWords));
   if (!g->words) { delete g; return 1; }
+  capture_begins();
   if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess || cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
+    capture_ends();
     step_graph_free(g);
     TF_FAIL("TfStepRecordBegin: stream capture is not available");
   }
@@ -196,6 +199,7 @@ int TfStepRecordEnd(void** graph, int keep) {
   }
   cudaGraph_t raw = nullptr;
   cudaError_t e = cudaStreamEndCapture(g->stream, &raw);
+  capture_ends();
   if (e != cudaSuccess || !raw) { ok = false; recording_refuse(cudaGetErrorString(e)); }
   if (ok) {
     e = cudaGraphInstantiate(&g->exec, raw, 0);
