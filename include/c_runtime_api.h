@@ -314,7 +314,7 @@ int TfArrayCopyOnStream(DLArrayHandle from, DLArrayHandle to, void **cudaStream)
 
 /* Recording a step and replaying it with one call.  Between Begin and End the calling thread issues the step's calls on
  * the stream Begin returns; they are recorded, not executed.  The arrays the calls name have to outlive the recording.
- * Calls that need the host in the middle (blocking copies, the legacy default stream) cannot be recorded: End returns 1
+ * Copies that the host waits for, and calls on other streams, cannot be recorded: they fail or do nothing, and End returns 1
  * then, as it does with keep = 0.  TfStepReplay: `seeds` for the dropout calls in order, Adam's beta powers of this step;
  * 0 = enqueued, 1 = out of date, record again (buffers moved or the arithmetic changed), 2 = not now (per-kernel timing
  * or the data-parallel exchange is on): use ordinary calls. */

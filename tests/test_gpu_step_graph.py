@@ -179,27 +179,30 @@ def test_new_mini_batch_arrays_every_step(lib_path, monkeypatch, name):
 
 
 def test_another_thread_waits_for_the_device_while_a_step_is_recorded(lib_path, monkeypatch):
-    """Neither the recordings nor the waits fail; the waiting thread shares no array with the step."""
+    """Neither the recordings nor the waits fail, whichever library waits; the waiting thread shares no array with the step."""
     import threading
+    import torch
     from tinyflow_b200 import gpu_op
     want = _train(monkeypatch, False, BUILDS["lenet5"], "sgd", fresh_batch=True)
-    stop, errors, waits = threading.Event(), [], [0]
+    stop, errors, waits = threading.Event(), [], []
 
-    def wait():
+    def wait(synchronize):
         while not stop.is_set():
             try:
-                gpu_op.device_synchronize()
-                waits[0] += 1
+                synchronize()
+                waits.append(1)
             except Exception as e:                                   # noqa: BLE001
                 errors.append(e)
-    thread = threading.Thread(target=wait)
-    thread.start()
+    threads = [threading.Thread(target=wait, args=(f,)) for f in (gpu_op.device_synchronize, torch.cuda.synchronize)]
+    for t in threads:
+        t.start()
     try:
         got = [_train(monkeypatch, True, BUILDS["lenet5"], "sgd", fresh_batch=True) for _ in range(8)]
     finally:
         stop.set()
-        thread.join()
-    assert not errors and waits[0] > 0
+        for t in threads:
+            t.join()
+    assert not errors and waits
     for run in got:
         assert run[2]
         _same(run, want)

@@ -6,6 +6,7 @@
 #include <stdlib.h>
 #include <string.h>
 #include <atomic>
+#include <tuple>
 #include "../../include/c_runtime_api.h"
 
 namespace tf {
@@ -81,12 +82,6 @@ inline cudaStream_t stream_of_keep_deferred(void** cell) { return cell ? (cudaSt
 void note_compute_stream(cudaStream_t s);   // remembered so side-stream copies can order after compute
 cudaStream_t last_compute_stream();         // launches a held-back kernel first
 
-// ---- waiting for the device ----------------------------------------------------------
-cudaError_t device_wait();                  // cudaDeviceSynchronize, between the recordings of other threads; an error inside a recording
-void capture_begins();
-void capture_ends();
-struct CaptureExclusion { CaptureExclusion(); ~CaptureExclusion(); };       // no other thread captures while one lives
-
 // ---- write versions -------------------------------------------------------------
 // Every entry point that writes a device array bumps the version of its data pointer; cached
 // derived data (packed tensor-core operands) is valid only while the version is unchanged.
@@ -139,8 +134,8 @@ bool contraction_path_is_cuda_cores();
 int contraction_path();
 
 // ---- recording a training step for replay (step_graph.cu) -----------------------------------------
-// While a step is recorded, its calls (of ONE thread) run on a private stream in capture mode and nothing executes; the
-// launch sequence becomes a CUDA graph that later replays the step with one host call.  What a call would keep on the
+// While a step is recorded, its calls (of ONE thread) name a private stream; nothing executes, but every launch, fill and copy
+// adds a node to a CUDA graph that later replays the step with one host call.  What a call would keep on the
 // host from one step to the next has to be fixed for the graph instead:
 //  * scratch blocks freed during the recording stay with the graph (its kernels use their addresses at every replay);
 //  * a tracked maximum gets a device word of the graph's own, cleared at the start of every replay, in place of the pair
@@ -204,30 +199,61 @@ inline int grid_for(int64_t work_items, int block, int per_thread = 1, int waves
   return (int)need;
 }
 
-// ---- programmatic dependent launch ---------------------------------------------------------
+// ---- launches ------------------------------------------------------------------------------
+// Every kernel that a step can contain is launched through one of these: while a step is recorded they add a node to its graph
+// instead.  launch_plain() is <<<>>>.
+//
 // A kernel launched through launch_dep() may be scheduled while the kernel in front of it on the stream is still
 // draining; its first statement has to be grid_dep_sync(), which blocks until that kernel has completed and its
 // writes are visible, and then lets the kernel behind start the same way.  Removes the launch gap between the
-// ~700 short kernels of a step; a kernel launched with <<<>>> serialises as usual.
+// ~700 short kernels of a step; a kernel launched with launch_plain() serialises as usual.  launch_cluster() is
+// launch_dep() with clusters of that many blocks along x.
 #ifdef __CUDACC__
 __device__ __forceinline__ void grid_dep_sync() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+struct LaunchShape { dim3 grid, block; size_t smem; bool dependent; int cluster; };
+cudaError_t recording_add_kernel(const void* kernel, const LaunchShape& l, void** args, cudaStream_t s);
 template <class... Params, class... Args>
-inline cudaError_t launch_dep(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+inline cudaError_t launch_shaped(void (*kernel)(Params...), LaunchShape l, cudaStream_t s, Args... args) {
   static const bool off = getenv("TINYFLOW_NO_DEPENDENT_LAUNCH") != nullptr;
+  if (off || s == (cudaStream_t)0) l.dependent = false;              // the legacy default stream keeps plain stream order
+  if (t_recording) {
+    std::tuple<Params...> values(static_cast<Params>(args)...);
+    return std::apply([&](auto&... v) { void* pointers[] = {(void*)&v...}; return recording_add_kernel((const void*)kernel, l, pointers, s); }, values);
+  }
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = s;
-  cudaLaunchAttribute attr;
-  memset(&attr, 0, sizeof(attr));
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = &attr; cfg.numAttrs = (off || s == (cudaStream_t)0) ? 0 : 1;      // the legacy default stream keeps plain stream order
+  cfg.gridDim = l.grid; cfg.blockDim = l.block; cfg.dynamicSmemBytes = l.smem; cfg.stream = s;
+  cudaLaunchAttribute attrs[2];
+  memset(attrs, 0, sizeof(attrs));
+  cfg.attrs = attrs;
+  if (l.dependent) {
+    attrs[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attrs[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (l.cluster > 0) {
+    attrs[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attrs[cfg.numAttrs].val.clusterDim.x = l.cluster; attrs[cfg.numAttrs].val.clusterDim.y = 1; attrs[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   return cudaLaunchKernelEx(&cfg, kernel, Params(args)...);
 }
+template <class... Params, class... Args>
+inline cudaError_t launch_dep(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  return launch_shaped(kernel, LaunchShape{grid, block, smem, true, 0}, s, args...);
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_plain(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  return launch_shaped(kernel, LaunchShape{grid, block, smem, false, 0}, s, args...);
+}
+template <class... Params, class... Args>
+inline cudaError_t launch_cluster(void (*kernel)(Params...), int cluster, dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
+  return launch_shaped(kernel, LaunchShape{grid, block, smem, true, cluster}, s, args...);
+}
 #endif
+cudaError_t clear_on_stream(void* p, size_t bytes, cudaStream_t s);                       // cudaMemsetAsync(p, 0, bytes, s), and its node
+cudaError_t copy_on_stream(void* to, const void* from, size_t bytes, cudaStream_t s);     // device to device
 
 // ---- plan structs stored in slot 0 of a descriptor list ----------------------
 enum PlanKind : int { kPlanConv = 0x7f01, kPlanPool, kPlanAct, kPlanReduce, kPlanBN, kPlanTensor, kPlanDropout };

@@ -176,13 +176,13 @@ static int launch_contract(AV A, BV B, OV O, int64_t M, int64_t N, int64_t K, fl
     float* part = (float*)stream_scratch(3, sizeof(float) * (size_t)splits * (size_t)M * (size_t)N, s);
     if (!part) { splits = 1; kps = (K + BK - 1) / BK * BK; grid.z = 1; }       // no scratch: run unsplit
     else {
-      contract_kernel<AV, BV, OV, B_KFAST, true><<<grid, 256, 0, s>>>(A, B, O, M, N, K, kps, part);
-      contract_reduce_kernel<OV><<<grid_for(M * N, 256), 256, 0, s>>>(part, O, M, N, splits);
+      launch_plain(contract_kernel<AV, BV, OV, B_KFAST, true>, grid, dim3(256), 0, s, A, B, O, M, N, K, kps, part);
+      launch_plain(contract_reduce_kernel<OV>, dim3(grid_for(M * N, 256)), dim3(256), 0, s, part, O, M, N, splits);
       if (after_launch(s, what, 2) != 0) return -1;
       return 0;
     }
   }
-  contract_kernel<AV, BV, OV, B_KFAST, false><<<grid, 256, 0, s>>>(A, B, O, M, N, K, kps, nullptr);
+  launch_plain(contract_kernel<AV, BV, OV, B_KFAST, false>, grid, dim3(256), 0, s, A, B, O, M, N, K, kps, nullptr);
   TF_AFTER(s, what);
   return 0;
 }

@@ -152,23 +152,11 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) simt_gemm_kernel(const 
 
 template <int BM, int BN, int TM, int TN, int BK, bool AK, bool BKF>
 static cudaError_t launch_simt(const SimtGemm& p, int cluster, cudaStream_t s) {
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3((unsigned)cluster * ((p.N + BN - 1) / BN), (p.M + BM - 1) / BM);
-  cfg.blockDim = dim3((BM / TM) * (BN / TN));
-  cfg.stream = s;
   if (cluster > 8) {
     static const cudaError_t allowed = cudaFuncSetAttribute(simt_gemm_kernel<BM, BN, TM, TN, BK, AK, BKF>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (allowed != cudaSuccess) return allowed;
   }
-  cudaLaunchAttribute attrs[2];
-  memset(attrs, 0, sizeof(attrs));
-  attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = cluster; attrs[0].val.clusterDim.y = 1; attrs[0].val.clusterDim.z = 1;
-  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attrs[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attrs; cfg.numAttrs = s == (cudaStream_t)0 ? 1 : 2;
-  return cudaLaunchKernelEx(&cfg, simt_gemm_kernel<BM, BN, TM, TN, BK, AK, BKF>, p);
+  return launch_cluster(simt_gemm_kernel<BM, BN, TM, TN, BK, AK, BKF>, cluster, dim3((unsigned)cluster * ((p.N + BN - 1) / BN), (p.M + BM - 1) / BM), dim3((BM / TM) * (BN / TN)), 0, s, p);
 }
 template <int BM, int BN, int TM, int TN, int BK>
 static cudaError_t launch_simt_layout(const SimtGemm& p, bool a_kfast, bool b_kfast, int cluster, cudaStream_t s) {

@@ -83,10 +83,12 @@ static uint32_t* amax_chunk_words(int n) {
   if (g_amax_left < n) {
     const int kWords = 16384;
     uint32_t* chunk = nullptr;
-    // cleared on a stream of its own: the words are needed on any stream, and a recording forbids waiting for the device
-    static cudaStream_t clearing = nullptr;
-    if ((!clearing && cudaStreamCreateWithFlags(&clearing, cudaStreamNonBlocking) != cudaSuccess) || cudaMalloc((void**)&chunk, kWords * sizeof(uint32_t)) != cudaSuccess ||
-        cudaMemsetAsync(chunk, 0, kWords * sizeof(uint32_t), clearing) != cudaSuccess || cudaStreamSynchronize(clearing) != cudaSuccess) {
+    // cleared on a stream of its own: the words are needed on any stream, and waiting for the device would wait for other threads' work
+    cudaStream_t clearing = nullptr;
+    const bool ok = cudaStreamCreateWithFlags(&clearing, cudaStreamNonBlocking) == cudaSuccess && cudaMalloc((void**)&chunk, kWords * sizeof(uint32_t)) == cudaSuccess &&
+                    cudaMemsetAsync(chunk, 0, kWords * sizeof(uint32_t), clearing) == cudaSuccess && cudaStreamSynchronize(clearing) == cudaSuccess;
+    if (clearing) cudaStreamDestroy(clearing);
+    if (!ok) {
       cudaGetLastError();
       return nullptr;
     }
@@ -1851,18 +1853,7 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
                        p.N, p.k_total, p.tap_tiles, BN, tiles, p.tail_tiles, p.tail_share, p.cluster, p.a_slots, p.a_rows, p.b_slots, p.b_resident ? "r" : "", what + 5);
   KernelTimer kt(detail ? name : (AR == kArithTF32 ? "gemm3xtf32_tcgen05" : "gemm3xf16_tcgen05"), s, flops, 0, 1);
   if (p.cluster > 1) {
-    static const bool no_dep = getenv("TINYFLOW_NO_DEPENDENT_LAUNCH") != nullptr;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(kGemmThreads); cfg.dynamicSmemBytes = (size_t)gemm_smem_bytes(p, BN); cfg.stream = s;
-    cudaLaunchAttribute attrs[2];
-    memset(attrs, 0, sizeof(attrs));
-    attrs[0].id = cudaLaunchAttributeClusterDimension;
-    attrs[0].val.clusterDim.x = p.cluster; attrs[0].val.clusterDim.y = 1; attrs[0].val.clusterDim.z = 1;
-    attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attrs[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attrs; cfg.numAttrs = (no_dep || s == (cudaStream_t)0) ? 1 : 2;
-    TF_CUDA(cudaLaunchKernelEx(&cfg, gemm3x_kernel<BN, AR>, p));
+    TF_CUDA(launch_cluster(gemm3x_kernel<BN, AR>, p.cluster, dim3(grid), dim3(kGemmThreads), (size_t)gemm_smem_bytes(p, BN), s, p));
   } else {
     TF_CUDA(launch_dep(gemm3x_kernel<BN, AR>, dim3(grid), dim3(kGemmThreads), (size_t)gemm_smem_bytes(p, BN), s, p));
   }
@@ -1891,21 +1882,10 @@ template <int AR> static int launch_gemm_pair(const GemmParams& p, cudaStream_t 
   const int pairs = std::min(device_sm_count() / 2, pair_tiles);
   note_compute_stream(s);
   static const bool detail = getenv("TINYFLOW_TIMING_DETAIL") != nullptr;
-  static const bool no_dep = getenv("TINYFLOW_NO_DEPENDENT_LAUNCH") != nullptr;
   char name[192];
   if (detail) snprintf(name, sizeof(name), "gemm3x%s pairs mode%d M%d N%d ktotal%d pairtiles%d %s", AR == kArithTF32 ? "tf32" : "f16", p.mode, p.M, p.N, p.k_total, pair_tiles, what + 5);
   KernelTimer kt(detail ? name : (AR == kArithTF32 ? "gemm3xtf32_tcgen05" : "gemm3xf16_tcgen05"), s, flops, 0, 1);
-  cudaLaunchConfig_t cfg;
-  memset(&cfg, 0, sizeof(cfg));
-  cfg.gridDim = dim3(2 * pairs); cfg.blockDim = dim3(kThreads); cfg.dynamicSmemBytes = (size_t)L::kTotal; cfg.stream = s;
-  cudaLaunchAttribute attrs[2];
-  memset(attrs, 0, sizeof(attrs));
-  attrs[0].id = cudaLaunchAttributeClusterDimension;
-  attrs[0].val.clusterDim.x = 2; attrs[0].val.clusterDim.y = 1; attrs[0].val.clusterDim.z = 1;
-  attrs[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attrs[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attrs; cfg.numAttrs = (no_dep || s == (cudaStream_t)0) ? 1 : 2;
-  TF_CUDA(cudaLaunchKernelEx(&cfg, gemm3x_pair_kernel<AR>, p));
+  TF_CUDA(launch_cluster(gemm3x_pair_kernel<AR>, 2, dim3(2 * pairs), dim3(kThreads), (size_t)L::kTotal, s, p));
   TF_AFTER(s, what);
   return 0;
 }
@@ -2517,7 +2497,7 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
   if (st->cls == 1) {
     // a strided 1x1 window reaches only every stride-th input position: the rest of dx is zero
     bool strided = p->stride_h > 1 || p->stride_w > 1;
-    if (strided && cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)p->N * p->C * p->H * p->W, s) != cudaSuccess) return -1;
+    if (strided && clear_on_stream(dx, sizeof(float) * (size_t)p->N * p->C * p->H * p->W, s) != cudaSuccess) return -1;
     TapList taps; taps.add(0, 0, 0);
     OutGeom og{p->P, p->Q, p->H, p->W, p->stride_h, p->stride_w, 0, 0};
     rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom, st->track_dx ? &track : nullptr);
@@ -2533,7 +2513,7 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
     // One launch per stride phase (a, b): dx_padded(sh*u + a, sw*v + b) = sum over the taps r = sh*r' + a, s = sw*s' + b of
     // dy(u - r', v - s') * w(r, s); dy sits at frame offset (hh, hw), so the shift is (hh - r') rows and (hw - s') columns.
     // The phases write disjoint positions of dx; positions no phase reaches stay zero.
-    if (cudaMemsetAsync(dx, 0, sizeof(float) * (size_t)p->N * p->C * p->H * p->W, s) != cudaSuccess) return -1;
+    if (clear_on_stream(dx, sizeof(float) * (size_t)p->N * p->C * p->H * p->W, s) != cudaSuccess) return -1;
     for (int a = 0; a < p->stride_h && !rc; ++a)
       for (int b = 0; b < p->stride_w && !rc; ++b) {
         TapList taps;

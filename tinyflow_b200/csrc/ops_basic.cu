@@ -126,7 +126,7 @@ template <class F> static int run_map1(const float* a, float* o, int64_t n, cuda
   note_compute_stream(s);
   KernelTimer kt(what, s, 0, 8.0 * n);
   if (aligned16(a) && aligned16(o)) launch_dep(map1_kernel<F>, dim3(grid_for(n, kBlock, 4)), dim3(kBlock), 0, s, a, o, n, f, track_of<F>(o));
-  else map1_scalar_kernel<<<grid_for(n, kBlock, 1), kBlock, 0, s>>>(a, o, n, f);
+  else launch_plain(map1_scalar_kernel<F>, dim3(grid_for(n, kBlock, 1)), dim3(kBlock), 0, s, a, o, n, f);
   TF_AFTER(s, what);
   return 0;
 }
@@ -135,7 +135,7 @@ template <class F> static int run_map2(const float* a, const float* b, float* o,
   note_compute_stream(s);
   KernelTimer kt(what, s, 0, 12.0 * n);
   if (aligned16(a) && aligned16(b) && aligned16(o)) launch_dep(map2_kernel<F>, dim3(grid_for(n, kBlock, 4)), dim3(kBlock), 0, s, a, b, o, n, f, track_of<F>(o));
-  else map2_scalar_kernel<<<grid_for(n, kBlock, 1), kBlock, 0, s>>>(a, b, o, n, f);
+  else launch_plain(map2_scalar_kernel<F>, dim3(grid_for(n, kBlock, 1)), dim3(kBlock), 0, s, a, b, o, n, f);
   TF_AFTER(s, what);
   return 0;
 }
@@ -144,7 +144,7 @@ template <class F> static int run_map3(const float* a, const float* b, const flo
   note_compute_stream(s);
   KernelTimer kt(what, s, 0, 16.0 * n);
   if (aligned16(a) && aligned16(b) && aligned16(c) && aligned16(o)) launch_dep(map3_kernel<F>, dim3(grid_for(n, kBlock, 4)), dim3(kBlock), 0, s, a, b, c, o, n, f, track_of<F>(o));
-  else map3_scalar_kernel<<<grid_for(n, kBlock, 1), kBlock, 0, s>>>(a, b, c, o, n, f);
+  else launch_plain(map3_scalar_kernel<F>, dim3(grid_for(n, kBlock, 1)), dim3(kBlock), 0, s, a, b, c, o, n, f);
   TF_AFTER(s, what);
   return 0;
 }
@@ -769,7 +769,7 @@ int DLGpuBroadcastTo0(const DLArrayHandle input, DLArrayHandle output, void** cu
     return 0;
   }
   note_compute_stream(s);
-  bcast_tail_kernel<<<grid_for(total, kBlock), kBlock, 0, s>>>(F(input), FM(output), inner, total);
+  launch_plain(bcast_tail_kernel, dim3(grid_for(total, kBlock)), dim3(kBlock), 0, s, F(input), FM(output), inner, total);
   TF_AFTER(s, "DLGpuBroadcastTo0");
   return 0;
 }
@@ -786,7 +786,7 @@ int DLGpuBroadcastTo1(const DLArrayHandle input, DLArrayHandle output, void** cu
     return 0;
   }
   note_compute_stream(s);
-  bcast_channel_kernel<<<grid_for(total, kBlock), kBlock, 0, s>>>(F(input), FM(output), output->shape[1], low, total);
+  launch_plain(bcast_channel_kernel, dim3(grid_for(total, kBlock)), dim3(kBlock), 0, s, F(input), FM(output), output->shape[1], low, total);
   TF_AFTER(s, "DLGpuBroadcastTo1");
   return 0;
 }
@@ -902,7 +902,7 @@ int DLGpuReduceSum(const DLArrayHandle input, DLArrayHandle output, void*** cudn
     if (g.reduced[d]) g.nred *= p->in_dims[d];
   }
   note_compute_stream(s);
-  reduce_general_kernel<<<(unsigned)nout, kBlock, 0, s>>>(F(input), FM(output), g);
+  launch_plain(reduce_general_kernel, dim3((unsigned)nout), dim3(kBlock), 0, s, F(input), FM(output), g);
   TF_AFTER(s, "DLGpuReduceSum");
   return 0;
 }
@@ -939,7 +939,7 @@ int DLGpuReduceSumAxisN(const DLArrayHandle input, DLArrayHandle output, const i
   TF_REQUIRE(numel(output) == outer * inner, "DLGpuReduceSumAxisN: output size mismatch");
   cudaStream_t s = legacy_stream();
   note_compute_stream(s);
-  axis_sum_kernel<<<grid_for(outer * inner, kBlock), kBlock, 0, s>>>(F(input), FM(output), outer, red, inner);
+  launch_plain(axis_sum_kernel, dim3(grid_for(outer * inner, kBlock)), dim3(kBlock), 0, s, F(input), FM(output), outer, red, inner);
   TF_AFTER(s, "DLGpuReduceSumAxisN");
   return 0;
 }
@@ -951,7 +951,7 @@ int DLGpuReduceSumAxisNBackward(const DLArrayHandle input, DLArrayHandle output,
   TF_REQUIRE(numel(input) == outer * inner, "DLGpuReduceSumAxisNBackward: input size mismatch");
   cudaStream_t s = legacy_stream();
   note_compute_stream(s);
-  axis_bcast_kernel<<<grid_for(numel(output), kBlock), kBlock, 0, s>>>(F(input), FM(output), outer, red, inner);
+  launch_plain(axis_bcast_kernel, dim3(grid_for(numel(output), kBlock)), dim3(kBlock), 0, s, F(input), FM(output), outer, red, inner);
   TF_AFTER(s, "DLGpuReduceSumAxisNBackward");
   return 0;
 }
@@ -1013,8 +1013,8 @@ int DLGpuReduceSumAllStatic(const DLArrayHandle input, DLArrayHandle output, voi
   int blocks = (int)((n + kStaticElemsPerBlock - 1) / kStaticElemsPerBlock);
   if (blocks < 1) blocks = 1;
   note_compute_stream(s);
-  partial_sum_kernel<<<blocks, kBlock, 0, s>>>(F(input), part, n);
-  final_sum_kernel<<<1, kBlock, 0, s>>>(part, FM(output), blocks, 1.f);
+  launch_plain(partial_sum_kernel, dim3(blocks), dim3(kBlock), 0, s, F(input), part, n);
+  launch_plain(final_sum_kernel, dim3(1), dim3(kBlock), 0, s, part, FM(output), blocks, 1.f);
   if (after_launch(s, "DLGpuReduceSumAllStatic", 2) != 0) return -1;
   return 0;
 }
@@ -1024,7 +1024,7 @@ int DLGpuReduceSumAllBackward(const DLArrayHandle input, DLArrayHandle output) {
   int64_t total = numel(output);
   cudaStream_t s = legacy_stream();
   note_compute_stream(s);
-  bcast_tail_kernel<<<grid_for(total, kBlock), kBlock, 0, s>>>(F(input), FM(output), 1, total);
+  launch_plain(bcast_tail_kernel, dim3(grid_for(total, kBlock)), dim3(kBlock), 0, s, F(input), FM(output), 1, total);
   TF_AFTER(s, "DLGpuReduceSumAllBackward");
   return 0;
 }
@@ -1111,7 +1111,7 @@ int DLGpuSoftmax(const DLArrayHandle input, DLArrayHandle output, void** cudaStr
   int64_t rows = input->shape[0], cols = input->shape[1];
   cudaStream_t s = stream_of(cudaStream);
   note_compute_stream(s);
-  row_softmax_kernel<<<grid_for(rows * 32, kBlock), kBlock, 0, s>>>(F(input), FM(output), rows, cols);
+  launch_plain(row_softmax_kernel, dim3(grid_for(rows * 32, kBlock)), dim3(kBlock), 0, s, F(input), FM(output), rows, cols);
   TF_AFTER(s, "DLGpuSoftmax");
   return 0;
 }
@@ -1137,8 +1137,8 @@ static int row_loss(int mode, const DLArrayHandle a, const DLArrayHandle b, DLAr
   if (b) TF_REQUIRE(numel(a) == numel(b), "%s: element counts differ", what);
   int64_t rows = a->shape[0], cols = rows ? numel(a) / rows : 0;
   cudaStream_t s = last_compute_stream();
-  if (mode == 1) row_loss_kernel<1><<<1, 1024, 0, s>>>(F(a), b ? F(b) : nullptr, FM(out), rows, cols, scale);
-  else row_loss_kernel<2><<<1, 1024, 0, s>>>(F(a), b ? F(b) : nullptr, FM(out), rows, cols, scale);
+  if (mode == 1) launch_plain(row_loss_kernel<1>, dim3(1), dim3(1024), 0, s, F(a), b ? F(b) : nullptr, FM(out), rows, cols, scale);
+  else launch_plain(row_loss_kernel<2>, dim3(1), dim3(1024), 0, s, F(a), b ? F(b) : nullptr, FM(out), rows, cols, scale);
   TF_AFTER(s, what);
   return 0;
 }
@@ -1147,8 +1147,8 @@ static int loss_grad(int mode, const DLArrayHandle a, const DLArrayHandle b, con
   int64_t n = numel(a);
   float inv = 1.f / (float)a->shape[0];
   cudaStream_t s = last_compute_stream();
-  if (mode == 1) loss_grad_kernel<1><<<grid_for(n, kBlock), kBlock, 0, s>>>(F(a), b ? F(b) : nullptr, F(g), FM(out), n, inv);
-  else loss_grad_kernel<2><<<grid_for(n, kBlock), kBlock, 0, s>>>(F(a), b ? F(b) : nullptr, F(g), FM(out), n, inv);
+  if (mode == 1) launch_plain(loss_grad_kernel<1>, dim3(grid_for(n, kBlock)), dim3(kBlock), 0, s, F(a), b ? F(b) : nullptr, F(g), FM(out), n, inv);
+  else launch_plain(loss_grad_kernel<2>, dim3(grid_for(n, kBlock)), dim3(kBlock), 0, s, F(a), b ? F(b) : nullptr, F(g), FM(out), n, inv);
   TF_AFTER(s, what);
   return 0;
 }
@@ -1274,7 +1274,7 @@ int DLGpuActivationForward(const DLArrayHandle input, DLArrayHandle output, int 
       int64_t rows = p ? p->batch : input->shape[0];
       TF_REQUIRE(rows > 0 && n % rows == 0, "DLGpuActivationForward(softmax): bad batch extent");
       note_compute_stream(s);
-      row_softmax_kernel<<<grid_for(rows * 32, kBlock), kBlock, 0, s>>>(F(input), FM(output), rows, n / rows);
+      launch_plain(row_softmax_kernel, dim3(grid_for(rows * 32, kBlock)), dim3(kBlock), 0, s, F(input), FM(output), rows, n / rows);
       TF_AFTER(s, "DLGpuActivationForward(softmax)");
       return 0;
     }
@@ -1302,7 +1302,7 @@ int DLGpuActivationBackward(const DLArrayHandle input, DLArrayHandle dinput, con
       int64_t rows = p ? p->batch : input->shape[0];
       TF_REQUIRE(rows > 0 && n % rows == 0, "DLGpuActivationBackward(softmax): bad batch extent");
       note_compute_stream(s);
-      row_softmax_bwd_kernel<<<grid_for(rows * 32, kBlock), kBlock, 0, s>>>(F(output), F(doutput), FM(dinput), rows, n / rows);
+      launch_plain(row_softmax_bwd_kernel, dim3(grid_for(rows * 32, kBlock)), dim3(kBlock), 0, s, F(output), F(doutput), FM(dinput), rows, n / rows);
       TF_AFTER(s, "DLGpuActivationBackward(softmax)");
       return 0;
     }
@@ -1369,7 +1369,7 @@ int DLGpuAdam_mv(DLArrayHandle m, DLArrayHandle v, const DLArrayHandle g, float 
   int took = dp_adam_moments(FM(m), FM(v), F(g), n, b1, b2, s);
   if (took < 0) return -1;
   if (took) return 0;
-  adam_moments_kernel<<<grid_for(n, kBlock), kBlock, 0, s>>>(FM(m), FM(v), F(g), n, b1, b2);
+  launch_plain(adam_moments_kernel, dim3(grid_for(n, kBlock)), dim3(kBlock), 0, s, FM(m), FM(v), F(g), n, b1, b2);
   TF_AFTER(s, "DLGpuAdam_mv");
   return 0;
 }
@@ -1442,7 +1442,7 @@ int DLGpuSgd_o(void**** n2list, const void*** indexlist, const int count, const 
   TF_REQUIRE(t && info && t->groups == 2 && t->n == info->count && (count == t->n || count == (int)info->total), "DLGpuSgd_o: tables do not match");
   cudaStream_t s = last_compute_stream();
   for (int i = 0; i < t->n; ++i) note_write(t->host[i]);                      // column 0: the parameters
-  sgd_table_kernel<<<grid_for(info->total, kBlock), kBlock, 0, s>>>((float* const*)t->dev, (float* const*)(t->dev + t->n), info->dev_prefix, t->n, info->total, learning_rate);
+  launch_plain(sgd_table_kernel, dim3(grid_for(info->total, kBlock)), dim3(kBlock), 0, s, (float* const*)t->dev, (float* const*)(t->dev + t->n), info->dev_prefix, t->n, info->total, learning_rate);
   TF_AFTER(s, "DLGpuSgd_o");
   return 0;
 }
@@ -1453,7 +1453,7 @@ int DLGpuAdam_o(void**** n4list, const void*** indexlist, const int count, const
   TF_REQUIRE(t && info && t->groups == 4 && t->n == info->count && (count == t->n || count == (int)info->total), "DLGpuAdam_o: tables do not match");
   cudaStream_t s = last_compute_stream();
   for (int i = 0; i < 3 * t->n; ++i) note_write(t->host[i]);                  // columns 0-2: parameters and both moments
-  adam_table_kernel<<<grid_for(info->total, kBlock), kBlock, 0, s>>>((float* const*)t->dev, (float* const*)(t->dev + t->n), (float* const*)(t->dev + 2 * t->n), (float* const*)(t->dev + 3 * t->n),
+  launch_plain(adam_table_kernel, dim3(grid_for(info->total, kBlock)), dim3(kBlock), 0, s, (float* const*)t->dev, (float* const*)(t->dev + t->n), (float* const*)(t->dev + 2 * t->n), (float* const*)(t->dev + 3 * t->n),
                                                                      info->dev_prefix, t->n, info->total, b1, b2, 1.f - b1t, 1.f - b2t, e, learning_rate);
   TF_AFTER(s, "DLGpuAdam_o");
   return 0;

@@ -232,7 +232,7 @@ int DLGpuPooling3DForward(const DLArrayHandle input, DLArrayHandle output, void*
   cudaStream_t s = last_compute_stream();
   const int64_t total = numel(output);
   note_compute_stream(s);
-  pool3_fwd_kernel<<<grid_for(total, 256), 256, 0, s>>>((const float*)input->data, out_f32(output), total, geom3(p), p->mode);
+  launch_plain(pool3_fwd_kernel, dim3(grid_for(total, 256)), dim3(256), 0, s, (const float*)input->data, out_f32(output), total, geom3(p), p->mode);
   TF_AFTER(s, "DLGpuPooling3DForward");
   return 0;
 }
@@ -245,7 +245,7 @@ int DLGpuPooling3DBackward(const DLArrayHandle input, const DLArrayHandle output
   cudaStream_t s = last_compute_stream();
   const int64_t total = numel(dinput);
   note_compute_stream(s);
-  pool3_bwd_kernel<<<grid_for(total, 256), 256, 0, s>>>((const float*)input->data, (const float*)doutput->data, out_f32(dinput), total, geom3(p), p->mode);
+  launch_plain(pool3_bwd_kernel, dim3(grid_for(total, 256)), dim3(256), 0, s, (const float*)input->data, (const float*)doutput->data, out_f32(dinput), total, geom3(p), p->mode);
   TF_AFTER(s, "DLGpuPooling3DBackward");
   return 0;
 }

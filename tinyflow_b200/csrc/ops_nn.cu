@@ -781,7 +781,7 @@ int DLGpuPooling2DBackward(const DLArrayHandle input, const DLArrayHandle output
     if (p->argmax && p->argmax_src == input->data && p->argmax_version == version_of(input->data) && p->argmax_recording == recording_id())
       launch_pool_gather<true>(p, p->argmax, (const float*)doutput->data, out_f32(dinput), total, 1.f, s);
     else
-      maxpool_bwd_kernel<<<grid_for(total, 256), 256, 0, s>>>((const float*)input->data, (const float*)doutput->data, out_f32(dinput), total, geom_of(p));
+      launch_plain(maxpool_bwd_kernel, dim3(grid_for(total, 256)), dim3(256), 0, s, (const float*)input->data, (const float*)doutput->data, out_f32(dinput), total, geom_of(p));
   }
   else if (mean3_fits(p, (const float*)doutput->data)) launch_mean3(p, (const float*)doutput->data, out_f32(dinput), s, AmaxOut{});
   else launch_pool_gather<false>(p, nullptr, (const float*)doutput->data, out_f32(dinput), total, 1.f / (float)(p->win_h * p->win_w), s);
@@ -851,9 +851,9 @@ int DLGpuBatchNormalizationForward(const DLArrayHandle input, DLArrayHandle outp
     int N = (int)p->N;
     p->last_y = y; p->last_y_version = version_of(y);
     if (N <= kBnMaxBatchInRegs) launch_bn_fwd_regs(x, y, p->save_mean, p->save_inv, N, F, s);
-    else bn_pa_fwd_loop_kernel<<<(unsigned)((F + 127) / 128), 128, 0, s>>>(x, y, p->save_mean, p->save_inv, N, F);
+    else launch_plain(bn_pa_fwd_loop_kernel, dim3((unsigned)((F + 127) / 128)), dim3(128), 0, s, x, y, p->save_mean, p->save_inv, N, F);
   } else {
-    bn_sp_fwd_kernel<<<(unsigned)p->C, 512, 0, s>>>(x, y, p->save_mean, p->save_inv, p->N, p->C, p->HW);
+    launch_plain(bn_sp_fwd_kernel, dim3((unsigned)p->C), dim3(512), 0, s, x, y, p->save_mean, p->save_inv, p->N, p->C, p->HW);
   }
   TF_AFTER(s, "DLGpuBatchNormalizationForward");
   return 0;
@@ -900,9 +900,9 @@ int DLGpuBatchNormalizationBackward(const DLArrayHandle input, const DLArrayHand
     int N = (int)p->N;
     unsigned grid = (unsigned)((F + 127) / 128);
     if (N <= kBnMaxBatchInRegs) launch_bn_bwd_regs(x, dy, dx, p->save_mean, p->save_inv, N, F, s);
-    else bn_pa_bwd_loop_kernel<<<grid, 128, 0, s>>>(x, dy, dx, p->save_mean, p->save_inv, N, F);
+    else launch_plain(bn_pa_bwd_loop_kernel, dim3(grid), dim3(128), 0, s, x, dy, dx, p->save_mean, p->save_inv, N, F);
   } else {
-    bn_sp_bwd_kernel<<<(unsigned)p->C, 512, 0, s>>>(x, dy, dx, p->save_mean, p->save_inv, p->N, p->C, p->HW);
+    launch_plain(bn_sp_bwd_kernel, dim3((unsigned)p->C), dim3(512), 0, s, x, dy, dx, p->save_mean, p->save_inv, p->N, p->C, p->HW);
   }
   TF_AFTER(s, "DLGpuBatchNormalizationBackward");
   return 0;

@@ -6,7 +6,6 @@
 #include <algorithm>
 #include <map>
 #include <mutex>
-#include <shared_mutex>
 #include <thread>
 #include <unordered_map>
 #include <vector>
@@ -99,24 +98,8 @@ void KernelTimer::end() {
   if (slot >= 0 && slot < (int)g_pending.size()) cudaEventRecord(g_pending[slot].b, stream);
 }
 
-// A wait for the whole device is an error while any stream of it is captured, and ends the capture: such waits take turns with
-// the recordings of other threads (which issue calls and wait for nothing).  No lock of the library may be held around one.
-static std::shared_mutex g_capture_mu;
-void capture_begins() { g_capture_mu.lock_shared(); }
-void capture_ends() { g_capture_mu.unlock_shared(); }
-CaptureExclusion::CaptureExclusion() { g_capture_mu.lock(); }
-CaptureExclusion::~CaptureExclusion() { g_capture_mu.unlock(); }
-cudaError_t device_wait() {
-  if (t_recording) return cudaErrorStreamCaptureUnsupported;
-  CaptureExclusion turn;
-  return cudaDeviceSynchronize();
-}
-
 static std::atomic<cudaStream_t> g_compute_stream{(cudaStream_t)0};
-void note_compute_stream(cudaStream_t s) {
-  if (!t_recording) g_compute_stream.store(s, std::memory_order_relaxed);                 // a recording's stream concerns nobody else
-  else if (s != recording_stream()) recording_refuse("an operator was called on another stream than the recording's");      // it has run, and no replay would run it
-}
+void note_compute_stream(cudaStream_t s) { if (!t_recording) g_compute_stream.store(s, std::memory_order_relaxed); }     // a recording's stream concerns nobody else
 cudaStream_t legacy_stream() { flush_deferred(); return t_recording ? recording_stream() : (cudaStream_t)0; }
 cudaStream_t last_compute_stream() { flush_deferred(); return t_recording ? recording_stream() : g_compute_stream.load(std::memory_order_relaxed); }
 
@@ -262,9 +245,8 @@ struct Pool {
     }
     if (e != cudaSuccess) {
       cudaGetLastError();
-      if (t_recording && !host) return nullptr;            // what follows waits for the device: the step is not recorded
       // Give cached blocks back to the driver and try once more before reporting OOM.
-      if (!host) { lk.unlock(); device_wait(); lk.lock(); }
+      if (!host) { lk.unlock(); cudaDeviceSynchronize(); lk.lock(); }
       release_cached_locked();
       e = raw_alloc(&p, b);
       if (e != cudaSuccess && !host) {
@@ -497,8 +479,11 @@ int DLArrayCopyFromTo(DLArrayHandle from, DLArrayHandle to, DLStreamHandle strea
     TF_CUDA(cudaEventRecord(ev, cs));
     TF_CUDA(cudaStreamWaitEvent(s, ev, 0));
   }
+  if (kind == cudaMemcpyDeviceToDevice && s == cs) {           // same-stream reshape copy: no host wait needed
+    TF_CUDA(copy_on_stream(to->data, from->data, bytes, s));
+    return 0;
+  }
   TF_CUDA(cudaMemcpyAsync(to->data, from->data, bytes, kind, s));
-  if (kind == cudaMemcpyDeviceToDevice && s == cs) return 0;   // same-stream reshape copy: no host wait needed
   TF_CUDA(cudaStreamSynchronize(s));
   return 0;
 }
@@ -509,7 +494,7 @@ int TfArrayCopyOnStream(DLArrayHandle from, DLArrayHandle to, void** cudaStream)
   cudaStream_t s = stream_of(cudaStream);
   note_compute_stream(s);
   note_write(to->data);
-  if (numel(from) > 0) TF_CUDA(cudaMemcpyAsync(to->data, from->data, data_bytes(from), cudaMemcpyDeviceToDevice, s));
+  if (numel(from) > 0) TF_CUDA(copy_on_stream(to->data, from->data, data_bytes(from), s));
   return 0;
 }
 
@@ -570,7 +555,7 @@ int testPcie(void) {
     cudaMemcpy(dst, src, bytes, k);   // warm-up
     auto t0 = std::chrono::steady_clock::now();
     for (int i = 0; i < 4; ++i) cudaMemcpy(dst, src, bytes, k);
-    device_wait();
+    cudaDeviceSynchronize();
     double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
     return 4.0 * bytes / s / 1e9;
   };
@@ -609,8 +594,7 @@ int TfKernelTimingReport(char* buf, int buflen) {
 
 int TfDeviceSynchronize(void) {
   flush_deferred();
-  if (t_recording) recording_refuse("a wait for the device");
-  TF_CUDA(device_wait());
+  TF_CUDA(cudaDeviceSynchronize());
   TF_REQUIRE(tensor_path_error() == 0, "a tensor-core kernel timed out waiting on a barrier (results of that launch are invalid)");
   return 0;
 }
@@ -632,8 +616,7 @@ int TfSetMemoryLimit(long long bytes) {
   return 0;
 }
 int TfReleaseCachedMemory(void) {
-  if (t_recording) return 0;               // its steps may use any of the blocks
-  device_wait();
+  cudaDeviceSynchronize();
   { Pool& p = device_pool(); std::lock_guard<std::mutex> lk(p.mu); p.release_cached_locked(); }
   { Pool& p = host_pool(); std::lock_guard<std::mutex> lk(p.mu); p.release_cached_locked(); }
   return 0;

@@ -1,10 +1,11 @@
 // Recording and replaying a training step.  The executor's node loop costs the host 5-9 us per operator call (Python,
 // ctypes, launch), which is what bounds every graph whose kernels are shorter than that: a 52-launch MLP step took 0.54 ms
-// of which the GPU worked 0.1, Inception-v3 at batch 2 (1289 launches) 8.8 ms.  Here one step's launches are captured once
+// of which the GPU worked 0.1, Inception-v3 at batch 2 (1289 launches) 8.8 ms.  Here one step's launches are collected once
 // into a CUDA graph (with the programmatic launch edges of launch_dep) and replayed with one call.
 //
-// The recording runs on a private non-blocking stream in relaxed mode: other threads' copies and the legacy default stream
-// are not drawn into it, and nothing of the step executes while it is recorded.  What has to differ from an ordinary call is
+// The graph is built node by node in the launch functions, a chain in the order of the calls; nothing of the step executes
+// meanwhile.  It is not captured from a stream: while any stream is captured, a wait for the whole device is an error in every
+// thread, in code that knows nothing of this library too, and ends the capture.  What has to differ from an ordinary call is
 // listed at the declarations in common.h.  A replay leaves the library's books as the step itself would: every tensor the
 // step writes gets a new write version, the packs it overwrites in the plans no longer count as what an ordinary call left
 // there, the launches are counted, and the maxima of the parameters stay known.
@@ -28,7 +29,10 @@ constexpr int kSeedWords = 1022;          // dropout calls of a step
 constexpr int kCarries = 1024;            // parameters whose maximum crosses steps
 
 struct StepGraph {
-  cudaStream_t stream = nullptr;
+  cudaStream_t stream = nullptr;          // the calls of the recording name it; nothing runs on it
+  cudaGraph_t graph = nullptr;
+  cudaGraphNode_t last = nullptr;         // the node every next one waits for
+  bool last_is_kernel = false;
   cudaGraphExec_t exec = nullptr;
   uint32_t* words = nullptr;              // [zeroed words][c1, c2][seeds]
   int used = 0;
@@ -100,6 +104,57 @@ void recording_note_write(const void* p) { t_recording->written.push_back(p); }
 void recording_note_made(const void** source) { t_recording->made.push_back(source); }
 cudaStream_t recording_stream() { return t_recording->stream; }
 
+// ---- nodes --------------------------------------------------------------------------------------
+static cudaError_t recorded(cudaError_t e, cudaGraphNode_t node, bool kernel, bool dependent) {
+  StepGraph* g = t_recording;
+  if (e == cudaSuccess && g->last) {
+    cudaGraphEdgeData edge;
+    memset(&edge, 0, sizeof(edge));
+    if (dependent && g->last_is_kernel) { edge.type = cudaGraphDependencyTypeProgrammatic; edge.from_port = cudaGraphKernelNodePortProgrammatic; }
+    e = cudaGraphAddDependencies_v2(g->graph, &g->last, &node, &edge, 1);
+  }
+  if (e != cudaSuccess) { recording_refuse(cudaGetErrorString(e)); return e; }
+  g->last = node; g->last_is_kernel = kernel;
+  return cudaSuccess;
+}
+static bool recorded_stream(cudaStream_t s) {
+  if (s == t_recording->stream) return true;
+  recording_refuse("an operator was called on another stream than the recording's");
+  return false;
+}
+cudaError_t recording_add_kernel(const void* kernel, const LaunchShape& l, void** args, cudaStream_t s) {
+  if (!recorded_stream(s)) return cudaErrorInvalidResourceHandle;
+  cudaKernelNodeParams p;
+  memset(&p, 0, sizeof(p));
+  p.func = (void*)kernel; p.gridDim = l.grid; p.blockDim = l.block; p.sharedMemBytes = (unsigned)l.smem; p.kernelParams = args;
+  cudaGraphNode_t node = nullptr;
+  cudaError_t e = cudaGraphAddKernelNode(&node, t_recording->graph, nullptr, 0, &p);
+  if (e == cudaSuccess && l.cluster > 0) {
+    cudaLaunchAttributeValue v;
+    memset(&v, 0, sizeof(v));
+    v.clusterDim.x = l.cluster; v.clusterDim.y = 1; v.clusterDim.z = 1;
+    e = cudaGraphKernelNodeSetAttribute(node, cudaLaunchAttributeClusterDimension, &v);
+  }
+  return recorded(e, node, true, l.dependent);
+}
+cudaError_t clear_on_stream(void* ptr, size_t bytes, cudaStream_t s) {
+  if (!t_recording) return cudaMemsetAsync(ptr, 0, bytes, s);
+  if (!recorded_stream(s)) return cudaErrorInvalidResourceHandle;
+  cudaMemsetParams p;
+  memset(&p, 0, sizeof(p));
+  p.dst = ptr; p.elementSize = bytes % 4 == 0 ? 4 : 1; p.width = bytes / p.elementSize; p.height = 1;
+  cudaGraphNode_t node = nullptr;
+  const cudaError_t e = cudaGraphAddMemsetNode(&node, t_recording->graph, nullptr, 0, &p);
+  return recorded(e, node, false, false);
+}
+cudaError_t copy_on_stream(void* to, const void* from, size_t bytes, cudaStream_t s) {
+  if (!t_recording) return cudaMemcpyAsync(to, from, bytes, cudaMemcpyDeviceToDevice, s);
+  if (!recorded_stream(s)) return cudaErrorInvalidResourceHandle;
+  cudaGraphNode_t node = nullptr;
+  const cudaError_t e = cudaGraphAddMemcpyNode1D(&node, t_recording->graph, nullptr, 0, to, from, bytes, cudaMemcpyDeviceToDevice);
+  return recorded(e, node, false, false);
+}
+
 // Values of this replay (bias corrections, seeds) into the words the recorded kernels read; up to 960 per launch by value.
 constexpr int kValuesPerLaunch = 960;
 struct StepValues { uint32_t v[kValuesPerLaunch]; };
@@ -118,10 +173,11 @@ static std::mutex g_graphs_mu;
 static std::vector<StepGraph*> g_graphs;
 static void step_graph_release(StepGraph* g) {
   if (g->exec) cudaGraphExecDestroy(g->exec);
+  if (g->graph) cudaGraphDestroy(g->graph);
   if (g->stream) cudaStreamDestroy(g->stream);
   if (g->words) pool_free(g->words);
   for (auto& kv : g->free_blocks) for (void* p : kv.second) pool_free(p);
-  g->exec = nullptr; g->stream = nullptr; g->words = nullptr;
+  g->exec = nullptr; g->graph = nullptr; g->stream = nullptr; g->words = nullptr;
   g->free_blocks.clear();
   cudaGetLastError();
 }
@@ -134,8 +190,7 @@ static void step_graph_free(StepGraph* g) {
   delete g;
 }
 bool recordings_give_up_memory() {
-  if (t_recording) return false;         // the blocks would go to the recording, and a capture forbids waiting for the device
-  CaptureExclusion turn;                 // in front of the lock, which a thread that records takes when it drops an older recording
+  if (t_recording) return false;         // the blocks would go to that recording
   std::lock_guard<std::mutex> lk(g_graphs_mu);
   if (g_graphs.empty()) return false;
   if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return false; }      // no replay is in flight
@@ -158,11 +213,9 @@ int TfStepRecordBegin(void** graph, void** stream_cell) {
   StepGraph* g = new StepGraph;
   g->words = (uint32_t*)pool_alloc(sizeof(uint32_t) * (kZeroedWords + 2 + kSeedWords));
   if (!g->words) { delete g; return 1; }
-  capture_begins();
-  if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess || cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
-    capture_ends();
+  if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess || cudaGraphCreate(&g->graph, 0) != cudaSuccess) {
     step_graph_free(g);
-    TF_FAIL("TfStepRecordBegin: stream capture is not available");
+    TF_FAIL("TfStepRecordBegin: no stream or graph could be created");
   }
   g->epoch = g_layout_epoch.load();
   g->id = g_recordings.fetch_add(1) + 1;
@@ -170,7 +223,7 @@ int TfStepRecordBegin(void** graph, void** stream_cell) {
   tc_recording_begins();
   *graph = g;
   *stream_cell = (void*)g->stream;
-  if (cudaMemsetAsync(g->words, 0, sizeof(uint32_t) * kZeroedWords, g->stream) != cudaSuccess) recording_refuse("the capture failed");
+  clear_on_stream(g->words, sizeof(uint32_t) * kZeroedWords, g->stream);
   return 0;
 }
 
@@ -191,21 +244,19 @@ int TfStepRecordEnd(void** graph, int keep) {
     CarryList list;
     int m = 0;
     for (const AmaxCarry& c : g->carries) if (c.from) { list.from[m] = c.from; list.to[m] = c.carry; ++m; }
-    if (ok && m) { step_carry_kernel<<<1, 256, 0, g->stream>>>(list, m); g->launches += 1; }
+    if (ok && m) { launch_plain(step_carry_kernel, dim3(1), dim3(256), 0, g->stream, list, m); g->launches += 1; }
   } else {
     int n = 0;
     AmaxCarry none;
     while (!amax_take_carries(g, &none, 1, &n)) {}
   }
-  cudaGraph_t raw = nullptr;
-  cudaError_t e = cudaStreamEndCapture(g->stream, &raw);
-  capture_ends();
-  if (e != cudaSuccess || !raw) { ok = false; recording_refuse(cudaGetErrorString(e)); }
+  ok = ok && !g->refused;
   if (ok) {
-    e = cudaGraphInstantiate(&g->exec, raw, 0);
+    const cudaError_t e = cudaGraphInstantiate(&g->exec, g->graph, 0);
     if (e != cudaSuccess) { ok = false; recording_refuse(cudaGetErrorString(e)); }
   }
-  if (raw) cudaGraphDestroy(raw);
+  cudaGraphDestroy(g->graph);
+  g->graph = nullptr;
   if (ok && g->epoch != g_layout_epoch.load()) { ok = false; recording_refuse("packed operands moved while the step was recorded"); }
   t_recording = nullptr;
   if (!ok) {
@@ -265,7 +316,7 @@ int TfStepReplay(void* graph, const unsigned* seeds, int nseeds, float b1t, floa
         const float c = k == 0 ? 1.f - b1t : 1.f - b2t;
         if (k < 2) memcpy(&vals.v[i], &c, 4); else vals.v[i] = seeds[k - 2];
       }
-      step_values_kernel<<<1, 256, 0, s>>>(vals, g->words + kZeroedWords + at, n);
+      launch_plain(step_values_kernel, dim3(1), dim3(256), 0, s, vals, g->words + kZeroedWords + at, n);
       TF_AFTER(s, "TfStepReplay");
     }
   }
