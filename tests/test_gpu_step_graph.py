@@ -178,6 +178,35 @@ def test_new_mini_batch_arrays_every_step(lib_path, monkeypatch, name):
     _same(got, want)
 
 
+def test_a_step_that_cannot_be_recorded_says_so_and_runs(lib_path, monkeypatch):
+    from tinyflow_b200 import autodiff as ad
+
+    class HostCopyOp(ad.Op):
+        name = "HostCopy"
+
+        def __call__(self, node):
+            return self._node([node])
+
+        def compute(self, node, input_vals, output_val, cudnnHandle, cublasHandle, cudaStream, use_numpy=False):
+            output_val[:] = input_vals[0].asnumpy()
+
+        def gradient(self, node, output_grad):
+            return [output_grad]
+
+        def infer_shape(self, node, input_shapes, cudnnHandle):
+            return input_shapes[0]
+
+    def build(m):
+        X, y_, W = ad.Placeholder("X"), ad.Placeholder("y_"), ad.Variable("W")
+        y = HostCopyOp()(ad.matmul_op(X, W))
+        return m.Model("host copy", X, y_, ad.l2loss_op(y, y_), y, {W: (20, 7)}, (33, 20), (33, 7))
+    want = _train(monkeypatch, False, build, "sgd", _overwrite_inputs)
+    with pytest.warns(RuntimeWarning, match="could not be recorded.*host waits") as said:
+        got = _train(monkeypatch, True, build, "sgd", _overwrite_inputs)
+    assert len(said) == 2 and "no further attempts" in str(said[1].message) and not got[2]
+    _same(got, want)
+
+
 def test_another_thread_waits_for_the_device_while_a_step_is_recorded(lib_path, monkeypatch):
     """Neither the recordings nor the waits fail, whichever library waits; the waiting thread shares no array with the step."""
     import threading

@@ -22,6 +22,7 @@ import queue
 import random
 import threading
 import time
+import warnings
 import weakref
 
 from . import gpu_op, ndarray, step_graph
@@ -191,6 +192,7 @@ class Executor(object):
         self._leases = {}          # node index -> weak references to the views of its array that were handed out
         self._recordings = step_graph.Recordings()
         self._record_failures = 0
+        self.recording_error = None          # why the last attempt to record a step failed
         self._constants = set()    # indices of the fill nodes whose array holds their constant already
         self.host_values = {}      # node index -> pinned host NDArray holding a swapped-out tensor
         self.have_plan = False
@@ -225,6 +227,7 @@ class Executor(object):
     # ---- shape inference (autodiff.py:2318-2336): builds every descriptor exactly once ----------
     def infer_shape(self, feed_shapes):
         self._forget_recordings()
+        self._record_failures = 0
         self.node_to_shape_map = dict(feed_shapes)
         for node in self.topo_order:
             if node in self.node_to_shape_map:
@@ -509,9 +512,12 @@ class Executor(object):
         self._feed = feed
         try:
             return step_graph.record(self, feed, copies)
-        except RuntimeError:
+        except RuntimeError as e:
             self._record_failures += 1
             self._feed, self._values = before
+            self.recording_error = str(e)
+            warnings.warn("this training step could not be recorded and runs as ordinary calls (%s)%s"
+                          % (e, "; no further attempts for these shapes" if self._record_failures > 1 else ""), RuntimeWarning, stacklevel=4)
             return None
         finally:
             random.setstate(draws)

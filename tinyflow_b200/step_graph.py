@@ -19,7 +19,7 @@ import os
 import weakref
 
 from . import gpu_op, ndarray
-from ._base import _LIB, check_call, new_cell
+from ._base import _LIB, check_call, last_error, new_cell
 from .graph import Convolution2DForwardOp
 
 ENABLED = os.environ.get("TINYFLOW_STEP_GRAPH", "1") != "0"
@@ -112,25 +112,26 @@ def _forget(table, key, entry_ref):
 
 
 def record(executor, feed_dict, staged):
-    """Records one step of ``executor`` on ``feed_dict`` (nothing is executed).  None if the step cannot be recorded."""
+    """Records one step of ``executor`` on ``feed_dict`` (nothing is executed).  None if that is not possible just now
+    (kernel timing, data-parallel exchange), RuntimeError with the reason if the step cannot be recorded."""
     graph, stream = ctypes.c_void_p(), new_cell(2)
     rc = _LIB.TfStepRecordBegin(ctypes.byref(graph), stream)
     if rc != 0:
         if rc < 0:
-            raise RuntimeError("recording is not available")
+            raise RuntimeError(last_error())
         return None
-    values, loss, keep = {}, None, 0
+    values, loss, keep, stopped = {}, None, 0, None
     try:
         convs = [n for n in executor.topo_order if type(n.op) is Convolution2DForwardOp and feed_dict.get(n.inputs[1]) is not None]
         gpu_op.pack_filters([feed_dict[n.inputs[1]] for n in convs], [n.cudnnlist[0] for n in convs], stream)
         values, loss = executor._issue(feed_dict, stream, recording=True)
         keep = 1
-    except Exception:                           # whatever stopped it: the ordinary step that follows reports it
-        pass
+    except Exception as e:                      # whatever stopped it: the caller runs the step as ordinary calls and says so
+        stopped = e
     finally:
         rc = _LIB.TfStepRecordEnd(ctypes.byref(graph), keep)
     if rc != 0:
-        raise RuntimeError("the step cannot be recorded")
+        raise RuntimeError("%s: %s" % (type(stopped).__name__, stopped) if stopped is not None else last_error()) from stopped
     kept = [n for n in feed_dict if n.isw == 1]
     seed_nodes = [n for n in executor.topo_order if hasattr(n, "seed")]
     return Recording(graph, values, loss, kept, seed_nodes, list(feed_dict.values()), staged, executor._changes[0])
