@@ -1597,17 +1597,19 @@ __global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restri
 // pad_d].  One launch packs any number of filters: a step's 50-150 filters, packed when their convolution came up, were as
 // many launches of 5 us for 1-2 us of traffic.  A block moves 32 x 32 filters through shared memory, so that the fp32 words are
 // read in order and both layouts are written in rows of 64 bytes; read straight from the filter, the backward-data layout took a
-// sector per element.  Bound by HBM (12 bytes an element); few blocks per filter, so by latency where filters are few.
+// sector per element.  Bound by HBM (12 bytes an element) where a launch packs many filters.  Where it packs one (an ordinary step
+// packs each filter when its convolution comes up), by the latency of a block's loads: it takes up to 9 taps, 36 loads a thread
+// one behind the other, unless `tap_step` spreads the taps over more blocks, which read the same sectors again from L2.
 struct FilterJob {
   const float* w;
   void *hi_f, *lo_f, *hi_d, *lo_d;       // a layout that is not wanted: null
   const uint32_t* amax; uint32_t* amax_next;
   float *scale_f, *scale_d;
-  int K, C, taps, pad_f, pad_d, k_blocks, first_block;
+  int K, C, taps, pad_f, pad_d, k_blocks, c_blocks, first_block;
 };
 // MAX is 1 or kFilterJobs: the table travels as a kernel parameter, and 13 KB of it cost a launch of one filter 10 us.
 constexpr int kFilterJobs = 128, kFilterTaps = 9, kFilterTile = 32;
-template <int MAX> struct FilterJobs { int n; FilterJob job[MAX]; };
+template <int MAX> struct FilterJobs { int n, tap_step; FilterJob job[MAX]; };
 template <class E, int MAX>
 __global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant__ FilterJobs<MAX> jobs) {
   grid_dep_sync();
@@ -1618,7 +1620,8 @@ __global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant
     if (jobs.job[mid].first_block <= (int)blockIdx.x) lo = mid; else hi = mid - 1;
   }
   const FilterJob& j = jobs.job[lo];
-  const int block = blockIdx.x - j.first_block, k0 = block % j.k_blocks * kFilterTile, c0 = block / j.k_blocks * kFilterTile;
+  const int block = blockIdx.x - j.first_block, kc = block / j.k_blocks;
+  const int k0 = (block - kc * j.k_blocks) * kFilterTile, c0 = kc % j.c_blocks * kFilterTile, t0 = kc / j.c_blocks * jobs.tap_step;
   const float sc = j.amax ? scale_from_amax(__ldg(j.amax)) : 1.f;
   if (block == 0 && threadIdx.x == 0) {
     if (j.scale_f) *j.scale_f = sc;
@@ -1627,32 +1630,29 @@ __global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant
   }
   const int taps = j.taps, K = j.K, C = j.C, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   E *const hi_f = (E*)j.hi_f, *const lo_f = (E*)j.lo_f, *const hi_d = (E*)j.hi_d, *const lo_d = (E*)j.lo_d;
-  for (int t0 = 0; t0 < taps; t0 += kFilterTaps) {
-    const int nt = min(kFilterTaps, taps - t0), row = kFilterTile * nt;
-    for (int r = warp; r < kFilterTile; r += 8) {
-      const float* src = j.w + ((long long)(k0 + r) * C + c0) * taps + t0;
-      for (int e = lane; e < row; e += 32) {
-        const int c = e / nt, t = e - c * nt;
-        tile[r][e] = k0 + r < K && c0 + c < C ? __ldg(src + (long long)c * taps + t) * sc : 0.f;
-      }
+  const int nt = min(jobs.tap_step, taps - t0), row = kFilterTile * nt;
+  for (int r = warp; r < kFilterTile; r += 8) {
+    const float* src = j.w + ((long long)(k0 + r) * C + c0) * taps + t0;
+    for (int e = lane; e < row; e += 32) {
+      const int c = e / nt, t = e - c * nt;
+      tile[r][e] = k0 + r < K && c0 + c < C ? __ldg(src + (long long)c * taps + t) * sc : 0.f;
     }
-    __syncthreads();
-    const int pair = (threadIdx.x & 15) * 2, line0 = threadIdx.x >> 4;
-    for (int line = line0; line < row; line += 16) {
-      const int r = line / nt, t = line - r * nt;
-      E h0, l0, h1, l1;
-      if (hi_f && k0 + r < K && c0 + pair < j.pad_f) {
-        split_pair(tile[r][pair * nt + t], h0, l0); split_pair(tile[r][(pair + 1) * nt + t], h1, l1);
-        const long long at = ((long long)(k0 + r) * taps + t0 + t) * j.pad_f + c0 + pair;
-        store_two(hi_f + at, h0, h1); store_two(lo_f + at, l0, l1);
-      }
-      if (hi_d && c0 + r < C && k0 + pair < j.pad_d) {
-        split_pair(tile[pair][r * nt + t], h0, l0); split_pair(tile[pair + 1][r * nt + t], h1, l1);
-        const long long at = ((long long)(c0 + r) * taps + taps - 1 - t0 - t) * j.pad_d + k0 + pair;
-        store_two(hi_d + at, h0, h1); store_two(lo_d + at, l0, l1);
-      }
+  }
+  __syncthreads();
+  const int pair = (threadIdx.x & 15) * 2, line0 = threadIdx.x >> 4;
+  for (int line = line0; line < row; line += 16) {
+    const int r = line / nt, t = line - r * nt;
+    E h0, l0, h1, l1;
+    if (hi_f && k0 + r < K && c0 + pair < j.pad_f) {
+      split_pair(tile[r][pair * nt + t], h0, l0); split_pair(tile[r][(pair + 1) * nt + t], h1, l1);
+      const long long at = ((long long)(k0 + r) * taps + t0 + t) * j.pad_f + c0 + pair;
+      store_two(hi_f + at, h0, h1); store_two(lo_f + at, l0, l1);
     }
-    __syncthreads();
+    if (hi_d && c0 + r < C && k0 + pair < j.pad_d) {
+      split_pair(tile[pair][r * nt + t], h0, l0); split_pair(tile[pair + 1][r * nt + t], h1, l1);
+      const long long at = ((long long)(c0 + r) * taps + taps - 1 - t0 - t) * j.pad_d + k0 + pair;
+      store_two(hi_d + at, h0, h1); store_two(lo_d + at, l0, l1);
+    }
   }
 }
 
@@ -2285,14 +2285,24 @@ static int filter_job(ConvTc* st, int ar, const float* w, const ConvPlan* p, int
   return 0;
 }
 template <int MAX> static int launch_filter_jobs(FilterJobs<MAX>& jobs, int ar, cudaStream_t s) {
-  int blocks = 0;
   double elems = 0;
   for (int i = 0; i < jobs.n; ++i) {
     FilterJob& j = jobs.job[i];
-    j.first_block = blocks;
     j.k_blocks = (std::max(j.K, j.pad_d) + kFilterTile - 1) / kFilterTile;
-    blocks += j.k_blocks * ((std::max(j.C, j.pad_f) + kFilterTile - 1) / kFilterTile);
+    j.c_blocks = (std::max(j.C, j.pad_f) + kFilterTile - 1) / kFilterTile;
     elems += (double)j.K * j.C * j.taps;
+  }
+  // As many taps a block as still give two blocks an SM.
+  int blocks = 0;
+  for (int step : {kFilterTaps, 3, 1}) {
+    jobs.tap_step = step;
+    blocks = 0;
+    for (int i = 0; i < jobs.n; ++i) {
+      FilterJob& j = jobs.job[i];
+      j.first_block = blocks;
+      blocks += j.k_blocks * j.c_blocks * ((j.taps + step - 1) / step);
+    }
+    if (blocks >= 2 * device_sm_count()) break;
   }
   KernelTimer kt("pack_filters", s, 0, elems * (4.0 + 4.0 * elem_of(ar)));
   TF_CUDA(ar == kArithTF32 ? launch_dep(pack_filters_kernel<float, MAX>, dim3(blocks), dim3(256), 0, s, jobs) : launch_dep(pack_filters_kernel<__half, MAX>, dim3(blocks), dim3(256), 0, s, jobs));
