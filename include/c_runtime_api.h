@@ -319,8 +319,8 @@ int TfArrayCopyOnStream(DLArrayHandle from, DLArrayHandle to, void **cudaStream)
  * 0 = enqueued, 1 = out of date, record again (buffers moved or the arithmetic changed), 2 = not now (per-kernel timing
  * or the data-parallel exchange is on): use ordinary calls. */
 int TfStepRecordBegin(void **graph, void **stream_cell);
-/* While a step is recorded, before its first operator: filters[i], read by the 2-D convolution plans[i], are packed in one
- * launch, where the convolutions of the step would pack them one by one.  A hint: what is left out is packed when its
+/* Before a step's first operator: filters[i], read by the 2-D convolution plans[i], are packed in one launch unless they are
+ * already, where the convolutions of the step would pack them one by one.  A hint: what is left out is packed when its
  * convolution comes. */
 int TfPackFilters(const DLArrayHandle *filters, void ***const *plans, int n, void **cudaStream);
 int TfStepRecordEnd(void **graph, int keep);

@@ -258,6 +258,14 @@ def test_a_recording_packs_filters_for_its_own_plans_only(lib_path, monkeypatch)
     assert launches[0] == launches[-1]
 
 
+@pytest.mark.parametrize("name", ["vgg16", "resnet50", "inceptionv3"])
+def test_filters_packed_ahead_have_the_bits_of_filters_packed_one_by_one(lib_path, monkeypatch, name):
+    from tinyflow_b200 import gpu_op
+    ahead = _train(monkeypatch, False, BUILDS[name], "sgd", _overwrite_a_parameter)
+    monkeypatch.setattr(gpu_op, "pack_filters", lambda *args: None)
+    _same(ahead, _train(monkeypatch, False, BUILDS[name], "sgd", _overwrite_a_parameter))
+
+
 def test_an_allocation_gets_the_memory_of_recordings(lib_path, monkeypatch):
     """What a recording keeps for its replays is given up before an allocation fails; the steps go on as ever."""
     from tinyflow_b200 import gpu_op, ndarray

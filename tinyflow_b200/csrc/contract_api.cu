@@ -55,7 +55,6 @@ int TfTensorPathError(void) { return tensor_path_error(); }
 int TfClearTensorPathError(void) { tensor_path_error_clear(); return 0; }
 int TfPackFilters(const DLArrayHandle* filters, void*** const* plans, int n, void** cudaStream) {
   TF_REQUIRE((filters && plans) || n == 0, "TfPackFilters: null argument");
-  if (!t_recording) return 0;
   std::vector<ConvPlan*> plan;
   std::vector<const float*> data;
   std::vector<int64_t> sizes;

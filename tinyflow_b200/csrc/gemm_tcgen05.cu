@@ -2309,17 +2309,19 @@ template <int MAX> static int launch_filter_jobs(FilterJobs<MAX>& jobs, int ar, 
   TF_AFTER(s, "pack_filters");
   return 0;
 }
+static bool filter_packed(const ConvTc* st, int ar, const float* w, const ConvPlan* p, int flip) {
+  const int rows = flip ? st->eC : p->K, pad = (int)round_up(flip ? p->K : st->eC, 64);
+  return pack_valid(flip ? st->wd : st->wf, ar, w, version_of(w), 10 + flip, rows, (long long)st->eR * st->eS * pad);
+}
 // `with_other` makes the forward call produce the backward-data pack in the same launch.
 static int pack_filter(ConvTc* st, int ar, const float* w, const ConvPlan* p, int flip, bool with_other, cudaStream_t s, int* oom) {
-  const Pack& pk = flip ? st->wd : st->wf;
-  const int rows = flip ? st->eC : p->K, pad = (int)round_up(flip ? p->K : st->eC, 64);
-  if (pack_valid(pk, ar, w, version_of(w), 10 + flip, rows, (long long)st->eR * st->eS * pad)) return 0;
+  if (filter_packed(st, ar, w, p, flip)) return 0;
   FilterJobs<1> one;
   one.n = 1;
   if (int rc = filter_job(st, ar, w, p, flip ? 2 : with_other ? 3 : 1, s, oom, &one.job[0])) return rc;
   return launch_filter_jobs(one, ar, s);
 }
-// While a step is recorded: the filters that its convolutions read, each for its plan, all in one launch ahead of the
+// The filters that a step's convolutions read, each for its plan: those that are not packed already, in one launch ahead of the
 // convolutions that find them packed.  What it leaves out the convolution packs when it comes up.
 int tc_pack_filters(ConvPlan* const* plans, const float* const* filters, const int64_t* sizes, int n, cudaStream_t s) {
   if (contraction_path_is_cuda_cores() || !encode_fn()) return 0;
@@ -2332,6 +2334,7 @@ int tc_pack_filters(ConvPlan* const* plans, const float* const* filters, const i
     if (!st || !st->cls || sizes[i] != (int64_t)p->K * p->C * p->R * p->S) continue;
     std::lock_guard<std::mutex> lk(st->mu);
     if (!st->wf.hi || st->wf.arith != ar || (ar == kArithF16 && !amax_tracked(filters[i]))) continue;
+    if (filter_packed(st, ar, filters[i], p, 0) && (!st->dgrad_seen || filter_packed(st, ar, filters[i], p, 1))) continue;
     int oom = 0;
     if (filter_job(st, ar, filters[i], p, st->dgrad_seen ? 3 : 1, s, &oom, &jobs.job[jobs.n])) continue;
     if (++jobs.n < kFilterJobs) continue;

@@ -26,7 +26,7 @@ import warnings
 import weakref
 
 from . import gpu_op, ndarray, step_graph
-from .graph import (AddOp, AdamOp, OnesLikeOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
+from .graph import (AddOp, AdamOp, Convolution2DForwardOp, OnesLikeOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
 
 
 def getcomputelist(Variable_node_list, Variable_node_grad_list, b1, b2, b1t, b2t, e, learning_rate):
@@ -187,6 +187,9 @@ class Executor(object):
         self.ctx_cpu, self.ctx_gpu = ndarray.cpu(0), ndarray.gpu(0)
         self.node_to_shape_map = None
         self.feed_shapes = None
+        # convolutions of a fed filter, and their descriptors as the library takes them (with the objects behind)
+        self._convs = [n for n in self.topo_order if type(n.op) is Convolution2DForwardOp and not n.inputs[1].inputs]
+        self._conv_cells = ([], None)
         self._values = {}          # node index -> NDArray on the GPU (None while swapped out)
         self._feed = {}            # what the most recent run was fed: node -> NDArray on the GPU
         self._leases = {}          # node index -> weak references to the views of its array that were handed out
@@ -365,6 +368,12 @@ class Executor(object):
             else:
                 gpu_op.adam_update_many(arrays[0], arrays[1], arrays[2], arrays[3], *rule, stream)
 
+    def _pack_filters(self, stream):
+        cells = [n.cudnnlist[0] for n in self._convs]
+        if len(self._conv_cells[0]) != len(cells) or any(a is not b for a, b in zip(self._conv_cells[0], cells)):
+            self._conv_cells = (cells, gpu_op.cell_array(cells))
+        gpu_op.pack_filters([self._feed[n.inputs[1]] for n in self._convs], self._conv_cells[1], stream)
+
     def _issue(self, feed_dict, stream, recording=False):
         """Issues every node's calls on ``stream``.  Returns (arrays by node index, loss array)."""
         # Without a plan a node writes the array it wrote in the previous step, unless a caller still looks at that.  Under
@@ -381,6 +390,8 @@ class Executor(object):
         shapes, timed = self.node_to_shape_map, self.top_message_queue is not None
         together = not (self.have_plan or timed or gpu_op.data_parallel_active())
         updates = []
+        if together and self._convs and all(n.inputs[1] in self._feed for n in self._convs):
+            self._pack_filters(stream)
         for node in self.topo_order:
             if not node.inputs and node in self._feed:
                 if self.have_plan:

@@ -423,9 +423,13 @@ def handle_array(arrs):
     return (_nd.DLArrayHandle * len(arrs))(*[_h(a) for a in arrs])
 
 
-def pack_filters(filters, cudnnlists, cudaStream):
-    """While a step is recorded: packs the filter of every (filter, convolution descriptor) pair in one launch."""
-    cells = (ctypes.c_void_p * len(cudnnlists))(*[ctypes.cast(c, ctypes.c_void_p) for c in cudnnlists])
+def cell_array(cudnnlists):
+    """The C array of descriptor cells :func:`pack_filters` takes (the cells have to outlive it)."""
+    return (ctypes.c_void_p * len(cudnnlists))(*[ctypes.cast(c, ctypes.c_void_p) for c in cudnnlists])
+
+
+def pack_filters(filters, cells, cudaStream):
+    """At the start of a step: packs ``filters[i]`` for the 2-D convolution ``cells[i]``, all in one launch."""
     check_call(_LIB.TfPackFilters(handle_array(filters), cells, len(filters), cudaStream))
 
 

@@ -20,7 +20,6 @@ import weakref
 
 from . import gpu_op, ndarray
 from ._base import _LIB, check_call, last_error, new_cell
-from .graph import Convolution2DForwardOp
 
 ENABLED = os.environ.get("TINYFLOW_STEP_GRAPH", "1") != "0"
 RUNS_BEFORE_RECORDING = 2        # of the same arrays: the first calls of a plan still learn what follows what
@@ -122,8 +121,6 @@ def record(executor, feed_dict, staged):
         return None
     values, loss, keep, stopped = {}, None, 0, None
     try:
-        convs = [n for n in executor.topo_order if type(n.op) is Convolution2DForwardOp and feed_dict.get(n.inputs[1]) is not None]
-        gpu_op.pack_filters([feed_dict[n.inputs[1]] for n in convs], [n.cudnnlist[0] for n in convs], stream)
         values, loss = executor._issue(feed_dict, stream, recording=True)
         keep = 1
     except Exception as e:                      # whatever stopped it: the caller runs the step as ordinary calls and says so
