@@ -1,4 +1,7 @@
 """Which steps are recorded, and on whose arrays (no device code)."""
+import gc
+import weakref
+
 import pytest
 
 from tinyflow_b200 import step_graph
@@ -39,3 +42,30 @@ def test_recordings_that_a_sequence_of_batches_makes(order, made):
 def test_arrays_that_keep_coming_in_turn_get_recordings_of_their_own():
     n = step_graph.RUNS_WITHOUT_STAGING
     assert _replay("AB" * (n + 2)) == [(4, True), (2 * n, False), (2 * n + 1, False)]
+
+
+@pytest.mark.parametrize("drop", ["clear", "batch array", "parameter", "table full"])
+def test_a_dropped_recording_goes_at_once(drop):
+    """Its device memory does not wait for the garbage collector."""
+    table, w, x = step_graph.Recordings(), _Node(1), _Node(2)
+    weights, batch = _Array(), _Array()
+    entry, _, _ = table.choose({w: weights, x: batch})
+    recording = entry.recording = _Array()
+    gone = weakref.ref(recording)
+    del entry, recording
+    gc.collect()
+    gc.disable()
+    try:
+        if drop == "clear":
+            table.clear()
+        elif drop == "batch array":
+            del batch
+        elif drop == "parameter":
+            del weights
+        else:
+            kept = [_Array() for _ in range(step_graph.MAX_FEEDS)]
+            for other in kept:
+                table.choose({w: other, x: batch})
+        assert gone() is None
+    finally:
+        gc.enable()

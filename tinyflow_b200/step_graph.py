@@ -53,12 +53,17 @@ class Recording(object):
         return rc
 
 
+class _Table(dict):
+    """Entries by key.  The entries refer to it weakly: a dropped one, and what was recorded for it, goes at once."""
+    __slots__ = ("__weakref__",)
+
+
 class _Feed(object):
     """How often a set of arrays was run, how often since another one, and what was recorded for it."""
     __slots__ = ("runs", "in_a_row", "refs", "recording", "batches", "latest", "__weakref__")
 
     def __init__(self):
-        self.runs, self.in_a_row, self.refs, self.recording, self.batches, self.latest = 0, 0, None, None, {}, None
+        self.runs, self.in_a_row, self.refs, self.recording, self.batches, self.latest = 0, 0, None, None, _Table(), None
 
     def settled(self):
         """Worth a recording on the arrays themselves."""
@@ -67,7 +72,7 @@ class _Feed(object):
 
 class Recordings(object):
     def __init__(self):
-        self.sets = {}
+        self.sets = _Table()
 
     def clear(self):
         self.sets.clear()
@@ -78,7 +83,7 @@ class Recordings(object):
         if entry is None:
             entry = _Feed()
             # (bound here: at interpreter exit the module's names go before the arrays do)
-            gone = lambda _ref, t=weakref.ref(entry), k=key, forget=_forget: forget(table, k, t)     # noqa: E731
+            gone = lambda _ref, t=weakref.ref(table), e=weakref.ref(entry), k=key, forget=_forget: forget(t(), k, e())     # noqa: E731
             entry.refs = [weakref.ref(a, gone) for a in arrays]
             while len(table) >= MAX_FEEDS:
                 del table[next(iter(table))]
@@ -104,9 +109,8 @@ class Recordings(object):
         return top if staged else below, staged, wanted
 
 
-def _forget(table, key, entry_ref):
-    entry = entry_ref()
-    if entry is not None and table.get(key) is entry:
+def _forget(table, key, entry):
+    if table is not None and entry is not None and table.get(key) is entry:
         del table[key]
 
 
