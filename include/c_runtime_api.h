@@ -356,6 +356,9 @@ int TfTensorPathTimeoutProbe(long long limit_cycles, void **cudaStream);
 int TfLastError(char *buf, int buflen);   /* message of the last -1 return on this thread */
 int TfAllocatorStats(long long *bytes_in_use, long long *bytes_cached);
 int TfReleaseCachedMemory(void);
+/* Device memory that a convolution, pooling or batch-norm descriptor keeps from call to call goes back to the pool; for a
+ * descriptor that is no longer used (its cell and slots stay the caller's).  What a recorded step still writes stays. */
+int TfReleaseDescriptor(void ***cudnnlist);
 int TfSetMemoryLimit(long long bytes);    /* device memory the pool of each GPU may own, cached blocks included; 0 = no limit */
 
 #ifdef __cplusplus

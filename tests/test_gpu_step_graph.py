@@ -292,6 +292,29 @@ def test_an_allocation_gets_the_memory_of_recordings(lib_path, monkeypatch):
     _same(got, _train(monkeypatch, False, build, "sgd"))
 
 
+@pytest.mark.parametrize("recorded", [False, True])
+@pytest.mark.parametrize("name", ["vgg16", "resnet50", "inceptionv3"])
+def test_changes_of_the_batch_size_keep_no_memory(lib_path, monkeypatch, name, recorded):
+    """A last, smaller batch comes with every epoch: what the descriptors of one size keep goes back with them."""
+    from tinyflow_b200 import autodiff as ad, gpu_op, models, ndarray, step_graph
+    monkeypatch.setattr(step_graph, "ENABLED", recorded)
+    model = CONV_FIRST.get(name, BUILDS[name])(models)
+    ex = ad.Executor(model.loss, model.y, 0.001, None, None, None, optimizer="sgd")
+    ctx = ndarray.gpu(0)
+    feed = {n: ndarray.array(v, ctx) for n, v in model.init_params(seed=5).items()}
+    X, Y = models.synthetic_batch(model, seed=8)
+    batches = {n: (ndarray.array(X[:n], ctx), ndarray.array(Y[:n], ctx)) for n in (X.shape[0], X.shape[0] - 3)}
+    used = []
+    for epoch in range(4):
+        for n in sorted(batches, reverse=True):
+            feed[model.X], feed[model.y_] = batches[n]
+            for _ in range(5):
+                ex.run(feed)
+        gpu_op.device_synchronize()
+        used.append(gpu_op.allocator_stats()[0])
+    assert used[3] - used[1] <= 64 * 1024, used
+
+
 @pytest.mark.parametrize("count", [1, 5, 400])
 def test_many_updates_in_one_launch(lib_path, count):
     from tinyflow_b200 import gpu_op, ndarray as nd

@@ -128,6 +128,7 @@ __device__ __forceinline__ void amax_commit(const AmaxOut& am, uint32_t m) {
 // ---- producers that feed the tensor path ------------------------------------------------------------
 // y = relu(x) fused with the packing of y for the convolution expected to read it (see gemm_tcgen05.cu); 1 = done,
 // 0 = not applicable (run the plain kernel), -1 = error.
+void tc_release(void* tc_state);               // the packs of a convolution plan that no call will use again
 int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cudaStream_t s);
 void tc_note_relu_output(const void* node, const void* y);     // the plain ReLU of graph node `node` wrote y (after the version bump)
 bool contraction_path_is_cuda_cores();
@@ -154,6 +155,7 @@ void* recording_take_block(size_t bytes);          // a block of exactly this (r
 void recording_keep_block(void* p, size_t bytes);  // instead of handing the block back to the pool
 const uint32_t* recording_seed(unsigned seed);     // device word that will hold the seed of this dropout call at every replay
 const float* recording_adam_corrections(float c1, float c2);   // two device words with this step's bias corrections
+bool recordings_use(const void* const* source);    // some finished recording called recording_note_made(source)
 bool recordings_give_up_memory();                  // every recording that is not being made returns its blocks to the pool and is out of date; false: there was none
 void recording_note_launches(int n);
 void recording_note_write(const void* p);
@@ -301,7 +303,7 @@ struct BNPlan {
   float* save_mean;      // library-owned, sized to the statistic count
   float* save_inv;
   int64_t nstat;
-  const float* last_y;   // output of the last forward call and its write version: a ReLU gradient whose mask tensor is
+  const void* last_y;    // output of the last forward call and its write version: a ReLU gradient whose mask tensor is
   uint64_t last_y_version;   // still exactly that output can take its mask from x-hat instead of reading the tensor
 };
 struct DropoutState {

@@ -2107,6 +2107,18 @@ static ConvTc* conv_state(ConvPlan* p) {
   return (ConvTc*)p->tc_state;
 }
 
+// The state itself stays: notes of producers may name it.  So do packs that a recording writes.
+void tc_release(void* tc_state) {
+  ConvTc* st = (ConvTc*)tc_state;
+  if (!st) return;
+  std::lock_guard<std::mutex> lk(st->mu);
+  for (Pack* pk : {&st->x, &st->dy, &st->wf, &st->wd}) {
+    if (recordings_use(&pk->src)) continue;
+    pack_release(*pk);
+    pk->src = nullptr;
+  }
+}
+
 // One launch of the frame pack: `chans` channels of an NCHW tensor (spatial dims H x W) into columns dst_c0 .. dst_c0 + cover
 // of pk (zeros past `chans`)
 static int launch_pack_nchw(Pack& pk, const ScaleRef& sr, const float* src, int N, int chans, int H, int W, int frame_h, int frame_w, int off_h, int off_w,

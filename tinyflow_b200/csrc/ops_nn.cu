@@ -846,6 +846,7 @@ int DLGpuBatchNormalizationForward(const DLArrayHandle input, DLArrayHandle outp
   float* y = out_f32(output);
   note_compute_stream(s);
   KernelTimer kt("DLGpuBatchNormalizationForward", s, 0, 8.0 * numel(input) + 8.0 * p->nstat);
+  if (t_recording) recording_note_made(&p->last_y);
   if (p->mode == 0) {
     int64_t F = p->nstat;
     int N = (int)p->N;
@@ -856,6 +857,23 @@ int DLGpuBatchNormalizationForward(const DLArrayHandle input, DLArrayHandle outp
     launch_plain(bn_sp_fwd_kernel, dim3((unsigned)p->C), dim3(512), 0, s, x, y, p->save_mean, p->save_inv, p->N, p->C, p->HW);
   }
   TF_AFTER(s, "DLGpuBatchNormalizationForward");
+  return 0;
+}
+
+// The device memory that a descriptor keeps from call to call (packed operands, indices of maxima, saved statistics) goes back to
+// the pool.  A later call on the descriptor starts anew.
+int TfReleaseDescriptor(void*** cudnnlist) {
+  if (ConvPlan* p = plan_of<ConvPlan>(cudnnlist, kPlanConv)) {
+    flush_deferred();
+    tc_release(p->tc_state);
+  } else if (PoolPlan* p = plan_of<PoolPlan>(cudnnlist, kPlanPool)) {
+    if (p->argmax && !recordings_use(&p->argmax_src)) { pool_free(p->argmax); p->argmax = nullptr; p->argmax_src = nullptr; }
+  } else if (BNPlan* p = plan_of<BNPlan>(cudnnlist, kPlanBN)) {
+    if (p->save_mean && !recordings_use(&p->last_y)) {
+      pool_free(p->save_mean); pool_free(p->save_inv);
+      p->save_mean = p->save_inv = nullptr; p->last_y = nullptr;
+    }
+  }
   return 0;
 }
 

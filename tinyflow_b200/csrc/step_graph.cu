@@ -171,6 +171,12 @@ void amax_of_array(const float* src, int64_t n, uint32_t* word, cudaStream_t s);
 // Finished recordings.  The lock is held while one is replayed, freed or made to give up its memory.
 static std::mutex g_graphs_mu;
 static std::vector<StepGraph*> g_graphs;
+// A finished recording writes the data that a plan keeps beside *source.
+bool recordings_use(const void* const* source) {
+  std::lock_guard<std::mutex> lk(g_graphs_mu);
+  for (const StepGraph* g : g_graphs) if (std::binary_search(g->made.begin(), g->made.end(), (const void**)source)) return true;
+  return false;
+}
 static void step_graph_release(StepGraph* g) {
   if (g->exec) cudaGraphExecDestroy(g->exec);
   if (g->graph) cudaGraphDestroy(g->graph);

@@ -26,7 +26,7 @@ import warnings
 import weakref
 
 from . import gpu_op, ndarray, step_graph
-from .graph import (AddOp, AdamOp, Convolution2DForwardOp, OnesLikeOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
+from .graph import (AddOp, AdamOp, BNForwardOp, Convolution2DForwardOp, OnesLikeOp, Pooling2DForwardOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
 
 
 def getcomputelist(Variable_node_list, Variable_node_grad_list, b1, b2, b1t, b2t, e, learning_rate):
@@ -236,7 +236,10 @@ class Executor(object):
             if node in self.node_to_shape_map:
                 continue
             input_shapes = [self.node_to_shape_map[i] for i in node.inputs]
+            replaced = node.cudnnlist[0] if isinstance(node.op, (Convolution2DForwardOp, Pooling2DForwardOp, BNForwardOp)) else 0
             self.node_to_shape_map[node] = tuple(node.op.infer_shape(node, input_shapes, self.cudnnHandle))
+            if replaced:                     # the descriptor of earlier shapes: what it keeps on the device goes back
+                gpu_op.release_descriptor(replaced)
 
     # ---- memory-plan messages ---------------------------------------------------------------------
     def _apply_plan(self, swap_list, release_list, recompute_list):

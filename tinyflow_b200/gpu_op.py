@@ -495,6 +495,11 @@ def allocator_stats():
     return used.value, cached.value
 
 
+def release_descriptor(cudnnlist):
+    """Device memory that a replaced operator descriptor keeps goes back to the pool."""
+    check_call(_LIB.TfReleaseDescriptor(cudnnlist))
+
+
 def set_memory_limit(nbytes):
     """Device memory the pool of each GPU may own, cached blocks included; 0 = no limit."""
     check_call(_LIB.TfSetMemoryLimit(ctypes.c_longlong(nbytes)))
