@@ -102,7 +102,7 @@ const uint32_t* amax_tracked(const void* data);
 // The maximum of a tensor that a recorded step reads before it writes it (see step_graph.cu): `carry` keeps the value
 // between replays, valid while the tensor's version is `*version`.
 struct AmaxCarry { const void* data; uint32_t* carry; const uint32_t* from; };       // from: the word the step itself writes, or null
-bool amax_take_carries(StepGraph* g, AmaxCarry* out, int max, int* count);           // the carries the recording g asked for
+bool amax_take_carries(uint64_t recording, AmaxCarry* out, int max, int* count);     // the carries that recording asked for; false: more than max
 bool amax_carry_valid(const void* data);
 void amax_set_carry_valid(const void* data);
 void bump_versions(const void* const* ptrs, size_t n);

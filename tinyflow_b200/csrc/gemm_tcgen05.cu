@@ -74,7 +74,7 @@ void invalidate_all_versions() {
 struct AmaxSlot {
   uint32_t* words = nullptr; unsigned uses = 0; uint64_t version = 0; int cur = 0;
   uint32_t* carry = nullptr; uint64_t carry_version = 0;
-  const StepGraph* rec = nullptr; uint32_t* rec_word = nullptr; uint64_t rec_version = 0; bool rec_wants_carry = false;
+  uint64_t rec = 0; uint32_t* rec_word = nullptr; uint64_t rec_version = 0; bool rec_wants_carry = false;
 };
 static std::unordered_map<const void*, AmaxSlot> g_amax;
 static uint32_t* g_amax_chunk = nullptr;
@@ -99,7 +99,7 @@ static uint32_t* amax_chunk_words(int n) {
   return w;
 }
 static void amax_enter_recording(AmaxSlot& sl) {
-  if (sl.rec != t_recording) { sl.rec = t_recording; sl.rec_word = nullptr; sl.rec_version = 0; sl.rec_wants_carry = false; }
+  if (sl.rec != recording_id()) { sl.rec = recording_id(); sl.rec_word = nullptr; sl.rec_version = 0; sl.rec_wants_carry = false; }
 }
 AmaxOut amax_track_begin(const void* data) {
   std::lock_guard<std::mutex> lk(g_ver_mu);
@@ -122,7 +122,7 @@ const uint32_t* amax_tracked(const void* data) {
   if (it == g_amax.end()) return nullptr;
   AmaxSlot& sl = it->second;
   const uint64_t v = version_locked(data);
-  if (t_recording && sl.rec == t_recording && sl.rec_word && sl.rec_version == v) return sl.rec_word;
+  if (t_recording && sl.rec == recording_id() && sl.rec_word && sl.rec_version == v) return sl.rec_word;
   const uint32_t* found = sl.words && sl.version == v ? sl.words + sl.cur : (sl.carry && sl.carry_version == v ? sl.carry : nullptr);
   if (!t_recording || !found) return found;
   // read before the recorded step has written it: at a replay the value has to come from the step before
@@ -131,18 +131,18 @@ const uint32_t* amax_tracked(const void* data) {
   sl.rec_wants_carry = true;
   return sl.carry;
 }
-bool amax_take_carries(StepGraph* g, AmaxCarry* out, int max, int* count) {
+bool amax_take_carries(uint64_t recording, AmaxCarry* out, int max, int* count) {
   std::lock_guard<std::mutex> lk(g_ver_mu);
   *count = 0;
   for (auto& kv : g_amax) {
     AmaxSlot& sl = kv.second;
-    if (sl.rec != g) continue;
+    if (sl.rec != recording) continue;
     if (sl.rec_wants_carry) {
       if (*count >= max) return false;
       const bool rewritten = sl.rec_word && sl.rec_version == version_locked(kv.first);     // by a kernel that tracks its maximum, last
       out[(*count)++] = AmaxCarry{kv.first, sl.carry, rewritten ? sl.rec_word : nullptr};
     }
-    sl.rec = nullptr;
+    sl.rec = 0;
   }
   return true;
 }

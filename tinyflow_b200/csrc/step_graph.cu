@@ -244,17 +244,13 @@ int TfStepRecordEnd(void** graph, int keep) {
   if (ok) {
     g->carries.resize(kCarries);
     int n = 0;
-    ok = amax_take_carries(g, g->carries.data(), kCarries, &n);
+    ok = amax_take_carries(g->id, g->carries.data(), kCarries, &n);
     if (!ok) recording_refuse("more parameters with a tracked maximum than a recording carries");
     g->carries.resize(n);
     CarryList list;
     int m = 0;
     for (const AmaxCarry& c : g->carries) if (c.from) { list.from[m] = c.from; list.to[m] = c.carry; ++m; }
     if (ok && m) { launch_plain(step_carry_kernel, dim3(1), dim3(256), 0, g->stream, list, m); g->launches += 1; }
-  } else {
-    int n = 0;
-    AmaxCarry none;
-    while (!amax_take_carries(g, &none, 1, &n)) {}
   }
   ok = ok && !g->refused;
   if (ok) {
