@@ -7,7 +7,7 @@
 // and the tile is added up through distributed shared memory, every CTA one slice of it, in rank order (bit-reproducible,
 // no workspace, no second kernel).  The next K block is fetched into registers while the current one is multiplied.
 //
-// Measured (B200, device time; the kernel this replaces in parentheses): see the table at pick_config().
+// Measured against the kernel it replaced and against the tensor path: the table in simt_matmul(), where the tile is chosen.
 #include "common.h"
 #include <cooperative_groups.h>
 
@@ -172,8 +172,8 @@ int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int6
   const int sms = device_sm_count();
   // Tile: 8 rows where there are no more (the rest of a taller tile would multiply nothing), 64 x 64 once those alone
   // give every SM one, else 32 x 32.  Cluster: the smallest power of two that occupies the SMs, with at least two K
-  // blocks to each CTA; the 8-row tile only streams the weights and wants several CTAs per SM, so it may take the
-  // non-portable 16.
+  // blocks to each CTA, at most 8; the 8-row tile only streams the weights and wants several CTAs per SM, so it may
+  // take the non-portable 16.
   //   M x K x N          this kernel   before      tensor path with its packs (us, back to back)
   //   64 x 784 x 256         6.4         20             19.0
   //   1000 x 256 x 100       6.7         22             15.6

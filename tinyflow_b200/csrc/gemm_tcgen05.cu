@@ -14,14 +14,17 @@
 //                     is a run-time flag that only changes the TMA box shape and the UMMA descriptor.
 //   conv forward      activations packed pixel-major [N * frame_h * frame_w][C] with the zero halo
 //                     materialised, filters packed [Cout][tap][C]; a filter tap is then a constant
-//                     row shift of the activation matrix, so the K loop is (tap, 64-channel chunk)
-//                     and each step is two plain 2-D TMA boxes.  Outputs computed for halo anchors
-//                     are discarded by the epilogue.
+//                     row shift of the activation matrix.  The K loop takes 64 channels at a time and
+//                     walks the taps for them: one 2-D TMA box of up to 192 activation rows serves
+//                     every tap whose shift lies inside it, and a tap's filter tile is a box of its own.
+//                     Outputs computed for halo anchors are discarded by the epilogue.
 //   conv backward-data  same kernel on the packed output gradient with the flipped filter
 //                     [Cin][tap'][Cout]; a strided 1x1 scatters into a zeroed dx.
 //   conv backward-filter  dW[k][c][tap] = sum_rows dy[row][k] * x[row + shift(tap)][c]: both operands
-//                     are M/N-major, the reduction runs over pixel rows, split over CTAs and combined
-//                     with fp32 atomics.
+//                     are M/N-major, the reduction runs over pixel rows.
+//
+// A last wave that is not full, and products of few tiles, cut their reductions over CTAs: raw partial sums, added in a fixed
+// order through a workspace or a cluster's shared memory.  No atomics on sums: the same bits on every run.
 //
 // Kernel roles (384 threads): warps 0 and 11 = TMA producers of A and B, warp 1 = TMEM owner and issuer of the wide MMAs, warp
 // 10 = issuer of the narrow ones, warps 2-9 = epilogue (two per TMEM lane quarter, half the columns each).  Shared memory holds
