@@ -29,7 +29,7 @@ constexpr int kSeedWords = 1022;          // dropout calls of a step
 constexpr int kCarries = 1024;            // parameters whose maximum crosses steps
 
 struct StepGraph {
-  cudaStream_t stream = nullptr;          // the calls of the recording name it; nothing runs on it
+  cudaStream_t stream = nullptr;          // the calls of the recording name it (name_stream)
   cudaGraph_t graph = nullptr;
   cudaGraphNode_t last = nullptr;         // the node every next one waits for
   bool last_is_kernel = false;
@@ -180,10 +180,9 @@ bool recordings_use(const void* const* source) {
 static void step_graph_release(StepGraph* g) {
   if (g->exec) cudaGraphExecDestroy(g->exec);
   if (g->graph) cudaGraphDestroy(g->graph);
-  if (g->stream) cudaStreamDestroy(g->stream);
   if (g->words) pool_free(g->words);
   for (auto& kv : g->free_blocks) for (void* p : kv.second) pool_free(p);
-  g->exec = nullptr; g->graph = nullptr; g->stream = nullptr; g->words = nullptr;
+  g->exec = nullptr; g->graph = nullptr; g->words = nullptr;
   g->free_blocks.clear();
   cudaGetLastError();
 }
@@ -205,6 +204,17 @@ bool recordings_give_up_memory() {
   return true;
 }
 
+// The stream that recorded calls name: one per device, so that a recording neither creates nor destroys one.  Nothing runs on it.
+static cudaStream_t name_stream() {
+  static std::mutex mu;
+  static cudaStream_t streams[64] = {nullptr};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) { cudaGetLastError(); return nullptr; }
+  std::lock_guard<std::mutex> lk(mu);
+  if (!streams[dev] && cudaStreamCreateWithFlags(&streams[dev], cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); streams[dev] = nullptr; }
+  return streams[dev];
+}
+
 }  // namespace tf
 using namespace tf;
 
@@ -219,7 +229,8 @@ int TfStepRecordBegin(void** graph, void** stream_cell) {
   StepGraph* g = new StepGraph;
   g->words = (uint32_t*)pool_alloc(sizeof(uint32_t) * (kZeroedWords + 2 + kSeedWords));
   if (!g->words) { delete g; return 1; }
-  if (cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking) != cudaSuccess || cudaGraphCreate(&g->graph, 0) != cudaSuccess) {
+  g->stream = name_stream();
+  if (!g->stream || cudaGraphCreate(&g->graph, 0) != cudaSuccess) {
     step_graph_free(g);
     TF_FAIL("TfStepRecordBegin: no stream or graph could be created");
   }
