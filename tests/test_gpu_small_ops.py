@@ -125,3 +125,35 @@ def test_reductions_without_a_stream_read_a_sum_just_issued(env, call):
         op.reduce_sum(total, out, -1 if call == "all" else 1)
     s = (a + b).astype(np.float64)
     assert np.all(np.abs(out.asnumpy() - s.sum(axes).reshape(result)) <= 2e-6 * np.abs(s).sum(axes).reshape(result))
+
+
+def test_split_reductions_in_a_capture_of_the_callers_own(env):
+    """The scratch of a stream that is first used while its caller captures it is not part of the capture."""
+    import ctypes
+    import torch
+    nd, op = env.nd, env.gpu_op
+    rng = np.random.RandomState(6)
+    logits, labels = nd.array(rng.randn(2000, 37).astype(np.float32), env.ctx), nd.array(np.eye(37, dtype=np.float32)[rng.randint(0, 37, 2000)], env.ctx)
+    x, plan = nd.array(rng.randn(64, 16, 33, 32).astype(np.float32), env.ctx), op.reduce_sum_get_cudnnlist((64, 16, 33, 32), (1, 16, 1, 1), "NCHW", env.cudnn)
+    want, got = ([nd.empty((1,), env.ctx), nd.empty((1, 16, 1, 1), env.ctx)] for _ in range(2))
+
+    def work(out, stream):
+        op.softmax_cross_entropy(logits, labels, out[0], stream)
+        op.reduce_sum_new(x, out[1], plan, env.cudnn, stream)
+    work(want, env.stream)
+    op.device_synchronize()
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    cell = ctypes.pointer(ctypes.c_void_p(side.cuda_stream))
+    with torch.cuda.graph(graph, stream=side):
+        work(got, cell)
+    for _ in range(3):
+        for v in got:
+            v[:] = np.zeros(v.shape, np.float32)
+        graph.replay()
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            np.testing.assert_array_equal(a.asnumpy(), b.asnumpy())
+    work(got, cell)                                      # and as ordinary calls on that stream
+    op.device_synchronize()
+    for a, b in zip(got, want):
+        np.testing.assert_array_equal(a.asnumpy(), b.asnumpy())

@@ -255,6 +255,7 @@ inline cudaError_t launch_cluster(void (*kernel)(Params...), int cluster, dim3 g
 }
 #endif
 cudaError_t clear_on_stream(void* p, size_t bytes, cudaStream_t s);                       // cudaMemsetAsync(p, 0, bytes, s), and its node
+cudaError_t clear_now(void* p, size_t bytes);                                             // of new memory, complete on return
 cudaError_t copy_on_stream(void* to, const void* from, size_t bytes, cudaStream_t s);     // device to device
 
 // ---- plan structs stored in slot 0 of a descriptor list ----------------------

@@ -86,12 +86,7 @@ static uint32_t* amax_chunk_words(int n) {
   if (g_amax_left < n) {
     const int kWords = 16384;
     uint32_t* chunk = nullptr;
-    // cleared on a stream of its own: the words are needed on any stream, and waiting for the device would wait for other threads' work
-    cudaStream_t clearing = nullptr;
-    const bool ok = cudaStreamCreateWithFlags(&clearing, cudaStreamNonBlocking) == cudaSuccess && cudaMalloc((void**)&chunk, kWords * sizeof(uint32_t)) == cudaSuccess &&
-                    cudaMemsetAsync(chunk, 0, kWords * sizeof(uint32_t), clearing) == cudaSuccess && cudaStreamSynchronize(clearing) == cudaSuccess;
-    if (clearing) cudaStreamDestroy(clearing);
-    if (!ok) {
+    if (cudaMalloc((void**)&chunk, kWords * sizeof(uint32_t)) != cudaSuccess || clear_now(chunk, kWords * sizeof(uint32_t)) != cudaSuccess) {
       cudaGetLastError();
       return nullptr;
     }

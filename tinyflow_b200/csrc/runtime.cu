@@ -98,6 +98,24 @@ void KernelTimer::end() {
   if (slot >= 0 && slot < (int)g_pending.size()) cudaEventRecord(g_pending[slot].b, stream);
 }
 
+// A caller may capture its own streams: allocations and the clearing of new counters are not part of what is captured.
+struct RelaxedCapture {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+  ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+// Zeroes memory that no kernel uses yet, on a stream of its own and before it returns.
+cudaError_t clear_now(void* p, size_t bytes) {
+  const RelaxedCapture allowed;
+  cudaStream_t s = nullptr;
+  cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMemsetAsync(p, 0, bytes, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  if (s) cudaStreamDestroy(s);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e;
+}
+
 static std::atomic<cudaStream_t> g_compute_stream{(cudaStream_t)0};
 void note_compute_stream(cudaStream_t s) { if (!t_recording) g_compute_stream.store(s, std::memory_order_relaxed); }     // a recording's stream concerns nobody else
 cudaStream_t legacy_stream() { flush_deferred(); return t_recording ? recording_stream() : (cudaStream_t)0; }
@@ -203,6 +221,7 @@ struct Pool {
   cudaError_t raw_alloc(void** p, size_t b) {
     const long long limit = host ? 0 : g_memory_limit.load(std::memory_order_relaxed);
     if (limit > 0 && in_use + cached + (long long)b > limit) return cudaErrorMemoryAllocation;
+    const RelaxedCapture allowed;
     return host ? cudaHostAlloc(p, b, cudaHostAllocDefault) : cudaMalloc(p, b);
   }
   void raw_free(void* p) { host ? cudaFreeHost(p) : cudaFree(p); }
@@ -339,7 +358,7 @@ static void* scratch_block(int slot, size_t bytes, cudaStream_t s) {
   const size_t want = std::max(bytes + bytes / 4, sc->cap[slot] + sc->cap[slot] / 2), got = Pool::round(want);
   lk.unlock();
   void* p = device_pool().alloc(want, nullptr, true);
-  if (p && slot == kCounterSlot && cudaMemsetAsync(p, 0, got, s) != cudaSuccess) { cudaGetLastError(); pool_free(p); p = nullptr; }
+  if (p && slot == kCounterSlot && clear_now(p, got) != cudaSuccess) { pool_free(p); p = nullptr; }
   if (!p) return nullptr;
   lk.lock();
   sc = &g_scratch[key];
