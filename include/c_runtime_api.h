@@ -313,12 +313,13 @@ int TfAdamUpdateMany(const DLArrayHandle *w, const DLArrayHandle *m, const DLArr
 int TfArrayCopyOnStream(DLArrayHandle from, DLArrayHandle to, void **cudaStream);
 
 /* Recording a step and replaying it with one call.  Between Begin and End the calling thread issues the step's calls on
- * the stream Begin returns; they are recorded, not executed.  The arrays the calls name have to outlive the recording.
+ * the stream Begin returns; they are recorded, not executed.  Replays go to *replay_stream, whose scratch they share.
+ * The arrays the calls name have to outlive the recording.
  * Copies that the host waits for, and calls on other streams, cannot be recorded: they fail or do nothing, and End returns 1
  * then, as it does with keep = 0.  TfStepReplay: `seeds` for the dropout calls in order, Adam's beta powers of this step;
  * 0 = enqueued, 1 = out of date, record again (buffers moved or the arithmetic changed), 2 = not now (per-kernel timing
  * or the data-parallel exchange is on): use ordinary calls. */
-int TfStepRecordBegin(void **graph, void **stream_cell);
+int TfStepRecordBegin(void **graph, void **stream_cell, void **replay_stream);
 /* Before a step's first operator: filters[i], read by the 2-D convolution plans[i], are packed in one launch unless they are
  * already, where the convolutions of the step would pack them one by one.  A hint: what is left out is packed when its
  * convolution comes. */

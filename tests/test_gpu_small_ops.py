@@ -157,3 +157,33 @@ def test_split_reductions_in_a_capture_of_the_callers_own(env):
     op.device_synchronize()
     for a, b in zip(got, want):
         np.testing.assert_array_equal(a.asnumpy(), b.asnumpy())
+
+
+@pytest.mark.parametrize("streams", [1, 2])
+def test_products_of_two_threads(env, streams):
+    """Packs and partial sums lie in the stream's scratch: two threads on one stream, or on two, do not disturb each other."""
+    import threading
+    nd, op, runs = env.nd, env.gpu_op, 40
+    rng = np.random.RandomState(3)
+    cells = [env.stream, env.stream if streams == 1 else op.create_cudaStream()]
+    shapes = [(700, 2048, 900), (640, 1500, 520)]                    # tensor path, reductions split over CTAs
+    state = [(nd.array(rng.randn(M, K).astype(np.float32), env.ctx), nd.array(rng.randn(K, N).astype(np.float32), env.ctx),
+              [nd.empty((M, N), env.ctx) for _ in range(runs + 1)]) for M, K, N in shapes]
+
+    def work(k, outs):
+        a, b, _ = state[k]
+        for c in outs:
+            op.matrix_multiply(a, False, b, False, c, env.cublas, cells[k])
+    for k in range(2):
+        work(k, state[k][2][:1])
+    op.device_synchronize()
+    threads = [threading.Thread(target=work, args=(k, state[k][2][1:])) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    op.device_synchronize()
+    for k in range(2):
+        want = state[k][2][0].asnumpy()
+        for c in state[k][2][1:]:
+            np.testing.assert_array_equal(c.asnumpy(), want)

@@ -266,29 +266,47 @@ def test_filters_packed_ahead_have_the_bits_of_filters_packed_one_by_one(lib_pat
     _same(ahead, _train(monkeypatch, False, BUILDS[name], "sgd", _overwrite_a_parameter))
 
 
-def test_an_allocation_gets_the_memory_of_recordings(lib_path, monkeypatch):
-    """What a recording keeps for its replays is given up before an allocation fails; the steps go on as ever."""
-    from tinyflow_b200 import gpu_op, ndarray
-    ctx, kept, seen = ndarray.gpu(0), [], {}
+@pytest.mark.parametrize("held_by", ["recording", "scratch"])
+def test_an_allocation_gets_the_memory_kept_for_later(lib_path, monkeypatch, held_by):
+    """Blocks of recordings and scratch of streams are given up before an allocation fails; the steps go on as ever."""
+    from tinyflow_b200 import autodiff as ad, gpu_op, ndarray
+    ctx, kept = ndarray.gpu(0), []
 
-    def between(step, model, ex, feed, x):
-        if step == 2:
-            seen["before"] = gpu_op.allocator_stats()[0]             # recorded in the fourth step
-        if step == 6 and ex._recordings.sets and not kept:
-            gpu_op.device_synchronize()
-            gpu_op.release_cached_memory()
-            seen["held"] = gpu_op.allocator_stats()[0] - seen["before"]
-            gpu_op.set_memory_limit(sum(gpu_op.allocator_stats()))
-            try:
-                kept.append(ndarray.empty((seen["held"] // 8,), ctx))
-            finally:
-                gpu_op.set_memory_limit(0)
+    class WorkOp(ad.Op):
+        name = "Work"
+
+        def __call__(self, node):
+            return self._node([node])
+
+        def compute(self, node, input_vals, output_val, cudnnHandle, cublasHandle, cudaStream, use_numpy=False):
+            work = ndarray.empty((2 << 20,), ctx)                    # 8 MB for the time of the call
+            gpu_op.array_set(work, 1.0, cudaStream)
+            gpu_op.matrix_elementwise_multiply_by_const(input_vals[0], 2.0, output_val, cudaStream)
+
+        def gradient(self, node, output_grad):
+            return [ad.mul_byconst_op(output_grad, 2.0)]
+
+        def infer_shape(self, node, input_shapes, cudnnHandle):
+            return input_shapes[0]
 
     def build(m):
-        return m.mlp(batch=512, sizes=(784, 1500, 1000, 10))         # products on the tensor path: packs of both operands
+        if held_by == "scratch":
+            return m.mlp(batch=512, sizes=(784, 1500, 1000, 10))     # products on the tensor path: packs of both operands
+        X, y_, W = ad.Placeholder("X"), ad.Placeholder("y_"), ad.Variable("W")
+        y = WorkOp()(ad.matmul_op(X, W))
+        return m.Model("work", X, y_, ad.l2loss_op(y, y_), y, {W: (20, 7)}, (33, 20), (33, 7))
+
+    def between(step, model, ex, feed, x):
+        if step == 6 and ex._recordings.sets and not kept:           # recorded in the fourth step
+            gpu_op.device_synchronize()
+            gpu_op.release_cached_memory()
+            gpu_op.set_memory_limit(sum(gpu_op.allocator_stats()))
+            try:
+                kept.append(ndarray.empty((1 << 20,), ctx))
+            finally:
+                gpu_op.set_memory_limit(0)
     got = _train(monkeypatch, True, build, "sgd", between)
-    assert seen["held"] > (1 << 20) and got[2]
-    assert isinstance(kept[0], ndarray.NDArray)                      # an int: the bytes that were short
+    assert got[2] and isinstance(kept[0], ndarray.NDArray)           # an int: the bytes that were short
     _same(got, _train(monkeypatch, False, build, "sgd"))
 
 

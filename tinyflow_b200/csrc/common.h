@@ -149,8 +149,7 @@ uint64_t recording_id();                           // of the recording this thre
 void recording_note_made(const void** source);     // the graph writes data derived from *source, kept by a plan: every replay sets *source to null,
                                                    // so that no ordinary call takes that data for what it left there itself
 uint32_t* recording_word();                        // a zeroed-per-replay device word of the graph being recorded
-void* recording_scratch(int slot, size_t bytes);   // stream_scratch() and arrival_counters() inside a recording: the graph's own
-uint32_t* recording_counters(int n);
+cudaStream_t recording_home();                     // the stream the step will be replayed on
 void* recording_take_block(size_t bytes);          // a block of exactly this (rounded) size freed earlier in the recording, or nullptr
 void recording_keep_block(void* p, size_t bytes);  // instead of handing the block back to the pool
 const uint32_t* recording_seed(unsigned seed);     // device word that will hold the seed of this dropout call at every replay
@@ -181,12 +180,24 @@ inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // Returns nullptr when the device is out of memory even after the cache was released.
 void* pool_alloc(size_t bytes);
 void pool_free(void* p);
-// Scratch of at least `bytes` for kernels on stream s, the same block at every call until a larger one is asked for; slot
-// ids are per purpose.  Kernels of one stream may share it, for they run in order; every stream, and every recorded step, has its own.
-constexpr int kScratchSlots = 4;
-void* stream_scratch(int slot, size_t bytes, cudaStream_t s);
-// n arrival counters of stream s: zero when a kernel on it starts, and the kernel leaves them zero (atomicInc wraps).
-uint32_t* arrival_counters(int n, cudaStream_t s);
+// Scratch for kernels on a stream: every stream has its own, and one operator at a time has the lease of it, from asking for a
+// block to the last launch that uses it.  A block is the same at every call until a larger one is asked for; slot ids are per
+// purpose, so that what one operator uses together does not collide.
+struct StreamScratch;
+enum { kScratchSums = 0, kScratchTiles = 1, kScratchSplit = 2, kScratchContract = 3, kScratchPackA = 4, kScratchPackB = 5, kScratchSlots = 6 };
+class StreamLease {
+ public:
+  explicit StreamLease(cudaStream_t s);
+  ~StreamLease();
+  StreamLease(const StreamLease&) = delete;
+  StreamLease& operator=(const StreamLease&) = delete;
+  void* scratch(int slot, size_t bytes);       // nullptr: out of memory
+  uint32_t* counters(int n);                   // zero when a kernel starts, and the kernel leaves them zero (atomicInc wraps)
+ private:
+  void* block(int slot, size_t bytes);
+  StreamScratch* scratch_;
+  bool locked_;
+};
 
 // ---- grid sizing: whole multiples of the SM count -----------------------------
 inline int grid_for(int64_t work_items, int block, int per_thread = 1, int waves = 8) {

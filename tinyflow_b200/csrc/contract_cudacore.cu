@@ -173,7 +173,8 @@ static int launch_contract(AV A, BV B, OV O, int64_t M, int64_t N, int64_t K, fl
   dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)splits);
   (void)out_base; (void)out_bytes;
   if (splits > 1) {
-    float* part = (float*)stream_scratch(3, sizeof(float) * (size_t)splits * (size_t)M * (size_t)N, s);
+    StreamLease lease(s);
+    float* part = (float*)lease.scratch(kScratchContract, sizeof(float) * (size_t)splits * (size_t)M * (size_t)N);
     if (!part) { splits = 1; kps = (K + BK - 1) / BK * BK; grid.z = 1; }       // no scratch: run unsplit
     else {
       launch_plain(contract_kernel<AV, BV, OV, B_KFAST, true>, grid, dim3(256), 0, s, A, B, O, M, N, K, kps, part);

@@ -228,7 +228,8 @@ int direct_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float*
   if (d.slices > 1 && floats < (size_t)d.slices * d.items * p->S) floats = (size_t)d.slices * d.items * p->S;
   if (floats * sizeof(float) > kDirectSmem) return 0;
   const int cols = d.items * p->S, grid = p->N < 2 * device_sm_count() ? p->N : 2 * device_sm_count();
-  d.part = (float*)stream_scratch(3, sizeof(float) * (size_t)grid * cols, s);
+  StreamLease lease(s);
+  d.part = (float*)lease.scratch(kScratchContract, sizeof(float) * (size_t)grid * cols);
   if (!d.part) return 0;
   note_compute_stream(s);
   KernelTimer kt("direct_conv", s, 2.0 * p->N * p->K * p->P * p->Q * p->C * p->R * p->S, 0, 1);

@@ -1752,7 +1752,7 @@ static float g_tail_cost = [] { const char* e = getenv("TINYFLOW_TAIL_COST"); re
 // the cluster (768 -> 192 channels, 17 x 17, 1x1, batch 2: 17.0 -> 15.3 us in clusters of 6).  Against it the workspace costs
 // 4 stages and 0.15 per tile (its traffic): 70 tiles of 36 stages 34.0 us split and 29.7 in clusters of 2, 40 of 72
 // stages 33.8 and 32.5 in clusters of 3, but 12 of 72 stages 19.2 and 23 in clusters of 8.
-template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, cudaStream_t s, int* oom, MaxClusters max_clusters) {
+template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, StreamLease& lease, int* oom, MaxClusters max_clusters) {
   const int sms = device_sm_count();
   const int tiles = g.m_tiles * g.n_tiles * g.tap_tiles;
   g.full_tiles = tiles; g.tail_tiles = 0; g.tail_share = 0; g.slots_per_cta = 0; g.workspace = nullptr; g.cluster = 1;
@@ -1778,7 +1778,7 @@ template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, cud
   g.slots_per_cta = (share - 1 + g.k_total - 1) / g.k_total + 1;       // tiles a range of `share` stages can touch
   const int ctas = (int)((units + share - 1) / share);
   const size_t bytes = (size_t)ctas * g.slots_per_cta * bn * BM * sizeof(float);
-  g.workspace = (float*)stream_scratch(1, bytes, s);
+  g.workspace = (float*)lease.scratch(kScratchTiles, bytes);
   if (!g.workspace) { if (oom) *oom = bytes > 0x7fffffffu ? 0x7fffffff : (int)bytes; return 1; }
   return 0;
 }
@@ -1825,7 +1825,8 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
   static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
   TF_CUDA(attr);
   TF_REQUIRE(tensor_path_error() == 0, "%s: an earlier tensor-core kernel timed out on a barrier; refusing to launch", what);
-  if (int rc = plan_schedule(p, BN, s, oom, max_clusters_of<BN, AR>)) return rc;
+  StreamLease lease(s);
+  if (int rc = plan_schedule(p, BN, lease, oom, max_clusters_of<BN, AR>)) return rc;
   static const int group_iters = getenv("TINYFLOW_GROUP_ITERS") ? atoi(getenv("TINYFLOW_GROUP_ITERS")) : 0;
   p.group_iters = group_iters > 0 ? group_iters : (p.data_by_data ? kGroupItersDataByData : (AR == kArithTF32 ? kGroupItersTF32 : kGroupIters));
   // cross terms promoted every 64 stages: 256 accumulations into a sum 2^-12 of the whole truncate less than 2^-28 of it
@@ -1919,7 +1920,6 @@ struct Pack {           // a packed operand living in pooled device memory
   uint32_t* words = nullptr;       // device: amax[0], amax[1] (alternating between uses), scale (float), spare
   unsigned uses = 0;
   int arith = kArithF16;           // element type of hi / lo
-  bool transient = false;          // belongs to one call (matrix products)
   long long rows = 0, cols = 0, pitch = 0;
   const void* src = nullptr; uint64_t version = 0; int tag = 0;   // cache key
   uint64_t recording = 0;          // the recording whose graph fills the pack, 0: an ordinary call did
@@ -1927,11 +1927,22 @@ struct Pack {           // a packed operand living in pooled device memory
   size_t bytes() const { return (size_t)rows * pitch * elem_of(arith); }
   const float* scale() const { return reinterpret_cast<const float*>(words + 2); }
 };
-static int pack_alloc(Pack& pk, int ar, long long rows, long long cols, cudaStream_t s, int* oom) {
-  long long pitch = round_up(cols, 64);
-  if (!pk.words && t_recording && pk.transient) {
-    for (int i = 0; i < 4; ++i) { uint32_t* w = recording_word(); if (!i) pk.words = w; }       // consecutive, cleared at every replay
+// A pack for one call, in the stream's scratch: hi, lo and (outside a recording, whose words are cleared at every replay) the words.
+static int pack_in_scratch(Pack& pk, StreamLease& lease, int slot, int ar, long long rows, long long cols, cudaStream_t s, int* oom) {
+  pk.rows = rows; pk.cols = cols; pk.pitch = round_up(cols, 64); pk.arith = ar;
+  char* const base = (char*)lease.scratch(slot, 2 * pk.bytes() + 16);          // bytes() is a multiple of 128
+  if (!base) { if (oom) *oom = pk.bytes() > 0x3ffffff0u ? 0x7fffffff : (int)(2 * pk.bytes() + 16); return 1; }
+  pk.hi = base; pk.lo = base + pk.bytes();
+  if (t_recording) {
+    for (int i = 0; i < 4; ++i) { uint32_t* w = recording_word(); if (!i) pk.words = w; }       // consecutive
+    return 0;
   }
+  pk.words = (uint32_t*)(base + 2 * pk.bytes());
+  TF_CUDA(cudaMemsetAsync(pk.words, 0, 16, s));
+  return 0;
+}
+static int pack_alloc(Pack& pk, int ar, long long rows, long long cols, cudaStream_t s, int* oom) {
+  const long long pitch = round_up(cols, 64);
   if (!pk.words) {
     if (t_recording) TF_FAIL("a packed operand of a recorded step has never been packed before");    // its words could not be cleared now
     pk.words = (uint32_t*)pool_alloc(16);
@@ -1953,7 +1964,7 @@ static int pack_alloc(Pack& pk, int ar, long long rows, long long cols, cudaStre
 }
 static void pack_release(Pack& pk) {
   if (pk.hi) { pool_free(pk.hi); pool_free(pk.lo); pk.hi = pk.lo = nullptr; }
-  if (pk.words && !(t_recording && pk.transient)) pool_free(pk.words);
+  if (pk.words) pool_free(pk.words);
   pk.words = nullptr;
 }
 // Starts one use of the pack: reduces max|src| over n contiguous floats into this use's amax word and returns the
@@ -2013,11 +2024,12 @@ int tc_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_
   const int ar = tensor_arithmetic(), bk = bk_of(ar);
   // A is stored [M][K] (K-major) or, transposed, [K][M] (M-major); B is stored [K][N] (N-major) or [N][K] (K-major)
   Pack pa, pb;
-  pa.transient = pb.transient = true;
+  StreamLease lease(s);
   long long a_rows = tA ? K : M, a_cols = tA ? M : K, b_rows = tB ? N : K, b_cols = tB ? K : N;
-  if (pack_alloc(pa, ar, a_rows, a_cols, s, oom)) { pack_release(pa); return 0; }
-  if (pack_alloc(pb, ar, b_rows, b_cols, s, oom)) { pack_release(pa); pack_release(pb); return 0; }
-  int rc = run_pack_matrix(A, a_cols, pa, s);
+  int rc = pack_in_scratch(pa, lease, kScratchPackA, ar, a_rows, a_cols, s, oom);
+  if (!rc) rc = pack_in_scratch(pb, lease, kScratchPackB, ar, b_rows, b_cols, s, oom);
+  if (rc) return rc < 0 ? -1 : 0;
+  rc = run_pack_matrix(A, a_cols, pa, s);
   if (!rc) rc = run_pack_matrix(B, b_cols, pb, s);
   GemmParams p;
   memset(&p, 0, sizeof(p));
@@ -2036,7 +2048,6 @@ int tc_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_
     p.a_scale = pa.scale(); p.b_scale = pb.scale();
     rc = launch_gemm_bn(bn, ar, p, s, 2.0 * M * N * K, "DLGpuMatrixMultiply", oom);
   }
-  pack_release(pa); pack_release(pb);       // stream order keeps the blocks valid until the kernel is done
   return rc < 0 ? -1 : (rc > 0 ? 0 : 1);    // a missing workspace sends the call to the CUDA-core kernel
 }
 

@@ -793,10 +793,11 @@ int DLGpuBroadcastTo1(const DLArrayHandle input, DLArrayHandle output, void** cu
 
 static int reduce_to_scalar(const float* in, float* out, int64_t n, float scale, cudaStream_t s, const char* what) {
   int blocks = grid_for(n, kBlock, 8, 4);
-  float* part = (float*)stream_scratch(0, sizeof(float) * 4096, s);
+  StreamLease lease(s);
+  float* part = (float*)lease.scratch(kScratchSums, sizeof(float) * 4096);
   TF_REQUIRE(part, "%s: scratch allocation failed", what);
   if (blocks > 4096) blocks = 4096;
-  uint32_t* counter = arrival_counters(1, s);
+  uint32_t* counter = lease.counters(1);
   TF_REQUIRE(counter, "%s: scratch allocation failed", what);
   note_compute_stream(s);
   launch_dep(sum_kernel, dim3(blocks), dim3(kBlock), 0, s, in, out, part, n, scale, counter);
@@ -813,11 +814,12 @@ static int channel_sums(const float* in, float* out, int64_t N, int64_t C, int64
   splits = std::max<int64_t>(splits, 1);
   const int64_t nps = std::max<int64_t>(1, (N + splits - 1) / splits);
   splits = std::max<int64_t>(1, (N + nps - 1) / nps);
+  StreamLease lease(s);
   float* part = nullptr;
   uint32_t* counters = nullptr;
   if (splits > 1) {
-    part = (float*)stream_scratch(2, sizeof(float) * (size_t)splits * (size_t)C, s);
-    counters = arrival_counters((int)C, s);
+    part = (float*)lease.scratch(kScratchSplit, sizeof(float) * (size_t)splits * (size_t)C);
+    counters = lease.counters((int)C);
     TF_REQUIRE(part && counters, "%s: scratch allocation failed", what);
   }
   const int vec = L % 4 == 0 && aligned16(in) && nps * (L / 4) < (1ll << 31);
@@ -838,11 +840,12 @@ static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, 
   }
   int64_t rps = (rows + splits - 1) / splits;
   splits = (int)((rows + rps - 1) / rps);
+  StreamLease lease(s);
   float* part = nullptr;
   uint32_t* counters = nullptr;
   if (splits > 1) {
-    part = (float*)stream_scratch(2, sizeof(float) * (size_t)splits * (size_t)cols, s);
-    counters = arrival_counters(gx, s);
+    part = (float*)lease.scratch(kScratchSplit, sizeof(float) * (size_t)splits * (size_t)cols);
+    counters = lease.counters(gx);
     if (!part || !counters) { splits = 1; rps = rows; }                                  // no scratch: one split
   }
   note_compute_stream(s);
@@ -1121,8 +1124,9 @@ int DLGpuSoftmaxCrossEntropy(const DLArrayHandle input_a, const DLArrayHandle in
   note_compute_stream(s);
   const int64_t rows = input_a->shape[0];
   const int blocks = (int)std::min<int64_t>(std::max<int64_t>(1, (rows + kBlock / 32 - 1) / (kBlock / 32)), 2 * device_sm_count());
-  float* part = (float*)stream_scratch(0, sizeof(float) * 4096, s);
-  uint32_t* counter = arrival_counters(1, s);
+  StreamLease lease(s);
+  float* part = (float*)lease.scratch(kScratchSums, sizeof(float) * 4096);
+  uint32_t* counter = lease.counters(1);
   TF_REQUIRE(part && counter, "DLGpuSoftmaxCrossEntropy: scratch allocation failed");
   launch_dep(softmax_xent_kernel, dim3(blocks), dim3(kBlock), 0, s, F(input_a), F(input_b), FM(output), part, rows, input_a->shape[1], counter);
   TF_AFTER(s, "DLGpuSoftmaxCrossEntropy");

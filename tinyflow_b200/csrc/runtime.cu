@@ -202,6 +202,7 @@ void flush_deferred_slow() {
 // can run ahead of, and overlap with, the compute queued in front of its consumer.
 // ---------------------------------------------------------------------------------
 static std::atomic<bool> g_side_copies_seen{false};
+static bool scratch_gives_up_memory();
 static std::atomic<long long> g_memory_limit{0};          // device bytes a pool may own, 0: what the device has
 struct Pool {
   std::mutex mu;
@@ -244,7 +245,7 @@ struct Pool {
   void* alloc(size_t bytes, bool* hard = nullptr, bool unused = false) {
     if (hard) *hard = false;
     size_t b = round(bytes);
-    if (t_recording && !host) if (void* p = recording_take_block(b)) return p;      // still counted as in use
+    if (t_recording && !host && !unused) if (void* p = recording_take_block(b)) return p;      // still counted as in use
     std::unique_lock<std::mutex> lk(mu);
     auto it = free_by_size.find(b);
     if (!unused && it != free_by_size.end() && !it->second.empty()) {
@@ -269,10 +270,10 @@ struct Pool {
       release_cached_locked();
       e = raw_alloc(&p, b);
       if (e != cudaSuccess && !host) {
-        // Then what recorded steps keep for their replays: they can be recorded again, or run as ordinary calls.
+        // Then what recorded steps keep for their replays (they can be recorded again, or run as ordinary calls), and scratch.
         cudaGetLastError();
         lk.unlock();
-        const bool some = recordings_give_up_memory();
+        const bool recordings = recordings_give_up_memory(), some = scratch_gives_up_memory() || recordings;
         lk.lock();
         if (some) { release_cached_locked(); e = raw_alloc(&p, b); }
       }
@@ -340,44 +341,60 @@ void pool_free(void* p) {
   }
 }
 
-// Scratch per (device, stream): the kernels of one stream run one after the other, so they can share a block; those of two
-// streams (two executors, two threads) cannot.  An outgrown block stays until its stream is destroyed, because another thread may
-// be about to launch a kernel on it; with a growth of at least 1.5x all of a stream's blocks of a slot are below three times the last.
+// Scratch per (device, stream).  A recorded step uses the blocks of the stream it is replayed on: the replays and the ordinary
+// calls of that stream run one after the other, and a recording keeps no scratch of its own.  (When it did, whatever came after a
+// recording had to allocate anew, and a cudaMalloc beside a busy GPU took 10-67 ms on some hosts: twenty steps of ResNet-50 with
+// one recording among them at half their rate.)  An outgrown block stays, because recordings name it, until the device is full
+// or the stream is destroyed; both make recordings out of date.
 constexpr int kCounterSlot = kScratchSlots;           // arrival counters, kept zero between kernels
-struct StreamScratch { void* ptr[kScratchSlots + 1] = {nullptr}; size_t cap[kScratchSlots + 1] = {0}; std::vector<void*> outgrown; };
-static std::mutex g_scratch_mu;
+struct StreamScratch {
+  std::recursive_mutex mu;                            // the lease
+  int depth = 0;
+  void* ptr[kScratchSlots + 1] = {nullptr};
+  size_t cap[kScratchSlots + 1] = {0};
+  std::vector<void*> outgrown;
+  void take_all(std::vector<void*>& blocks) {
+    for (int k = 0; k <= kScratchSlots; ++k) { if (ptr[k]) blocks.push_back(ptr[k]); ptr[k] = nullptr; cap[k] = 0; }
+    blocks.insert(blocks.end(), outgrown.begin(), outgrown.end());
+    outgrown.clear();
+  }
+};
+static std::mutex g_scratch_mu;                       // the table and the fields; never held while a lease is waited for
 static std::map<std::pair<int, std::pair<cudaStream_t, size_t>>, StreamScratch> g_scratch;
 static std::pair<int, std::pair<cudaStream_t, size_t>> scratch_key(cudaStream_t s) {        // a per-thread stream is another one in every thread
   return {current_device(), {s, s == cudaStreamPerThread ? std::hash<std::thread::id>()(std::this_thread::get_id()) : 0}};
 }
-static void* scratch_block(int slot, size_t bytes, cudaStream_t s) {
-  const auto key = scratch_key(s);
+StreamLease::StreamLease(cudaStream_t s) : locked_(!t_recording) {
+  const auto key = scratch_key(t_recording ? recording_home() : s);
+  {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    scratch_ = &g_scratch[key];
+  }
+  if (locked_) { scratch_->mu.lock(); ++scratch_->depth; }         // nothing of a recording runs: it disturbs nobody
+}
+StreamLease::~StreamLease() { if (locked_) { --scratch_->depth; scratch_->mu.unlock(); } }
+void* StreamLease::block(int slot, size_t bytes) {
   std::unique_lock<std::mutex> lk(g_scratch_mu);
-  StreamScratch* sc = &g_scratch[key];
-  if (sc->cap[slot] >= bytes) return sc->ptr[slot];
-  const size_t want = std::max(bytes + bytes / 4, sc->cap[slot] + sc->cap[slot] / 2), got = Pool::round(want);
+  if (scratch_->cap[slot] >= bytes) return scratch_->ptr[slot];
+  // a quarter more than asked for, so that slowly growing requests do not allocate each time; large blocks as they are
+  const size_t want = bytes < (size_t(32) << 20) ? bytes + bytes / 4 : bytes, got = Pool::round(want);
   lk.unlock();
   void* p = device_pool().alloc(want, nullptr, true);
   if (p && slot == kCounterSlot && clear_now(p, got) != cudaSuccess) { pool_free(p); p = nullptr; }
   if (!p) return nullptr;
   lk.lock();
-  sc = &g_scratch[key];
-  if (sc->cap[slot] >= got) {              // another thread of this stream was faster
-    sc->outgrown.push_back(p);
-    return sc->ptr[slot];
+  if (scratch_->cap[slot] >= got) {                   // a recording in another thread was faster
+    scratch_->outgrown.push_back(p);
+    return scratch_->ptr[slot];
   }
-  if (sc->ptr[slot]) sc->outgrown.push_back(sc->ptr[slot]);
-  sc->ptr[slot] = p;
-  sc->cap[slot] = got;
+  if (scratch_->ptr[slot]) scratch_->outgrown.push_back(scratch_->ptr[slot]);
+  scratch_->ptr[slot] = p;
+  scratch_->cap[slot] = got;
   return p;
 }
-void* stream_scratch(int slot, size_t bytes, cudaStream_t s) {
-  if (slot < 0 || slot >= kScratchSlots) return nullptr;
-  return t_recording ? recording_scratch(slot, bytes) : scratch_block(slot, bytes, s);
-}
-uint32_t* arrival_counters(int n, cudaStream_t s) {
-  return t_recording ? recording_counters(n) : (uint32_t*)scratch_block(kCounterSlot, sizeof(uint32_t) * (size_t)n, s);
-}
+void* StreamLease::scratch(int slot, size_t bytes) { return slot < 0 || slot >= kScratchSlots ? nullptr : block(slot, bytes); }
+uint32_t* StreamLease::counters(int n) { return (uint32_t*)block(kCounterSlot, sizeof(uint32_t) * (size_t)n); }
+
 // The stream is idle and about to be destroyed.
 static void release_stream_scratch(cudaStream_t s) {
   std::vector<void*> blocks;
@@ -385,11 +402,36 @@ static void release_stream_scratch(cudaStream_t s) {
     std::lock_guard<std::mutex> lk(g_scratch_mu);
     auto it = g_scratch.find(scratch_key(s));
     if (it == g_scratch.end()) return;
-    blocks = std::move(it->second.outgrown);
-    for (void* p : it->second.ptr) if (p) blocks.push_back(p);
+    it->second.take_all(blocks);
     g_scratch.erase(it);
   }
+  if (blocks.empty()) return;
+  bump_layout_epoch();
   for (void* p : blocks) pool_free(p);
+}
+// The device is full: the scratch of every stream on which no call is being issued goes back to the pool.
+static bool scratch_gives_up_memory() {
+  if (t_recording) return false;
+  std::vector<StreamScratch*> idle;
+  std::vector<void*> blocks;
+  {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    for (auto& kv : g_scratch) {
+      if (!kv.second.mu.try_lock()) continue;
+      if (kv.second.depth == 0) idle.push_back(&kv.second);
+      else kv.second.mu.unlock();                     // this thread's own call
+    }
+  }
+  bump_layout_epoch();
+  if (cudaDeviceSynchronize() == cudaSuccess) {
+    std::lock_guard<std::mutex> lk(g_scratch_mu);
+    for (StreamScratch* sc : idle) sc->take_all(blocks);
+  } else {
+    cudaGetLastError();
+  }
+  for (void* p : blocks) pool_free(p);
+  for (StreamScratch* sc : idle) sc->mu.unlock();
+  return !blocks.empty();
 }
 
 static inline size_t data_bytes(const DLArray* a) { return (size_t)numel(a) * 4; }

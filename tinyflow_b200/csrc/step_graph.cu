@@ -24,7 +24,7 @@ int tensor_path_error();
 void tc_recording_begins();
 bool dp_active();
 
-constexpr int kZeroedWords = 16384;       // maxima of a step's tensors, one word per tracked write (Inception-v4: about 900), and arrival counters
+constexpr int kZeroedWords = 12288;       // maxima of a step's tensors: one word per tracked write (Inception-v4: about 900)
 constexpr int kSeedWords = 1022;          // dropout calls of a step
 constexpr int kCarries = 1024;            // parameters whose maximum crosses steps
 
@@ -47,9 +47,7 @@ struct StepGraph {
   long long launches = 0;
   uint64_t epoch = 0;
   uint64_t id = 0;
-  struct { void* ptr = nullptr; size_t cap = 0; } scratch[kScratchSlots];
-  uint32_t* counters = nullptr;
-  int n_counters = 0;
+  cudaStream_t home = nullptr;            // where it is replayed, and whose scratch its kernels use
 };
 static std::atomic<uint64_t> g_recordings{0};
 uint64_t recording_id() { return t_recording ? t_recording->id : 0; }
@@ -68,25 +66,6 @@ void* recording_take_block(size_t bytes) {
   return p;
 }
 void recording_keep_block(void* p, size_t bytes) { t_recording->free_blocks[bytes].push_back(p); }
-// An outgrown block goes to the recording's own free blocks: its kernels run in front of those of whoever takes it next.
-void* recording_scratch(int slot, size_t bytes) {
-  auto& sc = t_recording->scratch[slot];
-  if (sc.cap >= bytes) return sc.ptr;
-  if (sc.ptr) pool_free(sc.ptr);
-  sc.ptr = pool_alloc(bytes);
-  sc.cap = sc.ptr ? bytes : 0;
-  return sc.ptr;
-}
-uint32_t* recording_counters(int n) {
-  StepGraph* g = t_recording;
-  if (n > g->n_counters) {
-    int m = 64;
-    while (m < n) m *= 2;
-    if (g->used + m > kZeroedWords) return nullptr;
-    g->counters = g->words + g->used; g->n_counters = m; g->used += m;
-  }
-  return g->counters;
-}
 const uint32_t* recording_seed(unsigned seed) {
   StepGraph* g = t_recording;
   if ((int)g->seeds.size() >= kSeedWords) { recording_refuse("more dropout calls than a recording has seeds for"); return g->words; }
@@ -102,6 +81,7 @@ const float* recording_adam_corrections(float c1, float c2) {
 void recording_note_launches(int n) { t_recording->launches += n; }
 void recording_note_write(const void* p) { t_recording->written.push_back(p); }
 void recording_note_made(const void** source) { t_recording->made.push_back(source); }
+cudaStream_t recording_home() { return t_recording->home; }
 cudaStream_t recording_stream() { return t_recording->stream; }
 
 // ---- nodes --------------------------------------------------------------------------------------
@@ -221,9 +201,9 @@ using namespace tf;
 extern "C" {
 
 // Starts recording the calls this thread makes from now on; *graph receives the recording and *stream_cell the stream the
-// calls have to be given.  0 = recording, 1 = not possible now (timing on, data-parallel exchange active), -1 = error.
-int TfStepRecordBegin(void** graph, void** stream_cell) {
-  TF_REQUIRE(graph && stream_cell && !t_recording, "TfStepRecordBegin: bad arguments, or this thread is recording already");
+// calls have to be given; the step will be replayed on *replay_stream.  0 = recording, 1 = not possible now (timing on, data-parallel exchange active), -1 = error.
+int TfStepRecordBegin(void** graph, void** stream_cell, void** replay_stream) {
+  TF_REQUIRE(graph && stream_cell && replay_stream && !t_recording, "TfStepRecordBegin: bad arguments, or this thread is recording already");
   flush_deferred();
   if (g_timing_level > 0 || g_sync_every_op || dp_active() || tensor_path_error() != 0) return 1;
   StepGraph* g = new StepGraph;
@@ -234,6 +214,7 @@ int TfStepRecordBegin(void** graph, void** stream_cell) {
     step_graph_free(g);
     TF_FAIL("TfStepRecordBegin: no stream or graph could be created");
   }
+  g->home = *(cudaStream_t*)replay_stream;
   g->epoch = g_layout_epoch.load();
   g->id = g_recordings.fetch_add(1) + 1;
   t_recording = g;
@@ -250,7 +231,6 @@ int TfStepRecordEnd(void** graph, int keep) {
   TF_REQUIRE(graph && *graph && t_recording == (StepGraph*)*graph, "TfStepRecordEnd: this thread is not recording that step");
   StepGraph* g = t_recording;
   flush_deferred();
-  for (auto& sc : g->scratch) if (sc.ptr) pool_free(sc.ptr);       // to the graph's own blocks, as all frees of a recording
   bool ok = keep != 0 && !g->refused;
   if (ok) {
     g->carries.resize(kCarries);
@@ -296,6 +276,7 @@ int TfStepReplay(void* graph, const unsigned* seeds, int nseeds, float b1t, floa
   StepGraph* g = (StepGraph*)graph;
   TF_REQUIRE(g && !t_recording, "TfStepReplay: nothing to replay");
   flush_deferred();
+  StreamLease lease(g->home);            // no operator of another thread between its launches
   std::lock_guard<std::mutex> lk(g_graphs_mu);
   if (!g->exec) return 1;                // gave up its memory
   if (g->epoch != g_layout_epoch.load()) return 1;
@@ -303,6 +284,7 @@ int TfStepReplay(void* graph, const unsigned* seeds, int nseeds, float b1t, floa
   TF_REQUIRE(tensor_path_error() == 0, "TfStepReplay: an earlier tensor-core kernel timed out on a barrier; refusing to launch");
   TF_REQUIRE(nseeds == (int)g->seeds.size(), "TfStepReplay: %d seeds for %d dropout calls", nseeds, (int)g->seeds.size());
   cudaStream_t s = stream_of(cudaStream);
+  TF_REQUIRE(s == g->home, "TfStepReplay: not the stream the step was recorded for");
   note_compute_stream(s);
   // maxima that no replay of this step left behind: the tensor was written by something else since
   for (const AmaxCarry& c : g->carries) {

@@ -8,9 +8,9 @@ What is replayed is keyed by identity.  Parameters and moments (updated in place
 second one below it.  A caller that brings new mini-batch arrays every step, or feeds several in turn, gets a *staged*
 recording, whose inputs are copied into arrays of the executor's own first.  Entries disappear with the arrays they name.
 
-A recording is paid for once, a staged input at every step.  ResNet-50 at batch 64: 5-16 ms of host time for the recording
-(calls 2-6, end of capture and instantiation 1.4-14), 15 us a step for the copies.  So arrays that come in turn get
-recordings of their own only after RUNS_WITHOUT_STAGING steps, when the copies have cost about as much.
+A recording is paid for once, a staged input at every step.  ResNet-50 at batch 64: 5 ms of host time for the recording
+(2.5-3.5 for the calls, the rest to instantiate the graph and to upload it), 15 us a step for the copies.  So arrays that come
+in turn get recordings of their own only after RUNS_WITHOUT_STAGING steps, when the copies have cost about as much.
 """
 from __future__ import annotations
 
@@ -118,7 +118,7 @@ def record(executor, feed_dict, staged):
     """Records one step of ``executor`` on ``feed_dict`` (nothing is executed).  None if that is not possible just now
     (kernel timing, data-parallel exchange), RuntimeError with the reason if the step cannot be recorded."""
     graph, stream = ctypes.c_void_p(), new_cell(2)
-    rc = _LIB.TfStepRecordBegin(ctypes.byref(graph), stream)
+    rc = _LIB.TfStepRecordBegin(ctypes.byref(graph), stream, executor.cudaStream)
     if rc != 0:
         if rc < 0:
             raise RuntimeError(last_error())
