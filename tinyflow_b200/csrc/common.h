@@ -138,7 +138,8 @@ int contraction_path();
 // While a step is recorded, its calls (of ONE thread) name a private stream; nothing executes, but every launch, fill and copy
 // adds a node to a CUDA graph that later replays the step with one host call.  What a call would keep on the
 // host from one step to the next has to be fixed for the graph instead:
-//  * scratch blocks freed during the recording stay with the graph (its kernels use their addresses at every replay);
+//  * arrays freed during the recording stay with the graph (its kernels use their addresses at every replay); scratch is that
+//    of the stream it is replayed on;
 //  * a tracked maximum gets a device word of the graph's own, cleared at the start of every replay, in place of the pair
 //    of words that alternates between calls; the maxima of tensors that a step reads before it writes them (parameters)
 //    are carried to the next replay in a word per tensor;

@@ -201,7 +201,8 @@ using namespace tf;
 extern "C" {
 
 // Starts recording the calls this thread makes from now on; *graph receives the recording and *stream_cell the stream the
-// calls have to be given; the step will be replayed on *replay_stream.  0 = recording, 1 = not possible now (timing on, data-parallel exchange active), -1 = error.
+// calls have to be given; the step will be replayed on *replay_stream.  0 = recording, 1 = not possible now (timing on,
+// data-parallel exchange active), -1 = error.
 int TfStepRecordBegin(void** graph, void** stream_cell, void** replay_stream) {
   TF_REQUIRE(graph && stream_cell && replay_stream && !t_recording, "TfStepRecordBegin: bad arguments, or this thread is recording already");
   flush_deferred();
