@@ -146,6 +146,12 @@ def test_split_reductions_in_a_capture_of_the_callers_own(env):
     cell = ctypes.pointer(ctypes.c_void_p(side.cuda_stream))
     with torch.cuda.graph(graph, stream=side):
         work(got, cell)
+    op.release_cached_memory()
+    op.set_memory_limit(sum(op.allocator_stats()))       # a full device: scratch is given up, but not what the graph names
+    try:
+        assert isinstance(nd.empty((1 << 28,), env.ctx), int)
+    finally:
+        op.set_memory_limit(0)
     for _ in range(3):
         for v in got:
             v[:] = np.zeros(v.shape, np.float32)

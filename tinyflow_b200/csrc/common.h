@@ -197,6 +197,7 @@ class StreamLease {
  private:
   void* block(int slot, size_t bytes);
   StreamScratch* scratch_;
+  cudaStream_t stream_;
   bool locked_;
 };
 

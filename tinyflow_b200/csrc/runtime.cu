@@ -353,7 +353,9 @@ struct StreamScratch {
   void* ptr[kScratchSlots + 1] = {nullptr};
   size_t cap[kScratchSlots + 1] = {0};
   std::vector<void*> outgrown;
+  bool captured = false;                              // a graph that the caller captured names some of the blocks: they stay for good
   void take_all(std::vector<void*>& blocks) {
+    if (captured) return;
     for (int k = 0; k <= kScratchSlots; ++k) { if (ptr[k]) blocks.push_back(ptr[k]); ptr[k] = nullptr; cap[k] = 0; }
     blocks.insert(blocks.end(), outgrown.begin(), outgrown.end());
     outgrown.clear();
@@ -364,7 +366,7 @@ static std::map<std::pair<int, std::pair<cudaStream_t, size_t>>, StreamScratch> 
 static std::pair<int, std::pair<cudaStream_t, size_t>> scratch_key(cudaStream_t s) {        // a per-thread stream is another one in every thread
   return {current_device(), {s, s == cudaStreamPerThread ? std::hash<std::thread::id>()(std::this_thread::get_id()) : 0}};
 }
-StreamLease::StreamLease(cudaStream_t s) : locked_(!t_recording) {
+StreamLease::StreamLease(cudaStream_t s) : stream_(s), locked_(!t_recording) {
   const auto key = scratch_key(t_recording ? recording_home() : s);
   {
     std::lock_guard<std::mutex> lk(g_scratch_mu);
@@ -374,7 +376,10 @@ StreamLease::StreamLease(cudaStream_t s) : locked_(!t_recording) {
 }
 StreamLease::~StreamLease() { if (locked_) { --scratch_->depth; scratch_->mu.unlock(); } }
 void* StreamLease::block(int slot, size_t bytes) {
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (!t_recording && cudaStreamIsCapturing(stream_, &capture) != cudaSuccess) { cudaGetLastError(); capture = cudaStreamCaptureStatusNone; }
   std::unique_lock<std::mutex> lk(g_scratch_mu);
+  if (capture != cudaStreamCaptureStatusNone) scratch_->captured = true;
   if (scratch_->cap[slot] >= bytes) return scratch_->ptr[slot];
   // a quarter more than asked for, so that slowly growing requests do not allocate each time; large blocks as they are
   const size_t want = bytes < (size_t(32) << 20) ? bytes + bytes / 4 : bytes, got = Pool::round(want);
@@ -403,7 +408,7 @@ static void release_stream_scratch(cudaStream_t s) {
     auto it = g_scratch.find(scratch_key(s));
     if (it == g_scratch.end()) return;
     it->second.take_all(blocks);
-    g_scratch.erase(it);
+    g_scratch.erase(it);                              // what a captured graph names is left to it
   }
   if (blocks.empty()) return;
   bump_layout_epoch();
