@@ -50,7 +50,8 @@ def test_a_dropped_recording_goes_at_once(drop):
     table, w, x = step_graph.Recordings(), _Node(1), _Node(2)
     weights, batch = _Array(), _Array()
     entry, _, _ = table.choose({w: weights, x: batch})
-    recording = entry.recording = _Array()
+    recording = _Array()
+    table.keep(entry, recording)
     gone = weakref.ref(recording)
     del entry, recording
     gc.collect()
@@ -65,7 +66,9 @@ def test_a_dropped_recording_goes_at_once(drop):
         else:
             kept = [_Array() for _ in range(step_graph.MAX_FEEDS)]
             for other in kept:
-                table.choose({w: other, x: batch})
+                assert gone() is not None
+                entry = table.choose({w: other, x: batch})[0]
+                table.keep(entry, _Array())
         assert gone() is None
     finally:
         gc.enable()

@@ -489,7 +489,7 @@ class Executor(object):
             recording = self._record(feed_dict, staged)
             if recording is None:
                 return None
-            entry.recording = recording
+            self._recordings.keep(entry, recording)
         self._feed = dict(feed_dict)
         if staged:
             for node, array in recording.staged:

@@ -26,6 +26,7 @@ RUNS_BEFORE_RECORDING = 2        # of the same arrays: the first calls of a plan
 RUNS_BEFORE_STAGING = 4          # of the same parameters with ever changing mini-batches
 RUNS_WITHOUT_STAGING = 512       # of the same arrays, others in between
 MAX_FEEDS = 4                    # parameter sets, and mini-batches per set, that keep a recording
+MAX_KNOWN = 16                   # that are counted
 
 
 class Recording(object):
@@ -85,7 +86,7 @@ class Recordings(object):
             # (bound here: at interpreter exit the module's names go before the arrays do)
             gone = lambda _ref, t=weakref.ref(table), e=weakref.ref(entry), k=key, forget=_forget: forget(t(), k, e())     # noqa: E731
             entry.refs = [weakref.ref(a, gone) for a in arrays]
-            while len(table) >= MAX_FEEDS:
+            while len(table) >= MAX_KNOWN:
                 del table[next(iter(table))]
         table[key] = entry                      # most recently used last
         return entry
@@ -107,6 +108,20 @@ class Recordings(object):
         below.runs += 1
         below.in_a_row += 1
         return top if staged else below, staged, wanted
+
+    def keep(self, entry, recording):
+        """Attaches a recording to its entry.  The oldest ones beyond MAX_FEEDS go now, beside the cost of making one (dropping
+        one takes 100-700 us), and not in front of the first step on new arrays."""
+        entry.recording = recording
+        for top in self.sets.values():
+            self._trim(top.batches, lambda e: e.recording)
+        self._trim(self.sets, lambda e: e.recording or any(b.recording for b in e.batches.values()))
+
+    @staticmethod
+    def _trim(table, recorded):
+        keys = [k for k, e in table.items() if recorded(e)]
+        for k in keys[:max(0, len(keys) - MAX_FEEDS)]:
+            del table[k]
 
 
 def _forget(table, key, entry):
