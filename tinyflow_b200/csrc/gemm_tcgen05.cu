@@ -1247,20 +1247,24 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_pair_kernel(const __grid_c
 }
 
 // Adds up the pieces of every split tile (the tail of the schedule) in a fixed order and writes the result where the
-// GEMM's own epilogue would have.  grid (tail_tiles, BN / kReduceCols), block (128 rows, kReduceWays): the pieces of a
-// tile are dealt round robin to the kReduceWays row groups, each adds its share in piece order, and the subtotals are
-// added in row-group order - the same order every run, so the result is bit-reproducible.
-constexpr int kReduceCols = 8, kReduceWays = 4;
-template <int BN>
-__global__ void __launch_bounds__(BM * kReduceWays) reduce_partials_kernel(const __grid_constant__ GemmParams p) {
-  __shared__ float part[kReduceWays][kReduceCols][BM];
+// GEMM's own epilogue would have.  grid (tail_tiles, BN / kReduceCols, BM / ROWS), block (ROWS, WAYS), 512 threads: the pieces of a
+// tile are dealt round robin to the WAYS row groups, each adds its share in piece order, and the subtotals are
+// added in row-group order - the same order every run, so the result is bit-reproducible.  Bound by latency: one memory round trip
+// per four pieces of a row group.  16 row groups of 32 rows where a launch has few tiles of many pieces (the filter gradients of
+// ResNet-50 at batch 19: step 4434 -> 4383 us, DenseNet-121: 14755 -> 14622); elsewhere 4 of 128, since there the blocks'
+// starts are what counts (16 everywhere: Inception-v4 20750 -> 23020 us).
+constexpr int kReduceCols = 8, kReduceThreads = 512;
+template <int BN, int WAYS>
+__global__ void __launch_bounds__(kReduceThreads) reduce_partials_kernel(const __grid_constant__ GemmParams p) {
+  constexpr int kReduceWays = WAYS, kReduceRows = kReduceThreads / WAYS;
+  __shared__ float part[kReduceWays][kReduceCols][kReduceRows];
   __shared__ uint32_t block_top;
   if (threadIdx.x == 0 && threadIdx.y == 0) block_top = 0u;
   grid_dep_sync();
   const int t = blockIdx.x;                            // tail tile
   int mt, nt, tap;
   decode_tile(p, p.full_tiles + t, mt, nt, tap);
-  const int row = threadIdx.x, way = threadIdx.y;
+  const int lane = threadIdx.x, way = threadIdx.y, row = blockIdx.z * kReduceRows + lane;
   // CTA g of the GEMM covered stages [g * share, (g + 1) * share) of the tail; its first piece belongs to tail tile
   // (g * share) / k_total and its pieces sit in consecutive workspace slots
   const int g_first = (int)(((long long)t * p.k_total) / p.tail_share);
@@ -1290,28 +1294,28 @@ __global__ void __launch_bounds__(BM * kReduceWays) reduce_partials_kernel(const
     for (int q = 0; q < kReduceCols; ++q) sum[q] += __ldcg(ws + (size_t)q * BM);
   }
 #pragma unroll
-  for (int q = 0; q < kReduceCols; ++q) part[way][q][row] = sum[q];
+  for (int q = 0; q < kReduceCols; ++q) part[way][q][lane] = sum[q];
   __syncthreads();
-  // every row group finishes a quarter of the block's columns: subtotals added in row-group order
-  const RowAddr ra = row_address(p, mt, tap, row);
-  const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));
+  // the row groups share the columns: subtotals added in row-group order
   uint32_t top = 0;
-  constexpr int kPer = kReduceCols / kReduceWays;
+  if (way < kReduceCols) {
+    const RowAddr ra = row_address(p, mt, tap, row);
+    const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));
 #pragma unroll
-  for (int j = 0; j < kPer; ++j) {
-    const int q = way * kPer + j;
-    float v = part[0][q][row];
+    for (int q = way; q < kReduceCols; q += kReduceWays) {
+      float v = part[0][q][lane];
 #pragma unroll
-    for (int w2 = 1; w2 < kReduceWays; ++w2) v += part[w2][q][row];
-    const int n = nt * BN + c_begin + q;
-    if (ra.ok && n < p.N) {
-      p.out[ra.base + (long long)n * ra.col_stride] = v * inv_scale;
-      top = max(top, amax_bits(v * inv_scale));
+      for (int w2 = 1; w2 < kReduceWays; ++w2) v += part[w2][q][lane];
+      const int n = nt * BN + c_begin + q;
+      if (ra.ok && n < p.N) {
+        p.out[ra.base + (long long)n * ra.col_stride] = v * inv_scale;
+        top = max(top, amax_bits(v * inv_scale));
+      }
     }
   }
   if (!p.amax) return;
   top = __reduce_max_sync(0xffffffffu, top);
-  if ((threadIdx.x & 31) == 0 && top) atomicMax(&block_top, top);
+  if ((lane & 31) == 0 && top) atomicMax(&block_top, top);
   __syncthreads();
   if (threadIdx.x == 0 && threadIdx.y == 0 && block_top) atomicMax(p.amax, block_top);
 }
@@ -1858,7 +1862,13 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
   }
   TF_AFTER(s, what);
   if (p.tail_share > 0) {
-    launch_dep(reduce_partials_kernel<BN>, dim3(p.tail_tiles, BN / kReduceCols), dim3(BM, kReduceWays), 0, s, p);
+    // Few tiles of many pieces: 16 row groups of 32 rows, four times the blocks and a quarter of the pieces one behind the other.
+    const bool many = p.tail_tiles * (BN / kReduceCols) <= 2 * sms && p.k_total >= 12 * p.tail_share;
+    auto reduce = [&](auto ways) {
+      constexpr int W = decltype(ways)::value;
+      launch_dep(reduce_partials_kernel<BN, W>, dim3(p.tail_tiles, BN / kReduceCols, BM * W / kReduceThreads), dim3(kReduceThreads / W, W), 0, s, p);
+    };
+    if (many) reduce(std::integral_constant<int, 16>()); else reduce(std::integral_constant<int, 4>());
     TF_AFTER(s, what);
   }
   return 0;
