@@ -44,3 +44,13 @@ def test_convolution_schedules(env, case, arith):
     got, want, mag = run(2, x, w, dy), run(1, x, w, dy), run(1, np.abs(x), np.abs(w), np.abs(dy))
     for name, g, e, m in zip(("forward", "backward-data", "backward-filter"), got, want, mag):
         assert np.all(np.abs(g - e) <= 2e-6 * m + 1e-30), (name, float(np.max(np.abs(g - e) / (m + 1e-30))))
+
+
+@pytest.mark.parametrize("case", [
+    (64, 256, 29, 29, 512, 3, 3, "SAME"),     # 72 tiles in 2 ranges, two sums each: running sums end after 384 stages
+    (7, 192, 24, 24, 64, 1, 1, "VALID"),      # 2 tiles of 63 stages in 31 ranges
+    (3, 100, 31, 17, 140, 3, 3, "SAME"),      # 18 tiles in 8 ranges, ragged everywhere
+])
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+def test_reductions_cut_at_common_stages(env, case, arith):
+    test_convolution_schedules(env, case, arith)

@@ -391,6 +391,9 @@ struct alignas(64) GemmParams {
   // workspace slot and reduce_partials_kernel adds the pieces of a tile in a fixed order (no atomics: results are
   // bit-identical from run to run).
   int full_tiles, tail_tiles, tail_share, slots_per_cta;
+  // tail_pieces > 0 instead: every tail tile is cut at the same stages into this many pieces; a CTA takes tail_run of one tile in
+  // a row, and the CTAs of one range of stages lie side by side.
+  int tail_pieces, tail_run;
   float* workspace;               // [slot][BN columns][128 rows] fp32
   int chunks_per_tap;             // kModeConv: K stages per tap
   int b_tap_pitch;                // kModeConv: columns per tap in the packed filter
@@ -407,6 +410,7 @@ struct alignas(64) GemmParams {
   // kModeWgrad: M-tile rows are taps_per_tile slots of `slot` input channels of one filter tap each.  slots_per_tap > 1: a tap takes that
   // many slots in a row, and m_tiles is 1
   int slot, taps_per_tile, slots_per_tap;
+  double operand_bytes;           // of A and B together (host side)
   int group_iters;                // stages accumulated in TMEM before the epilogue promotes them to registers
   int data_by_data;               // both operands are activations / gradients (filter gradients, X^T dY): host-side hint for group_iters
   // Shared memory: a ring of A blocks and a ring of B tiles.  A filter's taps read the same rows of the activation matrix
@@ -433,6 +437,7 @@ static inline int gemm_smem_bytes(const GemmParams& p, int bn) { return p.a_slot
 // One unit of a CTA's work: `kcount` stages of tile `tile` starting at stage k0.  slot < 0: the item is the tile's
 // whole reduction and its epilogue stores to the output; otherwise its partial sums go to that workspace slot.
 struct WorkItem { int tile, k0, kcount, slot; };
+__device__ __forceinline__ int piece_start(const GemmParams& p, int piece) { return (int)((long long)p.k_total * piece / p.tail_pieces); }
 // The sequence of items of this CTA; the three warp roles walk it independently and must see the same sequence.
 struct WorkIter {
   int tile, u, u1, first_tail_tile;
@@ -440,7 +445,11 @@ struct WorkIter {
     tile = blockIdx.x;
     u = u1 = first_tail_tile = 0;
     if (p.cluster > 1) return;
-    if (p.tail_share > 0) {
+    if (p.tail_pieces > 0) {
+      const int range = blockIdx.x / p.tail_tiles;
+      first_tail_tile = blockIdx.x - range * p.tail_tiles;
+      u = range * p.tail_run; u1 = min(u + p.tail_run, p.tail_pieces);
+    } else if (p.tail_share > 0) {
       u = blockIdx.x * p.tail_share;
       u1 = min(u + p.tail_share, p.tail_tiles * p.k_total);
       first_tail_tile = u / p.k_total;
@@ -460,6 +469,13 @@ struct WorkIter {
     if (tile < whole) {
       w.tile = tile; w.k0 = 0; w.kcount = p.k_total; w.slot = -1;
       tile += gridDim.x;
+      return true;
+    }
+    if (p.tail_pieces > 0) {
+      if (u >= u1) return false;
+      w.tile = p.full_tiles + first_tail_tile; w.slot = u * p.tail_tiles + first_tail_tile;
+      w.k0 = piece_start(p, u);
+      w.kcount = piece_start(p, ++u) - w.k0;
       return true;
     }
     if (u < u1) {
@@ -1267,8 +1283,9 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_partials_kernel(const _
   const int lane = threadIdx.x, way = threadIdx.y, row = blockIdx.z * kReduceRows + lane;
   // CTA g of the GEMM covered stages [g * share, (g + 1) * share) of the tail; its first piece belongs to tail tile
   // (g * share) / k_total and its pieces sit in consecutive workspace slots
-  const int g_first = (int)(((long long)t * p.k_total) / p.tail_share);
-  const int g_last = (int)((((long long)t + 1) * p.k_total - 1) / p.tail_share);
+  const bool aligned = p.tail_pieces > 0;              // piece g of the tile: slot g * tail_tiles + t
+  const int g_first = aligned ? 0 : (int)(((long long)t * p.k_total) / p.tail_share);
+  const int g_last = aligned ? p.tail_pieces - 1 : (int)((((long long)t + 1) * p.k_total - 1) / p.tail_share);
   const int c_begin = blockIdx.y * kReduceCols;
   float sum[kReduceCols];
 #pragma unroll
@@ -1276,7 +1293,7 @@ __global__ void __launch_bounds__(kReduceThreads) reduce_partials_kernel(const _
   // four pieces per trip: their loads are independent and all in flight before the first add (a tile of a long
   // reduction has dozens of pieces, and the loop would otherwise pay the memory latency once per piece)
   auto piece = [&](int g) -> const float* {
-    const int slot = g * p.slots_per_cta + (t - (int)(((long long)g * p.tail_share) / p.k_total));
+    const int slot = aligned ? g * p.tail_tiles + t : g * p.slots_per_cta + (t - (int)(((long long)g * p.tail_share) / p.k_total));
     return p.workspace + ((size_t)slot * BN + c_begin) * BM + row;
   };
   int g = g_first + way;
@@ -1756,10 +1773,20 @@ static float g_tail_cost = [] { const char* e = getenv("TINYFLOW_TAIL_COST"); re
 // the cluster (768 -> 192 channels, 17 x 17, 1x1, batch 2: 17.0 -> 15.3 us in clusters of 6).  Against it the workspace costs
 // 4 stages and 0.15 per tile (its traffic): 70 tiles of 36 stages 34.0 us split and 29.7 in clusters of 2, 40 of 72
 // stages 33.8 and 32.5 in clusters of 3, but 12 of 72 stages 19.2 and 23 in clusters of 8.
+// How the partial wave is cut.  With a contiguous range of stages per CTA all SMs work, but the ranges of different tiles begin at
+// different stages: a filter gradient, whose tiles all read both operands along K, then fetches them from HBM once per CTA when
+// L2 cannot hold them (256 -> 256 channels, 57 x 57 frames, batch 64, 36 tiles: 990 us, 7.5 TB/s of operands), and most CTAs
+// leave two partial sums.  Cut at the same stages into as many pieces as there are CTAs for, the CTAs of a range share what they
+// fetch (736 us), and each leaves one sum (768 -> 192 channels, 17 x 17, 1x1, batch 32: 33.0 -> 28.0 us).  The price is idle
+// CTAs where sms / tiles is not whole: up to 10 % where operands are read once, 25 % for filter gradients, 50 % beyond L2.
+static constexpr double kL2Holds = 64e6;
+// Stages that one running sum takes before it is put down: a sum's rounding grows with its length, and another 64 KB per 384 stages
+// (300 us) cost nothing.
+static constexpr int kLongestSum = 384;
 template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, StreamLease& lease, int* oom, MaxClusters max_clusters) {
   const int sms = device_sm_count();
   const int tiles = g.m_tiles * g.n_tiles * g.tap_tiles;
-  g.full_tiles = tiles; g.tail_tiles = 0; g.tail_share = 0; g.slots_per_cta = 0; g.workspace = nullptr; g.cluster = 1;
+  g.full_tiles = tiles; g.tail_tiles = 0; g.tail_share = 0; g.slots_per_cta = 0; g.tail_pieces = g.tail_run = 0; g.workspace = nullptr; g.cluster = 1;
   const int rem = tiles % sms;
   static const bool no_split = getenv("TINYFLOW_NO_TAIL_SPLIT") != nullptr;
   if (rem == 0 || no_split) return 0;
@@ -1780,7 +1807,17 @@ template <class MaxClusters> static int plan_schedule(GemmParams& g, int bn, Str
   g.cluster = 1;
   g.full_tiles = tiles - rem; g.tail_tiles = rem; g.tail_share = share;
   g.slots_per_cta = (share - 1 + g.k_total - 1) / g.k_total + 1;       // tiles a range of `share` stages can touch
-  const int ctas = (int)((units + share - 1) / share);
+  int ctas = (int)((units + share - 1) / share);
+  // All tiles cut at the same stages, one piece a CTA, wherever that leaves few CTAs idle.
+  const int pieces = std::min(sms / rem, g.k_total / 2);          // two stages at least
+  if (pieces >= 2) {
+    const int even = (g.k_total + pieces - 1) / pieces;
+    const double slack = !(g.a_mn && g.b_mn) ? 1.1 : g.operand_bytes > kL2Holds ? 1.5 : 1.25;
+    if (even <= share * slack) {
+      g.tail_run = (even + kLongestSum - 1) / kLongestSum;
+      g.tail_pieces = pieces * g.tail_run; g.tail_share = even; g.slots_per_cta = g.tail_run; ctas = rem * pieces;
+    }
+  }
   const size_t bytes = (size_t)ctas * g.slots_per_cta * bn * BM * sizeof(float);
   g.workspace = (float*)lease.scratch(kScratchTiles, bytes);
   if (!g.workspace) { if (oom) *oom = bytes > 0x7fffffffu ? 0x7fffffff : (int)bytes; return 1; }
@@ -1843,7 +1880,7 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
   const int tiles = p.full_tiles + p.tail_tiles;
   int grid = tiles < sms ? tiles : sms;
   if (p.tail_share > 0) {
-    const int ctas = (int)(((long long)p.tail_tiles * p.k_total + p.tail_share - 1) / p.tail_share);
+    const int ctas = p.tail_pieces > 0 ? p.tail_tiles * (p.tail_pieces / p.tail_run) : (int)(((long long)p.tail_tiles * p.k_total + p.tail_share - 1) / p.tail_share);
     grid = p.full_tiles > 0 ? sms : ctas;
   }
   if (p.cluster > 1) grid = tiles * p.cluster;
@@ -1852,8 +1889,8 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
   note_compute_stream(s);
   static const bool detail = getenv("TINYFLOW_TIMING_DETAIL") != nullptr;    // one timing row per distinct problem shape
   char name[192];
-  if (detail) snprintf(name, sizeof(name), "gemm3x%s mode%d M%d N%d ktotal%d taps%d bn%d tiles%d tail%d share%d cl%d a%dx%d b%d%s %s", AR == kArithTF32 ? "tf32" : "f16", p.mode, p.M,
-                       p.N, p.k_total, p.tap_tiles, BN, tiles, p.tail_tiles, p.tail_share, p.cluster, p.a_slots, p.a_rows, p.b_slots, p.b_resident ? "r" : "", what + 5);
+  if (detail) snprintf(name, sizeof(name), "gemm3x%s mode%d M%d N%d ktotal%d taps%d bn%d tiles%d tail%d share%d cl%d p%d a%dx%d b%d%s %s", AR == kArithTF32 ? "tf32" : "f16", p.mode, p.M,
+                       p.N, p.k_total, p.tap_tiles, BN, tiles, p.tail_tiles, p.tail_share, p.cluster, p.tail_pieces, p.a_slots, p.a_rows, p.b_slots, p.b_resident ? "r" : "", what + 5);
   KernelTimer kt(detail ? name : (AR == kArithTF32 ? "gemm3xtf32_tcgen05" : "gemm3xf16_tcgen05"), s, flops, 0, 1);
   if (p.cluster > 1) {
     TF_CUDA(launch_cluster(gemm3x_kernel<BN, AR>, p.cluster, dim3(grid), dim3(kGemmThreads), (size_t)gemm_smem_bytes(p, BN), s, p));
@@ -2602,6 +2639,7 @@ int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaS
       g.M = p->K; g.N = st->eC; g.ldc = st->eC;
       g.m_tiles = (p->K + BM - 1) / BM; g.n_tiles = (st->eC + bn - 1) / bn; g.tap_tiles = 1; g.ntaps = 1;
       g.k_total = kit;
+      g.operand_bytes = 2.0 * st->dy.bytes() + 2.0 * st->x_pack().bytes();
       return tc_result(launch_gemm_bn(bn, ar, g, s, conv_flops(p), "DLGpuConvolutionBackwardFilter", oom));
     }
   }
@@ -2640,6 +2678,7 @@ int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaS
       }
     }
   g.k_total = kit;
+  g.operand_bytes = 2.0 * st->dy.bytes() + 2.0 * st->x_pack().bytes();
   return tc_result(launch_gemm_bn(bn, ar, g, s, conv_flops(p), "DLGpuConvolutionBackwardFilter", oom));
 }
 
