@@ -754,7 +754,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
       //                     the cross terms accumulate for cross_groups groups before the epilogue takes them.  The wide
       //                     instruction goes to (main0, cross) or (cross, main1), hence the order of the B tiles;
       //   kAccPair          two sets of {cross, main} and one issuer: short reductions, where the next tile must not wait for the
-      //                     epilogue to read the cross terms, and groups of one stage, where the epilogue is the bound anyway.
+      //                     epilogue to read the cross terms, and short groups of one stage (see launch_gemm).
       // instruction descriptor: D = f32 (bits 4-5 = 1), A format at bit 7, B format at bit 10, majors at bits 15 / 16,
       // N >> 3 at bit 17, M >> 4 at bit 24
       const uint32_t idesc_base = (1u << 4) | (T::kFormat << 7) | (T::kFormat << 10) | ((uint32_t)p.a_mn << 15) | ((uint32_t)p.b_mn << 16) |
@@ -1777,7 +1777,7 @@ static float g_tail_cost = [] { const char* e = getenv("TINYFLOW_TAIL_COST"); re
 // different stages: a filter gradient, whose tiles all read both operands along K, then fetches them from HBM once per CTA when
 // L2 cannot hold them (256 -> 256 channels, 57 x 57 frames, batch 64, 36 tiles: 990 us, 7.5 TB/s of operands), and most CTAs
 // leave two partial sums.  Cut at the same stages into as many pieces as there are CTAs for, the CTAs of a range share what they
-// fetch (736 us), and each leaves one sum (768 -> 192 channels, 17 x 17, 1x1, batch 32: 33.0 -> 28.0 us).  The price is idle
+// fetch (736 us; with two issuers 672), and each leaves one sum (768 -> 192 channels, 17 x 17, 1x1, batch 32: 33.0 -> 28.0 us).  The price is idle
 // CTAs where sms / tiles is not whole: up to 10 % where operands are read once, 25 % for filter gradients, 50 % beyond L2.
 static constexpr double kL2Holds = 64e6;
 // Stages that one running sum takes before it is put down: a sum's rounding grows with its length, and another 64 KB per 384 stages
@@ -1875,7 +1875,9 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
     // Two issuers gain from 8 stages per CTA on (equal at 18 of 128 columns, 1 us of 65 at 36); at 96 columns the narrow MMAs
   // are short enough for one warp (12 stages: 19.2 against 21.2 us).
   const int longest = p.tail_share > 0 && p.full_tiles == 0 ? p.tail_share : p.k_total / p.cluster;
-  p.acc_mode = BN != 64 && p.k_total > p.group_iters && longest >= (BN == 128 ? 8 : 24) && p.group_iters > 1 ? kAccThree : kAccPair;
+  // Groups of one stage begin the main sum anew with two instructions instead of a wide one: equal at 22 stages, 4 % faster
+  // at 55, 9 % at 841 (512 -> 512 channels, 28 x 28, 3x3, batch 64: 750 -> 673 us).
+  p.acc_mode = BN != 64 && p.k_total > p.group_iters && longest >= (BN == 128 && p.group_iters > 1 ? 8 : 24) ? kAccThree : kAccPair;
   const int sms = device_sm_count();
   const int tiles = p.full_tiles + p.tail_tiles;
   int grid = tiles < sms ? tiles : sms;
