@@ -1262,79 +1262,101 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_pair_kernel(const __grid_c
   if (threadIdx.x == 0 && *abort_flag && p.err) atomicExch(p.err, 1);
 }
 
-// Adds up the pieces of every split tile (the tail of the schedule) in a fixed order and writes the result where the
-// GEMM's own epilogue would have.  grid (tail_tiles, BN / kReduceCols, BM / ROWS), block (ROWS, WAYS), 512 threads: the pieces of a
-// tile are dealt round robin to the WAYS row groups, each adds its share in piece order, and the subtotals are
-// added in row-group order - the same order every run, so the result is bit-reproducible.  Bound by latency: one memory round trip
-// per four pieces of a row group.  16 row groups of 32 rows where a launch has few tiles of many pieces (the filter gradients of
-// ResNet-50 at batch 19: step 4434 -> 4383 us, DenseNet-121: 14755 -> 14622); elsewhere 4 of 128, since there the blocks'
-// starts are what counts (16 everywhere: Inception-v4 20750 -> 23020 us).
-constexpr int kReduceCols = 8, kReduceThreads = 512;
-template <int BN, int WAYS>
-__global__ void __launch_bounds__(kReduceThreads) reduce_partials_kernel(const __grid_constant__ GemmParams p) {
-  constexpr int kReduceWays = WAYS, kReduceRows = kReduceThreads / WAYS;
-  __shared__ float part[kReduceWays][kReduceCols][kReduceRows];
-  __shared__ uint32_t block_top;
-  if (threadIdx.x == 0 && threadIdx.y == 0) block_top = 0u;
-  grid_dep_sync();
-  const int t = blockIdx.x;                            // tail tile
+// Adds up the pieces of every split tile in piece order and writes the result where the GEMM's own epilogue would have: the order
+// in which the grouped kernel adds them where it keeps a tile to itself, so both give the same bits.  Bound by latency.
+//   MANY = false (tiles of few pieces; the blocks' starts are what counts): grid (tiles, BN / 8), 256 threads, a thread has 4 columns
+//     of 4 pieces in flight.
+//   MANY = true (few tiles of many pieces): grid (tiles, BN / 8, 4), 16 warps take three pieces of 8 columns x 32 rows each to shared
+//     memory, so that 48 pieces cost one memory round trip, and 8 of them add one column each.  With 16 pieces of a column in flight
+//     in one thread instead ResNet-50 at batch 19 took 4524 us a step, with this 4389 (4434 with 4 row groups).
+constexpr int kReduceCols = 8;
+template <bool MANY> constexpr int kReduceThreads = MANY ? 512 : 256;
+template <int BN, bool MANY, class Piece>
+__device__ __forceinline__ void reduce_tile(const GemmParams& p, int tile, int pieces, Piece&& piece) {
   int mt, nt, tap;
-  decode_tile(p, p.full_tiles + t, mt, nt, tap);
-  const int lane = threadIdx.x, way = threadIdx.y, row = blockIdx.z * kReduceRows + lane;
-  // CTA g of the GEMM covered stages [g * share, (g + 1) * share) of the tail; its first piece belongs to tail tile
-  // (g * share) / k_total and its pieces sit in consecutive workspace slots
-  const bool aligned = p.tail_pieces > 0;              // piece g of the tile: slot g * tail_tiles + t
-  const int g_first = aligned ? 0 : (int)(((long long)t * p.k_total) / p.tail_share);
-  const int g_last = aligned ? p.tail_pieces - 1 : (int)((((long long)t + 1) * p.k_total - 1) / p.tail_share);
-  const int c_begin = blockIdx.y * kReduceCols;
-  float sum[kReduceCols];
+  decode_tile(p, tile, mt, nt, tap);
+  constexpr int COLS = MANY ? 1 : 4;
+  const int row = MANY ? blockIdx.z * 32 + (threadIdx.x & 31) : threadIdx.x & (BM - 1);
+  const int c0 = blockIdx.y * kReduceCols + (MANY ? threadIdx.x / 32 : threadIdx.x / BM * COLS);
+  float sum[COLS];
 #pragma unroll
-  for (int q = 0; q < kReduceCols; ++q) sum[q] = 0.f;
-  // four pieces per trip: their loads are independent and all in flight before the first add (a tile of a long
-  // reduction has dozens of pieces, and the loop would otherwise pay the memory latency once per piece)
-  auto piece = [&](int g) -> const float* {
-    const int slot = aligned ? g * p.tail_tiles + t : g * p.slots_per_cta + (t - (int)(((long long)g * p.tail_share) / p.k_total));
-    return p.workspace + ((size_t)slot * BN + c_begin) * BM + row;
-  };
-  int g = g_first + way;
-  for (; g + 3 * kReduceWays <= g_last; g += 4 * kReduceWays) {
-    const float *w0 = piece(g), *w1 = piece(g + kReduceWays), *w2 = piece(g + 2 * kReduceWays), *w3 = piece(g + 3 * kReduceWays);
-    float v0[kReduceCols], v1[kReduceCols], v2[kReduceCols], v3[kReduceCols];
+  for (int q = 0; q < COLS; ++q) sum[q] = 0.f;
+  if (MANY) {
+    constexpr int kEach = 3, kAtOnce = 16 * kEach;
+    __shared__ float held[kAtOnce][kReduceCols][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int g0 = 0; g0 < pieces; g0 += kAtOnce) {
+      float v[kEach][kReduceCols];
 #pragma unroll
-    for (int q = 0; q < kReduceCols; ++q) { v0[q] = __ldcg(w0 + (size_t)q * BM); v1[q] = __ldcg(w1 + (size_t)q * BM); v2[q] = __ldcg(w2 + (size_t)q * BM); v3[q] = __ldcg(w3 + (size_t)q * BM); }
+      for (int e = 0; e < kEach; ++e) {
+        const int g = g0 + e * 16 + warp;
+        if (g < pieces) {
+          const float* ws = piece(g) + (size_t)blockIdx.y * kReduceCols * BM + row;
 #pragma unroll
-    for (int q = 0; q < kReduceCols; ++q) sum[q] = (((sum[q] + v0[q]) + v1[q]) + v2[q]) + v3[q];
-  }
-  for (; g <= g_last; g += kReduceWays) {
-    const float* ws = piece(g);
-#pragma unroll
-    for (int q = 0; q < kReduceCols; ++q) sum[q] += __ldcg(ws + (size_t)q * BM);
-  }
-#pragma unroll
-  for (int q = 0; q < kReduceCols; ++q) part[way][q][lane] = sum[q];
-  __syncthreads();
-  // the row groups share the columns: subtotals added in row-group order
-  uint32_t top = 0;
-  if (way < kReduceCols) {
-    const RowAddr ra = row_address(p, mt, tap, row);
-    const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));
-#pragma unroll
-    for (int q = way; q < kReduceCols; q += kReduceWays) {
-      float v = part[0][q][lane];
-#pragma unroll
-      for (int w2 = 1; w2 < kReduceWays; ++w2) v += part[w2][q][lane];
-      const int n = nt * BN + c_begin + q;
-      if (ra.ok && n < p.N) {
-        p.out[ra.base + (long long)n * ra.col_stride] = v * inv_scale;
-        top = max(top, amax_bits(v * inv_scale));
+          for (int q = 0; q < kReduceCols; ++q) v[e][q] = __ldcg(ws + (size_t)q * BM);
+        }
       }
+      if (g0) __syncthreads();
+#pragma unroll
+      for (int e = 0; e < kEach; ++e)
+#pragma unroll
+        for (int q = 0; q < kReduceCols; ++q) held[e * 16 + warp][q][lane] = v[e][q];
+      __syncthreads();
+      const int n = min(kAtOnce, pieces - g0);
+      if (warp < kReduceCols)
+        for (int i = 0; i < n; ++i) sum[0] += held[i][warp][lane];
+    }
+    if (warp >= kReduceCols) return;
+  } else {
+    constexpr int DEPTH = 4;
+    for (int g = 0; g < pieces; g += DEPTH) {
+      float v[DEPTH][COLS];
+#pragma unroll
+      for (int d = 0; d < DEPTH; ++d) {
+        if (g + d < pieces) {
+          const float* ws = piece(g + d) + (size_t)c0 * BM + row;
+#pragma unroll
+          for (int q = 0; q < COLS; ++q) v[d][q] = __ldcg(ws + (size_t)q * BM);
+        }
+      }
+#pragma unroll
+      for (int d = 0; d < DEPTH; ++d)
+        if (g + d < pieces) {
+#pragma unroll
+          for (int q = 0; q < COLS; ++q) sum[q] += v[d][q];
+        }
+    }
+  }
+  const RowAddr ra = row_address(p, mt, tap, row);
+  const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));
+  uint32_t top = 0;
+#pragma unroll
+  for (int q = 0; q < COLS; ++q) {
+    const int n = nt * BN + c0 + q;
+    if (ra.ok && n < p.N) {
+      p.out[ra.base + (long long)n * ra.col_stride] = sum[q] * inv_scale;
+      top = max(top, amax_bits(sum[q] * inv_scale));
     }
   }
   if (!p.amax) return;
   top = __reduce_max_sync(0xffffffffu, top);
-  if ((lane & 31) == 0 && top) atomicMax(&block_top, top);
-  __syncthreads();
-  if (threadIdx.x == 0 && threadIdx.y == 0 && block_top) atomicMax(p.amax, block_top);
+  if ((threadIdx.x & 31) == 0 && top) atomicMax(p.amax, top);
+}
+template <int BN, bool MANY>
+__global__ void __launch_bounds__(kReduceThreads<MANY>) reduce_partials_kernel(const __grid_constant__ GemmParams p) {
+  grid_dep_sync();
+  const int t = blockIdx.x;                            // tail tile
+  // Cut at common stages: piece g sits in slot g * tail_tiles + t.  Otherwise CTA g of the GEMM covered stages
+  // [g * share, (g + 1) * share) of the tail; its first piece belongs to tail tile (g * share) / k_total and its pieces sit in
+  // consecutive slots
+  const bool aligned = p.tail_pieces > 0;
+  const int first = aligned ? 0 : (int)(((long long)t * p.k_total) / p.tail_share);
+  const int last = aligned ? p.tail_pieces - 1 : (int)((((long long)t + 1) * p.k_total - 1) / p.tail_share);
+  reduce_tile<BN, MANY>(p, p.full_tiles + t, last - first + 1, [&](int i) -> const float* {
+    const int g = first + i;
+    const int slot = aligned ? g * p.tail_tiles + t : g * p.slots_per_cta + (t - (int)(((long long)g * p.tail_share) / p.k_total));
+    return p.workspace + (size_t)slot * BN * BM;
+  });
 }
 
 // Exercises the bounded wait on its own: one thread waits, with a short limit, on a barrier that nothing arms; the wait
@@ -1862,6 +1884,12 @@ template <int BN, int AR> static int max_clusters_of(int c) {
   }
   return n;
 }
+// The form of the summing kernel for tiles of about that many pieces
+template <int BN, class F> static cudaError_t launch_reduce(int tiles, int pieces, F&& launch) {
+  const dim3 grid(tiles, BN / kReduceCols);
+  if (pieces >= 12 && tiles * (BN / kReduceCols) <= 2 * device_sm_count()) return launch(std::true_type(), dim3(grid.x, grid.y, BM / 32), dim3(kReduceThreads<true>));
+  return launch(std::false_type(), grid, dim3(kReduceThreads<false>));
+}
 template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, double flops, const char* what, int* oom) {
   static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
   TF_CUDA(attr);
@@ -1901,13 +1929,8 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
   }
   TF_AFTER(s, what);
   if (p.tail_share > 0) {
-    // Few tiles of many pieces: 16 row groups of 32 rows, four times the blocks and a quarter of the pieces one behind the other.
-    const bool many = p.tail_tiles * (BN / kReduceCols) <= 2 * sms && p.k_total >= 12 * p.tail_share;
-    auto reduce = [&](auto ways) {
-      constexpr int W = decltype(ways)::value;
-      launch_dep(reduce_partials_kernel<BN, W>, dim3(p.tail_tiles, BN / kReduceCols, BM * W / kReduceThreads), dim3(kReduceThreads / W, W), 0, s, p);
-    };
-    if (many) reduce(std::integral_constant<int, 16>()); else reduce(std::integral_constant<int, 4>());
+    const int pieces = p.tail_pieces > 0 ? p.tail_pieces : p.k_total / p.tail_share + 1;
+    launch_reduce<BN>(p.tail_tiles, pieces, [&](auto many, dim3 grid, dim3 block) { return launch_dep(reduce_partials_kernel<BN, decltype(many)::value>, grid, block, 0, s, p); });
     TF_AFTER(s, what);
   }
   return 0;
