@@ -324,6 +324,12 @@ int TfStepRecordBegin(void **graph, void **stream_cell, void **replay_stream);
  * already, where the convolutions of the step would pack them one by one.  A hint: what is left out is packed when its
  * convolution comes. */
 int TfPackFilters(const DLArrayHandle *filters, void ***const *plans, int n, void **cudaStream);
+/* Filter gradients called between TfHoldProducts(1) and TfHoldProducts(0) by this thread may wait for others, to share a launch with
+ * them: their results are there after TfLaunchHeld on the stream they were called on.  Until then nothing may read them, and the
+ * input and the incoming gradient of the convolution may not be freed.  TfDropHeld forgets those that wait (a step that failed). */
+int TfHoldProducts(int on);
+int TfLaunchHeld(void **cudaStream);
+int TfDropHeld(void);
 int TfStepRecordEnd(void **graph, int keep);
 int TfStepReplay(void *graph, const unsigned *seeds, int nseeds, float b1t, float b2t,
                  const DLArrayHandle *params, int nparams, void **cudaStream);

@@ -1,0 +1,68 @@
+"""Filter gradients that wait and share a launch: the bits of separate launches, whatever is held back together."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_step_graph import BUILDS, _same, _train
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+@pytest.mark.parametrize("name", ["inceptionv3", "resnet50", "vgg16", "densenet121"])
+def test_products_held_back_have_the_bits_of_separate_launches(lib_path, monkeypatch, name, arith):
+    from tinyflow_b200 import gpu_op
+    build = BUILDS.get(name, lambda m: m.densenet121(batch=16, classes=10, image=96))
+    gpu_op.set_tensor_arithmetic(arith)
+    try:
+        got = _train(monkeypatch, True, build, "sgd")
+        with monkeypatch.context() as m:
+            m.setattr(gpu_op, "hold_products", lambda on: None)
+            want = _train(monkeypatch, False, build, "sgd")
+    finally:
+        gpu_op.set_tensor_arithmetic("3xfp16")
+    assert got[2] and not want[2]
+    _same(got, want)
+
+
+# N, C, H, W, K, R, S, stride: with and without several taps a tile, odd numbers of 64-channel blocks, ragged tiles, cut and whole reductions
+LAYERS = [(2, 64, 9, 9, 96, 3, 3, 1), (3, 160, 12, 7, 160, 7, 1, 1), (2, 33 * 4, 9, 9, 68, 1, 7, 1), (5, 64, 14, 14, 256, 1, 1, 1), (5, 256, 14, 14, 64, 1, 1, 1),
+          (4, 288, 17, 17, 384, 3, 3, 2), (1, 48, 21, 21, 64, 5, 5, 1), (16, 96, 35, 35, 64, 1, 1, 1), (2, 768, 17, 17, 192, 1, 1, 1), (8, 128, 28, 28, 32, 3, 3, 1), (2, 3, 75, 75, 32, 3, 3, 2)]
+
+
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+@pytest.mark.parametrize("layers", [LAYERS, LAYERS[:1], LAYERS[7:8]], ids=["all", "one", "one cut"])
+def test_layers_in_one_launch(lib_path, layers, arith):
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, stream, rng = nd.gpu(0), gpu_op.create_cudaStream(), np.random.RandomState(1)
+    handle = gpu_op.create_cudnnHandle(stream)
+    gpu_op.set_tensor_arithmetic(arith)
+    calls = []
+    for N, C, H, W, K, R, S, u in layers:
+        out, cell = gpu_op.convolution_2d_forward_get_out_shape((N, C, H, W), (K, C, R, S), "NCHW", "VALID" if u > 1 else "SAME", u, u)
+        x, w, dy = (nd.array(rng.randn(*shape).astype(np.float32), ctx) for shape in ((N, C, H, W), (K, C, R, S), out))
+        calls.append((x, dy, w, nd.empty((K, C, R, S), ctx), nd.array(np.full((K, C, R, S), np.nan, np.float32), ctx), cell))
+    try:
+        for x, dy, w, apart, _, cell in calls:
+            gpu_op.convolution_backward_filter(x, dy, w, apart, cell, handle, stream)
+        for again in range(2):                       # the second time on packs that are there
+            gpu_op.hold_products(True)
+            for x, dy, w, _, together, cell in calls:
+                gpu_op.convolution_backward_filter(x, dy, w, together, cell, handle, stream)
+            gpu_op.hold_products(False)
+            gpu_op.launch_held(stream)
+            for shape, (_, _, _, apart, together, _) in zip(layers, calls):
+                np.testing.assert_array_equal(together.asnumpy(), apart.asnumpy(), err_msg=str(shape))
+        # a pack that is written again lets what has to read it go first
+        x, dy, w, apart, together, cell = calls[0]
+        gpu_op.hold_products(True)
+        gpu_op.convolution_backward_filter(x, dy, w, together, cell, handle, stream)
+        other = nd.array(rng.randn(*x.shape).astype(np.float32), ctx)
+        second = nd.empty(w.shape, ctx)
+        gpu_op.convolution_backward_filter(other, dy, w, second, cell, handle, stream)
+        gpu_op.hold_products(False)
+        np.testing.assert_array_equal(together.asnumpy(), apart.asnumpy())
+        gpu_op.launch_held(stream)
+        assert not np.array_equal(second.asnumpy(), apart.asnumpy())
+    finally:
+        gpu_op.drop_held()
+        gpu_op.set_tensor_arithmetic("3xfp16")

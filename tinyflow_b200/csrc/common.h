@@ -7,6 +7,7 @@
 #include <string.h>
 #include <atomic>
 #include <tuple>
+#include <vector>
 #include "../../include/c_runtime_api.h"
 
 namespace tf {
@@ -160,6 +161,7 @@ bool recordings_give_up_memory();                  // every recording that is no
 void recording_note_launches(int n);
 void recording_note_write(const void* p);
 cudaStream_t recording_stream();
+void* recording_own(std::vector<char>& bytes);     // device memory with these bytes, uploaded ahead of the first replay, for the recording's life; nullptr: out of memory
 void recording_refuse(const char* why);            // the step cannot be recorded: End gives this reason
 // Buffers that outlive a call (packs) were reallocated or the arithmetic changed: recorded steps are out of date.
 void bump_layout_epoch();
@@ -185,7 +187,7 @@ void pool_free(void* p);
 // block to the last launch that uses it.  A block is the same at every call until a larger one is asked for; slot ids are per
 // purpose, so that what one operator uses together does not collide.
 struct StreamScratch;
-enum { kScratchSums = 0, kScratchTiles = 1, kScratchSplit = 2, kScratchContract = 3, kScratchPackA = 4, kScratchPackB = 5, kScratchSlots = 6 };
+enum { kScratchSums = 0, kScratchTiles = 1, kScratchSplit = 2, kScratchContract = 3, kScratchPackA = 4, kScratchPackB = 5, kScratchGroup = 6, kScratchSlots = 7 };
 class StreamLease {
  public:
   explicit StreamLease(cudaStream_t s);

@@ -20,6 +20,9 @@ int direct_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float*
 int tc_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_t M, int64_t N, int64_t K, cudaStream_t s, int* oom_bytes);
 int tc_conv_fwd(ConvPlan* p, const float* x, const float* w, float* y, cudaStream_t s, int* oom_bytes);
 int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaStream_t s, int* oom_bytes);
+void hold_products(bool on);
+int launch_held(cudaStream_t s);
+void drop_held();
 int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaStream_t s, int* oom_bytes);
 
 static int g_path = [] { const char* e = getenv("TINYFLOW_CONTRACTION"); return e ? atoi(e) : 0; }();   // 0 auto, 1 CUDA cores, 2 tensor cores
@@ -65,6 +68,9 @@ int TfPackFilters(const DLArrayHandle* filters, void*** const* plans, int n, voi
   }
   return tc_pack_filters(plan.data(), data.data(), sizes.data(), (int)plan.size(), stream_of(cudaStream));
 }
+int TfHoldProducts(int on) { hold_products(on != 0); return 0; }
+int TfLaunchHeld(void** cudaStream) { return launch_held(stream_of(cudaStream)); }
+int TfDropHeld(void) { drop_held(); return 0; }
 int TfFusedReluPackCount(long long* count) { if (count) *count = fused_relu_pack_count(); return 0; }
 int TfFusedReluBnBackwardCount(long long* count) { if (count) *count = fused_relu_bn_bwd_count(); return 0; }
 int TfFusedAddReluCount(long long* count) { if (count) *count = fused_add_relu_count(); return 0; }

@@ -21,6 +21,8 @@ thread_local StepGraph* t_recording = nullptr;
 static std::atomic<uint64_t> g_layout_epoch{1};
 void bump_layout_epoch() { g_layout_epoch.fetch_add(1, std::memory_order_relaxed); }
 int tensor_path_error();
+int launch_held(cudaStream_t s);
+void drop_held();
 void tc_recording_begins();
 bool dp_active();
 
@@ -41,6 +43,7 @@ struct StepGraph {
   bool has_adam = false;
   float c1 = 0.f, c2 = 0.f;
   std::unordered_map<size_t, std::vector<void*>> free_blocks;
+  std::vector<std::pair<void*, std::vector<char>>> owned;      // tables that its kernels read, and the memory they were uploaded from
   std::vector<const void*> written;
   std::vector<const void**> made;         // sources of the packs and indices in plans that the graph writes
   std::vector<AmaxCarry> carries;
@@ -52,6 +55,17 @@ struct StepGraph {
 static std::atomic<uint64_t> g_recordings{0};
 uint64_t recording_id() { return t_recording ? t_recording->id : 0; }
 
+void* recording_own(std::vector<char>& bytes) {
+  StepGraph* g = t_recording;
+  t_recording = nullptr;                  // not a block that was freed in the recording: its kernels still write those
+  void* p = pool_alloc(bytes.size());
+  t_recording = g;
+  if (!p) return nullptr;
+  g->owned.emplace_back(p, std::move(bytes));
+  const std::vector<char>& kept = g->owned.back().second;
+  if (cudaMemcpyAsync(p, kept.data(), kept.size(), cudaMemcpyHostToDevice, g->home) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+  return p;
+}
 void recording_refuse(const char* why) { if (!t_recording->refused) t_recording->refused = why; }
 uint32_t* recording_word() {
   StepGraph* g = t_recording;
@@ -162,6 +176,8 @@ static void step_graph_release(StepGraph* g) {
   if (g->graph) cudaGraphDestroy(g->graph);
   if (g->words) pool_free(g->words);
   for (auto& kv : g->free_blocks) for (void* p : kv.second) pool_free(p);
+  for (auto& o : g->owned) pool_free(o.first);
+  g->owned.clear();
   g->exec = nullptr; g->graph = nullptr; g->words = nullptr;
   g->free_blocks.clear();
   cudaGetLastError();
@@ -232,6 +248,8 @@ int TfStepRecordEnd(void** graph, int keep) {
   TF_REQUIRE(graph && *graph && t_recording == (StepGraph*)*graph, "TfStepRecordEnd: this thread is not recording that step");
   StepGraph* g = t_recording;
   flush_deferred();
+  if (!keep) drop_held();
+  else if (launch_held(g->stream)) recording_refuse("the filter gradients that were held back could not be launched");
   bool ok = keep != 0 && !g->refused;
   if (ok) {
     g->carries.resize(kCarries);

@@ -26,7 +26,7 @@ import warnings
 import weakref
 
 from . import gpu_op, ndarray, step_graph
-from .graph import (AddOp, AdamOp, BNForwardOp, Convolution2DForwardOp, OnesLikeOp, Pooling2DForwardOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
+from .graph import (AddOp, AdamOp, BNForwardOp, Convolution2DBackwardOp, Convolution2DForwardOp, OnesLikeOp, Pooling2DForwardOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
 
 
 def getcomputelist(Variable_node_list, Variable_node_grad_list, b1, b2, b1t, b2t, e, learning_rate):
@@ -190,6 +190,13 @@ class Executor(object):
         # convolutions of a fed filter, and their descriptors as the library takes them (with the objects behind)
         self._convs = [n for n in self.topo_order if type(n.op) is Convolution2DForwardOp and not n.inputs[1].inputs]
         self._conv_cells = ([], None)
+        # filter gradients that only the optimiser reads: they may wait and share launches
+        readers = {}
+        for node in self.topo_order:
+            for i in node.inputs:
+                readers.setdefault(i, []).append(node)
+        self._patient = {n for n in self.topo_order if type(n.op) is Convolution2DBackwardOp and n.type == 1
+                         and all(type(r.op) in (SgdOp, AdamOp) for r in readers.get(n, ()))}
         self._values = {}          # node index -> NDArray on the GPU (None while swapped out)
         self._feed = {}            # what the most recent run was fed: node -> NDArray on the GPU
         self._leases = {}          # node index -> weak references to the views of its array that were handed out
@@ -422,7 +429,13 @@ class Executor(object):
             if self.have_plan:
                 for idx in node.recompute_list:
                     self._compute(self.topo_order[idx], None, stream)
-            if timed:
+            if together and node in self._patient:
+                gpu_op.hold_products(True)
+                try:
+                    self._compute(node, out, stream)
+                finally:
+                    gpu_op.hold_products(False)
+            elif timed:
                 t0 = time.perf_counter()
                 self._compute(node, out, stream)
                 node.runtime = (time.perf_counter() - t0) * 1000.0
@@ -430,6 +443,8 @@ class Executor(object):
                 self._compute(node, out, stream)
             if self.have_plan:
                 self._after_node(node)
+        if together:
+            gpu_op.launch_held(stream)
         if updates:
             self._update_parameters(updates, stream)
         previous.clear()
@@ -464,7 +479,11 @@ class Executor(object):
             self.feed_shapes = feed_shapes
         if self.top_control_queue is not None and not self.top_control_queue.empty():
             self._apply_plan(*self.top_control_queue.get())
-        self._issue(feed_dict, self.cudaStream)
+        try:
+            self._issue(feed_dict, self.cudaStream)
+        except BaseException:
+            gpu_op.drop_held()
+            raise
         if self._swap_worker is not None:
             self._swap_worker.drain()
         return self._resident(self.targetloss)

@@ -433,6 +433,19 @@ def pack_filters(filters, cells, cudaStream):
     check_call(_LIB.TfPackFilters(handle_array(filters), cells, len(filters), cudaStream))
 
 
+def hold_products(on):
+    """Filter gradients called from here on may wait for others until :func:`launch_held`: nobody reads them before."""
+    check_call(_LIB.TfHoldProducts(1 if on else 0))
+
+
+def launch_held(cudaStream):
+    check_call(_LIB.TfLaunchHeld(cudaStream))
+
+
+def drop_held():
+    check_call(_LIB.TfDropHeld())
+
+
 def sgd_update_many(params, grads, learning_rate, cudaStream):
     """``sgd_update`` of every pair in one launch; ``params`` and ``grads`` come from :func:`handle_array`."""
     check_call(_LIB.TfSgdUpdateMany(params, grads, len(params), _F(learning_rate), cudaStream))
