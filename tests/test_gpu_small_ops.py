@@ -47,6 +47,12 @@ def test_direct_convolution_of_few_channels(env, case):
         np.testing.assert_allclose(a, b, rtol=1e-4, atol=3e-5 * np.abs(b).max())
 
 
+@pytest.mark.parametrize("case", [(1, 16, 10, 10, 6, 5, 5, "SAME"), (300, 15, 6, 5, 12, 3, 3, "SAME"), (700, 4, 8, 9, 7, 3, 3, "VALID"),       # 4, 2 and 1 lanes an item
+                                  (2, 2, 5, 3, 9, 3, 3, "SAME"), (4, 1, 7, 1, 4, 3, 3, "SAME"), (3, 13, 30, 31, 10, 7, 7, "VALID"), (5, 8, 12, 12, 16, 5, 5, "SAME")])
+def test_direct_convolution_lanes_that_share_items(env, case):
+    test_direct_convolution_of_few_channels(env, case)
+
+
 @pytest.mark.parametrize("shape", [(1, 1, 1, 1), (256, 6, 28, 28), (3, 300, 5, 7), (64, 16, 10, 10), (1, 2, 129, 3)])
 def test_channel_sums(env, shape):
     x = np.random.RandomState(1).randn(*shape).astype(np.float32)
