@@ -54,3 +54,40 @@ def test_convolution_schedules(env, case, arith):
 @pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
 def test_reductions_cut_at_common_stages(env, case, arith):
     test_convolution_schedules(env, case, arith)
+
+
+# K, C, R, S: enough blocks that a block takes 9 taps, or 288 channels of a 1x1 filter
+@pytest.mark.parametrize("filters", [[(1024, 1160, 1, 1), (640, 1000, 1, 1), (256, 268, 3, 3), (100, 300, 1, 7), (36, 32, 5, 5)], [(512, 512, 3, 3), (68, 20, 1, 1)]])
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+def test_filters_packed_in_one_launch(env, filters, arith):
+    rng = np.random.RandomState(len(filters))
+    calls = []
+    env.gpu_op.set_tensor_arithmetic(arith)
+    try:
+        for K, C, R, S in filters:
+            x, w = rng.randn(2, C, 9, 9).astype(np.float32), rng.randn(K, C, R, S).astype(np.float32)
+            out, cell = env.gpu_op.convolution_2d_forward_get_out_shape(x.shape, w.shape, "NCHW", "SAME", 1, 1)
+            calls.append([env.nd.array(v, env.ctx) for v in (x, w, rng.randn(*out).astype(np.float32), np.zeros(w.shape, np.float32))] + [cell])
+
+        def run(path):
+            env.gpu_op.set_contraction_path(path)
+            results = []
+            for x, w, dy, _, cell in calls:
+                y, dx = env.nd.empty(dy.shape, env.ctx), env.nd.empty(x.shape, env.ctx)
+                env.gpu_op.convolution_2d_forward(x, w, y, cell, env.cudnn, env.stream)
+                env.gpu_op.convolution_backward_data(x, dy, w, dx, cell, env.cudnn, env.stream)
+                results.append((y.asnumpy(), dx.asnumpy()))
+            env.gpu_op.set_contraction_path(0)
+            return results
+        want = run(2)                            # each filter packed on its own
+        for x, w, dy, zero, cell in calls:
+            env.gpu_op.sgd_update(w, zero, 1.0, env.stream)        # a new version of the same values, and its maximum
+        env.gpu_op.pack_filters([c[1] for c in calls], env.gpu_op.cell_array([c[4] for c in calls]), env.stream)
+        got, exact = run(2), run(1)
+        for shape, g, w, e in zip(filters, got, want, exact):
+            for a, b, c in zip(g, w, e):
+                np.testing.assert_array_equal(a, b, err_msg=str(shape))
+                np.testing.assert_allclose(a, c, rtol=1e-4, atol=2e-5 * np.abs(c).max(), err_msg=str(shape))
+    finally:
+        env.gpu_op.set_contraction_path(0)
+        env.gpu_op.set_tensor_arithmetic("3xfp16")

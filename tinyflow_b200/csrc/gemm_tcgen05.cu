@@ -1916,7 +1916,9 @@ __global__ void __launch_bounds__(256) pack_patches_kernel(const float* __restri
 // pad_d].  One launch packs any number of filters: a step's 50-150 filters, packed when their convolution came up, were as
 // many launches of 5 us for 1-2 us of traffic.  A block moves 32 x 32 filters through shared memory, so that the fp32 words are
 // read in order and both layouts are written in rows of 64 bytes; read straight from the filter, the backward-data layout took a
-// sector per element.  Bound by HBM (12 bytes an element) where a launch packs many filters.  Where it packs one (an ordinary step
+// sector per element.  Where a launch packs many filters the instructions bound it before HBM (12 bytes an element) does: rows that lie in
+// one run are read 16 bytes at a time without a division, both layouts are written 16 bytes a thread, and a block of a 1x1 filter
+// takes 288 channels (Inception-v3, 24 million: 126 -> 68 us, 4.2 TB/s; VGG-16 at 15 million 63 -> 37).  Where it packs one (an ordinary step
 // packs each filter when its convolution comes up), by the latency of a block's loads: it takes up to 9 taps, 36 loads a thread
 // one behind the other, unless `tap_step` spreads the taps over more blocks, which read the same sectors again from L2.
 struct FilterJob {
@@ -1940,7 +1942,8 @@ __global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant
   }
   const FilterJob& j = jobs.job[lo];
   const int block = blockIdx.x - j.first_block, kc = block / j.k_blocks;
-  const int k0 = (block - kc * j.k_blocks) * kFilterTile, c0 = kc % j.c_blocks * kFilterTile, t0 = kc / j.c_blocks * jobs.tap_step;
+  const int wide = j.taps == 1 ? jobs.tap_step : 1;            // a 1x1 filter: as many blocks of 32 channels as others have taps
+  const int k0 = (block - kc * j.k_blocks) * kFilterTile, c0 = kc % j.c_blocks * kFilterTile * wide, t0 = kc / j.c_blocks * jobs.tap_step;
   const float sc = j.amax ? scale_from_amax(__ldg(j.amax)) : 1.f;
   if (block == 0 && threadIdx.x == 0) {
     if (j.scale_f) *j.scale_f = sc;
@@ -1949,28 +1952,48 @@ __global__ void __launch_bounds__(256) pack_filters_kernel(const __grid_constant
   }
   const int taps = j.taps, K = j.K, C = j.C, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   E *const hi_f = (E*)j.hi_f, *const lo_f = (E*)j.lo_f, *const hi_d = (E*)j.hi_d, *const lo_d = (E*)j.lo_d;
-  const int nt = min(jobs.tap_step, taps - t0), row = kFilterTile * nt;
-  for (int r = warp; r < kFilterTile; r += 8) {
-    const float* src = j.w + ((long long)(k0 + r) * C + c0) * taps + t0;
-    for (int e = lane; e < row; e += 32) {
-      const int c = e / nt, t = e - c * nt;
-      tile[r][e] = k0 + r < K && c0 + c < C ? __ldg(src + (long long)c * taps + t) * sc : 0.f;
+  const int nt = min(jobs.tap_step, taps - t0), row = kFilterTile * wide * nt;
+  const int there = min(kFilterTile * wide, C - c0) * taps;           // floats of a row of the tile when it holds all taps
+  if (nt == taps && ((uintptr_t)j.w & 15) == 0 && (C * taps & 3) == 0) {        // then they lie in one run, beginning at a multiple of 16 bytes
+    for (int r = warp; r < kFilterTile; r += 8) {
+      const float* src = j.w + ((long long)(k0 + r) * C + c0) * taps;
+      const int n = k0 + r < K ? there : 0;
+#pragma unroll
+      for (int i = 0; i < (kFilterTile * kFilterTaps + 127) / 128; ++i) {
+        const int e = 4 * (lane + 32 * i);
+        if (e >= row) break;
+        const float4 v = e < n ? __ldg(reinterpret_cast<const float4*>(src + e)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        tile[r][e] = v.x * sc; tile[r][e + 1] = v.y * sc; tile[r][e + 2] = v.z * sc; tile[r][e + 3] = v.w * sc;
+      }
+    }
+  } else {
+    for (int r = warp; r < kFilterTile; r += 8) {
+      const float* src = j.w + ((long long)(k0 + r) * C + c0) * taps + t0;
+      for (int e = lane; e < row; e += 32) {
+        const int c = e / nt, t = e - c * nt;
+        tile[r][e] = k0 + r < K && c0 + c < C ? __ldg(src + (long long)c * taps + t) * sc : 0.f;
+      }
     }
   }
   __syncthreads();
-  const int pair = (threadIdx.x & 15) * 2, line0 = threadIdx.x >> 4;
-  for (int line = line0; line < row; line += 16) {
-    const int r = line / nt, t = line - r * nt;
-    E h0, l0, h1, l1;
-    if (hi_f && k0 + r < K && c0 + pair < j.pad_f) {
-      split_pair(tile[r][pair * nt + t], h0, l0); split_pair(tile[r][(pair + 1) * nt + t], h1, l1);
-      const long long at = ((long long)(k0 + r) * taps + t0 + t) * j.pad_f + c0 + pair;
-      store_two(hi_f + at, h0, h1); store_two(lo_f + at, l0, l1);
+  // eight values along the packed dimension a thread: 4 lanes write 64 bytes of a row, lanes of a warp read different banks
+  const int eight = (threadIdx.x & 3) * 8;
+  const int per_row = nt * wide;
+  for (int line = threadIdx.x >> 2; line < row; line += 64) {
+    float v[8];
+    if (hi_f) {
+      const int r = line / per_row, u = line - r * per_row, t = wide > 1 ? 0 : u, c = (wide > 1 ? u * kFilterTile : 0) + eight;
+      if (k0 + r < K && c0 + c < j.pad_f) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) v[e] = tile[r][(c + e) * nt + t];
+        store8(hi_f, lo_f, ((long long)(k0 + r) * taps + t0 + t) * j.pad_f + c0 + c, v);
+      }
     }
-    if (hi_d && c0 + r < C && k0 + pair < j.pad_d) {
-      split_pair(tile[pair][r * nt + t], h0, l0); split_pair(tile[pair + 1][r * nt + t], h1, l1);
-      const long long at = ((long long)(c0 + r) * taps + taps - 1 - t0 - t) * j.pad_d + k0 + pair;
-      store_two(hi_d + at, h0, h1); store_two(lo_d + at, l0, l1);
+    const int r = line / nt, t = line - r * nt;
+    if (hi_d && c0 + r < C && k0 + eight < j.pad_d) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[e] = tile[eight + e][r * nt + t];
+      store8(hi_d, lo_d, ((long long)(c0 + r) * taps + taps - 1 - t0 - t) * j.pad_d + k0 + eight, v);
     }
   }
 }
@@ -2805,16 +2828,17 @@ template <int MAX> static int launch_filter_jobs(FilterJobs<MAX>& jobs, int ar, 
   for (int i = 0; i < jobs.n; ++i) {
     FilterJob& j = jobs.job[i];
     j.k_blocks = (std::max(j.K, j.pad_d) + kFilterTile - 1) / kFilterTile;
-    j.c_blocks = (std::max(j.C, j.pad_f) + kFilterTile - 1) / kFilterTile;
     elems += (double)j.K * j.C * j.taps;
   }
-  // As many taps a block as still give two blocks an SM.
+  // As many taps (1x1: blocks of channels) a block as still give two blocks an SM.
   int blocks = 0;
   for (int step : {kFilterTaps, 3, 1}) {
     jobs.tap_step = step;
     blocks = 0;
     for (int i = 0; i < jobs.n; ++i) {
       FilterJob& j = jobs.job[i];
+      const int channels = kFilterTile * (j.taps == 1 ? step : 1);
+      j.c_blocks = (std::max(j.C, j.pad_f) + channels - 1) / channels;
       j.first_block = blocks;
       blocks += j.k_blocks * j.c_blocks * ((j.taps + step - 1) / step);
     }
