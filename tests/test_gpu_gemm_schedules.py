@@ -57,7 +57,7 @@ def test_reductions_cut_at_common_stages(env, case, arith):
 
 
 # K, C, R, S: enough blocks that a block takes 9 taps, or 288 channels of a 1x1 filter
-@pytest.mark.parametrize("filters", [[(1024, 1160, 1, 1), (640, 1000, 1, 1), (256, 268, 3, 3), (100, 300, 1, 7), (36, 32, 5, 5)], [(512, 512, 3, 3), (68, 20, 1, 1)]])
+@pytest.mark.parametrize("filters", [[(1024, 1160, 1, 1), (640, 1000, 1, 1), (256, 268, 3, 3), (100, 300, 1, 7), (36, 32, 5, 5)], [(512, 512, 3, 3), (260, 100, 1, 1)]])
 @pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
 def test_filters_packed_in_one_launch(env, filters, arith):
     rng = np.random.RandomState(len(filters))
@@ -65,7 +65,7 @@ def test_filters_packed_in_one_launch(env, filters, arith):
     env.gpu_op.set_tensor_arithmetic(arith)
     try:
         for K, C, R, S in filters:
-            x, w = rng.randn(2, C, 9, 9).astype(np.float32), rng.randn(K, C, R, S).astype(np.float32)
+            x, w = rng.randn(2, C, 21, 21).astype(np.float32), rng.randn(K, C, R, S).astype(np.float32)
             out, cell = env.gpu_op.convolution_2d_forward_get_out_shape(x.shape, w.shape, "NCHW", "SAME", 1, 1)
             calls.append([env.nd.array(v, env.ctx) for v in (x, w, rng.randn(*out).astype(np.float32), np.zeros(w.shape, np.float32))] + [cell])
 
@@ -91,3 +91,31 @@ def test_filters_packed_in_one_launch(env, filters, arith):
     finally:
         env.gpu_op.set_contraction_path(0)
         env.gpu_op.set_tensor_arithmetic("3xfp16")
+
+
+# N, C, H, W, K, R, S, padding, stride: rows in one block and in several, windows past the edges, columns that are no multiple of 8
+@pytest.mark.parametrize("case", [(2, 15, 9, 90, 16, 7, 7, "SAME", 1), (5, 3, 33, 47, 64, 3, 3, "SAME", 1), (2, 3, 75, 75, 64, 7, 7, "VALID", 2), (1, 3, 41, 1201, 32, 7, 7, "SAME", 3),
+                                  (9, 1, 40, 41, 32, 5, 5, "SAME", 1), (9, 12, 64, 64, 64, 1, 1, "VALID", 1)])
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+def test_first_layers_as_patches(env, case, arith):
+    N, C, H, W, K, R, S, padding, u = case
+    rng = np.random.RandomState(C + W)
+    x, w = rng.randn(N, C, H, W).astype(np.float32), rng.randn(K, C, R, S).astype(np.float32)
+    out, cell = env.gpu_op.convolution_2d_forward_get_out_shape(x.shape, w.shape, "NCHW", padding, u, u)
+    dy = rng.randn(*out).astype(np.float32)
+
+    def run(path, x, w, dy):
+        X, Wd, DY = (env.nd.array(v, env.ctx) for v in (x, w, dy))
+        y, dw = env.nd.empty(out, env.ctx), env.nd.empty(w.shape, env.ctx)
+        env.gpu_op.set_contraction_path(path)
+        env.gpu_op.set_tensor_arithmetic(arith)
+        try:
+            env.gpu_op.convolution_2d_forward(X, Wd, y, cell, env.cudnn, env.stream)
+            env.gpu_op.convolution_backward_filter(X, DY, Wd, dw, cell, env.cudnn, env.stream)
+        finally:
+            env.gpu_op.set_contraction_path(0)
+            env.gpu_op.set_tensor_arithmetic("3xfp16")
+        return [v.asnumpy().astype(np.float64) for v in (y, dw)]
+
+    for g, e, m in zip(run(2, x, w, dy), run(1, x, w, dy), run(1, np.abs(x), np.abs(w), np.abs(dy))):
+        assert np.all(np.abs(g - e) <= 2e-6 * m + 1e-30), float(np.max(np.abs(g - e) / (m + 1e-30)))
