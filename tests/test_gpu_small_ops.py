@@ -23,6 +23,18 @@ def test_simt_product_at_tile_edges(env, M, K, N, tA, tB):
     assert np.all(np.abs(C.asnumpy() - want) <= 1e-5 * np.abs(want) + 8 * 2.0 ** -24 * mag)
 
 
+# few rows against a million weights and more: runs of K that are not whole, one and several CTAs, 8 and 16 rows, ragged columns
+@pytest.mark.parametrize("M,K,N", [(7, 4608, 4096), (1, 1000, 1004), (9, 25088, 64), (16, 25090, 132), (13, 36, 40004), (3, 8200, 516), (8, 1024, 1024), (2, 2044, 4100)])
+@pytest.mark.parametrize("tB", [False, True])
+def test_few_rows_against_large_weights(env, M, K, N, tB):
+    test_simt_product_at_tile_edges(env, M, K, N, False, tB)
+
+
+@pytest.mark.parametrize("M,K,N", [(1000, 7, 1028), (4100, 16, 260), (1004, 1, 1000), (2052, 9, 516), (36, 8, 40000)])
+def test_weight_gradients_of_few_rows(env, M, K, N):
+    test_simt_product_at_tile_edges(env, M, K, N, True, False)
+
+
 @pytest.mark.parametrize("case", [(3, 1, 28, 28, 6, 5, 5, "SAME"), (5, 6, 14, 14, 16, 5, 5, "VALID"), (2, 3, 9, 7, 5, 3, 3, "SAME"), (300, 2, 8, 8, 3, 7, 7, "SAME"),
                                   (2, 8, 11, 13, 32, 1, 3, "SAME"), (1, 5, 40, 33, 7, 3, 3, "VALID")])
 def test_direct_convolution_of_few_channels(env, case):

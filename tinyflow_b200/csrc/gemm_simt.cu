@@ -9,6 +9,7 @@
 //
 // Measured against the kernel it replaced and against the tensor path: the table in simt_matmul(), where the tile is chosen.
 #include "common.h"
+#include <algorithm>
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
@@ -164,6 +165,213 @@ static cudaError_t launch_simt_layout(const SimtGemm& p, bool a_kfast, bool b_kf
   return b_kfast ? launch_simt<BM, BN, TM, TN, BK, false, true>(p, cluster, s) : launch_simt<BM, BN, TM, TN, BK, false, false>(p, cluster, s);
 }
 
+// ---- a handful of rows against large weights: dense layers on small batches -------------------------------------------------
+// Reading (the weight gradient: writing) the weights once is the bound, and what it takes is enough 16-byte accesses in flight.  Three
+// kernels, one per place of the weights; up to 16 rows stay in registers.  Sums are cut over warps, and over a cluster's CTAs, and added in
+// a fixed order.  7 rows against 4608 x 4096 and 4096 x 4096 weights (11.6 and 10.3 us at the copy rate), each: product 22.5 us, gradient of
+// the rows 33.7, gradient of the weights 16.3 (the tiles above: 30.5, 44.5 and 24.2).  The first two still wait for memory: 3.1 and 2.0 TB/s.
+//
+// C = A[M x K] B[K x N]: a lane owns 4 columns, a warp a run of K, 8 rows of B in flight; the rows of A lie in shared memory.
+// (With 16 rows in flight a block took so many registers that an SM held one: 46 us.)
+constexpr int kRowThreads = 256, kRowWarps = kRowThreads / 32, kRowCols = 128;
+template <int MR>
+__global__ void __launch_bounds__(kRowThreads) rows_nn_kernel(const SimtGemm p) {
+  extern __shared__ __align__(16) float rows_smem[];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kw = p.k_per_cta / kRowWarps, seg = p.k_per_cta;
+  grid_dep_sync();
+  const int kbeg = rank * seg, count = max(0, min(seg, p.K - kbeg));
+  for (int m = warp; m < MR; m += kRowWarps)
+    for (int k = lane; k < seg; k += 32) {
+      const bool there = m < p.M && k < count;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(rows_smem + m * seg + k)),
+                   "l"(p.A + (there ? (long long)m * p.lda + kbeg + k : 0)), "r"(there ? 4 : 0) : "memory");
+    }
+  const int n = (int)(blockIdx.x / ranks) * kRowCols + lane * 4, k1 = min((warp + 1) * kw, count);
+  float4 w[8];
+  auto fetch = [&](int k) {
+    const float* const b = p.B + (long long)(kbeg + k) * p.ldb + n;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = n < p.N && k + j < k1 ? __ldg(reinterpret_cast<const float4*>(b + j * p.ldb)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  };
+  fetch(warp * kw);                      // the first rows of B come with those of A
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  float2 acc[MR][2];
+#pragma unroll
+  for (int m = 0; m < MR; ++m) acc[m][0] = acc[m][1] = make_float2(0.f, 0.f);
+  for (int k = warp * kw; k < k1; k += 8) {
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+      const float4 x0 = *reinterpret_cast<const float4*>(rows_smem + m * seg + k), x1 = *reinterpret_cast<const float4*>(rows_smem + m * seg + k + 4);
+      const float x[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float2 xx = make_float2(x[j], x[j]);
+        acc[m][0] = __ffma2_rn(xx, make_float2(w[j].x, w[j].y), acc[m][0]);
+        acc[m][1] = __ffma2_rn(xx, make_float2(w[j].z, w[j].w), acc[m][1]);
+      }
+    }
+    if (k + 8 < k1) fetch(k + 8);
+  }
+  __syncthreads();                       // the rows are done with
+  float4* const part = reinterpret_cast<float4*>(rows_smem);               // [warp][MR][32 lanes]
+#pragma unroll
+  for (int m = 0; m < MR; ++m) part[(warp * MR + m) * 32 + lane] = make_float4(acc[m][0].x, acc[m][0].y, acc[m][1].x, acc[m][1].y);
+  __syncthreads();
+  auto add = [](float4& a, const float4 b) { a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w; };
+  auto store = [&](int i, const float4 v) {
+    const int m = i >> 5, c = (int)(blockIdx.x / ranks) * kRowCols + (i & 31) * 4;
+    if (m >= p.M || c >= p.N) return;
+    float* const dst = p.C + (long long)m * p.ldc + c;
+    if (p.c_vec) *reinterpret_cast<float4*>(dst) = v;
+    else { dst[0] = v.x; dst[1] = v.y; dst[2] = v.z; dst[3] = v.w; }
+  };
+  for (int i = threadIdx.x; i < MR * 32; i += kRowThreads) {
+    float4 t = part[i];
+#pragma unroll
+    for (int w = 1; w < kRowWarps; ++w) add(t, part[w * MR * 32 + i]);
+    if (ranks == 1) store(i, t); else part[i] = t;
+  }
+  if (ranks == 1) return;
+  cluster.sync();
+  for (int i = rank * kRowThreads + threadIdx.x; i < MR * 32; i += ranks * kRowThreads) {
+    float4 t = *cluster.map_shared_rank(part + i, 0);
+    for (int r = 1; r < ranks; ++r) add(t, *cluster.map_shared_rank(part + i, r));
+    store(i, t);
+  }
+  cluster.sync();           // nobody leaves while its shared memory is still read
+}
+
+// C = A[M x K] B[N x K]^T: a warp owns two rows of B along a run of K, a lane 4 columns at a time; the rows of A come through L1.
+// (Four rows a warp halve those reads and take registers: the same time.)
+constexpr int kRowSet = 2;
+template <int MR>
+__global__ void __launch_bounds__(kRowThreads) rows_nt_kernel(const SimtGemm p) {
+  constexpr int kSums = MR * kRowSet;
+  __shared__ float part[kRowWarps][kSums];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, runs = (p.K + p.k_per_cta - 1) / p.k_per_cta;       // of K, neighbouring warps
+  grid_dep_sync();
+  const int set = ((int)blockIdx.x * kRowWarps + warp) / runs, run = warp % runs, n0 = set * kRowSet;
+  const int kend = min(p.K, (run + 1) * p.k_per_cta);
+  float2 acc[kSums];
+#pragma unroll
+  for (int i = 0; i < kSums; ++i) acc[i] = make_float2(0.f, 0.f);
+  const float* const b0 = p.B + (long long)min(n0, p.N - 1) * p.ldb;
+  const float* const b1 = p.B + (long long)min(n0 + 1, p.N - 1) * p.ldb;
+#pragma unroll 4
+  for (int k = run * p.k_per_cta + lane * 4; k < kend; k += 128) {
+    const float4 w[kRowSet] = {__ldg(reinterpret_cast<const float4*>(b0 + k)), __ldg(reinterpret_cast<const float4*>(b1 + k))};
+#pragma unroll
+    for (int m = 0; m < MR; ++m) {
+      const float4 x = __ldg(reinterpret_cast<const float4*>(p.A + (long long)min(m, p.M - 1) * p.lda + k));
+#pragma unroll
+      for (int r = 0; r < kRowSet; ++r) {
+        float2& a = acc[m * kRowSet + r];
+        a = __ffma2_rn(make_float2(x.z, x.w), make_float2(w[r].z, w[r].w), __ffma2_rn(make_float2(x.x, x.y), make_float2(w[r].x, w[r].y), a));
+      }
+    }
+  }
+  float sum[kSums];
+#pragma unroll
+  for (int i = 0; i < kSums; ++i) sum[i] = acc[i].x + acc[i].y;
+  // kSums sums over 32 lanes: a step adds pairs of lanes and halves what each keeps, lane i ends up with sum i
+  if (kSums == 16) {
+#pragma unroll
+    for (int i = 0; i < kSums; ++i) sum[i] += __shfl_xor_sync(0xffffffffu, sum[i], 16);
+  }
+#pragma unroll
+  for (int step = kSums / 2; step > 0; step /= 2)
+#pragma unroll
+    for (int i = 0; i < step; ++i) {
+      const bool upper = lane & step;
+      const float keep = upper ? sum[i + step] : sum[i], give = upper ? sum[i] : sum[i + step];
+      sum[i] = keep + __shfl_xor_sync(0xffffffffu, give, step);
+    }
+  if (lane < kSums) part[warp][lane] = sum[0];
+  __syncthreads();
+  if (run != 0 || lane >= kSums) return;
+  float t = part[warp][lane];
+  for (int r = 1; r < runs; ++r) t += part[warp + r][lane];
+  const int m = lane / kRowSet, n = n0 + lane % kRowSet;
+  if (m < p.M && n < p.N) p.C[(long long)m * p.ldc + n] = t;
+}
+
+// C = A[K x M]^T B[K x N] of at most KR rows: a thread keeps its 4 columns of B and writes them times one row of A^T after the other.
+constexpr int kOuterRows = 32;
+template <int KR>
+__global__ void __launch_bounds__(kRowThreads) rows_tn_kernel(const SimtGemm p) {
+  grid_dep_sync();
+  const int n = ((int)blockIdx.x * kRowThreads + threadIdx.x) * 4, m0 = blockIdx.y * kOuterRows;
+  if (n >= p.N) return;
+  float4 b[KR];
+#pragma unroll
+  for (int k = 0; k < KR; ++k) b[k] = k < p.K ? __ldg(reinterpret_cast<const float4*>(p.B + (long long)k * p.ldb + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int m1 = min(p.M, m0 + kOuterRows);
+  for (int m = m0; m < m1; m += 4) {
+    float4 out[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) out[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      if (k >= p.K) break;
+      const float4 a4 = __ldg(reinterpret_cast<const float4*>(p.A + (long long)k * p.lda + m));
+      const float a[4] = {a4.x, a4.y, a4.z, a4.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        out[j].x = fmaf(a[j], b[k].x, out[j].x); out[j].y = fmaf(a[j], b[k].y, out[j].y);
+        out[j].z = fmaf(a[j], b[k].z, out[j].z); out[j].w = fmaf(a[j], b[k].w, out[j].w);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) *reinterpret_cast<float4*>(p.C + (long long)(m + j) * p.ldc + n) = out[j];
+  }
+}
+
+// Takes the product if it is one of those: 1, 0 if not, -1 on error.  Below a million weights, or where these leave SMs without a block
+// (2048 x 1000: 13.4 us against 9.3), the tiles are faster; rows that cannot be read 16 bytes at a time stay with them, too.
+constexpr int kFewRows = 16;
+constexpr size_t kRowSmem = 200 * 1024;
+template <int MR> static int launch_rows_nn(SimtGemm p, cudaStream_t s) {
+  const int sms = device_sm_count(), groups = (p.N + kRowCols - 1) / kRowCols;
+  int cluster = 1;
+  auto smem = [&] { return std::max((size_t)p.k_per_cta * MR, (size_t)kRowWarps * MR * kRowCols) * sizeof(float); };
+  auto cut = [&] { p.k_per_cta = (int)(((long long)p.K + cluster * kRowWarps * 8 - 1) / (cluster * kRowWarps * 8)) * kRowWarps * 8; };        // a warp's run is a multiple of 8
+  cut();
+  while (cluster < 8 && (groups * cluster < 2 * sms || smem() > kRowSmem / 2) && p.K >= 64 * kRowWarps * cluster) { cluster *= 2; cut(); }
+  if (smem() > kRowSmem || groups * cluster < sms) return 0;
+  static const cudaError_t attr = cudaFuncSetAttribute(rows_nn_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmem);
+  TF_CUDA(attr);
+  TF_CUDA(launch_cluster(rows_nn_kernel<MR>, cluster, dim3(groups * cluster), dim3(kRowThreads), smem(), s, p));
+  return 1;
+}
+static int rows_matmul(const SimtGemm& p, bool tA, bool tB, cudaStream_t s) {
+  const int sms = device_sm_count();
+  if (!tA && p.M <= kFewRows && (double)p.K * p.N >= 1e6) {
+    if (!tB && p.b_vec && p.N % 4 == 0) return p.M <= 8 ? launch_rows_nn<8>(p, s) : launch_rows_nn<16>(p, s);
+    if (tB && p.a_vec && p.b_vec && p.K % 4 == 0) {
+      const long long sets = (p.N + kRowSet - 1) / kRowSet;
+      int runs = 1;
+      while (runs < kRowWarps && sets * runs < 24ll * sms && p.K >= 256 * runs) runs *= 2;
+      if (sets * runs < 8ll * sms) return 0;
+      SimtGemm q = p;
+      q.k_per_cta = (int)(((p.K + runs - 1) / runs + 127) / 128 * 128);
+      runs = (p.K + q.k_per_cta - 1) / q.k_per_cta;
+      while (kRowWarps % runs) { q.k_per_cta += 128; runs = (p.K + q.k_per_cta - 1) / q.k_per_cta; }       // whole sets in a block
+      const dim3 grid((unsigned)((sets * runs + kRowWarps - 1) / kRowWarps));
+      TF_CUDA(p.M <= 8 ? launch_dep(rows_nt_kernel<8>, grid, dim3(kRowThreads), 0, s, q) : launch_dep(rows_nt_kernel<16>, grid, dim3(kRowThreads), 0, s, q));
+      return 1;
+    }
+  }
+  if (tA && !tB && p.K <= kFewRows && (double)p.M * p.N >= 1e6 && p.a_vec && p.b_vec && p.c_vec && p.M % 4 == 0 && p.N % 4 == 0 && (p.M + kOuterRows - 1) / kOuterRows <= 65535) {
+    const dim3 grid((p.N + 4 * kRowThreads - 1) / (4 * kRowThreads), (p.M + kOuterRows - 1) / kOuterRows);
+    TF_CUDA(p.K <= 8 ? launch_dep(rows_tn_kernel<8>, grid, dim3(kRowThreads), 0, s, p) : launch_dep(rows_tn_kernel<16>, grid, dim3(kRowThreads), 0, s, p));
+    return 1;
+  }
+  return 0;
+}
+
 // C[M x N] = op(A) op(B), row-major, leading dimensions of the arrays as they are stored.
 int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, cudaStream_t s, const char* what) {
   if (M <= 0 || N <= 0) return 0;
@@ -189,6 +397,11 @@ int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int6
   p.k_per_cta = (int)(((K + cluster - 1) / cluster + bk - 1) / bk * bk);
   note_compute_stream(s);
   KernelTimer kt("simt_gemm", s, 2.0 * (double)M * (double)N * (double)K, 0, 1);
+  if (const int rc = rows_matmul(p, tA, tB, s)) {
+    if (rc < 0) return -1;
+    TF_AFTER(s, what);
+    return 0;
+  }
   const cudaError_t e = cfg == 0 ? launch_simt_layout<8, 64, 8, 1, 32>(p, !tA, tB, cluster, s)
                       : cfg == 1 ? launch_simt_layout<32, 32, 4, 2, 32>(p, !tA, tB, cluster, s)
                                  : launch_simt_layout<64, 64, 4, 4, 16>(p, !tA, tB, cluster, s);
