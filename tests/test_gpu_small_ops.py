@@ -211,3 +211,17 @@ def test_products_of_two_threads(env, streams):
         want = state[k][2][0].asnumpy()
         for c in state[k][2][1:]:
             np.testing.assert_array_equal(c.asnumpy(), want)
+
+
+# The batches at which the number of sample groups and the samples of each change; features in whole and in ragged vectors.  (Not a
+# batch of 2: there dx = inv * (g - mean(g) - xhat * mean(g * xhat)) cancels to eps / var ~ 1e-5 of its terms, whose fp32 rounding of
+# 2^-24 is then 6e-3 of the result.)
+@pytest.mark.parametrize("N", [5, 16, 17, 32, 33])
+@pytest.mark.parametrize("plane", [(4, 5, 7), (3, 2, 7), (5, 3, 3)])
+def test_batchnorm_at_group_edges(env, N, plane):
+    from tests.test_gpu_ops import test_batchnorm, test_relu_backward_runs_inside_the_batchnorm_backward_that_follows as fused
+    test_batchnorm(env, (N,) + plane, "pre_activation")
+    if np.prod(plane) % 2 == 0:
+        plane = (plane[0] * 2 ** 11 // N // 2 * 2,) + plane[1:]          # held back from 64 K elements on
+        fused(env, (N,) + plane, True)
+        fused(env, (N,) + plane, False)

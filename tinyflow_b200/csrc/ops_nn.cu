@@ -2,6 +2,7 @@
 // tensor is read once and written once; statistics are reduced in registers / warp shuffles.
 #include "common.h"
 #include <math.h>
+#include <type_traits>
 
 namespace tf {
 
@@ -402,21 +403,22 @@ template <bool MAXPOOL> static void launch_pool_gather(const PoolPlan* p, const 
 // pass, so x (and dy) cross HBM exactly once.
 // =====================================================================================
 constexpr float kBnEps = 1e-5f;
-constexpr int kBnMaxBatchInRegs = 64;     // = kBnGroups * kBnPerThread
 
 template <int VEC> struct VecT;
 template <> struct VecT<1> { using type = float; };
 template <> struct VecT<2> { using type = float2; };
 template <> struct VecT<4> { using type = float4; };
 
-// Block = 32 feature vectors x kBnGroups sample groups.  Thread (tx, ty) owns feature vector fv0 + tx and the
-// samples ty, ty + kBnGroups, ...: each warp reads 32 consecutive feature vectors of one sample (coalesced),
-// every thread keeps only N / kBnGroups values per tensor in registers, and the per-feature sums are combined
-// across the sample groups through shared memory.
-constexpr int kBnGroups = 8;
-constexpr int kBnPerThread = 8;          // covers batches up to 64
+// Block = 32 feature vectors x G sample groups.  Thread (tx, ty) owns feature vector fv0 + tx and the
+// samples ty, ty + G, ...: each warp reads 32 consecutive feature vectors of one sample (coalesced),
+// every thread keeps only its PER samples per tensor in registers, and the per-feature sums are combined
+// across the sample groups through shared memory.  Bound by HBM while enough loads are in flight, so registers decide: 4 or 8 groups of
+// 4 samples for batches up to 16 and 32 (with room for 64 samples, half of it idle, and therefore 8-byte vectors backward,
+// DenseNet-121 at batch 32 spent 2.27 ms a step in the fused backward, now 1.62; ResNet-50 at batch 19 0.61, now 0.46), 8 of 8 up to 64 (16 of
+// 4: forward of ResNet-50 1.03 -> 1.49 ms).
+constexpr int kBnMaxBatchInRegs = 64;
 
-template <int VEC>
+template <int VEC, int G>
 __device__ __forceinline__ void bn_group_sum(float (&part)[VEC], float (*red)[32][VEC], int tx, int ty) {
 #pragma unroll
   for (int k = 0; k < VEC; ++k) red[ty][tx][k] = part[k];
@@ -425,27 +427,27 @@ __device__ __forceinline__ void bn_group_sum(float (&part)[VEC], float (*red)[32
   for (int k = 0; k < VEC; ++k) {
     float t = 0.f;
 #pragma unroll
-    for (int g = 0; g < kBnGroups; ++g) t += red[g][tx][k];
+    for (int g = 0; g < G; ++g) t += red[g][tx][k];
     part[k] = t;
   }
   __syncthreads();
 }
 
-template <int VEC>
-__global__ void __launch_bounds__(32 * kBnGroups) bn_pa_fwd_regs_kernel(const float* __restrict__ x, float* __restrict__ y, float* __restrict__ save_mean, float* __restrict__ save_inv, int N, int64_t F, AmaxOut am) {
+template <int VEC, int G, int PER>
+__global__ void __launch_bounds__(32 * G) bn_pa_fwd_regs_kernel(const float* __restrict__ x, float* __restrict__ y, float* __restrict__ save_mean, float* __restrict__ save_inv, int N, int64_t F, AmaxOut am) {
   grid_dep_sync();
   using V = typename VecT<VEC>::type;
-  __shared__ float red[kBnGroups][32][VEC];
+  __shared__ float red[G][32][VEC];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t FV = F / VEC;
   const int64_t fv = (int64_t)blockIdx.x * 32 + tx;
   const bool live = fv < FV;
   const V* xv = reinterpret_cast<const V*>(x);
   V* yv = reinterpret_cast<V*>(y);
-  float v[kBnPerThread][VEC];
+  float v[PER][VEC];
 #pragma unroll
-  for (int i = 0; i < kBnPerThread; ++i) {
-    int n = ty + i * kBnGroups;
+  for (int i = 0; i < PER; ++i) {
+    int n = ty + i * G;
     V t = {};
     if (live && n < N) t = xv[(int64_t)n * FV + fv];
     const float* tp = reinterpret_cast<const float*>(&t);
@@ -458,19 +460,19 @@ __global__ void __launch_bounds__(32 * kBnGroups) bn_pa_fwd_regs_kernel(const fl
   for (int k = 0; k < VEC; ++k) {
     float s = 0.f;
 #pragma unroll
-    for (int i = 0; i < kBnPerThread; ++i) s += v[i][k];       // missing samples were loaded as 0
+    for (int i = 0; i < PER; ++i) s += v[i][k];       // missing samples were loaded as 0
     mean[k] = s;
   }
-  bn_group_sum<VEC>(mean, red, tx, ty);
+  bn_group_sum<VEC, G>(mean, red, tx, ty);
 #pragma unroll
   for (int k = 0; k < VEC; ++k) {
     mean[k] *= rn;
     float q = 0.f;
 #pragma unroll
-    for (int i = 0; i < kBnPerThread; ++i) { float d = v[i][k] - mean[k]; if (ty + i * kBnGroups < N) q += d * d; }
+    for (int i = 0; i < PER; ++i) { float d = v[i][k] - mean[k]; if (ty + i * G < N) q += d * d; }
     inv[k] = q;
   }
-  bn_group_sum<VEC>(inv, red, tx, ty);
+  bn_group_sum<VEC, G>(inv, red, tx, ty);
 #pragma unroll
   for (int k = 0; k < VEC; ++k) {
     float a = inv[k] * rn + kBnEps;
@@ -479,8 +481,8 @@ __global__ void __launch_bounds__(32 * kBnGroups) bn_pa_fwd_regs_kernel(const fl
   }
   uint32_t amax = 0;
 #pragma unroll
-  for (int i = 0; i < kBnPerThread; ++i) {
-    int n = ty + i * kBnGroups;
+  for (int i = 0; i < PER; ++i) {
+    int n = ty + i * G;
     if (live && n < N) {
       V t;
       float* tp = reinterpret_cast<float*>(&t);
@@ -496,11 +498,11 @@ __global__ void __launch_bounds__(32 * kBnGroups) bn_pa_fwd_regs_kernel(const fl
   amax_commit(am, amax);        // max|y|: the activation that follows can pack its output for the next convolution in its own pass
 }
 
-template <int VEC>
-__global__ void __launch_bounds__(32 * kBnGroups) bn_pa_bwd_regs_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dx, const float* __restrict__ save_mean, const float* __restrict__ save_inv, int N, int64_t F, AmaxOut am) {
+template <int VEC, int G, int PER>
+__global__ void __launch_bounds__(32 * G) bn_pa_bwd_regs_kernel(const float* __restrict__ x, const float* __restrict__ dy, float* __restrict__ dx, const float* __restrict__ save_mean, const float* __restrict__ save_inv, int N, int64_t F, AmaxOut am) {
   grid_dep_sync();
   using V = typename VecT<VEC>::type;
-  __shared__ float red[kBnGroups][32][VEC];
+  __shared__ float red[G][32][VEC];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t FV = F / VEC;
   const int64_t fv = (int64_t)blockIdx.x * 32 + tx;
@@ -511,10 +513,10 @@ __global__ void __launch_bounds__(32 * kBnGroups) bn_pa_bwd_regs_kernel(const fl
   float m[VEC], inv[VEC];
 #pragma unroll
   for (int k = 0; k < VEC; ++k) { m[k] = live ? save_mean[fv * VEC + k] : 0.f; inv[k] = live ? save_inv[fv * VEC + k] : 0.f; }
-  float xh[kBnPerThread][VEC], g[kBnPerThread][VEC];
+  float xh[PER][VEC], g[PER][VEC];
 #pragma unroll
-  for (int i = 0; i < kBnPerThread; ++i) {
-    int n = ty + i * kBnGroups;
+  for (int i = 0; i < PER; ++i) {
+    int n = ty + i * G;
     V a = {}, b = {};
     if (live && n < N) { a = xv[(int64_t)n * FV + fv]; b = gv[(int64_t)n * FV + fv]; }
     const float* ap = reinterpret_cast<const float*>(&a);
@@ -527,16 +529,16 @@ __global__ void __launch_bounds__(32 * kBnGroups) bn_pa_bwd_regs_kernel(const fl
   for (int k = 0; k < VEC; ++k) {
     float a = 0.f, b = 0.f;
 #pragma unroll
-    for (int i = 0; i < kBnPerThread; ++i) { a += g[i][k]; b += g[i][k] * xh[i][k]; }
+    for (int i = 0; i < PER; ++i) { a += g[i][k]; b += g[i][k] * xh[i][k]; }
     s1[k] = a; s2[k] = b;
   }
-  bn_group_sum<VEC>(s1, red, tx, ty);
-  bn_group_sum<VEC>(s2, red, tx, ty);
+  bn_group_sum<VEC, G>(s1, red, tx, ty);
+  bn_group_sum<VEC, G>(s2, red, tx, ty);
   const float rn = 1.f / (float)N;
   uint32_t amax = 0;
 #pragma unroll
-  for (int i = 0; i < kBnPerThread; ++i) {
-    int n = ty + i * kBnGroups;
+  for (int i = 0; i < PER; ++i) {
+    int n = ty + i * G;
     if (live && n < N) {
       V t;
       float* tp = reinterpret_cast<float*>(&t);
@@ -552,11 +554,11 @@ __global__ void __launch_bounds__(32 * kBnGroups) bn_pa_bwd_regs_kernel(const fl
 // to dg: other consumers of that tensor may exist) and the batch-norm's incoming gradient.  XHAT_MASK: the ReLU's input
 // is this layer's own forward output, which equals x-hat bit for bit (same subtraction and product of the same saved
 // statistics), so the mask tensor is not read at all.
-template <int VEC, bool XHAT_MASK>
-__global__ void __launch_bounds__(32 * kBnGroups) bn_pa_bwd_relu_regs_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ mask, float* __restrict__ dg, float* __restrict__ dx, const float* __restrict__ save_mean, const float* __restrict__ save_inv, int N, int64_t F, AmaxOut am) {
+template <int VEC, int G, int PER, bool XHAT_MASK>
+__global__ void __launch_bounds__(32 * G) bn_pa_bwd_relu_regs_kernel(const float* __restrict__ x, const float* __restrict__ dy, const float* __restrict__ mask, float* __restrict__ dg, float* __restrict__ dx, const float* __restrict__ save_mean, const float* __restrict__ save_inv, int N, int64_t F, AmaxOut am) {
   grid_dep_sync();
   using V = typename VecT<VEC>::type;
-  __shared__ float red[kBnGroups][32][VEC];
+  __shared__ float red[G][32][VEC];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int64_t FV = F / VEC;
   const int64_t fv = (int64_t)blockIdx.x * 32 + tx;
@@ -569,10 +571,10 @@ __global__ void __launch_bounds__(32 * kBnGroups) bn_pa_bwd_relu_regs_kernel(con
   float m[VEC], inv[VEC];
 #pragma unroll
   for (int k = 0; k < VEC; ++k) { m[k] = live ? save_mean[fv * VEC + k] : 0.f; inv[k] = live ? save_inv[fv * VEC + k] : 0.f; }
-  float xh[kBnPerThread][VEC], g[kBnPerThread][VEC];
+  float xh[PER][VEC], g[PER][VEC];
 #pragma unroll
-  for (int i = 0; i < kBnPerThread; ++i) {
-    const int n = ty + i * kBnGroups;
+  for (int i = 0; i < PER; ++i) {
+    const int n = ty + i * G;
     const bool on = live && n < N;
     V a = {}, b = {}, r = {};
     if (on) {
@@ -598,16 +600,16 @@ __global__ void __launch_bounds__(32 * kBnGroups) bn_pa_bwd_relu_regs_kernel(con
   for (int k = 0; k < VEC; ++k) {
     float a = 0.f, b = 0.f;
 #pragma unroll
-    for (int i = 0; i < kBnPerThread; ++i) { a += g[i][k]; b += g[i][k] * xh[i][k]; }
+    for (int i = 0; i < PER; ++i) { a += g[i][k]; b += g[i][k] * xh[i][k]; }
     s1[k] = a; s2[k] = b;
   }
-  bn_group_sum<VEC>(s1, red, tx, ty);
-  bn_group_sum<VEC>(s2, red, tx, ty);
+  bn_group_sum<VEC, G>(s1, red, tx, ty);
+  bn_group_sum<VEC, G>(s2, red, tx, ty);
   const float rn = 1.f / (float)N;
   uint32_t amax = 0;
 #pragma unroll
-  for (int i = 0; i < kBnPerThread; ++i) {
-    int n = ty + i * kBnGroups;
+  for (int i = 0; i < PER; ++i) {
+    int n = ty + i * G;
     if (live && n < N) {
       V t;
       float* tp = reinterpret_cast<float*>(&t);
@@ -678,28 +680,49 @@ __global__ void __launch_bounds__(512) bn_sp_bwd_kernel(const float* __restrict_
   for (int64_t i = threadIdx.x; i < cnt; i += blockDim.x) { int64_t o = ((i / HW) * C + c) * HW + i % HW; dx[o] = inv * (dy[o] - s1 - (x[o] - m) * inv * s2); }
 }
 
+// calls launch(G, PER) with the number of sample groups and the samples of each
+template <class F> static void with_bn_groups(int N, F&& launch) {
+  if (N <= 16) launch(std::integral_constant<int, 4>(), std::integral_constant<int, 4>());
+  else if (N <= 32) launch(std::integral_constant<int, 8>(), std::integral_constant<int, 4>());
+  else launch(std::integral_constant<int, 8>(), std::integral_constant<int, 8>());
+}
+static dim3 bn_grid(int64_t F, int vec) { return dim3((unsigned)((F / vec + 31) / 32)); }
 static void launch_bn_fwd_regs(const float* x, float* y, float* sm, float* si, int N, int64_t F, cudaStream_t s) {
   AmaxOut am = amax_track_begin(y);
-  if (F % 4 == 0 && aligned16(x) && aligned16(y)) launch_dep(bn_pa_fwd_regs_kernel<4>, dim3((unsigned)((F / 4 + 31) / 32)), dim3(32 * kBnGroups), 0, s, x, y, sm, si, N, F, am);
-  else launch_dep(bn_pa_fwd_regs_kernel<1>, dim3((unsigned)((F + 31) / 32)), dim3(32 * kBnGroups), 0, s, x, y, sm, si, N, F, am);
+  with_bn_groups(N, [&](auto g, auto per) {
+    constexpr int G = decltype(g)::value, PER = decltype(per)::value;
+    if (F % 4 == 0 && aligned16(x) && aligned16(y)) launch_dep(bn_pa_fwd_regs_kernel<4, G, PER>, bn_grid(F, 4), dim3(32 * G), 0, s, x, y, sm, si, N, F, am);
+    else launch_dep(bn_pa_fwd_regs_kernel<1, G, PER>, bn_grid(F, 1), dim3(32 * G), 0, s, x, y, sm, si, N, F, am);
+  });
 }
+// Widest vectors of the backward kernels: with 8 samples a thread the 16-byte variant holds 2 x 8 x 4 values (126 registers, two
+// blocks per SM) and its load / reduce / store phases overlap too little; with half the registers three blocks fit (1.89 -> 1.77 ms per
+// ResNet-50 step at batch 64)
+template <int PER> constexpr int kBnBwdVec = PER > 4 ? 2 : 4;
 static void launch_bn_bwd_regs(const float* x, const float* dy, float* dx, const float* sm, const float* si, int N, int64_t F, cudaStream_t s) {
   AmaxOut am = amax_track_begin(dx);          // dx is the output gradient of the convolution in front of this layer
-  // 8-byte vectors: the 16-byte variant holds 2 x 8 x 4 values per thread (126 registers, two blocks per SM) and its
-  // load / reduce / store phases overlap too little; with half the registers three blocks fit (1.89 -> 1.77 ms per
-  // ResNet-50 step)
-  if (F % 2 == 0 && aligned16(x) && aligned16(dy) && aligned16(dx)) launch_dep(bn_pa_bwd_regs_kernel<2>, dim3((unsigned)((F / 2 + 31) / 32)), dim3(32 * kBnGroups), 0, s, x, dy, dx, sm, si, N, F, am);
-  else if (F % 4 == 0 && aligned16(x) && aligned16(dy) && aligned16(dx)) launch_dep(bn_pa_bwd_regs_kernel<4>, dim3((unsigned)((F / 4 + 31) / 32)), dim3(32 * kBnGroups), 0, s, x, dy, dx, sm, si, N, F, am);
-  else launch_dep(bn_pa_bwd_regs_kernel<1>, dim3((unsigned)((F + 31) / 32)), dim3(32 * kBnGroups), 0, s, x, dy, dx, sm, si, N, F, am);
+  const bool aligned = aligned16(x) && aligned16(dy) && aligned16(dx);
+  with_bn_groups(N, [&](auto g, auto per) {
+    constexpr int G = decltype(g)::value, PER = decltype(per)::value, V = kBnBwdVec<PER>;
+    if (F % V == 0 && aligned) launch_dep(bn_pa_bwd_regs_kernel<V, G, PER>, bn_grid(F, V), dim3(32 * G), 0, s, x, dy, dx, sm, si, N, F, am);
+    else if (F % 2 == 0 && aligned) launch_dep(bn_pa_bwd_regs_kernel<2, G, PER>, bn_grid(F, 2), dim3(32 * G), 0, s, x, dy, dx, sm, si, N, F, am);
+    else launch_dep(bn_pa_bwd_regs_kernel<1, G, PER>, bn_grid(F, 1), dim3(32 * G), 0, s, x, dy, dx, sm, si, N, F, am);
+  });
 }
 // The fused pair (a held-back ReLU backward and this batch-norm backward).  Returns false when the operands do not allow
 // 8-byte vectors; the caller then runs the two kernels one after the other.
+template <bool XHAT_MASK> static void launch_bn_bwd_relu_of(const float* x, const float* dy, const float* mask, float* dg, float* dx, const float* sm, const float* si, int N, int64_t F, AmaxOut am, cudaStream_t s) {
+  with_bn_groups(N, [&](auto g, auto per) {
+    constexpr int G = decltype(g)::value, PER = decltype(per)::value, V = kBnBwdVec<PER>;
+    if (F % V == 0) launch_dep(bn_pa_bwd_relu_regs_kernel<V, G, PER, XHAT_MASK>, bn_grid(F, V), dim3(32 * G), 0, s, x, dy, mask, dg, dx, sm, si, N, F, am);
+    else launch_dep(bn_pa_bwd_relu_regs_kernel<2, G, PER, XHAT_MASK>, bn_grid(F, 2), dim3(32 * G), 0, s, x, dy, mask, dg, dx, sm, si, N, F, am);
+  });
+}
 static bool launch_bn_bwd_relu_regs(const float* x, const float* dy, const float* mask, bool xhat_mask, float* dg, float* dx, const float* sm, const float* si, int N, int64_t F, cudaStream_t s) {
   if (!(F % 2 == 0 && aligned16(x) && aligned16(dy) && aligned16(mask) && aligned16(dg) && aligned16(dx))) return false;
   AmaxOut am = amax_track_begin(dx);
-  const dim3 grid((unsigned)((F / 2 + 31) / 32)), block(32 * kBnGroups);
-  if (xhat_mask) launch_dep(bn_pa_bwd_relu_regs_kernel<2, true>, grid, block, 0, s, x, dy, mask, dg, dx, sm, si, N, F, am);
-  else launch_dep(bn_pa_bwd_relu_regs_kernel<2, false>, grid, block, 0, s, x, dy, mask, dg, dx, sm, si, N, F, am);
+  if (xhat_mask) launch_bn_bwd_relu_of<true>(x, dy, mask, dg, dx, sm, si, N, F, am, s);
+  else launch_bn_bwd_relu_of<false>(x, dy, mask, dg, dx, sm, si, N, F, am, s);
   return true;
 }
 static std::atomic<long long> g_fused_relu_bn_bwd{0};
