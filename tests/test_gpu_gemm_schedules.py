@@ -119,3 +119,10 @@ def test_first_layers_as_patches(env, case, arith):
 
     for g, e, m in zip(run(2, x, w, dy), run(1, x, w, dy), run(1, np.abs(x), np.abs(w), np.abs(dy))):
         assert np.all(np.abs(g - e) <= 2e-6 * m + 1e-30), float(np.max(np.abs(g - e) / (m + 1e-30)))
+
+
+@pytest.mark.parametrize("case", [(8, 64, 32, 32, 128, 1, 1, "VALID"), (33, 64, 16, 16, 192, 1, 1, "VALID"),       # 64 and 66 wide tiles
+                                  (2, 2048, 8, 8, 132, 1, 1, "VALID"), (2, 2112, 8, 8, 132, 1, 1, "VALID"), (2, 224, 9, 9, 100, 3, 3, "SAME")])      # 32, 33 and 36 stages
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+def test_narrow_tiles_of_short_reductions(env, case, arith):
+    test_convolution_schedules(env, case, arith)

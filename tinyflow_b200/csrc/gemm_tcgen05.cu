@@ -412,6 +412,7 @@ struct alignas(128) GemmParams {
   int slot, taps_per_tile, slots_per_tap;
   double operand_bytes;           // of A and B together (host side)
   int group_iters;                // stages accumulated in TMEM before the epilogue promotes them to registers
+  int group_limit;                // most stages of a group, 0: no limit of the launch's own (host side)
   int data_by_data;               // both operands are activations / gradients (filter gradients, X^T dY): host-side hint for group_iters
   // Shared memory: a ring of A blocks and a ring of B tiles.  A filter's taps read the same rows of the activation matrix
   // at different shifts, so in kModeConv an A block holds a_rows >= 128 rows, fetched once, and serves every tap of a run (taps
@@ -2183,6 +2184,7 @@ template <int BN, int AR> static size_t plan_launch(GemmParams& p) {
   const size_t bytes = plan_schedule(p, BN, max_clusters_of<BN, AR>);
   static const int group_iters = getenv("TINYFLOW_GROUP_ITERS") ? atoi(getenv("TINYFLOW_GROUP_ITERS")) : 0;
   p.group_iters = group_iters > 0 ? group_iters : (p.data_by_data ? kGroupItersDataByData : (AR == kArithTF32 ? kGroupItersTF32 : kGroupIters));
+  if (p.group_limit) p.group_iters = std::min(p.group_iters, p.group_limit);
   // cross terms promoted every 64 stages: 256 accumulations into a sum 2^-12 of the whole truncate less than 2^-28 of it
   p.cross_groups = 64 / p.group_iters;
   // Two issuers gain from 8 stages per CTA on (equal at 18 of 128 columns, 1 us of 65 at 36); at 96 columns the narrow MMAs
@@ -2914,12 +2916,23 @@ static void plan_runs(GemmParams& g, const TapList& taps, int bn) {
   }
   group(best, &g);
 }
+constexpr int kNarrowTiles = 64, kNarrowStages = 32;
 static int conv_like(const Pack& act, const Pack& filt, int ch_in, int ch_out, int frame_h, int frame_w, float* out, const TapList& taps,
                      const OutGeom& og, double flops, cudaStream_t s, const char* what, int* oom, AmaxOut* track) {
   GemmParams g;
   memset(&g, 0, sizeof(g));
   const int ar = act.arith, bk = bk_of(ar);
-  const int bn = pick_bn(ch_out, true);
+  int bn = pick_bn(ch_out, true);
+  // Few tiles of a short reduction: 64 columns, so that nearly twice the CTAs each do a stage of two thirds the time.  Up to 64 tiles
+  // and 32 stages: Inception-v3 b2 3616 -> 3490 us a step, DenseNet-121 b32 12.60 -> 12.50 ms (longer reductions fill the SMs by being
+  // cut, and a wide tile costs less a stage: all of up to 148 tiles, VGG-16 b7 1331 -> 1356 us).  Where fewer pieces are left, more stages
+  // gather in an accumulator; a promotion after every second one keeps the error where it was.
+  if (bn > 64) {
+    const long long mt = (act.rows + BM - 1) / BM;
+    if (mt * ((ch_out + bn - 1) / bn) <= kNarrowTiles && mt * ((ch_out + 63) / 64) <= device_sm_count() && taps.n * ((ch_in + bk - 1) / bk) <= kNarrowStages) {
+      bn = 64; g.group_limit = 2;
+    }
+  }
   g.mode = kModeConv; g.epi = kEpiNchw;
   g.M = (int)act.rows; g.N = ch_out;
   g.m_tiles = (int)((act.rows + BM - 1) / BM); g.n_tiles = (ch_out + bn - 1) / bn; g.tap_tiles = 1;
