@@ -49,3 +49,38 @@ def test_relu_between_convolutions(env, case, arith):
         np.testing.assert_array_equal(got[4], np.where(got[0] > 0, got[3], np.float32(0)))
         for g, e in zip(got, apart):              # packs made with another power-of-two scale round their low halves differently
             assert np.max(np.abs(g - e)) <= 2e-6 * np.max(np.abs(e))
+
+
+# a max pool between the ReLU and what comes behind (its gradient's maximum is the bound), first layers of few channels (patches) among them
+@pytest.mark.parametrize("case", [(6, 3, 33, 40, 64, 3, 1, 2, 2), (9, 3, 75, 75, 32, 3, 2, 3, 2), (6, 32, 24, 22, 64, 3, 1, 3, 2), (5, 16, 23, 21, 36, 3, 1, 2, 2), (6, 32, 18, 18, 48, 3, 1, 3, 1)])
+def test_relu_backward_behind_a_pool_writes_the_packed_gradient(env, case):
+    N, C, H, W, K, R, stride, win, step = case
+    rng = np.random.RandomState(H + K)
+    gpu, nd = env.gpu_op, env.nd
+    x, w = rng.randn(N, C, H, W).astype(np.float32), rng.randn(K, C, R, R).astype(np.float32)
+    mid, cell = gpu.convolution_2d_forward_get_out_shape(x.shape, w.shape, "NCHW", "SAME", stride, stride)
+    out, pool = gpu.pooling_2d_forward_get_out_shape(mid, "NCHW", "max", 0, 0, step, step, win, win)
+    act = gpu.activation_get_cudnnlist(mid, "NCHW", "relu")
+    X, Wd, DO = nd.array(x, env.ctx), nd.array(w, env.ctx), nd.array(rng.randn(*out).astype(np.float32), env.ctx)
+    y, a, da, dy = (nd.empty(mid, env.ctx) for _ in range(4))
+    o, dw = nd.empty(out, env.ctx), nd.empty(w.shape, env.ctx)
+    results = []
+    gpu.set_contraction_path(2)
+    try:
+        for apart in (True, False):
+            gpu.convolution_2d_forward(X, Wd, y, cell, env.cudnn, env.stream)
+            gpu.activation_forward(y, a, "relu", act, env.cudnn, env.stream)
+            gpu.pooling_2d_forward(a, o, pool, env.cudnn, env.stream)
+            gpu.pooling_2d_backward(a, o, DO, da, pool, env.cudnn, env.stream)
+            before = gpu.launch_count()
+            gpu.activation_backward(y, dy, a, da, "relu", act, env.cudnn, env.stream)
+            if apart:
+                gpu.device_synchronize()          # the ReLU's backward runs on its own
+            gpu.convolution_backward_filter(X, dy, Wd, dw, cell, env.cudnn, env.stream)
+            results.append([v.asnumpy() for v in (y, da, dy, dw)] + [gpu.launch_count() - before])
+    finally:
+        gpu.set_contraction_path(0)
+    assert results[1][4] < results[0][4]          # one kernel less
+    for got in results:
+        np.testing.assert_array_equal(got[2], np.where(got[0] > 0, got[1], np.float32(0)))
+        assert np.max(np.abs(got[3] - results[0][3])) <= 2e-6 * np.max(np.abs(results[0][3]))

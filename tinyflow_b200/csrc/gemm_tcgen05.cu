@@ -3002,7 +3002,9 @@ int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cu
 int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, float* out, cudaStream_t s) {
   static const bool on = [] { const char* e = getenv("TINYFLOW_FUSE_RELU_PACK"); return e ? atoi(e) != 0 : true; }();
   ConvTc* st = conv_state(p);
-  if (!on || !st->cls || p->K < 16 || p->C < 16 || !encode_fn() || out == mask || out == dy) return 0;
+  // (a layer of few channels goes through here as patches, unless the direct kernels take it: they have up to 32 filters at stride 1)
+  const bool taken = p->C >= 16 || (st->cls == 3 && (p->K > 32 || p->stride_h > 1 || p->stride_w > 1));
+  if (!on || !st->cls || p->K < 16 || !taken || !encode_fn() || out == mask || out == dy) return 0;
   const int ar = tensor_arithmetic();
   const uint32_t* bound = ar == kArithF16 ? bound_of(dy) : nullptr;       // max|dy| >= max|out|
   if (ar == kArithF16 && !bound) return 0;

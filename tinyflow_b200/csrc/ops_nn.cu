@@ -135,8 +135,9 @@ __global__ void __launch_bounds__(256) maxpool_bwd_kernel(const float* __restric
 // NP x NQ bounds the windows that can cover one input element (ceil(window / stride) per axis, 0 = take the bounds
 // at run time); with compile-time bounds all index and dy loads are issued before the first use.
 template <bool MAXPOOL, int NP, int NQ>
-__global__ void __launch_bounds__(256) pool_bwd_gather_kernel(const int32_t* __restrict__ idx, const float* __restrict__ dy, float* __restrict__ dx, int64_t total, float scale, PoolGeom g) {
+__global__ void __launch_bounds__(256) pool_bwd_gather_kernel(const int32_t* __restrict__ idx, const float* __restrict__ dy, float* __restrict__ dx, int64_t total, float scale, PoolGeom g, AmaxOut am) {
   grid_dep_sync();
+  uint32_t top = 0;
   int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
     int64_t plane; int h, w;
@@ -176,15 +177,18 @@ __global__ void __launch_bounds__(256) pool_bwd_gather_kernel(const int32_t* __r
         }
     }
     dx[i] = acc * scale;
+    top = max(top, amax_bits(acc * scale));
   }
+  amax_commit(am, top);
 }
 // Max-pool gradient for 3x3 windows, stride 2, padding 0 or 1 (the stem pools of ResNet, Inception and DenseNet): one thread per 2x2
 // block of dx.  The four elements share their candidate windows (p in {a-1, a} + padding, q alike), so the four index / dy
 // pairs are loaded once instead of 2.25 times per element; contributions are added in the same (p, q) order as the
 // general gather, so the result is bit-identical to it.
 __global__ void __launch_bounds__(256) maxpool_bwd_3x3s2_kernel(const int32_t* __restrict__ idx, const float* __restrict__ dy, float* __restrict__ dx,
-                                                                int64_t blocks_total, int H, int W, int P, int Q, int ph, int pw, FastDiv dAB, FastDiv dB) {
+                                                                int64_t blocks_total, int H, int W, int P, int Q, int ph, int pw, FastDiv dAB, FastDiv dB, AmaxOut am) {
   grid_dep_sync();
+  uint32_t top = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int PQ = P * Q, HW = H * W;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < blocks_total; i += stride) {
@@ -214,6 +218,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_3x3s2_kernel(const int32_t* _
 #pragma unroll
         for (int k = 0; k < 4; ++k) acc += id[k] == hw ? v[k] : 0.f;
         o[c] = acc;
+        top = max(top, amax_bits(acc));           // (0 past the last column: no index names it)
       }
       if (w0 + 1 < W) {
         if ((W & 1) == 0) *reinterpret_cast<float2*>(xp + h * W + w0) = make_float2(o[0], o[1]);
@@ -223,14 +228,16 @@ __global__ void __launch_bounds__(256) maxpool_bwd_3x3s2_kernel(const int32_t* _
       }
     }
   }
+  amax_commit(am, top);
 }
 
 // Max-pool gradient for 2x2 windows, stride 2, no padding (VGG, LeNet): windows do not overlap, so one thread owns
 // one window: it reads its index and dy and writes the window's four dx elements (dy at the maximum, 0 elsewhere).
 // Rows / columns of dx past the last window (odd extents) are zero-filled by the threads of the last window row / column.
 __global__ void __launch_bounds__(256) maxpool_bwd_2x2s2_kernel(const int32_t* __restrict__ idx, const float* __restrict__ dy, float* __restrict__ dx,
-                                                                int64_t total, int H, int W, int P, int Q, FastDiv dPQ, FastDiv dQ) {
+                                                                int64_t total, int H, int W, int P, int Q, FastDiv dPQ, FastDiv dQ, AmaxOut am) {
   grid_dep_sync();
+  uint32_t top = 0;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   const int PQ = P * Q, HW = H * W;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) {
@@ -238,6 +245,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_2x2s2_kernel(const int32_t* _
     split_index(i, dPQ, dQ, plane, p, q);
     const int id = __ldg(idx + plane * PQ + p * Q + q);
     const float v = __ldg(dy + plane * PQ + p * Q + q);
+    top = max(top, amax_bits(v));
     float* xp = dx + plane * HW;
     const int h0 = 2 * p, w0 = 2 * q;
     const int h_end = p == P - 1 ? H : h0 + 2, w_end = q == Q - 1 ? W : w0 + 2;     // the last windows also clear the leftover edge
@@ -250,6 +258,7 @@ __global__ void __launch_bounds__(256) maxpool_bwd_2x2s2_kernel(const int32_t* _
       }
     }
   }
+  amax_commit(am, top);
 }
 
 template <int KH, int KW>
@@ -367,6 +376,8 @@ static void launch_maxpool_fwd(const PoolPlan* p, const float* x, float* y, int3
   else launch_dep(maxpool_fwd_kernel<0, 0>, dim3(grid), dim3(256), 0, s, x, y, idx, total, g, am);
 }
 template <bool MAXPOOL> static void launch_pool_gather(const PoolPlan* p, const int32_t* idx, const float* dy, float* dx, int64_t total, float scale, cudaStream_t s) {
+  // max|dx| is the bound that lets the ReLU's backward in front write the next convolution's packed gradient in its pass
+  const AmaxOut am = amax_track_begin(dx);
   PoolGeom g = geom_of(p);
   if (MAXPOOL && p->win_h == 3 && p->win_w == 3 && p->stride_h == 2 && p->stride_w == 2 && p->pad_h <= 1 && p->pad_w <= 1 &&
       (reinterpret_cast<uintptr_t>(dx) & 7) == 0) {
@@ -374,22 +385,22 @@ template <bool MAXPOOL> static void launch_pool_gather(const PoolPlan* p, const 
     const int64_t blocks = (int64_t)p->N * p->C * A * B;
     FastDiv dAB, dB;
     dAB.init((uint32_t)(A * B)); dB.init((uint32_t)B);
-    launch_dep(maxpool_bwd_3x3s2_kernel, dim3(grid_for(blocks, 256)), dim3(256), 0, s, idx, dy, dx, blocks, p->H, p->W, p->P, p->Q, p->pad_h, p->pad_w, dAB, dB);
+    launch_dep(maxpool_bwd_3x3s2_kernel, dim3(grid_for(blocks, 256)), dim3(256), 0, s, idx, dy, dx, blocks, p->H, p->W, p->P, p->Q, p->pad_h, p->pad_w, dAB, dB, am);
     return;
   }
   if (MAXPOOL && p->win_h == 2 && p->win_w == 2 && p->stride_h == 2 && p->stride_w == 2 && p->pad_h == 0 && p->pad_w == 0 &&
       p->P > 0 && p->Q > 0 && (reinterpret_cast<uintptr_t>(dx) & 7) == 0) {
     const int64_t windows = (int64_t)p->N * p->C * p->P * p->Q;
-    launch_dep(maxpool_bwd_2x2s2_kernel, dim3(grid_for(windows, 256)), dim3(256), 0, s, idx, dy, dx, windows, p->H, p->W, p->P, p->Q, g.dPQ, g.dQ);
+    launch_dep(maxpool_bwd_2x2s2_kernel, dim3(grid_for(windows, 256)), dim3(256), 0, s, idx, dy, dx, windows, p->H, p->W, p->P, p->Q, g.dPQ, g.dQ, am);
     return;
   }
   int grid = grid_for(total, 256);
   auto bound = [](int win, int stride, int count) { int n = (win + stride - 1) / stride; return n < count ? n : count; };
   int np = bound(p->win_h, p->stride_h, p->P), nq = bound(p->win_w, p->stride_w, p->Q);
-  if (np == 1 && nq == 1) launch_dep(pool_bwd_gather_kernel<MAXPOOL, 1, 1>, dim3(grid), dim3(256), 0, s, idx, dy, dx, total, scale, g);
-  else if (np <= 2 && nq <= 2) launch_dep(pool_bwd_gather_kernel<MAXPOOL, 2, 2>, dim3(grid), dim3(256), 0, s, idx, dy, dx, total, scale, g);
-  else if (np <= 3 && nq <= 3) launch_dep(pool_bwd_gather_kernel<MAXPOOL, 3, 3>, dim3(grid), dim3(256), 0, s, idx, dy, dx, total, scale, g);
-  else launch_dep(pool_bwd_gather_kernel<MAXPOOL, 0, 0>, dim3(grid), dim3(256), 0, s, idx, dy, dx, total, scale, g);
+  if (np == 1 && nq == 1) launch_dep(pool_bwd_gather_kernel<MAXPOOL, 1, 1>, dim3(grid), dim3(256), 0, s, idx, dy, dx, total, scale, g, am);
+  else if (np <= 2 && nq <= 2) launch_dep(pool_bwd_gather_kernel<MAXPOOL, 2, 2>, dim3(grid), dim3(256), 0, s, idx, dy, dx, total, scale, g, am);
+  else if (np <= 3 && nq <= 3) launch_dep(pool_bwd_gather_kernel<MAXPOOL, 3, 3>, dim3(grid), dim3(256), 0, s, idx, dy, dx, total, scale, g, am);
+  else launch_dep(pool_bwd_gather_kernel<MAXPOOL, 0, 0>, dim3(grid), dim3(256), 0, s, idx, dy, dx, total, scale, g, am);
 }
 
 // =====================================================================================
@@ -806,7 +817,10 @@ int DLGpuPooling2DBackward(const DLArrayHandle input, const DLArrayHandle output
     else
       launch_plain(maxpool_bwd_kernel, dim3(grid_for(total, 256)), dim3(256), 0, s, (const float*)input->data, (const float*)doutput->data, out_f32(dinput), total, geom_of(p));
   }
-  else if (mean3_fits(p, (const float*)doutput->data)) launch_mean3(p, (const float*)doutput->data, out_f32(dinput), s, AmaxOut{});
+  else if (mean3_fits(p, (const float*)doutput->data)) {
+    float* dx = out_f32(dinput);
+    launch_mean3(p, (const float*)doutput->data, dx, s, amax_track_begin(dx));
+  }
   else launch_pool_gather<false>(p, nullptr, (const float*)doutput->data, out_f32(dinput), total, 1.f / (float)(p->win_h * p->win_w), s);
   TF_AFTER(s, "DLGpuPooling2DBackward");
   return 0;
