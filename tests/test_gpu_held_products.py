@@ -1,4 +1,4 @@
-"""Filter gradients that wait and share a launch: the bits of separate launches, whatever is held back together."""
+"""Gradients of parameters that wait and share a launch: the bits of separate launches, whatever is held back together."""
 import numpy as np
 import pytest
 
@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
-@pytest.mark.parametrize("name", ["inceptionv3", "resnet50", "vgg16", "densenet121"])
+@pytest.mark.parametrize("name", ["inceptionv3", "resnet50", "vgg16", "densenet121", "mlp", "lenet5"])
 def test_products_held_back_have_the_bits_of_separate_launches(lib_path, monkeypatch, name, arith):
     from tinyflow_b200 import gpu_op
     build = BUILDS.get(name, lambda m: m.densenet121(batch=16, classes=10, image=96))
@@ -66,3 +66,39 @@ def test_layers_in_one_launch(lib_path, layers, arith):
     finally:
         gpu_op.drop_held()
         gpu_op.set_tensor_arithmetic("3xfp16")
+
+
+# more than one launch of each kind; reductions of one CTA up to a cluster of 8, sums of one block up to many, ragged tiles
+@pytest.mark.parametrize("count", [1, 3, 37])
+def test_dense_gradients_in_one_launch(lib_path, count):
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, stream, rng = nd.gpu(0), gpu_op.create_cudaStream(), np.random.RandomState(count)
+    cublas, cudnn = gpu_op.create_cublasHandle(stream), gpu_op.create_cudnnHandle(stream)
+    calls = []
+    for i in range(count):
+        rows, a, b = (int(v) for v in (rng.choice([7, 64, 100, 1000, 1200]), rng.choice([9, 33, 120, 400]), rng.choice([10, 31, 84, 300])))
+        x, dy = (nd.array(rng.randn(rows, n).astype(np.float32), ctx) for n in (a, b))
+        image = nd.array(rng.randn(max(1, rows // 50), 6, 9, 1 + i % 5).astype(np.float32), ctx)
+        cells = [gpu_op.reduce_sum_get_cudnnlist(*gpu_op.reduce_sum_get_real_shape(s, o, f), f, cudnn) for s, o, f in (((rows, b), (b,), "NHWC"), (image.shape, (6,), "NCHW"))]
+        calls.append((x, dy, image, cells, [nd.empty((a, b), ctx), nd.empty((b,), ctx), nd.empty((6,), ctx)], [nd.empty((a, b), ctx), nd.empty((b,), ctx), nd.empty((6,), ctx)]))
+
+    def run(into):
+        for call in calls:
+            x, dy, image, cells, out = call[:4] + (call[into],)
+            gpu_op.matrix_multiply(x, True, dy, False, out[0], cublas, stream)
+            gpu_op.reduce_sum_new(dy, out[1], cells[0], cudnn, stream)
+            gpu_op.reduce_sum_new(image, out[2], cells[1], cudnn, stream)
+    run(4)
+    try:
+        gpu_op.hold_products(True)
+        run(5)
+        gpu_op.hold_products(False)
+        before = gpu_op.launch_count()
+        gpu_op.launch_held(stream)
+        assert gpu_op.launch_count() - before == (count + 15) // 16 + (2 * count + 31) // 32
+    finally:
+        gpu_op.drop_held()
+    for x, dy, _, _, apart, together in calls:
+        for one, other in zip(apart, together):
+            np.testing.assert_array_equal(one.asnumpy(), other.asnumpy())
+        np.testing.assert_allclose(together[0].asnumpy(), x.asnumpy().T.astype(np.float64) @ dy.asnumpy(), rtol=1e-4, atol=1e-2)

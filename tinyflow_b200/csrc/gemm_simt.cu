@@ -10,6 +10,7 @@
 // Measured against the kernel it replaced and against the tensor path: the table in simt_matmul(), where the tile is chosen.
 #include "common.h"
 #include <algorithm>
+#include <vector>
 #include <cooperative_groups.h>
 
 namespace cg = cooperative_groups;
@@ -67,8 +68,9 @@ template <int ROWS, int BK, int THREADS, bool KFAST> struct BlockLoader {
   }
 };
 
+// One tile, or the share of it of CTA `rank` of `ranks` (the first of them is CTA `first` of the cluster)
 template <int BM, int BN, int TM, int TN, int BK, bool A_KFAST, bool B_KFAST>
-__global__ void __launch_bounds__((BM / TM) * (BN / TN)) simt_gemm_kernel(const SimtGemm p) {
+__device__ __forceinline__ void simt_tile(const SimtGemm& p, int m0, int n0, int rank, int ranks, int first) {
   constexpr int THREADS = (BM / TM) * (BN / TN);
   constexpr int kTile = 2 * BK * (BM + 4) + 2 * BK * (BN + 4);
   constexpr int kSmem = kTile > BM * BN ? kTile : BM * BN;
@@ -76,9 +78,6 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) simt_gemm_kernel(const 
   float (*As)[BK][BM + 4] = reinterpret_cast<float (*)[BK][BM + 4]>(smem);
   float (*Bs)[BK][BN + 4] = reinterpret_cast<float (*)[BK][BN + 4]>(smem + 2 * BK * (BM + 4));
   cg::cluster_group cluster = cg::this_cluster();
-  const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
-  grid_dep_sync();
-  const int m0 = blockIdx.y * BM, n0 = (int)(blockIdx.x / ranks) * BN;      // the CTAs of a cluster are neighbours in x
   const int kbeg = rank * p.k_per_cta, kend = min(p.K, kbeg + p.k_per_cta);
   const int tx = threadIdx.x % (BN / TN), ty = threadIdx.x / (BN / TN);
   float acc[TM][TN];
@@ -139,7 +138,7 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) simt_gemm_kernel(const 
   cluster.sync();
   const float* part[16];
 #pragma unroll
-  for (int r = 0; r < 16; ++r) part[r] = r < ranks ? cluster.map_shared_rank(smem, r) : smem;
+  for (int r = 0; r < 16; ++r) part[r] = r < ranks ? cluster.map_shared_rank(smem, first + r) : smem;
   const int slice = (BM * BN + ranks - 1) / ranks, end = min(BM * BN, (rank + 1) * slice);
   for (int e = rank * slice + threadIdx.x; e < end; e += THREADS) {
     float t = 0.f;
@@ -149,6 +148,32 @@ __global__ void __launch_bounds__((BM / TM) * (BN / TN)) simt_gemm_kernel(const 
     if (m < p.M && n < p.N) p.C[(long long)m * p.ldc + n] = t;
   }
   cluster.sync();           // nobody leaves while its shared memory is still read
+}
+template <int BM, int BN, int TM, int TN, int BK, bool A_KFAST, bool B_KFAST>
+__global__ void __launch_bounds__((BM / TM) * (BN / TN)) simt_gemm_kernel(const SimtGemm p) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int rank = (int)cluster.block_rank(), ranks = (int)cluster.num_blocks();
+  grid_dep_sync();
+  simt_tile<BM, BN, TM, TN, BK, A_KFAST, B_KFAST>(p, blockIdx.y * BM, (int)(blockIdx.x / ranks) * BN, rank, ranks, 0);      // the CTAs of a cluster are neighbours in x
+}
+
+// ---- weight gradients of dense layers that wait for others --------------------------------------------------------------
+// As the filter gradients of convolutions (hold_products): nobody reads them before the parameters are updated, and a launch
+// each is a chain of 3-5 us kernels.  Tiles, shares of K and order of the sums are those of the separate launches.  All
+// clusters have the largest size that one of the products asks for; smaller ones share a cluster.
+constexpr int kSimtJobs = 16, kHeldTile = 32, kHeldTiles = 1024;
+struct SimtJob { SimtGemm p; int ranks, n_tiles, tiles, first_cluster; };
+struct SimtJobs { int n; SimtJob job[kSimtJobs]; };
+__global__ void __launch_bounds__(128) simt_group_kernel(const __grid_constant__ SimtJobs jobs) {
+  cg::cluster_group cluster = cg::this_cluster();
+  const int size = (int)cluster.num_blocks(), at = (int)cluster.block_rank(), id = blockIdx.x / size;
+  grid_dep_sync();
+  int k = 0;
+  while (k + 1 < jobs.n && jobs.job[k + 1].first_cluster <= id) ++k;
+  const SimtJob& j = jobs.job[k];
+  const int sub = at / j.ranks, tile = (id - j.first_cluster) * (size / j.ranks) + sub;
+  if (tile < j.tiles) simt_tile<32, 32, 4, 2, 32, false, false>(j.p, tile / j.n_tiles * kHeldTile, tile % j.n_tiles * kHeldTile, at - sub * j.ranks, j.ranks, sub * j.ranks);
+  if (size > 1 && (tile >= j.tiles || j.ranks == 1)) { cluster.sync(); cluster.sync(); }        // those of the tiles that are cut
 }
 
 template <int BM, int BN, int TM, int TN, int BK, bool AK, bool BKF>
@@ -372,6 +397,31 @@ static int rows_matmul(const SimtGemm& p, bool tA, bool tB, cudaStream_t s) {
   return 0;
 }
 
+static thread_local std::vector<SimtJob> t_held_simt;
+void drop_held_simt() { t_held_simt.clear(); }
+int launch_held_simt(cudaStream_t s) {
+  std::vector<SimtJob> all;
+  all.swap(t_held_simt);
+  for (size_t from = 0; from < all.size(); from += kSimtJobs) {
+    SimtJobs jobs;
+    jobs.n = (int)std::min(all.size() - from, (size_t)kSimtJobs);
+    int size = 1, clusters = 0;
+    double flops = 0;
+    for (int i = 0; i < jobs.n; ++i) size = std::max(size, all[from + i].ranks);
+    for (int i = 0; i < jobs.n; ++i) {
+      SimtJob& j = jobs.job[i] = all[from + i];
+      j.first_cluster = clusters;
+      clusters += (j.tiles * j.ranks + size - 1) / size;
+      flops += 2.0 * j.p.M * j.p.N * j.p.K;
+    }
+    note_compute_stream(s);
+    KernelTimer kt("simt_gemm", s, flops, 0, 1);
+    TF_CUDA(launch_cluster(simt_group_kernel, size, dim3((unsigned)(clusters * size)), dim3(128), 0, s, jobs));
+    TF_AFTER(s, "weight gradients");
+  }
+  return 0;
+}
+
 // C[M x N] = op(A) op(B), row-major, leading dimensions of the arrays as they are stored.
 int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldc, cudaStream_t s, const char* what) {
   if (M <= 0 || N <= 0) return 0;
@@ -395,6 +445,10 @@ int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int6
   int cluster = 1;
   while (cluster < (cfg == 0 ? 16 : 8) && tiles * cluster < want && (K + bk - 1) / bk >= 4 * cluster) cluster *= 2;
   p.k_per_cta = (int)(((K + cluster - 1) / cluster + bk - 1) / bk * bk);
+  if (cfg == 1 && tA && !tB && tiles <= kHeldTiles && may_hold(s)) {
+    t_held_simt.push_back(SimtJob{p, cluster, (int)((N + 31) / 32), (int)tiles, 0});
+    return 0;
+  }
   note_compute_stream(s);
   KernelTimer kt("simt_gemm", s, 2.0 * (double)M * (double)N * (double)K, 0, 1);
   if (const int rc = rows_matmul(p, tA, tB, s)) {

@@ -2248,8 +2248,19 @@ static thread_local double t_held_work = 0;           // tiles x stages
 // layout of the accumulators); at 64 columns 102 still gain (DenseNet-121 13.76 -> 13.50 ms against a limit of 24).
 template <int BN> constexpr int kHeldRun = BN == 64 ? 160 : 24;
 constexpr int kHeldWork = 1024;                       // stages per SM that are launched together at the latest (64: ResNet-50 b19 4096 us, 256: 3999, 512 and all: 3976)
+int launch_held_simt(cudaStream_t s);       // gemm_simt.cu: weight gradients of dense layers
+void drop_held_simt();
+int launch_held_sums(cudaStream_t s);       // ops_basic.cu: bias gradients
+void drop_held_sums();
 void hold_products(bool on) { t_hold = on; }
-void drop_held() { t_held.clear(); t_held_work = 0; t_hold = false; }
+void drop_held() { t_held.clear(); t_held_work = 0; t_hold = false; drop_held_simt(); drop_held_sums(); }
+// The call may wait: its caller says so, and no graph of the caller's own is being captured (it would copy from a table that is gone)
+bool may_hold(cudaStream_t s) {
+  if (!t_hold) return false;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(t_recording ? recording_home() : s, &capture) != cudaSuccess) { cudaGetLastError(); return false; }
+  return capture == cudaStreamCaptureStatusNone;
+}
 
 template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>& held, cudaStream_t s, double flops) {
   static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_group_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem<BN>);
@@ -2333,7 +2344,7 @@ template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>
   }
   return 0;
 }
-int launch_held(cudaStream_t s) try {
+static int launch_held_filters(cudaStream_t s) {
   if (t_held.empty()) return 0;
   std::vector<HeldProduct> all;
   all.swap(t_held);
@@ -2351,19 +2362,22 @@ int launch_held(cudaStream_t s) try {
       if (rc) return rc;
     }
   return 0;
-} catch (const std::bad_alloc&) { TF_FAIL("filter gradients: out of host memory"); }
+}
+int launch_held(cudaStream_t s) try {
+  if (int rc = launch_held_filters(s)) return rc;
+  if (int rc = launch_held_simt(s)) return rc;
+  return launch_held_sums(s);
+} catch (const std::bad_alloc&) { TF_FAIL("gradients that waited: out of host memory"); }
 // Before the pack at `hi` is written again: what still has to read it goes first.
 static int release_held(const void* hi, cudaStream_t s) {
   for (const HeldProduct& h : t_held)
-    if (h.g.pack_a == hi || h.g.pack_b == hi) return launch_held(s);
+    if (h.g.pack_a == hi || h.g.pack_b == hi) return launch_held_filters(s);
   return 0;
 }
 // Takes the product if it may wait; what has gathered goes when it fills the SMs.
 template <int BN, int AR> static bool held_back(const GemmParams& p, cudaStream_t s, double flops) {
-  if (BN == 96 || !t_hold || p.group_iters != 1 || p.acc_mode != kAccPair || longest_run(p) >= kHeldRun<BN> || (p.tail_share > 0 && p.tail_pieces == 0) || p.amax) return false;
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;      // a caller's own graph would copy from a table that is gone
-  if (cudaStreamIsCapturing(t_recording ? recording_home() : s, &capture) != cudaSuccess) { cudaGetLastError(); return false; }
-  if (capture != cudaStreamCaptureStatusNone) return false;
+  if (BN == 96 || p.group_iters != 1 || p.acc_mode != kAccPair || longest_run(p) >= kHeldRun<BN> || (p.tail_share > 0 && p.tail_pieces == 0) || p.amax) return false;
+  if (!may_hold(s)) return false;
   t_held.push_back(HeldProduct{p, BN, AR, flops});
   t_held_work += (double)p.m_tiles * p.n_tiles * p.tap_tiles * p.k_total;
   return true;
@@ -3093,7 +3107,7 @@ static int launch_wgrad(const ConvTc* st, int bn, int ar, GemmParams& g, cudaStr
   g.operand_bytes = 2.0 * st->dy.bytes() + 2.0 * st->x_pack().bytes();
   g.hold = 1; g.pack_a = st->x_pack().hi; g.pack_b = st->dy.hi;
   const int rc = launch_gemm_bn(bn, ar, g, s, flops, "DLGpuConvolutionBackwardFilter", oom);
-  if (rc == 0 && t_held_work >= (double)kHeldWork * device_sm_count() && launch_held(s)) return -1;
+  if (rc == 0 && t_held_work >= (double)kHeldWork * device_sm_count() && launch_held_filters(s)) return -1;
   return tc_result(rc);
 }
 int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaStream_t s, int* oom) {

@@ -6,6 +6,7 @@
 #include <math.h>
 #include <algorithm>
 #include <mutex>
+#include <vector>
 
 namespace tf {
 
@@ -187,16 +188,21 @@ __global__ void __launch_bounds__(kBlock) bcast_channel_kernel(const float* __re
 // ---- reductions --------------------------------------------------------------------
 // Column sums of a row-major [rows x cols] matrix, out[c] = sum_r in[r, c].
 // Block = 32 columns x 8 row lanes; grid.x tiles the columns, grid.y splits the rows.
-__global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ in, float* __restrict__ out, float* __restrict__ part, int64_t rows, int64_t cols, int64_t rows_per_split, uint32_t* counters) {
+struct SumJob {               // column sums of [rows][cols], or channel sums of [rows = images][cols = channels][length]
+  const float* in; float* out; float* part; uint32_t* counters;
+  int64_t rows, cols, length, per_split;
+  int splits, vec;            // vec: 16-byte loads along `length`
+  int first_block;            // of a group's launch
+};
+__device__ __forceinline__ void column_sum(const SumJob& p, int block, int split) {
   __shared__ float sm[8][33];
-  grid_dep_sync();
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t c = (int64_t)blockIdx.x * 32 + tx;
-  const int64_t r0 = (int64_t)blockIdx.y * rows_per_split, r1 = min(rows, r0 + rows_per_split);
+  const int64_t c = (int64_t)block * 32 + tx;
+  const int64_t r0 = (int64_t)split * p.per_split, r1 = min(p.rows, r0 + p.per_split);
   auto across = [&](float acc, float* dst) {
     sm[ty][tx] = acc;
     __syncthreads();
-    if (ty == 0 && c < cols) {
+    if (ty == 0 && c < p.cols) {
       float t = 0.f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) t += sm[j][tx];
@@ -204,29 +210,33 @@ __global__ void __launch_bounds__(256) colsum_kernel(const float* __restrict__ i
     }
   };
   float acc = 0.f;
-  if (c < cols) {
+  if (c < p.cols) {
 #pragma unroll 4
-    for (int64_t r = r0 + ty; r < r1; r += 8) acc += in[r * cols + c];
+    for (int64_t r = r0 + ty; r < r1; r += 8) acc += p.in[r * p.cols + c];
   }
-  if (gridDim.y == 1) { across(acc, out + c); return; }
-  across(acc, part + (int64_t)blockIdx.y * cols + c);
-  if (!arrives_last(counters + blockIdx.x, gridDim.y)) return;
+  if (p.splits == 1) { across(acc, p.out + c); return; }
+  across(acc, p.part + (int64_t)split * p.cols + c);
+  if (!arrives_last(p.counters + block, p.splits)) return;
   acc = 0.f;
-  if (c < cols) {
+  if (c < p.cols) {
 #pragma unroll 4
-    for (int z = ty; z < (int)gridDim.y; z += 8) acc += __ldcg(part + (int64_t)z * cols + c);
+    for (int z = ty; z < p.splits; z += 8) acc += __ldcg(p.part + (int64_t)z * p.cols + c);
   }
-  across(acc, out + c);
+  across(acc, p.out + c);
+}
+__global__ void __launch_bounds__(256) colsum_kernel(const __grid_constant__ SumJob p) {
+  grid_dep_sync();
+  column_sum(p, blockIdx.x, blockIdx.y);
 }
 // Sum over images and positions of every channel, in = [N][C][L] (the bias gradient of a convolution).  One block per
 // channel left all but 6 SMs idle on LeNet's first layer (467 us for 4.8 MB): the images are split over grid.y as well.
-__global__ void __launch_bounds__(kBlock) channel_sum_kernel(const float* __restrict__ in, float* __restrict__ out, float* __restrict__ part, int64_t N, int64_t C, int64_t L, int64_t n_per_split, int vec,
-                                                             uint32_t* counters) {
+__device__ __forceinline__ void channel_sum(const SumJob& p, int block, int split) {
   __shared__ float red[33];
-  grid_dep_sync();
-  const int64_t c = blockIdx.x, n0 = (int64_t)blockIdx.y * n_per_split, n1 = min(N, n0 + n_per_split);
+  const int64_t N = p.rows, C = p.cols, L = p.length;
+  const float* const in = p.in;
+  const int64_t c = block, n0 = (int64_t)split * p.per_split, n1 = min(N, n0 + p.per_split);
   float acc = 0.f;
-  if (vec) {
+  if (p.vec) {
     const uint32_t q = (uint32_t)(L >> 2), count = (uint32_t)(n1 - n0) * q;
 #pragma unroll 4
     for (uint32_t i = threadIdx.x; i < count; i += kBlock) {
@@ -239,13 +249,83 @@ __global__ void __launch_bounds__(kBlock) channel_sum_kernel(const float* __rest
       for (int64_t l = threadIdx.x; l < L; l += kBlock) acc += in[(n * C + c) * L + l];
   }
   acc = block_sum(acc, red);
-  if (gridDim.y == 1) { if (threadIdx.x == 0) out[c] = acc; return; }
-  if (threadIdx.x == 0) part[(int64_t)blockIdx.y * C + c] = acc;
-  if (!arrives_last(counters + blockIdx.x, gridDim.y)) return;
+  if (p.splits == 1) { if (threadIdx.x == 0) p.out[c] = acc; return; }
+  if (threadIdx.x == 0) p.part[(int64_t)split * C + c] = acc;
+  if (!arrives_last(p.counters + block, p.splits)) return;
   acc = 0.f;
-  for (int z = threadIdx.x; z < (int)gridDim.y; z += kBlock) acc += __ldcg(part + (int64_t)z * C + c);
+  for (int z = threadIdx.x; z < p.splits; z += kBlock) acc += __ldcg(p.part + (int64_t)z * C + c);
   acc = block_sum(acc, red);
-  if (threadIdx.x == 0) out[c] = acc;
+  if (threadIdx.x == 0) p.out[c] = acc;
+}
+__global__ void __launch_bounds__(kBlock) channel_sum_kernel(const __grid_constant__ SumJob p) {
+  grid_dep_sync();
+  channel_sum(p, blockIdx.x, blockIdx.y);
+}
+// Bias gradients that wait for others: as the products of hold_products(), 3-5 us apiece in a chain of their own.  Blocks and order of
+// the sums are those of the separate launches.
+constexpr int kSumJobs = 32, kHeldSumBlocks = 2048;
+struct SumJobs { int n; SumJob job[kSumJobs]; };
+__global__ void __launch_bounds__(256) sum_group_kernel(const __grid_constant__ SumJobs jobs) {
+  static_assert(kBlock == 256, "both kinds share the launch");
+  grid_dep_sync();
+  int k = 0;
+  while (k + 1 < jobs.n && jobs.job[k + 1].first_block <= (int)blockIdx.x) ++k;
+  const SumJob& j = jobs.job[k];
+  const int at = (int)blockIdx.x - j.first_block, across = j.length ? (int)j.cols : (int)((j.cols + 31) / 32), split = at / across;
+  if (j.length) channel_sum(j, at - split * across, split);
+  else column_sum(j, at - split * across, split);
+}
+static int sum_blocks(const SumJob& j) { return j.length ? (int)j.cols : (int)((j.cols + 31) / 32); }        // per split
+// Scratch of the jobs that are split; column sums do without where there is none
+static int sum_scratch(SumJob* jobs, int n, StreamLease& lease, const char* what) {
+  size_t floats = 0, counters = 0;
+  for (int i = 0; i < n; ++i)
+    if (jobs[i].splits > 1) { floats += (size_t)jobs[i].splits * (size_t)jobs[i].cols; counters += sum_blocks(jobs[i]); }
+  if (!counters) return 0;
+  float* part = (float*)lease.scratch(kScratchSplit, sizeof(float) * floats);
+  uint32_t* count = lease.counters((int)counters);
+  for (int i = 0; i < n; ++i) {
+    SumJob& j = jobs[i];
+    if (j.splits == 1) continue;
+    if (!part || !count) {
+      TF_REQUIRE(!j.length, "%s: scratch allocation failed", what);
+      j.splits = 1; j.per_split = j.rows;
+      continue;
+    }
+    j.part = part; j.counters = count;
+    part += (size_t)j.splits * (size_t)j.cols; count += sum_blocks(j);
+  }
+  return 0;
+}
+static thread_local std::vector<SumJob> t_held_sums;
+void drop_held_sums() { t_held_sums.clear(); }
+int launch_held_sums(cudaStream_t s) {
+  std::vector<SumJob> all;
+  all.swap(t_held_sums);
+  for (size_t from = 0; from < all.size(); from += kSumJobs) {
+    SumJobs jobs;
+    jobs.n = (int)std::min(all.size() - from, (size_t)kSumJobs);
+    std::copy(all.begin() + from, all.begin() + from + jobs.n, jobs.job);
+    StreamLease lease(s);
+    if (sum_scratch(jobs.job, jobs.n, lease, "bias gradients")) return -1;
+    int blocks = 0;
+    for (int i = 0; i < jobs.n; ++i) { jobs.job[i].first_block = blocks; blocks += sum_blocks(jobs.job[i]) * jobs.job[i].splits; }
+    note_compute_stream(s);
+    launch_dep(sum_group_kernel, dim3((unsigned)blocks), dim3(256), 0, s, jobs);
+    TF_AFTER(s, "bias gradients");
+  }
+  return 0;
+}
+static int run_sums(SumJob j, cudaStream_t s, const char* what) {
+  if ((long long)sum_blocks(j) * j.splits <= kHeldSumBlocks && may_hold(s)) { t_held_sums.push_back(j); return 0; }
+  StreamLease lease(s);
+  if (sum_scratch(&j, 1, lease, what)) return -1;
+  note_compute_stream(s);
+  const dim3 grid((unsigned)sum_blocks(j), (unsigned)j.splits);
+  if (j.length) launch_dep(channel_sum_kernel, grid, dim3(kBlock), 0, s, j);
+  else launch_dep(colsum_kernel, grid, dim3(256), 0, s, j);
+  TF_AFTER(s, what);
+  return 0;
 }
 // Sum of n contiguous floats into out[0], finished by the last block.
 __global__ void __launch_bounds__(kBlock) sum_kernel(const float* __restrict__ in, float* __restrict__ out, float* __restrict__ part, int64_t n, float scale, uint32_t* counter) {
@@ -818,19 +898,8 @@ static int channel_sums(const float* in, float* out, int64_t N, int64_t C, int64
   splits = std::max<int64_t>(splits, 1);
   const int64_t nps = std::max<int64_t>(1, (N + splits - 1) / splits);
   splits = std::max<int64_t>(1, (N + nps - 1) / nps);
-  StreamLease lease(s);
-  float* part = nullptr;
-  uint32_t* counters = nullptr;
-  if (splits > 1) {
-    part = (float*)lease.scratch(kScratchSplit, sizeof(float) * (size_t)splits * (size_t)C);
-    counters = lease.counters((int)C);
-    TF_REQUIRE(part && counters, "%s: scratch allocation failed", what);
-  }
   const int vec = L % 4 == 0 && aligned16(in) && nps * (L / 4) < (1ll << 31);
-  note_compute_stream(s);
-  launch_dep(channel_sum_kernel, dim3((unsigned)C, (unsigned)splits), dim3(kBlock), 0, s, in, out, part, N, C, L, nps, vec, counters);
-  TF_AFTER(s, what);
-  return 0;
+  return run_sums(SumJob{in, out, nullptr, nullptr, N, C, L, nps, (int)splits, vec, 0}, s, what);
 }
 
 static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, cudaStream_t s, const char* what) {
@@ -844,18 +913,7 @@ static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, 
   }
   int64_t rps = (rows + splits - 1) / splits;
   splits = (int)((rows + rps - 1) / rps);
-  StreamLease lease(s);
-  float* part = nullptr;
-  uint32_t* counters = nullptr;
-  if (splits > 1) {
-    part = (float*)lease.scratch(kScratchSplit, sizeof(float) * (size_t)splits * (size_t)cols);
-    counters = lease.counters(gx);
-    if (!part || !counters) { splits = 1; rps = rows; }                                  // no scratch: one split
-  }
-  note_compute_stream(s);
-  launch_dep(colsum_kernel, dim3(gx, splits), dim3(256), 0, s, in, out, part, rows, cols, rps, counters);
-  TF_AFTER(s, what);
-  return 0;
+  return run_sums(SumJob{in, out, nullptr, nullptr, rows, cols, 0, rps, splits, 0, 0}, s, what);
 }
 
 int DLGReduceSumGetCudnnlist(const int* input_shapes, const int* output_shapes, const int sizeofshape,

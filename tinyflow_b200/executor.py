@@ -26,7 +26,7 @@ import warnings
 import weakref
 
 from . import gpu_op, ndarray, step_graph
-from .graph import (AddOp, AdamOp, BNForwardOp, Convolution2DBackwardOp, Convolution2DForwardOp, OnesLikeOp, Pooling2DForwardOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
+from .graph import (AddOp, AdamOp, BNForwardOp, BroadcastToGradientOp, Convolution2DBackwardOp, Convolution2DForwardOp, MatMulOp, OnesLikeOp, Pooling2DForwardOp, SgdOp, Variable, ZerosLikeOp, adam_op, find_topo_sort, get_Variable_node_list, gradients, sgd_op)
 
 
 def getcomputelist(Variable_node_list, Variable_node_grad_list, b1, b2, b1t, b2t, e, learning_rate):
@@ -190,13 +190,12 @@ class Executor(object):
         # convolutions of a fed filter, and their descriptors as the library takes them (with the objects behind)
         self._convs = [n for n in self.topo_order if type(n.op) is Convolution2DForwardOp and not n.inputs[1].inputs]
         self._conv_cells = ([], None)
-        # filter gradients that only the optimiser reads: they may wait and share launches
+        # gradients of parameters that only the optimiser reads: they may wait and share launches
         readers = {}
         for node in self.topo_order:
             for i in node.inputs:
                 readers.setdefault(i, []).append(node)
-        self._patient = {n for n in self.topo_order if type(n.op) is Convolution2DBackwardOp and n.type == 1
-                         and all(type(r.op) in (SgdOp, AdamOp) for r in readers.get(n, ()))}
+        self._patient = {n for n in self.topo_order if self._is_parameter_gradient(n) and all(type(r.op) in (SgdOp, AdamOp) for r in readers.get(n, ()))}
         self._values = {}          # node index -> NDArray on the GPU (None while swapped out)
         self._feed = {}            # what the most recent run was fed: node -> NDArray on the GPU
         self._leases = {}          # node index -> weak references to the views of its array that were handed out
@@ -209,6 +208,12 @@ class Executor(object):
         self._swap_worker = None
         self._values_lock = threading.Lock()
         self.passive_swap_in = 0
+
+    @staticmethod
+    def _is_parameter_gradient(node):
+        if type(node.op) is Convolution2DBackwardOp:
+            return node.type == 1
+        return type(node.op) is BroadcastToGradientOp or (type(node.op) is MatMulOp and node.matmul_attr_trans_A)
 
     @property
     def values(self):
