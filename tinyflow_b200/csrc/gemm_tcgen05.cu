@@ -2652,7 +2652,12 @@ void tc_release(void* tc_state) {
 static int launch_pack_nchw(Pack& pk, const ScaleRef& sr, const float* src, int N, int chans, int H, int W, int frame_h, int frame_w, int off_h, int off_w,
                             int sh, int sw, int dst_c0, int cover, cudaStream_t s, float* relu_out = nullptr, AmaxOut relu_am = AmaxOut{}, const float* mask = nullptr) {
   PackGeom g{N, chans, H, W, frame_h, frame_w, off_h, off_w, sh, sw, (int)pk.pitch, dst_c0, cover};
-  const int tc = cover > 64 ? 128 : cover > 32 ? 64 : 32;
+  // The widest channel block, as long as that makes four blocks an SM (16 of tf32, whose blocks move twice the bytes): a small frame in
+  // wide blocks is one wave of long chains.  Inception-v4 b16 3xTF32 19.41 -> 18.83 ms a step (four: 19.11), VGG-16 b7 1323 -> 1301 us; with
+  // 16 blocks of fp16 DenseNet-121 b32 12.50 -> 12.65 ms.
+  int tc = cover > 64 ? 128 : cover > 32 ? 64 : 32;
+  const int enough = (pk.arith == kArithTF32 ? 16 : 4) * device_sm_count();
+  while (tc > 32 && (long long)N * ((cover + tc - 1) / tc) * ((frame_h * frame_w + 31) / 32) < enough) tc /= 2;
   dim3 grid(N * ((cover + tc - 1) / tc), (frame_h * frame_w + 31) / 32);
   TF_REQUIRE(grid.y <= 65535, "pack: frame of %d x %d positions is too large", frame_h, frame_w);
   const char* what = mask ? "relu_bwd_pack" : relu_out ? "relu_pack" : "pack_nchw";
