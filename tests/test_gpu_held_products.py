@@ -102,3 +102,29 @@ def test_dense_gradients_in_one_launch(lib_path, count):
         for one, other in zip(apart, together):
             np.testing.assert_array_equal(one.asnumpy(), other.asnumpy())
         np.testing.assert_allclose(together[0].asnumpy(), x.asnumpy().T.astype(np.float64) @ dy.asnumpy(), rtol=1e-4, atol=1e-2)
+
+
+@pytest.mark.parametrize("count", [1, 2, 11])
+def test_direct_filter_gradients_in_one_launch(lib_path, count):
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, stream, rng = nd.gpu(0), gpu_op.create_cudaStream(), np.random.RandomState(count)
+    handle = gpu_op.create_cudnnHandle(stream)
+    calls = []
+    for i in range(count):
+        N, C, H, W, K, R, S, padding = [(3, 1, 28, 28, 6, 5, 5, "SAME"), (40, 6, 14, 14, 16, 5, 5, "VALID"), (300, 3, 9, 7, 5, 3, 3, "SAME"), (7, 2, 8, 8, 3, 7, 7, "SAME")][i % 4]
+        out, cell = gpu_op.convolution_2d_forward_get_out_shape((N, C, H, W), (K, C, R, S), "NCHW", padding, 1, 1)
+        x, w, dy = (nd.array(rng.randn(*shape).astype(np.float32), ctx) for shape in ((N, C, H, W), (K, C, R, S), out))
+        calls.append((x, dy, w, nd.empty((K, C, R, S), ctx), nd.empty((K, C, R, S), ctx), cell))
+    try:
+        for k in (3, 4):
+            gpu_op.hold_products(k == 4)
+            for call in calls:
+                gpu_op.convolution_backward_filter(call[0], call[1], call[2], call[k], call[5], handle, stream)
+        gpu_op.hold_products(False)
+        before = gpu_op.launch_count()
+        gpu_op.launch_held(stream)
+        assert gpu_op.launch_count() - before == 2 * len({call[2].shape[3] for call in calls})
+    finally:
+        gpu_op.drop_held()
+    for call in calls:
+        np.testing.assert_array_equal(call[4].asnumpy(), call[3].asnumpy())

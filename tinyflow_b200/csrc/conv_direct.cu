@@ -13,6 +13,7 @@
 // gradients 16.7 -> 10.0 and 12.4 -> 6.1.
 #include "common.h"
 #include <algorithm>
+#include <vector>
 
 namespace tf {
 
@@ -137,14 +138,14 @@ struct DirectWgrad {
 };
 constexpr int kWgradThreads = 512, kWgradItems = 4;
 
+// Share `block` of `blocks` of the images of a layer; every block of the launch calls it with the same shared memory
 template <int S, int IT>
-__global__ void __launch_bounds__(kWgradThreads) direct_wgrad_kernel(const DirectWgrad p) {
+__device__ __forceinline__ void direct_wgrad(const DirectWgrad& p, int block, int blocks) {
   extern __shared__ __align__(16) float direct_smem[];
   float* xs = direct_smem;                          // [C][hp][wp]
   float* ds = direct_smem + p.dy_at;                // [K][P][Q]
   const int plane = p.image.plane, wp = p.image.wp;
   clear_halo(xs, p.image);
-  grid_dep_sync();
   const int slice = IT == 1 ? threadIdx.x / p.items : 0, first = IT == 1 ? threadIdx.x - slice * p.items : threadIdx.x;
   const bool live = slice < p.slices;
   float acc[IT][S];
@@ -152,7 +153,7 @@ __global__ void __launch_bounds__(kWgradThreads) direct_wgrad_kernel(const Direc
   for (int i = 0; i < IT; ++i)
 #pragma unroll
     for (int s = 0; s < S; ++s) acc[i][s] = 0.f;
-  for (int n = blockIdx.x; n < p.N; n += gridDim.x) {
+  for (int n = block; n < p.N; n += blocks) {
     __syncthreads();
     const float* dsrc = p.dy + (long long)n * p.K * p.P * p.Q;
     copy_image(xs, p.x + (long long)n * p.C * p.image.h * p.image.w, p.image);
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(kWgradThreads) direct_wgrad_kernel(const Direc
       }
     }
   }
-  float* out = p.part + (long long)blockIdx.x * p.items * S;
+  float* out = p.part + (long long)block * p.items * S;
   if (IT > 1 || p.slices == 1) {
 #pragma unroll
     for (int it = 0; it < IT; ++it) {
@@ -222,11 +223,15 @@ __global__ void __launch_bounds__(kWgradThreads) direct_wgrad_kernel(const Direc
     out[i] = t;
   }
 }
-// out[c] = sum over the blocks' partial filters, in block order within each of 32 warps
-__global__ void __launch_bounds__(1024) direct_wgrad_sum_kernel(const float* __restrict__ part, float* __restrict__ out, int rows, int cols) {
-  __shared__ float sm[32][33];
+template <int S, int IT>
+__global__ void __launch_bounds__(kWgradThreads) direct_wgrad_kernel(const DirectWgrad p) {
   grid_dep_sync();
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = blockIdx.x * 32 + tx;
+  direct_wgrad<S, IT>(p, blockIdx.x, gridDim.x);
+}
+// out[c] = sum over the blocks' partial filters, in block order within each of 32 warps
+__device__ __forceinline__ void direct_wgrad_sum(const float* __restrict__ part, float* __restrict__ out, int rows, int cols, int block) {
+  __shared__ float sm[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, c = block * 32 + tx;
   float acc = 0.f;
   if (c < cols) {
 #pragma unroll 10
@@ -240,6 +245,31 @@ __global__ void __launch_bounds__(1024) direct_wgrad_sum_kernel(const float* __r
     for (int j = 0; j < 32; ++j) t += sm[j][tx];
     out[c] = t;
   }
+}
+
+__global__ void __launch_bounds__(1024) direct_wgrad_sum_kernel(const float* __restrict__ part, float* __restrict__ out, int rows, int cols) {
+  grid_dep_sync();
+  direct_wgrad_sum(part, out, rows, cols, blockIdx.x);
+}
+// Layers whose gradients may wait (see hold_products in gemm_tcgen05.cu) share both launches: the two of LeNet at batch 256 took 24 us one after
+// the other, 20 together.  Blocks and order of the sums are those of the separate launches.
+constexpr int kWgradJobs = 8;
+struct DirectJob { DirectWgrad d; float* out; int blocks, cols, first, first_sum; };
+struct DirectJobs { int n; DirectJob job[kWgradJobs]; };
+template <int S>
+__global__ void __launch_bounds__(kWgradThreads) direct_wgrad_group_kernel(const __grid_constant__ DirectJobs jobs) {
+  grid_dep_sync();
+  int k = 0;
+  while (k + 1 < jobs.n && jobs.job[k + 1].first <= (int)blockIdx.x) ++k;
+  const DirectJob& j = jobs.job[k];
+  direct_wgrad<S, 1>(j.d, (int)blockIdx.x - j.first, j.blocks);
+}
+__global__ void __launch_bounds__(1024) direct_wgrad_group_sum_kernel(const __grid_constant__ DirectJobs jobs) {
+  grid_dep_sync();
+  int k = 0;
+  while (k + 1 < jobs.n && jobs.job[k + 1].first_sum <= (int)blockIdx.x) ++k;
+  const DirectJob& j = jobs.job[k];
+  direct_wgrad_sum(j.d.part, j.out, j.blocks, j.cols, (int)blockIdx.x - j.first_sum);
 }
 
 constexpr size_t kDirectSmem = 96 * 1024;
@@ -306,6 +336,47 @@ template <int S> static int launch_wgrad(const DirectWgrad& d, int grid, size_t 
   TF_CUDA(launch_dep(kernel, dim3(grid), dim3(kWgradThreads), smem, s, d));
   return 0;
 }
+struct HeldDirect { DirectJob job; int S; size_t smem; double flops; };
+static thread_local std::vector<HeldDirect> t_held_direct;
+void drop_held_direct() { t_held_direct.clear(); }
+template <int S> static int launch_direct_group(const DirectJobs& jobs, int blocks, size_t smem, cudaStream_t s) {
+  TF_CUDA(cudaFuncSetAttribute(direct_wgrad_group_kernel<S>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDirectSmem));
+  TF_CUDA(launch_dep(direct_wgrad_group_kernel<S>, dim3(blocks), dim3(kWgradThreads), smem, s, jobs));
+  return 0;
+}
+int launch_held_direct(cudaStream_t s) {
+  std::vector<HeldDirect> all;
+  all.swap(t_held_direct);
+  for (int S : {3, 5, 7}) {
+    size_t at = 0;
+    while (true) {
+      DirectJobs jobs;
+      jobs.n = 0;
+      int blocks = 0, sums = 0;
+      size_t smem = 0, floats = 0;
+      double flops = 0;
+      for (; at < all.size() && jobs.n < kWgradJobs; ++at) {
+        if (all[at].S != S) continue;
+        DirectJob& j = jobs.job[jobs.n++] = all[at].job;
+        j.first = blocks; blocks += j.blocks;
+        j.first_sum = sums; sums += (j.cols + 31) / 32;
+        smem = std::max(smem, all[at].smem); floats += (size_t)j.blocks * j.cols; flops += all[at].flops;
+      }
+      if (!jobs.n) break;
+      StreamLease lease(s);
+      float* part = (float*)lease.scratch(kScratchContract, sizeof(float) * floats);
+      TF_REQUIRE(part, "filter gradients: no memory for %zu bytes of partial sums", sizeof(float) * floats);
+      for (int i = 0; i < jobs.n; ++i) { jobs.job[i].d.part = part; part += (size_t)jobs.job[i].blocks * jobs.job[i].cols; }
+      note_compute_stream(s);
+      KernelTimer kt("direct_conv", s, flops, 0, 1);
+      if ((S == 3 ? launch_direct_group<3>(jobs, blocks, smem, s) : S == 5 ? launch_direct_group<5>(jobs, blocks, smem, s) : launch_direct_group<7>(jobs, blocks, smem, s)) != 0) return -1;
+      TF_AFTER(s, "filter gradients");
+      TF_CUDA(launch_dep(direct_wgrad_group_sum_kernel, dim3(sums), dim3(1024), 0, s, jobs));
+      TF_AFTER(s, "filter gradients");
+    }
+  }
+  return 0;
+}
 int direct_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float* dw, cudaStream_t s) {
   if (!direct_shape(p) || p->K * p->C * p->R > kWgradThreads * kWgradItems) return 0;
   DirectWgrad d{x, dy, nullptr, p->N, p->C, p->K, p->P, p->Q, p->R, HaloImage{p->C, p->H, p->W, p->P + p->R - 1, 0, p->pad_h, p->pad_w, 0, p->H, p->W}, p->K * p->C * p->R, 1, p->P};
@@ -322,6 +393,10 @@ int direct_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float*
   if (d.slices > 1 && floats < (size_t)d.slices * d.items * p->S) floats = (size_t)d.slices * d.items * p->S;
   if (floats * sizeof(float) > kDirectSmem) return 0;
   const int cols = d.items * p->S, grid = p->N < 2 * device_sm_count() ? p->N : 2 * device_sm_count();
+  if (d.items <= kWgradThreads && may_hold(s)) {
+    t_held_direct.push_back(HeldDirect{DirectJob{d, dw, grid, cols, 0, 0}, p->S, floats * sizeof(float), 2.0 * p->N * p->K * p->P * p->Q * p->C * p->R * p->S});
+    return 1;
+  }
   StreamLease lease(s);
   d.part = (float*)lease.scratch(kScratchContract, sizeof(float) * (size_t)grid * cols);
   if (!d.part) return 0;

@@ -2252,8 +2252,10 @@ int launch_held_simt(cudaStream_t s);       // gemm_simt.cu: weight gradients of
 void drop_held_simt();
 int launch_held_sums(cudaStream_t s);       // ops_basic.cu: bias gradients
 void drop_held_sums();
+int launch_held_direct(cudaStream_t s);     // conv_direct.cu: filter gradients of layers of few channels
+void drop_held_direct();
 void hold_products(bool on) { t_hold = on; }
-void drop_held() { t_held.clear(); t_held_work = 0; t_hold = false; drop_held_simt(); drop_held_sums(); }
+void drop_held() { t_held.clear(); t_held_work = 0; t_hold = false; drop_held_simt(); drop_held_sums(); drop_held_direct(); }
 // The call may wait: its caller says so, and no graph of the caller's own is being captured (it would copy from a table that is gone)
 bool may_hold(cudaStream_t s) {
   if (!t_hold) return false;
@@ -2365,6 +2367,7 @@ static int launch_held_filters(cudaStream_t s) {
 }
 int launch_held(cudaStream_t s) try {
   if (int rc = launch_held_filters(s)) return rc;
+  if (int rc = launch_held_direct(s)) return rc;
   if (int rc = launch_held_simt(s)) return rc;
   return launch_held_sums(s);
 } catch (const std::bad_alloc&) { TF_FAIL("gradients that waited: out of host memory"); }
