@@ -2264,6 +2264,7 @@ bool may_hold(cudaStream_t s) {
   return capture == cudaStreamCaptureStatusNone;
 }
 
+constexpr size_t kStagedCopy = 1 << 16;
 template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>& held, cudaStream_t s, double flops) {
   static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_group_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem<BN>);
   TF_CUDA(attr);
@@ -2332,7 +2333,9 @@ template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>
     dev = (char*)recording_own(table);                // lives and is uploaded with the recording
   } else {
     dev = (char*)lease.scratch(kScratchGroup, table.size());
-    if (dev) TF_CUDA(cudaMemcpyAsync(dev, table.data(), table.size(), cudaMemcpyHostToDevice, s));       // pageable: staged before the call returns
+    // pageable: staged before the call returns, without waiting for the stream up to 64 KB a copy
+    for (size_t at = 0; dev && at < table.size(); at += kStagedCopy)
+      TF_CUDA(cudaMemcpyAsync(dev + at, table.data() + at, std::min(kStagedCopy, table.size() - at), cudaMemcpyHostToDevice, s));
   }
   TF_REQUIRE(dev, "filter gradients: no memory for a table of %zu bytes", table.size());
   t.problems = (const GemmParams*)dev; t.items = (const int4*)(dev + at_items); t.sums = (const int4*)(dev + at_sums); t.first = (const int*)(dev + at_first);

@@ -404,7 +404,7 @@ class Executor(object):
         previous.pop(self.targetloss.index, None)        # the loss belongs to the caller
         shapes, timed = self.node_to_shape_map, self.top_message_queue is not None
         together = not (self.have_plan or timed or gpu_op.data_parallel_active())
-        updates = []
+        updates, holding = [], False
         if together and self._convs and all(n.inputs[1] in self._feed for n in self._convs):
             self._pack_filters(stream)
         for node in self.topo_order:
@@ -434,13 +434,10 @@ class Executor(object):
             if self.have_plan:
                 for idx in node.recompute_list:
                     self._compute(self.topo_order[idx], None, stream)
-            if together and node in self._patient:
-                gpu_op.hold_products(True)
-                try:
-                    self._compute(node, out, stream)
-                finally:
-                    gpu_op.hold_products(False)
-            elif timed:
+            if together and (node in self._patient) != holding:        # an error drops what is held, and the switch
+                holding = not holding
+                gpu_op.hold_products(holding)
+            if timed:
                 t0 = time.perf_counter()
                 self._compute(node, out, stream)
                 node.runtime = (time.perf_counter() - t0) * 1000.0
@@ -449,6 +446,8 @@ class Executor(object):
             if self.have_plan:
                 self._after_node(node)
         if together:
+            if holding:
+                gpu_op.hold_products(False)
             gpu_op.launch_held(stream)
         if updates:
             self._update_parameters(updates, stream)
