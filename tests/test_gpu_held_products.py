@@ -26,11 +26,13 @@ def test_products_held_back_have_the_bits_of_separate_launches(lib_path, monkeyp
 
 # N, C, H, W, K, R, S, stride: with and without several taps a tile, odd numbers of 64-channel blocks, ragged tiles, cut and whole reductions
 LAYERS = [(2, 64, 9, 9, 96, 3, 3, 1), (3, 160, 12, 7, 160, 7, 1, 1), (2, 33 * 4, 9, 9, 68, 1, 7, 1), (5, 64, 14, 14, 256, 1, 1, 1), (5, 256, 14, 14, 64, 1, 1, 1),
-          (4, 288, 17, 17, 384, 3, 3, 2), (1, 48, 21, 21, 64, 5, 5, 1), (16, 96, 35, 35, 64, 1, 1, 1), (2, 768, 17, 17, 192, 1, 1, 1), (8, 128, 28, 28, 32, 3, 3, 1), (2, 3, 75, 75, 32, 3, 3, 2)]
+          (4, 288, 17, 17, 384, 3, 3, 2), (1, 48, 21, 21, 64, 5, 5, 1), (16, 96, 35, 35, 64, 1, 1, 1), (2, 768, 17, 17, 192, 1, 1, 1), (8, 128, 28, 28, 32, 3, 3, 1), (2, 3, 75, 75, 32, 3, 3, 2),
+          # runs of 4 pieces: 9, 16, 17 and more of one tile, kept to a CTA's chunks among the others and dealt out one by one alone
+          (2, 128, 17, 17, 128, 1, 1, 1), (4, 128, 16, 16, 128, 1, 1, 1), (17, 128, 8, 8, 128, 1, 1, 1), (9, 256, 17, 17, 96, 1, 1, 1)]
 
 
 @pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
-@pytest.mark.parametrize("layers", [LAYERS, LAYERS[:1], LAYERS[7:8]], ids=["all", "one", "one cut"])
+@pytest.mark.parametrize("layers", [LAYERS, LAYERS[:1], LAYERS[7:8], LAYERS[-4:]], ids=["all", "one", "one cut", "runs"])
 def test_layers_in_one_launch(lib_path, layers, arith):
     from tinyflow_b200 import gpu_op, ndarray as nd
     ctx, stream, rng = nd.gpu(0), gpu_op.create_cudaStream(), np.random.RandomState(1)

@@ -32,6 +32,7 @@
 // sets so that promoting one group of stages to registers overlaps the MMAs of the next.  Every mbarrier wait is bounded: on
 // time-out the CTA raises an error flag the host reads, drains its outstanding copies, frees its TMEM and returns.
 #include "common.h"
+#include <cfloat>
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <algorithm>
@@ -421,6 +422,7 @@ struct alignas(128) GemmParams {
   int a_rows, a_slots, b_slots, b_resident;
   int one_ring;                   // A and B of a stage share slot number and barriers (every block serves one stage)
   const void *pack_a, *pack_b;    // host side: the packs that the operands are (filter gradients)
+  int sum_run;                    // pieces that reduce_partials_kernel adds in one run (see reduce_tile)
   int hold;                       // host side: the product may wait for others (a filter gradient; see hold_products)
   int acc_mode;                   // where the accumulators sit in TMEM: kAccPair or kAccThree (see the MMA issuer)
   int cross_groups;               // kAccThree: groups whose cross terms accumulate before they are promoted
@@ -1016,7 +1018,7 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
     cluster_sync_all();
     if (!*abort_flag) {
       for (int c0 = BN * rank / p.cluster + (int)threadIdx.x / BM; c0 < c1; c0 += kUnroll * kLanes) {
-        float sum[kUnroll] = {0.f, 0.f, 0.f, 0.f};
+        float sum[kUnroll] = {0.f, 0.f, 0.f, 0.f}, rest[kUnroll] = {0.f, 0.f, 0.f, 0.f};
         float v[kMaxCluster][kUnroll];
 #pragma unroll
         for (int r = 0; r < kMaxCluster; ++r)
@@ -1029,10 +1031,11 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
         for (int r = 0; r < kMaxCluster; ++r)
           if (r < p.cluster) {
 #pragma unroll
-            for (int j = 0; j < kUnroll; ++j) sum[j] += v[r][j];
+            for (int j = 0; j < kUnroll; ++j) (r < kMaxCluster / 2 ? sum : rest)[j] += v[r][j];
           }
 #pragma unroll
         for (int j = 0; j < kUnroll; ++j) {
+          sum[j] += rest[j];                  // runs of kSumChunk, as reduce_tile adds them
           const int c = c0 + j * kLanes;
           if (ra.ok && c < c1) {
             p.out[ra.base + (long long)(nt * BN + c) * ra.col_stride] = sum[j] * inv_scale;
@@ -1066,17 +1069,20 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
 // executor lets the library hold them back (hold_product), and one launch works through the tiles of several, dealt to the CTAs so
 // that all finish together: whole tiles where the reduction is short, their pieces where it is long.
 //
-// The bits are those of the separate launches: a tile kept whole is still added up piece by piece, in the order of the pieces, with
-// the same accumulator blocks; the second set of sums just fits the 168 registers a thread can have.  Roles: warps 0 and 3 copy A and B,
+// The bits are those of the separate launches: a tile kept whole (or one of its chunks of kSumChunk pieces, see reduce_tile) is
+// still added up piece by piece, in the order of the pieces, with the same accumulator blocks; the second set of sums just fits the
+// 168 registers a thread can have.  Roles: warps 0 and 3 copy A and B,
 // 1 and 2 issue, 4-11 epilogue.  Both operands M/N-major, groups of one stage.
 // A step of Inception-v3 at batch 2 has 94 of them, 1.1 ms in separate launches and 0.22 in two: 4495 -> 3702 us.  ResNet-50 at batch 19
 // 4453 -> 3938, DenseNet-121 at batch 32 14.58 -> 13.39 ms.
 // ------------------------------------------------------------------------------------------------
+constexpr int kSumChunk = 4;      // pieces added in order before their sum goes to the tile's
+static_assert(2 * kSumChunk == kMaxCluster, "the sum over a cluster takes two runs");
 struct GroupTable {
   const GemmParams* problems;
-  const int4* items;              // {problem, tile, piece or -1: all of the tile's pieces, workspace slot of the piece}
+  const int4* items;              // {problem, tile, pieces or -1: all of the tile's, the workspace slot of their sum}; pieces: the first + (their number << 16)
   const int* first;               // CTA -> its first item; one more than CTAs
-  const int4* sums;               // tiles whose pieces were dealt out: {problem, tile, slot of the first piece, slots between pieces}
+  const int4* sums;               // tiles that were dealt out: {problem, tile, their first slot, from one to the next; negative: each holds a chunk, not a piece}
   float* workspace;
   int* err;
 };
@@ -1100,8 +1106,8 @@ struct GroupIter {
       q = t.problems + item.x;
       k_total = q->k_total;
       pieces = tile_pieces(*q, item.y);
-      piece = max(item.z, 0);
-      last = item.z < 0 ? pieces - 1 : piece;
+      piece = item.z < 0 ? 0 : item.z & 0xffff;
+      last = item.z < 0 ? pieces - 1 : piece + (item.z >> 16) - 1;
     }
     k0 = (int)((long long)k_total * piece / pieces);
     kcount = (int)((long long)k_total * (piece + 1) / pieces) - k0;
@@ -1287,15 +1293,15 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_group_kernel(const __g
         if (lane == 0) mbar_arrive(&acc_empty[acc]);
       }
       if (!ok) break;
-      if (iter.item.z >= 0) {                   // one piece: raw sums for reduce_group_kernel
-        float* ws = t.workspace + (size_t)iter.item.w * BN * BM + half * HC * BM + row_in_tile;
-#pragma unroll
-        for (int q = 0; q < HC / 2; ++q) { ws[(size_t)(2 * q) * BM] = accv[q].x; ws[(size_t)(2 * q + 1) * BM] = accv[q].y; }
-        continue;
-      }
 #pragma unroll
       for (int q = 0; q < HC / 2; ++q) total[q] = __fadd2_rn(total[q], accv[q]);
       if (!done) continue;
+      if (iter.item.z >= 0) {                   // not the whole tile: raw sums for reduce_group_kernel
+        float* ws = t.workspace + (size_t)iter.item.w * BN * BM + half * HC * BM + row_in_tile;
+#pragma unroll
+        for (int q = 0; q < HC / 2; ++q) { ws[(size_t)(2 * q) * BM] = total[q].x; ws[(size_t)(2 * q + 1) * BM] = total[q].y; }
+        continue;
+      }
       const GemmParams& q = *iter.q;
       int mt, nt, tap;
       decode_tile(q, iter.item.y, mt, nt, tap);
@@ -1534,7 +1540,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_pair_kernel(const __grid_c
 }
 
 // Adds up the pieces of every split tile in piece order and writes the result where the GEMM's own epilogue would have: the order
-// in which the grouped kernel adds them where it keeps a tile to itself, so both give the same bits.  Bound by latency.
+// in which the grouped kernel adds them where it keeps a tile to itself, so both give the same bits.  Every `chunk`
+// pieces (one where no grouped kernel adds them, else kSumChunk) their sum goes to the tile's, whose rounding errors are carried along
+// (two-sum): with 49 pieces in one run the error of a filter gradient is 20 % larger.  Bound by latency.
 //   MANY = false (tiles of few pieces; the blocks' starts are what counts): grid (tiles, BN / 8), 256 threads, a thread has 4 columns
 //     of 4 pieces in flight.
 //   MANY = true (few tiles of many pieces): grid (tiles, BN / 8, 4), 16 warps take three pieces of 8 columns x 32 rows each to shared
@@ -1543,15 +1551,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm3x_pair_kernel(const __grid_c
 constexpr int kReduceCols = 8;
 template <bool MANY> constexpr int kReduceThreads = MANY ? 512 : 256;
 template <int BN, bool MANY, class Piece>
-__device__ __forceinline__ void reduce_tile(const GemmParams& p, int tile, int pieces, Piece&& piece) {
+__device__ __forceinline__ void reduce_tile(const GemmParams& p, int tile, int pieces, int chunk, Piece&& piece) {
   int mt, nt, tap;
   decode_tile(p, tile, mt, nt, tap);
   constexpr int COLS = MANY ? 1 : 4;
   const int row = MANY ? blockIdx.z * 32 + (threadIdx.x & 31) : threadIdx.x & (BM - 1);
   const int c0 = blockIdx.y * kReduceCols + (MANY ? threadIdx.x / 32 : threadIdx.x / BM * COLS);
-  float sum[COLS];
+  float sum[COLS], run[COLS], lost[COLS];
 #pragma unroll
-  for (int q = 0; q < COLS; ++q) sum[q] = 0.f;
+  for (int q = 0; q < COLS; ++q) sum[q] = run[q] = lost[q] = 0.f;
+  auto close_run = [&](int q) {
+    const float s = __fadd_rn(sum[q], run[q]), b = __fsub_rn(s, sum[q]);
+    lost[q] = __fadd_rn(lost[q], __fadd_rn(__fsub_rn(sum[q], __fsub_rn(s, b)), __fsub_rn(run[q], b)));
+    sum[q] = s;
+    run[q] = 0.f;
+  };
   if (MANY) {
     constexpr int kEach = 3, kAtOnce = 16 * kEach;
     __shared__ float held[kAtOnce][kReduceCols][32];
@@ -1575,7 +1589,10 @@ __device__ __forceinline__ void reduce_tile(const GemmParams& p, int tile, int p
       __syncthreads();
       const int n = min(kAtOnce, pieces - g0);
       if (warp < kReduceCols)
-        for (int i = 0; i < n; ++i) sum[0] += held[i][warp][lane];
+        for (int i = 0; i < n; ++i) {
+          run[0] = __fadd_rn(run[0], held[i][warp][lane]);
+          if (((i + 1) & (chunk - 1)) == 0) close_run(0);
+        }
     }
     if (warp >= kReduceCols) return;
   } else {
@@ -1594,9 +1611,18 @@ __device__ __forceinline__ void reduce_tile(const GemmParams& p, int tile, int p
       for (int d = 0; d < DEPTH; ++d)
         if (g + d < pieces) {
 #pragma unroll
-          for (int q = 0; q < COLS; ++q) sum[q] += v[d][q];
+          for (int q = 0; q < COLS; ++q) {
+            run[q] = __fadd_rn(run[q], v[d][q]);
+            if (((g + d + 1) & (chunk - 1)) == 0) close_run(q);
+          }
         }
     }
+  }
+#pragma unroll
+  for (int q = 0; q < COLS; ++q) {
+    close_run(q);
+    // infinities and NaN as a plain sum has them
+    if (fabsf(sum[q]) <= FLT_MAX) sum[q] = __fadd_rn(sum[q], lost[q]);
   }
   const RowAddr ra = row_address(p, mt, tap, row);
   const float inv_scale = (1.f / __ldg(p.a_scale)) * (1.f / __ldg(p.b_scale));
@@ -1623,7 +1649,7 @@ __global__ void __launch_bounds__(kReduceThreads<MANY>) reduce_partials_kernel(c
   const bool aligned = p.tail_pieces > 0;
   const int first = aligned ? 0 : (int)(((long long)t * p.k_total) / p.tail_share);
   const int last = aligned ? p.tail_pieces - 1 : (int)((((long long)t + 1) * p.k_total - 1) / p.tail_share);
-  reduce_tile<BN, MANY>(p, p.full_tiles + t, last - first + 1, [&](int i) -> const float* {
+  reduce_tile<BN, MANY>(p, p.full_tiles + t, last - first + 1, p.sum_run, [&](int i) -> const float* {
     const int g = first + i;
     const int slot = aligned ? g * p.tail_tiles + t : g * p.slots_per_cta + (t - (int)(((long long)g * p.tail_share) / p.k_total));
     return p.workspace + (size_t)slot * BN * BM;
@@ -1635,7 +1661,9 @@ __global__ void __launch_bounds__(kReduceThreads<MANY>) reduce_group_kernel(cons
   grid_dep_sync();
   const int4 e = __ldg(t.sums + blockIdx.x);
   const GemmParams& p = t.problems[e.x];
-  reduce_tile<BN, MANY>(p, e.y, tile_pieces(p, e.y), [&](int g) -> const float* { return t.workspace + (size_t)(e.z + g * e.w) * BN * BM; });
+  const int pieces = tile_pieces(p, e.y), between = abs(e.w);
+  reduce_tile<BN, MANY>(p, e.y, e.w < 0 ? (pieces + kSumChunk - 1) / kSumChunk : pieces, e.w < 0 ? 1 : kSumChunk,
+                        [&](int g) -> const float* { return t.workspace + (size_t)(e.z + g * between) * BN * BM; });
 }
 
 // Exercises the bounded wait on its own: one thread waits, with a short limit, on a barrier that nothing arms; the wait
@@ -2179,6 +2207,11 @@ template <int BN, class F> static cudaError_t launch_reduce(int tiles, int piece
   if (pieces >= 12 && tiles * (BN / kReduceCols) <= 2 * device_sm_count()) return launch(std::true_type(), dim3(grid.x, grid.y, BM / 32), dim3(kReduceThreads<true>));
   return launch(std::false_type(), grid, dim3(kReduceThreads<false>));
 }
+template <int BN> constexpr int kHeldRun = BN == 64 ? 160 : 24;
+// By its schedule the product could wait for others (see held_back)
+template <int BN> static bool could_wait(const GemmParams& p) {
+  return BN != 96 && p.group_iters == 1 && p.acc_mode == kAccPair && longest_run(p) < kHeldRun<BN> && (p.tail_share == 0 || p.tail_pieces > 0);
+}
 // Schedule, stages per accumulator group and accumulator blocks of a launch: what decides the bits of its result
 template <int BN, int AR> static size_t plan_launch(GemmParams& p) {
   const size_t bytes = plan_schedule(p, BN, max_clusters_of<BN, AR>);
@@ -2192,6 +2225,7 @@ template <int BN, int AR> static size_t plan_launch(GemmParams& p) {
   // Groups of one stage begin the main sum anew with two instructions instead of a wide one: equal at 22 stages, 4 % faster
   // at 55, 9 % at 841 (512 -> 512 channels, 28 x 28, 3x3, batch 64: 750 -> 673 us).
   p.acc_mode = BN != 64 && p.k_total > p.group_iters && longest_run(p) >= (BN == 128 && p.group_iters > 1 ? 8 : 24) ? kAccThree : kAccPair;
+  p.sum_run = could_wait<BN>(p) ? kSumChunk : 1;
   return bytes;
 }
 template <int BN, int AR> static bool held_back(const GemmParams& p, cudaStream_t s, double flops);
@@ -2246,7 +2280,6 @@ static thread_local std::vector<HeldProduct> t_held;
 static thread_local double t_held_work = 0;           // tiles x stages
 // Stages per CTA from which a product is launched on its own: at 128 columns those that take two issuers (groups hold products of one
 // layout of the accumulators); at 64 columns 102 still gain (DenseNet-121 13.76 -> 13.50 ms against a limit of 24).
-template <int BN> constexpr int kHeldRun = BN == 64 ? 160 : 24;
 constexpr int kHeldWork = 1024;                       // stages per SM that are launched together at the latest (64: ResNet-50 b19 4096 us, 256: 3999, 512 and all: 3976)
 int launch_held_simt(cudaStream_t s);       // gemm_simt.cu: weight gradients of dense layers
 void drop_held_simt();
@@ -2269,7 +2302,7 @@ template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>
   static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_group_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem<BN>);
   TF_CUDA(attr);
   const int sms = device_sm_count();
-  // Whole tiles up to half of a CTA's share (a fifth: 0.3 % slower); longer reductions as their pieces.  Longest first, to the CTA that is free first.
+  // Whole tiles, or chunks of their pieces, up to half of a CTA's share (a fifth: 0.3 % slower); longer reductions as their pieces.  Longest first, to the CTA that is free first.
   constexpr int kItemCost = 4;                        // an item's start and end, in stages
   struct Item { int4 what; int stages; };
   std::vector<Item> items;
@@ -2281,46 +2314,56 @@ template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>
   for (int i = 0; i < (int)held.size(); ++i) {
     const GemmParams& g = *held[i];
     const int tiles = g.m_tiles * g.n_tiles * g.tap_tiles;
-    for (int piece = 0, more = 1; more; ++piece) {      // the pieces of one range of stages side by side
+    const int width = g.k_total <= whole ? kSumChunk : 1;
+    for (int part = 0, more = 1; more; ++part) {        // the parts of one range of stages side by side
       more = 0;
       for (int tile = 0; tile < tiles; ++tile) {
-        const int n = tile_pieces(g, tile);
-        if (n == 1 || g.k_total <= whole) {
-          if (piece == 0) items.push_back({make_int4(i, tile, -1, 0), g.k_total});
+        const int n = tile_pieces(g, tile), parts = (n + width - 1) / width;
+        if (parts == 1) {
+          if (part == 0) items.push_back({make_int4(i, tile, -1, 0), g.k_total});
           continue;
         }
-        if (piece >= n) continue;
+        if (part >= parts) continue;
         const int split = tiles - (g.cluster > 1 ? 0 : g.full_tiles), t = tile - (tiles - split);
-        if (piece == 0) { sums.push_back(make_int4(i, tile, slots + t, split)); most_pieces = std::max(most_pieces, n); }
-        items.push_back({make_int4(i, tile, piece, slots + piece * split + t), (int)((long long)g.k_total * (piece + 1) / n - (long long)g.k_total * piece / n)});
-        if (piece + 1 < n) more = 1;
-        else if (tile + 1 == tiles) slots += n * split;
+        const int first = part * width, end = std::min(n, first + width);
+        if (part == 0) { sums.push_back(make_int4(i, tile, slots + t, width > 1 ? -split : split)); most_pieces = std::max(most_pieces, parts); }
+        items.push_back({make_int4(i, tile, first + ((end - first) << 16), slots + part * split + t), (int)((long long)g.k_total * end / n - (long long)g.k_total * first / n)});
+        if (part + 1 < parts) more = 1;
+        else if (tile + 1 == tiles) slots += parts * split;
       }
     }
   }
-  std::stable_sort(items.begin(), items.end(), [](const Item& a, const Item& b) { return a.stages > b.stages; });
-  const int grid = std::min(sms, (int)items.size());
-  std::vector<std::vector<int4>> of(grid);
-  std::vector<std::pair<int, int>> heap;               // (-load, -cta): the least loaded on top
-  for (int c = 0; c < grid; ++c) heap.push_back({0, -c});
-  std::make_heap(heap.begin(), heap.end());
-  for (const Item& it : items) {
-    std::pop_heap(heap.begin(), heap.end());
-    of[-heap.back().second].push_back(it.what);
-    heap.back().first -= it.stages + kItemCost;
-    std::push_heap(heap.begin(), heap.end());
+  const int count = (int)items.size(), grid = std::min(sms, count);
+  std::vector<int> order(count), cta(count), first(grid + 1, 0);
+  {
+    int longest = 0;
+    for (const Item& it : items) longest = std::max(longest, it.stages);
+    std::vector<int> at(longest + 2, 0);
+    for (const Item& it : items) ++at[longest - it.stages + 1];
+    for (int k = 0; k <= longest; ++k) at[k + 1] += at[k];
+    for (int i = 0; i < count; ++i) order[at[longest - items[i].stages]++] = i;
   }
+  std::vector<long long> heap(grid);                   // load * 65536 + CTA, the least first
+  for (int c = 0; c < grid; ++c) heap[c] = c;
+  for (int i : order) {
+    cta[i] = (int)(heap[0] & 0xffff);
+    ++first[cta[i] + 1];
+    const long long now = heap[0] + (long long)(items[i].stages + kItemCost) * 65536;
+    int at = 0;
+    for (int below; (below = 2 * at + 1) < grid; at = below) {
+      if (below + 1 < grid && heap[below + 1] < heap[below]) ++below;
+      if (heap[below] >= now) break;
+      heap[at] = heap[below];
+    }
+    heap[at] = now;
+  }
+  for (int c = 0; c < grid; ++c) first[c + 1] += first[c];
   // one table on the device: the problems, the items of every CTA, the sums
   const size_t at_items = held.size() * sizeof(GemmParams), at_sums = at_items + items.size() * sizeof(int4), at_first = at_sums + sums.size() * sizeof(int4);
   std::vector<char> table(at_first + (grid + 1) * sizeof(int));
   for (size_t i = 0; i < held.size(); ++i) memcpy(table.data() + i * sizeof(GemmParams), held[i], sizeof(GemmParams));
-  int n = 0;
-  for (int c = 0; c < grid; ++c) {
-    memcpy(table.data() + at_first + c * sizeof(int), &n, sizeof(int));
-    memcpy(table.data() + at_items + n * sizeof(int4), of[c].data(), of[c].size() * sizeof(int4));
-    n += (int)of[c].size();
-  }
-  memcpy(table.data() + at_first + grid * sizeof(int), &n, sizeof(int));
+  memcpy(table.data() + at_first, first.data(), (grid + 1) * sizeof(int));
+  for (int i : order) memcpy(table.data() + at_items + sizeof(int4) * first[cta[i]]++, &items[i].what, sizeof(int4));
   if (!sums.empty()) memcpy(table.data() + at_sums, sums.data(), sums.size() * sizeof(int4));
   StreamLease lease(s);
   GroupTable t;
@@ -2382,7 +2425,7 @@ static int release_held(const void* hi, cudaStream_t s) {
 }
 // Takes the product if it may wait; what has gathered goes when it fills the SMs.
 template <int BN, int AR> static bool held_back(const GemmParams& p, cudaStream_t s, double flops) {
-  if (BN == 96 || p.group_iters != 1 || p.acc_mode != kAccPair || longest_run(p) >= kHeldRun<BN> || (p.tail_share > 0 && p.tail_pieces == 0) || p.amax) return false;
+  if (!could_wait<BN>(p) || p.amax) return false;
   if (!may_hold(s)) return false;
   t_held.push_back(HeldProduct{p, BN, AR, flops});
   t_held_work += (double)p.m_tiles * p.n_tiles * p.tap_tiles * p.k_total;
