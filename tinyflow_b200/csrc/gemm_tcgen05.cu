@@ -1073,7 +1073,8 @@ __global__ void __launch_bounds__(kGemmThreads, 1) gemm3x_kernel(const __grid_co
 // still added up piece by piece, in the order of the pieces, with the same accumulator blocks; the second set of sums just fits the
 // 168 registers a thread can have.  Roles: warps 0 and 3 copy A and B,
 // 1 and 2 issue, 4-11 epilogue.  Both operands M/N-major, groups of one stage.
-// A step of Inception-v3 at batch 2 has 94 of them, 1.1 ms in separate launches and 0.22 in two: 4495 -> 3702 us.  ResNet-50 at batch 19
+// A step of Inception-v3 at batch 2 has 94 of them, 1.1 ms in separate launches and 0.22 in two: 4495 -> 3702 us
+// (chunks instead of whole tiles 0.06 more, see reduce_tile).  ResNet-50 at batch 19
 // 4453 -> 3938, DenseNet-121 at batch 32 14.58 -> 13.39 ms.
 // ------------------------------------------------------------------------------------------------
 constexpr int kSumChunk = 4;      // pieces added in order before their sum goes to the tile's
