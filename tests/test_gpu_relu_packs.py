@@ -84,3 +84,50 @@ def test_relu_backward_behind_a_pool_writes_the_packed_gradient(env, case):
     for got in results:
         np.testing.assert_array_equal(got[2], np.where(got[0] > 0, got[1], np.float32(0)))
         assert np.max(np.abs(got[3] - results[0][3])) <= 2e-6 * np.max(np.abs(results[0][3]))
+
+
+# channel 0 in front of the ReLU is negative and large, and so is its gradient: the bounds that fused packs are scaled by lie 2^10 and more above what
+# the ReLU lets through, so that a pack scaled by its own maximum differs from them in the low halves of most values
+@pytest.mark.parametrize("readers", [(1,), (3,), (1, 3), (3, 1, 3)], ids=str)
+@pytest.mark.parametrize("whole", [True, False], ids=["whole", "cut"])
+def test_a_first_step_has_the_bits_of_later_ones(env, readers, whole):
+    N, C, H, W, K = (40, 64, 22, 23, 64) if whole else (24, 96, 14, 15, 48)
+    rng = np.random.RandomState(7)
+    gpu, nd = env.gpu_op, env.nd
+    f = lambda *shape: rng.randn(*shape).astype(np.float32)
+    x, w1 = np.abs(f(N, C, H, W)), f(K, C, 3, 3)
+    w1[0] = -300 * np.abs(w1[0])
+    mid, cell1 = gpu.convolution_2d_forward_get_out_shape(x.shape, w1.shape, "NCHW", "SAME", 1, 1)
+    act = gpu.activation_get_cudnnlist(mid, "NCHW", "relu")
+    X, W1 = nd.array(x, env.ctx), nd.array(w1, env.ctx)
+    y1, a1, da, dy1, dx, dw1 = (nd.empty(s, env.ctx) for s in (mid, mid, mid, mid, x.shape, w1.shape))
+    behind = []
+    for r in readers:
+        w = f(64, K, r, r)
+        w[:, 0] *= 2000
+        out, cell = gpu.convolution_2d_forward_get_out_shape(mid, w.shape, "NCHW", "SAME", 1, 1)
+        behind.append((nd.array(w, env.ctx), nd.array(f(*out), env.ctx), nd.empty(out, env.ctx), nd.empty(w.shape, env.ctx), cell))
+    steps, fused = [], []
+    gpu.set_contraction_path(2)
+    try:
+        for step in range(5):
+            before = gpu.fused_relu_pack_count()
+            gpu.convolution_2d_forward(X, W1, y1, cell1, env.cudnn, env.stream)
+            gpu.activation_forward(y1, a1, "relu", act, env.cudnn, env.stream)
+            for w, do, y, dw, cell in behind:
+                gpu.convolution_2d_forward(a1, w, y, cell, env.cudnn, env.stream)
+            fused.append(gpu.fused_relu_pack_count() - before)
+            for w, do, y, dw, cell in behind:
+                gpu.convolution_backward_filter(a1, do, w, dw, cell, env.cudnn, env.stream)
+                gpu.convolution_backward_data(a1, do, w, da, cell, env.cudnn, env.stream)
+            gpu.activation_backward(y1, dy1, a1, da, "relu", act, env.cudnn, env.stream)
+            gpu.convolution_backward_filter(X, dy1, W1, dw1, cell1, env.cudnn, env.stream)
+            gpu.convolution_backward_data(X, dy1, W1, dx, cell1, env.cudnn, env.stream)
+            steps.append([v.asnumpy() for v in [y1, a1, da, dy1, dx, dw1] + [b[k] for b in behind for k in (2, 3)]])
+    finally:
+        gpu.set_contraction_path(0)
+    assert fused[0] == 0 and fused[-1] == 1
+    assert steps[0][0].min() < -2.0 ** 10 * steps[0][1].max() and np.abs(steps[0][2][:, 0]).max() > 2.0 ** 10 * np.abs(steps[0][3]).max()
+    for later in steps[1:]:
+        for a, b in zip(steps[0], later):
+            np.testing.assert_array_equal(a, b)

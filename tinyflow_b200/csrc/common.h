@@ -133,7 +133,10 @@ bool may_hold(cudaStream_t s);
 // 0 = not applicable (run the plain kernel), -1 = error.
 void tc_release(void* tc_state);               // the packs of a convolution plan that no call will use again
 int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cudaStream_t s);
-void tc_note_relu_output(const void* node, const void* y);     // the plain ReLU of graph node `node` wrote y (after the version bump)
+struct ReluBound { const uint32_t* from = nullptr; uint32_t* to = nullptr; };
+ReluBound tc_relu_bound(const float* x, const float* y);       // for the kernel that runs y = relu(x) on its own: it copies the word `from` to the word `to`
+// The plain ReLU of graph node `node` wrote y (after the version bump); bound: its kernel copied the word
+void tc_note_relu_output(const void* node, const void* y, const void* x, bool bound);
 bool contraction_path_is_cuda_cores();
 int contraction_path();
 

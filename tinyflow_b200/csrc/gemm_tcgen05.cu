@@ -1711,7 +1711,8 @@ __global__ void __launch_bounds__(256) amax_kernel(const float* __restrict__ src
 }
 // Scale words of one pack: amax[0..1] alternate between uses (the pack kernel of use k reads amax[k & 1] and clears
 // amax[(k + 1) & 1] for the next use, so no separate clearing launch is needed), scale = the power of two in force.
-struct ScaleRef { const uint32_t* amax_cur; uint32_t* amax_next; float* scale; };
+// keep: where the maximum in force is left for other packs of the same tensor.
+struct ScaleRef { const uint32_t* amax_cur; uint32_t* amax_next; float* scale; uint32_t* keep; };
 // s = 2^(14 - floor(log2 amax)): amax * s lies in [2^14, 2^15), below the fp16 maximum 65504 after rounding
 __device__ __forceinline__ float scale_from_amax(uint32_t bits) {
   int e = (int)((bits >> 23) & 0xff);
@@ -1724,7 +1725,7 @@ __device__ __forceinline__ float scale_from_amax(uint32_t bits) {
 // A tf32 pack is not scaled: its ScaleRef has no amax word and the scale in force is 1.
 __device__ __forceinline__ float pack_scale(const ScaleRef& r, bool first_thread) {
   const float s = r.amax_cur ? scale_from_amax(__ldg(r.amax_cur)) : 1.f;
-  if (first_thread) { *r.scale = s; if (r.amax_next) *r.amax_next = 0; }
+  if (first_thread) { *r.scale = s; if (r.amax_next) *r.amax_next = 0; if (r.keep) *r.keep = __ldg(r.amax_cur); }
   return s;
 }
 // hi / lo pair of one value: fp16 (22 mantissa bits together) or tf32 (round to nearest, low 13 bits zero)
@@ -2538,10 +2539,10 @@ static void pack_release(Pack& pk) {
 }
 // Starts one use of the pack: reduces max|src| over n contiguous floats into this use's amax word and returns the
 // references the pack kernel needs.  Several pack launches of the same use (stride phases) share one ScaleRef.
-// A tf32 pack needs no maximum: its scale is 1.
-static ScaleRef begin_pack(Pack& pk, const float* src, long long n, cudaStream_t s) {
-  if (pk.arith == kArithTF32) return ScaleRef{nullptr, nullptr, reinterpret_cast<float*>(pk.words + 2)};
-  ScaleRef r{nullptr, nullptr, reinterpret_cast<float*>(pk.words + 2)};
+// A tf32 pack needs no maximum: its scale is 1.  `bound`: take the scale from this word instead.
+static ScaleRef begin_pack(Pack& pk, const float* src, long long n, cudaStream_t s, const uint32_t* bound = nullptr) {
+  ScaleRef r{nullptr, nullptr, reinterpret_cast<float*>(pk.words + 2), nullptr};
+  if (pk.arith == kArithTF32) return r;
   uint32_t* fresh;                      // zero when the amax kernel below adds to it
   if (t_recording) {
     fresh = recording_word();
@@ -2550,7 +2551,8 @@ static ScaleRef begin_pack(Pack& pk, const float* src, long long n, cudaStream_t
     fresh = pk.words + k;
     r.amax_next = pk.words + (k ^ 1);
   }
-  r.amax_cur = fresh;
+  r.amax_cur = bound ? bound : fresh;
+  if (bound) return r;
   static const bool no_track = getenv("TINYFLOW_NO_AMAX_TRACKING") != nullptr;
   if (const uint32_t* tracked = no_track ? nullptr : amax_tracked(src)) {
     r.amax_cur = tracked;               // the producer of src already reduced max|src| in its own pass
@@ -2637,6 +2639,8 @@ struct ConvTc {
   int cp = 0;                                            // class D: columns per stride phase (C rounded up to 64)
   bool dgrad_seen = false;                               // backward-data has run on this plan: forward also packs its filter layout
   bool track_y = false, track_dx = false;                // a ReLU asked for max|y| / max|dx|: the epilogue leaves it
+  bool y_made = false, dx_made = false;                  // ... and so does the first call, before anybody can have asked
+  static bool tracks(bool asked, bool* made, int ar) { const bool t = asked || !*made; if (ar == kArithF16) *made = true; return t; }
   Pack x, dy, wf, wd;
   ConvTc* x_owner = this;                                // whose x pack the plan reads: another plan's of the same recorded step, or its own
   std::mutex mu;
@@ -2740,17 +2744,34 @@ static bool pack_valid(const Pack& pk, int ar, const void* src, uint64_t ver, in
 // plan is remembered under the node.  From the next step on that node's ReLU packs its output for the plan in the same
 // pass (relu_pack), whatever address the executor hands it, and the convolution finds the pack valid.  A wrong guess
 // costs one unused pack.
+//
+// The fused kernel takes the pack's scale from max|x|, the bound of max|y| that is known when it starts.  A step's bits may not depend on
+// what earlier steps taught the plans, so the same scale goes into every pack of y that a ReLU could have written: the plain ReLU, too,
+// leaves the bound of its input behind (tc_relu_bound, under a key beside y's address), and pack_x takes it.  For the same reason the first call of a
+// convolution tracks its output's maximum whether somebody asked or not.  (While first steps scaled by max|y|, 5 of 150 of them, of graphs of
+// any size, differed from the second in the last bits of their smallest operands: up to 4e-8 of Adam's moments after one step.)
 struct PackTarget { ConvTc* st; int N, C, H, W; };
 static std::atomic<long long> g_fused_relu_packs{0};
 static std::mutex g_targets_mu;
-struct ReluNote { const void* node; uint64_t version; };
+struct ReluNote { const void* node; uint64_t version; const void* x; uint64_t x_version; bool bound; };
 static std::unordered_map<const void*, ReluNote> g_relu_writer;             // output address -> the ReLU node that wrote it, and the write version it left
 static std::unordered_map<const void*, PackTarget> g_pack_targets;          // ReLU descriptor -> plan that packs its output
-void tc_note_relu_output(const void* node, const void* y) {     // call after the output's write version was bumped
+static bool fuse_relu_packs() {
+  static const bool on = [] { const char* e = getenv("TINYFLOW_FUSE_RELU_PACK"); return e ? atoi(e) != 0 : true; }();
+  return on;
+}
+static const void* bound_key(const void* y) { return (const char*)y + 1; }
+// Before y = relu(x) runs on its own: the word that bounds max|x|, if there is one, and the word that the kernel copies it to.
+ReluBound tc_relu_bound(const float* x, const float* y) {
+  if (!fuse_relu_packs() || x == y || tensor_arithmetic() != kArithF16) return ReluBound{};
+  const uint32_t* from = amax_tracked(x);
+  return from ? ReluBound{from, amax_track_begin(bound_key(y)).word} : ReluBound{};
+}
+void tc_note_relu_output(const void* node, const void* y, const void* x, bool bound) {     // call after the output's write version was bumped
   if (!node) return;
-  const uint64_t ver = version_of(y);
+  const uint64_t ver = version_of(y), x_ver = version_of(x);
   std::lock_guard<std::mutex> lk(g_targets_mu);
-  g_relu_writer[y] = ReluNote{node, ver};
+  g_relu_writer[y] = ReluNote{node, ver, x, x_ver, bound};
 }
 // A convolution's output is what a ReLU reads, forward and backward; its maximum, folded into the epilogue, is the bound that
 // lets the ReLU write the next pack too.  Only outputs that a ReLU has asked about are tracked (behind a batch
@@ -2762,18 +2783,33 @@ static void note_conv_output(const float* out, bool* wanted) {      // call afte
   std::lock_guard<std::mutex> lk(g_targets_mu);
   g_conv_writer[out] = ConvNote{wanted, ver};
 }
-static const uint32_t* bound_of(const float* x) {
-  if (const uint32_t* word = amax_tracked(x)) return word;
-  const uint64_t ver = version_of(x);
-  std::lock_guard<std::mutex> lk(g_targets_mu);
+static void ask_for_maximum_locked(const void* x, uint64_t ver) {
   auto it = g_conv_writer.find(x);
   if (it != g_conv_writer.end() && it->second.version == ver) *it->second.wanted = true;
-  return nullptr;
+}
+static const uint32_t* bound_of(const float* x) {
+  const uint64_t ver = version_of(x);
+  {
+    std::lock_guard<std::mutex> lk(g_targets_mu);
+    ask_for_maximum_locked(x, ver);
+  }
+  return amax_tracked(x);
+}
+// The bound that the ReLU which wrote x scales the pack with when it writes it itself; null: no ReLU did, or it does not write packs
+static const uint32_t* relu_bound_of(const float* x, uint64_t ver) {
+  {
+    std::lock_guard<std::mutex> lk(g_targets_mu);
+    auto it = g_relu_writer.find(x);
+    if (it == g_relu_writer.end() || it->second.version != ver || !it->second.bound) return nullptr;
+  }
+  return amax_tracked((const float*)bound_key(x));
 }
 static void remember_pack_target(const void* x, uint64_t ver, ConvTc* st, const ConvPlan* p) {
   std::lock_guard<std::mutex> lk(g_targets_mu);
   auto it = g_relu_writer.find(x);
-  if (it != g_relu_writer.end() && it->second.version == ver) g_pack_targets[it->second.node] = PackTarget{st, p->N, p->C, p->H, p->W};
+  if (it == g_relu_writer.end() || it->second.version != ver) return;
+  g_pack_targets[it->second.node] = PackTarget{st, p->N, p->C, p->H, p->W};
+  ask_for_maximum_locked(it->second.x, it->second.x_version);
 }
 
 // Inside a recorded step the branches of a module read one pack of their common input: convolutions whose frames agree (1x1 windows
@@ -2833,7 +2869,8 @@ static int pack_x(ConvTc* st, int ar, const ConvPlan* p, const float* x, cudaStr
     if (ConvTc* o = find_shared_pack(st, ar, p, x, ver, rows, cols)) { st->x_owner = o; return 0; }
   if (release_held(pk.hi, s)) return -1;
   if (pack_alloc(pk, ar, rows, cols, s, oom)) return 1;
-  ScaleRef sr = begin_pack(pk, x, n_src, s);
+  const bool relu_writes = (st->cls == 1 || st->cls == 2) && p->stride_h == 1 && p->stride_w == 1;      // the packs that a ReLU can write
+  ScaleRef sr = begin_pack(pk, x, n_src, s, relu_writes && ar == kArithF16 ? relu_bound_of(x, ver) : nullptr);
   int rc = 0;
   if (st->cls == 4) {
     // phase (a, b) holds x_padded(sh*u + a, sw*v + b) = x(sh*u + a - pad_h, sw*v + b - pad_w) at frame position (u, v)
@@ -2848,7 +2885,7 @@ static int pack_x(ConvTc* st, int ar, const ConvPlan* p, const float* x, cudaStr
   if (rc) return -1;
   pk.made_from(x, ver, st->cls);
   if (st->cls == 1 || st->cls == 2) offer_pack(x, st, p->N, p->C, p->H, p->W, p->stride_h, p->stride_w);
-  if ((st->cls == 1 || st->cls == 2) && p->stride_h == 1 && p->stride_w == 1) remember_pack_target(x, ver, st, p);
+  if (relu_writes) remember_pack_target(x, ver, st, p);
   return 0;
 }
 static int pack_dy(ConvTc* st, int ar, const ConvPlan* p, const float* dy, cudaStream_t s, int* oom) {
@@ -3036,8 +3073,7 @@ static inline int tc_result(int rc) { return rc < 0 ? -1 : (rc > 0 ? 1 : 1); }
 // y = relu(x) and the consumer plan's frame pack of y in one pass.  Returns 1 when it did that, 0 when the caller should run the plain ReLU (no known consumer, or in the
 // fp16 arithmetic no recorded max|x| to bound the scale with), -1 on error.
 int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cudaStream_t s) {
-  static const bool on = [] { const char* e = getenv("TINYFLOW_FUSE_RELU_PACK"); return e ? atoi(e) != 0 : true; }();
-  if (!on || !node || contraction_path_is_cuda_cores()) return 0;
+  if (!fuse_relu_packs() || !node || contraction_path_is_cuda_cores()) return 0;
   PackTarget t;
   {
     std::lock_guard<std::mutex> lk(g_targets_mu);
@@ -3058,22 +3094,22 @@ int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cu
   if (pack_alloc(pk, ar, rows, t.C, s, &oom)) return 0;
   note_write(y);
   AmaxOut am = amax_track_begin(y);
-  ScaleRef sr{bound, nullptr, reinterpret_cast<float*>(pk.words + 2)};       // scale from max|x| >= max|relu(x)|; tf32: no scale
+  uint32_t* const keep = bound ? amax_track_begin(bound_key(y)).word : nullptr;
+  ScaleRef sr{bound, nullptr, reinterpret_cast<float*>(pk.words + 2), keep};       // scale from max|x| >= max|relu(x)|; tf32: no scale
   note_compute_stream(s);
   if (launch_pack_nchw(pk, sr, x, t.N, t.C, t.H, t.W, st->frame_h, st->frame_w, st->x_off_h, st->x_off_w, 1, 1, 0, (int)pk.pitch, s, y, am)) return -1;
   pk.made_from(y, version_of(y), st->cls);
-  tc_note_relu_output(node, y);
+  tc_note_relu_output(node, y, x, keep != nullptr);
   g_fused_relu_packs.fetch_add(1, std::memory_order_relaxed);
   return 1;
 }
 // ReLU backward (held back by its entry point) whose output is the dy of a convolution's backward call: out = mask > 0 ? dy : 0
 // and the plan's pack of it in one pass.  1 when it did that, 0 when the caller should run the ReLU on its own.
 int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, float* out, cudaStream_t s) {
-  static const bool on = [] { const char* e = getenv("TINYFLOW_FUSE_RELU_PACK"); return e ? atoi(e) != 0 : true; }();
   ConvTc* st = conv_state(p);
   // (a layer of few channels goes through here as patches, unless the direct kernels take it: they have up to 32 filters at stride 1)
   const bool taken = p->C >= 16 || (st->cls == 3 && (p->K > 32 || p->stride_h > 1 || p->stride_w > 1));
-  if (!on || !st->cls || p->K < 16 || !taken || !encode_fn() || out == mask || out == dy) return 0;
+  if (!fuse_relu_packs() || !st->cls || p->K < 16 || !taken || !encode_fn() || out == mask || out == dy) return 0;
   const int ar = tensor_arithmetic();
   const uint32_t* bound = ar == kArithF16 ? bound_of(dy) : nullptr;       // max|dy| >= max|out|
   if (ar == kArithF16 && !bound) return 0;
@@ -3085,7 +3121,7 @@ int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, floa
   note_write(out);
   const AmaxOut am = amax_track_begin(out);
   note_compute_stream(s);
-  ScaleRef sr{bound, nullptr, reinterpret_cast<float*>(pk.words + 2)};
+  ScaleRef sr{bound, nullptr, reinterpret_cast<float*>(pk.words + 2), nullptr};
   if (launch_pack_nchw(pk, sr, dy, p->N, p->K, p->P, p->Q, st->frame_h, st->frame_w, st->dy_off_h, st->dy_off_w, 1, 1, 0, (int)pk.pitch, s, out, am, mask)) return -1;
   pk.made_from(out, version_of(out), 2);
   return 1;
@@ -3109,7 +3145,8 @@ int tc_conv_fwd(ConvPlan* p, const float* x, const float* w, float* y, cudaStrea
   OutGeom og{p->P, p->Q, p->P, p->Q, 1, 1, 0, 0};
   AmaxOut track;
   note_conv_output(y, &st->track_y);
-  return tc_result(conv_like(st->x_pack(), st->wf, st->eC, p->K, st->frame_h, st->frame_w, y, taps, og, conv_flops(p), s, "DLGpuConvolution2DForward", oom, st->track_y ? &track : nullptr));
+  const bool tracks = ConvTc::tracks(st->track_y, &st->y_made, ar);
+  return tc_result(conv_like(st->x_pack(), st->wf, st->eC, p->K, st->frame_h, st->frame_w, y, taps, og, conv_flops(p), s, "DLGpuConvolution2DForward", oom, tracks ? &track : nullptr));
 }
 
 int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaStream_t s, int* oom) {
@@ -3124,13 +3161,14 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
   int rc = 0;
   AmaxOut track;
   note_conv_output(dx, &st->track_dx);
+  const bool tracks = ConvTc::tracks(st->track_dx, &st->dx_made, ar);
   if (st->cls == 1) {
     // a strided 1x1 window reaches only every stride-th input position: the rest of dx is zero
     bool strided = p->stride_h > 1 || p->stride_w > 1;
     if (strided && clear_on_stream(dx, sizeof(float) * (size_t)p->N * p->C * p->H * p->W, s) != cudaSuccess) return -1;
     TapList taps; taps.add(0, 0, 0);
     OutGeom og{p->P, p->Q, p->H, p->W, p->stride_h, p->stride_w, 0, 0};
-    rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom, st->track_dx ? &track : nullptr);
+    rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom, tracks ? &track : nullptr);
   } else if (st->cls == 2) {
     TapList taps;
     // dx(h, w), anchored at frame position (h, w), reads dy(h - lo_h + r, w - lo_w + s) with lo = window - 1 - pad
@@ -3138,7 +3176,7 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
       for (int q = 0; q < p->S; ++q)
         taps.add((r - (p->R - 1 - p->pad_h) + st->dy_off_h) * st->frame_w + (q - (p->S - 1 - p->pad_w) + st->dy_off_w), 0, r * p->S + q);
     OutGeom og{p->H, p->W, p->H, p->W, 1, 1, 0, 0};
-    rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom, st->track_dx ? &track : nullptr);
+    rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p), s, "DLGpuConvolutionBackwardData", oom, tracks ? &track : nullptr);
   } else {
     // One launch per stride phase (a, b): dx_padded(sh*u + a, sw*v + b) = sum over the taps r = sh*r' + a, s = sw*s' + b of
     // dy(u - r', v - s') * w(r, s); dy sits at frame offset (hh, hw), so the shift is (hh - r') rows and (hw - s') columns.
@@ -3152,7 +3190,7 @@ int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaS
             taps.add((st->dy_off_h - r / p->stride_h) * st->frame_w + (st->dy_off_w - q / p->stride_w), 0, ntap - 1 - (r * p->S + q));
         if (!taps.n) continue;      // no tap lands on this phase: it stays zero
         OutGeom og{st->frame_h, st->frame_w, p->H, p->W, p->stride_h, p->stride_w, a - p->pad_h, b - p->pad_w};
-        rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p) * taps.n / ntap, s, "DLGpuConvolutionBackwardData", oom, st->track_dx ? &track : nullptr);
+        rc = conv_like(st->dy, st->wd, p->K, p->C, st->frame_h, st->frame_w, dx, taps, og, conv_flops(p) * taps.n / ntap, s, "DLGpuConvolutionBackwardData", oom, tracks ? &track : nullptr);
       }
   }
   return tc_result(rc);

@@ -59,6 +59,9 @@ template <class F> struct TracksAmax<F, decltype((void)F::kTrackAmax)> { static 
 __device__ __forceinline__ uint32_t amax4(uint32_t m, const float4& r) {
   return max(max(m, amax_bits(r.x)), max(amax_bits(r.y), max(amax_bits(r.z), amax_bits(r.w))));
 }
+// Functors with once(): one thread of the launch calls it.
+template <class F, class = void> struct HasOnce { static constexpr bool value = false; };
+template <class F> struct HasOnce<F, decltype((void)&F::once)> { static constexpr bool value = true; };
 template <class F> __global__ void __launch_bounds__(kBlock) map1_kernel(const float* __restrict__ a, float* __restrict__ o, int64_t n, F f, AmaxOut am) {
   grid_dep_sync();
   int64_t nv = n >> 2, stride = (int64_t)gridDim.x * blockDim.x;
@@ -72,6 +75,7 @@ template <class F> __global__ void __launch_bounds__(kBlock) map1_kernel(const f
     if (TracksAmax<F>::value) m = amax4(m, x);
   }
   for (int64_t i = (nv << 2) + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) { float r = f(a[i]); o[i] = r; if (TracksAmax<F>::value) m = max(m, amax_bits(r)); }
+  if constexpr (HasOnce<F>::value) if (blockIdx.x == 0 && threadIdx.x == 0) f.once();
   if (TracksAmax<F>::value) amax_commit(am, m);
 }
 template <class F> __global__ void __launch_bounds__(kBlock) map1_scalar_kernel(const float* a, float* o, int64_t n, F f) {
@@ -156,6 +160,7 @@ struct FMulC { float c; __device__ float operator()(float x) const { return x * 
 struct FAddArr { const float* c; __device__ float operator()(float x) const { return x + __ldg(c); } };      // the scalar lies in device memory
 struct FMulArr { const float* c; __device__ float operator()(float x) const { return x * __ldg(c); } };
 struct FRelu { static constexpr bool kTrackAmax = true; __device__ float operator()(float x) const { return x > 0.f ? x : (x != x ? x : 0.f); } };   // NaN propagates
+struct FReluKeep : FRelu { ReluBound bound; __device__ void once() const { if (bound.to) *bound.to = *bound.from; } };      // and the bound of its input
 struct FExp { __device__ float operator()(float x) const { return expf(x); } };
 struct FLog { __device__ float operator()(float x) const { return logf(x); } };
 struct FRecip { __device__ float operator()(float x) const { return 1.f / x; } };
@@ -1300,7 +1305,7 @@ int DLGpuActivationForward(const DLArrayHandle input, DLArrayHandle output, int 
     const cudaStream_t s_here = stream_of_keep_deferred(cudaStream);
     int rc = 0;
     if (t_recording && relu_of_bias_sum(input, output, s_here, &rc)) {
-      tc_note_relu_output(plan_of<TensorPlan>(cudnnlist, kPlanTensor), output->data);
+      tc_note_relu_output(plan_of<TensorPlan>(cudnnlist, kPlanTensor), output->data, input->data, false);
       return rc;
     }
     if (take_deferred(kDeferAdd, F(input), n, &add)) {
@@ -1314,7 +1319,7 @@ int DLGpuActivationForward(const DLArrayHandle input, DLArrayHandle output, int 
       if (!fused) launch_deferred_now(add);
       release_deferred();
       if (fused) {
-        tc_note_relu_output(plan_of<TensorPlan>(cudnnlist, kPlanTensor), output->data);
+        tc_note_relu_output(plan_of<TensorPlan>(cudnnlist, kPlanTensor), output->data, input->data, false);
         TF_AFTER(s_here, "DLGpuActivationForward(relu)");
         return 0;
       }
@@ -1329,8 +1334,10 @@ int DLGpuActivationForward(const DLArrayHandle input, DLArrayHandle output, int 
       int fused = tc_fused_relu_pack(node, F(input), (float*)output->data, n, s);
       if (fused < 0) return -1;
       if (fused) return 0;
-      int rc = run_map1(F(input), FM(output), n, s, "DLGpuActivationForward(relu)", FRelu{});
-      tc_note_relu_output(node, output->data);
+      FReluKeep relu;
+      if (node && aligned16(input->data) && aligned16(output->data)) relu.bound = tc_relu_bound(F(input), F(output));
+      int rc = run_map1(F(input), FM(output), n, s, "DLGpuActivationForward(relu)", relu);
+      tc_note_relu_output(node, output->data, input->data, relu.bound.to != nullptr);
       return rc;
     }
     case 2: return run_map1(F(input), FM(output), n, s, "DLGpuActivationForward(tanh)", FTanh{});
