@@ -225,3 +225,25 @@ def test_batchnorm_at_group_edges(env, N, plane):
         plane = (plane[0] * 2 ** 11 // N // 2 * 2,) + plane[1:]          # held back from 64 K elements on
         fused(env, (N,) + plane, True)
         fused(env, (N,) + plane, False)
+
+
+# an image of no positions, no images: sums of nothing, not of what lies behind the array; one alone and among others that wait
+@pytest.mark.parametrize("shape", [(3, 40, 0), (70, 5, 4, 0), (2, 300, 0, 6), (0, 7, 4, 4)], ids=str)
+@pytest.mark.parametrize("held", [False, True])
+def test_channel_sums_of_nothing(env, shape, held):
+    gpu, nd = env.gpu_op, env.nd
+    some = np.random.RandomState(3).randn(9, 6, 5).astype(np.float32)
+    calls = []
+    for x in (nd.empty(shape, env.ctx), nd.array(some, env.ctx)):
+        ins, outs = gpu.reduce_sum_get_real_shape(x.shape, (x.shape[1],), "NCHW")
+        calls.append((x, nd.array(np.full(x.shape[1], 7, np.float32), env.ctx), gpu.reduce_sum_get_cudnnlist(ins, outs, "NCHW", env.cudnn)))
+    try:
+        gpu.hold_products(held)
+        for x, out, cell in calls:
+            gpu.reduce_sum_new(x, out, cell, env.cudnn, env.stream)
+        gpu.hold_products(False)
+        gpu.launch_held(env.stream)
+    finally:
+        gpu.drop_held()
+    np.testing.assert_array_equal(calls[0][1].asnumpy(), np.zeros(shape[1], np.float32))
+    np.testing.assert_allclose(calls[1][1].asnumpy(), some.astype(np.float64).sum(axis=(0, 2)), rtol=1e-5, atol=1e-5)

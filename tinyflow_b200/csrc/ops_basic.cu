@@ -193,7 +193,9 @@ __global__ void __launch_bounds__(kBlock) bcast_channel_kernel(const float* __re
 // ---- reductions --------------------------------------------------------------------
 // Column sums of a row-major [rows x cols] matrix, out[c] = sum_r in[r, c].
 // Block = 32 columns x 8 row lanes; grid.x tiles the columns, grid.y splits the rows.
-struct SumJob {               // column sums of [rows][cols], or channel sums of [rows = images][cols = channels][length]
+enum { kColumnSums, kChannelSums };
+struct SumJob {               // column sums of [rows][cols], or channel sums of [rows = images][cols = channels][length, which may be 0]
+  int kind;
   const float* in; float* out; float* part; uint32_t* counters;
   int64_t rows, cols, length, per_split;
   int splits, vec;            // vec: 16-byte loads along `length`
@@ -276,11 +278,11 @@ __global__ void __launch_bounds__(256) sum_group_kernel(const __grid_constant__ 
   int k = 0;
   while (k + 1 < jobs.n && jobs.job[k + 1].first_block <= (int)blockIdx.x) ++k;
   const SumJob& j = jobs.job[k];
-  const int at = (int)blockIdx.x - j.first_block, across = j.length ? (int)j.cols : (int)((j.cols + 31) / 32), split = at / across;
-  if (j.length) channel_sum(j, at - split * across, split);
+  const int at = (int)blockIdx.x - j.first_block, across = j.kind == kChannelSums ? (int)j.cols : (int)((j.cols + 31) / 32), split = at / across;
+  if (j.kind == kChannelSums) channel_sum(j, at - split * across, split);
   else column_sum(j, at - split * across, split);
 }
-static int sum_blocks(const SumJob& j) { return j.length ? (int)j.cols : (int)((j.cols + 31) / 32); }        // per split
+static int sum_blocks(const SumJob& j) { return j.kind == kChannelSums ? (int)j.cols : (int)((j.cols + 31) / 32); }        // per split
 // Scratch of the jobs that are split; column sums do without where there is none
 static int sum_scratch(SumJob* jobs, int n, StreamLease& lease, const char* what) {
   size_t floats = 0, counters = 0;
@@ -293,7 +295,7 @@ static int sum_scratch(SumJob* jobs, int n, StreamLease& lease, const char* what
     SumJob& j = jobs[i];
     if (j.splits == 1) continue;
     if (!part || !count) {
-      TF_REQUIRE(!j.length, "%s: scratch allocation failed", what);
+      TF_REQUIRE(j.kind == kColumnSums, "%s: scratch allocation failed", what);
       j.splits = 1; j.per_split = j.rows;
       continue;
     }
@@ -327,7 +329,7 @@ static int run_sums(SumJob j, cudaStream_t s, const char* what) {
   if (sum_scratch(&j, 1, lease, what)) return -1;
   note_compute_stream(s);
   const dim3 grid((unsigned)sum_blocks(j), (unsigned)j.splits);
-  if (j.length) launch_dep(channel_sum_kernel, grid, dim3(kBlock), 0, s, j);
+  if (j.kind == kChannelSums) launch_dep(channel_sum_kernel, grid, dim3(kBlock), 0, s, j);
   else launch_dep(colsum_kernel, grid, dim3(256), 0, s, j);
   TF_AFTER(s, what);
   return 0;
@@ -904,7 +906,7 @@ static int channel_sums(const float* in, float* out, int64_t N, int64_t C, int64
   const int64_t nps = std::max<int64_t>(1, (N + splits - 1) / splits);
   splits = std::max<int64_t>(1, (N + nps - 1) / nps);
   const int vec = L % 4 == 0 && aligned16(in) && nps * (L / 4) < (1ll << 31);
-  return run_sums(SumJob{in, out, nullptr, nullptr, N, C, L, nps, (int)splits, vec, 0}, s, what);
+  return run_sums(SumJob{kChannelSums, in, out, nullptr, nullptr, N, C, L, nps, (int)splits, vec, 0}, s, what);
 }
 
 static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, cudaStream_t s, const char* what) {
@@ -918,7 +920,7 @@ static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, 
   }
   int64_t rps = (rows + splits - 1) / splits;
   splits = (int)((rows + rps - 1) / rps);
-  return run_sums(SumJob{in, out, nullptr, nullptr, rows, cols, 0, rps, splits, 0, 0}, s, what);
+  return run_sums(SumJob{kColumnSums, in, out, nullptr, nullptr, rows, cols, 0, rps, splits, 0, 0}, s, what);
 }
 
 int DLGReduceSumGetCudnnlist(const int* input_shapes, const int* output_shapes, const int sizeofshape,
