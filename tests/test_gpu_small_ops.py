@@ -247,3 +247,12 @@ def test_channel_sums_of_nothing(env, shape, held):
         gpu.drop_held()
     np.testing.assert_array_equal(calls[0][1].asnumpy(), np.zeros(shape[1], np.float32))
     np.testing.assert_allclose(calls[1][1].asnumpy(), some.astype(np.float64).sum(axis=(0, 2)), rtol=1e-5, atol=1e-5)
+
+
+@pytest.mark.parametrize("rows,cols", [(0, 5), (0, 70), (0, 1), (100, 0), (3, 0)])
+def test_column_sums_of_nothing(env, rows, cols):
+    gpu, nd = env.gpu_op, env.nd
+    x, out = nd.empty((rows, cols), env.ctx), nd.array(np.full(cols, 7, np.float32), env.ctx) if cols else nd.empty((0,), env.ctx)
+    ins, outs = gpu.reduce_sum_get_real_shape(x.shape, (cols,), "NHWC")
+    gpu.reduce_sum_new(x, out, gpu.reduce_sum_get_cudnnlist(ins, outs, "NHWC", env.cudnn), env.cudnn, env.stream)
+    np.testing.assert_array_equal(out.asnumpy(), np.zeros(cols, np.float32))

@@ -899,6 +899,7 @@ static int reduce_to_scalar(const float* in, float* out, int64_t n, float scale,
 // Channel sums of [N][C][L]: the images split so that about four blocks per SM run, each with a few thousand elements.
 static int channel_sums(const float* in, float* out, int64_t N, int64_t C, int64_t L, cudaStream_t s, const char* what) {
   TF_REQUIRE(C < (1ll << 31), "%s: too many channels", what);
+  if (C == 0) return 0;
   int64_t splits = std::max<int64_t>(1, 4 * device_sm_count() / C);
   splits = std::min(splits, std::max<int64_t>(1, N * L / 4096));
   splits = std::min<int64_t>(std::min(splits, N), 65535);
@@ -910,6 +911,7 @@ static int channel_sums(const float* in, float* out, int64_t N, int64_t C, int64
 }
 
 static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, cudaStream_t s, const char* what) {
+  if (cols == 0) return 0;
   int gx = (int)((cols + 31) / 32);
   int splits = 1;
   int sms = device_sm_count();
@@ -918,8 +920,8 @@ static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, 
     if (splits > rows / 16) splits = (int)(rows / 16);
     if (splits < 1) splits = 1;
   }
-  int64_t rps = (rows + splits - 1) / splits;
-  splits = (int)((rows + rps - 1) / rps);
+  const int64_t rps = std::max<int64_t>(1, (rows + splits - 1) / splits);
+  splits = std::max(1, (int)((rows + rps - 1) / rps));
   return run_sums(SumJob{kColumnSums, in, out, nullptr, nullptr, rows, cols, 0, rps, splits, 0, 0}, s, what);
 }
 
@@ -948,6 +950,7 @@ int DLGpuReduceSum(const DLArrayHandle input, DLArrayHandle output, void*** cudn
   for (int i = 0; i < p->ndim; ++i) { nin *= p->in_dims[i]; nout *= p->out_dims[i]; }
   TF_REQUIRE(nin == numel(input) && nout == numel(output), "DLGpuReduceSum: arrays do not match the plan");
   cudaStream_t s = stream_of(cudaStream);
+  if (nout == 0) return 0;
   if (nout == 1) return reduce_to_scalar(F(input), FM(output), nin, 1.f, s, "DLGpuReduceSum");
   // leading axes reduced, trailing kept  ->  column sums
   int first_kept = 0;
