@@ -130,3 +130,69 @@ def test_direct_filter_gradients_in_one_launch(lib_path, count):
         gpu_op.drop_held()
     for call in calls:
         np.testing.assert_array_equal(call[4].asnumpy(), call[3].asnumpy())
+
+
+DIRECT = [(300, 3, 9, 7, 5, 3, 3, 1), (40, 6, 14, 14, 16, 5, 5, 1), (200, 2, 8, 8, 8, 3, 3, 1), (64, 6, 11, 11, 16, 5, 5, 1), (30, 1, 28, 28, 6, 5, 5, 1)]
+
+
+# the device has no byte left but the workspaces of separate launches: what waits is launched in parts, with the same bits
+@pytest.mark.parametrize("recorded", [False, True])
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+def test_a_full_device_launches_fewer_together(lib_path, arith, recorded):
+    import ctypes
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    from tinyflow_b200._base import _LIB, check_call, new_cell
+    ctx, stream, rng = nd.gpu(0), gpu_op.create_cudaStream(), np.random.RandomState(5)
+    handle = gpu_op.create_cudnnHandle(stream)
+    gpu_op.set_tensor_arithmetic(arith)
+    calls = []
+    for N, C, H, W, K, R, S, u in LAYERS + DIRECT:
+        out, cell = gpu_op.convolution_2d_forward_get_out_shape((N, C, H, W), (K, C, R, S), "NCHW", "VALID" if u > 1 else "SAME", u, u)
+        x, w, dy = (nd.array(rng.randn(*shape).astype(np.float32), ctx) for shape in ((N, C, H, W), (K, C, R, S), out))
+        sums = gpu_op.reduce_sum_get_cudnnlist(*gpu_op.reduce_sum_get_real_shape(out, (K,), "NCHW"), "NCHW", handle)
+        calls.append((x, dy, w, cell, sums) + tuple(nd.array(np.full(s, np.nan, np.float32), ctx) for _ in range(2) for s in ((K, C, R, S), (K,))))
+
+    def run(into, on):
+        for call in calls:
+            gpu_op.convolution_backward_filter(call[0], call[1], call[2], call[into], call[3], handle, on)
+            gpu_op.reduce_sum_new(call[1], call[into + 1], call[4], handle, on)
+
+    def hold_all():
+        graph, on = ctypes.c_void_p(), stream
+        if recorded:
+            on = new_cell(2)
+            check_call(_LIB.TfStepRecordBegin(ctypes.byref(graph), on, stream))
+        before = gpu_op.launch_count()
+        gpu_op.hold_products(True)
+        run(7, on)
+        gpu_op.hold_products(False)
+        held = gpu_op.launch_count()
+        gpu_op.launch_held(on)
+        launches = gpu_op.launch_count() - held
+        if recorded:
+            check_call(_LIB.TfStepRecordEnd(ctypes.byref(graph), 1))
+            before = gpu_op.launch_count()
+            check_call(_LIB.TfStepReplay(graph, None, 0, ctypes.c_float(0), ctypes.c_float(0), None, 0, stream))
+            gpu_op.device_synchronize()
+            launches = gpu_op.launch_count() - before
+            check_call(_LIB.TfStepGraphFree(graph))
+        for call in calls:
+            for apart, together in zip(call[5:7], call[7:9]):
+                np.testing.assert_array_equal(together.asnumpy(), apart.asnumpy())
+                together[:] = np.full(together.shape, np.nan, np.float32)
+        return launches
+    try:
+        gpu_op.set_memory_limit(1)
+        assert isinstance(nd.empty((1 << 30,), ctx), int)          # the scratch of every stream goes back
+        gpu_op.set_memory_limit(0)
+        run(5, stream)
+        gpu_op.device_synchronize()
+        gpu_op.release_cached_memory()
+        gpu_op.set_memory_limit(sum(gpu_op.allocator_stats()) + (recorded << 20))        # a recording needs a little for itself
+        in_parts = hold_all()
+        gpu_op.set_memory_limit(0)
+        assert hold_all() < in_parts
+    finally:
+        gpu_op.drop_held()
+        gpu_op.set_memory_limit(0)
+        gpu_op.set_tensor_arithmetic("3xfp16")

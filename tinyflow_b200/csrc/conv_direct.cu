@@ -349,13 +349,15 @@ int launch_held_direct(cudaStream_t s) {
   all.swap(t_held_direct);
   for (int S : {3, 5, 7}) {
     size_t at = 0;
+    int most = kWgradJobs;
     while (true) {
       DirectJobs jobs;
       jobs.n = 0;
       int blocks = 0, sums = 0;
       size_t smem = 0, floats = 0;
       double flops = 0;
-      for (; at < all.size() && jobs.n < kWgradJobs; ++at) {
+      const size_t begin = at;
+      for (; at < all.size() && jobs.n < most; ++at) {
         if (all[at].S != S) continue;
         DirectJob& j = jobs.job[jobs.n++] = all[at].job;
         j.first = blocks; blocks += j.blocks;
@@ -365,7 +367,8 @@ int launch_held_direct(cudaStream_t s) {
       if (!jobs.n) break;
       StreamLease lease(s);
       float* part = (float*)lease.scratch(kScratchContract, sizeof(float) * floats);
-      TF_REQUIRE(part, "filter gradients: no memory for %zu bytes of partial sums", sizeof(float) * floats);
+      if (!part && jobs.n > 1) { most = jobs.n / 2; at = begin; continue; }        // a full device: fewer together (the call of each has seen to its own)
+      TF_REQUIRE(part, "filter gradients: the device is out of memory, %zu bytes of partial sums short", sizeof(float) * floats);
       for (int i = 0; i < jobs.n; ++i) { jobs.job[i].d.part = part; part += (size_t)jobs.job[i].blocks * jobs.job[i].cols; }
       note_compute_stream(s);
       KernelTimer kt("direct_conv", s, flops, 0, 1);
@@ -393,13 +396,13 @@ int direct_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float*
   if (d.slices > 1 && floats < (size_t)d.slices * d.items * p->S) floats = (size_t)d.slices * d.items * p->S;
   if (floats * sizeof(float) > kDirectSmem) return 0;
   const int cols = d.items * p->S, grid = p->N < 2 * device_sm_count() ? p->N : 2 * device_sm_count();
+  StreamLease lease(s);
+  d.part = (float*)lease.scratch(kScratchContract, sizeof(float) * (size_t)grid * cols);
+  if (!d.part) return 0;
   if (d.items <= kWgradThreads && may_hold(s)) {
     t_held_direct.push_back(HeldDirect{DirectJob{d, dw, grid, cols, 0, 0}, p->S, floats * sizeof(float), 2.0 * p->N * p->K * p->P * p->Q * p->C * p->R * p->S});
     return 1;
   }
-  StreamLease lease(s);
-  d.part = (float*)lease.scratch(kScratchContract, sizeof(float) * (size_t)grid * cols);
-  if (!d.part) return 0;
   note_compute_stream(s);
   KernelTimer kt("direct_conv", s, 2.0 * p->N * p->K * p->P * p->Q * p->C * p->R * p->S, 0, 1);
   if ((p->S == 3 ? launch_wgrad<3>(d, grid, floats * sizeof(float), s) : p->S == 5 ? launch_wgrad<5>(d, grid, floats * sizeof(float), s) : launch_wgrad<7>(d, grid, floats * sizeof(float), s)) != 0) return -1;

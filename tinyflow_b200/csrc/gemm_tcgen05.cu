@@ -2230,18 +2230,23 @@ template <int BN, int AR> static size_t plan_launch(GemmParams& p) {
   p.sum_run = could_wait<BN>(p) ? kSumChunk : 1;
   return bytes;
 }
-template <int BN, int AR> static bool held_back(const GemmParams& p, cudaStream_t s, double flops);
+template <int BN, int AR> static bool held_back(const GemmParams& p, size_t workspace_bytes, cudaStream_t s, double flops);
+template <int BN, int AR> static int launch_planned(GemmParams& p, size_t workspace_bytes, bool may_wait, cudaStream_t s, double flops, const char* what, int* oom);
 template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, double flops, const char* what, int* oom) {
-  static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
-  TF_CUDA(attr);
   TF_REQUIRE(tensor_path_error() == 0, "%s: an earlier tensor-core kernel timed out on a barrier; refusing to launch", what);
   const size_t bytes = plan_launch<BN, AR>(p);
-  if (p.hold && held_back<BN, AR>(p, s, flops)) return 0;
+  return launch_planned<BN, AR>(p, bytes, p.hold != 0, s, flops, what, oom);
+}
+template <int BN, int AR> static int launch_planned(GemmParams& p, size_t bytes, bool may_wait, cudaStream_t s, double flops, const char* what, int* oom) {
+  static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  TF_CUDA(attr);
   StreamLease lease(s);
+  // (one that waits has the workspace of a launch of its own, too: a shortage is reported by the call that meets it, see launch_some)
   if (bytes && !(p.workspace = (float*)lease.scratch(kScratchTiles, bytes))) {
     if (oom) *oom = bytes > 0x7fffffffu ? 0x7fffffff : (int)bytes;
     return 1;
   }
+  if (may_wait && held_back<BN, AR>(p, bytes, s, flops)) return 0;
   const int sms = device_sm_count();
   const int tiles = p.full_tiles + p.tail_tiles;
   int grid = tiles < sms ? tiles : sms;
@@ -2276,7 +2281,7 @@ template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, 
 // (the executor: only the parameter updates at the end of the step read it), and that what the product reads, the packs of its
 // plan, is not packed anew before (release_held() looks after that).  Products whose CTAs have many stages to do are launched
 // at once: they gain nothing, and their operands are in L2 now.
-struct HeldProduct { GemmParams g; int bn, ar; double flops; };
+struct HeldProduct { GemmParams g; int bn, ar; size_t workspace_bytes; double flops; };
 static thread_local bool t_hold = false;
 static thread_local std::vector<HeldProduct> t_held;
 static thread_local double t_held_work = 0;           // tiles x stages
@@ -2300,7 +2305,11 @@ bool may_hold(cudaStream_t s) {
 }
 
 constexpr size_t kStagedCopy = 1 << 16;
-template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>& held, cudaStream_t s, double flops) {
+// Partial sums that the products of one launch may have between them: the largest of the benchmark's graphs has 345 MB (DenseNet-121 at
+// batch 56), one product on its own 10 MB at most.
+constexpr size_t kGroupBytes = size_t(512) << 20;
+// 0: launched, -1: error, 1: too many at once, or no memory for the table or the partial sums; nothing was launched
+template <int BN, int AR> static int launch_group(HeldProduct* const* products, int n, cudaStream_t s) {
   static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_group_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem<BN>);
   TF_CUDA(attr);
   const int sms = device_sm_count();
@@ -2309,7 +2318,9 @@ template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>
   struct Item { int4 what; int stages; };
   std::vector<Item> items;
   std::vector<int4> sums;
-  double work = 0;
+  std::vector<const GemmParams*> held;
+  double work = 0, flops = 0;
+  for (int i = 0; i < n; ++i) { held.push_back(&products[i]->g); flops += products[i]->flops; }
   for (const GemmParams* g : held) work += (double)g->m_tiles * g->n_tiles * g->tap_tiles * (g->k_total + kItemCost);
   const int whole = std::max(8, (int)(work / sms / 2));
   int slots = 0, most_pieces = 0;
@@ -2372,7 +2383,8 @@ template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>
   t.err = error_word();
   t.workspace = nullptr;
   const size_t bytes = (size_t)slots * BN * BM * sizeof(float);
-  if (bytes) TF_REQUIRE(t.workspace = (float*)lease.scratch(kScratchTiles, bytes), "filter gradients: no memory for %zu bytes of partial sums", bytes);
+  if (n > 1 && bytes > kGroupBytes) return 1;
+  if (bytes && !(t.workspace = (float*)lease.scratch(kScratchTiles, bytes))) return 1;
   char* dev;
   if (t_recording) {
     dev = (char*)recording_own(table);                // lives and is uploaded with the recording
@@ -2382,7 +2394,7 @@ template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>
     for (size_t at = 0; dev && at < table.size(); at += kStagedCopy)
       TF_CUDA(cudaMemcpyAsync(dev + at, table.data() + at, std::min(kStagedCopy, table.size() - at), cudaMemcpyHostToDevice, s));
   }
-  TF_REQUIRE(dev, "filter gradients: no memory for a table of %zu bytes", table.size());
+  if (!dev) return 1;
   t.problems = (const GemmParams*)dev; t.items = (const int4*)(dev + at_items); t.sums = (const int4*)(dev + at_sums); t.first = (const int*)(dev + at_first);
   note_compute_stream(s);
   KernelTimer kt(AR == kArithTF32 ? "gemm3xtf32_tcgen05" : "gemm3xf16_tcgen05", s, flops, 0, 1);
@@ -2394,6 +2406,21 @@ template <int BN, int AR> static int launch_group(std::vector<const GemmParams*>
   }
   return 0;
 }
+// As many together as there is memory for: on a full device a group gives way to its halves, and one product to the launch of its own whose
+// workspace its call has seen to.  The bits are the same either way.
+template <int BN, int AR> static int launch_some(HeldProduct* const* products, int n, cudaStream_t s) {
+  const int rc = launch_group<BN, AR>(products, n, s);
+  if (rc != 1) return rc;
+  if (n > 1) {
+    if (const int first = launch_some<BN, AR>(products, n / 2, s)) return first;
+    return launch_some<BN, AR>(products + n / 2, n - n / 2, s);
+  }
+  int oom = 0;
+  HeldProduct& h = *products[0];
+  if (launch_planned<BN, AR>(h.g, h.workspace_bytes, false, s, h.flops, "DLGpuConvolutionBackwardFilter", &oom) == 0) return 0;
+  TF_REQUIRE(!oom, "filter gradients: the device is out of memory, %d bytes of partial sums short", oom);
+  return -1;
+}
 static int launch_held_filters(cudaStream_t s) {
   if (t_held.empty()) return 0;
   std::vector<HeldProduct> all;
@@ -2402,13 +2429,13 @@ static int launch_held_filters(cudaStream_t s) {
   TF_REQUIRE(tensor_path_error() == 0, "filter gradients: an earlier tensor-core kernel timed out on a barrier; refusing to launch");
   for (int ar : {kArithF16, kArithTF32})
     for (int bn : {64, 128}) {
-      std::vector<const GemmParams*> some;
-      double flops = 0;
-      for (const HeldProduct& h : all)
-        if (h.bn == bn && h.ar == ar) { some.push_back(&h.g); flops += h.flops; }
+      std::vector<HeldProduct*> some;
+      for (HeldProduct& h : all)
+        if (h.bn == bn && h.ar == ar) some.push_back(&h);
       if (some.empty()) continue;
-      const int rc = ar == kArithTF32 ? (bn == 64 ? launch_group<64, kArithTF32>(some, s, flops) : launch_group<128, kArithTF32>(some, s, flops))
-                                      : (bn == 64 ? launch_group<64, kArithF16>(some, s, flops) : launch_group<128, kArithF16>(some, s, flops));
+      const int n = (int)some.size();
+      const int rc = ar == kArithTF32 ? (bn == 64 ? launch_some<64, kArithTF32>(some.data(), n, s) : launch_some<128, kArithTF32>(some.data(), n, s))
+                                      : (bn == 64 ? launch_some<64, kArithF16>(some.data(), n, s) : launch_some<128, kArithF16>(some.data(), n, s));
       if (rc) return rc;
     }
   return 0;
@@ -2426,10 +2453,10 @@ static int release_held(const void* hi, cudaStream_t s) {
   return 0;
 }
 // Takes the product if it may wait; what has gathered goes when it fills the SMs.
-template <int BN, int AR> static bool held_back(const GemmParams& p, cudaStream_t s, double flops) {
+template <int BN, int AR> static bool held_back(const GemmParams& p, size_t workspace_bytes, cudaStream_t s, double flops) {
   if (!could_wait<BN>(p) || p.amax) return false;
   if (!may_hold(s)) return false;
-  t_held.push_back(HeldProduct{p, BN, AR, flops});
+  t_held.push_back(HeldProduct{p, BN, AR, workspace_bytes, flops});
   t_held_work += (double)p.m_tiles * p.n_tiles * p.tap_tiles * p.k_total;
   return true;
 }

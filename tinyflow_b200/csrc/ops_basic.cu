@@ -283,7 +283,7 @@ __global__ void __launch_bounds__(256) sum_group_kernel(const __grid_constant__ 
   else column_sum(j, at - split * across, split);
 }
 static int sum_blocks(const SumJob& j) { return j.kind == kChannelSums ? (int)j.cols : (int)((j.cols + 31) / 32); }        // per split
-// Scratch of the jobs that are split; column sums do without where there is none
+// Scratch of the jobs that are split.  Where there is none, a column sum does without; 1: there is none for several
 static int sum_scratch(SumJob* jobs, int n, StreamLease& lease, const char* what) {
   size_t floats = 0, counters = 0;
   for (int i = 0; i < n; ++i)
@@ -291,6 +291,7 @@ static int sum_scratch(SumJob* jobs, int n, StreamLease& lease, const char* what
   if (!counters) return 0;
   float* part = (float*)lease.scratch(kScratchSplit, sizeof(float) * floats);
   uint32_t* count = lease.counters((int)counters);
+  if (n > 1 && (!part || !count)) return 1;
   for (int i = 0; i < n; ++i) {
     SumJob& j = jobs[i];
     if (j.splits == 1) continue;
@@ -309,12 +310,16 @@ void drop_held_sums() { t_held_sums.clear(); }
 int launch_held_sums(cudaStream_t s) {
   std::vector<SumJob> all;
   all.swap(t_held_sums);
-  for (size_t from = 0; from < all.size(); from += kSumJobs) {
+  int most = kSumJobs;
+  for (size_t from = 0; from < all.size();) {
     SumJobs jobs;
-    jobs.n = (int)std::min(all.size() - from, (size_t)kSumJobs);
+    jobs.n = (int)std::min(all.size() - from, (size_t)most);
     std::copy(all.begin() + from, all.begin() + from + jobs.n, jobs.job);
     StreamLease lease(s);
-    if (sum_scratch(jobs.job, jobs.n, lease, "bias gradients")) return -1;
+    const int rc = sum_scratch(jobs.job, jobs.n, lease, "bias gradients");
+    if (rc < 0) return -1;
+    if (rc) { most = jobs.n / 2; continue; }              // a full device: fewer together (the call of each has seen to its own)
+    from += jobs.n;
     int blocks = 0;
     for (int i = 0; i < jobs.n; ++i) { jobs.job[i].first_block = blocks; blocks += sum_blocks(jobs.job[i]) * jobs.job[i].splits; }
     note_compute_stream(s);
@@ -324,9 +329,9 @@ int launch_held_sums(cudaStream_t s) {
   return 0;
 }
 static int run_sums(SumJob j, cudaStream_t s, const char* what) {
-  if ((long long)sum_blocks(j) * j.splits <= kHeldSumBlocks && may_hold(s)) { t_held_sums.push_back(j); return 0; }
   StreamLease lease(s);
   if (sum_scratch(&j, 1, lease, what)) return -1;
+  if ((long long)sum_blocks(j) * j.splits <= kHeldSumBlocks && may_hold(s)) { t_held_sums.push_back(j); return 0; }
   note_compute_stream(s);
   const dim3 grid((unsigned)sum_blocks(j), (unsigned)j.splits);
   if (j.kind == kChannelSums) launch_dep(channel_sum_kernel, grid, dim3(kBlock), 0, s, j);
