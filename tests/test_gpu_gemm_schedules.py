@@ -126,3 +126,38 @@ def test_first_layers_as_patches(env, case, arith):
 @pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
 def test_narrow_tiles_of_short_reductions(env, case, arith):
     test_convolution_schedules(env, case, arith)
+
+
+# the first product of a process asks how many clusters fit on the device before it launches anything
+_FIRST_PRODUCT = """
+import ctypes, json
+import numpy as np
+from tinyflow_b200 import gpu_op, ndarray as nd
+from tinyflow_b200._base import _LIB
+ctx, stream = nd.gpu(0), gpu_op.create_cudaStream()
+handle = gpu_op.create_cudnnHandle(stream)
+gpu_op.set_tensor_arithmetic("%s")
+shape, filters = (2, 768, 17, 17), (192, 768, 1, 1)
+out, cell = gpu_op.convolution_2d_forward_get_out_shape(shape, filters, "NCHW", "SAME", 1, 1)
+x, w, y = (nd.array(np.ones(s, np.float32), ctx) for s in (shape, filters, out))
+for step in range(2):
+    _LIB.TfKernelTimingEnable(1)
+    gpu_op.convolution_2d_forward(x, w, y, cell, handle, stream)
+    gpu_op.device_synchronize()
+    report = ctypes.create_string_buffer(1 << 16)
+    _LIB.TfKernelTimingReport(report, len(report))
+    print([r["name"] for r in json.loads(report.value.decode())])
+"""
+
+
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+def test_a_first_product_is_cut_over_clusters(lib_path, arith):
+    import os
+    import re
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    ran = subprocess.run([sys.executable, "-c", _FIRST_PRODUCT % arith], cwd=root, env=dict(os.environ, TINYFLOW_TIMING_DETAIL="1"), capture_output=True, text=True, timeout=300)
+    lines = ran.stdout.strip().splitlines()
+    assert ran.returncode == 0 and len(lines) == 2 and lines[0] == lines[1], ran.stdout + ran.stderr
+    assert int(re.search(r" cl(\d+) ", lines[0]).group(1)) > 1, lines[0]

@@ -2184,6 +2184,11 @@ static int plan_smem(GemmParams& g, int bn, int grid) {
   return grid;
 }
 
+// The kernel may use all shared memory: asked for ahead of its first launch and of the first question how many clusters of it fit
+template <int BN, int AR> static cudaError_t gemm_kernel_ready() {
+  static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
+  return attr;
+}
 template <int BN, int AR> static int max_clusters_of(int c) {
   static std::atomic<int> known[9];
   int n = known[c].load(std::memory_order_relaxed);
@@ -2233,13 +2238,12 @@ template <int BN, int AR> static size_t plan_launch(GemmParams& p) {
 template <int BN, int AR> static bool held_back(const GemmParams& p, size_t workspace_bytes, cudaStream_t s, double flops);
 template <int BN, int AR> static int launch_planned(GemmParams& p, size_t workspace_bytes, bool may_wait, cudaStream_t s, double flops, const char* what, int* oom);
 template <int BN, int AR> static int launch_gemm(GemmParams& p, cudaStream_t s, double flops, const char* what, int* oom) {
+  TF_CUDA((gemm_kernel_ready<BN, AR>()));
   TF_REQUIRE(tensor_path_error() == 0, "%s: an earlier tensor-core kernel timed out on a barrier; refusing to launch", what);
   const size_t bytes = plan_launch<BN, AR>(p);
   return launch_planned<BN, AR>(p, bytes, p.hold != 0, s, flops, what, oom);
 }
 template <int BN, int AR> static int launch_planned(GemmParams& p, size_t bytes, bool may_wait, cudaStream_t s, double flops, const char* what, int* oom) {
-  static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit + 1024);
-  TF_CUDA(attr);
   StreamLease lease(s);
   // (one that waits has the workspace of a launch of its own, too: a shortage is reported by the call that meets it, see launch_some)
   if (bytes && !(p.workspace = (float*)lease.scratch(kScratchTiles, bytes))) {
