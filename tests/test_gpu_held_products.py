@@ -196,3 +196,36 @@ def test_a_full_device_launches_fewer_together(lib_path, arith, recorded):
         gpu_op.drop_held()
         gpu_op.set_memory_limit(0)
         gpu_op.set_tensor_arithmetic("3xfp16")
+
+
+# what waits was called on one stream and goes there; calls on another stream do not wait, and do not overtake it
+def test_products_wait_on_their_own_stream(lib_path):
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, rng = nd.gpu(0), np.random.RandomState(2)
+    one, two = gpu_op.create_cudaStream(), gpu_op.create_cudaStream()
+    handle = gpu_op.create_cudnnHandle(one)
+    calls = []
+    for N, C, H, W, K, R, S, u in (LAYERS[9], LAYERS[4]):
+        out, cell = gpu_op.convolution_2d_forward_get_out_shape((N, C, H, W), (K, C, R, S), "NCHW", "SAME", u, u)
+        x, other, w, dy = (nd.array(rng.randn(*shape).astype(np.float32), ctx) for shape in ((N, C, H, W), (N, C, H, W), (K, C, R, S), out))
+        calls.append([x, dy, w, cell, other] + [nd.array(np.full((K, C, R, S), np.nan, np.float32), ctx) for _ in range(3)])
+    wgrad = lambda call, x, out, on: gpu_op.convolution_backward_filter(x, call[1], call[2], out, call[3], handle, on)       # noqa: E731
+    try:
+        for call in calls:
+            wgrad(call, call[0], call[5], one)
+        gpu_op.device_synchronize()
+        gpu_op.hold_products(True)
+        wgrad(calls[0], calls[0][0], calls[0][6], one)
+        wgrad(calls[1], calls[1][0], calls[1][6], two)             # launched at once
+        gpu_op.launch_held(two)
+        gpu_op.device_synchronize()
+        assert np.isnan(calls[0][6].asnumpy()).all()
+        np.testing.assert_array_equal(calls[1][6].asnumpy(), calls[1][5].asnumpy())
+        wgrad(calls[0], calls[0][4], calls[0][7], two)             # packs another input for the same plan, behind what still reads the first
+        gpu_op.hold_products(False)
+        gpu_op.device_synchronize()
+        np.testing.assert_array_equal(calls[0][6].asnumpy(), calls[0][5].asnumpy())
+        assert not np.isnan(calls[0][7].asnumpy()).any() and not np.array_equal(calls[0][7].asnumpy(), calls[0][5].asnumpy())
+        gpu_op.launch_held(one)
+    finally:
+        gpu_op.drop_held()

@@ -126,7 +126,8 @@ __device__ __forceinline__ void amax_commit(const AmaxOut& am, uint32_t m) {
 }
 #endif
 
-// A gradient's call may wait for others (see hold_products in gemm_tcgen05.cu) until launch_held()
+// A gradient's call may wait for others (see hold_products in gemm_tcgen05.cu) until launch_held(): true, and the caller keeps it until
+// its own launch_held_...() is called
 bool may_hold(cudaStream_t s);
 // ---- producers that feed the tensor path ------------------------------------------------------------
 // y = relu(x) fused with the packing of y for the convolution expected to read it (see gemm_tcgen05.cu); 1 = done,

@@ -2298,14 +2298,24 @@ int launch_held_sums(cudaStream_t s);       // ops_basic.cu: bias gradients
 void drop_held_sums();
 int launch_held_direct(cudaStream_t s);     // conv_direct.cu: filter gradients of layers of few channels
 void drop_held_direct();
+// Whatever a thread holds was called on one stream, and is launched there.
+static thread_local bool t_waiting = false;           // something is held, on t_waiting_stream
+static thread_local cudaStream_t t_waiting_stream = nullptr;
 void hold_products(bool on) { t_hold = on; }
-void drop_held() { t_held.clear(); t_held_work = 0; t_hold = false; drop_held_simt(); drop_held_sums(); drop_held_direct(); }
-// The call may wait: its caller says so, and no graph of the caller's own is being captured (it would copy from a table that is gone)
-bool may_hold(cudaStream_t s) {
-  if (!t_hold) return false;
+static void forget_held() { t_held.clear(); t_held_work = 0; t_waiting = false; drop_held_simt(); drop_held_sums(); drop_held_direct(); }
+void drop_held() { forget_held(); t_hold = false; }
+static bool capturing(cudaStream_t s) {
   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(t_recording ? recording_home() : s, &capture) != cudaSuccess) { cudaGetLastError(); return false; }
-  return capture == cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &capture) == cudaSuccess) return capture != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+// The call may wait: its caller says so, nothing that waits was called on another stream, and no graph of the caller's own is being
+// captured (it would copy from a table that is gone).  True: the caller holds it now.
+bool may_hold(cudaStream_t s) {
+  if (!t_hold || (t_waiting && s != t_waiting_stream) || capturing(t_recording ? recording_home() : s)) return false;
+  t_waiting = true; t_waiting_stream = s;
+  return true;
 }
 
 constexpr size_t kStagedCopy = 1 << 16;
@@ -2444,16 +2454,35 @@ static int launch_held_filters(cudaStream_t s) {
     }
   return 0;
 }
-int launch_held(cudaStream_t s) try {
-  if (int rc = launch_held_filters(s)) return rc;
-  if (int rc = launch_held_direct(s)) return rc;
-  if (int rc = launch_held_simt(s)) return rc;
-  return launch_held_sums(s);
-} catch (const std::bad_alloc&) { TF_FAIL("gradients that waited: out of host memory"); }
-// Before the pack at `hi` is written again: what still has to read it goes first.
+// All that waits, on its own stream; after an error nothing waits any more
+int launch_waiting() try {
+  if (!t_waiting) return 0;
+  const cudaStream_t s = t_waiting_stream;
+  t_waiting = false;
+  int rc = launch_held_filters(s);
+  if (!rc) rc = launch_held_direct(s);
+  if (!rc) rc = launch_held_simt(s);
+  if (!rc) rc = launch_held_sums(s);
+  if (rc) forget_held();
+  return rc;
+} catch (const std::bad_alloc&) { forget_held(); TF_FAIL("gradients that waited: out of host memory"); }
+// What waits if it was called on this stream
+int launch_held(cudaStream_t s) { return t_waiting && s == t_waiting_stream ? launch_waiting() : 0; }
+// Before the pack at `hi` is written again, on stream s: what still has to read it goes first.  (While s is captured nothing is written;
+// the order of what the caller makes of the capture is the caller's.)
 static int release_held(const void* hi, cudaStream_t s) {
-  for (const HeldProduct& h : t_held)
-    if (h.g.pack_a == hi || h.g.pack_b == hi) return launch_held_filters(s);
+  for (const HeldProduct& h : t_held) {
+    if (h.g.pack_a != hi && h.g.pack_b != hi) continue;
+    if (int rc = launch_held_filters(t_waiting_stream)) return rc;
+    if (s == t_waiting_stream || capturing(s)) return 0;
+    cudaEvent_t read;
+    TF_CUDA(cudaEventCreateWithFlags(&read, cudaEventDisableTiming));
+    cudaError_t e = cudaEventRecord(read, t_waiting_stream);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, read, 0);
+    cudaEventDestroy(read);
+    TF_CUDA(e);
+    return 0;
+  }
   return 0;
 }
 // Takes the product if it may wait; what has gathered goes when it fills the SMs.
@@ -3231,7 +3260,7 @@ static int launch_wgrad(const ConvTc* st, int bn, int ar, GemmParams& g, cudaStr
   g.operand_bytes = 2.0 * st->dy.bytes() + 2.0 * st->x_pack().bytes();
   g.hold = 1; g.pack_a = st->x_pack().hi; g.pack_b = st->dy.hi;
   const int rc = launch_gemm_bn(bn, ar, g, s, flops, "DLGpuConvolutionBackwardFilter", oom);
-  if (rc == 0 && t_held_work >= (double)kHeldWork * device_sm_count() && launch_held_filters(s)) return -1;
+  if (rc == 0 && t_held_work >= (double)kHeldWork * device_sm_count() && launch_held_filters(t_waiting_stream)) return -1;
   return tc_result(rc);
 }
 int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaStream_t s, int* oom) {

@@ -22,6 +22,7 @@ static std::atomic<uint64_t> g_layout_epoch{1};
 void bump_layout_epoch() { g_layout_epoch.fetch_add(1, std::memory_order_relaxed); }
 int tensor_path_error();
 int launch_held(cudaStream_t s);
+int launch_waiting();
 void drop_held();
 void tc_recording_begins();
 bool dp_active();
@@ -222,6 +223,7 @@ extern "C" {
 int TfStepRecordBegin(void** graph, void** stream_cell, void** replay_stream) {
   TF_REQUIRE(graph && stream_cell && replay_stream && !t_recording, "TfStepRecordBegin: bad arguments, or this thread is recording already");
   flush_deferred();
+  if (launch_waiting()) return -1;       // called before, and not for the recording's stream
   if (g_timing_level > 0 || g_sync_every_op || dp_active() || tensor_path_error() != 0) return 1;
   StepGraph* g = new StepGraph;
   g->words = (uint32_t*)pool_alloc(sizeof(uint32_t) * (kZeroedWords + 2 + kSeedWords));
