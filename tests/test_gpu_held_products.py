@@ -229,3 +229,27 @@ def test_products_wait_on_their_own_stream(lib_path):
         gpu_op.launch_held(one)
     finally:
         gpu_op.drop_held()
+
+
+def test_a_released_descriptor_lets_what_waits_go_first(lib_path):
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, stream, rng = nd.gpu(0), gpu_op.create_cudaStream(), np.random.RandomState(4)
+    handle = gpu_op.create_cudnnHandle(stream)
+    N, C, H, W, K, R, S, u = LAYERS[4]
+    out, cell = gpu_op.convolution_2d_forward_get_out_shape((N, C, H, W), (K, C, R, S), "NCHW", "SAME", u, u)
+    x, w, dy = (nd.array(rng.randn(*shape).astype(np.float32), ctx) for shape in ((N, C, H, W), (K, C, R, S), out))
+    apart, waits = (nd.array(np.full((K, C, R, S), np.nan, np.float32), ctx) for _ in range(2))
+    try:
+        gpu_op.convolution_backward_filter(x, dy, w, apart, cell, handle, stream)
+        gpu_op.hold_products(True)
+        gpu_op.convolution_backward_filter(x, dy, w, waits, cell, handle, stream)
+        gpu_op.hold_products(False)
+        gpu_op.release_descriptor(cell)
+        # arrays of the packs' sizes, in whose place they come
+        rows = N * H * W
+        kept = [nd.array(np.full(rows * c // 2, np.nan, np.float32), ctx) for c in (C, K) for _ in range(4)]
+        gpu_op.launch_held(stream)
+        np.testing.assert_array_equal(waits.asnumpy(), apart.asnumpy())
+        assert len(kept) == 8
+    finally:
+        gpu_op.drop_held()

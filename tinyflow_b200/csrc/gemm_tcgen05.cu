@@ -2470,9 +2470,12 @@ int launch_waiting() try {
 int launch_held(cudaStream_t s) { return t_waiting && s == t_waiting_stream ? launch_waiting() : 0; }
 // Before the pack at `hi` is written again, on stream s: what still has to read it goes first.  (While s is captured nothing is written;
 // the order of what the caller makes of the capture is the caller's.)
+static bool held_reads(const void* hi) {
+  for (const HeldProduct& h : t_held) if (h.g.pack_a == hi || h.g.pack_b == hi) return true;
+  return false;
+}
 static int release_held(const void* hi, cudaStream_t s) {
-  for (const HeldProduct& h : t_held) {
-    if (h.g.pack_a != hi && h.g.pack_b != hi) continue;
+  if (held_reads(hi)) {
     if (int rc = launch_held_filters(t_waiting_stream)) return rc;
     if (s == t_waiting_stream || capturing(s)) return 0;
     cudaEvent_t read;
@@ -2749,13 +2752,15 @@ static ConvTc* conv_state(ConvPlan* p) {
   return (ConvTc*)p->tc_state;
 }
 
-// The state itself stays: notes of producers may name it.  So do packs that a recording writes.
+// The state itself stays: notes of producers may name it.  So do packs that a recording writes.  A product of this thread that waits reads
+// its packs first (if its launch fails it is forgotten, and the error is the thread's last one).
 void tc_release(void* tc_state) {
   ConvTc* st = (ConvTc*)tc_state;
   if (!st) return;
   std::lock_guard<std::mutex> lk(st->mu);
   for (Pack* pk : {&st->x, &st->dy, &st->wf, &st->wd}) {
     if (recordings_use(&pk->src)) continue;
+    if (pk->hi && held_reads(pk->hi)) launch_held_filters(t_waiting_stream);
     pack_release(*pk);
     pk->src = nullptr;
   }
