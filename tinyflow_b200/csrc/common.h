@@ -6,6 +6,7 @@
 #include <stdlib.h>
 #include <string.h>
 #include <atomic>
+#include <new>
 #include <tuple>
 #include <vector>
 #include "../../include/c_runtime_api.h"
@@ -129,6 +130,10 @@ __device__ __forceinline__ void amax_commit(const AmaxOut& am, uint32_t m) {
 // A gradient's call may wait for others (see hold_products in gemm_tcgen05.cu) until launch_held(): true, and the caller keeps it until
 // its own launch_held_...() is called
 bool may_hold(cudaStream_t s);
+template <class T> inline bool held(std::vector<T>& waiting, const T& call) {        // false: no memory to remember it; the call is launched now
+  try { waiting.push_back(call); } catch (const std::bad_alloc&) { return false; }
+  return true;
+}
 // ---- producers that feed the tensor path ------------------------------------------------------------
 // y = relu(x) fused with the packing of y for the convolution expected to read it (see gemm_tcgen05.cu); 1 = done,
 // 0 = not applicable (run the plain kernel), -1 = error.

@@ -399,10 +399,8 @@ int direct_conv_wgrad(const ConvPlan* p, const float* x, const float* dy, float*
   StreamLease lease(s);
   d.part = (float*)lease.scratch(kScratchContract, sizeof(float) * (size_t)grid * cols);
   if (!d.part) return 0;
-  if (d.items <= kWgradThreads && may_hold(s)) {
-    t_held_direct.push_back(HeldDirect{DirectJob{d, dw, grid, cols, 0, 0}, p->S, floats * sizeof(float), 2.0 * p->N * p->K * p->P * p->Q * p->C * p->R * p->S});
-    return 1;
-  }
+  const HeldDirect call{DirectJob{d, dw, grid, cols, 0, 0}, p->S, floats * sizeof(float), 2.0 * p->N * p->K * p->P * p->Q * p->C * p->R * p->S};
+  if (d.items <= kWgradThreads && may_hold(s) && held(t_held_direct, call)) return 1;
   note_compute_stream(s);
   KernelTimer kt("direct_conv", s, 2.0 * p->N * p->K * p->P * p->Q * p->C * p->R * p->S, 0, 1);
   if ((p->S == 3 ? launch_wgrad<3>(d, grid, floats * sizeof(float), s) : p->S == 5 ? launch_wgrad<5>(d, grid, floats * sizeof(float), s) : launch_wgrad<7>(d, grid, floats * sizeof(float), s)) != 0) return -1;

@@ -445,10 +445,7 @@ int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int6
   int cluster = 1;
   while (cluster < (cfg == 0 ? 16 : 8) && tiles * cluster < want && (K + bk - 1) / bk >= 4 * cluster) cluster *= 2;
   p.k_per_cta = (int)(((K + cluster - 1) / cluster + bk - 1) / bk * bk);
-  if (cfg == 1 && tA && !tB && tiles <= kHeldTiles && may_hold(s)) {
-    t_held_simt.push_back(SimtJob{p, cluster, (int)((N + 31) / 32), (int)tiles, 0});
-    return 0;
-  }
+  if (cfg == 1 && tA && !tB && tiles <= kHeldTiles && may_hold(s) && held(t_held_simt, SimtJob{p, cluster, (int)((N + 31) / 32), (int)tiles, 0})) return 0;
   note_compute_stream(s);
   KernelTimer kt("simt_gemm", s, 2.0 * (double)M * (double)N * (double)K, 0, 1);
   if (const int rc = rows_matmul(p, tA, tB, s)) {

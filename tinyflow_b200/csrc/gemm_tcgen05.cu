@@ -2435,7 +2435,7 @@ template <int BN, int AR> static int launch_some(HeldProduct* const* products, i
   TF_REQUIRE(!oom, "filter gradients: the device is out of memory, %d bytes of partial sums short", oom);
   return -1;
 }
-static int launch_held_filters(cudaStream_t s) {
+static int launch_held_filters(cudaStream_t s) try {
   if (t_held.empty()) return 0;
   std::vector<HeldProduct> all;
   all.swap(t_held);
@@ -2453,7 +2453,7 @@ static int launch_held_filters(cudaStream_t s) {
       if (rc) return rc;
     }
   return 0;
-}
+} catch (const std::bad_alloc&) { TF_FAIL("filter gradients: out of host memory"); }
 // All that waits, on its own stream; after an error nothing waits any more
 int launch_waiting() try {
   if (!t_waiting) return 0;
@@ -2491,8 +2491,7 @@ static int release_held(const void* hi, cudaStream_t s) {
 // Takes the product if it may wait; what has gathered goes when it fills the SMs.
 template <int BN, int AR> static bool held_back(const GemmParams& p, size_t workspace_bytes, cudaStream_t s, double flops) {
   if (!could_wait<BN>(p) || p.amax) return false;
-  if (!may_hold(s)) return false;
-  t_held.push_back(HeldProduct{p, BN, AR, workspace_bytes, flops});
+  if (!may_hold(s) || !held(t_held, HeldProduct{p, BN, AR, workspace_bytes, flops})) return false;
   t_held_work += (double)p.m_tiles * p.n_tiles * p.tap_tiles * p.k_total;
   return true;
 }

@@ -331,7 +331,7 @@ int launch_held_sums(cudaStream_t s) {
 static int run_sums(SumJob j, cudaStream_t s, const char* what) {
   StreamLease lease(s);
   if (sum_scratch(&j, 1, lease, what)) return -1;
-  if ((long long)sum_blocks(j) * j.splits <= kHeldSumBlocks && may_hold(s)) { t_held_sums.push_back(j); return 0; }
+  if ((long long)sum_blocks(j) * j.splits <= kHeldSumBlocks && may_hold(s) && held(t_held_sums, j)) return 0;
   note_compute_stream(s);
   const dim3 grid((unsigned)sum_blocks(j), (unsigned)j.splits);
   if (j.kind == kChannelSums) launch_dep(channel_sum_kernel, grid, dim3(kBlock), 0, s, j);
