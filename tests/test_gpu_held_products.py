@@ -253,3 +253,93 @@ def test_a_released_descriptor_lets_what_waits_go_first(lib_path):
         assert len(kept) == 8
     finally:
         gpu_op.drop_held()
+
+
+def _half_way(monkeypatch, ex, node, feed):
+    """A step that ends with an error at `node`, behind gradients that wait."""
+    import random
+    compute, draws, waiting = type(node.op).compute, random.getstate(), []
+
+    def stop(op, n, *rest):
+        if n is node:
+            raise ArithmeticError("stopped")
+        return compute(op, n, *rest)
+    with monkeypatch.context() as m:
+        from tinyflow_b200 import gpu_op
+        m.setattr(type(node.op), "compute", stop)
+        m.setattr(gpu_op, "launch_held", lambda stream: waiting.append("launched"))
+        with pytest.raises(ArithmeticError):
+            ex.run(feed)
+    random.setstate(draws)
+    assert not waiting
+
+
+# a step that an operator stops: what waits is forgotten, and the step after it is the one that would have come
+@pytest.mark.parametrize("name", ["inceptionv3", "lenet5", "mlp"])
+def test_a_step_that_fails_leaves_nothing_behind(lib_path, monkeypatch, name):
+    from tinyflow_b200 import gpu_op
+
+    def fail(step, model, ex, feed, x):
+        if step not in (2, 5):
+            return
+        last = [n for n in ex.topo_order if n in ex._patient]
+        between = [n for n in ex.topo_order if n not in ex._patient and n.index > last[len(last) // 2].index and n.inputs and not n.issgd and type(n.op).__name__ != "AddOp"]
+        _half_way(monkeypatch, ex, between[0], feed)
+        from tinyflow_b200 import ndarray as nd
+        a, b, c = (nd.array(np.full(s, v, np.float32), nd.gpu(0)) for s, v in (((100, 120), 1), ((100, 84), 1), ((120, 84), np.nan)))
+        gpu_op.matrix_multiply(a, True, b, False, c, ex.cublasHandle, ex.cudaStream)       # the switch is off again
+        gpu_op.device_synchronize()
+        assert not np.isnan(c.asnumpy()).any()
+    want = _train(monkeypatch, False, BUILDS[name], "sgd")
+    got = _train(monkeypatch, False, BUILDS[name], "sgd", between=fail)
+    _same(got, want)
+
+
+def _shared_filter(m):
+    """One filter and one bias that two layers share: their gradients are summed before the update reads them."""
+    from tinyflow_b200 import autodiff as ad
+    X, y_, w0, w, b, d = (ad.Placeholder("X"), ad.Placeholder("y_")) + tuple(ad.Variable(n) for n in ("w0", "w", "b", "d"))
+    h = ad.activation_forward_op(ad.convolution_2d_forward_op(X, w0, "NCHW", "SAME", 1, 1), "NCHW", "relu")
+    for _ in range(2):
+        h = ad.activation_forward_op(ad.conv2withbias(h, w, b, "NCHW", "SAME", 1, 1), "NCHW", "relu")
+    y = ad.matmul_op(ad.flatten_op(h), d)
+    return m.Model("shared", X, y_, ad.softmaxcrossentropy_op(y, y_), y, {w0: (32, 16, 3, 3), w: (32, 32, 3, 3), b: (32,), d: (32 * 81, 10)}, (40, 16, 9, 9), (40, 10))
+
+
+def test_a_gradient_that_something_reads_does_not_wait(lib_path, monkeypatch):
+    from tinyflow_b200 import autodiff as ad, gpu_op, models
+    ex = ad.Executor(*(lambda m: (m.loss, m.y))(_shared_filter(models)), 0.01, None, None, None, optimizer="sgd")
+    gradients = [n for n in ex.topo_order if ex._is_parameter_gradient(n)]
+    assert sorted(n in ex._patient for n in gradients) == [False] * 4 + [True] * 2        # w and b twice each; w0 and d
+    got = _train(monkeypatch, True, _shared_filter, "sgd")
+    with monkeypatch.context() as m:
+        m.setattr(gpu_op, "hold_products", lambda on: None)
+        want = _train(monkeypatch, False, _shared_filter, "sgd")
+    _same(got, want)
+
+
+# more than the stages that are launched together at the latest: some go while the rest is still being called
+def test_much_work_does_not_wait_for_the_end(lib_path):
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, stream, rng = nd.gpu(0), gpu_op.create_cudaStream(), np.random.RandomState(6)
+    handle = gpu_op.create_cudnnHandle(stream)
+    N, C, H, W, K = 16, 2048, 24, 24, 64                         # 16 tiles of 144 stages
+    out, cell = gpu_op.convolution_2d_forward_get_out_shape((N, C, H, W), (K, C, 1, 1), "NCHW", "SAME", 1, 1)
+    x, w, dy = (nd.array(rng.randn(*shape).astype(np.float32), ctx) for shape in ((N, C, H, W), (K, C, 1, 1), out))
+    apart = nd.empty((K, C, 1, 1), ctx)
+    gpu_op.convolution_backward_filter(x, dy, w, apart, cell, handle, stream)
+    results = [nd.array(np.full((K, C, 1, 1), np.nan, np.float32), ctx) for _ in range(80)]          # 184,320 tile stages; 148 SMs take 151,552
+    try:
+        gpu_op.hold_products(True)
+        counts = [gpu_op.launch_count()]
+        for r in results:
+            gpu_op.convolution_backward_filter(x, dy, w, r, cell, handle, stream)
+            counts.append(gpu_op.launch_count())
+        gpu_op.hold_products(False)
+        assert sum(b > a for a, b in zip(counts, counts[1:])) == 1
+        gpu_op.launch_held(stream)
+        assert gpu_op.launch_count() > counts[-1]
+    finally:
+        gpu_op.drop_held()
+    for r in results:
+        np.testing.assert_array_equal(r.asnumpy(), apart.asnumpy())
