@@ -324,9 +324,14 @@ int TfStepRecordBegin(void **graph, void **stream_cell, void **replay_stream);
  * already, where the convolutions of the step would pack them one by one.  A hint: what is left out is packed when its
  * convolution comes. */
 int TfPackFilters(const DLArrayHandle *filters, void ***const *plans, int n, void **cudaStream);
-/* Filter gradients called between TfHoldProducts(1) and TfHoldProducts(0) by this thread may wait for others, to share a launch with
- * them: their results are there after TfLaunchHeld on the stream they were called on.  Until then nothing may read them, and the
- * input and the incoming gradient of the convolution may not be freed.  TfDropHeld forgets those that wait (a step that failed). */
+/* Gradients of parameters called between TfHoldProducts(1) and TfHoldProducts(0) by this thread may wait for others, to share launches
+ * with them: DLGpuConvolutionBackwardFilter, DLGpuMatrixMultiply whose first operand is transposed and whose second is not, and the sums
+ * DLGpuReduceSum, DLGpuReduceSumAxisZero and DLGpuBroadcastToBackward0/1.  The result of every such call is there after TfLaunchHeld on
+ * the stream it was called on (the sums without a stream argument: the stream they run on).  Until then nothing may read the result, the arrays that the
+ * call reads may be neither freed nor written, and no other thread may call or release the convolution's descriptor.
+ * What waits was called on one stream; calls on another one meanwhile do not wait, and TfLaunchHeld there launches nothing.
+ * A call sees to what memory it needs on its own before it waits, and reports a shortage as it does without waiting.  After an
+ * error of TfLaunchHeld nothing waits.  TfDropHeld forgets what waits (a step that failed) and ends the holding. */
 int TfHoldProducts(int on);
 int TfLaunchHeld(void **cudaStream);
 int TfDropHeld(void);

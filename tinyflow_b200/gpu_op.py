@@ -434,7 +434,9 @@ def pack_filters(filters, cells, cudaStream):
 
 
 def hold_products(on):
-    """Filter gradients called from here on may wait for others until :func:`launch_held`: nobody reads them before."""
+    """Between ``hold_products(True)`` and ``hold_products(False)`` gradients of parameters may wait for others until :func:`launch_held`:
+    filter gradients, ``matrix_multiply`` of a transposed first operand, and sums (``reduce_sum_new``, ``reduce_sum_axis_zero``,
+    ``broadcast_to_backward``).  Until then nobody may read their results, nor free or write what they read."""
     check_call(_LIB.TfHoldProducts(1 if on else 0))
 
 
