@@ -1087,7 +1087,7 @@ struct GroupTable {
   float* workspace;
   int* err;
 };
-// stages of the pieces that tile `tile` of a held-back product is added up from
+// number of pieces that tile `tile` of a held-back product is added up from
 __host__ __device__ inline int tile_pieces(const GemmParams& p, int tile) { return p.cluster > 1 ? p.cluster : p.tail_pieces > 0 && tile >= p.full_tiles ? p.tail_pieces : 1; }
 struct GroupIter {
   int at, end, piece, last;
@@ -2214,6 +2214,8 @@ template <int BN, class F> static cudaError_t launch_reduce(int tiles, int piece
   if (pieces >= 12 && tiles * (BN / kReduceCols) <= 2 * device_sm_count()) return launch(std::true_type(), dim3(grid.x, grid.y, BM / 32), dim3(kReduceThreads<true>));
   return launch(std::false_type(), grid, dim3(kReduceThreads<false>));
 }
+// Stages per CTA from which a product is launched on its own: at 128 columns those that take two issuers (groups hold products of one
+// layout of the accumulators); at 64 columns 102 still gain (DenseNet-121 13.76 -> 13.50 ms against a limit of 24).
 template <int BN> constexpr int kHeldRun = BN == 64 ? 160 : 24;
 // By its schedule the product could wait for others (see held_back)
 template <int BN> static bool could_wait(const GemmParams& p) {
@@ -2283,14 +2285,12 @@ template <int BN, int AR> static int launch_planned(GemmParams& p, size_t bytes,
 // ---- filter gradients that wait for others -------------------------------------------------------------------------
 // Between TfHoldProducts(1) and (0) the caller says that nothing but TfLaunchHeld() stands between a filter gradient and its readers
 // (the executor: only the parameter updates at the end of the step read it), and that what the product reads, the packs of its
-// plan, is not packed anew before (release_held() looks after that).  Products whose CTAs have many stages to do are launched
+// plan, is not packed anew before (release_held() looks after that; the kernels of the other files read the arrays themselves).  Products whose CTAs have many stages to do are launched
 // at once: they gain nothing, and their operands are in L2 now.
 struct HeldProduct { GemmParams g; int bn, ar; size_t workspace_bytes; double flops; };
 static thread_local bool t_hold = false;
 static thread_local std::vector<HeldProduct> t_held;
 static thread_local double t_held_work = 0;           // tiles x stages
-// Stages per CTA from which a product is launched on its own: at 128 columns those that take two issuers (groups hold products of one
-// layout of the accumulators); at 64 columns 102 still gain (DenseNet-121 13.76 -> 13.50 ms against a limit of 24).
 constexpr int kHeldWork = 1024;                       // stages per SM that are launched together at the latest (64: ResNet-50 b19 4096 us, 256: 3999, 512 and all: 3976)
 int launch_held_simt(cudaStream_t s);       // gemm_simt.cu: weight gradients of dense layers
 void drop_held_simt();
@@ -2488,7 +2488,7 @@ static int release_held(const void* hi, cudaStream_t s) {
   }
   return 0;
 }
-// Takes the product if it may wait; what has gathered goes when it fills the SMs.
+// Takes the product if it may wait
 template <int BN, int AR> static bool held_back(const GemmParams& p, size_t workspace_bytes, cudaStream_t s, double flops) {
   if (!could_wait<BN>(p) || p.amax) return false;
   if (!may_hold(s) || !held(t_held, HeldProduct{p, BN, AR, workspace_bytes, flops})) return false;
@@ -3096,7 +3096,9 @@ static int conv_like(const Pack& act, const Pack& filt, int ch_in, int ch_out, i
   // Few tiles of a short reduction: 64 columns, so that nearly twice the CTAs each do a stage of two thirds the time.  Up to 64 tiles
   // and 32 stages: Inception-v3 b2 3616 -> 3490 us a step, DenseNet-121 b32 12.60 -> 12.50 ms (longer reductions fill the SMs by being
   // cut, and a wide tile costs less a stage: all of up to 148 tiles, VGG-16 b7 1331 -> 1356 us).  Where fewer pieces are left, more stages
-  // gather in an accumulator; a promotion after every second one keeps the error where it was.
+  // gather in an accumulator; a promotion after every second one keeps the error where it was: rms against float64 over twelve layers, in
+  // 2^-24 of the result's, forward / input gradient, 4.28 / 4.37 with wide tiles and 3.27 / 3.40 so.  3xTF32 promotes after every
+  // second stage anyway, 3.10 / 3.36 with wide tiles and 3.06 / 3.31 so.
   if (bn > 64) {
     const long long mt = (act.rows + BM - 1) / BM;
     if (mt * ((ch_out + bn - 1) / bn) <= kNarrowTiles && mt * ((ch_out + 63) / 64) <= device_sm_count() && taps.n * ((ch_in + bk - 1) / bk) <= kNarrowStages) {
@@ -3168,7 +3170,9 @@ int tc_fused_relu_pack(const void* node, const float* x, float* y, int64_t n, cu
   return 1;
 }
 // ReLU backward (held back by its entry point) whose output is the dy of a convolution's backward call: out = mask > 0 ? dy : 0
-// and the plan's pack of it in one pass.  1 when it did that, 0 when the caller should run the ReLU on its own.
+// and the plan's pack of it in one pass.  1 when it did that, 0 when the caller should run the ReLU on its own.  The scale comes from max|dy|: where
+// that lies 2^r above max|out|, because the mask takes the largest values away, the pack keeps out to 2^(r-39) of max|out| and better: half an fp32
+// ulp of it, 2^-25, up to r = 14.
 int tc_fused_relu_bwd_pack(ConvPlan* p, const float* mask, const float* dy, float* out, cudaStream_t s) {
   ConvTc* st = conv_state(p);
   // (a layer of few channels goes through here as patches, unless the direct kernels take it: they have up to 32 filters at stride 1)
@@ -3264,6 +3268,7 @@ static int launch_wgrad(const ConvTc* st, int bn, int ar, GemmParams& g, cudaStr
   g.operand_bytes = 2.0 * st->dy.bytes() + 2.0 * st->x_pack().bytes();
   g.hold = 1; g.pack_a = st->x_pack().hi; g.pack_b = st->dy.hi;
   const int rc = launch_gemm_bn(bn, ar, g, s, flops, "DLGpuConvolutionBackwardFilter", oom);
+  // what has gathered goes when it fills the SMs
   if (rc == 0 && t_held_work >= (double)kHeldWork * device_sm_count() && launch_held_filters(t_waiting_stream)) return -1;
   return tc_result(rc);
 }
