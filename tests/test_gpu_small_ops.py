@@ -35,6 +35,29 @@ def test_weight_gradients_of_few_rows(env, M, K, N):
     test_simt_product_at_tile_edges(env, M, K, N, True, False)
 
 
+def _kernels(run):
+    import ctypes
+    import json
+    from tinyflow_b200._base import _LIB
+    report = ctypes.create_string_buffer(1 << 16)
+    _LIB.TfKernelTimingEnable(1)
+    try:
+        run()
+        _LIB.TfKernelTimingReport(report, len(report))
+    finally:
+        _LIB.TfKernelTimingEnable(0)
+    return [r["name"] for r in json.loads(report.value.decode())]
+
+
+# shapes that the kernels for a handful of rows take on 148 SMs: 8 and 16 rows to a block, runs of K and clusters that are not whole (clusters of
+# 8, 4 and 1 CTAs, K of 4602, 2052, 2100, 1100 and 36; C = A B^T: 1, 2, 4 and 8 runs of a row), ragged columns
+@pytest.mark.parametrize("M,K,N,tA,tB", [(7, 4608, 4096, False, False), (7, 4602, 4096, False, False), (16, 2052, 4096, False, False), (11, 2100, 2500, False, False), (13, 36, 40004, False, False),
+                                         (9, 1100, 9004, False, False), (12, 1000, 4096, False, True), (16, 2052, 4098, False, True), (9, 4100, 2401, False, True), (5, 4604, 3000, False, True), (9, 4096, 1601, False, True),
+                                         (15, 132, 9001, False, True), (1000, 7, 1028, True, False), (2052, 9, 516, True, False), (36, 16, 40000, True, False)])
+def test_products_of_few_rows_take_their_kernels(env, M, K, N, tA, tB):
+    assert _kernels(lambda: test_simt_product_at_tile_edges(env, M, K, N, tA, tB)) == ["rows_gemm"]
+
+
 @pytest.mark.parametrize("case", [(3, 1, 28, 28, 6, 5, 5, "SAME"), (5, 6, 14, 14, 16, 5, 5, "VALID"), (2, 3, 9, 7, 5, 3, 3, "SAME"), (300, 2, 8, 8, 3, 7, 7, "SAME"),
                                   (2, 8, 11, 13, 32, 1, 3, "SAME"), (1, 5, 40, 33, 7, 3, 3, "VALID")])
 def test_direct_convolution_of_few_channels(env, case):

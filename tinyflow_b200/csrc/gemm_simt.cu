@@ -368,6 +368,7 @@ template <int MR> static int launch_rows_nn(SimtGemm p, cudaStream_t s) {
   if (smem() > kRowSmem || groups * cluster < sms) return 0;
   static const cudaError_t attr = cudaFuncSetAttribute(rows_nn_kernel<MR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowSmem);
   TF_CUDA(attr);
+  KernelTimer kt("rows_gemm", s, 2.0 * (double)p.M * p.N * p.K, 0, 1);
   TF_CUDA(launch_cluster(rows_nn_kernel<MR>, cluster, dim3(groups * cluster), dim3(kRowThreads), smem(), s, p));
   return 1;
 }
@@ -385,12 +386,14 @@ static int rows_matmul(const SimtGemm& p, bool tA, bool tB, cudaStream_t s) {
       runs = (p.K + q.k_per_cta - 1) / q.k_per_cta;
       while (kRowWarps % runs) { q.k_per_cta += 128; runs = (p.K + q.k_per_cta - 1) / q.k_per_cta; }       // whole sets in a block
       const dim3 grid((unsigned)((sets * runs + kRowWarps - 1) / kRowWarps));
+      KernelTimer kt("rows_gemm", s, 2.0 * (double)p.M * p.N * p.K, 0, 1);
       TF_CUDA(p.M <= 8 ? launch_dep(rows_nt_kernel<8>, grid, dim3(kRowThreads), 0, s, q) : launch_dep(rows_nt_kernel<16>, grid, dim3(kRowThreads), 0, s, q));
       return 1;
     }
   }
   if (tA && !tB && p.K <= kFewRows && (double)p.M * p.N >= 1e6 && p.a_vec && p.b_vec && p.c_vec && p.M % 4 == 0 && p.N % 4 == 0 && (p.M + kOuterRows - 1) / kOuterRows <= 65535) {
     const dim3 grid((p.N + 4 * kRowThreads - 1) / (4 * kRowThreads), (p.M + kOuterRows - 1) / kOuterRows);
+    KernelTimer kt("rows_gemm", s, 2.0 * (double)p.M * p.N * p.K, 0, 1);
     TF_CUDA(p.K <= 8 ? launch_dep(rows_tn_kernel<8>, grid, dim3(kRowThreads), 0, s, p) : launch_dep(rows_tn_kernel<16>, grid, dim3(kRowThreads), 0, s, p));
     return 1;
   }
@@ -447,12 +450,12 @@ int simt_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int6
   p.k_per_cta = (int)(((K + cluster - 1) / cluster + bk - 1) / bk * bk);
   if (cfg == 1 && tA && !tB && tiles <= kHeldTiles && may_hold(s) && held(t_held_simt, SimtJob{p, cluster, (int)((N + 31) / 32), (int)tiles, 0})) return 0;
   note_compute_stream(s);
-  KernelTimer kt("simt_gemm", s, 2.0 * (double)M * (double)N * (double)K, 0, 1);
   if (const int rc = rows_matmul(p, tA, tB, s)) {
     if (rc < 0) return -1;
     TF_AFTER(s, what);
     return 0;
   }
+  KernelTimer kt("simt_gemm", s, 2.0 * (double)M * (double)N * (double)K, 0, 1);
   const cudaError_t e = cfg == 0 ? launch_simt_layout<8, 64, 8, 1, 32>(p, !tA, tB, cluster, s)
                       : cfg == 1 ? launch_simt_layout<32, 32, 4, 2, 32>(p, !tA, tB, cluster, s)
                                  : launch_simt_layout<64, 64, 4, 4, 16>(p, !tA, tB, cluster, s);
