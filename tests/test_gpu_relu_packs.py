@@ -131,3 +131,49 @@ def test_a_first_step_has_the_bits_of_later_ones(env, readers, whole):
     for later in steps[1:]:
         for a, b in zip(steps[0], later):
             np.testing.assert_array_equal(a, b)
+
+
+# the mask takes away gradients 2^4, 2^10 and 2^14 times the largest that is left: the fused pack, scaled by the larger maximum, against the one on its own and 64 bits
+@pytest.mark.parametrize("power", [4, 10, 14])
+@pytest.mark.parametrize("case", [(6, 3, 33, 40, 64, 3, 1, 2, 2), (6, 32, 24, 22, 64, 3, 1, 3, 2)])
+def test_a_bound_far_above_what_the_mask_leaves(env, case, power):
+    import torch
+    N, C, H, W, K, R, stride, win, step = case
+    rng = np.random.RandomState(H + K)
+    gpu, nd = env.gpu_op, env.nd
+    x, w = np.abs(rng.randn(N, C, H, W)).astype(np.float32), rng.randn(K, C, R, R).astype(np.float32)
+    w[0] = -np.abs(w[0])                          # channel 0 is never positive
+    mid, cell = gpu.convolution_2d_forward_get_out_shape(x.shape, w.shape, "NCHW", "SAME", stride, stride)
+    out, pool = gpu.pooling_2d_forward_get_out_shape(mid, "NCHW", "max", 0, 0, step, step, win, win)
+    act = gpu.activation_get_cudnnlist(mid, "NCHW", "relu")
+    do = rng.randn(*out).astype(np.float32)
+    do[:, 0] *= 2.0 ** power
+    X, Wd, DO = (nd.array(v, env.ctx) for v in (x, w, do))
+    y, a, da, dy = (nd.empty(mid, env.ctx) for _ in range(4))
+    o, dw = nd.empty(out, env.ctx), nd.empty(w.shape, env.ctx)
+    got = []
+    gpu.set_contraction_path(2)
+    try:
+        for apart in (True, False):
+            gpu.convolution_2d_forward(X, Wd, y, cell, env.cudnn, env.stream)
+            gpu.activation_forward(y, a, "relu", act, env.cudnn, env.stream)
+            gpu.pooling_2d_forward(a, o, pool, env.cudnn, env.stream)
+            gpu.pooling_2d_backward(a, o, DO, da, pool, env.cudnn, env.stream)
+            before = gpu.launch_count()
+            gpu.activation_backward(y, dy, a, da, "relu", act, env.cudnn, env.stream)
+            if apart:
+                gpu.device_synchronize()
+            gpu.convolution_backward_filter(X, dy, Wd, dw, cell, env.cudnn, env.stream)
+            got.append((gpu.launch_count() - before, dw.asnumpy()))
+    finally:
+        gpu.set_contraction_path(0)
+    assert got[1][0] < got[0][0]
+    grad = dy.asnumpy()
+    bound, left = np.abs(da.asnumpy()).max(), np.abs(grad).max()
+    assert bound > 2.0 ** (power - 1) * left
+    # a kept value is off by 2^-22 of itself or 2^-25 / scale, scale >= 2^14 / bound, whichever is more; products are summed in fp32
+    exact = lambda g: torch.nn.grad.conv2d_weight(torch.from_numpy(x).double(), w.shape, torch.from_numpy(g).double(), stride, R // 2).numpy()       # noqa: E731
+    want, mag, each = exact(grad), exact(np.abs(grad)), exact(np.ones_like(grad))
+    for _, dwv in got:
+        assert np.all(np.abs(dwv - want) <= 8 * 2.0 ** -24 * mag + 2.0 ** -39 * bound * each)
+    np.testing.assert_array_equal(got[1][1][0], 0)
