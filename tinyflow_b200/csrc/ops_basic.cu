@@ -59,11 +59,14 @@ template <class F> struct TracksAmax<F, decltype((void)F::kTrackAmax)> { static 
 __device__ __forceinline__ uint32_t amax4(uint32_t m, const float4& r) {
   return max(max(m, amax_bits(r.x)), max(amax_bits(r.y), max(amax_bits(r.z), amax_bits(r.w))));
 }
-// Functors with once(): one thread of the launch calls it.
-template <class F, class = void> struct HasOnce { static constexpr bool value = false; };
-template <class F> struct HasOnce<F, decltype((void)&F::once)> { static constexpr bool value = true; };
+// Functors with begin() and end(): one thread of the launch calls them around its elements, end() with what begin() read, so that the read
+// is in flight meanwhile (a kernel of one wave would otherwise end with it).
+template <class F, class = void> struct HasBegin { static constexpr bool value = false; };
+template <class F> struct HasBegin<F, decltype((void)&F::begin)> { static constexpr bool value = true; };
 template <class F> __global__ void __launch_bounds__(kBlock) map1_kernel(const float* __restrict__ a, float* __restrict__ o, int64_t n, F f, AmaxOut am) {
   grid_dep_sync();
+  [[maybe_unused]] uint32_t word = 0;
+  if constexpr (HasBegin<F>::value) if (blockIdx.x == 0 && threadIdx.x == 0) word = f.begin();
   int64_t nv = n >> 2, stride = (int64_t)gridDim.x * blockDim.x;
   const float4* a4 = reinterpret_cast<const float4*>(a);
   float4* o4 = reinterpret_cast<float4*>(o);
@@ -75,7 +78,7 @@ template <class F> __global__ void __launch_bounds__(kBlock) map1_kernel(const f
     if (TracksAmax<F>::value) m = amax4(m, x);
   }
   for (int64_t i = (nv << 2) + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) { float r = f(a[i]); o[i] = r; if (TracksAmax<F>::value) m = max(m, amax_bits(r)); }
-  if constexpr (HasOnce<F>::value) if (blockIdx.x == 0 && threadIdx.x == 0) f.once();
+  if constexpr (HasBegin<F>::value) if (blockIdx.x == 0 && threadIdx.x == 0) f.end(word);
   if (TracksAmax<F>::value) amax_commit(am, m);
 }
 template <class F> __global__ void __launch_bounds__(kBlock) map1_scalar_kernel(const float* a, float* o, int64_t n, F f) {
@@ -160,7 +163,7 @@ struct FMulC { float c; __device__ float operator()(float x) const { return x * 
 struct FAddArr { const float* c; __device__ float operator()(float x) const { return x + __ldg(c); } };      // the scalar lies in device memory
 struct FMulArr { const float* c; __device__ float operator()(float x) const { return x * __ldg(c); } };
 struct FRelu { static constexpr bool kTrackAmax = true; __device__ float operator()(float x) const { return x > 0.f ? x : (x != x ? x : 0.f); } };   // NaN propagates
-struct FReluKeep : FRelu { ReluBound bound; __device__ void once() const { if (bound.to) *bound.to = *bound.from; } };      // and the bound of its input
+struct FReluKeep : FRelu { ReluBound bound; __device__ uint32_t begin() const { return *bound.from; } __device__ void end(uint32_t word) const { *bound.to = word; } };      // and the bound of its input
 struct FExp { __device__ float operator()(float x) const { return expf(x); } };
 struct FLog { __device__ float operator()(float x) const { return logf(x); } };
 struct FRecip { __device__ float operator()(float x) const { return 1.f / x; } };
@@ -195,11 +198,11 @@ __global__ void __launch_bounds__(kBlock) bcast_channel_kernel(const float* __re
 // Block = 32 columns x 8 row lanes; grid.x tiles the columns, grid.y splits the rows.
 enum { kColumnSums, kChannelSums };
 struct SumJob {               // column sums of [rows][cols], or channel sums of [rows = images][cols = channels][length, which may be 0]
-  int kind;
   const float* in; float* out; float* part; uint32_t* counters;
   int64_t rows, cols, length, per_split;
   int splits, vec;            // vec: 16-byte loads along `length`
   int first_block;            // of a group's launch
+  int kind;
 };
 __device__ __forceinline__ void column_sum(const SumJob& p, int block, int split) {
   __shared__ float sm[8][33];
@@ -912,7 +915,7 @@ static int channel_sums(const float* in, float* out, int64_t N, int64_t C, int64
   const int64_t nps = std::max<int64_t>(1, (N + splits - 1) / splits);
   splits = std::max<int64_t>(1, (N + nps - 1) / nps);
   const int vec = L % 4 == 0 && aligned16(in) && nps * (L / 4) < (1ll << 31);
-  return run_sums(SumJob{kChannelSums, in, out, nullptr, nullptr, N, C, L, nps, (int)splits, vec, 0}, s, what);
+  return run_sums(SumJob{in, out, nullptr, nullptr, N, C, L, nps, (int)splits, vec, 0, kChannelSums}, s, what);
 }
 
 static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, cudaStream_t s, const char* what) {
@@ -927,7 +930,7 @@ static int column_sums(const float* in, float* out, int64_t rows, int64_t cols, 
   }
   const int64_t rps = std::max<int64_t>(1, (rows + splits - 1) / splits);
   splits = std::max(1, (int)((rows + rps - 1) / rps));
-  return run_sums(SumJob{kColumnSums, in, out, nullptr, nullptr, rows, cols, 0, rps, splits, 0, 0}, s, what);
+  return run_sums(SumJob{in, out, nullptr, nullptr, rows, cols, 0, rps, splits, 0, 0, kColumnSums}, s, what);
 }
 
 int DLGReduceSumGetCudnnlist(const int* input_shapes, const int* output_shapes, const int sizeofshape,
@@ -1346,7 +1349,7 @@ int DLGpuActivationForward(const DLArrayHandle input, DLArrayHandle output, int 
       if (fused) return 0;
       FReluKeep relu;
       if (node && aligned16(input->data) && aligned16(output->data)) relu.bound = tc_relu_bound(F(input), F(output));
-      int rc = run_map1(F(input), FM(output), n, s, "DLGpuActivationForward(relu)", relu);
+      int rc = relu.bound.to ? run_map1(F(input), FM(output), n, s, "DLGpuActivationForward(relu)", relu) : run_map1(F(input), FM(output), n, s, "DLGpuActivationForward(relu)", FRelu{});
       tc_note_relu_output(node, output->data, input->data, relu.bound.to != nullptr);
       return rc;
     }
