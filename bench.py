@@ -35,12 +35,12 @@ WORKLOADS = {
 }
 
 
-# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the contraction kernel, from one profiler
-# capture: every distinct convolution layer of the workload at its benchmark batch launched on its own (`--layer WORKLOAD`,
-# a few hundred MB on the device at a time), each layer's three launches weighted by how often the layer occurs in the graph.
+# DRAM traffic (dram__bytes_read.sum + dram__bytes_write.sum) of a step's convolution products, from one profiler capture:
+# every distinct convolution layer of the workload at its benchmark batch launched on its own (`--layer WORKLOAD`,
+# a few hundred MB on the device at a time), each layer's three products weighted by how often the layer occurs in the graph.
 # The full step holds tens of GB and its counters need several replay passes, so it is not captured whole; a layer's
 # operands are the same size either way.  profiles/gemm3x_dram_traffic_resnet50_b64.md has the command and the table.
-CONTRACTION_DRAM_BYTES_PER_LAUNCH = {("resnet50", "3xfp16"): 88.9e6}
+CONTRACTION_DRAM_BYTES_PER_STEP = {("resnet50", "3xfp16"): 12.90e9}
 
 
 def build_model(name, batch=None):
@@ -567,9 +567,10 @@ def main():
             # tensor rate (fp16 runs at the bf16 rate), sustained figure because the kernel runs inside a long step
             peak = peaks.get("bf16_tflops_sustained", peaks["bf16_tflops"])
             ach = top["flops"] / (top["ms"] / 1000.0) / 1e12
+            layer_bytes = CONTRACTION_DRAM_BYTES_PER_STEP.get((args.workload, gpu_op.tensor_arithmetic()))
             roofline = {"bound": "tensor", "kernel": top["name"], "achieved": ach, "peak": peak, "unit": "TFLOP/s", "frac": ach / peak,
-                        "traffic": CONTRACTION_DRAM_BYTES_PER_LAUNCH.get((args.workload, gpu_op.tensor_arithmetic())) if args.batch is None else None,
-                        "traffic_source": "DRAM read+write bytes per launch: profiler capture of each distinct convolution layer of this workload at this batch, launched on its own, weighted by its count in the graph (not captured in this run)",
+                        "traffic": layer_bytes * args.steps / top["launches"] if layer_bytes and args.batch is None else None,
+                        "traffic_source": "DRAM read+write bytes per launch: profiler capture of each distinct convolution layer of this workload at this batch, launched on its own, weighted by its count in the graph, over the launches of a step, some of which hold many filter gradients (not captured in this run)",
                         "launches": top["launches"], "avg_us": 1000.0 * top["ms"] / max(top["launches"], 1),
                         "issued": 3.0 * ach, "issued_frac": 3.0 * ach / peak,
                         "timed_over": "%d steps repeated right after the timed region with an event pair around each launch (%.3f ms per step there)" % (args.steps, instrumented_ms),
