@@ -177,3 +177,61 @@ def test_a_bound_far_above_what_the_mask_leaves(env, case, power):
     for _, dwv in got:
         assert np.all(np.abs(dwv - want) <= 8 * 2.0 ** -24 * mag + 2.0 ** -39 * bound * each)
     np.testing.assert_array_equal(got[1][1][0], 0)
+
+
+# an operator call ahead of a recorded step writes what its first convolution packs: another bound by the next replay, or none
+@pytest.mark.parametrize("how", ["relu", "copy"])
+@pytest.mark.parametrize("arith", ["3xfp16", "3xtf32"])
+def test_a_replay_packs_what_a_relu_wrote_since(env, how, arith):
+    import ctypes
+    from tinyflow_b200._base import _LIB, check_call, new_cell
+    N, C, H, W, K = 24, 64, 14, 15, 48
+    rng = np.random.RandomState(11)
+    gpu, nd = env.gpu_op, env.nd
+    f = lambda *shape: nd.array(rng.randn(*shape).astype(np.float32), env.ctx)       # noqa: E731
+    X, W1, W2 = f(N, C, H, W), f(K, C, 3, 3), f(64, K, 3, 3)
+    mid, cell1 = gpu.convolution_2d_forward_get_out_shape(X.shape, W1.shape, "NCHW", "SAME", 1, 1)
+    out, cell2 = gpu.convolution_2d_forward_get_out_shape(mid, W2.shape, "NCHW", "SAME", 1, 1)
+    act = gpu.activation_get_cudnnlist(mid, "NCHW", "relu")
+    y1, a1, y2 = nd.empty(mid, env.ctx), nd.empty(mid, env.ctx), nd.empty(out, env.ctx)
+
+    def ahead():
+        gpu.convolution_2d_forward(X, W1, y1, cell1, env.cudnn, env.stream)
+        gpu.activation_forward(y1, a1, "relu", act, env.cudnn, env.stream)
+
+    def record():
+        graph, on = ctypes.c_void_p(), new_cell(2)
+        check_call(_LIB.TfStepRecordBegin(ctypes.byref(graph), on, env.stream))
+        gpu.convolution_2d_forward(a1, W2, y2, cell2, env.cudnn, on)
+        check_call(_LIB.TfStepRecordEnd(ctypes.byref(graph), 1))
+        return graph
+    gpu.set_contraction_path(2)
+    gpu.set_tensor_arithmetic(arith)
+    graph = None
+    try:
+        ahead()
+        gpu.convolution_2d_forward(a1, W2, y2, cell2, env.cudnn, env.stream)
+        ahead()
+        graph = record()
+        small = None
+        for scale in (1.0, 2.0 ** 12):                       # a power of two: every bit but the exponent stays
+            if scale > 1 and how == "relu":
+                W1[:] = W1.asnumpy() * np.float32(scale)
+                ahead()
+            elif scale > 1:
+                a1[:] = a1.asnumpy() * np.float32(scale)
+            y2[:] = np.full(out, np.nan, np.float32)
+            rc = _LIB.TfStepReplay(graph, None, 0, ctypes.c_float(0), ctypes.c_float(0), None, 0, env.stream)
+            assert rc == 0 or (rc == 1 and scale > 1 and how == "copy")
+            if rc == 1:                                      # nothing knows the new maximum: the caller records again
+                _LIB.TfStepGraphFree(graph)
+                graph = record()
+                check_call(_LIB.TfStepReplay(graph, None, 0, ctypes.c_float(0), ctypes.c_float(0), None, 0, env.stream))
+            got = y2.asnumpy()
+            small = got if scale == 1 else small
+            np.testing.assert_allclose(got, small * np.float32(scale), rtol=0, atol=2e-6 * scale * np.abs(small).max())
+    finally:
+        if graph is not None:
+            _LIB.TfStepGraphFree(graph)
+        gpu.set_contraction_path(0)
+        gpu.set_tensor_arithmetic("3xfp16")

@@ -81,6 +81,8 @@ struct AmaxSlot {
   uint64_t rec = 0; uint32_t* rec_word = nullptr; uint64_t rec_version = 0; bool rec_wants_carry = false;
 };
 static std::unordered_map<const void*, AmaxSlot> g_amax;
+// A key is an array's address, or an odd address in its first word (bound_key): such a word is as old as the array, whoever writes that.
+static uint64_t array_version_locked(const void* key) { return version_locked(reinterpret_cast<const void*>(reinterpret_cast<uintptr_t>(key) & ~uintptr_t(3))); }
 static uint32_t* g_amax_chunk = nullptr;
 static int g_amax_left = 0;
 static uint32_t* amax_chunk_words(int n) {
@@ -106,13 +108,13 @@ AmaxOut amax_track_begin(const void* data) {
   if (t_recording) {
     amax_enter_recording(sl);
     sl.rec_word = recording_word();
-    sl.rec_version = version_locked(data);
+    sl.rec_version = array_version_locked(data);
     return AmaxOut{sl.rec_word, nullptr};
   }
   if (!sl.words && !(sl.words = amax_chunk_words(2))) return AmaxOut{};
   const int k = (int)(sl.uses++ & 1u);
   sl.cur = k;
-  sl.version = version_locked(data);
+  sl.version = array_version_locked(data);
   return AmaxOut{sl.words + k, sl.words + (k ^ 1)};
 }
 const uint32_t* amax_tracked(const void* data) {
@@ -120,7 +122,7 @@ const uint32_t* amax_tracked(const void* data) {
   auto it = g_amax.find(data);
   if (it == g_amax.end()) return nullptr;
   AmaxSlot& sl = it->second;
-  const uint64_t v = version_locked(data);
+  const uint64_t v = array_version_locked(data);
   if (t_recording && sl.rec == recording_id() && sl.rec_word && sl.rec_version == v) return sl.rec_word;
   const uint32_t* found = sl.words && sl.version == v ? sl.words + sl.cur : (sl.carry && sl.carry_version == v ? sl.carry : nullptr);
   if (!t_recording || !found) return found;
@@ -138,7 +140,7 @@ bool amax_take_carries(uint64_t recording, AmaxCarry* out, int max, int* count) 
     if (sl.rec != recording) continue;
     if (sl.rec_wants_carry) {
       if (*count >= max) return false;
-      const bool rewritten = sl.rec_word && sl.rec_version == version_locked(kv.first);     // by a kernel that tracks its maximum, last
+      const bool rewritten = sl.rec_word && sl.rec_version == array_version_locked(kv.first);     // by a kernel that tracks its maximum, last
       out[(*count)++] = AmaxCarry{kv.first, sl.carry, rewritten ? sl.rec_word : nullptr};
     }
     sl.rec = 0;
@@ -148,11 +150,11 @@ bool amax_take_carries(uint64_t recording, AmaxCarry* out, int max, int* count) 
 bool amax_carry_valid(const void* data) {
   std::lock_guard<std::mutex> lk(g_ver_mu);
   auto it = g_amax.find(data);
-  return it != g_amax.end() && it->second.carry && it->second.carry_version == version_locked(data);
+  return it != g_amax.end() && it->second.carry && it->second.carry_version == array_version_locked(data);
 }
 void amax_set_carry_valid(const void* data) {
   std::lock_guard<std::mutex> lk(g_ver_mu);
-  g_amax[data].carry_version = version_locked(data);
+  g_amax[data].carry_version = array_version_locked(data);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -2825,7 +2827,7 @@ static bool fuse_relu_packs() {
   return on;
 }
 static const void* bound_key(const void* y) { return (const char*)y + 1; }
-// Before y = relu(x) runs on its own: the word that bounds max|x|, if there is one, and the word that the kernel copies it to.
+// Before y = relu(x) runs on its own, after the version bump: the word that bounds max|x|, if there is one, and the word that the kernel copies it to.
 ReluBound tc_relu_bound(const float* x, const float* y) {
   if (!fuse_relu_packs() || x == y || tensor_arithmetic() != kArithF16) return ReluBound{};
   const uint32_t* from = amax_tracked(x);

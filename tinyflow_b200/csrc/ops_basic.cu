@@ -1348,8 +1348,9 @@ int DLGpuActivationForward(const DLArrayHandle input, DLArrayHandle output, int 
       if (fused < 0) return -1;
       if (fused) return 0;
       FReluKeep relu;
-      if (node && aligned16(input->data) && aligned16(output->data)) relu.bound = tc_relu_bound(F(input), F(output));
-      int rc = relu.bound.to ? run_map1(F(input), FM(output), n, s, "DLGpuActivationForward(relu)", relu) : run_map1(F(input), FM(output), n, s, "DLGpuActivationForward(relu)", FRelu{});
+      float* const y = FM(output);
+      if (node && aligned16(input->data) && aligned16(y)) relu.bound = tc_relu_bound(F(input), y);
+      int rc = relu.bound.to ? run_map1(F(input), y, n, s, "DLGpuActivationForward(relu)", relu) : run_map1(F(input), y, n, s, "DLGpuActivationForward(relu)", FRelu{});
       tc_note_relu_output(node, output->data, input->data, relu.bound.to != nullptr);
       return rc;
     }
