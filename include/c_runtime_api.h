@@ -330,6 +330,7 @@ int TfPackFilters(const DLArrayHandle *filters, void ***const *plans, int n, voi
  * the stream it was called on (the sums without a stream argument: the stream they run on).  Until then nothing may read the result, the arrays that the
  * call reads may be neither freed nor written, and no other thread may call or release the convolution's descriptor.
  * What waits was called on one stream; calls on another one meanwhile do not wait, and TfLaunchHeld there launches nothing.
+ * DLGpuDestroycudaStream launches what the thread called on the stream.
  * A call sees to what memory it needs on its own before it waits, and reports a shortage as it does without waiting.  After an
  * error of TfLaunchHeld nothing waits.  TfDropHeld forgets what waits (a step that failed) and ends the holding. */
 int TfHoldProducts(int on);

@@ -255,6 +255,36 @@ def test_a_released_descriptor_lets_what_waits_go_first(lib_path):
         gpu_op.drop_held()
 
 
+def test_what_waits_goes_before_its_stream(lib_path):
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, stream, later, rng = nd.gpu(0), gpu_op.create_cudaStream(), gpu_op.create_cudaStream(), np.random.RandomState(8)
+    handle = gpu_op.create_cudnnHandle(later)
+    N, C, H, W, K, R, S, u = LAYERS[4]
+    out, cell = gpu_op.convolution_2d_forward_get_out_shape((N, C, H, W), (K, C, R, S), "NCHW", "SAME", u, u)
+    x, w, dy = (nd.array(rng.randn(*shape).astype(np.float32), ctx) for shape in ((N, C, H, W), (K, C, R, S), out))
+    sums = gpu_op.reduce_sum_get_cudnnlist(*gpu_op.reduce_sum_get_real_shape(out, (K,), "NCHW"), "NCHW", handle)
+    apart, waits = ([nd.array(np.full(s, np.nan, np.float32), ctx) for s in ((K, C, R, S), (K,))] for _ in range(2))
+
+    def run(into, on):
+        gpu_op.convolution_backward_filter(x, dy, w, into[0], cell, handle, on)
+        gpu_op.reduce_sum_new(dy, into[1], sums, handle, on)
+    try:
+        run(apart, later)
+        gpu_op.device_synchronize()
+        gpu_op.hold_products(True)
+        run(waits, stream)
+        gpu_op.destroy_cudaStream(stream)
+        again = [nd.array(np.full(a.shape, np.nan, np.float32), ctx) for a in apart]
+        run(again, later)                                          # waits in its turn
+        gpu_op.hold_products(False)
+        gpu_op.launch_held(later)
+        for got in (waits, again):
+            for a, b in zip(got, apart):
+                np.testing.assert_array_equal(a.asnumpy(), b.asnumpy())
+    finally:
+        gpu_op.drop_held()
+
+
 def _half_way(monkeypatch, ex, node, feed):
     """A step that ends with an error at `node`, behind gradients that wait."""
     import random

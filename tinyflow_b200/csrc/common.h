@@ -130,6 +130,7 @@ __device__ __forceinline__ void amax_commit(const AmaxOut& am, uint32_t m) {
 // A gradient's call may wait for others (see hold_products in gemm_tcgen05.cu) until launch_held(): true, and the caller keeps it until
 // its own launch_held_...() is called
 bool may_hold(cudaStream_t s);
+int launch_held(cudaStream_t s);               // what waits if it was called on this stream
 template <class T> inline bool held(std::vector<T>& waiting, const T& call) {        // false: no memory to remember it; the call is launched now
   try { waiting.push_back(call); } catch (const std::bad_alloc&) { return false; }
   return true;

@@ -21,7 +21,6 @@ int tc_matmul(const float* A, bool tA, const float* B, bool tB, float* C, int64_
 int tc_conv_fwd(ConvPlan* p, const float* x, const float* w, float* y, cudaStream_t s, int* oom_bytes);
 int tc_conv_dgrad(ConvPlan* p, const float* dy, const float* w, float* dx, cudaStream_t s, int* oom_bytes);
 void hold_products(bool on);
-int launch_held(cudaStream_t s);
 void drop_held();
 int tc_conv_wgrad(ConvPlan* p, const float* x, const float* dy, float* dw, cudaStream_t s, int* oom_bytes);
 

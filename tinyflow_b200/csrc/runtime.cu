@@ -574,6 +574,7 @@ int DLGpuCreatecudaStream(void** cudaStream) {
 int DLGpuDestroycudaStream(void** cudaStream) {
   TF_REQUIRE(cudaStream, "null cell");
   cudaStream_t s = (cudaStream_t)*cudaStream;
+  if (launch_held(s)) return -1;         // what this thread called on it and waits; after an error nothing waits
   if (last_compute_stream() == s) note_compute_stream(0);
   TF_CUDA(cudaStreamSynchronize(s));
   release_stream_scratch(s);

@@ -21,7 +21,6 @@ thread_local StepGraph* t_recording = nullptr;
 static std::atomic<uint64_t> g_layout_epoch{1};
 void bump_layout_epoch() { g_layout_epoch.fetch_add(1, std::memory_order_relaxed); }
 int tensor_path_error();
-int launch_held(cudaStream_t s);
 int launch_waiting();
 void drop_held();
 void tc_recording_begins();
