@@ -285,6 +285,43 @@ def test_what_waits_goes_before_its_stream(lib_path):
         gpu_op.drop_held()
 
 
+# called before the caller's own capture begins, launched inside: the graph names nothing that is gone when it is replayed
+def test_what_waits_is_launched_in_a_capture(lib_path):
+    import ctypes
+    import torch
+    from tinyflow_b200 import gpu_op, ndarray as nd
+    ctx, rng = nd.gpu(0), np.random.RandomState(9)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    stream = ctypes.pointer(ctypes.c_void_p(side.cuda_stream))
+    handle = gpu_op.create_cudnnHandle(stream)
+    calls = []
+    for N, C, H, W, K, R, S, u in LAYERS[1:5] + DIRECT[:2]:           # (tiles of 96 columns, LAYERS[0], do not wait)
+        out, cell = gpu_op.convolution_2d_forward_get_out_shape((N, C, H, W), (K, C, R, S), "NCHW", "VALID" if u > 1 else "SAME", u, u)
+        x, w, dy = (nd.array(rng.randn(*shape).astype(np.float32), ctx) for shape in ((N, C, H, W), (K, C, R, S), out))
+        calls.append((x, dy, w, cell) + tuple(nd.array(np.full((K, C, R, S), np.nan, np.float32), ctx) for _ in range(2)))
+    try:
+        for call in calls:
+            gpu_op.convolution_backward_filter(*call[:3], call[4], call[3], handle, stream)
+        before = gpu_op.launch_count()
+        gpu_op.hold_products(True)
+        for call in calls:
+            gpu_op.convolution_backward_filter(*call[:3], call[5], call[3], handle, stream)
+        gpu_op.hold_products(False)
+        assert gpu_op.launch_count() == before
+        gpu_op.device_synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            gpu_op.launch_held(stream)
+        for _ in range(3):
+            for call in calls:
+                call[5][:] = np.full(call[5].shape, np.nan, np.float32)
+            graph.replay()
+            torch.cuda.synchronize()
+            for call in calls:
+                np.testing.assert_array_equal(call[5].asnumpy(), call[4].asnumpy())
+    finally:
+        gpu_op.drop_held()
+
+
 def _half_way(monkeypatch, ex, node, feed):
     """A step that ends with an error at `node`, behind gradients that wait."""
     import random

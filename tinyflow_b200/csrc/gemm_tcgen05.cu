@@ -2324,10 +2324,12 @@ constexpr size_t kStagedCopy = 1 << 16;
 // Partial sums that the products of one launch may have between them: the largest of the benchmark's graphs has 345 MB (DenseNet-121 at
 // batch 56), one product on its own 10 MB at most.
 constexpr size_t kGroupBytes = size_t(512) << 20;
-// 0: launched, -1: error, 1: too many at once, or no memory for the table or the partial sums; nothing was launched
+// 0: launched, -1: error, 1: too many at once, no memory for the table or the partial sums, or a graph of the caller's own is being captured
+// (its copy of the table would read host memory that is gone at a replay); nothing was launched
 template <int BN, int AR> static int launch_group(HeldProduct* const* products, int n, cudaStream_t s) {
   static const cudaError_t attr = cudaFuncSetAttribute(gemm3x_group_kernel<BN, AR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGroupSmem<BN>);
   TF_CUDA(attr);
+  if (!t_recording && capturing(s)) return 1;
   const int sms = device_sm_count();
   // Whole tiles, or chunks of their pieces, up to half of a CTA's share (a fifth: 0.3 % slower); longer reductions as their pieces.  Longest first, to the CTA that is free first.
   constexpr int kItemCost = 4;                        // an item's start and end, in stages
